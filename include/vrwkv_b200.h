@@ -69,6 +69,13 @@ int vrwkv_set_path(int path);
  * no reference counterpart (the reference never checks its launches). */
 int vrwkv_workspace_status(const void* workspace, void* stream, unsigned* status_out);
 
+/* Failure bits (as in vrwkv_workspace_status) that launches on `device` have reported since the last call, and
+ * clears them; 0 if none.  Kernels that give up a bounded wait write the word through mapped host memory, so the
+ * call is one read of host memory: no synchronisation, no copy.  A launch that is still running reports later:
+ * synchronise first to see its result.  The first call (per process) sets the word up; launches made before it
+ * report through their workspace only. */
+unsigned vrwkv_take_failures(int device);
+
 /* ---- Bi-WKV --------------------------------------------------------------------
  * y[b,t,c] = sum_j p_tj v[b,j,c] / sum_j p_tj,  log p_tj = k[b,j,c] - w[c]|t-j| for
  * j != t and u[c] + k[b,t,c] for j == t.  w, u: (C,).

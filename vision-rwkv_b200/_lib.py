@@ -6,9 +6,10 @@ the caller gets an exception.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
-from ._build import LIB_PATH
+from ._build import LIB_PATH, NATIVE_PATH
 
 _c_int = ctypes.c_int
 _c_size_t = ctypes.c_size_t
@@ -22,6 +23,7 @@ SIGNATURES = {
     "vrwkv_launch_count": (ctypes.c_ulonglong, []),
     "vrwkv_set_path": (_c_int, [_c_int]),
     "vrwkv_workspace_status": (_c_int, [_ptr, _ptr, ctypes.POINTER(ctypes.c_uint)]),
+    "vrwkv_take_failures": (ctypes.c_uint, [_c_int]),
     "vrwkv_biwkv_forward_workspace_bytes": (_c_size_t, [_c_int] * 3),
     "vrwkv_biwkv_forward_f32": (_c_int, [_c_int] * 3 + [_ptr] * 6 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_backward_workspace_bytes": (_c_size_t, [_c_int] * 3),
@@ -73,8 +75,28 @@ def load():
         fn = getattr(lib, name)       # AttributeError if the symbol is not exported
         fn.restype = restype
         fn.argtypes = argtypes
+    lib.vrwkv_take_failures(-1)          # sets the failure words up before the first launch
     _lib = lib
     return lib
+
+
+_native = None
+
+
+def native():
+    """The torch extension: the operators' host path (checks, allocation, autograd) in C++ over the same library."""
+    global _native
+    if _native is None:
+        load()
+        if not os.path.exists(NATIVE_PATH):
+            raise VrwkvError(f"{NATIVE_PATH} is missing: build it first (python -m vision_rwkv_b200._build).")
+        import torch  # noqa: F401  (its libraries have to be in the process first)
+        spec = importlib.util.spec_from_file_location("_native", NATIVE_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.set_error_class(VrwkvError)
+        _native = module
+    return _native
 
 
 def check(status: int, what: str):

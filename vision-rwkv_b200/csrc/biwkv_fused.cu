@@ -99,6 +99,7 @@ struct Params {
     float* exch;       // [n_tiles][levels][kRows][kCs]
     unsigned* flags;   // [n_tiles][levels], zero before launch, 2 when both halves are written
     unsigned* status;  // device status word
+    unsigned* mirror;  // host-visible copy of a failure (may be null)
     float* partial;    // backward: [n_tiles][2][kCs]
     const unsigned* run_if;   // when set: every kernel of the launch returns at once while this word is zero
 };
@@ -310,7 +311,7 @@ __device__ __forceinline__ Entering exchange_collect(const Params& p, float* ext
             }
             const unsigned seen_all = seen[0] | seen[1] | seen[2] | seen[3];
             const size_t dep = seen_all >> 31;
-            if (!ok && lane == 0) atomicOr(p.status, 1u);
+            if (!ok && lane == 0) report_failure(p.status, p.mirror, 1u);
             // all loads of the batch first, then the arithmetic
             float r0[4], r1[4], r2[4], r3[4], x[4];
             float mP = kMinExp, mS = kMinExp;
@@ -547,7 +548,7 @@ biwkv_fused_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             const int next = tile + gridDim.x;
             if (next < p.n_tiles) issue_loads(next, stage ^ 1);
         }
-        if (!sm100::mbar_wait(&full[stage], (it >> 1) & 1, kSpinLimit)) atomicOr(p.status, 2u);
+        if (!sm100::mbar_wait(&full[stage], (it >> 1) & 1, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
         const int t0 = tc.chunk * kTc + warp * kL;               // first token of this sub-chunk
         const int n = max(0, min(kL, p.T - t0));
         const Col<E> ks(slot_k, warp, lane), vs(slot_v, warp, lane), gs(slot_g, warp, lane);
@@ -790,7 +791,7 @@ biwkv_forward_pipelined_kernel(const __grid_constant__ CUtensorMap map_k, const 
             const int c = tc.strip * kCs + lane;
             const float w = (c < p.C) ? p.w[c] : 0.f;
             const float u = (c < p.C) ? p.u[c] : 0.f;
-            if (!sm100::mbar_wait(&full[stage], (n / kFwdStages) & 1, kSpinLimit)) atomicOr(p.status, 2u);
+            if (!sm100::mbar_wait(&full[stage], (n / kFwdStages) & 1, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
             const int nv = max(0, min(kL, p.T - (tc.chunk * kTc + warp * kL)));
             const Col<E> ks(stage_base + stage * kStageBytes, warp, lane);
             const Col<E> vs(stage_base + stage * kStageBytes + kSlotBytes<E>, warp, lane);
@@ -1016,7 +1017,7 @@ __device__ __forceinline__ Entering4 exchange_collect4(const Params& p, float* e
             }
             const unsigned seen_all = seen[0] | seen[1] | seen[2] | seen[3];
             const size_t dep = seen_all >> 31;
-            if (!ok && lane == 0) atomicOr(p.status, 1u);
+            if (!ok && lane == 0) report_failure(p.status, p.mirror, 1u);
             float r0[4], r1[4], r2[4], r3[4], x[4];
             float mP = kMinExp, mS = kMinExp;
 #pragma unroll
@@ -1177,7 +1178,7 @@ biwkv_backward_saved_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         const int c = tc.strip * kCs + lane;
         const float w = (c < p.C) ? p.w[c] : 0.f;
         const float u = (c < p.C) ? p.u[c] : 0.f;
-        if (!sm100::mbar_wait(full, it & 1, kSpinLimit)) atomicOr(p.status, 2u);
+        if (!sm100::mbar_wait(full, it & 1, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
         const int t0 = tc.chunk * kTc + warp * kL;
         const int n = max(0, min(kL, p.T - t0));
         const Col<float> ks(slots, warp, lane), vs(slots + kSlot, warp, lane), gs(slots + 2 * kSlot, warp, lane);
@@ -1418,6 +1419,7 @@ static int launch(Layout& l, const float* w, const float* u, const E* k, const E
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     p.w = w; p.u = u;
     p.status = reinterpret_cast<unsigned*>(ws + l.off_status);
+    p.mirror = failure_mirror();
     p.flags = reinterpret_cast<unsigned*>(ws + l.off_flags);
     p.exch = reinterpret_cast<float*>(ws + l.off_exch);
     p.partial = reinterpret_cast<float*>(ws + l.off_partial);
@@ -1526,6 +1528,7 @@ int backward_saved(int B, int T, int C, const float* w, const float* u, const fl
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     p.w = w; p.u = u;
     p.status = reinterpret_cast<unsigned*>(ws + l.off_status);
+    p.mirror = failure_mirror();
     p.flags = reinterpret_cast<unsigned*>(ws + l.off_flags);
     p.exch = reinterpret_cast<float*>(ws + l.off_exch);
     p.partial = reinterpret_cast<float*>(ws + l.off_partial);

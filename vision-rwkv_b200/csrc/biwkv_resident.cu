@@ -95,6 +95,7 @@ struct Params {
     const float* w;
     const float* u;
     unsigned* status;   // device status word
+    unsigned* mirror;   // host-visible copy of a failure (may be null)
     float* partial;     // backward: [grid][2][kCs]
     unsigned* redo_count;   // units the fast kernel left to the exact kernel ...
     int* redo_list;         // ... and which
@@ -204,6 +205,7 @@ struct Ctx {
     float* consts;   // [kConstRows][kCs]
     uint64_t* xbar;  // [kLevels] mbarriers counting the bytes the other CTAs send
     unsigned* status;
+    unsigned* mirror;
     uint32_t spin_limit;
     bool withhold;   // test only: this CTA sends nothing to the others
     int warp, lane, n_warps, n_tok, cluster, rank;
@@ -288,7 +290,7 @@ __device__ __forceinline__ unsigned seg_wait(const Ctx& c, int first, int count,
         }
         if (seen) seen = sm100::flag_acquire(f);
     }
-    if (!__all_sync(0xffffffffu, seen != 0u) && c.lane == 0) atomicOr(c.status, 4u);
+    if (!__all_sync(0xffffffffu, seen != 0u) && c.lane == 0) report_failure(c.status, c.mirror, 4u);
     unsigned bits = seen;
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, m);
@@ -499,7 +501,7 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     TL_MARK(13 + level * 5);
     // (3) wait for the other CTAs' bytes, combine them
     if (c.cluster > 1 && (warp == scanF || warp == scanR)) {
-        if (!sm100::mbar_wait(c.xbar + level, 0, c.spin_limit) && lane == 0) atomicOr(c.status, 1u);
+        if (!sm100::mbar_wait(c.xbar + level, 0, c.spin_limit) && lane == 0) report_failure(c.status, c.mirror, 1u);
     }
     TL_MARK(14 + level * 5);
     if (warp == scanF) {
@@ -807,6 +809,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     c.xbar = gfull + kMaxWarps;
     c.flag = reinterpret_cast<unsigned*>(c.xbar + 2);
     c.status = p.status;
+    c.mirror = p.mirror;
     c.warp = warp; c.lane = lane; c.n_warps = nw; c.n_tok = p.n_tok; c.cluster = p.cluster;
     c.rank = p.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
     c.spin_limit = p.spin_limit;
@@ -906,7 +909,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     const float2 c2 = *reinterpret_cast<const float2*>(c.consts + kCuw * kCs + 2 * pr);
 
     TL_MARK(1);
-    if (!sm100::mbar_wait(full + warp, 0, kSpinLimit)) atomicOr(p.status, 2u);
+    if (!sm100::mbar_wait(full + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
     if (p.cluster > 1) cluster_wait();
     TL_MARK(2);
 
@@ -971,7 +974,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     TL_MARK(4);
 
     float2 gw = f2(0.f, 0.f), gu = f2(0.f, 0.f);
-    if (kBwd && !sm100::mbar_wait(gfull + warp, 0, kSpinLimit)) atomicOr(p.status, 2u);
+    if (kBwd && !sm100::mbar_wait(gfull + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
     if (unsafe) {
         // the whole cluster takes this branch together: the unit is left to the exact kernel, which
         // runs right after this one (nothing of this CTA is in flight any more: its tiles have
@@ -1200,6 +1203,7 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     c.xbar = full + 1;
     c.flag = reinterpret_cast<unsigned*>(full + 4);
     c.status = p.status;
+    c.mirror = p.mirror;
     c.spin_limit = kSpinLimit;
     c.withhold = false;
     c.seg = 0; c.segs = 1; c.unit = 0; c.xseg = nullptr; c.xflag = nullptr;
@@ -1244,7 +1248,7 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         const int ch0 = strip * kCs + 2 * pr;
         const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
         const float2 u2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.u + ch0) : f2(0.f, 0.f);
-        if (!sm100::mbar_wait(full, phase, kSpinLimit)) atomicOr(p.status, 2u);
+        if (!sm100::mbar_wait(full, phase, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
         phase ^= 1u;
         if (kHalf) {
             // widen this thread's 16 rows in place, walking up (see ld_in)
@@ -1485,6 +1489,7 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     p.w = w; p.u = u;
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     p.status = reinterpret_cast<unsigned*>(ws);
+    p.mirror = failure_mirror();
     const size_t units = static_cast<size_t>(B) * p.n_strips;
     const Carve cv = carve(B, C, pl, kBwd);
     p.redo_count = reinterpret_cast<unsigned*>(ws) + 1;

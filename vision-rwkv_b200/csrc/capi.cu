@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include "vrwkv_b200.h"
 #include "vrwkv_internal.h"
 
@@ -38,6 +39,21 @@ void set_error_detail(const char* text) {
 }
 
 int record_launches(int launched) { return finish(launched); }
+
+// One word per device in pinned, mapped host memory: kernels write it only when a bounded wait runs out, the host
+// reads it as ordinary memory, so watching for failures costs neither a copy nor an event per launch.
+namespace {
+constexpr int kMirrorDevices = 64;
+std::atomic<unsigned*> g_mirror{nullptr};
+std::mutex g_mirror_mutex;
+}  // namespace
+
+unsigned* failure_mirror() {
+    unsigned* base = g_mirror.load(std::memory_order_acquire);
+    int dev = 0;
+    if (base == nullptr || cudaGetDevice(&dev) != cudaSuccess || dev >= kMirrorDevices) return nullptr;
+    return base + dev;
+}
 
 extern "C" {
 
@@ -78,6 +94,34 @@ int vrwkv_workspace_status(const void* workspace, void* stream, unsigned* status
         return VRWKV_ERR_LAUNCH;
     }
     return VRWKV_OK;
+}
+
+unsigned vrwkv_take_failures(int device) {
+    unsigned* base = g_mirror.load(std::memory_order_acquire);
+    if (base == nullptr) {
+        std::lock_guard<std::mutex> lock(g_mirror_mutex);
+        base = g_mirror.load(std::memory_order_acquire);
+        if (base == nullptr) {
+            // not an operation a stream capture may contain: leave the thread's capture mode out of it
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            void* p = nullptr;
+            const cudaError_t err = cudaHostAlloc(&p, kMirrorDevices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (err != cudaSuccess) {
+                cudaGetLastError();
+                return 0;
+            }
+            std::memset(p, 0, kMirrorDevices * sizeof(unsigned));
+            base = static_cast<unsigned*>(p);
+            g_mirror.store(base, std::memory_order_release);
+        }
+    }
+    if (device < 0 || device >= kMirrorDevices) return 0;
+    volatile unsigned* word = base + device;
+    const unsigned bits = *word;
+    if (bits != 0) *word = 0;
+    return bits;
 }
 
 // The resident kernels' workspace; for sequences of several segments the chunked kernels' workspace follows it

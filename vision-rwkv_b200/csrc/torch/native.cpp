@@ -1,0 +1,292 @@
+// Host path of the operators as a torch extension: the checks, allocations, dtype rules and autograd
+// nodes that sit between a model's call and the C ABI, in C++.
+//
+// A call on a small input is all host time: through ctypes and a Python autograd Function a forward took
+// 65 us of which the GPU worked 11.  The rules are those of the reference's Python wrappers
+// (classification/mmcls_custom/models/backbones/vrwkv.py:29-65, vrwkv6.py:22-73); the Python modules
+// above this file keep the public names.
+#include <torch/csrc/utils/pybind.h>
+#include "glue.h"
+#include "native.h"
+
+namespace vrwkv {
+
+namespace {
+PyObject* g_error_class = nullptr;     // vision_rwkv_b200._lib.VrwkvError
+}
+
+void raise(const std::string& text) {
+    pybind11::gil_scoped_acquire gil;
+    PyErr_SetString(g_error_class ? g_error_class : PyExc_RuntimeError, text.c_str());
+    python_error e;
+    e.persist();
+    throw e;
+}
+
+void raise_status(int status, const char* what) {
+    std::string text = std::string(what) + " failed with status " + std::to_string(status) + ": " + vrwkv_status_string(status);
+    const char* detail = vrwkv_last_error_detail();
+    if (detail && *detail) text += std::string(" [") + detail + "]";
+    raise(text);
+}
+
+void raise_failures(int device, const char* what) {
+    const unsigned bits = vrwkv_take_failures(device);
+    if (bits == 0) return;
+    char word[16];
+    snprintf(word, sizeof(word), "%#x", bits);
+    raise(std::string("device status word ") + word + ", seen at " + what +
+          " (a bounded device-side wait ran out in an earlier launch: its outputs, and everything computed from them, are invalid)");
+}
+
+namespace {
+
+void check_cuda(const Tensor& t, const char* name, const Tensor& like) {
+    TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor");
+    TORCH_CHECK(t.device() == like.device(), name, " is on ", t.device(), ", expected ", like.device());
+}
+
+// ---- Bi-WKV ------------------------------------------------------------------------------------
+void check_biwkv(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+    check_cuda(k, "k", k);
+    check_cuda(v, "v", k);
+    check_cuda(w, "w", k);
+    check_cuda(u, "u", k);
+    TORCH_CHECK(k.dim() == 3, "k must be (B, T, C), got ", k.sizes());
+    TORCH_CHECK(v.sizes() == k.sizes(), "k, v (and gy) must have the same shape");
+    TORCH_CHECK(w.numel() == k.size(2) && u.numel() == k.size(2), "w and u must hold C=", k.size(2), " values");
+}
+
+at::ScalarType result_dtype(const Tensor& w) {
+    return w.scalar_type() == at::kHalf || w.scalar_type() == at::kBFloat16 ? w.scalar_type() : at::kFloat;
+}
+
+// k, v float32 or both bfloat16, contiguous; y in their dtype
+Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+    const int B = k.size(0), T = k.size(1), C = k.size(2);
+    Tensor y = at::empty_like(k);
+    if (k.numel() == 0) return y;
+    Tensor ws = workspace(vrwkv_biwkv_forward_workspace_bytes(B, T, C), k);
+    if (is_bf16(k)) {
+        const int st = vrwkv_biwkv_forward_bf16(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
+                                                static_cast<uint16_t*>(v.data_ptr()), static_cast<uint16_t*>(y.data_ptr()),
+                                                ws.data_ptr(), ws.numel(), stream_of(k));
+        if (st == VRWKV_ERR_UNSUPPORTED) return biwkv_forward_raw(w, u, f32(k), f32(v)).to(at::kBFloat16);
+        check(st, "vrwkv_biwkv_forward_bf16");
+    } else {
+        check(vrwkv_biwkv_forward_f32(B, T, C, fp(w), fp(u), fp(k), fp(v), fp(y), ws.data_ptr(), ws.numel(), stream_of(k)),
+              "vrwkv_biwkv_forward_f32");
+    }
+    raise_failures(k.get_device(), "vrwkv_biwkv_forward");
+    return y;
+}
+
+Tensor biwkv_forward(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, bool bf16_io) {
+    const c10::cuda::CUDAGuard guard(k.device());
+    const bool half = bf16_io && is_bf16(k) && is_bf16(v);
+    const Tensor y = half ? biwkv_forward_raw(f32(w), f32(u), k.contiguous(), v.contiguous())
+                          : biwkv_forward_raw(f32(w), f32(u), f32(k), f32(v));
+    return y.to(result_dtype(w));
+}
+
+std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& gy) {
+    const int B = k.size(0), T = k.size(1), C = k.size(2);
+    Tensor gk = at::empty_like(k), gv = at::empty_like(k);
+    Tensor gwgu = at::empty({2, C}, k.options().dtype(at::kFloat));
+    if (k.numel() == 0) {
+        gwgu.zero_();
+        return {gwgu.select(0, 0), gwgu.select(0, 1), gk, gv};
+    }
+    Tensor ws = workspace(vrwkv_biwkv_backward_workspace_bytes(B, T, C), k);
+    if (is_bf16(k)) {
+        const int st = vrwkv_biwkv_backward_bf16(
+            B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()),
+            static_cast<uint16_t*>(gy.data_ptr()), fp(gwgu), static_cast<uint16_t*>(gk.data_ptr()),
+            static_cast<uint16_t*>(gv.data_ptr()), ws.data_ptr(), ws.numel(), stream_of(k));
+        if (st == VRWKV_ERR_UNSUPPORTED) {
+            auto g = biwkv_backward_raw(w, u, f32(k), f32(v), f32(gy));
+            return {g[0], g[1], g[2].to(at::kBFloat16), g[3].to(at::kBFloat16)};
+        }
+        check(st, "vrwkv_biwkv_backward_bf16");
+    } else {
+        check(vrwkv_biwkv_backward_f32(B, T, C, fp(w), fp(u), fp(k), fp(v), fp(gy), fp(gwgu), fp(gk), fp(gv), ws.data_ptr(),
+                                       ws.numel(), stream_of(k)),
+              "vrwkv_biwkv_backward_f32");
+    }
+    raise_failures(k.get_device(), "vrwkv_biwkv_backward");
+    return {gwgu.select(0, 0), gwgu.select(0, 1), gk, gv};
+}
+
+struct BiWkv : torch::autograd::Function<BiWkv> {
+    static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& w, const Tensor& u, const Tensor& k,
+                          const Tensor& v, bool bf16_io) {
+        Tensor y = biwkv_forward(w, u, k, v, bf16_io);
+        ctx->save_for_backward({w, u, k, v});
+        ctx->saved_data["bf16_io"] = bf16_io;
+        return y;
+    }
+    static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &w = saved[0], &u = saved[1], &k = saved[2], &v = saved[3], &gy = grads[0];
+        const c10::cuda::CUDAGuard guard(k.device());
+        const at::NoGradGuard no_grad;
+        const at::ScalarType out = result_dtype(w);
+        const bool half = ctx->saved_data["bf16_io"].toBool() && is_bf16(k) && is_bf16(v);
+        auto g = half ? biwkv_backward_raw(f32(w), f32(u), k.contiguous(), v.contiguous(), gy.to(at::kBFloat16).contiguous())
+                      : biwkv_backward_raw(f32(w), f32(u), f32(k), f32(v), f32(gy));
+        // on the bfloat16 path gk, gv stay bfloat16 (what autograd hands to a bfloat16 k anyway) unless w is half
+        if (!half || out == at::kHalf) { g[2] = g[2].to(out); g[3] = g[3].to(out); }
+        return {g[0].to(out), g[1].to(out), g[2], g[3], Tensor()};
+    }
+};
+
+Tensor biwkv(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, bool bf16_io) {
+    check_biwkv(w, u, k, v);
+    if (!any_requires_grad({&w, &u, &k, &v})) return biwkv_forward(w, u, k, v, bf16_io);
+    return BiWkv::apply(w, u, k, v, bf16_io);
+}
+
+// ---- WKV6 --------------------------------------------------------------------------------------
+bool all_bf16(std::initializer_list<const Tensor*> ts) {
+    for (const Tensor* t : ts)
+        if (!is_bf16(*t)) return false;
+    return true;
+}
+
+void check_wkv6(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w,
+                const Tensor& u) {
+    check_cuda(r, "r", r);
+    check_cuda(k, "k", r);
+    check_cuda(v, "v", r);
+    check_cuda(w, "w", r);
+    check_cuda(u, "u", r);
+    TORCH_CHECK(r.dim() == 3 && r.size(0) == B && r.size(1) == T && r.size(2) == C, "r has shape ", r.sizes(), ", expected (", B, ", ",
+                T, ", ", C, ")");
+    TORCH_CHECK(k.sizes() == r.sizes(), "k must have the shape of r");
+    TORCH_CHECK(v.sizes() == r.sizes(), "v must have the shape of r");
+    TORCH_CHECK(w.sizes() == r.sizes(), "w must have the shape of r");
+    TORCH_CHECK(C == 64 * H, "head size must be 64: C=", C, ", H=", H);
+    TORCH_CHECK(u.numel() == C, "u must hold C=", C, " values");
+}
+
+Tensor wkv6_forward(int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w_, const Tensor& u_,
+                    bool tensor_cores) {
+    const c10::cuda::CUDAGuard guard(r.device());
+    const int B = r.size(0), T = r.size(1), C = r.size(2);
+    const Tensor w = f32(w_), u = f32(u_);
+    Tensor y = at::empty({B, T, C}, r.options().dtype(at::kFloat));
+    if (y.numel() == 0) return y;
+    if (tensor_cores) {
+        Tensor ws = workspace(256, r);
+        if (all_bf16({&r, &k, &v})) {
+            check(vrwkv_wkv6_forward_tc_bf16(B, T, C, H, static_cast<uint16_t*>(r.data_ptr()), static_cast<uint16_t*>(k.data_ptr()),
+                                             static_cast<uint16_t*>(v.data_ptr()), fp(w), fp(u), fp(y), ws.data_ptr(), ws.numel(),
+                                             stream_of(r)),
+                  "vrwkv_wkv6_forward_tc_bf16");
+        } else {
+            const Tensor r32 = f32(r), k32 = f32(k), v32 = f32(v);
+            check(vrwkv_wkv6_forward_tc_f32(B, T, C, H, fp(r32), fp(k32), fp(v32), fp(w), fp(u), fp(y), ws.data_ptr(), ws.numel(),
+                                            stream_of(r)),
+                  "vrwkv_wkv6_forward_tc_f32");
+        }
+        raise_failures(r.get_device(), "vrwkv_wkv6_forward_tc");
+        return y;
+    }
+    const Tensor r32 = f32(r), k32 = f32(k), v32 = f32(v);
+    check(vrwkv_wkv6_forward_f32(B, T, C, H, fp(r32), fp(k32), fp(v32), fp(w), fp(u), fp(y), stream_of(r)), "vrwkv_wkv6_forward_f32");
+    return y;
+}
+
+struct Wkv6 : torch::autograd::Function<Wkv6> {
+    static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w,
+                          const Tensor& u, int64_t H, bool tensor_cores) {
+        Tensor y = wkv6_forward(H, r, k, v, w, u, tensor_cores);
+        ctx->save_for_backward({r, k, v, w, u});
+        ctx->saved_data["H"] = H;
+        ctx->saved_data["tc"] = tensor_cores;
+        return y;
+    }
+    static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &r = saved[0], &k = saved[1], &v = saved[2], &gy = grads[0];
+        const c10::cuda::CUDAGuard guard(r.device());
+        const at::NoGradGuard no_grad;
+        const int64_t H = ctx->saved_data["H"].toInt();
+        const int B = r.size(0), T = r.size(1), C = r.size(2);
+        const Tensor w = f32(saved[3]), u = f32(saved[4]);
+        const auto opt = r.options().dtype(at::kFloat);
+        Tensor gr = at::empty({B, T, C}, opt), gk = at::empty({B, T, C}, opt), gv = at::empty({B, T, C}, opt),
+               gw = at::empty({B, T, C}, opt), gu = at::empty({H, C / H}, opt);
+        if (gr.numel() == 0) {
+            gu.zero_();
+        } else if (ctx->saved_data["tc"].toBool()) {
+            Tensor ws = workspace(vrwkv_wkv6_backward_tc_workspace_bytes(B, T, C, H), r);
+            if (all_bf16({&r, &k, &v})) {
+                const Tensor g = gy.to(at::kBFloat16).contiguous();
+                check(vrwkv_wkv6_backward_tc_bf16(B, T, C, H, static_cast<uint16_t*>(r.data_ptr()), static_cast<uint16_t*>(k.data_ptr()),
+                                                  static_cast<uint16_t*>(v.data_ptr()), fp(w), fp(u), static_cast<uint16_t*>(g.data_ptr()),
+                                                  fp(gr), fp(gk), fp(gv), fp(gw), fp(gu), ws.data_ptr(), ws.numel(), stream_of(r)),
+                      "vrwkv_wkv6_backward_tc_bf16");
+            } else {
+                const Tensor r32 = f32(r), k32 = f32(k), v32 = f32(v), g = f32(gy);
+                check(vrwkv_wkv6_backward_tc_f32(B, T, C, H, fp(r32), fp(k32), fp(v32), fp(w), fp(u), fp(g), fp(gr), fp(gk), fp(gv),
+                                                 fp(gw), fp(gu), ws.data_ptr(), ws.numel(), stream_of(r)),
+                      "vrwkv_wkv6_backward_tc_f32");
+            }
+            raise_failures(r.get_device(), "vrwkv_wkv6_backward_tc");
+        } else {
+            const Tensor r32 = f32(r), k32 = f32(k), v32 = f32(v), g = f32(gy);
+            Tensor ws = workspace(vrwkv_wkv6_backward_workspace_bytes(B, T, C, H), r);
+            check(vrwkv_wkv6_backward_f32(B, T, C, H, fp(r32), fp(k32), fp(v32), fp(w), fp(u), fp(g), fp(gr), fp(gk), fp(gv), fp(gw),
+                                          fp(gu), ws.data_ptr(), ws.numel(), stream_of(r)),
+                  "vrwkv_wkv6_backward_f32");
+        }
+        return {gr, gk, gv, gw, gu.view({H, C / H}), Tensor(), Tensor()};
+    }
+};
+
+Tensor wkv6(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w,
+            const Tensor& u, bool tensor_cores) {
+    check_wkv6(B, T, C, H, r, k, v, w, u);
+    if (!any_requires_grad({&r, &k, &v, &w, &u})) return wkv6_forward(H, r, k, v, w, u, tensor_cores);
+    return Wkv6::apply(r, k, v, w, u, H, tensor_cores);
+}
+
+// python_error carries its exception through C++; hand it back to the interpreter at the boundary
+template <typename F>
+auto guarded(F f) {
+    return [f](auto... args) {
+        try {
+            pybind11::gil_scoped_release release;
+            return f(args...);
+        } catch (python_error& e) {
+            e.restore();
+            throw pybind11::error_already_set();
+        }
+    };
+}
+
+}  // namespace
+}  // namespace vrwkv
+
+PYBIND11_MODULE(_native, m) {
+    using at::Tensor;
+    m.def("set_error_class", [](pybind11::object cls) { vrwkv::g_error_class = cls.release().ptr(); });
+    m.def("biwkv", [](const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, bool bf16_io) {
+        return vrwkv::guarded([&] { return vrwkv::biwkv(w, u, k, v, bf16_io); })();
+    });
+    m.def("qshift_mix", [](const Tensor& x, std::vector<Tensor> mixes, int64_t H, int64_t W, int64_t shift, int64_t group, bool per_head) {
+        return vrwkv::guarded([&] { return vrwkv::qshift_mix(x, mixes, H, W, shift, group, per_head); })();
+    });
+    m.def("qshift_ddlerp", [](const Tensor& x, std::vector<Tensor> maas, std::vector<std::optional<Tensor>> offsets, int64_t H, int64_t W,
+                              int64_t shift, int64_t head_dim) {
+        return vrwkv::guarded([&] { return vrwkv::qshift_ddlerp(x, maas, offsets, H, W, shift, head_dim); })();
+    });
+    m.def("norm_gate", [](const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, int64_t group, double eps, int64_t act) {
+        return vrwkv::guarded([&] { return vrwkv::norm_gate(x, gate, weight, bias, group, eps, act); })();
+    });
+    m.def("wkv6", [](int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w,
+                     const Tensor& u, bool tensor_cores) {
+        return vrwkv::guarded([&] { return vrwkv::wkv6(B, T, C, H, r, k, v, w, u, tensor_cores); })();
+    });
+}

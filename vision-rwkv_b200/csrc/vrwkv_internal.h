@@ -8,6 +8,17 @@
 void set_error_detail(const char* text);
 // Add `launched` kernels to the process-wide count and turn the CUDA error state into a status.
 int record_launches(int launched);
+// Host-visible word of the current device that kernels set when a bounded wait runs out (pinned, mapped; null
+// until vrwkv_take_failures() has been called once).  It costs a successful launch nothing.
+unsigned* failure_mirror();
+
+#ifdef __CUDACC__
+// A bounded wait ran out: `status` is the launch's own device word, `mirror` the host-visible one (may be null).
+__device__ __forceinline__ void report_failure(unsigned* status, unsigned* mirror, unsigned bits) {
+    atomicOr(status, bits);
+    if (mirror != nullptr) *reinterpret_cast<volatile unsigned*>(mirror) = bits;
+}
+#endif
 
 namespace biwkv {
 // Each launcher returns the number of kernels it enqueued.

@@ -61,6 +61,7 @@ struct Args {
     const float* u;      // (H, 64)
     float* y;
     unsigned* status;    // set to 1 if a bounded wait ran out
+    unsigned* mirror;    // host-visible copy (may be null)
 };
 
 struct __align__(1024) Smem {
@@ -188,7 +189,7 @@ wkv6_tc_forward_kernel(const Args a, const __grid_constant__ CUtensorMap map_r, 
     uint32_t phase_main = 0, phase_score = 0, phase_load = 0;
     bool failed = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
-        if (!failed && !sm100::mbar_wait(bar, parity, kWaitLimit)) { failed = true; atomicExch(a.status, 1u); }
+        if (!failed && !sm100::mbar_wait(bar, parity, kWaitLimit)) { failed = true; report_failure(a.status, a.mirror, 1u); }
     };
 
     for (int step = 0; step < n_steps; ++step) {
@@ -559,7 +560,7 @@ wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r
 
     bool failed = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
-        if (!failed && !sm100::mbar_wait(bar, parity, kWaitLimit)) { failed = true; atomicExch(a.status, 1u); }
+        if (!failed && !sm100::mbar_wait(bar, parity, kWaitLimit)) { failed = true; report_failure(a.status, a.mirror, 1u); }
     };
 
     if (is_producer) {
@@ -864,6 +865,7 @@ struct MixArgs {
     float* out_left;     // sums over later source tokens
     float* dots;         // (B, T, H): p_t . q_t, written by the rightward CTAs when not null
     unsigned* status;
+    unsigned* mirror;
 };
 
 struct __align__(1024) SmemMix {
@@ -955,7 +957,7 @@ wkv6_tc_mix_kernel(const MixArgs a, const __grid_constant__ CUtensorMap map_a, c
     uint32_t phase_main = 0, phase_score = 0, phase_load = 0;
     bool failed = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
-        if (!failed && !sm100::mbar_wait(bar, parity, kWaitLimit)) { failed = true; atomicExch(a.status, 1u); }
+        if (!failed && !sm100::mbar_wait(bar, parity, kWaitLimit)) { failed = true; report_failure(a.status, a.mirror, 1u); }
     };
 
     for (int blk = 0; blk < n_blocks; ++blk) {
@@ -1405,7 +1407,7 @@ static int launch(int B, int T, int H, const void* r, const void* k, const void*
         return -1;
     }
     Args a{B, T, H, static_cast<const float*>(r), static_cast<const float*>(k), static_cast<const float*>(v), w_raw, u, y,
-           status};
+           status, failure_mirror()};
     if (clear_status) cudaMemsetAsync(status, 0, sizeof(unsigned), stream);
     if (pipelined || half_in) {
         // both directions add into y
@@ -1439,7 +1441,7 @@ static int launch_mix(int B, int T, int H, const void* a_, const void* p_, const
         set_error_detail("cuTensorMapEncodeTiled rejected a (C, T, B) tensor map");
         return -1;
     }
-    MixArgs m{B, T, H, a_, p_, q_, w_raw, out_right, out_left, dots, status};
+    MixArgs m{B, T, H, a_, p_, q_, w_raw, out_right, out_left, dots, status, failure_mirror()};
     if (half_in) wkv6_tc_mix_kernel<true><<<2 * B * H, kThreads, sizeof(SmemMix), stream>>>(m, ma, mp, mq, mw, mor, mol);
     else wkv6_tc_mix_kernel<false><<<2 * B * H, kThreads, sizeof(SmemMix), stream>>>(m, ma, mp, mq, mw, mor, mol);
     return 1;

@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import torch
 
-from .vrwkv import biwkv_backward_as_reference, biwkv_forward_as_reference
+from .vrwkv import _run, biwkv_backward_as_reference, biwkv_forward_as_reference
 
 
 class WKV(torch.autograd.Function):
@@ -32,4 +32,7 @@ class WKV(torch.autograd.Function):
 
 
 def RUN_CUDA(B, T, C, w, u, k, v):
-    return WKV.apply(B, T, C, w.cuda(), u.cuda(), k.cuda(), v.cuda())
+    w, u, k, v = w.cuda(), u.cuda(), k.cuda(), v.cuda()
+    if tuple(k.shape) != (B, T, C):
+        raise RuntimeError(f"k has shape {tuple(k.shape)}, expected {(B, T, C)}")
+    return _run(w, u, k, v)

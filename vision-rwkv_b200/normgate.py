@@ -14,36 +14,15 @@ above 1024) are refused by the library; `supported(C, group)` tells beforehand.
 """
 from __future__ import annotations
 
-import torch
-
-from . import ops
+from . import _lib, ops
 
 
 def supported(C: int, group: int) -> bool:
     return group > 0 and group % 64 == 0 and group <= 1024 and C % group == 0
 
 
-class _NormGate(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, gate, weight, bias, group, eps, act):
-        xf = x.float().contiguous()
-        gt = gate.contiguous() if gate.dtype in (torch.float32, torch.bfloat16) else gate.float().contiguous()
-        wf, bf = weight.float().contiguous(), bias.float().contiguous()
-        out, mean, rstd = ops.normgate_forward(xf, gt, wf, bf, group, eps, act)
-        ctx.save_for_backward(xf, gt, wf, bf, mean, rstd)
-        ctx.group, ctx.act, ctx.dtypes = group, act, (x.dtype, gate.dtype, weight.dtype, bias.dtype)
-        return out
-
-    @staticmethod
-    def backward(ctx, gout):
-        xf, gt, wf, bf, mean, rstd = ctx.saved_tensors
-        gx, ggate, gw, gb = ops.normgate_backward(gout.float().contiguous(), xf, gt, wf, bf, mean, rstd, ctx.group, ctx.act)
-        dx, dg, dw, db = ctx.dtypes
-        return gx.to(dx), ggate.to(dg), gw.to(dw), gb.to(db), None, None, None
-
-
 def norm_gate(x, gate, weight, bias, group=None, eps=1e-5, act=None):
     """x, gate: (..., C); weight, bias: (C,); group: channels per normalisation group (default C); act: None when
     `gate` is the gate itself, "sigmoid" / "silu" when it is the projection the gate is that activation of (the
     activation and its derivative then run inside the same pass)."""
-    return _NormGate.apply(x, gate, weight, bias, x.shape[-1] if group is None else group, eps, act)
+    return _lib.native().norm_gate(x, gate, weight, bias, x.shape[-1] if group is None else group, eps, ops.GATE_ACTIVATIONS[act])

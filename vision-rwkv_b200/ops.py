@@ -17,66 +17,30 @@ from . import _lib
 # When true, every call synchronises and raises if a bounded device-side wait ran out
 # (the kernels then return garbage instead of hanging).  Off by default: it costs a sync.
 CHECK_STATUS = False
-# Without CHECK_STATUS a failed launch is still reported, one or more calls late and with no
-# synchronisation: after every launch the 4-byte status word is copied to pinned host memory on
-# the same stream, and the next call into this module (or `raise_if_failed()`) raises for every
-# earlier launch whose copy has landed with a non-zero word.
-STATUS_MIRROR = True
+# Without CHECK_STATUS a failed launch is still reported, one or more calls late and with no synchronisation: the
+# kernel that gives up a wait writes a word of mapped host memory (one per device), and the next call into this
+# module (or `raise_if_failed()`) reads it and raises.
 
 
-class _StatusMirror:
-    """Ring of pinned status words for one device, each with the event that marks its copy."""
-    SLOTS = 32
-
-    def __init__(self):
-        self.host = torch.zeros(self.SLOTS, dtype=torch.int32).pin_memory()
-        self.events = [torch.cuda.Event() for _ in range(self.SLOTS)]
-        self.names = [None] * self.SLOTS
-        self.head = 0                    # next slot to fill
-        self.tail = 0                    # oldest slot not yet looked at
-        self.failed = []                 # reports not yet raised
-
-    def post(self, ws, what):
-        if self.head - self.tail == self.SLOTS:          # ring full: the oldest copy has long been queued
-            self.collect(wait=True, limit=1)
-        slot = self.head % self.SLOTS
-        self.host[slot:slot + 1].copy_(ws[:4].view(torch.int32), non_blocking=True)
-        self.events[slot].record()
-        self.names[slot] = what
-        self.head += 1
-
-    def collect(self, wait=False, limit=None):
-        while self.tail < self.head and (limit is None or limit > 0):
-            slot = self.tail % self.SLOTS
-            if wait:
-                self.events[slot].synchronize()
-            elif not self.events[slot].query():
-                break
-            word = int(self.host[slot])
-            if word:
-                self.failed.append(f"{self.names[slot]}: device status word {word & 0xffffffff:#x}")
-            self.tail += 1
-            if limit is not None:
-                limit -= 1
-
-    def raise_pending(self):
-        if self.failed:
-            failed, self.failed = self.failed, []
-            raise _lib.VrwkvError("; ".join(failed) + " (a bounded device-side wait ran out in an earlier launch: "
-                                  "its outputs, and everything computed from them, are invalid)")
-
-
-_mirrors = {}
+def _raise_failures(lib, index, what):
+    bits = lib.vrwkv_take_failures(index)
+    if bits:
+        raise _lib.VrwkvError(f"device status word {bits:#x}, seen at {what} (a bounded device-side wait ran out in an earlier "
+                              "launch: its outputs, and everything computed from them, are invalid)")
 
 
 def raise_if_failed(device=None, wait=True):
-    """Raise VrwkvError if any launch issued through this module on `device` (default: all) reported a
-    timed-out wait.  wait=True synchronises with the status copies still in flight: call it where a
-    step's results are consumed (after the optimizer step, before a checkpoint)."""
-    for index, mirror in list(_mirrors.items()):
-        if device is None or torch.device(device).index in (None, index):
-            mirror.collect(wait=wait)
-            mirror.raise_pending()
+    """Raise VrwkvError if any launch issued through this package on `device` (default: all) reported a
+    timed-out wait.  wait=True synchronises with the launches still running: call it where a step's
+    results are consumed (after the optimizer step, before a checkpoint)."""
+    lib = _lib.load()
+    if not torch.cuda.is_initialized():
+        return
+    wanted = torch.device(device).index if device is not None else None
+    for index in range(torch.cuda.device_count()) if wanted is None else (wanted,):
+        if wait and torch.cuda.memory_reserved(index) > 0:      # a device nothing was allocated on has run nothing
+            torch.cuda.synchronize(index)
+        _raise_failures(lib, index, "raise_if_failed")
 
 
 def _check_status(lib, ws, what):
@@ -85,18 +49,11 @@ def _check_status(lib, ws, what):
         st = lib.vrwkv_workspace_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream,
                                         ctypes.byref(word))
         _lib.check(st, "vrwkv_workspace_status")
+        lib.vrwkv_take_failures(ws.device.index)       # reported here
         if word.value:
             raise _lib.VrwkvError(f"{what}: device status word {word.value:#x} (a bounded wait ran out)")
         return
-    if not STATUS_MIRROR or torch.cuda.is_current_stream_capturing():
-        return
-    index = ws.device.index
-    mirror = _mirrors.get(index)
-    if mirror is None:
-        mirror = _mirrors[index] = _StatusMirror()
-    mirror.post(ws, what)
-    mirror.collect()                     # earlier launches whose word has landed
-    mirror.raise_pending()
+    _raise_failures(lib, ws.device.index, what)
 
 
 UNSUPPORTED = 8      # VRWKV_ERR_UNSUPPORTED: the bf16 kernels do not cover this shape / alignment
@@ -295,6 +252,9 @@ def wkv6_forward(r, k, v, w, u, H, tensor_cores=False):
     else:
         dev = _check_inputs((("r", r), ("k", k), ("v", v), ("w", w), ("u", u)))
     B, T, C = _wkv6_shapes(r, k, v, w, u, H)
+    if not CHECK_STATUS:
+        with torch.no_grad():
+            return _lib.native().wkv6(B, T, C, H, r, k, v, w, u, bool(tensor_cores))
     lib = _lib.load()
     y = torch.empty((B, T, C), device=dev, dtype=torch.float32)
     if y.numel() == 0:
@@ -375,7 +335,27 @@ def _ptr_array(tensors):
     return arr
 
 
-def _qshift_args(x, mixes, resolution, shift_pixel, gamma, head_dim=None):
+def qshift_group(C, gamma=0.25, head_dim=None):
+    """Channels per shifted group (head_dim=None), or per head; refuses what the kernel would shift differently."""
+    if head_dim is not None:
+        if head_dim % 4 or C % head_dim:                                # vrwkv6.py:78-79 asserts the same
+            raise RuntimeError(f"head_dim={head_dim} must be a multiple of 4 that divides C={C}")
+        return head_dim
+    if gamma > 0.25:
+        raise RuntimeError("channel_gamma must be <= 1/4")        # the reference asserts the same
+    group = int(C * gamma)
+    if group <= 0:
+        raise RuntimeError(f"int(C * gamma) = 0 for C={C}")
+    # the reference slices at int(C * gamma * k), k = 1..4 (vrwkv.py:72-76); the kernel's groups are k * int(C * gamma).
+    # The two agree whenever C * gamma is an integer (every shipped configuration: gamma = 1/4, C % 4 == 0);
+    # anything else is refused rather than shifted at slightly different channels.
+    if any(int(C * gamma * j) != j * group for j in (2, 3, 4)):
+        raise RuntimeError(f"C * gamma = {C * gamma} is not an integer: the group boundaries int(C * gamma * k) of the "
+                           f"reference are not multiples of one group size, which this kernel requires")
+    return group
+
+
+def _qshift_args(x, mixes, resolution, gamma, head_dim=None):
     if x.dim() != 3:
         raise RuntimeError(f"x must be (B, T, C), got {tuple(x.shape)}")
     B, T, C = x.shape
@@ -384,22 +364,7 @@ def _qshift_args(x, mixes, resolution, shift_pixel, gamma, head_dim=None):
         raise RuntimeError(f"patch resolution {H}x{W} does not match T={T}")
     if not 1 <= len(mixes) <= 3:
         raise RuntimeError("between one and three mix vectors")
-    if head_dim is not None:
-        if head_dim % 4 or C % head_dim:                                # vrwkv6.py:78-79 asserts the same
-            raise RuntimeError(f"head_dim={head_dim} must be a multiple of 4 that divides C={C}")
-        group = head_dim
-    else:
-        if gamma > 0.25:
-            raise RuntimeError("channel_gamma must be <= 1/4")        # the reference asserts the same
-        group = int(C * gamma)
-        if group <= 0:
-            raise RuntimeError(f"int(C * gamma) = 0 for C={C}")
-        # the reference slices at int(C * gamma * k), k = 1..4 (vrwkv.py:72-76); the kernel's groups are k * int(C * gamma).
-        # The two agree whenever C * gamma is an integer (every shipped configuration: gamma = 1/4, C % 4 == 0);
-        # anything else is refused rather than shifted at slightly different channels.
-        if any(int(C * gamma * j) != j * group for j in (2, 3, 4)):
-            raise RuntimeError(f"C * gamma = {C * gamma} is not an integer: the group boundaries int(C * gamma * k) of the "
-                               f"reference are not multiples of one group size, which this kernel requires")
+    group = qshift_group(C, gamma, head_dim)
     for m in mixes:
         if m.numel() != C:
             raise RuntimeError(f"mix vectors must hold C={C} values")
@@ -410,7 +375,7 @@ def qshift_mix_forward(x, mixes, resolution, shift_pixel=1, gamma=0.25, head_dim
     """[x * mix + q_shift(x) * (1 - mix) for mix in mixes], one fused pass.  head_dim=None: the four
     shifted groups are int(C * gamma) channels each (VRWKV); head_dim=n: the per-head shift of VRWKV6."""
     dev = _check_inputs([("x", x)] + [(f"mix{i}", m) for i, m in enumerate(mixes)])
-    B, H, W, C, group = _qshift_args(x, mixes, resolution, shift_pixel, gamma, head_dim)
+    B, H, W, C, group = _qshift_args(x, mixes, resolution, gamma, head_dim)
     lib = _lib.load()
     entry = lib.vrwkv_qshift_mix_forward_f32 if head_dim is None else lib.vrwkv_qshift_multihead_mix_forward_f32
     outs = [torch.empty_like(x) for _ in mixes]
@@ -427,7 +392,7 @@ def qshift_mix_backward(x, mixes, gouts, resolution, shift_pixel=1, gamma=0.25, 
     """(gx, [gmix...]) for `qshift_mix_forward`."""
     dev = _check_inputs([("x", x)] + [(f"mix{i}", m) for i, m in enumerate(mixes)]
                         + [(f"gout{i}", g) for i, g in enumerate(gouts)])
-    B, H, W, C, group = _qshift_args(x, mixes, resolution, shift_pixel, gamma, head_dim)
+    B, H, W, C, group = _qshift_args(x, mixes, resolution, gamma, head_dim)
     if len(gouts) != len(mixes) or any(g.shape != x.shape for g in gouts):
         raise RuntimeError("one output gradient of the shape of x per mix vector")
     lib = _lib.load()

@@ -29,7 +29,7 @@ import os
 
 import torch
 
-from . import ops
+from . import _lib, ops
 
 BF16_IO = os.environ.get("VRWKV_BF16_IO", "1") != "0"
 # Off by default: the forward keeps nothing and the backward rebuilds y and Den inside the
@@ -98,6 +98,14 @@ class WKV(torch.autograd.Function):
         return biwkv_backward_as_reference(w, u, k, v, gy, kept)
 
 
+def _run(w, u, k, v):
+    """`WKV.apply` through the C++ autograd node (same rules, about a fifth of the host time); the modes that only the
+    Python node has - kept denominators, synchronous status checks - stay with it."""
+    if SAVE_DENOMINATOR or ops.CHECK_STATUS:
+        return WKV.apply(w, u, k, v)
+    return _lib.native().biwkv(w, u, k, v, BF16_IO)
+
+
 def RUN_CUDA(w, u, k, v, decay_offset: int = 0):
     """y = Bi-WKV with decay exp(-w * (|t - j| - decay_offset)) between distinct tokens.
 
@@ -108,4 +116,4 @@ def RUN_CUDA(w, u, k, v, decay_offset: int = 0):
     w, u, k, v = w.cuda(), u.cuda(), k.cuda(), v.cuda()
     if decay_offset:
         u = u - decay_offset * w
-    return WKV.apply(w, u, k, v)
+    return _run(w, u, k, v)

@@ -21,7 +21,7 @@ import os
 
 import torch
 
-from . import ops
+from . import _lib, ops
 
 HEAD_SIZE = 64
 FORWARD_PATH = os.environ.get("VRWKV6_FORWARD_PATH", "auto")
@@ -86,4 +86,17 @@ class WKV_6(torch.autograd.Function):
 
 
 def RUN_CUDA_RWKV6(B, T, C, H, r, k, v, w, u):
-    return WKV_6.apply(B, T, C, H, r, k, v, w, u)
+    """`WKV_6.apply` with the autograd node in C++ (same rules); the modes only the Python node has stay with it."""
+    if ops.CHECK_STATUS or BACKWARD_TC != "full":
+        return WKV_6.apply(B, T, C, H, r, k, v, w, u)
+    assert HEAD_SIZE == C // H
+    for x in (r, k, v, w, u):
+        assert x.is_contiguous()
+    tensor_cores = _use_tensor_cores(r, k, v)
+    if torch.is_grad_enabled() and (r.requires_grad or k.requires_grad or v.requires_grad or w.requires_grad or u.requires_grad):
+        return _lib.native().wkv6(B, T, C, H, r, k, v, w, u, tensor_cores)
+    if tuple(r.shape) != (B, T, C):
+        raise RuntimeError(f"r has shape {tuple(r.shape)}, expected {(B, T, C)}")
+    if tensor_cores and r.dtype == k.dtype == v.dtype == torch.bfloat16:       # read as they are, no widening pass
+        return ops.wkv6_forward(r, k, v, _f32(w), _f32(u), H, tensor_cores=True)
+    return ops.wkv6_forward(_f32(r), _f32(k), _f32(v), _f32(w), _f32(u), H, tensor_cores=tensor_cores)
