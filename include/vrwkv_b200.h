@@ -168,24 +168,29 @@ int vrwkv_biwkv_forward_f32_noalloc(int B, int T, int C, const float* w, const f
  *   cuda_forward(int B,int T,int C,int H,float*r,float*k,float*v,float*w,float*u,float*y)
  *       CLS/cuda_v6/wkv6_op.cpp:4,7-9 (kernel CLS/cuda_v6/wkv6_cuda.cu:6-97,348-353)
  * It takes the raw decay input and forms -exp(w_raw) itself, where the reference's Python
- * wrapper does that in a separate pass (CLS/vrwkv6.py:48).
+ * wrapper does that in a separate pass (CLS/vrwkv6.py:48).  It needs no scratch memory and walks the
+ * sequence token by token; vrwkv_wkv6_forward is several times faster.
  */
 int vrwkv_wkv6_forward_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
                            const float* w_raw, const float* u, float* y, void* stream);
 
-/* vrwkv_wkv6_forward_tc_f32: the same forward on the tensor cores (tcgen05, state in tensor
- * memory): r, k, v and the state copy enter the matrix products rounded to bfloat16, sums are
- * fp32.  Results agree with vrwkv_wkv6_forward_f32 to about 1e-2 of max|y|: meant for callers
- * whose r, k, v are bfloat16 already.  `workspace`: 256 bytes, 256-byte aligned; its first word is
- * a status word as in vrwkv_workspace_status.  Stands in for the same reference entry point as
- * vrwkv_wkv6_forward_f32. */
+/* vrwkv_wkv6_forward: the same forward in 64-token chunks on the tensor cores (the states that enter each chunk,
+ * then all chunks in parallel).  exact = 1: float32 r, k, v and float32 accuracy.  exact = 0: r, k, v enter the matrix
+ * products as bfloat16 (in_bf16 = 1: they are bfloat16 bit patterns and are read as such; 0: float32, rounded on the
+ * way in), sums are fp32; results agree with exact = 1 to about 1e-2 of max|y|.  w_raw, u and y are float32.
+ * Replaces the same reference entry point, and with in_bf16 the `.float()` passes in front of the reference's call
+ * (CLS/vrwkv6.py:220 hands whatever dtype the projections produced to a kernel that reads float). */
+size_t vrwkv_wkv6_forward_workspace_bytes(int B, int T, int C, int H, int exact);
+int vrwkv_wkv6_forward(int B, int T, int C, int H, const void* r, const void* k, const void* v, int in_bf16, int exact,
+                       const float* w_raw, const float* u, float* y, void* workspace, size_t workspace_bytes, void* stream);
+
+/* vrwkv_wkv6_forward_tc_f32 / _bf16: vrwkv_wkv6_forward with exact = 0 for float32 / bfloat16 r, k, v.  A workspace of
+ * 256 bytes (256-byte aligned; its first word is a status word as in vrwkv_workspace_status) is enough: they then walk
+ * the sequence with the state in tensor memory, which is slower than the chunks they run when the workspace has
+ * vrwkv_wkv6_forward_workspace_bytes(B, T, C, H, 0) bytes. */
 int vrwkv_wkv6_forward_tc_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
                               const float* w_raw, const float* u, float* y, void* workspace,
                               size_t workspace_bytes, void* stream);
-/* The same kernel for callers whose r, k, v are bfloat16 (uint16_t bit patterns; the usual case
- * under autocast): the tiles are read as bfloat16, so the `.float()` passes in front of the
- * reference's call (CLS/vrwkv6.py:220 hands whatever dtype the projections produced to a kernel
- * that reads float) disappear.  w_raw, u and y stay float32. */
 int vrwkv_wkv6_forward_tc_bf16(int B, int T, int C, int H, const uint16_t* r, const uint16_t* k,
                                const uint16_t* v, const float* w_raw, const float* u, float* y,
                                void* workspace, size_t workspace_bytes, void* stream);
@@ -197,8 +202,7 @@ int vrwkv_wkv6_forward_tc_bf16(int B, int T, int C, int H, const uint16_t* r, co
  * without its T <= 256 limit.  gw is the gradient w.r.t. w_raw (as in the reference, whose
  * kernels multiply by -exp(w_raw)); gu is already summed over batch (the reference returns
  * (B, C) and sums in Python, CLS/vrwkv6.py:69).  gv may be NULL: the value gradient is then left
- * out (a third of the work); by the symmetry of the operator it equals the forward applied to
- * (r, k, v) := (k, r, gy), which a half-precision caller can take from vrwkv_wkv6_forward_tc_*.
+ * out; by the symmetry of the operator it equals the forward applied to (r, k, v) := (k, r, gy).
  */
 size_t vrwkv_wkv6_backward_workspace_bytes(int B, int T, int C, int H);
 int vrwkv_wkv6_backward_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
@@ -206,15 +210,18 @@ int vrwkv_wkv6_backward_f32(int B, int T, int C, int H, const float* r, const fl
                             float* gv, float* gw, float* gu, void* workspace, size_t workspace_bytes,
                             void* stream);
 
-/* The same gradients on the tensor cores (tcgen05, states in tensor memory), for callers whose
- * activations are half precision anyway: r, k, v, gy enter the matrix products rounded to bfloat16,
- * sums are fp32; results agree with vrwkv_wkv6_backward_f32 to about 1e-2 of each tensor's maximum.
- * gv is the forward kernel applied to (k, r, gy); gr and gk come from a second kernel of the same
- * block structure; gw and gu from their one-sided sums.  vrwkv_wkv6_backward_tc_bf16 reads r, k, v,
- * gy as bfloat16 bit patterns directly (the reference hands whatever dtype the projections produced
- * to kernels that read float, CLS/vrwkv6.py:60-70, so a half-precision caller pays widening passes
- * there).  All gradients are float32; gw is w.r.t. w_raw; gu is summed over batch.  They stand in for
- * the same reference entry point as vrwkv_wkv6_backward_f32 (CLS/cuda_v6/wkv6_op.cpp:5,10-12). */
+/* The general form of the backward.  exact = 1: float32 tensors and accuracy (vrwkv_wkv6_backward_f32).  exact = 0, for
+ * callers whose activations are half precision anyway: r, k, v, gy enter the matrix products as bfloat16, sums are fp32;
+ * gv agrees with exact = 1 to about 1e-2 of its maximum, gr, gk, gw, gu (whose scaled operands are carried to 16 bits)
+ * to about 1e-4 for bfloat16 inputs.  in_bf16: r, k, v are bfloat16 bit patterns; gy_bf16: gy is (needs in_bf16; else
+ * gy is float32 and rounded on the way in); out_bf16: gr, gk, gv are written as bfloat16 (needs in_bf16).  gw, gu are
+ * float32.  gv may be NULL. */
+size_t vrwkv_wkv6_backward_bytes(int B, int T, int C, int H, int exact);
+int vrwkv_wkv6_backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, int in_bf16, int exact,
+                        const float* w_raw, const float* u, const void* gy, int gy_bf16, void* gr, void* gk, void* gv, int out_bf16,
+                        float* gw, float* gu, void* workspace, size_t workspace_bytes, void* stream);
+
+/* vrwkv_wkv6_backward with exact = 0 and float32 gradients, for float32 / bfloat16 r, k, v, gy. */
 size_t vrwkv_wkv6_backward_tc_workspace_bytes(int B, int T, int C, int H);
 int vrwkv_wkv6_backward_tc_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
                                const float* w_raw, const float* u, const float* gy, float* gr, float* gk, float* gv,

@@ -34,6 +34,11 @@ SIGNATURES = {
     "vrwkv_biwkv_backward_bf16": (_c_int, [_c_int] * 3 + [_ptr] * 9 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_forward_f32_noalloc": (_c_int, [_c_int] * 3 + [_ptr] * 6),
     "vrwkv_wkv6_forward_f32": (_c_int, [_c_int] * 4 + [_ptr] * 7),
+    "vrwkv_wkv6_forward_workspace_bytes": (_c_size_t, [_c_int] * 5),
+    "vrwkv_wkv6_forward": (_c_int, [_c_int] * 4 + [_ptr] * 3 + [_c_int] * 2 + [_ptr] * 4 + [_c_size_t, _ptr]),
+    "vrwkv_wkv6_backward_bytes": (_c_size_t, [_c_int] * 5),
+    "vrwkv_wkv6_backward": (_c_int, [_c_int] * 4 + [_ptr] * 3 + [_c_int] * 2 + [_ptr] * 3 + [_c_int] + [_ptr] * 3 + [_c_int]
+                            + [_ptr] * 3 + [_c_size_t, _ptr]),
     "vrwkv_wkv6_forward_tc_f32": (_c_int, [_c_int] * 4 + [_ptr] * 7 + [_c_size_t, _ptr]),
     "vrwkv_wkv6_forward_tc_bf16": (_c_int, [_c_int] * 4 + [_ptr] * 7 + [_c_size_t, _ptr]),
     "vrwkv_wkv6_backward_workspace_bytes": (_c_size_t, [_c_int] * 4),

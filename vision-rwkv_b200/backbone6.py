@@ -23,7 +23,7 @@ import torch.utils.checkpoint as cp
 from .backbone import _PatchEmbed, _ramp
 from . import normgate
 from .qshift import qshift_ddlerp, qshift_mix
-from .vrwkv6 import HEAD_SIZE, RUN_CUDA_RWKV6
+from .vrwkv6 import HEAD_SIZE, inference_rwkv6
 
 MIX_RANK = 32       # width of the low-rank branch that produces the five mixing offsets
 DECAY_RANK = 64     # width of the low-rank branch that produces the decay offset
@@ -98,8 +98,8 @@ class SpatialMixV6(nn.Module):
         v = self.value(xv)
         g_raw = self.gate(xg)
         w = self.time_decay + torch.tanh(xw @ self.time_decay_w1) @ self.time_decay_w2
-        y = RUN_CUDA_RWKV6(B, T, C, self.n_head, r.contiguous(), k.contiguous(), v.contiguous(),
-                           w.float().contiguous(), self.time_faaaa)
+        y = inference_rwkv6(B, T, C, self.n_head, r.contiguous(), k.contiguous(), v.contiguous(),
+                            w.float().contiguous(), self.time_faaaa)
         if self.key_norm is not None:
             y = self.key_norm(y)
         if y.is_cuda and normgate.supported(C, HEAD_SIZE):

@@ -287,7 +287,26 @@ static inline bool misaligned16(const void* p) { return (reinterpret_cast<uintpt
 
 size_t vrwkv_wkv6_backward_workspace_bytes(int B, int T, int C, int H) {
     if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
-    return wkv6::backward_workspace(B, T, H);
+    return wkv6c::backward_workspace(B, T, H, true);
+}
+
+size_t vrwkv_wkv6_forward_workspace_bytes(int B, int T, int C, int H, int exact) {
+    if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
+    return wkv6c::forward_workspace(B, T, H, exact != 0);
+}
+
+int vrwkv_wkv6_forward(int B, int T, int C, int H, const void* r, const void* k, const void* v, int in_bf16, int exact,
+                       const float* w_raw, const float* u, float* y, void* workspace, size_t workspace_bytes, void* stream) {
+    if (int st = check_wkv6(B, T, C, H)) return st;
+    if (!r || !k || !v || !w_raw || !u || !y || !workspace) return VRWKV_ERR_NULL;
+    if (in_bf16 && exact) return VRWKV_ERR_UNSUPPORTED;
+    if (misaligned16(r) || misaligned16(k) || misaligned16(v) || misaligned16(w_raw) || misaligned4(u) || misaligned4(y) ||
+        (reinterpret_cast<uintptr_t>(workspace) & 255u))
+        return VRWKV_ERR_ALIGNMENT;
+    if (workspace_bytes < wkv6c::forward_workspace(B, T, H, exact != 0)) return VRWKV_ERR_WORKSPACE;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
+    return finish(wkv6c::forward(B, T, H, r, k, v, w_raw, u, y, in_bf16 != 0, exact != 0, workspace, s));
 }
 
 int vrwkv_wkv6_forward_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
@@ -309,8 +328,9 @@ int vrwkv_wkv6_forward_tc_f32(int B, int T, int C, int H, const float* r, const 
         misaligned16(y) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < 256) return VRWKV_ERR_WORKSPACE;
-    return finish(wkv6tc::forward(B, T, H, r, k, v, w_raw, u, y, static_cast<unsigned*>(workspace),
-                                  g_path.load() != 1, static_cast<cudaStream_t>(stream)));
+    if (g_path.load() != 1 && workspace_bytes >= wkv6c::forward_workspace(B, T, H, false))
+        return vrwkv_wkv6_forward(B, T, C, H, r, k, v, 0, 0, w_raw, u, y, workspace, workspace_bytes, stream);
+    return finish(wkv6tc::forward(B, T, H, r, k, v, w_raw, u, y, static_cast<unsigned*>(workspace), static_cast<cudaStream_t>(stream)));
 }
 
 int vrwkv_wkv6_forward_tc_bf16(int B, int T, int C, int H, const uint16_t* r, const uint16_t* k,
@@ -322,55 +342,67 @@ int vrwkv_wkv6_forward_tc_bf16(int B, int T, int C, int H, const uint16_t* r, co
         misaligned16(y) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < 256) return VRWKV_ERR_WORKSPACE;
+    if (g_path.load() != 1 && workspace_bytes >= wkv6c::forward_workspace(B, T, H, false))
+        return vrwkv_wkv6_forward(B, T, C, H, r, k, v, 1, 0, w_raw, u, y, workspace, workspace_bytes, stream);
     return finish(wkv6tc::forward_bf16in(B, T, H, r, k, v, w_raw, u, y, static_cast<unsigned*>(workspace),
                                          static_cast<cudaStream_t>(stream)));
+}
+
+static int wkv6_backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, bool in_bf16, bool exact,
+                         const float* w_raw, const float* u, const void* gy, bool gy_bf16, void* gr, void* gk, void* gv, bool out_bf16,
+                         float* gw, float* gu, void* workspace, size_t workspace_bytes, void* stream) {
+    if (int st = check_wkv6(B, T, C, H)) return st;
+    if (!r || !k || !v || !w_raw || !u || !gy || !gr || !gk || !gw || !gu || !workspace) return VRWKV_ERR_NULL;      // gv may be NULL
+    if ((in_bf16 || gy_bf16 || out_bf16) && exact) return VRWKV_ERR_UNSUPPORTED;
+    if (!in_bf16 && (gy_bf16 || out_bf16)) return VRWKV_ERR_UNSUPPORTED;
+    if (misaligned16(r) || misaligned16(k) || misaligned16(v) || misaligned16(w_raw) || misaligned16(gy) || misaligned4(u) ||
+        misaligned4(gw) || misaligned4(gu) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
+        return VRWKV_ERR_ALIGNMENT;
+    for (const void* p : {static_cast<const void*>(gr), static_cast<const void*>(gk), static_cast<const void*>(gv)})
+        if (reinterpret_cast<uintptr_t>(p) & (out_bf16 ? 1u : 3u)) return VRWKV_ERR_ALIGNMENT;
+    if (workspace_bytes < wkv6c::backward_workspace(B, T, H, exact)) return VRWKV_ERR_WORKSPACE;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
+    return finish(wkv6c::backward(B, T, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, in_bf16, gy_bf16, out_bf16, exact, workspace, s));
+}
+
+size_t vrwkv_wkv6_backward_bytes(int B, int T, int C, int H, int exact) {
+    if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
+    return wkv6c::backward_workspace(B, T, H, exact != 0);
+}
+
+int vrwkv_wkv6_backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, int in_bf16, int exact,
+                        const float* w_raw, const float* u, const void* gy, int gy_bf16, void* gr, void* gk, void* gv, int out_bf16,
+                        float* gw, float* gu, void* workspace, size_t workspace_bytes, void* stream) {
+    return wkv6_backward(B, T, C, H, r, k, v, in_bf16 != 0, exact != 0, w_raw, u, gy, gy_bf16 != 0, gr, gk, gv, out_bf16 != 0, gw, gu,
+                         workspace, workspace_bytes, stream);
 }
 
 int vrwkv_wkv6_backward_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
                             const float* w_raw, const float* u, const float* gy, float* gr, float* gk,
                             float* gv, float* gw, float* gu, void* workspace, size_t workspace_bytes,
                             void* stream) {
-    if (int st = check_wkv6(B, T, C, H)) return st;
-    if (!r || !k || !v || !w_raw || !u || !gy || !gr || !gk || !gw || !gu || !workspace)      // gv may be NULL
-        return VRWKV_ERR_NULL;
-    if (misaligned16(r) || misaligned16(k) || misaligned16(v) || misaligned16(w_raw) || misaligned16(gy) ||
-        misaligned4(u) || misaligned4(gr) || misaligned4(gk) || misaligned4(gv) || misaligned4(gw) ||
-        misaligned4(gu) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
-        return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < wkv6::backward_workspace(B, T, H)) return VRWKV_ERR_WORKSPACE;
-    return finish(wkv6::backward(B, T, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, workspace,
-                                 static_cast<cudaStream_t>(stream)));
+    return wkv6_backward(B, T, C, H, r, k, v, false, true, w_raw, u, gy, false, gr, gk, gv, false, gw, gu, workspace, workspace_bytes,
+                         stream);
 }
 
 size_t vrwkv_wkv6_backward_tc_workspace_bytes(int B, int T, int C, int H) {
     if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
-    return wkv6tc::backward_workspace(B, T, H);
-}
-
-static int wkv6_backward_tc(int B, int T, int C, int H, const void* r, const void* k, const void* v, const float* w_raw,
-                            const float* u, const void* gy, float* gr, float* gk, float* gv, float* gw, float* gu,
-                            void* workspace, size_t workspace_bytes, void* stream, bool half_in) {
-    if (int st = check_wkv6(B, T, C, H)) return st;
-    if (!r || !k || !v || !w_raw || !u || !gy || !gr || !gk || !gv || !gw || !gu || !workspace) return VRWKV_ERR_NULL;
-    if (misaligned16(r) || misaligned16(k) || misaligned16(v) || misaligned16(w_raw) || misaligned16(gy) || misaligned4(u) ||
-        misaligned16(gr) || misaligned16(gk) || misaligned16(gv) || misaligned4(gw) || misaligned4(gu) ||
-        (reinterpret_cast<uintptr_t>(workspace) & 255u))
-        return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < wkv6tc::backward_workspace(B, T, H)) return VRWKV_ERR_WORKSPACE;
-    return finish(wkv6tc::backward(B, T, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, workspace, half_in,
-                                   static_cast<cudaStream_t>(stream)));
+    return wkv6c::backward_workspace(B, T, H, false);
 }
 
 int vrwkv_wkv6_backward_tc_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
                                const float* w_raw, const float* u, const float* gy, float* gr, float* gk, float* gv,
                                float* gw, float* gu, void* workspace, size_t workspace_bytes, void* stream) {
-    return wkv6_backward_tc(B, T, C, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, workspace, workspace_bytes, stream, false);
+    return wkv6_backward(B, T, C, H, r, k, v, false, false, w_raw, u, gy, false, gr, gk, gv, false, gw, gu, workspace, workspace_bytes,
+                         stream);
 }
 
 int vrwkv_wkv6_backward_tc_bf16(int B, int T, int C, int H, const uint16_t* r, const uint16_t* k, const uint16_t* v,
                                 const float* w_raw, const float* u, const uint16_t* gy, float* gr, float* gk, float* gv,
                                 float* gw, float* gu, void* workspace, size_t workspace_bytes, void* stream) {
-    return wkv6_backward_tc(B, T, C, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, workspace, workspace_bytes, stream, true);
+    return wkv6_backward(B, T, C, H, r, k, v, true, false, w_raw, u, gy, true, gr, gk, gv, false, gw, gu, workspace, workspace_bytes,
+                         stream);
 }
 
 }  // extern "C"

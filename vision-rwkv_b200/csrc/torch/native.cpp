@@ -176,24 +176,30 @@ Tensor wkv6_forward(int64_t H, const Tensor& r, const Tensor& k, const Tensor& v
     const Tensor w = f32(w_), u = f32(u_);
     Tensor y = at::empty({B, T, C}, r.options().dtype(at::kFloat));
     if (y.numel() == 0) return y;
-    if (tensor_cores) {
-        Tensor ws = workspace(256, r);
-        if (all_bf16({&r, &k, &v})) {
-            check(vrwkv_wkv6_forward_tc_bf16(B, T, C, H, static_cast<uint16_t*>(r.data_ptr()), static_cast<uint16_t*>(k.data_ptr()),
-                                             static_cast<uint16_t*>(v.data_ptr()), fp(w), fp(u), fp(y), ws.data_ptr(), ws.numel(),
-                                             stream_of(r)),
-                  "vrwkv_wkv6_forward_tc_bf16");
-        } else {
-            const Tensor r32 = f32(r), k32 = f32(k), v32 = f32(v);
-            check(vrwkv_wkv6_forward_tc_f32(B, T, C, H, fp(r32), fp(k32), fp(v32), fp(w), fp(u), fp(y), ws.data_ptr(), ws.numel(),
-                                            stream_of(r)),
-                  "vrwkv_wkv6_forward_tc_f32");
-        }
-        raise_failures(r.get_device(), "vrwkv_wkv6_forward_tc");
-        return y;
-    }
-    const Tensor r32 = f32(r), k32 = f32(k), v32 = f32(v);
-    check(vrwkv_wkv6_forward_f32(B, T, C, H, fp(r32), fp(k32), fp(v32), fp(w), fp(u), fp(y), stream_of(r)), "vrwkv_wkv6_forward_f32");
+    const bool half = tensor_cores && all_bf16({&r, &k, &v});
+    const Tensor r_ = half ? r.contiguous() : f32(r), k_ = half ? k.contiguous() : f32(k), v_ = half ? v.contiguous() : f32(v);
+    Tensor ws = workspace(vrwkv_wkv6_forward_workspace_bytes(B, T, C, H, !tensor_cores), r);
+    check(vrwkv_wkv6_forward(B, T, C, H, r_.data_ptr(), k_.data_ptr(), v_.data_ptr(), half, !tensor_cores, fp(w), fp(u), fp(y), ws.data_ptr(),
+                             ws.numel(), stream_of(r)),
+          "vrwkv_wkv6_forward");
+    raise_failures(r.get_device(), "vrwkv_wkv6_forward");
+    return y;
+}
+
+// The walk in 16-token blocks (vrwkv_wkv6_forward_tc_bf16 without scratch memory): slower than wkv6_forward, other roundings.
+Tensor wkv6_walk(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w_, const Tensor& u_) {
+    const int B = r.size(0), T = r.size(1), C = r.size(2), H = C / 64;
+    check_wkv6(B, T, C, H, r, k, v, w_, u_);
+    TORCH_CHECK(all_bf16({&r, &k, &v}), "r, k, v must be bfloat16");
+    const c10::cuda::CUDAGuard guard(r.device());
+    const Tensor w = f32(w_), u = f32(u_), r_ = r.contiguous(), k_ = k.contiguous(), v_ = v.contiguous();
+    Tensor y = at::empty({B, T, C}, r.options().dtype(at::kFloat));
+    if (y.numel() == 0) return y;
+    Tensor ws = workspace(256, r);
+    check(vrwkv_wkv6_forward_tc_bf16(B, T, C, H, static_cast<uint16_t*>(r_.data_ptr()), static_cast<uint16_t*>(k_.data_ptr()),
+                                     static_cast<uint16_t*>(v_.data_ptr()), fp(w), fp(u), fp(y), ws.data_ptr(), 256, stream_of(r)),
+          "vrwkv_wkv6_forward_tc_bf16");
+    raise_failures(r.get_device(), "vrwkv_wkv6_forward_tc_bf16");
     return y;
 }
 
@@ -215,31 +221,22 @@ struct Wkv6 : torch::autograd::Function<Wkv6> {
         const int B = r.size(0), T = r.size(1), C = r.size(2);
         const Tensor w = f32(saved[3]), u = f32(saved[4]);
         const auto opt = r.options().dtype(at::kFloat);
-        Tensor gr = at::empty({B, T, C}, opt), gk = at::empty({B, T, C}, opt), gv = at::empty({B, T, C}, opt),
+        const bool exact = !ctx->saved_data["tc"].toBool(), half = !exact && all_bf16({&r, &k, &v});
+        // bfloat16 r, k, v take their gradients in bfloat16 (what autograd would round them to); gy is read as it comes
+        const auto out = half ? r.options() : opt;
+        Tensor gr = at::empty({B, T, C}, out), gk = at::empty({B, T, C}, out), gv = at::empty({B, T, C}, out),
                gw = at::empty({B, T, C}, opt), gu = at::empty({H, C / H}, opt);
         if (gr.numel() == 0) {
             gu.zero_();
-        } else if (ctx->saved_data["tc"].toBool()) {
-            Tensor ws = workspace(vrwkv_wkv6_backward_tc_workspace_bytes(B, T, C, H), r);
-            if (all_bf16({&r, &k, &v})) {
-                const Tensor g = gy.to(at::kBFloat16).contiguous();
-                check(vrwkv_wkv6_backward_tc_bf16(B, T, C, H, static_cast<uint16_t*>(r.data_ptr()), static_cast<uint16_t*>(k.data_ptr()),
-                                                  static_cast<uint16_t*>(v.data_ptr()), fp(w), fp(u), static_cast<uint16_t*>(g.data_ptr()),
-                                                  fp(gr), fp(gk), fp(gv), fp(gw), fp(gu), ws.data_ptr(), ws.numel(), stream_of(r)),
-                      "vrwkv_wkv6_backward_tc_bf16");
-            } else {
-                const Tensor r32 = f32(r), k32 = f32(k), v32 = f32(v), g = f32(gy);
-                check(vrwkv_wkv6_backward_tc_f32(B, T, C, H, fp(r32), fp(k32), fp(v32), fp(w), fp(u), fp(g), fp(gr), fp(gk), fp(gv),
-                                                 fp(gw), fp(gu), ws.data_ptr(), ws.numel(), stream_of(r)),
-                      "vrwkv_wkv6_backward_tc_f32");
-            }
-            raise_failures(r.get_device(), "vrwkv_wkv6_backward_tc");
         } else {
-            const Tensor r32 = f32(r), k32 = f32(k), v32 = f32(v), g = f32(gy);
-            Tensor ws = workspace(vrwkv_wkv6_backward_workspace_bytes(B, T, C, H), r);
-            check(vrwkv_wkv6_backward_f32(B, T, C, H, fp(r32), fp(k32), fp(v32), fp(w), fp(u), fp(g), fp(gr), fp(gk), fp(gv), fp(gw),
-                                          fp(gu), ws.data_ptr(), ws.numel(), stream_of(r)),
-                  "vrwkv_wkv6_backward_f32");
+            const Tensor r_ = half ? r.contiguous() : f32(r), k_ = half ? k.contiguous() : f32(k), v_ = half ? v.contiguous() : f32(v);
+            const Tensor g = half && is_bf16(gy) ? gy.contiguous() : f32(gy);
+            Tensor ws = workspace(vrwkv_wkv6_backward_bytes(B, T, C, H, exact), r);
+            check(vrwkv_wkv6_backward(B, T, C, H, r_.data_ptr(), k_.data_ptr(), v_.data_ptr(), half, exact, fp(w), fp(u), g.data_ptr(),
+                                      is_bf16(g), gr.data_ptr(), gk.data_ptr(), gv.data_ptr(), half, fp(gw), fp(gu), ws.data_ptr(),
+                                      ws.numel(), stream_of(r)),
+                  "vrwkv_wkv6_backward");
+            raise_failures(r.get_device(), "vrwkv_wkv6_backward");
         }
         return {gr, gk, gv, gw, gu.view({H, C / H}), Tensor(), Tensor()};
     }
@@ -284,6 +281,9 @@ PYBIND11_MODULE(_native, m) {
     });
     m.def("norm_gate", [](const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, int64_t group, double eps, int64_t act) {
         return vrwkv::guarded([&] { return vrwkv::norm_gate(x, gate, weight, bias, group, eps, act); })();
+    });
+    m.def("wkv6_walk", [](const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
+        return vrwkv::guarded([&] { return vrwkv::wkv6_walk(r, k, v, w, u); })();
     });
     m.def("wkv6", [](int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w,
                      const Tensor& u, bool tensor_cores) {

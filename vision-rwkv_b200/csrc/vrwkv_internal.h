@@ -78,27 +78,29 @@ int backward_bf16(int B, int T, int C, const float* w, const float* u, const voi
 }  // namespace biwkv
 
 namespace wkv6 {
-size_t backward_workspace(int B, int T, int H);
+// float32 forward without scratch memory (wkv6_sweeps.cu)
 int forward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
             const float* u, float* y, cudaStream_t stream);
-int backward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
-             const float* u, const float* gy, float* gr, float* gk, float* gv, float* gw, float* gu,
-             void* workspace, cudaStream_t stream);
 }  // namespace wkv6
 
 namespace wkv6tc {
-// Tensor-core forward (bf16 operands, fp32 state).  `status` points at 4 writable device bytes.
-// pipelined = false runs the first-generation kernel (all warps do every phase in turn).
+// Tensor-core forward (bf16 operands, fp32 state) without scratch memory.  `status` points at 4 writable device bytes.
 int forward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
-            const float* u, float* y, unsigned* status, bool pipelined, cudaStream_t stream);
+            const float* u, float* y, unsigned* status, cudaStream_t stream);
 // r, k, v in bfloat16 (read as such by the kernel: no widening pass), w_raw, u, y float32.
 int forward_bf16in(int B, int T, int H, const void* r, const void* k, const void* v, const float* w_raw,
                    const float* u, float* y, unsigned* status, cudaStream_t stream);
-// Tensor-core backward: gv through the forward kernel with permuted operands, gr and gk through a
-// token-mixing kernel of the same structure, gw and gu from their one-sided sums.  half_in: r, k, v, gy
-// point at bfloat16 (read as such).  Gradients are float32.
-size_t backward_workspace(int B, int T, int H);
-int backward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w_raw, const float* u,
-             const void* gy, float* gr, float* gk, float* gv, float* gw, float* gu, void* workspace, bool half_in,
-             cudaStream_t stream);
 }  // namespace wkv6tc
+
+namespace wkv6c {
+// Chunked tensor-core kernels (wkv6_chunk.cu).  exact: float32 tensors, float32 accuracy; else bfloat16 operands
+// (r, k, v, gy in bfloat16, or float32 rounded on the way in), scaled operands of gr, gk, gw carried to 16 bits.
+// gv may be null.
+size_t forward_workspace(int B, int T, int H, bool exact);
+size_t backward_workspace(int B, int T, int H, bool exact);
+int forward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, float* y,
+            bool bf16_in, bool exact, void* workspace, cudaStream_t stream);
+int backward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, const void* gy,
+             void* gr, void* gk, void* gv, float* gw, float* gu, bool bf16_in, bool gy_bf16, bool bf16_out, bool exact,
+             void* workspace, cudaStream_t stream);
+}  // namespace wkv6c

@@ -1,0 +1,1179 @@
+// WKV6 (head size 64, bidirectional), forward and backward, in 64-token chunks on the tensor cores.
+//
+// With l_m = log2 of the decays (log2 e * -exp(w_raw)) and D(t, s) = 2^(sum of l strictly between t and s), the operator is
+//   y_t = sum_{s != t} (sum_i r_t[i] D(t,s)[i] k_s[i]) v_s + (sum_i r_t[i] u[i] k_t[i]) v_t
+// and its gradients are sums over the same pairs.  Two kernels:
+//
+//   1. states: per (batch, head, direction) one CTA walks the chunks and leaves in global memory the 64 x 64 state
+//      that ENTERS every chunk,  X <- 2^(sum l) X + sum_s (x_s 2^(decay to the chunk's edge)) z_s^T,
+//      (x, z) = (k, v) for the forward; the backward needs (k, v) and the adjoint pair (r, gy).
+//   2. outputs: one CTA per chunk, all chunks in parallel, both directions at once: read-out of the entering states,
+//      the 64 x 64 pairs inside the chunk, and (backward) the decay gradient.
+//
+// What bounds it: memory.  Per element of a (B, T, C) tensor the bfloat16 forward moves 12 bytes in the first kernel and
+// 18 in the second (the states are 4 of each), the backward 28 and 38; the products are 2.2 and 11 kFLOP, a third of
+// that time.  The walk of the first kernel is serial over T / 64 chunks but holds only the state update; everything else
+// is parallel over chunks, which a walk over the whole sequence per CTA (16 tokens at a time with the state in tensor
+// memory: 1.47 + 7.8 ms at B=32, T=4096, H=12) was not.  64-wide heads make 16 x 64 x 64 products: mma.sync keeps their
+// operands, scalings and masks in registers, where tcgen05 would stage each through shared memory and tensor memory for
+// a product that takes 30 cycles.  The chunk length trades state traffic (1 / length) against pairs inside the chunk.
+//
+// Stability.  No exponent is positive except inside 16-token blocks: block b's tokens are scaled towards the block's edges
+// (2^(<= 0)), and a block further away takes the decay across the blocks in between as one more factor <= 1, so nothing
+// overflows however strong the decay is.  Inside a block the pairs are split at its middle token, which needs
+// 2^(8 tokens' decay) on one side; where a channel exceeds 2^kSafe there, the block takes its pairs in four levels of
+// halves (16, 8, 4, 2 tokens), again with factors <= 1 only.
+//
+// Decay gradient.  With R> = r gr>, K> = k gk> (one-sided parts, elementwise) and the mirrored R<, K<, the gradient with
+// respect to l_m counts the pairs that have m strictly between them.  Counted from the chunk's right edge,
+//   g_m = edge + sum_{t > m} (R> + K< - K> - R<)_t - K>_m - R<_m,   edge[i] = sum_j (S> A> + A< S<)[i][j]
+// where S>, A< have passed the edge rightward and A>, S< leftward.  Rounding errors stay within one chunk.
+//
+// Reference being replaced: classification/mmcls_custom/models/backbones/cuda_v6/wkv6_cuda.cu:6-346.
+#include <algorithm>
+#include <mutex>
+#include <set>
+#include <utility>
+#include "sm100_async.cuh"
+#include "tensor_map.h"
+#include "vrwkv_internal.h"
+#include "wkv6_chunk.cuh"
+
+namespace wkv6c {
+
+constexpr float kSafe = 64.f;       // largest |sum of l| over a block for which its own pairs may use factors above 1
+
+typedef float Totals[kBlocks][N];   // sum of l over each block
+typedef float Table[kChunk][kTab];
+
+// ---- kernel 1: states entering every chunk ----------------------------------------------------------------
+struct StateArgs {
+    int T, H, n_chunks;
+    uint4* out;              // [pair][direction][b h][chunk][part][kStateWords / 4]
+    size_t plane;            // uint4 per (pair, direction)
+    unsigned* status;        // the launch's status word and its host-visible copy
+    unsigned* mirror;
+};
+constexpr uint32_t kWaitLimit = 1u << 20;      // polls before a wait for a tile gives up
+
+// Shared memory of a CTA: the raw tiles of one chunk as the copy engine delivers them (w | x, z of every pair), then per
+// pair the operand planes and twice the totals (the next chunk's are written while this one's are read).
+template <typename XT, typename ZT0, typename ZT1, int kZ, int kX, int kPairs>
+struct StateSmem {
+    static constexpr size_t kTile = kChunk * N;
+    static constexpr size_t w = 0;
+    static constexpr size_t x0 = kTile * 4, z0 = x0 + kTile * sizeof(XT);
+    static constexpr size_t x1 = z0 + kTile * sizeof(ZT0), z1 = x1 + (kPairs > 1 ? kTile * sizeof(XT) : 0);
+    static constexpr size_t planes = z1 + (kPairs > 1 ? kTile * sizeof(ZT1) : 0);
+    static constexpr size_t per_pair = static_cast<size_t>(kZ + kX) * kPlane * 2 + 2 * sizeof(Totals);
+    static constexpr size_t bar = planes + kPairs * per_pair;
+    static constexpr size_t bytes = bar + 16;
+    static constexpr uint32_t loaded = static_cast<uint32_t>(planes);
+};
+
+// The work of one pair's four warps (a block each) on one chunk: lane = two channels, one token after the other, so decays,
+// their running sums and the scaling need no shuffles.  Leaves the scaled operand planes; `tot` gets the blocks' sums.
+template <typename XT, typename ZT, int kZ, int kX>
+__device__ __forceinline__ void scale_chunk(const float* wt, const XT* xt, const ZT* zt, int valid, int dir, Totals& tot, __nv_bfloat16* xs,
+                                            __nv_bfloat16* zs, int warp, int lane) {
+    const int word = col_word(lane), row0 = warp * kBlock;
+    float2 sum[kBlock];
+    float2 run = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) {
+        const float2 w = *reinterpret_cast<const float2*>(wt + (row0 + t) * N + 2 * lane);
+        if (row0 + t < valid) {
+            run.x += log2_decay<(kX > 2)>(w.x);
+            run.y += log2_decay<(kX > 2)>(w.y);
+        }
+        sum[t] = run;
+    }
+    *reinterpret_cast<float2*>(&tot[warp][2 * lane]) = run;
+    __syncthreads();       // totals are there; every warp is past the previous chunk's products
+    float2 edge = make_float2(0.f, 0.f);        // decay from the block to the chunk's edge
+    for (int j = dir == 0 ? warp + 1 : 0; j < (dir == 0 ? kBlocks : warp); ++j) {
+        const float2 t = *reinterpret_cast<const float2*>(&tot[j][2 * lane]);
+        edge.x += t.x;
+        edge.y += t.y;
+    }
+    if (dir == 0) { edge.x += run.x; edge.y += run.y; }
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) {
+        Pair<XT> xr;
+        Pair<ZT> zr;
+        xr.lds(xt + (row0 + t) * N + 2 * lane);
+        zr.lds(zt + (row0 + t) * N + 2 * lane);
+        const float2 xv = round2<(kX < 3 && sizeof(XT) == 4)>(xr.get()), zv = round2<(kZ < 3 && sizeof(ZT) == 4)>(zr.get());
+        const float2 prev = t > 0 ? sum[t > 0 ? t - 1 : 0] : make_float2(0.f, 0.f);
+        const float ex = dir == 0 ? edge.x - sum[t].x : edge.x + prev.x, ey = dir == 0 ? edge.y - sum[t].y : edge.y + prev.y;
+        col_store<kX>(xs, row0 + t, word, xv.x * ex2(ex), xv.y * ex2(ey));
+        if (kZ == 1 && sizeof(ZT) == 2) *reinterpret_cast<uint32_t*>(zs + (row0 + t) * kRow + 2 * word) = zr.bits();
+        else col_store<kZ>(zs, row0 + t, word, zv.x, zv.y);
+    }
+}
+
+// grid (b h, direction); direction 0 walks rightward (decay to the chunk's right edge), 1 leftward; four warps per pair of
+// inputs (the backward's two share the decays' tile).  kZ parts of z, kX parts of the scaled x; kRows: the state's rows are
+// the channels of x (else its columns).  A chunk's tiles are fetched while the previous chunk's products run, and the tiles
+// of the two chunks behind it into L2, so a step costs its arithmetic (about 2.4 k cycles) and not a trip to memory.
+template <typename XT, typename ZT0, typename ZT1, int kZ, int kX, bool kRows, int kPairs>
+__global__ void __launch_bounds__(128 * kPairs, kPairs == 1 ? 4 : 2)
+wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mx0,
+                  const __grid_constant__ CUtensorMap mz0, const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mz1) {
+    typedef StateSmem<XT, ZT0, ZT1, kZ, kX, kPairs> S;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int bh = blockIdx.x, dir = blockIdx.y, pair = kPairs > 1 ? threadIdx.x >> 7 : 0;
+    const int b = bh / a.H, h = bh - b * a.H;
+    const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    constexpr int kState = kX * kStateWords / 4;
+    uint4* out = a.out + (static_cast<size_t>(pair) * 2 + dir) * a.plane + static_cast<size_t>(bh) * a.n_chunks * kState;
+    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem + S::planes + pair * S::per_pair);
+    __nv_bfloat16* zs = xs + kX * kPlane;
+    Totals* tots = reinterpret_cast<Totals*>(zs + kZ * kPlane);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::bar);
+    const auto chunk_of = [&](int step) { return dir == 0 ? step : a.n_chunks - 1 - step; };
+    const auto fetch = [&](int step) {
+        const int t0 = chunk_of(step) * kChunk;
+        sm100::mbar_expect_tx(bar, S::loaded);
+        sm100::tma_load_3d(smem + S::w, &mw, bar, h * N, t0, b);
+        sm100::tma_load_3d(smem + S::x0, &mx0, bar, h * N, t0, b);
+        sm100::tma_load_3d(smem + S::z0, &mz0, bar, h * N, t0, b);
+        if (kPairs > 1) {
+            sm100::tma_load_3d(smem + S::x1, &mx1, bar, h * N, t0, b);
+            sm100::tma_load_3d(smem + S::z1, &mz1, bar, h * N, t0, b);
+        }
+    };
+    const auto fetch_l2 = [&](int step) {
+        const int t0 = chunk_of(step) * kChunk;
+        sm100::tma_prefetch_3d(&mw, h * N, t0, b);
+        sm100::tma_prefetch_3d(&mx0, h * N, t0, b);
+        sm100::tma_prefetch_3d(&mz0, h * N, t0, b);
+        if (kPairs > 1) {
+            sm100::tma_prefetch_3d(&mx1, h * N, t0, b);
+            sm100::tma_prefetch_3d(&mz1, h * N, t0, b);
+        }
+    };
+    const int last = a.n_chunks - 1;        // steps that update the state
+    if (threadIdx.x == 0) {
+        sm100::mbar_init(bar, 1);
+        sm100::mbar_init_fence();
+        fetch(0);
+        for (int s = 1; s < 3 && s < last; ++s) fetch_l2(s);
+    }
+    __syncthreads();
+    Acc c;
+    zero(c);
+    for (int step = 0; step < last; ++step) {
+        const int n = chunk_of(step);
+        const int valid = a.T - n * kChunk;
+        Totals& tot = tots[step & 1];
+        if (!sm100::mbar_wait(bar, step & 1, kWaitLimit)) report_failure(a.status, a.mirror, 2u);
+        const float* wt = reinterpret_cast<const float*>(smem + S::w);
+        if (kPairs == 1 || pair == 0)
+            scale_chunk<XT, ZT0, kZ, kX>(wt, reinterpret_cast<const XT*>(smem + S::x0), reinterpret_cast<const ZT0*>(smem + S::z0), valid, dir, tot,
+                                         xs, zs, warp, lane);
+        else
+            scale_chunk<XT, ZT1, kZ, kX>(wt, reinterpret_cast<const XT*>(smem + S::x1), reinterpret_cast<const ZT1*>(smem + S::z1), valid, dir, tot,
+                                         xs, zs, warp, lane);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (step + 1 < last) fetch(step + 1);
+            if (step + 3 < last) fetch_l2(step + 3);
+        }
+        // decay of the state across the chunk
+        if (kRows) {
+            const int ch = 16 * warp + 4 * (g >> 1) + (g & 1);
+            const float s0 = ex2((tot[0][ch] + tot[1][ch]) + (tot[2][ch] + tot[3][ch]));
+            const float s1 = ex2((tot[0][ch + 2] + tot[1][ch + 2]) + (tot[2][ch + 2] + tot[3][ch + 2]));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { c[i][0] *= s0; c[i][1] *= s0; c[i][2] *= s1; c[i][3] *= s1; }
+        } else {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int j = 0; j < kBlocks; ++j) {
+                    float t[4];
+                    row4(tot[j], kk, q, t);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[e] += t[e];
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float d = ex2(s[e]);
+                    at(c, 0, kk, e) *= d;
+                    at(c, 1, kk, e) *= d;
+                }
+            }
+        }
+        const __nv_bfloat16* pm = kRows ? xs : zs;       // rows of the state
+        const __nv_bfloat16* pn = kRows ? zs : xs;       // columns
+        constexpr int kM = kRows ? kX : kZ, kN = kRows ? kZ : kX;
+#pragma unroll
+        for (int s = 0; s < kBlocks; ++s) {
+            uint32_t am[kM][4];
+#pragma unroll
+            for (int i = 0; i < kM; ++i) ldsm4t(am[i], smem_addr(pm + i * kPlane + s * kBlock * kRow + 16 * warp + off_tok(lane)));
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int ib = 0; ib < kN; ++ib) {
+                    uint32_t r[4];
+                    ldsm4t(r, smem_addr(pn + ib * kPlane + s * kBlock * kRow + 16 * kk + off_pos(lane)));
+#pragma unroll
+                    for (int ia = 0; ia < kM; ++ia)
+                        if (Keep<kM, kN>::on(ia, ib)) {
+                            mma(c[2 * kk], am[ia], r[0], r[1]);
+                            mma(c[2 * kk + 1], am[ia], r[2], r[3]);
+                        }
+                }
+        }
+        uint4* o = out + static_cast<size_t>(chunk_of(step + 1)) * kState;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            uint32_t w0[kX], w1[kX], w2[kX], w3[kX];
+            split<kX>(c[2 * kk][0], c[2 * kk][1], w0);
+            split<kX>(c[2 * kk + 1][0], c[2 * kk + 1][1], w1);
+            split<kX>(c[2 * kk][2], c[2 * kk][3], w2);
+            split<kX>(c[2 * kk + 1][2], c[2 * kk + 1][3], w3);
+#pragma unroll
+            for (int s = 0; s < kX; ++s)
+                o[s * (kStateWords / 4) + (warp * 4 + kk) * 32 + lane] = make_uint4(w0[s], w1[s], w2[s], w3[s]);
+        }
+    }
+}
+
+// ---- pieces of kernel 2 ----------------------------------------------------------------------------------------
+// Eight warps.  Token-by-token matrices (pairs inside the chunk) are formed by warp (block, dir): the block's rows against
+// itself and everything earlier (dir 0) or later (dir 1).  Results with channel columns are formed by warp (slice, half):
+// 16 channels, 32 tokens, both directions, so that a warp reads only its slice of the states and planes.
+// Table tab holds the inclusive sums of l over each block (row = token).
+
+// x (16 x 64, A layout) of a row range of a tensor
+template <typename T, bool kRound>
+__device__ __forceinline__ void load_block(Block& x, const T* p, int C, int rows, int g, int q) {
+    Raw<T> raw;
+    raw.load(p, C, rows, g, q);
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            float t[4];
+            raw.get(half, kk, t);
+            round4<kRound>(t);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[half][kk][e] = t[e];
+        }
+}
+// Exponent of a row's factor towards the partners' side: dir 0: sum before the row (to the block's left edge), dir 1:
+// sum after it (right edge); minus the block's whole sum when `inner` (the operand then meets the block's own partners,
+// whose planes are scaled to the far edge).
+__device__ __forceinline__ void row_exponents(const Table& tab, int blk, int row, int dir, bool inner, int kk, int q, float (&x)[4]) {
+    float total[4] = {0.f, 0.f, 0.f, 0.f};
+    if ((dir == 0) == inner) row4(tab[blk * kBlock + kBlock - 1], kk, q, total);
+    if (dir == 0) {
+        if (row == 0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] = 0.f - total[e];
+        } else {
+            row4(tab[blk * kBlock + row - 1], kk, q, x);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] -= total[e];
+        }
+    } else {
+        row4(tab[blk * kBlock + row], kk, q, x);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = total[e] - x[e];
+    }
+}
+// columns times 2^(sum over block j)
+__device__ __forceinline__ void cross_block(Block& x, const Table& tab, int j, int q) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        float f[4];
+        row4(tab[j * kBlock + kBlock - 1], kk, q, f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float d = ex2(f[e]);
+            x[0][kk][e] *= d;
+            x[1][kk][e] *= d;
+        }
+    }
+}
+__device__ __forceinline__ bool block_is_safe(const Table& tab, int blk, int lane) {
+    const float2 t = *reinterpret_cast<const float2*>(&tab[blk * kBlock + kBlock - 1][2 * lane]);
+    return !__any_sync(0xffffffffu, !(t.x > -kSafe && t.y > -kSafe));
+}
+
+// row and column of C-fragment element (nt, i) inside the block
+__device__ __forceinline__ int frag_row(int i, int g) { return g + 8 * (i >> 1); }
+__device__ __forceinline__ int frag_col(int nt, int i, int q) { return 8 * nt + 2 * q + (i & 1); }
+
+// Levels of halves for a block whose decay is too strong for factors above 1: at half size hs a token is scaled towards
+// the boundary between the two halves of its 2 hs tokens, the same factor whichever role it plays.
+__device__ __forceinline__ void level_factors(const Table& tab, int blk, int hs, int row, int kk, int q, float (&f)[4]) {
+    const int mid = (row & ~(2 * hs - 1)) + hs;          // first row behind the boundary
+    float b[4], x[4];
+    row4(tab[blk * kBlock + mid - 1], kk, q, b);
+    const bool later = row >= mid;
+    row4(tab[blk * kBlock + (later ? row - 1 : row)], kk, q, x);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = ex2(later ? x[e] - b[e] : b[e] - x[e]);
+}
+__device__ __forceinline__ bool on_level(int t, int s, int hs) { return (t / (2 * hs)) == (s / (2 * hs)) && ((t & hs) != (s & hs)); }
+template <int NS>
+__device__ __forceinline__ void level_frag(AFrag<NS>& o, const Block& x, const Table& tab, int blk, int hs, int g, int q) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        float f0[4], f1[4];
+        level_factors(tab, blk, hs, g, kk, q, f0);
+        level_factors(tab, blk, hs, g + 8, kk, q, f1);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { f0[e] *= x[0][kk][e]; f1[e] *= x[1][kk][e]; }
+        o.set(kk, f0, f1);
+    }
+}
+// p[row][col] = sum_i a_row[i] b_col[i] D(row, col)[i] for all pairs of the block (both directions)
+template <int NS>
+__device__ __noinline__ void strong_pairs(float (&p)[2][4], const Block& a, const Block& b, const Table& tab, int blk, int g, int q) {
+#pragma unroll 1
+    for (int hs = 8; hs >= 1; hs >>= 1) {
+        AFrag<NS> A, Bf;
+        level_frag<NS>(A, a, tab, blk, hs, g, q);
+        level_frag<NS>(Bf, b, tab, blk, hs, g, q);
+        float c[2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int ib = 0; ib < NS; ++ib)
+#pragma unroll
+                for (int ia = 0; ia < NS; ++ia)
+                    if (Keep<NS, NS>::on(ia, ib)) {      // a block's B fragments are its A fragments, half by half
+                        mma(c[0], A.w[ia][kk], Bf.w[ib][kk][0], Bf.w[ib][kk][2]);
+                        mma(c[1], A.w[ia][kk], Bf.w[ib][kk][1], Bf.w[ib][kk][3]);
+                    }
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (on_level(frag_row(i, g), frag_col(nt, i, q), hs)) p[nt][i] = c[nt][i];
+    }
+}
+// out[row half][e] += sum_s m[t][s] D(t, s) (x) x_s over the pairs of block blk on one side (dir 0: s earlier), for the 16
+// channels of slice cs; m: the whole matrix (planes of NS parts, transposed if kTransM), x: the block's rows of the partner
+template <typename T, int NS, bool kTransM, bool kRound>
+__device__ __noinline__ void strong_gradients(float (&out)[2][4], const __nv_bfloat16* m, const T* x, int C, int rows, const Table& tab,
+                                              int blk, int cs, int dir, int lane) {
+    const int g = lane >> 2, q = lane & 3;
+    uint32_t a[NS][4];
+#pragma unroll
+    for (int ia = 0; ia < NS; ++ia) {
+        if (kTransM) ldsm4t(a[ia], smem_addr(m + ia * kPlane + blk * kBlock * kRow + blk * kBlock + off_tok(lane)));
+        else ldsm4(a[ia], smem_addr(m + ia * kPlane + blk * kBlock * kRow + blk * kBlock + off_a(lane)));
+    }
+    float xv[2][4];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) xv[half][e] = 0.f;
+        if (g + 8 * half < rows) load4(x + static_cast<size_t>(g + 8 * half) * C + 16 * cs + 4 * q, xv[half]);
+        round4<kRound>(xv[half]);
+    }
+#pragma unroll 1
+    for (int hs = 8; hs >= 1; hs >>= 1) {
+        float f[2][4], c[2][4] = {};
+        level_factors(tab, blk, hs, g, cs, q, f[0]);
+        level_factors(tab, blk, hs, g + 8, cs, q, f[1]);
+        // fragment words of m: word i holds row g (+ 8 for odd i), columns 2 q, 2 q + 1 (+ 8 for i >= 2)
+        uint32_t am[NS][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = g + 8 * (i & 1), col = 2 * q + 8 * (i >> 1);
+            uint32_t keep = 0u;
+            if (on_level(row, col, hs) && (dir == 0 ? col < row : col > row)) keep |= 0x0000ffffu;
+            if (on_level(row, col + 1, hs) && (dir == 0 ? col + 1 < row : col + 1 > row)) keep |= 0xffff0000u;
+#pragma unroll
+            for (int ia = 0; ia < NS; ++ia) am[ia][i] = a[ia][i] & keep;
+        }
+        uint32_t w0[NS], w1[NS], w2[NS], w3[NS];
+        split<NS>(xv[0][0] * f[0][0], xv[0][1] * f[0][1], w0);
+        split<NS>(xv[1][0] * f[1][0], xv[1][1] * f[1][1], w1);
+        split<NS>(xv[0][2] * f[0][2], xv[0][3] * f[0][3], w2);
+        split<NS>(xv[1][2] * f[1][2], xv[1][3] * f[1][3], w3);
+#pragma unroll
+        for (int ib = 0; ib < NS; ++ib) {
+            const uint32_t b0 = movm_trans(w0[ib]), b1 = movm_trans(w1[ib]), b2 = movm_trans(w2[ib]), b3 = movm_trans(w3[ib]);
+#pragma unroll
+            for (int ia = 0; ia < NS; ++ia)
+                if (Keep<NS, NS>::on(ia, ib)) {
+                    mma(c[0], am[ia], b0, b1);
+                    mma(c[1], am[ia], b2, b3);
+                }
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) out[half][e] = fmaf(f[half][e], c[e >> 1][half * 2 + (e & 1)], out[half][e]);
+    }
+}
+__device__ __forceinline__ void copy(Block& to, const Block& from) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) to[half][kk][e] = from[half][kk][e];
+}
+
+// sum over this thread's quad of x . u . y per row
+__device__ __forceinline__ void bonus_terms(const Block& x, const Block& y, const float* u, int q, float (&out)[2]) {
+    out[0] = out[1] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        float uu[4];
+        row4(u, kk, q, uu);
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) out[half] += x[half][kk][e] * uu[e] * y[half][kk][e];
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        out[half] += __shfl_xor_sync(0xffffffffu, out[half], 1);
+        out[half] += __shfl_xor_sync(0xffffffffu, out[half], 2);
+    }
+}
+// sums of l over a block's tokens into the table (a warp per block, lane = two channels)
+template <bool kAccurate>
+__device__ __forceinline__ void scan_block(Table& tab, const float* w, int C, int rows, int blk, int lane) {
+    Pair<float> wr[kBlock];
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) wr[t].load(w + static_cast<size_t>(t) * C + 2 * lane, t < rows);
+    float2 run = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) {
+        if (t < rows) {
+            run.x += log2_decay<kAccurate>(wr[t].v.x);
+            run.y += log2_decay<kAccurate>(wr[t].v.y);
+        }
+        *reinterpret_cast<float2*>(&tab[blk * kBlock + t][2 * lane]) = run;
+    }
+}
+// a block's rows as they are, into planes
+template <typename T, int NS, bool kRound>
+__device__ __forceinline__ void stage_rows(__nv_bfloat16* planes, const T* p, int C, int rows, int blk, int lane) {
+    Pair<T> x[kBlock];
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) x[t].load(p + static_cast<size_t>(t) * C + 2 * lane, t < rows);
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) {
+        const float2 v = round2<kRound>(x[t].get());
+        col_store<NS>(planes, blk * kBlock + t, col_word(lane), v.x, v.y);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void load_rows(Pair<T> (&x)[kBlock], const T* p, int C, int rows, int lane) {
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) x[t].load(p + static_cast<size_t>(t) * C + 2 * lane, t < rows);
+}
+// a block's rows scaled to its right edge (for partners later than it: dir 0) or left edge (dir 1), into planes
+template <typename T, int NS, bool kRound>
+__device__ __forceinline__ void stage_scaled(__nv_bfloat16* planes, const Pair<T> (&x)[kBlock], const Table& tab, int blk, int dir, int lane) {
+    const float2 total = *reinterpret_cast<const float2*>(&tab[blk * kBlock + kBlock - 1][2 * lane]);
+    float2 prev = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) {
+        const float2 v = round2<kRound>(x[t].get());
+        const float2 s = *reinterpret_cast<const float2*>(&tab[blk * kBlock + t][2 * lane]);
+        const float ex = dir == 0 ? total.x - s.x : prev.x, ey = dir == 0 ? total.y - s.y : prev.y;
+        col_store<NS>(planes, blk * kBlock + t, col_word(lane), v.x * ex2(ex), v.y * ex2(ey));
+        prev = s;
+    }
+}
+// a 16 x 16 tile (C fragments) into planes of 64 x 64 token-by-token parts
+template <int NS>
+__device__ __forceinline__ void store_tile(__nv_bfloat16* planes, const float (&m)[2][4], int mrow, int mcol, int g, int q) {
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            uint32_t t[NS];
+            split<NS>(m[nt][2 * half], m[nt][2 * half + 1], t);
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                *reinterpret_cast<uint32_t*>(planes + s * kPlane + (mrow * kBlock + g + 8 * half) * kRow + mcol * kBlock + 8 * nt + 2 * q) = t[s];
+        }
+}
+
+// Row-mapped part of y (rows r, columns k) and gv (rows k, columns r): warp (blk, dir) forms its pairs of the token matrix
+// and leaves the rows scaled to the chunk's edge (for the entering state) in the planes `edges`.  The two directions of
+// a diagonal tile are merged by the masks: dir 0 writes below the diagonal and on it, dir 1 above.
+template <typename T, int kX, bool kRound>
+__device__ __forceinline__ void pair_rows(const T* row_in, const T* col_in, const float* u, const Table& tab, const __nv_bfloat16* planes,
+                                          __nv_bfloat16* pairs, __nv_bfloat16* edges, int C, int rows, int blk, int dir, int lane) {
+    const int g = lane >> 2, q = lane & 3;
+    const bool safe = block_is_safe(tab, blk, lane);
+    Block x;
+    load_block<T, kRound>(x, row_in, C, rows, g, q);
+    AFrag<kX> f;
+    {
+        float p[2][4] = {}, diag[2] = {0.f, 0.f};
+        if (dir == 0 || !safe) {
+            Block c;
+            load_block<T, kRound>(c, col_in, C, rows, g, q);
+            if (dir == 0) bonus_terms(x, c, u, q, diag);
+            if (!safe) {
+                // copies: what a call takes by reference lives in memory, and x stays in registers
+                Block xc, cc;
+                float pc[2][4] = {};
+                copy(xc, x);
+                copy(cc, c);
+                strong_pairs<kX>(pc, xc, cc, tab, blk, g, q);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) p[i >> 2][i & 3] = pc[i >> 2][i & 3];
+            }
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                float e4[4];
+                row_exponents(tab, blk, g + 8 * half, dir, safe, kk, q, e4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[half][kk][e] *= ex2(e4[e]);
+            }
+        if (safe) {
+            f.set(x);
+            prod_tokens<kX, kX>(p, f, planes, blk, lane);
+            cross_block(x, tab, blk, q);
+        }
+        // merge with the other direction's half of the tile
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int row = g + 8 * half, col = 8 * nt + 2 * q;
+                if (dir == 0) {
+                    if (col == row) p[nt][2 * half] = diag[half];
+                    if (col + 1 == row) p[nt][2 * half + 1] = diag[half];
+                }
+                const bool on0 = dir == 0 ? col <= row : col > row, on1 = dir == 0 ? col + 1 <= row : col + 1 > row;
+                uint32_t t[kX];
+                split<kX>(p[nt][2 * half], p[nt][2 * half + 1], t);
+#pragma unroll
+                for (int s = 0; s < kX; ++s) {
+                    __nv_bfloat16* d = pairs + s * kPlane + (blk * kBlock + row) * kRow + blk * kBlock + col;
+                    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&t[s]);
+                    if (on0 && on1) *reinterpret_cast<uint32_t*>(d) = t[s];
+                    else if (on0) d[0] = v.x;
+                    else if (on1) d[1] = v.y;
+                }
+            }
+    }
+#pragma unroll 1
+    for (int j = dir == 0 ? blk - 1 : blk + 1; j >= 0 && j < kBlocks; j += dir == 0 ? -1 : 1) {
+        f.set(x);
+        float p[2][4] = {};
+        prod_tokens<kX, kX>(p, f, planes, j, lane);
+        store_tile<kX>(pairs, p, blk, j, g, q);
+        cross_block(x, tab, j, q);
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            __nv_bfloat16* d = edges + (blk * kBlock + g + 8 * half) * kRow + 16 * kk + 2 * q;
+            uint32_t t[kX];
+            split<kX>(x[half][kk][0], x[half][kk][1], t);
+#pragma unroll
+            for (int s = 0; s < kX; ++s) *reinterpret_cast<uint32_t*>(d + s * kPlane) = t[s];
+            split<kX>(x[half][kk][2], x[half][kk][3], t);
+#pragma unroll
+            for (int s = 0; s < kX; ++s) *reinterpret_cast<uint32_t*>(d + s * kPlane + 8) = t[s];
+        }
+}
+// Slice-mapped part: y[32 tokens x 16 channels] = pairs * values + edge-scaled rows * entering states
+template <int kZ, int kX, bool kTrans>
+__device__ __forceinline__ void pair_outputs(float (&y)[2][2][4], const __nv_bfloat16* pairs, const __nv_bfloat16* values,
+                                             const __nv_bfloat16* edges_left, const __nv_bfloat16* edges_right, const uint4* from_left,
+                                             const uint4* from_right, int cs, int th, int lane) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) y[i >> 3][(i >> 2) & 1][i & 3] = 0.f;
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        const uint4* st = dir ? from_right : from_left;
+        if (st == nullptr) continue;
+        const __nv_bfloat16* ed = dir ? edges_right : edges_left;
+        uint32_t f[4][kX][4];
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) state_frag<kX, kTrans>(f[kk], st, cs, kk, lane);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int ia = 0; ia < kX; ++ia) {
+                    uint32_t a[4];
+                    ldsm4(a, smem_addr(ed + ia * kPlane + (2 * th + m) * kBlock * kRow + 16 * kk + off_a(lane)));
+#pragma unroll
+                    for (int ib = 0; ib < kX; ++ib)
+                        if (Keep<kX, kX>::on(ia, ib)) {
+                            mma(y[m][0], a, f[kk][ib][0], f[kk][ib][1]);
+                            mma(y[m][1], a, f[kk][ib][2], f[kk][ib][3]);
+                        }
+                }
+    }
+#pragma unroll
+    for (int b = 0; b < kBlocks; ++b)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) prod_slice<kX, kZ, false>(y[m], pairs, 2 * th + m, b, values, b, cs, lane);
+}
+
+// ---- kernel 2, forward ---------------------------------------------------------------------------------------
+struct OutArgs {
+    int T, H, n_chunks;
+    const void* r;
+    const void* k;
+    const void* v;
+    const float* w;
+    const float* u;
+    float* y;
+    bool scalar;              // y is not 16-byte aligned: 4-byte stores
+    const uint4* states;      // [direction][b h][chunk][part][..], rows = value channels
+    size_t plane;
+};
+
+// kX parts of the scaled operands and states, kZ parts of v
+template <typename T, int kZ, int kX>
+__global__ void __launch_bounds__(256, kX == 1 ? 3 : 1) wkv6_forward_kernel(const OutArgs a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __nv_bfloat16* kf = reinterpret_cast<__nv_bfloat16*>(smem);       // k towards the right edge of its block, left edge behind it
+    __nv_bfloat16* pairs = kf + 2 * kX * kPlane;
+    __nv_bfloat16* edges = pairs + kX * kPlane;
+    __nv_bfloat16* vs = edges + 2 * kX * kPlane;
+    Table& tab = *reinterpret_cast<Table*>(vs + kZ * kPlane);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int n = blockIdx.x % a.n_chunks, bh = blockIdx.x / a.n_chunks;
+    const int b = bh / a.H, h = bh - b * a.H, C = a.H * N;
+    const size_t base = (static_cast<size_t>(b) * a.T + n * kChunk) * C + static_cast<size_t>(h) * N;
+    constexpr bool kRound = kX < 3 && sizeof(T) == 4;
+    {
+        const int blk = warp & 3, dir = warp >> 2;
+        const int rows = a.T - (n * kChunk + blk * kBlock);
+        const size_t at0 = base + static_cast<size_t>(blk) * kBlock * C;
+        const T* k = static_cast<const T*>(a.k) + at0;
+        __nv_bfloat16* planes = kf + dir * kX * kPlane;
+        Pair<T> kr[kBlock];
+        load_rows<T>(kr, k, C, rows, lane);
+        if (dir == 0) scan_block<(kX > 2)>(tab, a.w + at0, C, rows, blk, lane);
+        else stage_rows<T, kZ, kRound>(vs, static_cast<const T*>(a.v) + at0, C, rows, blk, lane);
+        __syncthreads();
+        stage_scaled<T, kX, kRound>(planes, kr, tab, blk, dir, lane);
+        __syncthreads();
+        pair_rows<T, kX, kRound>(static_cast<const T*>(a.r) + at0, k, a.u + h * N, tab, planes, pairs, edges + dir * kX * kPlane, C, rows, blk, dir, lane);
+    }
+    __syncthreads();
+    const int cs = warp & 3, th = warp >> 2;
+    const uint4* st = a.states + (static_cast<size_t>(bh) * a.n_chunks + n) * (kX * kStateWords / 4);
+    float y[2][2][4];
+    pair_outputs<kZ, kX, false>(y, pairs, vs, edges, edges + kX * kPlane, n > 0 ? st : nullptr, n + 1 < a.n_chunks ? st + a.plane : nullptr, cs, th, lane);
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int t = 32 * th + 16 * m + 8 * half + g;
+            if (n * kChunk + t < a.T)
+                put4(a.scalar, a.y + base + static_cast<size_t>(t) * C + 16 * cs + 4 * q, y[m][0][2 * half], y[m][0][2 * half + 1],
+                     y[m][1][2 * half], y[m][1][2 * half + 1]);
+        }
+}
+
+// ---- kernel 2, backward --------------------------------------------------------------------------------------
+struct GradArgs {
+    int T, H, n_chunks;
+    const void* r;
+    const void* k;
+    const void* v;
+    const void* gy;
+    const float* w;
+    const float* u;
+    void* gr;
+    void* gk;
+    void* gv;
+    float* gw;
+    float* gu_part;           // [b][chunk][C]
+    bool scalar;              // an output is not 16-byte aligned: element stores
+    const uint4* states;      // [pair][direction][b h][chunk][part][..], rows = channels of r, k
+    size_t plane;
+};
+
+// gr (own = gy, partners k, m = gy v^T) or gk (own = v, partners r, m transposed) for 32 tokens x 16 channels:
+//   early / late[m tile][row half][e] = sum over earlier / later tokens s of (own_t . other_s) D(t, s) (x) partner_s,
+// from the entering state inward: every block the sum crosses decays it, the block's own pairs come last.
+template <typename T, int kZ, int kX, bool kTransM, bool kRound>
+__device__ __forceinline__ void slice_gradient(float (&out)[2][2][2][4], const __nv_bfloat16* own, const __nv_bfloat16* m, const __nv_bfloat16* planes,
+                                               const uint4* from_left, const uint4* from_right, const Table& tab, const T* partner, int C,
+                                               int rows, unsigned strong, int cs, int th, int lane) {
+    const int g = lane >> 2, q = lane & 3;
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        float c[2][2][4];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) c[i >> 3][(i >> 2) & 1][i & 3] = 0.f;
+        const uint4* st = dir ? from_right : from_left;
+        if (st != nullptr) {
+            uint32_t f[4][kX][4];
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) state_frag<kX, false>(f[kk], st, cs, kk, lane);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                    for (int ia = 0; ia < kZ; ++ia) {
+                        uint32_t a[4];
+                        ldsm4(a, smem_addr(own + ia * kPlane + (2 * th + mt) * kBlock * kRow + 16 * kk + off_a(lane)));
+#pragma unroll
+                        for (int ib = 0; ib < kX; ++ib)
+                            if (Keep<kZ, kX>::on(ia, ib)) {
+                                mma(c[mt][0], a, f[kk][ib][0], f[kk][ib][1]);
+                                mma(c[mt][1], a, f[kk][ib][2], f[kk][ib][3]);
+                            }
+                    }
+        }
+        const __nv_bfloat16* pl = planes + dir * kX * kPlane;
+#pragma unroll
+        for (int step = 0; step < kBlocks; ++step) {
+            const int j = dir == 0 ? step : kBlocks - 1 - step;
+            if (dir == 0 ? j > 2 * th + 1 : j < 2 * th) continue;            // beyond both tiles of this warp
+            float d[4];
+            row4(tab[j * kBlock + kBlock - 1], cs, q, d);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d[e] = ex2(d[e]);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                const int blk = 2 * th + mt;
+                if (dir == 0 ? j > blk : j < blk) continue;
+                if (j == blk && ((strong >> blk) & 1u)) continue;
+#pragma unroll
+                for (int half = 0; half < 2; ++half)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) c[mt][e >> 1][2 * half + (e & 1)] *= d[e];
+                if (j != blk) {
+                    prod_slice<kX, kX, kTransM>(c[mt], m, blk, j, pl, j, cs, lane);
+                } else {
+                    // the block's own tile, masked to this direction
+                    uint32_t a[kX][4];
+#pragma unroll
+                    for (int ia = 0; ia < kX; ++ia) {
+                        if (kTransM) ldsm4t(a[ia], smem_addr(m + ia * kPlane + blk * kBlock * kRow + blk * kBlock + off_tok(lane)));
+                        else ldsm4(a[ia], smem_addr(m + ia * kPlane + blk * kBlock * kRow + blk * kBlock + off_a(lane)));
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int row = g + 8 * (i & 1), col = 2 * q + 8 * (i >> 1);
+                            const uint32_t keep = ((dir == 0 ? col < row : col > row) ? 0x0000ffffu : 0u) |
+                                                  ((dir == 0 ? col + 1 < row : col + 1 > row) ? 0xffff0000u : 0u);
+                            a[ia][i] &= keep;
+                        }
+                    }
+#pragma unroll
+                    for (int ib = 0; ib < kX; ++ib) {
+                        uint32_t r[4];
+                        ldsm4t(r, smem_addr(pl + ib * kPlane + blk * kBlock * kRow + cs * 16 + off_pos(lane)));
+#pragma unroll
+                        for (int ia = 0; ia < kX; ++ia)
+                            if (Keep<kX, kX>::on(ia, ib)) {
+                                mma(c[mt][0], a[ia], r[0], r[1]);
+                                mma(c[mt][1], a[ia], r[2], r[3]);
+                            }
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            const int blk = 2 * th + mt;
+            const bool safe = ((strong >> blk) & 1u) == 0u;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float f[4];
+                row_exponents(tab, blk, g + 8 * half, dir, safe, cs, q, f);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) out[dir][mt][half][e] = ex2(f[e]) * c[mt][e >> 1][2 * half + (e & 1)];
+            }
+            if (!safe) {
+                float o[2][4];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i >> 2][i & 3] = out[dir][mt][i >> 2][i & 3];
+                strong_gradients<T, kX, kTransM, kRound>(o, m, partner + static_cast<size_t>(blk) * kBlock * C, C, rows - blk * kBlock, tab, blk, cs,
+                                                         dir, lane);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) out[dir][mt][i >> 2][i & 3] = o[i >> 2][i & 3];
+            }
+        }
+    }
+}
+
+// kZ parts of v, gy; kX parts of scaled operands, token products and states; kP parts where only gv is concerned
+template <typename T, typename G, typename O, int kZ, int kX, int kP>
+__global__ void __launch_bounds__(256, kX < 3 ? 2 : 1) wkv6_backward_kernel(const GradArgs a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __nv_bfloat16* vs = reinterpret_cast<__nv_bfloat16*>(smem);
+    __nv_bfloat16* gs = vs + kZ * kPlane;
+    __nv_bfloat16* pf = gs + kZ * kPlane;        // k, then r, towards the right edge of its block, left edge behind it
+    __nv_bfloat16* ms = pf + 2 * kX * kPlane;    // gy v^T inside the chunk, later the pairs of gv
+    Table& tab = *reinterpret_cast<Table*>(ms + kX * kPlane);
+    float* dots = reinterpret_cast<float*>(&tab + 1);       // [kChunk]: gy_t . v_t
+    float* edge = dots + N;                                 // [2][N]
+    float* gus = edge + 2 * N;                              // [2][N]
+    float* seg = gus + 2 * N;                               // [8][N]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int blk = warp & 3, dir = warp >> 2;              // row-mapped phases
+    const int cs = warp & 3, th = warp >> 2;                // slice-mapped phases
+    const int n = blockIdx.x % a.n_chunks, bh = blockIdx.x / a.n_chunks;
+    const int b = bh / a.H, h = bh - b * a.H, C = a.H * N;
+    const int tokens = a.T - n * kChunk, rows = tokens - blk * kBlock;
+    const size_t base = (static_cast<size_t>(b) * a.T + n * kChunk) * C + static_cast<size_t>(h) * N;
+    const size_t at0 = base + static_cast<size_t>(blk) * kBlock * C;
+    constexpr bool kRound = kX < 3 && sizeof(T) == 4, kRoundG = kX < 3 && sizeof(G) == 4;
+    constexpr int kState = kX * kStateWords / 4;
+    // states entering this chunk, [pair (k v | r gy)][from the left | from the right]
+    const uint4* st = a.states + (static_cast<size_t>(bh) * a.n_chunks + n) * kState;
+    const bool left = n > 0, right = n + 1 < a.n_chunks;
+    const uint4 *s_left = left ? st : nullptr, *s_right = right ? st + a.plane : nullptr;
+    const uint4 *a_left = left ? st + 2 * a.plane : nullptr, *a_right = right ? st + 3 * a.plane : nullptr;
+    const T* rp = static_cast<const T*>(a.r);
+    const T* kp = static_cast<const T*>(a.k);
+
+    Pair<T> col[kBlock];
+    load_rows<T>(col, kp + at0, C, rows, lane);
+    if (dir == 0) {
+        scan_block<(kX > 2)>(tab, a.w + at0, C, rows, blk, lane);
+    } else {
+        stage_rows<T, kZ, kRound>(vs, static_cast<const T*>(a.v) + at0, C, rows, blk, lane);
+        stage_rows<G, kZ, kRoundG>(gs, static_cast<const G*>(a.gy) + at0, C, rows, blk, lane);
+    }
+    __syncthreads();
+    stage_scaled<T, kX, kRound>(pf + dir * kX * kPlane, col, tab, blk, dir, lane);
+    // m = gy v^T: two of the sixteen tiles per warp
+    {
+        AFrag<kZ> own;
+#pragma unroll
+        for (int s = 0; s < kZ; ++s)
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) ldsm4(own.w[s][kk], smem_addr(gs + s * kPlane + blk * kBlock * kRow + 16 * kk + off_a(lane)));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int j = 2 * dir + i;
+            float m[2][4] = {};
+            prod_tokens<kZ, kZ>(m, own, vs, j, lane);
+            store_tile<kX>(ms, m, blk, j, g, q);
+            if (j == blk) {
+                // diagonal: row g sits in lane (g, g / 2), row g + 8 likewise in the second half
+                if (q == (g >> 1)) {
+                    dots[blk * kBlock + g] = (g & 1) ? m[0][1] : m[0][0];
+                    dots[blk * kBlock + g + 8] = (g & 1) ? m[1][3] : m[1][2];
+                }
+            }
+        }
+    }
+    // pairs that straddle the chunk's right edge, per channel (see the file header)
+    {
+        float e0 = 0.f, e1 = 0.f;
+        if (right) {
+            const uint4* sx = dir == 0 ? st + kState : st + 2 * a.plane + kState;       // passed the edge rightward
+            const uint4* sy = dir == 0 ? st + 3 * a.plane : st + a.plane;               // ... leftward
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                float x[8] = {}, y[8] = {};
+#pragma unroll
+                for (int i = 0; i < kX; ++i) {
+                    const int o = i * (kStateWords / 4) + (blk * 4 + kk) * 32 + lane;
+                    const uint4 fx = __ldg(sx + o), fy = __ldg(sy + o);
+                    const uint32_t wx[4] = {fx.x, fx.y, fx.z, fx.w}, wy[4] = {fy.x, fy.y, fy.z, fy.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        x[2 * j] += lo_f(wx[j]); x[2 * j + 1] += hi_f(wx[j]);
+                        y[2 * j] += lo_f(wy[j]); y[2 * j + 1] += hi_f(wy[j]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { e0 = fmaf(x[j], y[j], e0); e1 = fmaf(x[4 + j], y[4 + j], e1); }
+            }
+        }
+        e0 += __shfl_xor_sync(0xffffffffu, e0, 1); e0 += __shfl_xor_sync(0xffffffffu, e0, 2);
+        e1 += __shfl_xor_sync(0xffffffffu, e1, 1); e1 += __shfl_xor_sync(0xffffffffu, e1, 2);
+        const int ch = 16 * blk + 4 * (g >> 1) + (g & 1);
+        if (q == 0) { edge[dir * N + ch] = e0; edge[dir * N + ch + 2] = e1; }
+    }
+    unsigned strong = 0u;
+#pragma unroll
+    for (int j = 0; j < kBlocks; ++j) strong |= block_is_safe(tab, j, lane) ? 0u : 1u << j;
+    __syncthreads();
+
+    float mine[2][2][4], diff[2][2][4];          // r gr> + k gk<, and that minus (r gr< + k gk>)
+    {
+        float u4[4], gu[4] = {0.f, 0.f, 0.f, 0.f};
+        row4(a.u + h * N, cs, q, u4);
+        float o[2][2][2][4];
+        slice_gradient<T, kZ, kX, false, kRound>(o, gs, ms, pf, s_left, s_right, tab, kp + base, C, tokens, strong, cs, th, lane);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int t = 32 * th + 16 * mt + 8 * half + g;
+                float r4[4] = {0.f, 0.f, 0.f, 0.f}, k4[4] = {0.f, 0.f, 0.f, 0.f};
+                const size_t at_t = base + static_cast<size_t>(t) * C + 16 * cs + 4 * q;
+                if (t < tokens) { load4(rp + at_t, r4); load4(kp + at_t, k4); }
+                round4<kRound>(r4);
+                round4<kRound>(k4);
+                const float dot = dots[t];
+                float g4[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float early = o[0][mt][half][e], late = o[1][mt][half][e], kd = k4[e] * dot;
+                    g4[e] = early + late + u4[e] * kd;
+                    mine[mt][half][e] = r4[e] * early;
+                    diff[mt][half][e] = r4[e] * (early - late);
+                    gu[e] = fmaf(r4[e], kd, gu[e]);
+                }
+                if (t < tokens) put4(a.scalar, static_cast<O*>(a.gr) + at_t, g4[0], g4[1], g4[2], g4[3]);
+            }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            gu[e] += __shfl_xor_sync(0xffffffffu, gu[e], 4);
+            gu[e] += __shfl_xor_sync(0xffffffffu, gu[e], 8);
+            gu[e] += __shfl_xor_sync(0xffffffffu, gu[e], 16);
+        }
+        if (g == 0) put_row4(gus + th * N, cs, q, gu[0], gu[1], gu[2], gu[3]);
+        load_rows<T>(col, rp + at0, C, rows, lane);
+    }
+    __syncthreads();               // everyone is done with the planes of k
+    stage_scaled<T, kX, kRound>(pf + dir * kX * kPlane, col, tab, blk, dir, lane);
+    __syncthreads();
+    {
+        float u4[4];
+        row4(a.u + h * N, cs, q, u4);
+        float o[2][2][2][4];
+        slice_gradient<T, kZ, kX, true, kRound>(o, vs, ms, pf, a_left, a_right, tab, rp + base, C, tokens, strong, cs, th, lane);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int t = 32 * th + 16 * mt + 8 * half + g;
+                float r4[4] = {0.f, 0.f, 0.f, 0.f}, k4[4] = {0.f, 0.f, 0.f, 0.f};
+                const size_t at_t = base + static_cast<size_t>(t) * C + 16 * cs + 4 * q;
+                if (t < tokens) { load4(rp + at_t, r4); load4(kp + at_t, k4); }
+                round4<kRound>(r4);
+                round4<kRound>(k4);
+                const float dot = dots[t];
+                float g4[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float early = o[0][mt][half][e], late = o[1][mt][half][e];
+                    g4[e] = early + late + u4[e] * r4[e] * dot;
+                    mine[mt][half][e] = fmaf(k4[e], early, mine[mt][half][e]);
+                    diff[mt][half][e] = fmaf(k4[e], early - late, diff[mt][half][e]);
+                }
+                if (t < tokens) put4(a.scalar, static_cast<O*>(a.gk) + at_t, g4[0], g4[1], g4[2], g4[3]);
+            }
+    }
+    __syncthreads();               // m has been read
+    if (a.gv != nullptr) {
+        // gv: rows are k, columns r, values gy: the forward with exchanged roles.  Its edge planes take the room of the
+        // scaled rows' second parts where gv needs only the first, else that of v and one more set of planes.
+        __nv_bfloat16* e0 = kX > kP ? pf + kP * kPlane : vs;
+        __nv_bfloat16* e1 = kX > kP ? pf + (kX + kP) * kPlane : reinterpret_cast<__nv_bfloat16*>(seg + 8 * N);
+        pair_rows<T, kP, kRound>(kp + at0, rp + at0, a.u + h * N, tab, pf + dir * kX * kPlane, ms, dir ? e1 : e0, C, rows, blk, dir, lane);
+        __syncthreads();
+        float y[2][2][4];
+        pair_outputs<kZ, kP, true>(y, ms, gs, e0, e1, a_left, a_right, cs, th, lane);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int t = 32 * th + 16 * mt + 8 * half + g;
+                if (t < tokens)
+                    put4(a.scalar, static_cast<O*>(a.gv) + base + static_cast<size_t>(t) * C + 16 * cs + 4 * q, y[mt][0][2 * half],
+                         y[mt][0][2 * half + 1], y[mt][1][2 * half], y[mt][1][2 * half + 1]);
+            }
+        __syncthreads();
+    }
+    // gw: g_m = edge + sum_{t >= m} diff_t - mine_m
+    Table& dt = *reinterpret_cast<Table*>(pf);
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int t = 32 * th + 16 * mt + 8 * half + g;
+            put_row4(tab[t], cs, q, mine[mt][half][0], mine[mt][half][1], mine[mt][half][2], mine[mt][half][3]);
+            put_row4(dt[t], cs, q, diff[mt][half][0], diff[mt][half][1], diff[mt][half][2], diff[mt][half][3]);
+        }
+    __syncthreads();
+    {
+        const int t0 = warp * 8;                       // eight tokens per warp, lane = two channels
+        float2 d[8];
+        float2 run = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int t = 7; t >= 0; --t) {
+            const float2 x = *reinterpret_cast<const float2*>(&dt[t0 + t][2 * lane]);
+            const float2 m = *reinterpret_cast<const float2*>(&tab[t0 + t][2 * lane]);
+            run.x += x.x;
+            run.y += x.y;
+            d[t] = make_float2(run.x - m.x, run.y - m.y);
+        }
+        *reinterpret_cast<float2*>(seg + warp * N + 2 * lane) = run;
+        __syncthreads();
+        float2 later = make_float2(edge[2 * lane] + edge[N + 2 * lane], edge[2 * lane + 1] + edge[N + 2 * lane + 1]);
+        for (int j = warp + 1; j < 8; ++j) {
+            const float2 s = *reinterpret_cast<const float2*>(seg + j * N + 2 * lane);
+            later.x += s.x;
+            later.y += s.y;
+        }
+        const size_t o0 = base + static_cast<size_t>(t0) * C + 2 * lane;
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+            if (t0 + t < tokens) {
+                const size_t o = o0 + static_cast<size_t>(t) * C;
+                const float2 w = __ldg(reinterpret_cast<const float2*>(a.w + o));
+                const float gx = (later.x + d[t].x) * (kX > 2 ? -expf(w.x) : -ex2(w.x * kLog2e));
+                const float gz = (later.y + d[t].y) * (kX > 2 ? -expf(w.y) : -ex2(w.y * kLog2e));
+                if (!a.scalar) *reinterpret_cast<float2*>(a.gw + o) = make_float2(gx, gz);
+                else { a.gw[o] = gx; a.gw[o + 1] = gz; }
+            }
+        if (threadIdx.x < N)
+            a.gu_part[(static_cast<size_t>(b) * a.n_chunks + n) * C + h * N + threadIdx.x] = gus[threadIdx.x] + gus[N + threadIdx.x];
+    }
+}
+
+// gu[c] = sum over batch and chunks of the parts, in a fixed order
+__global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, const float* __restrict__ part, float* __restrict__ gu) {
+    __shared__ float red[32][33];
+    const int c = blockIdx.x * 32 + threadIdx.x;
+    float acc = 0.f;
+    for (int i = threadIdx.y; i < parts; i += 32) acc += part[static_cast<size_t>(i) * C + c];
+    red[threadIdx.y][threadIdx.x] = acc;
+    __syncthreads();
+    if (threadIdx.y == 0) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) t += red[i][threadIdx.x];
+        gu[c] = t;
+    }
+}
+
+// ---- host side -------------------------------------------------------------------------------------------------
+static size_t forward_smem(int kz, int kx) { return static_cast<size_t>(kz + 5 * kx) * kPlane * 2 + sizeof(Table); }
+static size_t backward_smem(int kz, int kx, int kp) {
+    return static_cast<size_t>(2 * kz + 3 * kx + (kx > kp ? 0 : kp)) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 8) * N * sizeof(float);
+}
+
+static int chunks_of(int T) { return (T + kChunk - 1) / kChunk; }
+static size_t state_plane(int B, int T, int H, int parts) {      // uint4 per (pair, direction)
+    return static_cast<size_t>(B) * H * chunks_of(T) * parts * (kStateWords / 4);
+}
+size_t forward_workspace(int B, int T, int H, bool exact) { return 256 + 2 * state_plane(B, T, H, exact ? 3 : 1) * sizeof(uint4); }
+size_t backward_workspace(int B, int T, int H, bool exact) {
+    return 256 + 4 * state_plane(B, T, H, exact ? 3 : 2) * sizeof(uint4) + static_cast<size_t>(B) * chunks_of(T) * H * N * sizeof(float);
+}
+
+// dynamic shared memory above 48 KB is a per-device attribute of each kernel: set the first time the kernel meets the device
+static bool allow_smem(const void* kernel, size_t bytes) {
+    static std::mutex lock;
+    static std::set<std::pair<int, const void*>> done;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> guard(lock);
+    if (done.count({dev, kernel})) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) != cudaSuccess) return false;
+    done.insert({dev, kernel});
+    return true;
+}
+static bool unaligned16(std::initializer_list<const void*> ps) {
+    for (const void* p : ps)
+        if (reinterpret_cast<uintptr_t>(p) & 15u) return true;
+    return false;
+}
+
+// launches the first kernel; gy: null for the forward
+template <typename T, typename G, int kZ, int kX, bool kRows>
+static bool run_states(int B, int T_, int H, const void* r, const void* k, const void* v, const float* w, const void* gy, uint4* states,
+                       size_t plane, void* workspace, cudaStream_t stream) {
+    constexpr int kPairs = kRows ? 2 : 1;
+    typedef StateSmem<T, T, G, kZ, kX, kPairs> S;
+    tensor_map::bind_primary_context();   // the tensor-map encoder is a driver call
+    const int C = H * N;
+    const auto map = [&](CUtensorMap* m, const void* p, bool half) { return tensor_map::make_btc(m, p, B, T_, C, N, kChunk, half); };
+    CUtensorMap mw, mk, mv, mr, mg;
+    if (!(map(&mw, w, false) && map(&mk, k, sizeof(T) == 2) && map(&mv, v, sizeof(T) == 2))) return false;
+    if (kPairs > 1) {
+        if (!(map(&mr, r, sizeof(T) == 2) && map(&mg, gy, sizeof(G) == 2))) return false;
+    } else {
+        mr = mk;
+        mg = mv;
+    }
+    const StateArgs a{T_, H, chunks_of(T_), states, plane, static_cast<unsigned*>(workspace), failure_mirror()};
+    const auto kernel = wkv6_state_kernel<T, T, G, kZ, kX, kRows, kPairs>;
+    if (!allow_smem(reinterpret_cast<const void*>(kernel), S::bytes)) return false;
+    kernel<<<dim3(B * H, 2), 128 * kPairs, S::bytes, stream>>>(a, mw, mk, mv, mr, mg);
+    return true;
+}
+
+template <typename T, int kZ, int kX>
+static int run_forward(int B, int T_, int H, const void* r, const void* k, const void* v, const float* w, const float* u, float* y,
+                       void* workspace, cudaStream_t stream) {
+    uint4* states = reinterpret_cast<uint4*>(static_cast<char*>(workspace) + 256);
+    const size_t plane = state_plane(B, T_, H, kX);
+    const int n_chunks = chunks_of(T_);
+    int launched = 1;
+    if (n_chunks > 1) {
+        if (!run_states<T, T, kZ, kX, false>(B, T_, H, nullptr, k, v, w, nullptr, states, plane, workspace, stream)) return -1;
+        ++launched;
+    }
+    OutArgs o{T_, H, n_chunks, r, k, v, w, u, y, unaligned16({y}), states, plane};
+    const auto kernel = wkv6_forward_kernel<T, kZ, kX>;
+    if (!allow_smem(reinterpret_cast<const void*>(kernel), forward_smem(kZ, kX))) return -1;
+    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, forward_smem(kZ, kX), stream>>>(o);
+    return launched;
+}
+
+template <typename T, typename G, typename O, int kZ, int kX, int kP>
+static int run_backward(int B, int T_, int H, const void* r, const void* k, const void* v, const float* w, const float* u, const void* gy,
+                        void* gr, void* gk, void* gv, float* gw, float* gu, void* workspace, cudaStream_t stream) {
+    uint4* states = reinterpret_cast<uint4*>(static_cast<char*>(workspace) + 256);
+    const size_t plane = state_plane(B, T_, H, kX);
+    const int n_chunks = chunks_of(T_), C = H * N;
+    int launched = 2;
+    if (n_chunks > 1) {
+        if (!run_states<T, G, kZ, kX, true>(B, T_, H, r, k, v, w, gy, states, plane, workspace, stream)) return -1;
+        ++launched;
+    }
+    float* gu_part = reinterpret_cast<float*>(states + 4 * plane);
+    GradArgs o{T_, H, n_chunks, r, k, v, gy, w, u, gr, gk, gv, gw, gu_part, unaligned16({gr, gk, gv, gw}), states, plane};
+    const auto kernel = wkv6_backward_kernel<T, G, O, kZ, kX, kP>;
+    if (!allow_smem(reinterpret_cast<const void*>(kernel), backward_smem(kZ, kX, kP))) return -1;
+    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, backward_smem(kZ, kX, kP), stream>>>(o);
+    wkv6_bonus_kernel<<<C / 32, dim3(32, 32), 0, stream>>>(B * n_chunks, C, gu_part, gu);
+    return launched;
+}
+
+int forward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, float* y, bool bf16_in,
+            bool exact, void* workspace, cudaStream_t stream) {
+    if (exact) return run_forward<float, 3, 3>(B, T, H, r, k, v, w, u, y, workspace, stream);
+    return bf16_in ? run_forward<__nv_bfloat16, 1, 1>(B, T, H, r, k, v, w, u, y, workspace, stream)
+                   : run_forward<float, 1, 1>(B, T, H, r, k, v, w, u, y, workspace, stream);
+}
+
+int backward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, const void* gy, void* gr,
+             void* gk, void* gv, float* gw, float* gu, bool bf16_in, bool gy_bf16, bool bf16_out, bool exact, void* workspace,
+             cudaStream_t stream) {
+    typedef __nv_bfloat16 H16;
+#define RUN(T_, G_, O_, Z_, X_, P_) run_backward<T_, G_, O_, Z_, X_, P_>(B, T, H, r, k, v, w, u, gy, gr, gk, gv, gw, gu, workspace, stream)
+    if (exact) return RUN(float, float, float, 3, 3, 3);
+    if (!bf16_in) return RUN(float, float, float, 1, 2, 1);
+    if (gy_bf16) return bf16_out ? RUN(H16, H16, H16, 1, 2, 1) : RUN(H16, H16, float, 1, 2, 1);
+    return bf16_out ? RUN(H16, float, H16, 1, 2, 1) : RUN(H16, float, float, 1, 2, 1);
+#undef RUN
+}
+
+}  // namespace wkv6c

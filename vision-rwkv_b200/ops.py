@@ -243,7 +243,7 @@ def _wkv6_shapes(r, k, v, w, u, H, gy=None):
 
 def wkv6_forward(r, k, v, w, u, H, tensor_cores=False):
     """y (float32) of the bidirectional WKV6; w is the raw decay input (decay = exp(-exp(w))).
-    tensor_cores=True runs the tcgen05 kernel (bf16 operand rounding, about 1e-2 accuracy); it also
+    tensor_cores=True rounds the matrix operands to bfloat16 (about 1e-2 accuracy); it also
     accepts r, k, v in bfloat16 (w, u float32) and then reads them without a widening pass."""
     half_in = tensor_cores and _is_bf16(r) and _is_bf16(k) and _is_bf16(v)
     if half_in:
@@ -259,32 +259,24 @@ def wkv6_forward(r, k, v, w, u, H, tensor_cores=False):
     y = torch.empty((B, T, C), device=dev, dtype=torch.float32)
     if y.numel() == 0:
         return y
-    if tensor_cores:
-        name = "vrwkv_wkv6_forward_tc_bf16" if half_in else "vrwkv_wkv6_forward_tc_f32"
-        with torch.cuda.device(dev):
-            ws = _workspace(256, dev)
-            st = getattr(lib, name)(B, T, C, H, r.data_ptr(), k.data_ptr(), v.data_ptr(), w.data_ptr(), u.data_ptr(),
-                                    y.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
-            _lib.check(st, name)
-            _check_status(lib, ws, name)
-        return y
     with torch.cuda.device(dev):
-        st = lib.vrwkv_wkv6_forward_f32(B, T, C, H, r.data_ptr(), k.data_ptr(), v.data_ptr(),
-                                        w.data_ptr(), u.data_ptr(), y.data_ptr(),
-                                        torch.cuda.current_stream().cuda_stream)
-    _lib.check(st, "vrwkv_wkv6_forward_f32")
+        exact = 0 if tensor_cores else 1
+        ws = _workspace(lib.vrwkv_wkv6_forward_workspace_bytes(B, T, C, H, exact), dev)
+        st = lib.vrwkv_wkv6_forward(B, T, C, H, r.data_ptr(), k.data_ptr(), v.data_ptr(), int(half_in), exact, w.data_ptr(), u.data_ptr(),
+                                    y.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+        _lib.check(st, "vrwkv_wkv6_forward")
+        _check_status(lib, ws, "vrwkv_wkv6_forward")
     return y
 
 
 def wkv6_backward(r, k, v, w, u, gy, H, tensor_cores=False, _skip_gv=False):
     """(gr, gk, gv, gw, gu), float32; gw w.r.t. the raw decay input, gu of shape (H, 64).
-    tensor_cores=True runs everything on the tcgen05 kernels: gv with bf16 operand rounding (about 4e-3 of
-    its maximum); gr, gk, and gw (a difference of long running sums of those) from a kernel that carries
-    its derived operands as hi + lo bfloat16 pairs, accurate to about 1e-4 when r, k, v, gy are bfloat16
-    values.  tensor_cores="gv" takes only gv from the tensor cores and the rest from the exact float32
-    sweeps.  Both accept r, k, v, gy in bfloat16 (w, u float32) and read them without a widening pass."""
+    tensor_cores=True takes r, k, v, gy as bfloat16 operands: gv with every operand rounded to bfloat16 (about 4e-3
+    of its maximum); gr, gk and gw with scaled operands carried as hi + lo bfloat16 pairs, accurate to about 1e-4
+    when r, k, v, gy are bfloat16 values.  tensor_cores="gv" takes only gv that way and the rest at float32
+    accuracy.  Both accept r, k, v, gy in bfloat16 (w, u float32) and read them without a widening pass."""
     if tensor_cores == "gv":
-        # gv = forward(k, r, gy) on the tensor cores (bfloat16 read as it is); gr, gk, gw, gu from the exact sweeps
+        # gv = forward(k, r, gy) (bfloat16 read as it is); gr, gk, gw, gu at float32 accuracy
         gv = wkv6_forward(k, r, gy, w, u, H, tensor_cores=True)
         gr, gk, _, gw, gu = wkv6_backward(r.float(), k.float(), v.float(), w, u, gy.float(), H, _skip_gv=True)
         return gr, gk, gv, gw, gu

@@ -8,12 +8,10 @@ the raw `w` and `gu` of shape (H, C // H) (:69-70).  Dropped: `T_MAX = 256`, a l
 reference's backward kernels only.  The reference's extension reads every tensor as float32;
 here half / bfloat16 inputs are accepted too and cast up for the kernel.
 
-Two forward kernels sit behind this surface: exact fp32 state sweeps, and a tcgen05 kernel that
-keeps the state in tensor memory and rounds its matrix operands to bfloat16 (about 1e-2 of
-max|y|, 2-3x faster).  `FORWARD_PATH` picks: "auto" (default) takes the tensor-core kernel when
-r, k and v arrive in half / bfloat16 - their own rounding is already of that size - and the exact
-sweeps for float32 callers; "exact" and "tensor_cores" force one.  The backward always
-recomputes from the saved inputs in fp32 and does not depend on the choice.
+Two precisions sit behind this surface: float32, and bfloat16 matrix operands with float32 sums (about 1e-2 of
+max|y|, several times faster).  `FORWARD_PATH` picks: "auto" (default) takes bfloat16 operands when
+r, k and v arrive in half / bfloat16 - their own rounding is already of that size - and float32
+accuracy for float32 callers; "exact" and "tensor_cores" force one.
 """
 from __future__ import annotations
 
@@ -27,8 +25,8 @@ HEAD_SIZE = 64
 FORWARD_PATH = os.environ.get("VRWKV6_FORWARD_PATH", "auto")
 
 
-BACKWARD_TC = "full"    # half-precision callers: "full" = every gradient from the tcgen05 kernels (bfloat16 read as it is;
-                        # measured faster than widening + exact sweeps); "gv" = only the value gradient there, rest exact
+BACKWARD_TC = "full"    # half-precision callers: "full" = every gradient from bfloat16 operands (read as they are);
+                        # "gv" = only the value gradient that way, the rest at float32 accuracy
 
 
 def _use_tensor_cores(r, k, v):
@@ -71,8 +69,6 @@ class WKV_6(torch.autograd.Function):
             assert gy.is_contiguous()
             r, k, v, w, u = ctx.saved_tensors
             if _use_tensor_cores(r, k, v):
-                # half-precision callers: the tcgen05 kernels, bfloat16 read as it is (BACKWARD_TC = "gv" keeps the
-                # decay-carrying gradients on the exact sweeps)
                 if all(x.dtype == torch.bfloat16 for x in (r, k, v)):
                     gr, gk, gv, gw, gu = ops.wkv6_backward(r, k, v, _f32(w), _f32(u), gy.bfloat16().contiguous(), ctx.H,
                                                            tensor_cores=True if BACKWARD_TC == "full" else "gv")
@@ -100,3 +96,13 @@ def RUN_CUDA_RWKV6(B, T, C, H, r, k, v, w, u):
     if tensor_cores and r.dtype == k.dtype == v.dtype == torch.bfloat16:       # read as they are, no widening pass
         return ops.wkv6_forward(r, k, v, _f32(w), _f32(u), H, tensor_cores=True)
     return ops.wkv6_forward(_f32(r), _f32(k), _f32(v), _f32(w), _f32(u), H, tensor_cores=tensor_cores)
+
+
+def inference_rwkv6(B, T, C, H, r, k, v, w, u):
+    """The recurrence inside `backbone6` networks: `RUN_CUDA_RWKV6`, except that inference on bfloat16 r, k, v keeps the
+    kernel that walks 16-token blocks.  In these networks a change of a single rounding anywhere ends up, twelve blocks
+    on, as a relative change of about 0.02 to 0.03 of the result (measured with kernels that agree to 1e-6), so a
+    network that is only being run keeps the bits it had."""
+    if not torch.is_grad_enabled() and FORWARD_PATH == "auto" and r.dtype == k.dtype == v.dtype == torch.bfloat16 and not ops.CHECK_STATUS:
+        return _lib.native().wkv6_walk(r, k, v, w, u)
+    return RUN_CUDA_RWKV6(B, T, C, H, r, k, v, w, u)
