@@ -780,9 +780,13 @@ __device__ __noinline__ void exact_subchunk(const Ctx& c, int sub, int ch, float
 // kStash: tokens whose leftward state a thread keeps in registers at a time (16: one reverse sweep
 // per sub-chunk; 8: the second half is swept twice, for half the registers).
 // kHalf: k, v, gy and the outputs are bfloat16 tensors (float32 arithmetic and shared-memory state all the same).
+// kWide (with kHalf): y and gy are float32 tensors, what a model with float32 w, u under autocast has; y still holds
+// bfloat16 values, gy is not rounded.  Without it the caller widens y (6 bytes per element) and narrows gy (6 more) in
+// passes of their own, as many bytes as this kernel's own forward moves.  B=64, T=576, C=1024, forward + backward:
+// 468 us with those passes, 332 us without (forward alone at B=256, T=196, C=384: 103 and 53 us).
 // kMulti: several clusters per sequence (T above what one cluster holds); compiled apart so that the
 // single-cluster kernels carry none of it.
-template <bool kBwd, int kStash, bool kHalf, bool kMulti>
+template <bool kBwd, int kStash, bool kHalf, bool kWide, bool kMulti>
 __global__ void __launch_bounds__(kMaxThreads, kBwd ? 2 : 3)
 biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                       const __grid_constant__ CUtensorMap map_g,     // backward: gy
@@ -790,6 +794,8 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                       const __grid_constant__ CUtensorMap map_o1,    // backward: gv
                       const Params p) {
     using RW = Rows<kBwd>;
+    constexpr bool kHalfG = kHalf && !kWide;                    // gy arrives as bfloat16
+    constexpr bool kHalfOut = kHalf && (kBwd || !kWide);        // results leave as bfloat16
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pr = lane & 15, upper = lane >> 4;
@@ -850,22 +856,22 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         if (kHalf) {
             // bfloat16: one box per 16-token sub-chunk, into the upper half of the sub-chunk's own area
             sm100::mbar_expect_tx(full + warp, 4 * kHalfAreaBytes);
-            if (kBwd) sm100::mbar_expect_tx(gfull + warp, 2 * kHalfAreaBytes);
+            if (kBwd && kHalfG) sm100::mbar_expect_tx(gfull + warp, 2 * kHalfAreaBytes);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int r = warp * kSpan + h * kL;
                 sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_k + r * kCs) + kHalfAreaBytes, &map_k, full + warp, strip * kCs, tok0 + r, b);
                 sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_v + r * kCs) + kHalfAreaBytes, &map_v, full + warp, strip * kCs, tok0 + r, b);
-                if (kBwd) sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_g + r * kCs) + kHalfAreaBytes, &map_g, gfull + warp, strip * kCs, tok0 + r, b);
+                if (kBwd && kHalfG) sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_g + r * kCs) + kHalfAreaBytes, &map_g, gfull + warp, strip * kCs, tok0 + r, b);
             }
         } else {
             sm100::mbar_expect_tx(full + warp, 2 * kSpanBytes);
             sm100::tma_load_3d(slot_k + warp * kSpan * kCs, &map_k, full + warp, strip * kCs, tok0 + warp * kSpan, b);
             sm100::tma_load_3d(slot_v + warp * kSpan * kCs, &map_v, full + warp, strip * kCs, tok0 + warp * kSpan, b);
-            if (kBwd) {
-                sm100::mbar_expect_tx(gfull + warp, kSpanBytes);
-                sm100::tma_load_3d(slot_g + warp * kSpan * kCs, &map_g, gfull + warp, strip * kCs, tok0 + warp * kSpan, b);
-            }
+        }
+        if (kBwd && !kHalfG) {
+            sm100::mbar_expect_tx(gfull + warp, kSpanBytes);
+            sm100::tma_load_3d(slot_g + warp * kSpan * kCs, &map_g, gfull + warp, strip * kCs, tok0 + warp * kSpan, b);
         }
     }
     if (threadIdx.x == 0) {
@@ -1012,7 +1018,8 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                     const float2 zx = zxs[j], zy = zys[j];
                     const float2 nn = fma2(c2, zx, add2(P.n, sn[g + j]));
                     const float2 dd = fma2(c2, zy, add2(P.d, sd[g + j]));
-                    st_out<kHalf>(area_k, i, pr, mul2(nn, f2(rcp(dd.x), rcp(dd.y))));
+                    const float2 y = mul2(nn, f2(rcp(dd.x), rcp(dd.y)));
+                    st_out<kHalfOut>(area_k, i, pr, kHalf && kWide ? __bfloat1622float2(__float22bfloat162_rn(y)) : y);
                     P.n = fma2(lam2, P.n, zx);
                     P.d = fma2(lam2, P.d, zy);
                 }
@@ -1047,7 +1054,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 #pragma unroll
                     for (int j = 0; j < kGroupB; ++j) {
                         const int i = blk * kStash + g + j;
-                        zxs[j] = k2[i * kRow]; zys[j] = v2[i * kRow]; gys[j] = ld_in<kHalf>(area_g, i, pr);
+                        zxs[j] = k2[i * kRow]; zys[j] = v2[i * kRow]; gys[j] = ld_in<kHalfG>(area_g, i, pr);
                     }
                     if (kHalf) __syncwarp();
 #pragma unroll
@@ -1145,7 +1152,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     }
     sm100::fence_proxy_async_smem();
     __syncthreads();
-    if (kHalf) {
+    if (kHalfOut) {
         // one box per sub-chunk (its 16 dense bfloat16 rows), issued by the warp that wrote them
         if (lane == 0) {
 #pragma unroll
@@ -1171,7 +1178,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         }
     }
     TL_MARK(8);
-    if (kHalf ? lane == 0 : threadIdx.x == 0) sm100::tma_store_wait_read();   // shared memory may go once the stores have read it
+    if (kHalfOut ? lane == 0 : threadIdx.x == 0) sm100::tma_store_wait_read();   // shared memory may go once the stores have read it
     TL_MARK(9);
 }
 
@@ -1179,12 +1186,14 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 // Runs after the fast kernel with a small persistent grid of clusters and serves the units it left
 // behind (normally none: one load and out).  Same shared-memory layout, same tiles, same work split
 // between the CTAs of a cluster, per-token max-shifted arithmetic.
-template <bool kBwd, bool kHalf>
+template <bool kBwd, bool kHalf, bool kWide>
 __global__ void __launch_bounds__(kMaxThreads, 1)
 biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                    const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_o0,
                    const __grid_constant__ CUtensorMap map_o1, const Params p) {
     using RW = Rows<kBwd>;
+    constexpr bool kHalfG = kHalf && !kWide;                    // as in biwkv_resident_kernel
+    constexpr bool kHalfOut = kHalf && (kBwd || !kWide);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pr = lane & 15, upper = lane >> 4;
@@ -1230,20 +1239,22 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         const int unit = p.redo_list[j];
         const int b = unit / p.n_strips, strip = unit - b * p.n_strips;
         if (threadIdx.x == 0) {
-            sm100::mbar_expect_tx(full, RW::kSlots * (kHalf ? slot_bytes / 2 : slot_bytes));
+            sm100::mbar_expect_tx(full, 2 * (kHalf ? slot_bytes / 2 : slot_bytes) + (kBwd ? (kHalfG ? slot_bytes / 2 : slot_bytes) : 0));
             if (kHalf) {
                 for (int r = 0; r < nw * kSpan; r += kL) {   // one box per 16-token sub-chunk, into the upper half of its area
                     sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_k + r * kCs) + kHalfAreaBytes, &map_k, full, strip * kCs, tok0 + r, b);
                     sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_v + r * kCs) + kHalfAreaBytes, &map_v, full, strip * kCs, tok0 + r, b);
-                    if (kBwd) sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_g + r * kCs) + kHalfAreaBytes, &map_g, full, strip * kCs, tok0 + r, b);
+                    if (kBwd && kHalfG) sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_g + r * kCs) + kHalfAreaBytes, &map_g, full, strip * kCs, tok0 + r, b);
                 }
             } else {
                 for (int sp = 0; sp < nw; ++sp) {            // the load maps describe one span per box
                     sm100::tma_load_3d(slot_k + sp * kSpan * kCs, &map_k, full, strip * kCs, tok0 + sp * kSpan, b);
                     sm100::tma_load_3d(slot_v + sp * kSpan * kCs, &map_v, full, strip * kCs, tok0 + sp * kSpan, b);
-                    if (kBwd) sm100::tma_load_3d(slot_g + sp * kSpan * kCs, &map_g, full, strip * kCs, tok0 + sp * kSpan, b);
                 }
             }
+            if (kBwd && !kHalfG)
+                for (int sp = 0; sp < nw; ++sp)
+                    sm100::tma_load_3d(slot_g + sp * kSpan * kCs, &map_g, full, strip * kCs, tok0 + sp * kSpan, b);
         }
         const int ch0 = strip * kCs + 2 * pr;
         const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
@@ -1254,11 +1265,11 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             // widen this thread's 16 rows in place, walking up (see ld_in)
             for (int i = 0; i < kL; ++i) {
                 const float2 a = ld_in<true>(slot_k + row0 * kCs, i, pr), bb = ld_in<true>(slot_v + row0 * kCs, i, pr);
-                const float2 g_ = kBwd ? ld_in<true>(slot_g + row0 * kCs, i, pr) : f2(0.f, 0.f);
+                const float2 g_ = kBwd && kHalfG ? ld_in<true>(slot_g + row0 * kCs, i, pr) : f2(0.f, 0.f);
                 __syncwarp();
                 *reinterpret_cast<float2*>(ks + i * kCs) = a;
                 *reinterpret_cast<float2*>(vs + i * kCs) = bb;
-                if (kBwd) *reinterpret_cast<float2*>(gs + i * kCs) = g_;
+                if (kBwd && kHalfG) *reinterpret_cast<float2*>(gs + i * kCs) = g_;
                 __syncwarp();
             }
         }
@@ -1270,7 +1281,12 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             *reinterpret_cast<float2*>(gs) = gw;
             *reinterpret_cast<float2*>(gs + kCs) = gu;
         }
-        if (kHalf) {
+        if (kHalf && kWide && !kBwd)
+            for (int i = 0; i < kL; ++i) {
+                float2* row = reinterpret_cast<float2*>(ks + i * kCs);
+                *row = __bfloat1622float2(__float22bfloat162_rn(*row));
+            }
+        if (kHalfOut) {
             // narrow the results in place, walking up: dense bfloat16 rows at the start of the area
             __syncwarp();
             for (int i = 0; i < kL; ++i) {
@@ -1284,7 +1300,7 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         }
         sm100::fence_proxy_async_smem();
         __syncthreads();
-        if (kHalf) {
+        if (kHalfOut) {
             if (lane == 0) {
                 for (int h = 0; h < 2; ++h) {
                     const int r = warp * kSpan + h * kL;
@@ -1307,7 +1323,7 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 p.partial[((static_cast<size_t>(unit) * p.cluster + c.rank) * 2 + jj) * kCs + lane] = acc;
             }
         }
-        if (kHalf ? lane == 0 : threadIdx.x == 0) sm100::tma_store_wait_read();
+        if (kHalfOut ? lane == 0 : threadIdx.x == 0) sm100::tma_store_wait_read();
         __syncthreads();      // the slots are free for the next unit
     }
 }
@@ -1377,22 +1393,25 @@ static bool make_plan(int T, Plan& pl) {
 
 struct DeviceState {
     bool probed = false, ok = false;
-    // [segments > 1][bfloat16][bwd][log2 cluster][n_warps]: 0 unknown, 1 launchable, -1 not
-    signed char fits[2][2][2][5][kMaxWarps + 1] = {};   // first index: several segments per sequence
+    // [segments > 1][tensor types][bwd][log2 cluster][n_warps]: 0 unknown, 1 launchable, -1 not
+    signed char fits[2][3][2][5][kMaxWarps + 1] = {};   // first index: several segments per sequence
 };
 static std::mutex g_mutex;
 static DeviceState g_dev[64];
 
-template <bool kBwd, bool kHalf, bool kMulti = false>
-static const void* kernel_ptr() {
-    return reinterpret_cast<const void*>(biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kHalf, kMulti>);
+// kWide kernels exist for sequences of one segment (the chunked kernels that stand by behind several have no such form)
+template <bool kBwd, Types kTypes, bool kMulti = false>
+static auto kernel() {
+    return biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kTypes != Types::f32, kTypes == Types::wide, kMulti && kTypes != Types::wide>;
 }
-template <bool kBwd, bool kHalf>
-static const void* exact_ptr() {
-    return reinterpret_cast<const void*>(biwkv_exact_kernel<kBwd, kHalf>);
+template <bool kBwd, Types kTypes>
+static auto exact_kernel() {
+    return biwkv_exact_kernel<kBwd, kTypes != Types::f32, kTypes == Types::wide>;
 }
+template <typename F>
+static const void* ptr(F* f) { return reinterpret_cast<const void*>(f); }
 
-template <bool kBwd, bool kHalf>
+template <bool kBwd, Types kTypes>
 static bool fits(const Plan& pl) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
@@ -1403,13 +1422,16 @@ static bool fits(const Plan& pl) {
         int cl = 0;
         cudaDeviceGetAttribute(&cl, cudaDevAttrClusterLaunch, dev);
         bool good = cl != 0 && tensor_map::encode_fn() != nullptr;
-        const void* fn[12] = {kernel_ptr<false, false>(), kernel_ptr<false, true>(), exact_ptr<false, false>(), exact_ptr<false, true>(),
-                              kernel_ptr<false, false, true>(), kernel_ptr<false, true, true>(),
-                              kernel_ptr<true, false>(),  kernel_ptr<true, true>(),  exact_ptr<true, false>(),  exact_ptr<true, true>(),
-                              kernel_ptr<true, false, true>(), kernel_ptr<true, true, true>()};
-        for (int i = 0; i < 12; ++i) {
+        constexpr Types kF = Types::f32, kH = Types::bf16, kW = Types::wide;
+        const void* fn[16] = {ptr(kernel<false, kF>()), ptr(kernel<false, kH>()), ptr(kernel<false, kW>()), ptr(kernel<false, kF, true>()),
+                              ptr(kernel<false, kH, true>()), ptr(exact_kernel<false, kF>()), ptr(exact_kernel<false, kH>()),
+                              ptr(exact_kernel<false, kW>()),
+                              ptr(kernel<true, kF>()), ptr(kernel<true, kH>()), ptr(kernel<true, kW>()), ptr(kernel<true, kF, true>()),
+                              ptr(kernel<true, kH, true>()), ptr(exact_kernel<true, kF>()), ptr(exact_kernel<true, kH>()),
+                              ptr(exact_kernel<true, kW>())};
+        for (int i = 0; i < 16; ++i) {
             good = good && cudaFuncSetAttribute(fn[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                static_cast<int>(i >= 6 ? smem_bytes<true>(kMaxWarps) : smem_bytes<false>(kMaxWarps))) == cudaSuccess;
+                                                static_cast<int>(i >= 8 ? smem_bytes<true>(kMaxWarps) : smem_bytes<false>(kMaxWarps))) == cudaSuccess;
             good = good && cudaFuncSetAttribute(fn[i], cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         }
         if (!good) cudaGetLastError();
@@ -1418,7 +1440,7 @@ static bool fits(const Plan& pl) {
     if (!d.ok) return false;
     int lg = 0;
     while ((1 << lg) < pl.cluster) ++lg;
-    signed char& slot = d.fits[pl.segs > 1 ? 1 : 0][kHalf ? 1 : 0][kBwd ? 1 : 0][lg][pl.n_warps];
+    signed char& slot = d.fits[pl.segs > 1 ? 1 : 0][static_cast<int>(kTypes)][kBwd ? 1 : 0][lg][pl.n_warps];
     if (slot == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(pl.cluster);
@@ -1429,23 +1451,24 @@ static bool fits(const Plan& pl) {
         at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
         int n = 0;
-        const cudaError_t err = cudaOccupancyMaxActiveClusters(&n, pl.segs > 1 ? kernel_ptr<kBwd, kHalf, true>() : kernel_ptr<kBwd, kHalf>(), &cfg);
+        const cudaError_t err = cudaOccupancyMaxActiveClusters(&n, pl.segs > 1 ? ptr(kernel<kBwd, kTypes, true>()) : ptr(kernel<kBwd, kTypes>()), &cfg);
         if (err != cudaSuccess) cudaGetLastError();
         slot = (err == cudaSuccess && n > 0) ? 1 : -1;
     }
     return slot > 0;
 }
 
-bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, bool bf16) {
-    if (C % (bf16 ? 8 : 4) != 0) return false;                     // TMA row pitch must be 16-byte
+bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types) {
+    if (C % (types != Types::f32 ? 8 : 4) != 0) return false;                     // TMA row pitch must be 16-byte
     for (const void* q : ptrs)
         if (reinterpret_cast<uintptr_t>(q) & 15u) return false;    // TMA base alignment
     Plan pl;
     if (!make_plan(T, pl)) return false;
     const long long ctas = static_cast<long long>(B) * ((C + kCs - 1) / kCs) * pl.cluster * pl.segs;
     if (ctas > (1LL << 30)) return false;
-    if (bf16) return bwd ? fits<true, true>(pl) : fits<false, true>(pl);
-    return bwd ? fits<true, false>(pl) : fits<false, false>(pl);
+    if (types == Types::wide) return pl.segs == 1 && (bwd ? fits<true, Types::wide>(pl) : fits<false, Types::wide>(pl));
+    if (types == Types::bf16) return bwd ? fits<true, Types::bf16>(pl) : fits<false, Types::bf16>(pl);
+    return bwd ? fits<true, Types::f32>(pl) : fits<false, Types::f32>(pl);
 }
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -1477,9 +1500,11 @@ bool multi_segment(int T) {
     return make_plan(T, pl) && pl.segs > 1;
 }
 
-template <bool kBwd, bool kHalf>
+template <bool kBwd, Types kTypes>
 static int launch(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy,
                   void* o0, void* o1, float* gwgu, void* workspace, cudaStream_t stream) {
+    constexpr bool kHalf = kTypes != Types::f32, kWide = kTypes == Types::wide;
+    constexpr bool kHalfOut = kHalf && (kBwd || !kWide), kHalfG = kHalf && !kWide;
     Plan pl;
     if (!make_plan(T, pl)) return -1;
     Params p{};
@@ -1503,11 +1528,11 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     tensor_map::bind_primary_context();   // the tensor-map encoder is a driver call
     CUtensorMap mk, mv, mg, m0, m1;
     // float32: loads one box per 32-token span, stores one box per CTA; bfloat16: one box per 16-token sub-chunk both ways
-    const int box_in = kHalf ? kL : kSpan, box_out = kHalf ? kL : pl.n_tok;
+    const int box_in = kHalf ? kL : kSpan, box_g = kHalfG ? kL : kSpan, box_out = kHalfOut ? kL : pl.n_tok;
     bool ok = tensor_map::make_btc(&mk, k, B, T, C, kCs, box_in, kHalf) && tensor_map::make_btc(&mv, v, B, T, C, kCs, box_in, kHalf) &&
-              tensor_map::make_btc(&m0, o0, B, T, C, kCs, box_out, kHalf);
-    ok = ok && tensor_map::make_btc(&mg, kBwd ? gy : k, B, T, C, kCs, box_in, kHalf) &&
-         tensor_map::make_btc(&m1, kBwd ? o1 : o0, B, T, C, kCs, box_out, kHalf);
+              tensor_map::make_btc(&m0, o0, B, T, C, kCs, box_out, kHalfOut);
+    ok = ok && (kBwd ? tensor_map::make_btc(&mg, gy, B, T, C, kCs, box_g, kHalfG) : tensor_map::make_btc(&mg, k, B, T, C, kCs, box_in, kHalf)) &&
+         tensor_map::make_btc(&m1, kBwd ? o1 : o0, B, T, C, kCs, box_out, kHalfOut);
     if (!ok) {
         set_error_detail("cuTensorMapEncodeTiled rejected a (C, T, B) tensor map");
         return -1;
@@ -1523,9 +1548,7 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    const cudaError_t err = pl.segs > 1
-        ? cudaLaunchKernelEx(&cfg, biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kHalf, true>, mk, mv, mg, m0, m1, p)
-        : cudaLaunchKernelEx(&cfg, biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kHalf, false>, mk, mv, mg, m0, m1, p);
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, pl.segs > 1 ? kernel<kBwd, kTypes, true>() : kernel<kBwd, kTypes>(), mk, mv, mg, m0, m1, p);
     if (err != cudaSuccess) {
         set_error_detail(cudaGetErrorName(err));
         return -1;
@@ -1534,7 +1557,7 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     if (pl.segs == 1) {
         // the exact kernel: a few clusters that serve whatever the fast kernel left behind
         cfg.gridDim = dim3(static_cast<unsigned>(std::min<size_t>(units, 16)) * pl.cluster);
-        const cudaError_t err2 = cudaLaunchKernelEx(&cfg, biwkv_exact_kernel<kBwd, kHalf>, mk, mv, mg, m0, m1, p);
+        const cudaError_t err2 = cudaLaunchKernelEx(&cfg, exact_kernel<kBwd, kTypes>(), mk, mv, mg, m0, m1, p);
         if (err2 != cudaSuccess) {
             set_error_detail(cudaGetErrorName(err2));
             return -1;
@@ -1548,24 +1571,16 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     return launched;
 }
 
-int forward(int B, int T, int C, const float* w, const float* u, const float* k, const float* v, float* y,
+int forward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, Types types,
             void* workspace, cudaStream_t stream) {
-    return launch<false, false>(B, T, C, w, u, k, v, nullptr, y, nullptr, nullptr, workspace, stream);
+    const auto fn = types == Types::f32 ? launch<false, Types::f32> : types == Types::bf16 ? launch<false, Types::bf16> : launch<false, Types::wide>;
+    return fn(B, T, C, w, u, k, v, nullptr, y, nullptr, nullptr, workspace, stream);
 }
 
-int backward(int B, int T, int C, const float* w, const float* u, const float* k, const float* v, const float* gy,
-             float* gwgu, float* gk, float* gv, void* workspace, cudaStream_t stream) {
-    return launch<true, false>(B, T, C, w, u, k, v, gy, gk, gv, gwgu, workspace, stream);
-}
-
-int forward_bf16(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y,
-                 void* workspace, cudaStream_t stream) {
-    return launch<false, true>(B, T, C, w, u, k, v, nullptr, y, nullptr, nullptr, workspace, stream);
-}
-
-int backward_bf16(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy,
-                  float* gwgu, void* gk, void* gv, void* workspace, cudaStream_t stream) {
-    return launch<true, true>(B, T, C, w, u, k, v, gy, gk, gv, gwgu, workspace, stream);
+int backward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, float* gwgu,
+             void* gk, void* gv, Types types, void* workspace, cudaStream_t stream) {
+    const auto fn = types == Types::f32 ? launch<true, Types::f32> : types == Types::bf16 ? launch<true, Types::bf16> : launch<true, Types::wide>;
+    return fn(B, T, C, w, u, k, v, gy, gk, gv, gwgu, workspace, stream);
 }
 
 }  // namespace resident

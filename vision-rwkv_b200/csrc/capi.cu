@@ -8,6 +8,8 @@
 #include "vrwkv_b200.h"
 #include "vrwkv_internal.h"
 
+using biwkv::resident::Types;
+
 namespace {
 std::atomic<unsigned long long> g_launches{0};
 std::atomic<int> g_path{0};   // 0 auto (resident, else fused, else generic), 1 generic only, 2 skip the resident path
@@ -150,9 +152,9 @@ int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u,
     if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool multi = biwkv::resident::multi_segment(T);
-    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, y}, false) &&
+    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, y}, false, Types::f32) &&
         (!multi || biwkv::fused::eligible(B, T, C, {k, v, y}))) {
-        int n = biwkv::resident::forward(B, T, C, w, u, k, v, y, workspace, s);
+        int n = biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::f32, workspace, s);
         if (n >= 0 && multi) {
             const int m = biwkv::fused::forward(B, T, C, w, u, k, v, y, static_cast<char*>(workspace) + resident_offset(B, T, C, false), s,
                                                 static_cast<const unsigned*>(workspace) + 1);
@@ -184,9 +186,9 @@ int vrwkv_biwkv_backward_f32(int B, int T, int C, const float* w, const float* u
     if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool multi = biwkv::resident::multi_segment(T);
-    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, gy, gk, gv}, true) &&
+    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, gy, gk, gv}, true, Types::f32) &&
         (!multi || biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}))) {
-        int n = biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, workspace, s);
+        int n = biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::f32, workspace, s);
         if (n >= 0 && multi) {
             const int m = biwkv::fused::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv,
                                                  static_cast<char*>(workspace) + resident_offset(B, T, C, true), s,
@@ -235,10 +237,10 @@ int vrwkv_biwkv_forward_bf16(int B, int T, int C, const float* w, const float* u
     if (misaligned4(w) || misaligned4(u) || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
     const bool multi = biwkv::resident::multi_segment(T);
-    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, y}, false, true) &&
+    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, y}, false, Types::bf16) &&
         (!multi || biwkv::fused::eligible(B, T, C, {k, v, y}, true))) {
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        int n = biwkv::resident::forward_bf16(B, T, C, w, u, k, v, y, workspace, s);
+        int n = biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::bf16, workspace, s);
         if (n >= 0 && multi) {
             const int m = biwkv::fused::forward_bf16(B, T, C, w, u, k, v, y, static_cast<char*>(workspace) + resident_offset(B, T, C, false), s,
                                                      static_cast<const unsigned*>(workspace) + 1);
@@ -259,10 +261,10 @@ int vrwkv_biwkv_backward_bf16(int B, int T, int C, const float* w, const float* 
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
     const bool multi = biwkv::resident::multi_segment(T);
-    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, gy, gk, gv}, true, true) &&
+    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, gy, gk, gv}, true, Types::bf16) &&
         (!multi || biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}, true))) {
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        int n = biwkv::resident::backward_bf16(B, T, C, w, u, k, v, gy, gwgu, gk, gv, workspace, s);
+        int n = biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::bf16, workspace, s);
         if (n >= 0 && multi) {
             const int m = biwkv::fused::backward_bf16(B, T, C, w, u, k, v, gy, gwgu, gk, gv,
                                                       static_cast<char*>(workspace) + resident_offset(B, T, C, true), s,
@@ -274,6 +276,28 @@ int vrwkv_biwkv_backward_bf16(int B, int T, int C, const float* w, const float* 
     if (!biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}, true)) return VRWKV_ERR_UNSUPPORTED;
     return finish(biwkv::fused::backward_bf16(B, T, C, w, u, k, v, gy, gwgu, gk, gv, workspace,
                                               static_cast<cudaStream_t>(stream)));
+}
+
+int vrwkv_biwkv_forward_bf16_wide(int B, int T, int C, const float* w, const float* u, const uint16_t* k, const uint16_t* v, float* y,
+                                  void* workspace, size_t workspace_bytes, void* stream) {
+    if (int st = check_shape(B, T, C)) return st;
+    if (!w || !u || !k || !v || !y || !workspace) return VRWKV_ERR_NULL;
+    if (misaligned4(w) || misaligned4(u) || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return VRWKV_ERR_ALIGNMENT;
+    if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    if (g_path.load() != 0 || !biwkv::resident::eligible(B, T, C, {k, v, y}, false, Types::wide)) return VRWKV_ERR_UNSUPPORTED;
+    return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::wide, workspace, static_cast<cudaStream_t>(stream)));
+}
+
+int vrwkv_biwkv_backward_bf16_wide(int B, int T, int C, const float* w, const float* u, const uint16_t* k, const uint16_t* v,
+                                   const float* gy, float* gwgu, uint16_t* gk, uint16_t* gv, void* workspace, size_t workspace_bytes,
+                                   void* stream) {
+    if (int st = check_shape(B, T, C)) return st;
+    if (!w || !u || !k || !v || !gy || !gwgu || !gk || !gv || !workspace) return VRWKV_ERR_NULL;
+    if (misaligned4(w) || misaligned4(u) || misaligned4(gwgu) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
+        return VRWKV_ERR_ALIGNMENT;
+    if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    if (g_path.load() != 0 || !biwkv::resident::eligible(B, T, C, {k, v, gy, gk, gv}, true, Types::wide)) return VRWKV_ERR_UNSUPPORTED;
+    return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::wide, workspace, static_cast<cudaStream_t>(stream)));
 }
 
 // ---- WKV6 ---------------------------------------------------------------------------------------

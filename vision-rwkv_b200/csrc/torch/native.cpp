@@ -81,14 +81,34 @@ Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, cons
     return y;
 }
 
+// k, v bfloat16, contiguous; y float32 holding bfloat16 values.  Undefined where the kernel does not cover the call.
+Tensor biwkv_forward_wide(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+    const int B = k.size(0), T = k.size(1), C = k.size(2);
+    Tensor y = at::empty_like(k, k.options().dtype(at::kFloat));
+    if (k.numel() == 0) return y;
+    Tensor ws = workspace(vrwkv_biwkv_forward_workspace_bytes(B, T, C), k);
+    const int st = vrwkv_biwkv_forward_bf16_wide(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
+                                                 static_cast<uint16_t*>(v.data_ptr()), fp(y), ws.data_ptr(), ws.numel(), stream_of(k));
+    if (st == VRWKV_ERR_UNSUPPORTED) return Tensor();
+    check(st, "vrwkv_biwkv_forward_bf16_wide");
+    raise_failures(k.get_device(), "vrwkv_biwkv_forward");
+    return y;
+}
+
 Tensor biwkv_forward(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, bool bf16_io) {
     const c10::cuda::CUDAGuard guard(k.device());
     const bool half = bf16_io && is_bf16(k) && is_bf16(v);
+    if (half && result_dtype(w) == at::kFloat) {
+        // float32 w, u under autocast: the kernel writes the widened result itself
+        const Tensor y = biwkv_forward_wide(f32(w), f32(u), k.contiguous(), v.contiguous());
+        if (y.defined()) return y;
+    }
     const Tensor y = half ? biwkv_forward_raw(f32(w), f32(u), k.contiguous(), v.contiguous())
                           : biwkv_forward_raw(f32(w), f32(u), f32(k), f32(v));
     return y.to(result_dtype(w));
 }
 
+// k, v float32, or bfloat16 (then gy in either type); all contiguous
 std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& gy) {
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor gk = at::empty_like(k), gv = at::empty_like(k);
@@ -98,7 +118,13 @@ std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const
         return {gwgu.select(0, 0), gwgu.select(0, 1), gk, gv};
     }
     Tensor ws = workspace(vrwkv_biwkv_backward_workspace_bytes(B, T, C), k);
-    if (is_bf16(k)) {
+    if (is_bf16(k) && !is_bf16(gy)) {
+        const int st = vrwkv_biwkv_backward_bf16_wide(
+            B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()), fp(gy), fp(gwgu),
+            static_cast<uint16_t*>(gk.data_ptr()), static_cast<uint16_t*>(gv.data_ptr()), ws.data_ptr(), ws.numel(), stream_of(k));
+        if (st == VRWKV_ERR_UNSUPPORTED) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16));
+        check(st, "vrwkv_biwkv_backward_bf16_wide");
+    } else if (is_bf16(k)) {
         const int st = vrwkv_biwkv_backward_bf16(
             B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()),
             static_cast<uint16_t*>(gy.data_ptr()), fp(gwgu), static_cast<uint16_t*>(gk.data_ptr()),
@@ -132,7 +158,7 @@ struct BiWkv : torch::autograd::Function<BiWkv> {
         const at::NoGradGuard no_grad;
         const at::ScalarType out = result_dtype(w);
         const bool half = ctx->saved_data["bf16_io"].toBool() && is_bf16(k) && is_bf16(v);
-        auto g = half ? biwkv_backward_raw(f32(w), f32(u), k.contiguous(), v.contiguous(), gy.to(at::kBFloat16).contiguous())
+        auto g = half ? biwkv_backward_raw(f32(w), f32(u), k.contiguous(), v.contiguous(), is_bf16(gy) ? gy.contiguous() : f32(gy))
                       : biwkv_backward_raw(f32(w), f32(u), f32(k), f32(v), f32(gy));
         // on the bfloat16 path gk, gv stay bfloat16 (what autograd hands to a bfloat16 k anyway) unless w is half
         if (!half || out == at::kHalf) { g[2] = g[2].to(out); g[3] = g[3].to(out); }

@@ -30,25 +30,25 @@ int generic_backward(int B, int T, int C, const float* w, const float* u, const 
                      const float* v, const float* gy, float* gwgu, float* gk, float* gv,
                      void* workspace, cudaStream_t stream);
 namespace resident {
-// Cluster-resident single-pass path (biwkv_resident.cu): float32 (C % 4 == 0) or bfloat16 (C % 8 == 0)
-// tensors, 16-byte aligned, T <= 4096.  True when it can serve this call on the current device.
-bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, bool bf16 = false);
+// Cluster-resident single-pass path (biwkv_resident.cu): C % 4 == 0 (f32) or C % 8 == 0 (the others), 16-byte aligned
+// tensors, T <= 32768 (wide: 4096).  w, u, gwgu are float32 always, arithmetic and shared-memory state too.
+enum class Types {
+    f32,      // every tensor float32
+    bf16,     // k, v, y, gy, gk, gv bfloat16
+    wide,     // k, v, gk, gv bfloat16; gy float32; y float32 holding bfloat16 values
+};
+// True when it can serve this call on the current device.
+bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types);
 void set_withhold_test(bool on);   // test only: one rank per cluster sends nothing, waits give up early
 size_t workspace_bytes(int B, int T, int C, bool bwd);
 // Sequences longer than one cluster holds (T > 4096) run as several clusters per sequence.  Inputs outside the
 // plain-float range then leave workspace word 1 non-zero instead of results: the caller follows up with the
 // chunked kernels switched on by that word.
 bool multi_segment(int T);
-int forward(int B, int T, int C, const float* w, const float* u, const float* k, const float* v,
-            float* y, void* workspace, cudaStream_t stream);
-int backward(int B, int T, int C, const float* w, const float* u, const float* k, const float* v,
-             const float* gy, float* gwgu, float* gk, float* gv, void* workspace,
-             cudaStream_t stream);
-// k, v, y, gy, gk, gv hold bfloat16; w, u, gwgu stay float; arithmetic and shared-memory state are the float kernels'.
-int forward_bf16(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y,
-                 void* workspace, cudaStream_t stream);
-int backward_bf16(int B, int T, int C, const float* w, const float* u, const void* k, const void* v,
-                  const void* gy, float* gwgu, void* gk, void* gv, void* workspace, cudaStream_t stream);
+int forward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, Types types,
+            void* workspace, cudaStream_t stream);
+int backward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, float* gwgu,
+             void* gk, void* gv, Types types, void* workspace, cudaStream_t stream);
 }  // namespace resident
 namespace fused {
 // True when the fused TMA path can serve this call on the current device.
