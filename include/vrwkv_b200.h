@@ -272,6 +272,11 @@ int vrwkv_qshift_multihead_mix_backward_f32(int B, int H, int W, int C, int head
                                             const float* const* gout, float* gx, float* const* gmix,
                                             void* workspace, size_t workspace_bytes, void* stream);
 
+/* Either forward with bfloat16 outputs, what the linear layers behind it round them to under autocast (head_dim 0:
+ * `group` as in vrwkv_qshift_mix_forward_f32, else the per-head form and `group` is ignored). */
+int vrwkv_qshift_mix_forward_bf16out(int B, int H, int W, int C, int group, int head_dim, int shift, int n_out, const float* x,
+                                     const float* const* mix, uint16_t* const* out, void* stream);
+
 /* The per-head shift fused with the data-dependent interpolations of the VRWKV6 spatial mix
  * (CLS/vrwkv6.py:75-100, 180-193):  out_j = x + (q_shift_multihead(x) - x) * (maa_j[c] + m_j[b,t,c]),
  * j < n_out <= 5.  maa: n_out device pointers to (C,) float vectors; m: n_out device pointers to
@@ -283,6 +288,10 @@ int vrwkv_qshift_multihead_mix_backward_f32(int B, int H, int W, int C, int head
 int vrwkv_qshift_ddlerp_forward_f32(int B, int H, int W, int C, int head_dim, int shift, int n_out, const float* x,
                                     const float* const* maa, const void* const* m, int m_is_bf16, float* const* out,
                                     void* stream);
+/* ... with bfloat16 outputs */
+int vrwkv_qshift_ddlerp_forward_bf16out(int B, int H, int W, int C, int head_dim, int shift, int n_out, const float* x,
+                                        const float* const* maa, const void* const* m, int m_is_bf16, uint16_t* const* out,
+                                        void* stream);
 size_t vrwkv_qshift_ddlerp_backward_workspace_bytes(int B, int H, int W, int C, int n_out);
 int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, int shift, int n_out, const float* x,
                                      const float* const* maa, const void* const* m, int m_is_bf16,

@@ -148,3 +148,56 @@ def test_data_dependent_mix_rejects_bad_head_size(cuda_device):
     x = torch.randn(1, 4, 72, device=cuda_device)
     with pytest.raises(RuntimeError, match="multiple of 16"):
         ops.qshift_ddlerp_forward(x, [torch.rand(72, device=cuda_device)], [None], (2, 2), 1, 24)
+
+
+# stretches of the walks (8 tokens at most): grids whose sides fill them, leave one token over, or are a single line;
+# unshifted channels behind the four groups; several walkers per block (narrow C) and several blocks per row (wide C)
+WALK_CASES = [(1, 8, 9, 64, 0.25, None), (2, 17, 7, 40, 0.2, None), (3, 1, 8, 16, 0.25, None), (2, 16, 1, 192, 0.25, None), (1, 33, 31, 192, 0.25, None),
+              (2, 9, 25, 128, None, 64), (70, 14, 14, 64, 0.25, None), (1, 10, 11, 1040, 0.25, None)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,W,C,gamma,head_dim", WALK_CASES)
+def test_walks_along_the_grid(cuda_device, B, H, W, C, gamma, head_dim):
+    from vision_rwkv_b200 import _lib, ops
+    from vision_rwkv_b200.qshift import qshift_mix
+    g = torch.Generator().manual_seed(H * 100 + W)
+    x, mixes = torch.randn(B, H * W, C, generator=g), [torch.rand(1, 1, C, generator=g) for _ in range(3)]
+    gouts = [torch.randn(B, H * W, C, generator=g) for _ in range(3)]
+    xr, mr = x.double().requires_grad_(True), [m.double().requires_grad_(True) for m in mixes]
+    xx = O.q_shift(xr, (H, W), 1, gamma) if head_dim is None else O.q_shift_multihead(xr, (H, W), 1, head_dim)
+    ref = [xr * m + xx * (1 - m) for m in mr]
+    torch.autograd.backward(ref, [go.double() for go in gouts])
+    xd, md = x.to(cuda_device).requires_grad_(True), [m.to(cuda_device).requires_grad_(True) for m in mixes]
+    outs = qshift_mix(xd, md, (H, W), 1, gamma or 0.25, head_dim)
+    torch.autograd.backward(outs, [go.to(cuda_device) for go in gouts])
+    for o, r in zip(outs, ref):
+        assert rel_err(o, r.detach()) < 1e-6
+    assert rel_err(xd.grad, xr.grad) < 1e-6
+    for a, b in zip(md, mr):
+        assert rel_err(a.grad, b.grad) < 1e-5
+    # bfloat16 outputs are the float32 ones rounded once, whichever kernel runs (shift 2 takes the token-by-token one)
+    group = ops.qshift_group(C, gamma or 0.25, head_dim)
+    for shift in (1, 2):
+        wide = qshift_mix(xd.detach(), [m.detach() for m in md], (H, W), shift, gamma or 0.25, head_dim)
+        half = _lib.native().qshift_mix_half(xd.detach(), [m.detach() for m in md], H, W, shift, group, head_dim is not None)
+        assert all(torch.equal(h, f.bfloat16()) for h, f in zip(half, wide))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,W,C,head_dim", [(2, 9, 7, 64, 64), (1, 8, 17, 192, 64), (3, 1, 5, 32, 16), (40, 14, 14, 128, 64)])
+@pytest.mark.parametrize("offsets", [torch.float32, torch.bfloat16, None])
+def test_data_dependent_walks(cuda_device, B, H, W, C, head_dim, offsets):
+    from vision_rwkv_b200 import _lib
+    from vision_rwkv_b200.qshift import qshift_ddlerp
+    g = torch.Generator().manual_seed(H * 100 + W)
+    x, maas = torch.randn(B, H * W, C, generator=g), [torch.rand(1, 1, C, generator=g) for _ in range(5)]
+    ms = [None if offsets is None or j == 2 else (torch.randn(B, H * W, C, generator=g) * 0.3).to(offsets) for j in range(5)]
+    xx = O.q_shift_multihead(x.double(), (H, W), 1, head_dim) - x.double()
+    ref = [x.double() + xx * (a.double() + (0 if m is None else m.double())) for a, m in zip(maas, ms)]
+    xd, ad, md = x.to(cuda_device), [a.to(cuda_device) for a in maas], [None if m is None else m.to(cuda_device) for m in ms]
+    outs = qshift_ddlerp(xd, ad, md, (H, W), 1, head_dim)
+    half = _lib.native().qshift_ddlerp_half(xd, ad, md, H, W, 1, head_dim)
+    for o, h, r in zip(outs, half, ref):
+        assert rel_err(o, r) < 1e-6
+        assert torch.equal(h, o.bfloat16())

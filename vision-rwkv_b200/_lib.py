@@ -32,6 +32,8 @@ SIGNATURES = {
     "vrwkv_biwkv_backward_saved_f32": (_c_int, [_c_int] * 3 + [_ptr] * 11 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_forward_bf16": (_c_int, [_c_int] * 3 + [_ptr] * 6 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_backward_bf16": (_c_int, [_c_int] * 3 + [_ptr] * 9 + [_c_size_t, _ptr]),
+    "vrwkv_qshift_mix_forward_bf16out": (_c_int, [_c_int] * 8 + [_ptr] * 4),
+    "vrwkv_qshift_ddlerp_forward_bf16out": (_c_int, [_c_int] * 7 + [_ptr] * 3 + [_c_int] + [_ptr] * 2),
     "vrwkv_biwkv_forward_bf16_wide": (_c_int, [_c_int] * 3 + [_ptr] * 6 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_backward_bf16_wide": (_c_int, [_c_int] * 3 + [_ptr] * 9 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_forward_f32_noalloc": (_c_int, [_c_int] * 3 + [_ptr] * 6),

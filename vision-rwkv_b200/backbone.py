@@ -21,7 +21,7 @@ import torch.nn.functional as F
 import torch.utils.checkpoint as cp
 
 from . import normgate
-from .qshift import qshift_mix
+from .qshift import qshift_mix_to
 from .vrwkv import RUN_CUDA
 
 
@@ -51,8 +51,9 @@ class SpatialMix(nn.Module):
     def forward(self, x, resolution):
         T = x.shape[1]
         if self.shift_pixel > 0:
-            xk, xv, xr = qshift_mix(x, (self.spatial_mix_k, self.spatial_mix_v, self.spatial_mix_r),
-                                    resolution, self.shift_pixel, self.channel_gamma)
+            xk, xv, xr = qshift_mix_to((self.key, self.value, self.receptance), x,
+                                       (self.spatial_mix_k, self.spatial_mix_v, self.spatial_mix_r),
+                                       resolution, self.shift_pixel, self.channel_gamma)
         else:
             xk = xv = xr = x
         k, v = self.key(xk), self.value(xv)
@@ -84,8 +85,8 @@ class ChannelMix(nn.Module):
 
     def forward(self, x, resolution):
         if self.shift_pixel > 0:
-            xk, xr = qshift_mix(x, (self.spatial_mix_k, self.spatial_mix_r), resolution,
-                                self.shift_pixel, self.channel_gamma)
+            xk, xr = qshift_mix_to((self.key, self.receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution,
+                                   self.shift_pixel, self.channel_gamma)
         else:
             xk = xr = x
         k = torch.square(torch.relu(self.key(xk)))

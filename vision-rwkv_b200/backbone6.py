@@ -22,7 +22,7 @@ import torch.utils.checkpoint as cp
 
 from .backbone import _PatchEmbed, _ramp
 from . import normgate
-from .qshift import qshift_ddlerp, qshift_mix
+from .qshift import qshift_ddlerp_to, qshift_mix_to
 from .vrwkv6 import HEAD_SIZE, inference_rwkv6
 
 MIX_RANK = 32       # width of the low-rank branch that produces the five mixing offsets
@@ -79,7 +79,8 @@ class SpatialMixV6(nn.Module):
         fused = x.is_cuda and C % HEAD_SIZE == 0 and self.shift_pixel > 0
         if fused:
             # the shift and every interpolation in two passes over x (qshift.qshift_ddlerp)
-            (xxx,) = qshift_ddlerp(x, [self.time_maa_x], [None], resolution, self.shift_pixel, HEAD_SIZE)
+            layers = (self.key, self.value, self.receptance, self.gate)
+            (xxx,) = qshift_ddlerp_to(layers, x, [self.time_maa_x], [None], resolution, self.shift_pixel, HEAD_SIZE)
         else:
             xx = q_shift_multihead(x, self.shift_pixel, resolution) - x
             xxx = x + xx * self.time_maa_x
@@ -87,8 +88,8 @@ class SpatialMixV6(nn.Module):
         low = torch.tanh(xxx @ self.time_maa_w1).view(B * T, 5, MIX_RANK).transpose(0, 1)
         mw, mk, mv, mr, mg = torch.bmm(low, self.time_maa_w2).view(5, B, T, C).unbind(0)
         if fused:
-            xw, xk, xv, xr, xg = qshift_ddlerp(
-                x, [self.time_maa_w, self.time_maa_k, self.time_maa_v, self.time_maa_r, self.time_maa_g],
+            xw, xk, xv, xr, xg = qshift_ddlerp_to(
+                layers, x, [self.time_maa_w, self.time_maa_k, self.time_maa_v, self.time_maa_r, self.time_maa_g],
                 [mw, mk, mv, mr, mg], resolution, self.shift_pixel, HEAD_SIZE)
         else:
             xw, xk, xv, xr, xg = (x + xx * (maa + m) for maa, m in (
@@ -124,8 +125,8 @@ class ChannelMixV6(nn.Module):
         self.value = nn.Linear(hidden, n_embd, bias=False)
 
     def forward(self, x, resolution):
-        xk, xr = qshift_mix(x, (self.spatial_mix_k, self.spatial_mix_r), resolution, self.shift_pixel,
-                            head_dim=HEAD_SIZE)          # per-head shift + both interpolations in one pass
+        xk, xr = qshift_mix_to((self.key, self.receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution, self.shift_pixel,
+                               head_dim=HEAD_SIZE)       # per-head shift + both interpolations in one pass
         k = torch.square(torch.relu(self.key(xk)))
         if self.key_norm is not None:
             k = self.key_norm(k)

@@ -16,6 +16,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "qshift_lines.cuh"
 #include "vrwkv_b200.h"
 #include "vrwkv_internal.h"
 
@@ -34,7 +35,7 @@ struct Args {
     const float* x;
     const float* maa[kMaxOut];   // (C,)
     const void* m[kMaxOut];      // (B, T, C) or null
-    float* out[kMaxOut];
+    float* out[kMaxOut];         // float32 or bfloat16
     const float* gout[kMaxOut];
     float* gx;
     void* gm[kMaxOut];           // null where m is null
@@ -90,7 +91,7 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(
 
 // thread = 4 consecutive channels (one quarter of a head never splits them: head_dim % 16 == 0); a block walks
 // kTokensPerBlock tokens
-template <bool kHalfM>
+template <bool kHalfM, typename Out>
 __global__ void __launch_bounds__(kThreads) ddlerp_forward(const Args a) {
     const int cv = (blockIdx.x * kThreads + threadIdx.x) * kVec;
     if (cv >= a.C) return;
@@ -118,8 +119,40 @@ __global__ void __launch_bounds__(kThreads) ddlerp_forward(const Args a) {
         for (int j = 0; j < kMaxOut; ++j)
             if (j < a.n_out) {
                 const float4 mu = add4(maa[j], load_m<kHalfM>(a.m[j], base));
-                *reinterpret_cast<float4*>(a.out[j] + base) =
-                    make_float4(fmaf(d4.x, mu.x, x4.x), fmaf(d4.y, mu.y, x4.y), fmaf(d4.z, mu.z, x4.z), fmaf(d4.w, mu.w, x4.w));
+                qlines::st4(reinterpret_cast<Out*>(a.out[j]) + base, qlines::fma4(d4, mu, x4));
+            }
+    }
+}
+
+// the same for a shift of one pixel, in walks along the lines of the grid (qshift_lines.cuh)
+template <bool kHalfM, typename Out>
+__global__ void __launch_bounds__(qlines::kMaxThreads, 2) ddlerp_lines_forward(const Args a, const qlines::Grid g) {
+    using namespace qlines;
+    const int cv = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    if (cv >= g.C) return;
+    const int which = group_of(g, cv);
+    const unsigned first = (blockIdx.x * blockDim.y + threadIdx.y) * static_cast<unsigned>(g.per_walker);
+    for (unsigned line = first; line < min(first + g.per_walker, g.lines); ++line) {
+        const Stretch s = stretch_at(g, line, which, cv);
+        float4 x[kStretch], d[kStretch], prev = zero4();
+        if (s.before) prev = ld4(a.x + s.base - s.step);
+#pragma unroll
+        for (int i = 0; i < kStretch; ++i) x[i] = i < s.n ? ld4(a.x + s.base + i * s.step) : zero4();
+#pragma unroll
+        for (int i = 0; i < kStretch; ++i) {
+            d[i] = sub4(prev, x[i]);
+            prev = x[i];
+        }
+#pragma unroll
+        for (int j = 0; j < kMaxOut; ++j)
+            if (j < a.n_out) {
+                const float4 maa = ld4(a.maa[j] + cv);
+                float4 mu[kStretch];
+#pragma unroll
+                for (int i = 0; i < kStretch; ++i) mu[i] = i < s.n ? load_m<kHalfM>(a.m[j], s.base + i * s.step) : zero4();
+#pragma unroll
+                for (int i = 0; i < kStretch; ++i)
+                    if (i < s.n) st4(reinterpret_cast<Out*>(a.out[j]) + s.base + i * s.step, fma4(d[i], add4(maa, mu[i]), x[i]));
             }
     }
 }
@@ -215,10 +248,20 @@ static bool misaligned(const void* p, uintptr_t a) { return (reinterpret_cast<ui
 
 }  // namespace ddlerp
 
-extern "C" int vrwkv_qshift_ddlerp_forward_f32(int B, int H, int W, int C, int head_dim, int shift, int n_out, const float* x,
-                                               const float* const* maa, const void* const* m, int m_is_bf16, float* const* out,
-                                               void* stream) {
-    using namespace ddlerp;
+namespace ddlerp {
+template <bool kHalfM, typename Out>
+static void launch_forward(const Args& a, cudaStream_t s) {
+    const qlines::Grid g = qlines::make_grid(a.B, a.H, a.W, a.C, a.head_dim / 4, a.head_dim);
+    if (a.shift == 1 && g.lines != 0) {       // any other shift: token by token
+        const qlines::Shape shape = qlines::make_shape(g);
+        ddlerp_lines_forward<kHalfM, Out><<<shape.grid, shape.block, 0, s>>>(a, g);
+    } else {
+        ddlerp_forward<kHalfM, Out><<<dim3((a.C / kVec + kThreads - 1) / kThreads, row_blocks(a.B, a.H, a.W)), kThreads, 0, s>>>(a);
+    }
+}
+
+static int forward_any(int B, int H, int W, int C, int head_dim, int shift, int n_out, const float* x, const float* const* maa,
+                       const void* const* m, int m_is_bf16, void* const* out, bool out_bf16, void* stream) {
     if (int st = check(B, H, W, C, head_dim, shift, n_out)) return st;
     if (!x || !maa || !m || !out) return VRWKV_ERR_NULL;
     Args a{};
@@ -227,13 +270,25 @@ extern "C" int vrwkv_qshift_ddlerp_forward_f32(int B, int H, int W, int C, int h
     for (int j = 0; j < n_out; ++j) {
         if (!maa[j] || !out[j]) return VRWKV_ERR_NULL;
         if (misaligned(maa[j], 16) || misaligned(out[j], 16) || (m[j] && misaligned(m[j], m_is_bf16 ? 8 : 16))) return VRWKV_ERR_ALIGNMENT;
-        a.maa[j] = maa[j]; a.m[j] = m[j]; a.out[j] = out[j];
+        a.maa[j] = maa[j]; a.m[j] = m[j]; a.out[j] = static_cast<float*>(out[j]);
     }
-    const dim3 grid((C / kVec + kThreads - 1) / kThreads, row_blocks(B, H, W));
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (m_is_bf16) ddlerp_forward<true><<<grid, kThreads, 0, s>>>(a);
-    else ddlerp_forward<false><<<grid, kThreads, 0, s>>>(a);
+    const auto launch = out_bf16 ? (m_is_bf16 ? launch_forward<true, __nv_bfloat16> : launch_forward<false, __nv_bfloat16>)
+                                 : (m_is_bf16 ? launch_forward<true, float> : launch_forward<false, float>);
+    launch(a, static_cast<cudaStream_t>(stream));
     return record_launches(1);
+}
+}  // namespace ddlerp
+
+extern "C" int vrwkv_qshift_ddlerp_forward_f32(int B, int H, int W, int C, int head_dim, int shift, int n_out, const float* x,
+                                               const float* const* maa, const void* const* m, int m_is_bf16, float* const* out,
+                                               void* stream) {
+    return ddlerp::forward_any(B, H, W, C, head_dim, shift, n_out, x, maa, m, m_is_bf16, reinterpret_cast<void* const*>(out), false, stream);
+}
+
+extern "C" int vrwkv_qshift_ddlerp_forward_bf16out(int B, int H, int W, int C, int head_dim, int shift, int n_out, const float* x,
+                                                   const float* const* maa, const void* const* m, int m_is_bf16, uint16_t* const* out,
+                                                   void* stream) {
+    return ddlerp::forward_any(B, H, W, C, head_dim, shift, n_out, x, maa, m, m_is_bf16, reinterpret_cast<void* const*>(out), true, stream);
 }
 
 extern "C" size_t vrwkv_qshift_ddlerp_backward_workspace_bytes(int B, int H, int W, int C, int n_out) {

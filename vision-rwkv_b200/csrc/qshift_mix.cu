@@ -13,6 +13,7 @@
 // fixed order.  Pure bandwidth work: 4 (1 + n) bytes per element forward, 4 (n + 2) backward.
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "qshift_lines.cuh"
 #include "vrwkv_internal.h"
 
 namespace qshift {
@@ -30,6 +31,7 @@ struct Args {
     const float* x;
     const float* mix[kMaxOut];     // (C,)
     float* out[kMaxOut];           // forward outputs (B, T, C)
+    bool out_bf16;                 // ... in bfloat16 (what an autocast linear layer behind them would round them to)
     const float* gout[kMaxOut];    // backward: output gradients
     float* gx;
     float* partial;                // backward: [blocks_y][n_out][C]
@@ -58,8 +60,9 @@ __device__ __forceinline__ int reader_token(const Args& a, int h, int w, int c) 
     return hd * a.W + wd;
 }
 
+// ---- any shift, any alignment: token by token ----------------------------------------------------
 // kVec: 4 channels per thread (needs C % 4 == 0, group % 4 == 0 and 16-byte aligned tensors)
-template <int kVec>
+template <int kVec, typename Out>
 __global__ void __launch_bounds__(kThreads) qshift_mix_forward(const Args a) {
     const int cv = (blockIdx.x * kThreads + threadIdx.x) * kVec;
     if (cv >= a.C) return;
@@ -96,8 +99,9 @@ __global__ void __launch_bounds__(kThreads) qshift_mix_forward(const Args a) {
                 float o[kVec];
 #pragma unroll
                 for (int j = 0; j < kVec; ++j) o[j] = fmaf(mixv[m][j], xv[j] - sv[j], sv[j]);
-                if (kVec == 4) *reinterpret_cast<float4*>(a.out[m] + base) = make_float4(o[0], o[1], o[2], o[3]);
-                else a.out[m][base] = o[0];
+                Out* const to = reinterpret_cast<Out*>(a.out[m]) + base;
+                if (kVec == 4) qlines::st4(to, make_float4(o[0], o[1], o[2], o[3]));
+                else *to = static_cast<Out>(o[0]);
             }
         }
     }
@@ -158,6 +162,90 @@ __global__ void __launch_bounds__(kThreads) qshift_mix_backward(const Args a) {
                 a.partial[(static_cast<size_t>(blockIdx.y) * a.n_out + m) * a.C + cv + j] = gmix[m][j];
 }
 
+// ---- a shift of one pixel: walks along the lines of the grid (qshift_lines.cuh) ----------------------
+template <typename Out>
+__global__ void __launch_bounds__(qlines::kMaxThreads) qshift_lines_forward(const Args a, const qlines::Grid g) {
+    using namespace qlines;
+    const int cv = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    if (cv >= g.C) return;
+    const int which = group_of(g, cv);
+    const unsigned first = (blockIdx.x * blockDim.y + threadIdx.y) * static_cast<unsigned>(g.per_walker);
+    float4 mix[kMaxOut];
+#pragma unroll
+    for (int m = 0; m < kMaxOut; ++m) mix[m] = m < a.n_out ? ld4(a.mix[m] + cv) : zero4();
+    for (unsigned line = first; line < min(first + g.per_walker, g.lines); ++line) {
+        const Stretch s = stretch_at(g, line, which, cv);
+        float4 x[kStretch], prev = zero4();
+        if (s.before) prev = ld4(a.x + s.base - s.step);
+#pragma unroll
+        for (int j = 0; j < kStretch; ++j) x[j] = j < s.n ? ld4(a.x + s.base + j * s.step) : zero4();
+#pragma unroll
+        for (int j = 0; j < kStretch; ++j) {
+            if (j < s.n) {
+                const float4 from = which > 3 ? x[j] : prev;
+                const float4 d = sub4(x[j], from);
+#pragma unroll
+                for (int m = 0; m < kMaxOut; ++m)
+                    if (m < a.n_out) st4(reinterpret_cast<Out*>(a.out[m]) + s.base + j * s.step, fma4(mix[m], d, from));
+            }
+            prev = x[j];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(qlines::kMaxThreads, 2) qshift_lines_backward(const Args a, const qlines::Grid g) {
+    using namespace qlines;
+    const int cv = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    if (cv >= g.C) return;
+    const int which = group_of(g, cv);
+    const unsigned walker = blockIdx.x * blockDim.y + threadIdx.y, first = walker * static_cast<unsigned>(g.per_walker);
+    float4 gmix[kMaxOut];
+#pragma unroll
+    for (int m = 0; m < kMaxOut; ++m) gmix[m] = zero4();
+    for (unsigned line = first; line < min(first + g.per_walker, g.lines); ++line) {
+        const Stretch s = stretch_at(g, line, which, cv);
+        float4 d[kStretch], gx[kStretch];          // x minus its shifted value; gradient of x
+        {
+            float4 prev = zero4();
+            if (s.before) prev = ld4(a.x + s.base - s.step);
+#pragma unroll
+            for (int j = 0; j < kStretch; ++j) {
+                d[j] = j < s.n ? ld4(a.x + s.base + j * s.step) : zero4();
+                gx[j] = zero4();
+            }
+#pragma unroll
+            for (int j = 0; j < kStretch; ++j) {
+                const float4 x = d[j];
+                d[j] = sub4(x, which > 3 ? x : prev);
+                prev = x;
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < kMaxOut; ++m) {
+            if (m < a.n_out) {
+                // the token that reads token j through the shift is token j + 1 of the line
+                float4 go[kStretch + 1];
+#pragma unroll
+                for (int j = 0; j <= kStretch; ++j)
+                    go[j] = j < s.n || (j == s.n && s.after) ? ld4(a.gout[m] + s.base + j * s.step) : zero4();
+                const float4 mix = ld4(a.mix[m] + cv), rest = make_float4(1.f - mix.x, 1.f - mix.y, 1.f - mix.z, 1.f - mix.w);
+#pragma unroll
+                for (int j = 0; j < kStretch; ++j)
+                    if (j < s.n) {
+                        gmix[m] = fma4(go[j], d[j], gmix[m]);
+                        gx[j] = fma4(which > 3 ? go[j] : go[j + 1], rest, fma4(go[j], mix, gx[j]));
+                    }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kStretch; ++j)
+            if (j < s.n) st4(a.gx + s.base + j * s.step, gx[j]);
+    }
+#pragma unroll
+    for (int m = 0; m < kMaxOut; ++m)
+        if (m < a.n_out) st4(a.partial + (static_cast<size_t>(walker) * a.n_out + m) * g.C + cv, gmix[m]);
+}
+
 // gmix[m][c] = sum over row blocks of partial[block][m][c], fixed order
 __global__ void __launch_bounds__(1024) qshift_reduce(const float* __restrict__ partial, int blocks, int n_out, int C,
                                                       float* __restrict__ gmix0, float* __restrict__ gmix1,
@@ -184,9 +272,11 @@ static bool vector_ok(const Args& a, bool bwd) {
         bits |= reinterpret_cast<uintptr_t>(a.mix[m]);
         bits |= reinterpret_cast<uintptr_t>(bwd ? static_cast<const void*>(a.gout[m]) : static_cast<const void*>(a.out[m]));
     }
-    if (bwd) bits |= reinterpret_cast<uintptr_t>(a.gx);
+    if (bwd) bits |= reinterpret_cast<uintptr_t>(a.gx) | reinterpret_cast<uintptr_t>(a.partial);
     return (bits & 15u) == 0;
 }
+// the walks cover a shift of one pixel (the only one the models use) on whole 4-channel vectors
+static bool walks(const Args& a, const qlines::Grid& g, bool bwd) { return a.shift == 1 && g.lines != 0 && vector_ok(a, bwd); }
 
 static int row_blocks(const Args& a) {
     const long long ntok = static_cast<long long>(a.B) * a.H * a.W;
@@ -196,28 +286,45 @@ static int row_blocks(const Args& a) {
 size_t backward_workspace(int B, int H, int W, int C, int n_out) {
     Args a{};
     a.B = B; a.H = H; a.W = W;
-    return static_cast<size_t>(row_blocks(a)) * n_out * C * sizeof(float);
+    // rows of partial sums of the general kernels, or of the walks (neither depends on the shift's group)
+    const long long walkers = qlines::make_shape(qlines::make_grid(B, H, W, C, 1, 0)).walkers;
+    return static_cast<size_t>(std::max<long long>(row_blocks(a), walkers)) * n_out * C * sizeof(float);
+}
+
+template <typename Out>
+static void forward_as(const Args& a, cudaStream_t stream) {
+    const qlines::Grid g = qlines::make_grid(a.B, a.H, a.W, a.C, a.group, a.period);
+    const int by = row_blocks(a);
+    if (walks(a, g, false)) {
+        const qlines::Shape s = qlines::make_shape(g);
+        qshift_lines_forward<Out><<<s.grid, s.block, 0, stream>>>(a, g);
+    } else if (vector_ok(a, false)) {
+        qshift_mix_forward<4, Out><<<dim3((a.C / 4 + kThreads - 1) / kThreads, by), kThreads, 0, stream>>>(a);
+    } else {
+        qshift_mix_forward<1, Out><<<dim3((a.C + kThreads - 1) / kThreads, by), kThreads, 0, stream>>>(a);
+    }
 }
 
 int forward(const Args& a, cudaStream_t stream) {
-    const int by = row_blocks(a);
-    if (vector_ok(a, false)) {
-        qshift_mix_forward<4><<<dim3((a.C / 4 + kThreads - 1) / kThreads, by), kThreads, 0, stream>>>(a);
-    } else {
-        qshift_mix_forward<1><<<dim3((a.C + kThreads - 1) / kThreads, by), kThreads, 0, stream>>>(a);
-    }
+    if (a.out_bf16) forward_as<__nv_bfloat16>(a, stream);
+    else forward_as<float>(a, stream);
     return 1;
 }
 
 int backward(const Args& a, float* const gmix[kMaxOut], cudaStream_t stream) {
-    const int by = row_blocks(a);
-    // the vector path of the backward only needs the group boundary rule (scalar loads inside)
-    if (a.C % 4 == 0 && a.group % 4 == 0) {
-        qshift_mix_backward<4><<<dim3((a.C / 4 + kThreads - 1) / kThreads, by), kThreads, 0, stream>>>(a);
+    const qlines::Grid g = qlines::make_grid(a.B, a.H, a.W, a.C, a.group, a.period);
+    int rows = row_blocks(a);
+    if (walks(a, g, true)) {
+        const qlines::Shape s = qlines::make_shape(g);
+        rows = static_cast<int>(s.walkers);
+        qshift_lines_backward<<<s.grid, s.block, 0, stream>>>(a, g);
+    } else if (a.C % 4 == 0 && a.group % 4 == 0) {
+        // the vector form of the general kernel only needs the group boundary rule (scalar loads inside)
+        qshift_mix_backward<4><<<dim3((a.C / 4 + kThreads - 1) / kThreads, rows), kThreads, 0, stream>>>(a);
     } else {
-        qshift_mix_backward<1><<<dim3((a.C + kThreads - 1) / kThreads, by), kThreads, 0, stream>>>(a);
+        qshift_mix_backward<1><<<dim3((a.C + kThreads - 1) / kThreads, rows), kThreads, 0, stream>>>(a);
     }
-    qshift_reduce<<<dim3((a.C + 31) / 32, a.n_out), dim3(32, 32), 0, stream>>>(a.partial, by, a.n_out, a.C, gmix[0],
+    qshift_reduce<<<dim3((a.C + 31) / 32, a.n_out), dim3(32, 32), 0, stream>>>(a.partial, rows, a.n_out, a.C, gmix[0],
                                                                               gmix[1], gmix[2]);
     return 2;
 }
@@ -235,7 +342,7 @@ static int qshift_check(int B, int H, int W, int C, int group, int shift, int n_
 }
 
 static int qshift_forward_any(int B, int H, int W, int C, int group, int period, int shift, int n_out, const float* x,
-                              const float* const* mix, float* const* out, void* stream) {
+                              const float* const* mix, void* const* out, bool out_bf16, void* stream) {
     if (int st = qshift_check(B, H, W, C, group, shift, n_out)) return st;
     if (!x || !mix || !out) return VRWKV_ERR_NULL;
     qshift::Args a{};
@@ -243,8 +350,9 @@ static int qshift_forward_any(int B, int H, int W, int C, int group, int period,
     for (int m = 0; m < n_out; ++m) {
         if (!mix[m] || !out[m]) return VRWKV_ERR_NULL;
         a.mix[m] = mix[m];
-        a.out[m] = out[m];
+        a.out[m] = static_cast<float*>(out[m]);
     }
+    a.out_bf16 = out_bf16;
     return record_launches(qshift::forward(a, static_cast<cudaStream_t>(stream)));
 }
 
@@ -276,14 +384,22 @@ static int multihead_check(int C, int head_dim) {
 extern "C" int vrwkv_qshift_mix_forward_f32(int B, int H, int W, int C, int group, int shift, int n_out,
                                             const float* x, const float* const* mix, float* const* out,
                                             void* stream) {
-    return qshift_forward_any(B, H, W, C, group, 0, shift, n_out, x, mix, out, stream);
+    return qshift_forward_any(B, H, W, C, group, 0, shift, n_out, x, mix, reinterpret_cast<void* const*>(out), false, stream);
 }
 
 extern "C" int vrwkv_qshift_multihead_mix_forward_f32(int B, int H, int W, int C, int head_dim, int shift, int n_out,
                                                       const float* x, const float* const* mix, float* const* out,
                                                       void* stream) {
     if (int st = multihead_check(C, head_dim)) return st;
-    return qshift_forward_any(B, H, W, C, head_dim / 4, head_dim, shift, n_out, x, mix, out, stream);
+    return qshift_forward_any(B, H, W, C, head_dim / 4, head_dim, shift, n_out, x, mix, reinterpret_cast<void* const*>(out), false, stream);
+}
+
+extern "C" int vrwkv_qshift_mix_forward_bf16out(int B, int H, int W, int C, int group, int head_dim, int shift, int n_out, const float* x,
+                                                const float* const* mix, uint16_t* const* out, void* stream) {
+    if (head_dim)
+        if (int st = multihead_check(C, head_dim)) return st;
+    return qshift_forward_any(B, H, W, C, head_dim ? head_dim / 4 : group, head_dim, shift, n_out, x, mix,
+                              reinterpret_cast<void* const*>(out), true, stream);
 }
 
 extern "C" size_t vrwkv_qshift_mix_backward_workspace_bytes(int B, int H, int W, int C, int n_out) {

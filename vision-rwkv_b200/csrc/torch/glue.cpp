@@ -44,17 +44,25 @@ struct QShiftArgs {
     bool per_head;
 };
 
-std::vector<Tensor> qshift_forward(const Tensor& xf, const std::vector<Tensor>& mixes, const QShiftArgs& a) {
+std::vector<Tensor> qshift_forward(const Tensor& xf, const std::vector<Tensor>& mixes, const QShiftArgs& a, bool half_out = false) {
     const Grid g = grid_of(xf, a.H, a.W);
     std::vector<Tensor> outs;
     Pointers<const float*> pm;
     Pointers<float*> po;
+    Pointers<uint16_t*> ph;
     for (size_t i = 0; i < mixes.size(); ++i) {
-        outs.push_back(at::empty_like(xf));
+        outs.push_back(at::empty_like(xf, half_out ? xf.options().dtype(at::kBFloat16) : xf.options()));
         pm.set(i, mixes[i]);
         po.set(i, outs[i]);
+        ph.set(i, outs[i]);
     }
     if (xf.numel() == 0) return outs;
+    if (half_out) {
+        check(vrwkv_qshift_mix_forward_bf16out(g.B, g.H, g.W, g.C, a.per_head ? 0 : a.group, a.per_head ? a.group : 0, a.shift, mixes.size(),
+                                               fp(xf), pm.at, ph.at, stream_of(xf)),
+              "vrwkv_qshift_mix_forward_bf16out");
+        return outs;
+    }
     const auto entry = a.per_head ? vrwkv_qshift_multihead_mix_forward_f32 : vrwkv_qshift_mix_forward_f32;
     check(entry(g.B, g.H, g.W, g.C, a.group, a.shift, mixes.size(), fp(xf), pm.at, po.at, stream_of(xf)), "vrwkv_qshift_mix_forward_f32");
     return outs;
@@ -256,6 +264,53 @@ std::vector<Tensor> qshift_mix(const Tensor& x, std::vector<Tensor> mixes, int64
     check_vectors(mixes, x);
     const c10::cuda::CUDAGuard guard(x.device());
     return QShiftMix::apply(x, at::TensorList(mixes), H, W, shift, group, per_head);
+}
+
+std::vector<Tensor> qshift_mix_half(const Tensor& x, std::vector<Tensor> mixes, int64_t H, int64_t W, int64_t shift, int64_t group,
+                                    bool per_head) {
+    TORCH_CHECK(mixes.size() >= 1 && mixes.size() <= 3, "between one and three mix vectors");
+    grid_of(x, H, W);
+    check_vectors(mixes, x);
+    const c10::cuda::CUDAGuard guard(x.device());
+    return qshift_forward(f32(x), flat_f32(mixes), QShiftArgs{H, W, shift, group, per_head}, true);
+}
+
+std::vector<Tensor> qshift_ddlerp_half(const Tensor& x, std::vector<Tensor> maas, std::vector<std::optional<Tensor>> offsets, int64_t H,
+                                       int64_t W, int64_t shift, int64_t head_dim) {
+    TORCH_CHECK(maas.size() >= 1 && maas.size() <= kMost && offsets.size() == maas.size(),
+                "between one and five mix vectors, and as many offsets (None for no offset)");
+    TORCH_CHECK(head_dim > 0 && head_dim % 16 == 0 && x.size(-1) % head_dim == 0, "head_dim=", head_dim,
+                " must be a multiple of 16 that divides C=", x.size(-1));
+    const Grid g = grid_of(x, H, W);
+    check_vectors(maas, x);
+    const c10::cuda::CUDAGuard guard(x.device());
+    const Tensor xf = f32(x);
+    const std::vector<Tensor> flat = flat_f32(maas);
+    bool half = true, any = false;
+    for (const auto& m : offsets)
+        if (m.has_value()) {
+            TORCH_CHECK(m->sizes() == x.sizes() && m->device() == x.device(), "offsets must have the shape of x and be on its device");
+            any = true;
+            half = half && is_bf16(*m);
+        }
+    half = half && any;
+    std::vector<Tensor> outs, kept;
+    Pointers<const float*> pa;
+    Pointers<const void*> pm;
+    Pointers<uint16_t*> po;
+    for (size_t i = 0; i < maas.size(); ++i) {
+        outs.push_back(at::empty_like(xf, xf.options().dtype(at::kBFloat16)));
+        pa.set(i, flat[i]);
+        po.set(i, outs[i]);
+        if (offsets[i].has_value()) {
+            kept.push_back(half ? offsets[i]->contiguous() : f32(*offsets[i]));
+            pm.set(i, kept.back());
+        }
+    }
+    if (xf.numel() == 0) return outs;
+    check(vrwkv_qshift_ddlerp_forward_bf16out(g.B, g.H, g.W, g.C, head_dim, shift, maas.size(), fp(xf), pa.at, pm.at, half, po.at, stream_of(xf)),
+          "vrwkv_qshift_ddlerp_forward_bf16out");
+    return outs;
 }
 
 std::vector<Tensor> qshift_ddlerp(const Tensor& x, std::vector<Tensor> maas, std::vector<std::optional<Tensor>> offsets, int64_t H, int64_t W,

@@ -6,5 +6,10 @@ namespace vrwkv {
 std::vector<Tensor> qshift_mix(const Tensor& x, std::vector<Tensor> mixes, int64_t H, int64_t W, int64_t shift, int64_t group, bool per_head);
 std::vector<Tensor> qshift_ddlerp(const Tensor& x, std::vector<Tensor> maas, std::vector<std::optional<Tensor>> offsets, int64_t H, int64_t W,
                                   int64_t shift, int64_t head_dim);
+// bfloat16 results, no autograd node
+std::vector<Tensor> qshift_mix_half(const Tensor& x, std::vector<Tensor> mixes, int64_t H, int64_t W, int64_t shift, int64_t group,
+                                    bool per_head);
+std::vector<Tensor> qshift_ddlerp_half(const Tensor& x, std::vector<Tensor> maas, std::vector<std::optional<Tensor>> offsets, int64_t H,
+                                       int64_t W, int64_t shift, int64_t head_dim);
 Tensor norm_gate(const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, int64_t group, double eps, int64_t act);
 }  // namespace vrwkv

@@ -305,6 +305,13 @@ PYBIND11_MODULE(_native, m) {
                               int64_t shift, int64_t head_dim) {
         return vrwkv::guarded([&] { return vrwkv::qshift_ddlerp(x, maas, offsets, H, W, shift, head_dim); })();
     });
+    m.def("qshift_mix_half", [](const Tensor& x, std::vector<Tensor> mixes, int64_t H, int64_t W, int64_t shift, int64_t group, bool per_head) {
+        return vrwkv::guarded([&] { return vrwkv::qshift_mix_half(x, mixes, H, W, shift, group, per_head); })();
+    });
+    m.def("qshift_ddlerp_half", [](const Tensor& x, std::vector<Tensor> maas, std::vector<std::optional<Tensor>> offsets, int64_t H, int64_t W,
+                                   int64_t shift, int64_t head_dim) {
+        return vrwkv::guarded([&] { return vrwkv::qshift_ddlerp_half(x, maas, offsets, H, W, shift, head_dim); })();
+    });
     m.def("norm_gate", [](const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, int64_t group, double eps, int64_t act) {
         return vrwkv::guarded([&] { return vrwkv::norm_gate(x, gate, weight, bias, group, eps, act); })();
     });

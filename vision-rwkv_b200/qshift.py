@@ -9,7 +9,18 @@
 """
 from __future__ import annotations
 
+import torch
+import torch.nn as nn
+
 from . import _lib, ops
+
+
+def feeds_autocast_linears(x, *layers):
+    """True when results may leave in bfloat16 because the next step rounds them to it: inference (training keeps the
+    float32 graph) under bfloat16 autocast, and every layer that takes them is a stock `nn.Linear` without hooks."""
+    return (not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.float32 and torch.is_autocast_enabled("cuda")
+            and torch.get_autocast_dtype("cuda") == torch.bfloat16
+            and all(type(m) is nn.Linear and not m._forward_hooks and not m._forward_pre_hooks for m in layers))
 
 
 def qshift_mix(x, mixes, patch_resolution, shift_pixel=1, channel_gamma=0.25, head_dim=None):
@@ -20,6 +31,16 @@ def qshift_mix(x, mixes, patch_resolution, shift_pixel=1, channel_gamma=0.25, he
     return tuple(_lib.native().qshift_mix(x, list(mixes), H, W, shift_pixel, group, head_dim is not None))
 
 
+def qshift_mix_to(layers, x, mixes, patch_resolution, shift_pixel=1, channel_gamma=0.25, head_dim=None):
+    """`qshift_mix` for the linear layers `layers`: in bfloat16 where those would round to it first anyway (the same bits
+    reach the matrix product, for 2 instead of 4 + 4 + 2 bytes per element and output)."""
+    if not feeds_autocast_linears(x, *layers):
+        return qshift_mix(x, mixes, patch_resolution, shift_pixel, channel_gamma, head_dim)
+    H, W = patch_resolution
+    group = ops.qshift_group(x.shape[-1], channel_gamma, head_dim)
+    return tuple(_lib.native().qshift_mix_half(x, list(mixes), H, W, shift_pixel, group, head_dim is not None))
+
+
 def qshift_ddlerp(x, maas, offsets, patch_resolution, shift_pixel=1, head_dim=64):
     """`[x + xx * (maa + m) for maa, m in zip(maas, offsets)]` with `xx = q_shift_multihead(x) - x`: the mixing steps of
     VRWKV6's spatial mix (classification/mmcls_custom/models/backbones/vrwkv6.py:180-193) in one pass.  `offsets`
@@ -27,3 +48,11 @@ def qshift_ddlerp(x, maas, offsets, patch_resolution, shift_pixel=1, head_dim=64
     float32 or bfloat16 offsets are read as they are."""
     H, W = patch_resolution
     return tuple(_lib.native().qshift_ddlerp(x, list(maas), list(offsets), H, W, shift_pixel, head_dim))
+
+
+def qshift_ddlerp_to(layers, x, maas, offsets, patch_resolution, shift_pixel=1, head_dim=64):
+    """`qshift_ddlerp` for the linear layers `layers` and plain matrix products, as `qshift_mix_to`."""
+    if not feeds_autocast_linears(x, *layers):
+        return qshift_ddlerp(x, maas, offsets, patch_resolution, shift_pixel, head_dim)
+    H, W = patch_resolution
+    return tuple(_lib.native().qshift_ddlerp_half(x, list(maas), list(offsets), H, W, shift_pixel, head_dim))
