@@ -1,0 +1,94 @@
+"""The inference steps between a block's matrix products (epilogue.py) against the tensor operations they stand for, which
+run under autograd (`torch.enable_grad`) in the same functions."""
+import pytest
+import torch
+import torch.nn as nn
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def normal(dev, *shape, dtype=torch.float32, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(dev, dtype)
+
+
+def both(fn):
+    """fn through the kernel and through the tensor operations"""
+    from vision_rwkv_b200 import _lib
+    lib = _lib.load()
+    with torch.no_grad():
+        before = lib.vrwkv_launch_count()
+        fast = fn()
+        assert lib.vrwkv_launch_count() > before
+    with torch.enable_grad():
+        return fast, fn()
+
+
+# one element, fewer than a thread's eight, one block (2048) and one over, and a ragged tail
+@pytest.mark.parametrize("n", [1, 7, 2048, 2049, 40003])
+@pytest.mark.parametrize("r_type,y_type", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+def test_elementwise_steps(cuda_device, n, r_type, y_type):
+    from vision_rwkv_b200 import epilogue
+    r, y = normal(cuda_device, n, dtype=r_type, seed=n) * 4, normal(cuda_device, n, dtype=y_type, seed=n + 1)
+    a, b = both(lambda: epilogue.sigmoid_gate(r, y))
+    # the same roundings; the two compilations of the sigmoid may differ in a last float32 bit
+    assert a.dtype == r_type and a.isfinite().all()
+    assert rel_err(a.float(), b.double()) < (1e-2 if r_type == torch.bfloat16 else 1e-6)
+    if r_type == torch.bfloat16:
+        assert (a != b).float().mean().item() < 1e-3 + 1.0 / n
+    for special in (float("nan"), float("inf"), -float("inf")):
+        r[n // 2] = special
+        a, b = both(lambda: epilogue.relu_square(r))
+        assert a.dtype == r_type and torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(), b.nan_to_num())
+
+
+# a row in one lane, a row that fills 128 channels, one vector more, the model widths, the widest
+@pytest.mark.parametrize("rows,C", [(1, 4), (9, 128), (17, 132), (200, 192), (33, 768), (8, 1024)])
+@pytest.mark.parametrize("a_type", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("scaled", [True, False])
+def test_residual_steps(cuda_device, rows, C, a_type, scaled):
+    from vision_rwkv_b200 import epilogue
+    x, a = normal(cuda_device, rows, C, seed=C), normal(cuda_device, rows, C, dtype=a_type, seed=rows) * 3 + 1
+    gamma = normal(cuda_device, C, seed=3) if scaled else None
+    norm = nn.LayerNorm(C).to(cuda_device)
+    norm.weight.data.copy_(normal(cuda_device, C, seed=4))
+    norm.bias.data.copy_(normal(cuda_device, C, seed=5))
+    fast, chain = both(lambda: epilogue.residual(x, a, gamma))
+    assert torch.equal(fast, chain)
+    with torch.autocast("cuda", torch.bfloat16):
+        fast, chain = both(lambda: epilogue.norm_residual(x, a, norm, gamma))
+    assert fast.dtype == chain.dtype == torch.float32
+    want = nn.functional.layer_norm(a.double(), (C,), norm.weight.double(), norm.bias.double(), norm.eps)
+    want = x.double() + (want if gamma is None else gamma.double() * want)
+    assert rel_err(fast, want.detach()) < 1e-6 and rel_err(chain.detach(), want.detach()) < 1e-6
+
+
+def test_layers_that_are_not_stock_keep_their_calls(cuda_device):
+    from vision_rwkv_b200 import epilogue
+    x, a, seen = normal(cuda_device, 4, 64), normal(cuda_device, 4, 64, seed=1), []
+    norm = nn.LayerNorm(64).to(cuda_device)
+    norm.register_forward_hook(lambda *args: seen.append(1))
+    with torch.no_grad():
+        epilogue.norm_residual(x, a, norm, None)
+        epilogue.norm_residual(x.half(), a.half(), nn.LayerNorm(64).to(cuda_device).half(), None)
+        wide = normal(cuda_device, 3, 1028)
+        epilogue.norm_residual(wide, wide, nn.LayerNorm(1028).to(cuda_device), None)
+    assert seen == [1]
+
+
+# a part of one block, exactly one block (64 heads), one head more, odd numbers of heads per row
+@pytest.mark.parametrize("rows,C", [(1, 64), (64, 64), (65, 64), (7, 192), (196, 768)])
+@pytest.mark.parametrize("gate_type", [torch.float32, torch.bfloat16])
+def test_head_norm_gate_is_the_float32_result_rounded(cuda_device, rows, C, gate_type):
+    from vision_rwkv_b200 import epilogue
+    x, gate = normal(cuda_device, 1, rows, C, seed=C) * 2 + 0.5, normal(cuda_device, 1, rows, C, dtype=gate_type, seed=rows)
+    norm, layer = nn.GroupNorm(C // 64, C).to(cuda_device), nn.Linear(C, 8).to(cuda_device)
+    norm.weight.data.copy_(normal(cuda_device, C, seed=4))
+    norm.bias.data.copy_(normal(cuda_device, C, seed=5))
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        half = epilogue.head_norm_gate(x, gate, norm, 64, layer, "silu")
+    with torch.no_grad():
+        wide = epilogue.head_norm_gate(x, gate, norm, 64, layer, "silu")
+    assert half.dtype == torch.bfloat16 and wide.dtype == torch.float32
+    assert torch.equal(half, wide.bfloat16())

@@ -20,9 +20,9 @@ import torch.nn as nn
 import torch.nn.functional as F
 import torch.utils.checkpoint as cp
 
-from . import normgate
+from . import epilogue, normgate
 from .qshift import qshift_mix_to
-from .vrwkv import RUN_CUDA
+from .vrwkv import RUN_CUDA, inference_biwkv
 
 
 def _ramp(n_embd):
@@ -58,15 +58,16 @@ class SpatialMix(nn.Module):
             xk = xv = xr = x
         k, v = self.key(xk), self.value(xv)
         r = self.receptance(xr)
-        y = RUN_CUDA(self.spatial_decay / T, self.spatial_first / T, k, v)
+        # the plain gate rounds y to the dtype of r; a norm in between takes it as it is
+        run = inference_biwkv if self.key_norm is None and r.dtype == torch.bfloat16 else RUN_CUDA
+        y = run(self.spatial_decay / T, self.spatial_first / T, k, v)
         if self.key_norm is not None and y.is_cuda and normgate.supported(y.shape[-1], y.shape[-1]):
             # LayerNorm, sigmoid and gate in one pass over y (normgate.py)
             return self.output(normgate.norm_gate(y, r, self.key_norm.weight, self.key_norm.bias, y.shape[-1],
                                                   self.key_norm.eps, act="sigmoid"))
-        sr = torch.sigmoid(r)
         if self.key_norm is not None:
             y = self.key_norm(y)
-        return self.output(sr * y.to(sr.dtype))
+        return self.output(epilogue.sigmoid_gate(r, y))
 
 
 class ChannelMix(nn.Module):
@@ -89,10 +90,10 @@ class ChannelMix(nn.Module):
                                    self.shift_pixel, self.channel_gamma)
         else:
             xk = xr = x
-        k = torch.square(torch.relu(self.key(xk)))
+        k = epilogue.relu_square(self.key(xk))
         if self.key_norm is not None:
             k = self.key_norm(k)
-        return torch.sigmoid(self.receptance(xr)) * self.value(k)
+        return epilogue.sigmoid_gate(self.receptance(xr), self.value(k))
 
 
 class Block(nn.Module):
@@ -113,14 +114,14 @@ class Block(nn.Module):
     def _inner(self, x, resolution):
         if self.layer_id == 0:
             x = self.ln0(x)
-        g1 = self.gamma1 if self.layer_scale else 1.0
-        g2 = self.gamma2 if self.layer_scale else 1.0
+        g1 = self.gamma1 if self.layer_scale else None
+        g2 = self.gamma2 if self.layer_scale else None
         if self.post_norm:
-            x = x + g1 * self.ln1(self.att(x, resolution))
-            x = x + g2 * self.ln2(self.ffn(x, resolution))
+            x = epilogue.norm_residual(x, self.att(x, resolution), self.ln1, g1)
+            x = epilogue.norm_residual(x, self.ffn(x, resolution), self.ln2, g2)
         else:
-            x = x + g1 * self.att(self.ln1(x), resolution)
-            x = x + g2 * self.ffn(self.ln2(x), resolution)
+            x = epilogue.residual(x, self.att(self.ln1(x), resolution), g1)
+            x = epilogue.residual(x, self.ffn(self.ln2(x), resolution), g2)
         return x
 
     def forward(self, x, resolution):

@@ -21,7 +21,7 @@ import torch.nn.functional as F
 import torch.utils.checkpoint as cp
 
 from .backbone import _PatchEmbed, _ramp
-from . import normgate
+from . import epilogue, normgate
 from .qshift import qshift_ddlerp_to, qshift_mix_to
 from .vrwkv6 import HEAD_SIZE, inference_rwkv6
 
@@ -105,7 +105,7 @@ class SpatialMixV6(nn.Module):
             y = self.key_norm(y)
         if y.is_cuda and normgate.supported(C, HEAD_SIZE):
             # per-head GroupNorm, SiLU and gate in one pass over y (normgate.py)
-            return self.output(normgate.norm_gate(y, g_raw, self.ln_x.weight, self.ln_x.bias, HEAD_SIZE, self.ln_x.eps, act="silu"))
+            return self.output(epilogue.head_norm_gate(y, g_raw, self.ln_x, HEAD_SIZE, self.output, "silu"))
         g = F.silu(g_raw)
         y = self.ln_x(y.reshape(B * T, C)).view(B, T, C)
         return self.output(y.to(g.dtype) * g)
@@ -127,10 +127,10 @@ class ChannelMixV6(nn.Module):
     def forward(self, x, resolution):
         xk, xr = qshift_mix_to((self.key, self.receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution, self.shift_pixel,
                                head_dim=HEAD_SIZE)       # per-head shift + both interpolations in one pass
-        k = torch.square(torch.relu(self.key(xk)))
+        k = epilogue.relu_square(self.key(xk))
         if self.key_norm is not None:
             k = self.key_norm(k)
-        return torch.sigmoid(self.receptance(xr)) * self.value(k)
+        return epilogue.sigmoid_gate(self.receptance(xr), self.value(k))
 
 
 class BlockV6(nn.Module):
@@ -151,14 +151,16 @@ class BlockV6(nn.Module):
     def _inner(self, x, resolution):
         if self.layer_id == 0:
             x = self.ln0(x)
-        g1 = self.gamma1 if self.layer_scale else 1.0
-        g2 = self.gamma2 if self.layer_scale else 1.0
+        g1 = self.gamma1 if self.layer_scale else None
+        g2 = self.gamma2 if self.layer_scale else None
+        # torch's own LayerNorm: these networks answer a change of a single rounding with 2 % of their result (see
+        # vrwkv6.inference_rwkv6), so only steps that keep every bit are taken over
         if self.post_norm:
-            x = x + g1 * self.ln1(self.att(x, resolution))
-            x = x + g2 * self.ln2(self.ffn(x, resolution))
+            x = epilogue.residual(x, self.ln1(self.att(x, resolution)), g1)
+            x = epilogue.residual(x, self.ln2(self.ffn(x, resolution)), g2)
         else:
-            x = x + g1 * self.att(self.ln1(x), resolution)
-            x = x + g2 * self.ffn(self.ln2(x), resolution)
+            x = epilogue.residual(x, self.att(self.ln1(x), resolution), g1)
+            x = epilogue.residual(x, self.ffn(self.ln2(x), resolution), g2)
         return x
 
     def forward(self, x, resolution):

@@ -1,0 +1,307 @@
+// What a block computes between its matrix products, for inference: one pass each instead of torch's chains.
+//
+//   sigmoid_gate    sigmoid(r) * y                   classification/mmcls_custom/models/backbones/vrwkv.py:182-187, 253-257
+//   relu_square     relu(x)^2                        vrwkv.py:250-251
+//   norm_residual   x + gamma * LayerNorm(a), or x + gamma * a             vrwkv.py:297-318 (post- and pre-norm blocks)
+//   head_norm_gate  (GroupNorm per 64-channel head) * activation(gate)     vrwkv6.py:133, 205-212, bfloat16 result
+//
+// All are bound by HBM.  Bytes per element under bfloat16 autocast, the tensor-op chains against these: the gate 4 + 6 + 6
+// (activation, cast of y, product) against 6; relu_square 8 against 4; norm_residual 34 (cast, norm, scale, add) against
+// 10; head_norm_gate 6 + 4 and the cast of its consumer, 6, against 8.  Every intermediate that a chain holds in bfloat16 is
+// rounded to bfloat16 here too, and products and sums are rounded one by one, so only the order of LayerNorm's sums
+// differs from torch's.
+// Networks at 224 pixels under bfloat16 autocast, these kernels and bfloat16 outputs of the token shift together: the small
+// model on 256 images 20.2 -> 8.0 ms, the matrix-state base model on 64 images 15.7 -> 11.6 ms.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <algorithm>
+#include <cstdint>
+#include "vrwkv_b200.h"
+#include "vrwkv_internal.h"
+
+namespace epilogue {
+
+constexpr int kThreads = 256;
+constexpr int kVec = 8;            // elements per thread and step of the elementwise kernels
+constexpr int kMaxC = 1024;        // of norm_residual: a row fits a warp's registers
+
+// N consecutive elements as floats
+template <int N>
+__device__ __forceinline__ void load(const float* p, float (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(p + i);
+        v[i] = t.x; v[i + 1] = t.y; v[i + 2] = t.z; v[i + 3] = t.w;
+    }
+}
+__device__ __forceinline__ void widen(uint32_t w, float& a, float& b) {
+    a = __uint_as_float(w << 16);
+    b = __uint_as_float(w & 0xffff0000u);
+}
+__device__ __forceinline__ uint32_t narrow(float a, float b) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&t);
+}
+template <int N>
+__device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[N]) {
+    if (N == 8) {
+        const uint4 t = *reinterpret_cast<const uint4*>(p);
+        widen(t.x, v[0], v[1]); widen(t.y, v[2], v[3]); widen(t.z, v[N - 4], v[N - 3]); widen(t.w, v[N - 2], v[N - 1]);
+    } else {
+        const uint2 t = *reinterpret_cast<const uint2*>(p);
+        widen(t.x, v[0], v[1]); widen(t.y, v[2], v[3]);
+    }
+}
+__device__ __forceinline__ void store(float* p, const float (&v)[kVec]) {
+#pragma unroll
+    for (int i = 0; i < kVec; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+}
+__device__ __forceinline__ void store(__nv_bfloat16* p, const float (&v)[kVec]) {
+    *reinterpret_cast<uint4*>(p) = make_uint4(narrow(v[0], v[1]), narrow(v[2], v[3]), narrow(v[4], v[5]), narrow(v[6], v[7]));
+}
+template <typename T>
+__device__ __forceinline__ float rounded(float x) { return x; }
+template <>
+__device__ __forceinline__ float rounded<__nv_bfloat16>(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
+template <typename R>
+__device__ __forceinline__ float gated(float r, float y) { return rounded<R>(1.f / (1.f + expf(-r))) * rounded<R>(y); }
+__device__ __forceinline__ float relu2(float x) {
+    const float t = x < 0.f ? 0.f : x;      // NaN stays NaN
+    return t * t;
+}
+
+// out = sigmoid(r) * y; the last n % kVec elements go to one thread
+template <typename R, typename Y>
+__global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, const R* __restrict__ r, const Y* __restrict__ y, R* __restrict__ out) {
+    const long long i = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVec;
+    if (i + kVec <= n) {
+        float a[kVec], b[kVec];
+        load(r + i, a);
+        load(y + i, b);
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) a[j] = gated<R>(a[j], b[j]);
+        store(out + i, a);
+    } else {
+        for (long long j = i; j < n; ++j)
+            out[j] = static_cast<R>(gated<R>(static_cast<float>(r[j]), static_cast<float>(y[j])));
+    }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, const R* __restrict__ x, R* __restrict__ out) {
+    const long long i = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVec;
+    if (i + kVec <= n) {
+        float a[kVec];
+        load(x + i, a);
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) a[j] = relu2(a[j]);
+        store(out + i, a);
+    } else {
+        for (long long j = i; j < n; ++j) out[j] = static_cast<R>(relu2(static_cast<float>(x[j])));
+    }
+}
+
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    return v;
+}
+
+// One warp per row, lane = 4 channels of each 128; kIters = ceil(C / 128).  Both inputs of a row are requested before the
+// first sum, so 6 C bytes per warp are in flight.
+template <typename A, int kIters>
+__global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C, float eps, const A* __restrict__ a, const float* __restrict__ weight,
+                                                                 const float* __restrict__ bias, const float* __restrict__ gamma,
+                                                                 const float* __restrict__ x, float* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const size_t base = static_cast<size_t>(row) * C + 4 * lane;
+    float v[kIters][4], res[kIters][4];
+#pragma unroll
+    for (int i = 0; i < kIters; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[i][j] = res[i][j] = 0.f;
+        if (128 * i + 4 * lane < C) {
+            load(a + base + 128 * i, v[i]);
+            load(x + base + 128 * i, res[i]);
+        }
+    }
+    if (weight != nullptr) {
+        const float inv = 1.f / static_cast<float>(C);
+        float s = 0.f, q = 0.f;
+#pragma unroll
+        for (int i = 0; i < kIters; ++i) s += (v[i][0] + v[i][1]) + (v[i][2] + v[i][3]);
+        const float mean = warp_sum(s) * inv;
+#pragma unroll
+        for (int i = 0; i < kIters; ++i)
+            if (128 * i + 4 * lane < C) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v[i][j] -= mean;
+                    q = fmaf(v[i][j], v[i][j], q);
+                }
+            }
+        const float rstd = rsqrtf(warp_sum(q) * inv + eps);
+#pragma unroll
+        for (int i = 0; i < kIters; ++i)
+            if (128 * i + 4 * lane < C) {
+                float w[4], b[4];
+                load(weight + 128 * i + 4 * lane, w);
+                load(bias + 128 * i + 4 * lane, b);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[i][j] = fmaf(v[i][j] * rstd, w[j], b[j]);
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < kIters; ++i)
+        if (128 * i + 4 * lane < C) {
+            float g[4] = {1.f, 1.f, 1.f, 1.f};
+            if (gamma != nullptr) load(gamma + 128 * i + 4 * lane, g);
+            float4 o;
+            o.x = __fadd_rn(res[i][0], __fmul_rn(g[0], v[i][0])); o.y = __fadd_rn(res[i][1], __fmul_rn(g[1], v[i][1]));
+            o.z = __fadd_rn(res[i][2], __fmul_rn(g[2], v[i][2])); o.w = __fadd_rn(res[i][3], __fmul_rn(g[3], v[i][3]));
+            *reinterpret_cast<float4*>(out + base + 128 * i) = o;
+        }
+}
+
+// Per-head norm and gate, a half-warp per 64-channel head: lane q holds channel pairs q and q + 16, which makes the sums'
+// order that of normgate_forward_kernel (a warp per head, one pair per lane; its butterfly adds those two first), and so
+// the bits of the float32 result before it is rounded.  kHeads heads per half-warp are requested together: one 256-byte
+// request per warp in flight left that kernel at about half of the HBM rate.
+constexpr int kHeads = 4;
+__device__ __forceinline__ float half_warp_sum(float v) {
+#pragma unroll
+    for (int m = 8; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    return v;
+}
+__device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 load2(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
+__device__ __forceinline__ float activation(float x, int act) {
+    if (act == 0) return x;
+    const float s = 1.f / (1.f + __expf(-x));
+    return act == 1 ? s : x * s;
+}
+template <typename G>
+__global__ void __launch_bounds__(kThreads) head_norm_gate_kernel(long long heads, int per_row, float eps, const float* __restrict__ x,
+                                                                  const G* __restrict__ gate, int act, const float* __restrict__ gamma,
+                                                                  const float* __restrict__ beta, __nv_bfloat16* __restrict__ out) {
+    const int q = threadIdx.x & 15;
+    const long long first = static_cast<long long>(blockIdx.x) * (kThreads / 16 * kHeads) + (threadIdx.x >> 4);
+    float2 v[kHeads][2], g[kHeads][2];
+#pragma unroll
+    for (int j = 0; j < kHeads; ++j) {
+        const long long head = min(first + j * (kThreads / 16), heads - 1);      // repeated heads are computed and not stored
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            v[j][i] = load2(x + head * 64 + 2 * q + 32 * i);
+            g[j][i] = load2(gate + head * 64 + 2 * q + 32 * i);
+        }
+    }
+    const float inv = 1.f / 64.f;
+#pragma unroll
+    for (int j = 0; j < kHeads; ++j) {
+        const long long head = first + j * (kThreads / 16);
+        const float mean = half_warp_sum((v[j][0].x + v[j][0].y) + (v[j][1].x + v[j][1].y)) * inv;
+        float part[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            float s = 0.f;
+            const float dx = v[j][i].x - mean, dy = v[j][i].y - mean;
+            s += dx * dx + dy * dy;
+            part[i] = s;
+        }
+        const float rstd = rsqrtf(half_warp_sum(part[0] + part[1]) * inv + eps);
+        if (head < heads) {
+            const int c = static_cast<int>(head % per_row) * 64 + 2 * q;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float2 ga = load2(gamma + c + 32 * i), be = load2(beta + c + 32 * i);
+                const float ox = ((v[j][i].x - mean) * rstd * ga.x + be.x) * activation(g[j][i].x, act);
+                const float oy = ((v[j][i].y - mean) * rstd * ga.y + be.y) * activation(g[j][i].y, act);
+                *reinterpret_cast<uint32_t*>(out + head * 64 + 2 * q + 32 * i) = narrow(ox, oy);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+static bool misaligned(std::initializer_list<const void*> ps) {
+    uintptr_t bits = 0;
+    for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
+    return (bits & 15u) != 0;
+}
+static long long blocks_of(long long n) { return (n + static_cast<long long>(kThreads) * kVec - 1) / (static_cast<long long>(kThreads) * kVec); }
+
+template <typename A, int kIters = 1>
+static void launch_norm_residual(int rows, int C, float eps, const A* a, const float* weight, const float* bias, const float* gamma, const float* x,
+                                 float* out, cudaStream_t s) {
+    if constexpr (kIters < kMaxC / 128) {
+        if (C > 128 * kIters) return launch_norm_residual<A, kIters + 1>(rows, C, eps, a, weight, bias, gamma, x, out, s);
+    }
+    const int per = kThreads / 32;
+    norm_residual_kernel<A, kIters><<<(rows + per - 1) / per, kThreads, 0, s>>>(rows, C, eps, a, weight, bias, gamma, x, out);
+}
+
+}  // namespace epilogue
+
+extern "C" int vrwkv_sigmoid_gate(long long n, const void* r, int r_is_bf16, const void* y, int y_is_bf16, void* out, void* stream) {
+    using namespace epilogue;
+    if (n <= 0 || blocks_of(n) > 0x7fffffffLL) return VRWKV_ERR_SHAPE;
+    if (!r || !y || !out) return VRWKV_ERR_NULL;
+    if (misaligned({r, y, out})) return VRWKV_ERR_ALIGNMENT;
+    if (y_is_bf16 && !r_is_bf16) return VRWKV_ERR_UNSUPPORTED;
+    const unsigned grid = static_cast<unsigned>(blocks_of(n));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    using H = __nv_bfloat16;
+    if (y_is_bf16) sigmoid_gate_kernel<H, H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(r), static_cast<const H*>(y), static_cast<H*>(out));
+    else if (r_is_bf16) sigmoid_gate_kernel<H, float><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(r), static_cast<const float*>(y), static_cast<H*>(out));
+    else sigmoid_gate_kernel<float, float><<<grid, kThreads, 0, s>>>(n, static_cast<const float*>(r), static_cast<const float*>(y), static_cast<float*>(out));
+    return record_launches(1);
+}
+
+extern "C" int vrwkv_relu_square(long long n, const void* x, int is_bf16, void* out, void* stream) {
+    using namespace epilogue;
+    if (n <= 0 || blocks_of(n) > 0x7fffffffLL) return VRWKV_ERR_SHAPE;
+    if (!x || !out) return VRWKV_ERR_NULL;
+    if (misaligned({x, out})) return VRWKV_ERR_ALIGNMENT;
+    const unsigned grid = static_cast<unsigned>(blocks_of(n));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    using H = __nv_bfloat16;
+    if (is_bf16) relu_square_kernel<H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(x), static_cast<H*>(out));
+    else relu_square_kernel<float><<<grid, kThreads, 0, s>>>(n, static_cast<const float*>(x), static_cast<float*>(out));
+    return record_launches(1);
+}
+
+extern "C" int vrwkv_norm_residual(int rows, int C, float eps, const void* a, int a_is_bf16, const float* weight, const float* bias,
+                                   const float* gamma, const float* x, float* out, void* stream) {
+    using namespace epilogue;
+    if (rows <= 0 || C <= 0) return VRWKV_ERR_SHAPE;
+    if (!a || !x || !out || (weight != nullptr) != (bias != nullptr)) return VRWKV_ERR_NULL;
+    if (C % 4 != 0 || C > kMaxC) return VRWKV_ERR_UNSUPPORTED;
+    if (misaligned({a, weight, bias, gamma, x, out})) return VRWKV_ERR_ALIGNMENT;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (a_is_bf16) launch_norm_residual(rows, C, eps, static_cast<const __nv_bfloat16*>(a), weight, bias, gamma, x, out, s);
+    else launch_norm_residual(rows, C, eps, static_cast<const float*>(a), weight, bias, gamma, x, out, s);
+    return record_launches(1);
+}
+
+extern "C" int vrwkv_head_norm_gate_bf16out(int rows, int C, float eps, const float* x, const void* gate, int gate_is_bf16, int gate_act,
+                                            const float* gamma, const float* beta, uint16_t* out, void* stream) {
+    using namespace epilogue;
+    if (rows <= 0 || C <= 0 || C % 64 != 0 || gate_act < 0 || gate_act > 2) return VRWKV_ERR_SHAPE;
+    if (!x || !gate || !gamma || !beta || !out) return VRWKV_ERR_NULL;
+    if (misaligned({x, gate, gamma, beta, out})) return VRWKV_ERR_ALIGNMENT;
+    const long long heads = static_cast<long long>(rows) * (C / 64), per = kThreads / 16 * kHeads, grid = (heads + per - 1) / per;
+    if (grid > 0x7fffffffLL) return VRWKV_ERR_SHAPE;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    auto* const o = reinterpret_cast<__nv_bfloat16*>(out);
+    if (gate_is_bf16)
+        head_norm_gate_kernel<<<static_cast<unsigned>(grid), kThreads, 0, s>>>(heads, C / 64, eps, x, static_cast<const __nv_bfloat16*>(gate), gate_act,
+                                                                               gamma, beta, o);
+    else
+        head_norm_gate_kernel<<<static_cast<unsigned>(grid), kThreads, 0, s>>>(heads, C / 64, eps, x, static_cast<const float*>(gate), gate_act, gamma,
+                                                                               beta, o);
+    return record_launches(1);
+}

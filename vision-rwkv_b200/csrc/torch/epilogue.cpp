@@ -1,0 +1,79 @@
+// Host path of the inference-only steps between a block's matrix products (csrc/mixer_epilogue.cu).  The rules that decide
+// whether a call may come here are epilogue.py's.
+#include "glue.h"
+
+namespace vrwkv {
+
+namespace {
+// contiguous and 16-byte aligned (a view may start anywhere)
+Tensor flat(const Tensor& t) {
+    const Tensor c = t.contiguous();
+    return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15u) ? c.clone() : c;
+}
+void same_place(const Tensor& t, const Tensor& like, const char* name) {
+    TORCH_CHECK(t.is_cuda() && t.device() == like.device(), name, " must be on ", like.device());
+}
+}  // namespace
+
+Tensor sigmoid_gate(const Tensor& r_, const Tensor& y_) {
+    same_place(y_, r_, "y");
+    TORCH_CHECK(r_.sizes() == y_.sizes(), "r and y must have the same shape");
+    const c10::cuda::CUDAGuard guard(r_.device());
+    const Tensor r = flat(r_), y = flat(y_);
+    Tensor out = at::empty(r.sizes(), r.options());
+    if (r.numel() != 0)
+        check(vrwkv_sigmoid_gate(r.numel(), r.data_ptr(), is_bf16(r), y.data_ptr(), is_bf16(y), out.data_ptr(), stream_of(r)), "vrwkv_sigmoid_gate");
+    return out;
+}
+
+Tensor relu_square(const Tensor& x_) {
+    same_place(x_, x_, "x");
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = flat(x_);
+    Tensor out = at::empty(x.sizes(), x.options());
+    if (x.numel() != 0) check(vrwkv_relu_square(x.numel(), x.data_ptr(), is_bf16(x), out.data_ptr(), stream_of(x)), "vrwkv_relu_square");
+    return out;
+}
+
+Tensor norm_residual(const Tensor& x_, const Tensor& a_, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
+                     const std::optional<Tensor>& gamma, double eps) {
+    same_place(a_, x_, "a");
+    const int64_t C = x_.size(-1), rows = C ? x_.numel() / C : 0;
+    TORCH_CHECK(a_.sizes() == x_.sizes(), "a must have the shape of x");
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = flat(x_), a = flat(a_);
+    Tensor kept[3];
+    const std::optional<Tensor>* given[3] = {&weight, &bias, &gamma};
+    const float* p[3] = {};
+    for (int i = 0; i < 3; ++i)
+        if (given[i]->has_value()) {
+            same_place(**given[i], x_, "a parameter");
+            kept[i] = flat(f32(**given[i]));
+            TORCH_CHECK(kept[i].numel() == C, "parameters must hold C values");
+            p[i] = fp(kept[i]);
+        }
+    Tensor out = at::empty(x.sizes(), x.options());
+    if (x.numel() != 0)
+        check(vrwkv_norm_residual(rows, C, static_cast<float>(eps), a.data_ptr(), is_bf16(a), p[0], p[1], p[2], fp(x), fp(out), stream_of(x)),
+              "vrwkv_norm_residual");
+    return out;
+}
+
+Tensor head_norm_gate_half(const Tensor& x_, const Tensor& gate_, const Tensor& weight_, const Tensor& bias_, double eps, int64_t act) {
+    same_place(gate_, x_, "gate");
+    same_place(weight_, x_, "weight");
+    same_place(bias_, x_, "bias");
+    const int64_t C = x_.size(-1), rows = C ? x_.numel() / C : 0;
+    TORCH_CHECK(gate_.sizes() == x_.sizes() && weight_.numel() == C && bias_.numel() == C,
+                "gate must have the shape of x; gamma and beta must hold C values");
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = flat(f32(x_)), gate = flat(is_bf16(gate_) ? gate_ : f32(gate_)), weight = flat(f32(weight_)), bias = flat(f32(bias_));
+    Tensor out = at::empty(x.sizes(), x.options().dtype(at::kBFloat16));
+    if (x.numel() != 0)
+        check(vrwkv_head_norm_gate_bf16out(rows, C, static_cast<float>(eps), fp(x), gate.data_ptr(), is_bf16(gate), act, fp(weight), fp(bias),
+                                           static_cast<uint16_t*>(out.data_ptr()), stream_of(x)),
+              "vrwkv_head_norm_gate_bf16out");
+    return out;
+}
+
+}  // namespace vrwkv

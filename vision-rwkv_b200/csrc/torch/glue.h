@@ -12,4 +12,10 @@ std::vector<Tensor> qshift_mix_half(const Tensor& x, std::vector<Tensor> mixes, 
 std::vector<Tensor> qshift_ddlerp_half(const Tensor& x, std::vector<Tensor> maas, std::vector<std::optional<Tensor>> offsets, int64_t H,
                                        int64_t W, int64_t shift, int64_t head_dim);
 Tensor norm_gate(const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, int64_t group, double eps, int64_t act);
+// epilogue.cpp
+Tensor sigmoid_gate(const Tensor& r, const Tensor& y);
+Tensor relu_square(const Tensor& x);
+Tensor norm_residual(const Tensor& x, const Tensor& a, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
+                     const std::optional<Tensor>& gamma, double eps);
+Tensor head_norm_gate_half(const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, double eps, int64_t act);
 }  // namespace vrwkv

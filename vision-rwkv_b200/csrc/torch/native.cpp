@@ -166,6 +166,14 @@ struct BiWkv : torch::autograd::Function<BiWkv> {
     }
 };
 
+// bfloat16 k, v to a bfloat16 y whatever the dtype of w: the values that biwkv widens where w is float32
+Tensor biwkv_half(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+    check_biwkv(w, u, k, v);
+    TORCH_CHECK(is_bf16(k) && is_bf16(v), "k, v must be bfloat16");
+    const c10::cuda::CUDAGuard guard(k.device());
+    return biwkv_forward_raw(f32(w), f32(u), k.contiguous(), v.contiguous());
+}
+
 Tensor biwkv(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, bool bf16_io) {
     check_biwkv(w, u, k, v);
     if (!any_requires_grad({&w, &u, &k, &v})) return biwkv_forward(w, u, k, v, bf16_io);
@@ -304,6 +312,18 @@ PYBIND11_MODULE(_native, m) {
     m.def("qshift_ddlerp", [](const Tensor& x, std::vector<Tensor> maas, std::vector<std::optional<Tensor>> offsets, int64_t H, int64_t W,
                               int64_t shift, int64_t head_dim) {
         return vrwkv::guarded([&] { return vrwkv::qshift_ddlerp(x, maas, offsets, H, W, shift, head_dim); })();
+    });
+    m.def("biwkv_half", [](const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+        return vrwkv::guarded([&] { return vrwkv::biwkv_half(w, u, k, v); })();
+    });
+    m.def("sigmoid_gate", [](const Tensor& r, const Tensor& y) { return vrwkv::guarded([&] { return vrwkv::sigmoid_gate(r, y); })(); });
+    m.def("relu_square", [](const Tensor& x) { return vrwkv::guarded([&] { return vrwkv::relu_square(x); })(); });
+    m.def("norm_residual", [](const Tensor& x, const Tensor& a, std::optional<Tensor> weight, std::optional<Tensor> bias,
+                              std::optional<Tensor> gamma, double eps) {
+        return vrwkv::guarded([&] { return vrwkv::norm_residual(x, a, weight, bias, gamma, eps); })();
+    });
+    m.def("head_norm_gate_half", [](const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, double eps, int64_t act) {
+        return vrwkv::guarded([&] { return vrwkv::head_norm_gate_half(x, gate, weight, bias, eps, act); })();
     });
     m.def("qshift_mix_half", [](const Tensor& x, std::vector<Tensor> mixes, int64_t H, int64_t W, int64_t shift, int64_t group, bool per_head) {
         return vrwkv::guarded([&] { return vrwkv::qshift_mix_half(x, mixes, H, W, shift, group, per_head); })();

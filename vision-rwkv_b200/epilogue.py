@@ -1,0 +1,62 @@
+"""The steps between a block's matrix products, for the networks of `backbone` and `backbone6`.
+
+Each function is the reference's expression; when a network is only being run (no gradients wanted) on CUDA tensors in
+float32 or bfloat16 it is one kernel of csrc/mixer_epilogue.cu instead of a chain of tensor operations.  Training keeps the
+tensor operations and their graph.  Layers whose work a kernel takes over must be the stock ones without hooks.
+"""
+from __future__ import annotations
+
+import torch
+import torch.nn as nn
+
+from . import _lib, normgate, ops
+from .qshift import feeds_autocast_linears
+
+KERNEL_DTYPES = (torch.float32, torch.bfloat16)
+MOST_NORM_CHANNELS = 1024       # a row of norm_residual lives in one warp's registers
+
+
+def _inference(*tensors):
+    return not torch.is_grad_enabled() and all(t.is_cuda and t.dtype in KERNEL_DTYPES for t in tensors)
+
+
+def relu_square(x):
+    """relu(x)^2 (classification/mmcls_custom/models/backbones/vrwkv.py:251)."""
+    return _lib.native().relu_square(x) if _inference(x) else torch.square(torch.relu(x))
+
+
+def sigmoid_gate(r, y):
+    """sigmoid(r) * y in the dtype of r (vrwkv.py:182-187, 253-257)."""
+    if _inference(r, y) and r.shape == y.shape and (y.dtype == torch.float32 or r.dtype == torch.bfloat16):
+        return _lib.native().sigmoid_gate(r, y)
+    return torch.sigmoid(r) * y.to(r.dtype)
+
+
+def _residual_kernel(x, a, gamma):
+    return (_inference(x, a) and x.dtype == torch.float32 and x.shape == a.shape and x.shape[-1] % 4 == 0
+            and x.shape[-1] <= MOST_NORM_CHANNELS and (gamma is None or gamma.dtype == torch.float32))
+
+
+def residual(x, a, gamma):
+    """x + gamma * a (gamma None: x + a)."""
+    if _residual_kernel(x, a, gamma):
+        return _lib.native().norm_residual(x, a, None, None, gamma, 0.0)
+    return x + (a if gamma is None else gamma * a)
+
+
+def norm_residual(x, a, norm, gamma):
+    """x + gamma * norm(a) for a LayerNorm `norm` (post-norm blocks).  Under autocast torch computes that norm in float32."""
+    C = x.shape[-1]
+    if (_residual_kernel(x, a, gamma) and type(norm) is nn.LayerNorm and norm.normalized_shape == (C,) and norm.bias is not None
+            and norm.weight.dtype == norm.bias.dtype == torch.float32 and not norm._forward_hooks and not norm._forward_pre_hooks
+            and (a.dtype == torch.float32 or torch.is_autocast_enabled("cuda"))):
+        return _lib.native().norm_residual(x, a, norm.weight, norm.bias, gamma, norm.eps)
+    return residual(x, norm(a), gamma)
+
+
+def head_norm_gate(x, gate, norm, head_size, layer, act):
+    """Per-head GroupNorm `norm` of x times the activated gate (vrwkv6.py:205-212), for the linear layer `layer`: in
+    bfloat16 where that layer would round to it first anyway."""
+    if head_size == 64 and feeds_autocast_linears(x, layer) and _inference(gate):
+        return _lib.native().head_norm_gate_half(x, gate, norm.weight, norm.bias, norm.eps, ops.GATE_ACTIVATIONS[act])
+    return normgate.norm_gate(x, gate, norm.weight, norm.bias, head_size, norm.eps, act=act)

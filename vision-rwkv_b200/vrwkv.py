@@ -117,3 +117,12 @@ def RUN_CUDA(w, u, k, v, decay_offset: int = 0):
     if decay_offset:
         u = u - decay_offset * w
     return _run(w, u, k, v)
+
+
+def inference_biwkv(w, u, k, v):
+    """`RUN_CUDA` for a consumer that rounds y to bfloat16 (the gate of a network under autocast): where y would hold bfloat16
+    values widened to float32 it stays in bfloat16.  Everything else is `RUN_CUDA`."""
+    if (not torch.is_grad_enabled() and k.is_cuda and _bf16_path(k, v) and w.dtype == torch.float32
+            and not (SAVE_DENOMINATOR or ops.CHECK_STATUS)):
+        return _lib.native().biwkv_half(w, u, k, v)
+    return RUN_CUDA(w, u, k, v)
