@@ -124,8 +124,30 @@ __global__ void __launch_bounds__(kThreads) ddlerp_forward(const Args a) {
     }
 }
 
-// the same for a shift of one pixel, in walks along the lines of the grid (qshift_lines.cuh)
-template <bool kHalfM, typename Out>
+// The same for a shift of one pixel, in walks along the lines of the grid (qshift_lines.cuh).  The offsets are most of what is
+// read, so stretches are short and all kMaxOut offsets of a stretch are requested before the first output is formed
+// (bfloat16: 20 requests of 8 bytes and 5 of 16 per thread).  Stretches of 8 with one offset's requests in flight
+// at a time took 160 us for five outputs at B=64, 14 x 14, C=768 (231 MB); this takes 66 us.
+constexpr int kShort = 4;
+template <bool kHalfM>
+struct RawM;
+template <>
+struct RawM<true> {
+    uint2 v;
+    __device__ __forceinline__ void get(const void* m, size_t at) { v = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(m) + at)); }
+    __device__ __forceinline__ float4 f() const {
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+        return make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+};
+template <>
+struct RawM<false> {
+    float4 v;
+    __device__ __forceinline__ void get(const void* m, size_t at) { v = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(m) + at)); }
+    __device__ __forceinline__ float4 f() const { return v; }
+};
+// kOffsets = false: no output has an offset, nothing but x is read; stretches of qlines::kStretch then.
+template <bool kHalfM, bool kOffsets, typename Out>
 __global__ void __launch_bounds__(qlines::kMaxThreads, 2) ddlerp_lines_forward(const Args a, const qlines::Grid g) {
     using namespace qlines;
     const int cv = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
@@ -134,12 +156,22 @@ __global__ void __launch_bounds__(qlines::kMaxThreads, 2) ddlerp_lines_forward(c
     const unsigned first = (blockIdx.x * blockDim.y + threadIdx.y) * static_cast<unsigned>(g.per_walker);
     for (unsigned line = first; line < min(first + g.per_walker, g.lines); ++line) {
         const Stretch s = stretch_at(g, line, which, cv);
-        float4 x[kStretch], d[kStretch], prev = zero4();
+        constexpr int kTokens = kOffsets ? kShort : kStretch;
+        float4 x[kTokens], prev = zero4();
+        RawM<kHalfM> mu[kOffsets ? kMaxOut : 1][kShort];
         if (s.before) prev = ld4(a.x + s.base - s.step);
 #pragma unroll
-        for (int i = 0; i < kStretch; ++i) x[i] = i < s.n ? ld4(a.x + s.base + i * s.step) : zero4();
+        for (int i = 0; i < kTokens; ++i) x[i] = i < s.n ? ld4(a.x + s.base + i * s.step) : zero4();
 #pragma unroll
-        for (int i = 0; i < kStretch; ++i) {
+        for (int j = 0; j < kMaxOut; ++j)
+            if (kOffsets && j < a.n_out && a.m[j] != nullptr) {
+#pragma unroll
+                for (int i = 0; i < kShort; ++i)
+                    if (i < s.n) mu[kOffsets ? j : 0][i].get(a.m[j], s.base + i * s.step);
+            }
+        float4 d[kTokens];
+#pragma unroll
+        for (int i = 0; i < kTokens; ++i) {
             d[i] = sub4(prev, x[i]);
             prev = x[i];
         }
@@ -147,12 +179,12 @@ __global__ void __launch_bounds__(qlines::kMaxThreads, 2) ddlerp_lines_forward(c
         for (int j = 0; j < kMaxOut; ++j)
             if (j < a.n_out) {
                 const float4 maa = ld4(a.maa[j] + cv);
-                float4 mu[kStretch];
 #pragma unroll
-                for (int i = 0; i < kStretch; ++i) mu[i] = i < s.n ? load_m<kHalfM>(a.m[j], s.base + i * s.step) : zero4();
-#pragma unroll
-                for (int i = 0; i < kStretch; ++i)
-                    if (i < s.n) st4(reinterpret_cast<Out*>(a.out[j]) + s.base + i * s.step, fma4(d[i], add4(maa, mu[i]), x[i]));
+                for (int i = 0; i < kTokens; ++i)
+                    if (i < s.n) {
+                        const float4 m = kOffsets && a.m[j] != nullptr ? mu[kOffsets ? j : 0][i % kShort].f() : zero4();
+                        st4(reinterpret_cast<Out*>(a.out[j]) + s.base + i * s.step, fma4(d[i], add4(maa, m), x[i]));
+                    }
             }
     }
 }
@@ -251,10 +283,13 @@ static bool misaligned(const void* p, uintptr_t a) { return (reinterpret_cast<ui
 namespace ddlerp {
 template <bool kHalfM, typename Out>
 static void launch_forward(const Args& a, cudaStream_t s) {
-    const qlines::Grid g = qlines::make_grid(a.B, a.H, a.W, a.C, a.head_dim / 4, a.head_dim);
+    bool offsets = false;
+    for (int j = 0; j < a.n_out; ++j) offsets = offsets || a.m[j] != nullptr;
+    const qlines::Grid g = qlines::make_grid(a.B, a.H, a.W, a.C, a.head_dim / 4, a.head_dim, offsets ? kShort : qlines::kStretch);
     if (a.shift == 1 && g.lines != 0) {       // any other shift: token by token
         const qlines::Shape shape = qlines::make_shape(g);
-        ddlerp_lines_forward<kHalfM, Out><<<shape.grid, shape.block, 0, s>>>(a, g);
+        if (offsets) ddlerp_lines_forward<kHalfM, true, Out><<<shape.grid, shape.block, 0, s>>>(a, g);
+        else ddlerp_lines_forward<kHalfM, false, Out><<<shape.grid, shape.block, 0, s>>>(a, g);
     } else {
         ddlerp_forward<kHalfM, Out><<<dim3((a.C / kVec + kThreads - 1) / kThreads, row_blocks(a.B, a.H, a.W)), kThreads, 0, s>>>(a);
     }

@@ -6,7 +6,8 @@
 // neighbour needs is already in a register: one halo load per stretch replaces a second load per token, and all loads of a
 // stretch are issued together (9 independent 16-byte loads in flight per thread and tensor).  Channels of different
 // groups walk different lines; a warp's accesses still cover whole 32-byte sectors.  Token-by-token code with
-// one load and a 64-bit division per token in flight measured 0.56 of the HBM rate (B=64, 24 x 24, C=1024, three outputs, forward + backward: 376 us); this measures 0.80 (262 us).
+// one load and a 64-bit division per token in flight measured 0.56 of the HBM rate; this measures 0.80 (B=64, 24 x 24, C=1024,
+// three outputs, forward + backward: 376 and 262 us).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -15,7 +16,7 @@
 
 namespace qlines {
 
-constexpr int kStretch = 8;        // tokens a thread holds at a time
+constexpr int kStretch = 8;        // tokens a thread holds at a time (at most)
 constexpr int kMaxThreads = 256;   // of a block: channel vectors x walkers
 
 struct Grid {
@@ -35,12 +36,12 @@ struct Shape {
 
 // (host) stretches as even as possible; enough of them per walker that partial sums stay small beside the tensors, few
 // enough that the blocks fill the device
-inline Grid make_grid(int B, int H, int W, int C, int group, int period) {
+inline Grid make_grid(int B, int H, int W, int C, int group, int period, int stretch = kStretch) {
     Grid g{};
     g.B = B; g.H = H; g.W = W; g.C = C; g.group = group; g.period = period;
-    g.row_parts = (W + kStretch - 1) / kStretch;
+    g.row_parts = (W + stretch - 1) / stretch;
     g.row_len = (W + g.row_parts - 1) / g.row_parts;
-    g.col_parts = (H + kStretch - 1) / kStretch;
+    g.col_parts = (H + stretch - 1) / stretch;
     g.col_len = (H + g.col_parts - 1) / g.col_parts;
     const long long each = std::max(static_cast<long long>(H) * g.row_parts, static_cast<long long>(W) * g.col_parts);
     const long long lines = each * B;
