@@ -92,3 +92,38 @@ def test_head_norm_gate_is_the_float32_result_rounded(cuda_device, rows, C, gate
         wide = epilogue.head_norm_gate(x, gate, norm, 64, layer, "silu")
     assert half.dtype == torch.bfloat16 and wide.dtype == torch.float32
     assert torch.equal(half, wide.bfloat16())
+
+
+# one vector, one block of vectors (2048 elements) and more, tables of one row and of several
+@pytest.mark.parametrize("shape,table", [((1, 1, 8), (1, 1, 8)), ((2, 128, 8), (1, 1, 8)), ((3, 50, 192), (1, 1, 192)), ((5, 49, 40), (1, 49, 40)),
+                                         ((2, 9, 12), (1, 1, 12)), ((1, 7, 64), (1, 1, 64))])
+def test_add_rows(cuda_device, shape, table):
+    from vision_rwkv_b200 import epilogue
+    t, a = normal(cuda_device, *table, seed=1), normal(cuda_device, *shape, dtype=torch.bfloat16, seed=2)
+    with torch.no_grad():
+        out = epilogue.add_rows(t, a)
+    assert out.dtype == torch.float32 and torch.equal(out, t + a)
+    with pytest.raises(RuntimeError):
+        epilogue.add_rows(t[..., :-1], a)
+
+
+# a single patch, patches of 8 pixels, sides that leave pixels over, widths that only the convolution takes
+@pytest.mark.parametrize("B,channels,H,W,patch", [(1, 3, 16, 16, 16), (2, 3, 40, 72, 16), (3, 1, 24, 20, 8), (2, 3, 35, 47, 16), (1, 3, 224, 224, 16)])
+def test_patch_embedding(cuda_device, B, channels, H, W, patch):
+    from vision_rwkv_b200 import epilogue
+    img, conv = normal(cuda_device, B, channels, H, W, seed=H), nn.Conv2d(channels, 24, patch, stride=patch).to(cuda_device)
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        tokens = epilogue.patch_embedding(img, conv)
+        by_conv = conv(img)
+    if W % 4:
+        assert tokens is None
+        return
+    want = nn.functional.conv2d(img.bfloat16().double(), conv.weight.bfloat16().double(), conv.bias.bfloat16().double(), stride=patch)
+    want = want.flatten(2).transpose(1, 2).detach()
+    assert tokens.dtype == torch.bfloat16 and tokens.shape == want.shape
+    # a rounding to bfloat16 moves an element by up to 2^-8 of it; both round before and behind the bias (which may make
+    # the first of the two a little larger than the result)
+    bound = 2 * 2.0 ** -8 * 1.25
+    assert rel_err(tokens.double(), want) < bound and rel_err(by_conv.flatten(2).transpose(1, 2).double(), want) < bound
+    with torch.no_grad():
+        assert epilogue.patch_embedding(img, conv) is None                       # float32 networks keep the convolution

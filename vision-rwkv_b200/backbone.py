@@ -131,11 +131,17 @@ class Block(nn.Module):
 
 
 class _PatchEmbed(nn.Module):
-    def __init__(self, in_channels, embed_dims, patch_size):
+    # as_product: inference may take the projection as a matrix product over the patches (another order of its sums)
+    def __init__(self, in_channels, embed_dims, patch_size, as_product=False):
         super().__init__()
+        self.as_product = as_product
         self.projection = nn.Conv2d(in_channels, embed_dims, patch_size, stride=patch_size, bias=True)
 
     def forward(self, img):
+        x = epilogue.patch_embedding(img, self.projection) if self.as_product else None
+        if x is not None:
+            p = self.projection.kernel_size[0]
+            return x, (img.shape[2] // p, img.shape[3] // p)
         x = self.projection(img)
         return x.flatten(2).transpose(1, 2), (x.shape[2], x.shape[3])
 
@@ -155,7 +161,7 @@ class VRWKV(nn.Module):
                  out_indices=(-1,)):
         super().__init__()
         size = (img_size, img_size) if isinstance(img_size, int) else tuple(img_size)
-        self.patch_embed = _PatchEmbed(in_channels, embed_dims, patch_size)
+        self.patch_embed = _PatchEmbed(in_channels, embed_dims, patch_size, as_product=True)
         self.patch_resolution = (size[0] // patch_size, size[1] // patch_size)
         self.interpolate_mode = interpolate_mode
         self.pos_embed = nn.Parameter(torch.zeros(1, self.patch_resolution[0] * self.patch_resolution[1], embed_dims))
@@ -177,7 +183,7 @@ class VRWKV(nn.Module):
 
     def forward(self, img):
         x, resolution = self.patch_embed(img)
-        x = x + self._pos(resolution)
+        x = epilogue.add_rows(self._pos(resolution), x)
         outs = []
         for i, layer in enumerate(self.layers):
             x = layer(x, resolution)

@@ -98,7 +98,7 @@ class SpatialMixV6(nn.Module):
         k = self.key(xk)
         v = self.value(xv)
         g_raw = self.gate(xg)
-        w = self.time_decay + torch.tanh(xw @ self.time_decay_w1) @ self.time_decay_w2
+        w = epilogue.add_rows(self.time_decay, torch.tanh(xw @ self.time_decay_w1) @ self.time_decay_w2)
         y = inference_rwkv6(B, T, C, self.n_head, r.contiguous(), k.contiguous(), v.contiguous(),
                             w.float().contiguous(), self.time_faaaa)
         if self.key_norm is not None:

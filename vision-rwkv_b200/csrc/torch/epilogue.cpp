@@ -35,6 +35,30 @@ Tensor relu_square(const Tensor& x_) {
     return out;
 }
 
+Tensor add_rows(const Tensor& table_, const Tensor& a_) {
+    same_place(table_, a_, "table");
+    TORCH_CHECK(is_bf16(a_) && table_.scalar_type() == at::kFloat, "a must be bfloat16 and the table float32");
+    TORCH_CHECK(table_.numel() > 0 && a_.numel() % table_.numel() == 0, "a must hold whole tables");
+    const c10::cuda::CUDAGuard guard(a_.device());
+    const Tensor a = flat(a_), table = flat(table_);
+    Tensor out = at::empty(a.sizes(), table.options());
+    if (a.numel() != 0)
+        check(vrwkv_add_rows(a.numel(), table.numel(), fp(table), static_cast<uint16_t*>(a.data_ptr()), fp(out), stream_of(a)), "vrwkv_add_rows");
+    return out;
+}
+
+Tensor patch_rows(const Tensor& img_, int64_t patch) {
+    same_place(img_, img_, "img");
+    TORCH_CHECK(img_.dim() == 4 && img_.scalar_type() == at::kFloat && patch > 0, "img must be (B, channels, H, W) in float32");
+    const c10::cuda::CUDAGuard guard(img_.device());
+    const Tensor img = flat(img_);
+    const int64_t B = img.size(0), c = img.size(1), H = img.size(2), W = img.size(3);
+    Tensor out = at::empty({B, (H / patch) * (W / patch), c * patch * patch}, img.options().dtype(at::kBFloat16));
+    if (out.numel() != 0)
+        check(vrwkv_patch_rows(B, c, H, W, patch, fp(img), static_cast<uint16_t*>(out.data_ptr()), stream_of(img)), "vrwkv_patch_rows");
+    return out;
+}
+
 Tensor norm_residual(const Tensor& x_, const Tensor& a_, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
                      const std::optional<Tensor>& gamma, double eps) {
     same_place(a_, x_, "a");

@@ -15,6 +15,8 @@ Tensor norm_gate(const Tensor& x, const Tensor& gate, const Tensor& weight, cons
 // epilogue.cpp
 Tensor sigmoid_gate(const Tensor& r, const Tensor& y);
 Tensor relu_square(const Tensor& x);
+Tensor add_rows(const Tensor& table, const Tensor& a);
+Tensor patch_rows(const Tensor& img, int64_t patch);
 Tensor norm_residual(const Tensor& x, const Tensor& a, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
                      const std::optional<Tensor>& gamma, double eps);
 Tensor head_norm_gate_half(const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, double eps, int64_t act);

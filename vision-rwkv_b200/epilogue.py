@@ -60,3 +60,30 @@ def head_norm_gate(x, gate, norm, head_size, layer, act):
     if head_size == 64 and feeds_autocast_linears(x, layer) and _inference(gate):
         return _lib.native().head_norm_gate_half(x, gate, norm.weight, norm.bias, norm.eps, ops.GATE_ACTIVATIONS[act])
     return normgate.norm_gate(x, gate, norm.weight, norm.bias, head_size, norm.eps, act=act)
+
+
+def add_rows(table, a):
+    """table + a, the table (leading sizes 1) repeated over the rows of a: the decay of vrwkv6.py:200, the positions of
+    vrwkv.py:392."""
+    sizes = list(table.shape)
+    while sizes and sizes[0] == 1:
+        sizes.pop(0)
+    if (_inference(table, a) and a.dtype == torch.bfloat16 and table.dtype == torch.float32 and a.is_contiguous()
+            and table.numel() % 8 == 0 and 0 < table.numel() and a.numel() < 2 ** 33 and table.dim() <= a.dim()
+            and list(a.shape[a.dim() - len(sizes):]) == sizes):
+        return _lib.native().add_rows(table, a)
+    return table + a
+
+
+def patch_embedding(img, conv):
+    """The tokens (B, h * w, C) of a patch embedding `conv` (kernel = stride; vrwkv.py:357) as one matrix product over the
+    patches, or None where the convolution itself has to run (training, other data types, other convolutions)."""
+    p = conv.kernel_size[0]
+    if not (feeds_autocast_linears(img) and type(conv) is nn.Conv2d and not conv._forward_hooks and not conv._forward_pre_hooks
+            and conv.kernel_size == conv.stride == (p, p) and conv.padding == (0, 0) and conv.dilation == (1, 1) and conv.groups == 1
+            and img.dim() == 4 and img.shape[1] == conv.in_channels and img.is_contiguous() and p % 8 == 0
+            and img.shape[2] >= p and img.shape[3] >= p and img.shape[3] % 4 == 0 and img.numel() < 2 ** 33):
+        return None
+    tokens = nn.functional.linear(_lib.native().patch_rows(img, p), conv.weight.flatten(1))
+    # the convolution rounds to bfloat16 before its bias too
+    return tokens if conv.bias is None else tokens + conv.bias.to(tokens.dtype)
