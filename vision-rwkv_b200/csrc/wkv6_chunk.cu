@@ -57,7 +57,10 @@ struct StateArgs {
 constexpr uint32_t kWaitLimit = 1u << 20;      // polls before a wait for a tile gives up
 
 // Shared memory of a CTA: the raw tiles of one chunk as the copy engine delivers them (w | x, z of every pair), then per
-// pair the operand planes and twice the totals (the next chunk's are written while this one's are read).
+// pair the operand planes, then twice the totals (the next chunk's are written while this one's are read).  Both pairs
+// read the first one's totals: with a copy each, the backward on bfloat16 tensors and float32 gy was 1 KB above half of an
+// SM's shared memory.  Forward + backward at B=32, H=12
+// with one CTA of it per SM, and with two: T=196 303 and 286 us, T=4096 4.73 and 4.68 ms.
 template <typename XT, typename ZT0, typename ZT1, int kZ, int kX, int kPairs>
 struct StateSmem {
     static constexpr size_t kTile = kChunk * N;
@@ -65,17 +68,19 @@ struct StateSmem {
     static constexpr size_t x0 = kTile * 4, z0 = x0 + kTile * sizeof(XT);
     static constexpr size_t x1 = z0 + kTile * sizeof(ZT0), z1 = x1 + (kPairs > 1 ? kTile * sizeof(XT) : 0);
     static constexpr size_t planes = z1 + (kPairs > 1 ? kTile * sizeof(ZT1) : 0);
-    static constexpr size_t per_pair = static_cast<size_t>(kZ + kX) * kPlane * 2 + 2 * sizeof(Totals);
-    static constexpr size_t bar = planes + kPairs * per_pair;
+    static constexpr size_t per_pair = static_cast<size_t>(kZ + kX) * kPlane * 2;
+    static constexpr size_t totals = planes + kPairs * per_pair;
+    static constexpr size_t bar = totals + 2 * sizeof(Totals);
     static constexpr size_t bytes = bar + 16;
     static constexpr uint32_t loaded = static_cast<uint32_t>(planes);
 };
 
 // The work of one pair's four warps (a block each) on one chunk: lane = two channels, one token after the other, so decays,
-// their running sums and the scaling need no shuffles.  Leaves the scaled operand planes; `tot` gets the blocks' sums.
+// their running sums and the scaling need no shuffles.  Leaves the scaled operand planes; `tot` gets the blocks' sums
+// (from the pair that `writes`).
 template <typename XT, typename ZT, int kZ, int kX>
-__device__ __forceinline__ void scale_chunk(const float* wt, const XT* xt, const ZT* zt, int valid, int dir, Totals& tot, __nv_bfloat16* xs,
-                                            __nv_bfloat16* zs, int warp, int lane) {
+__device__ __forceinline__ void scale_chunk(const float* wt, const XT* xt, const ZT* zt, int valid, int dir, Totals& tot, bool writes,
+                                            __nv_bfloat16* xs, __nv_bfloat16* zs, int warp, int lane) {
     const int word = col_word(lane), row0 = warp * kBlock;
     float2 sum[kBlock];
     float2 run = make_float2(0.f, 0.f);
@@ -88,7 +93,7 @@ __device__ __forceinline__ void scale_chunk(const float* wt, const XT* xt, const
         }
         sum[t] = run;
     }
-    *reinterpret_cast<float2*>(&tot[warp][2 * lane]) = run;
+    if (writes) *reinterpret_cast<float2*>(&tot[warp][2 * lane]) = run;
     __syncthreads();       // totals are there; every warp is past the previous chunk's products
     float2 edge = make_float2(0.f, 0.f);        // decay from the block to the chunk's edge
     for (int j = dir == 0 ? warp + 1 : 0; j < (dir == 0 ? kBlocks : warp); ++j) {
@@ -129,7 +134,7 @@ wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, con
     uint4* out = a.out + (static_cast<size_t>(pair) * 2 + dir) * a.plane + static_cast<size_t>(bh) * a.n_chunks * kState;
     __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem + S::planes + pair * S::per_pair);
     __nv_bfloat16* zs = xs + kX * kPlane;
-    Totals* tots = reinterpret_cast<Totals*>(zs + kZ * kPlane);
+    Totals* tots = reinterpret_cast<Totals*>(smem + S::totals);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::bar);
     const auto chunk_of = [&](int step) { return dir == 0 ? step : a.n_chunks - 1 - step; };
     const auto fetch = [&](int step) {
@@ -171,10 +176,10 @@ wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, con
         const float* wt = reinterpret_cast<const float*>(smem + S::w);
         if (kPairs == 1 || pair == 0)
             scale_chunk<XT, ZT0, kZ, kX>(wt, reinterpret_cast<const XT*>(smem + S::x0), reinterpret_cast<const ZT0*>(smem + S::z0), valid, dir, tot,
-                                         xs, zs, warp, lane);
+                                         true, xs, zs, warp, lane);
         else
             scale_chunk<XT, ZT1, kZ, kX>(wt, reinterpret_cast<const XT*>(smem + S::x1), reinterpret_cast<const ZT1*>(smem + S::z1), valid, dir, tot,
-                                         xs, zs, warp, lane);
+                                         false, xs, zs, warp, lane);
         __syncthreads();
         if (threadIdx.x == 0) {
             if (step + 1 < last) fetch(step + 1);
