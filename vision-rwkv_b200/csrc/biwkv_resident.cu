@@ -3,8 +3,8 @@
 // element of k, v (and gy) crosses HBM once in and every output once out, and nothing but the
 // cluster's own CTAs ever has to be waited for.
 //
-// Work unit: one (sequence b, strip of kCs = 32 channels).  A cluster of `cluster` CTAs (1, 2, 4, 8
-// or 16) splits its T tokens into contiguous ranges of n_tok = 32 * n_warps tokens, one per CTA.
+// Work unit: one (sequence b, strip of kCs = 32 channels).  A cluster of `cluster` CTAs (1 to 16)
+// splits its T tokens into contiguous ranges of n_tok = 32 * n_warps tokens, one per CTA.
 // Inside a CTA warp s owns the span of 32 tokens [32 s, 32 s + 32); its lower half-warp walks the
 // first kL = 16 tokens of the span, its upper half-warp the last 16; lane p of a half-warp owns the
 // channel pair (2p, 2p+1).  A thread walks its 16 tokens sequentially with 64-bit shared accesses
@@ -1366,35 +1366,39 @@ struct Plan {
     int cluster = 0, n_warps = 0, n_tok = 0, segs = 1;
 };
 
+// How many CTAs hold a sequence, and in how many clusters.
+//
+// One cluster (T <= 4096): as few CTAs as hold T, 256 tokens each, then only as many warps as the tokens need.  A CTA's life
+// is a chain whose length hardly depends on its tokens, so the fewest CTAs win, whether their number is a power of two or
+// not (forward / backward us at 131072 tokens, C=768): T=1500 6 CTAs 220 / 544, 8 CTAs 266 / 652; T=3000 12 CTAs 249 / 592,
+// 16 CTAs 301 / 756.  (Powers of two also left CTAs without tokens at T=2049..2400, 2561..2880 and the like, which the
+// tile kernels then served: T=3136 588 / 1453 against 258 / 689.)  Between 3 and 4 CTAs the smaller padding decides, because
+// 3 CTAs of 7 warps share an SM worse than 4 of 5: T=600 244 / 607 against 230 / 565, but T=520 (3 of 6) 257 / 634 against
+// 257 / 652.
+//
+// Several clusters: about 2048 tokens (8 CTAs) each, since clusters of 8 fill more SMs than clusters of 16, up to kMaxSegs of
+// them: T=16384 8 clusters of 8 517 / 1418, 4 of 16 563 / 1618; T=6000 3 of 8 454 / 1177, 2 of 12 464 / 1209; T=4700 2 of 10
+// 449 / 1222, 3 of 7 475 / 1293.  The CTAs of a cluster again follow from the tokens: T=4200 2 of 9 465 / 1217, 2 of 16
+// 626 / 1652.
 static bool make_plan(int T, Plan& pl) {
-    constexpr int kSegMax = kMaxCluster * kMaxWarps * kSpan;      // tokens one cluster holds
-    if (T > kSegMax) {
-        // several clusters per sequence, tokens spread evenly over them
-        const int segs = (T + kSegMax - 1) / kSegMax;
-        if (segs > kMaxSegs) return false;
-        const int per = (T + segs * kMaxCluster - 1) / (segs * kMaxCluster);
-        pl.segs = segs;
-        pl.cluster = kMaxCluster;
-        pl.n_warps = (per + kSpan - 1) / kSpan;
-        pl.n_tok = pl.n_warps * kSpan;
-        return true;
-    }
-    pl.segs = 1;
-    int cluster = 1;
-    while ((T + cluster - 1) / cluster > kMaxWarps * kSpan && cluster < kMaxCluster) cluster *= 2;
-    const int per = (T + cluster - 1) / cluster;
-    if (per > kMaxWarps * kSpan) return false;
-    pl.cluster = cluster;
-    pl.n_warps = (per + kSpan - 1) / kSpan;
+    constexpr int kCtaMax = kMaxWarps * kSpan;              // tokens one CTA holds
+    constexpr int kSegMax = kMaxCluster * kCtaMax;          // tokens one cluster holds
+    const auto up = [](int a, int b) { return (a + b - 1) / b; };
+    const auto warps = [&](int ctas) { return up(up(T, ctas), kSpan); };
+    pl.segs = T <= kSegMax ? 1 : std::max(up(T, kSegMax), std::min(kMaxSegs, (T + 1024) / 2048));
+    if (pl.segs > kMaxSegs) return false;
+    pl.cluster = up(up(T, pl.segs), kCtaMax);
+    if (pl.segs == 1 && pl.cluster == 3 && 4 * warps(4) < 3 * warps(3)) pl.cluster = 4;
+    pl.n_warps = warps(pl.segs * pl.cluster);
     pl.n_tok = pl.n_warps * kSpan;
-    // every CTA of the cluster must own at least one token
-    return static_cast<long long>(cluster - 1) * pl.n_tok < T;
+    // every CTA of a single cluster owns a token, and so does every segment
+    return static_cast<long long>(pl.segs == 1 ? pl.cluster - 1 : (pl.segs - 1) * pl.cluster) * pl.n_tok < T;
 }
 
 struct DeviceState {
     bool probed = false, ok = false;
-    // [segments > 1][tensor types][bwd][log2 cluster][n_warps]: 0 unknown, 1 launchable, -1 not
-    signed char fits[2][3][2][5][kMaxWarps + 1] = {};   // first index: several segments per sequence
+    // [segments > 1][tensor types][bwd][cluster][n_warps]: 0 unknown, 1 launchable, -1 not
+    signed char fits[2][3][2][kMaxCluster + 1][kMaxWarps + 1] = {};   // first index: several segments per sequence
 };
 static std::mutex g_mutex;
 static DeviceState g_dev[64];
@@ -1438,9 +1442,7 @@ static bool fits(const Plan& pl) {
         d.ok = good;
     }
     if (!d.ok) return false;
-    int lg = 0;
-    while ((1 << lg) < pl.cluster) ++lg;
-    signed char& slot = d.fits[pl.segs > 1 ? 1 : 0][static_cast<int>(kTypes)][kBwd ? 1 : 0][lg][pl.n_warps];
+    signed char& slot = d.fits[pl.segs > 1 ? 1 : 0][static_cast<int>(kTypes)][kBwd ? 1 : 0][pl.cluster][pl.n_warps];
     if (slot == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(pl.cluster);
