@@ -42,3 +42,23 @@ def test_host_call_checks_its_arguments(cuda_device):
         biwkv_forward_backward_host(w, u, k.contiguous(), pinned[1], pinned[2], *outs, gwgu, device=cuda_device)
     with pytest.raises(RuntimeError, match="shape"):
         biwkv_forward_backward_host(w, u, pinned[0][:1], pinned[1], pinned[2], *outs, gwgu, device=cuda_device)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grad", [True, False])
+def test_forward_mode_is_refused_and_not_dropped(cuda_device, grad):
+    """The operators have no forward-mode derivative; inputs that carry a tangent are refused, with and without gradients."""
+    import torch.autograd.forward_ad as fwAD
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    from vision_rwkv_b200.vrwkv6 import RUN_CUDA_RWKV6
+    from vision_rwkv_b200.epilogue import relu_square
+    w, k = torch.rand(64, device=cuda_device), torch.randn(1, 8, 64, device=cuda_device)
+    with torch.set_grad_enabled(grad), fwAD.dual_level():
+        dual = fwAD.make_dual(k, torch.ones_like(k))
+        with pytest.raises(RuntimeError):
+            RUN_CUDA(w, w, dual, k)
+        with pytest.raises(RuntimeError):
+            RUN_CUDA_RWKV6(1, 8, 64, 1, k, dual, k, k, w.view(1, 64))
+        if not grad:
+            with pytest.raises(RuntimeError):
+                relu_square(dual)

@@ -12,6 +12,7 @@ Tensor flat(const Tensor& t) {
 }
 void same_place(const Tensor& t, const Tensor& like, const char* name) {
     TORCH_CHECK(t.is_cuda() && t.device() == like.device(), name, " must be on ", like.device());
+    refuse_tangents({&t, &like});
 }
 }  // namespace
 

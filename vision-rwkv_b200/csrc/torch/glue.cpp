@@ -271,6 +271,7 @@ std::vector<Tensor> qshift_mix_half(const Tensor& x, std::vector<Tensor> mixes, 
     TORCH_CHECK(mixes.size() >= 1 && mixes.size() <= 3, "between one and three mix vectors");
     grid_of(x, H, W);
     check_vectors(mixes, x);
+    refuse_tangents({&x});
     const c10::cuda::CUDAGuard guard(x.device());
     return qshift_forward(f32(x), flat_f32(mixes), QShiftArgs{H, W, shift, group, per_head}, true);
 }
@@ -283,6 +284,7 @@ std::vector<Tensor> qshift_ddlerp_half(const Tensor& x, std::vector<Tensor> maas
                 " must be a multiple of 16 that divides C=", x.size(-1));
     const Grid g = grid_of(x, H, W);
     check_vectors(maas, x);
+    refuse_tangents({&x});
     const c10::cuda::CUDAGuard guard(x.device());
     const Tensor xf = f32(x);
     const std::vector<Tensor> flat = flat_f32(maas);

@@ -170,6 +170,7 @@ struct BiWkv : torch::autograd::Function<BiWkv> {
 Tensor biwkv_half(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
     check_biwkv(w, u, k, v);
     TORCH_CHECK(is_bf16(k) && is_bf16(v), "k, v must be bfloat16");
+    refuse_tangents({&w, &u, &k, &v});
     const c10::cuda::CUDAGuard guard(k.device());
     return biwkv_forward_raw(f32(w), f32(u), k.contiguous(), v.contiguous());
 }
@@ -225,6 +226,7 @@ Tensor wkv6_walk(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor
     const int B = r.size(0), T = r.size(1), C = r.size(2), H = C / 64;
     check_wkv6(B, T, C, H, r, k, v, w_, u_);
     TORCH_CHECK(all_bf16({&r, &k, &v}), "r, k, v must be bfloat16");
+    refuse_tangents({&r, &k, &v, &w_, &u_});
     const c10::cuda::CUDAGuard guard(r.device());
     const Tensor w = f32(w_), u = f32(u_), r_ = r.contiguous(), k_ = k.contiguous(), v_ = v.contiguous();
     Tensor y = at::empty({B, T, C}, r.options().dtype(at::kFloat));

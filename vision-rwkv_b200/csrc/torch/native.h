@@ -28,7 +28,15 @@ inline Tensor workspace(size_t bytes, const Tensor& like) {
 inline Tensor f32(const Tensor& t) { return t.scalar_type() == at::kFloat ? t.contiguous() : t.to(at::kFloat).contiguous(); }
 inline float* fp(const Tensor& t) { return static_cast<float*>(t.data_ptr()); }
 inline bool is_bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
+// Forward-mode tangents: the autograd nodes refuse them, and a call that does without a node must not drop them.
+inline bool has_tangent(const Tensor& t) { return t._fw_grad(/*level=*/0).defined(); }
+inline void refuse_tangents(std::initializer_list<const Tensor*> ts) {
+    for (const Tensor* t : ts) TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent(*t), "forward-mode differentiation is not implemented for this operator");
+}
+// whether the call needs its autograd node
 inline bool any_requires_grad(std::initializer_list<const Tensor*> ts) {
+    for (const Tensor* t : ts)
+        if (has_tangent(*t)) return true;
     if (!at::GradMode::is_enabled()) return false;
     for (const Tensor* t : ts)
         if (t->requires_grad()) return true;
