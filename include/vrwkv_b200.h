@@ -141,7 +141,7 @@ int vrwkv_biwkv_backward_bf16(int B, int T, int C, const float* w, const float* 
                               const uint16_t* v, const uint16_t* gy, float* gwgu, uint16_t* gk,
                               uint16_t* gv, void* workspace, size_t workspace_bytes, void* stream);
 /* The same with float32 y and gy, what autograd has when w, u are float32 parameters and k, v come out of autocast
- * (CLS/vrwkv.py:42-44, 56-61 widen y and cast gy there): y holds the bfloat16 result widened, gy is read unrounded.
+ * (CLS/vrwkv.py:42-44, 56-61 widen y and cast gy there): y holds the bfloat16 result widened, gy is rounded to bfloat16 as it is read.
  * T <= 4096; anything outside the cluster-resident kernels returns VRWKV_ERR_UNSUPPORTED before launching. */
 int vrwkv_biwkv_forward_bf16_wide(int B, int T, int C, const float* w, const float* u, const uint16_t* k, const uint16_t* v, float* y,
                                   void* workspace, size_t workspace_bytes, void* stream);

@@ -242,6 +242,7 @@ __device__ __forceinline__ float2 ld_in(const float* area, int i, int pr) {
     }
     return *(reinterpret_cast<const float2*>(area + i * kCs) + pr);
 }
+__device__ __forceinline__ float2 round2(float2 v) { return __bfloat1622float2(__float22bfloat162_rn(v)); }
 template <bool kHalf>
 __device__ __forceinline__ void st_out(float* area, int i, int pr, float2 v) {
     if (kHalf) {
@@ -781,7 +782,7 @@ __device__ __noinline__ void exact_subchunk(const Ctx& c, int sub, int ch, float
 // per sub-chunk; 8: the second half is swept twice, for half the registers).
 // kHalf: k, v, gy and the outputs are bfloat16 tensors (float32 arithmetic and shared-memory state all the same).
 // kWide (with kHalf): y and gy are float32 tensors, what a model with float32 w, u under autocast has; y still holds
-// bfloat16 values, gy is not rounded.  Without it the caller widens y (6 bytes per element) and narrows gy (6 more) in
+// bfloat16 values, and gy is rounded to bfloat16 as it is read: the results are those of the bfloat16 kernel.  Without it the caller widens y (6 bytes per element) and narrows gy (6 more) in
 // passes of their own, as many bytes as this kernel's own forward moves.  B=64, T=576, C=1024, forward + backward:
 // 468 us with those passes, 332 us without (forward alone at B=256, T=196, C=384: 103 and 53 us).
 // kMulti: several clusters per sequence (T above what one cluster holds); compiled apart so that the
@@ -1019,7 +1020,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                     const float2 nn = fma2(c2, zx, add2(P.n, sn[g + j]));
                     const float2 dd = fma2(c2, zy, add2(P.d, sd[g + j]));
                     const float2 y = mul2(nn, f2(rcp(dd.x), rcp(dd.y)));
-                    st_out<kHalfOut>(area_k, i, pr, kHalf && kWide ? __bfloat1622float2(__float22bfloat162_rn(y)) : y);
+                    st_out<kHalfOut>(area_k, i, pr, kHalf && kWide ? round2(y) : y);
                     P.n = fma2(lam2, P.n, zx);
                     P.d = fma2(lam2, P.d, zy);
                 }
@@ -1055,6 +1056,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                     for (int j = 0; j < kGroupB; ++j) {
                         const int i = blk * kStash + g + j;
                         zxs[j] = k2[i * kRow]; zys[j] = v2[i * kRow]; gys[j] = ld_in<kHalfG>(area_g, i, pr);
+                        if (kHalf && kWide) gys[j] = round2(gys[j]);
                     }
                     if (kHalf) __syncwarp();
 #pragma unroll
@@ -1270,6 +1272,7 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 *reinterpret_cast<float2*>(ks + i * kCs) = a;
                 *reinterpret_cast<float2*>(vs + i * kCs) = bb;
                 if (kBwd && kHalfG) *reinterpret_cast<float2*>(gs + i * kCs) = g_;
+                if (kBwd && kWide) *reinterpret_cast<float2*>(gs + i * kCs) = round2(*reinterpret_cast<const float2*>(gs + i * kCs));
                 __syncwarp();
             }
         }
@@ -1284,7 +1287,7 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         if (kHalf && kWide && !kBwd)
             for (int i = 0; i < kL; ++i) {
                 float2* row = reinterpret_cast<float2*>(ks + i * kCs);
-                *row = __bfloat1622float2(__float22bfloat162_rn(*row));
+                *row = round2(*row);
             }
         if (kHalfOut) {
             // narrow the results in place, walking up: dense bfloat16 rows at the start of the area

@@ -35,7 +35,7 @@ namespace resident {
 enum class Types {
     f32,      // every tensor float32
     bf16,     // k, v, y, gy, gk, gv bfloat16
-    wide,     // k, v, gk, gv bfloat16; gy float32; y float32 holding bfloat16 values
+    wide,     // k, v, gk, gv bfloat16; gy float32, rounded as it is read; y float32 holding bfloat16 values
 };
 // True when it can serve this call on the current device.
 bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types);

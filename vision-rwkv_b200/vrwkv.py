@@ -21,7 +21,7 @@ write y / gk / gv as bfloat16 directly with float32 arithmetic inside, instead o
 widen-compute-narrow passes (:34-37, :51-55).  The values are the same wherever the reference
 would itself return bfloat16 (`w` in bfloat16).  With a float32 `w` the reference returns a
 float32 y computed from the bfloat16 inputs; here that y has passed through bfloat16 once
-(relative difference up to 2^-9).  gy is read as float32 for T <= 4096 and rounded to bfloat16 on its way in above.
+(relative difference up to 2^-9).  gy is rounded to bfloat16 on its way in.
 """
 from __future__ import annotations
 
