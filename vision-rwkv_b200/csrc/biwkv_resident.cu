@@ -242,6 +242,8 @@ __device__ __forceinline__ float2 ld_in(const float* area, int i, int pr) {
     }
     return *(reinterpret_cast<const float2*>(area + i * kCs) + pr);
 }
+// w and u are vectors that a caller may have cut out of a larger buffer: 4-byte alignment is all they promise
+__device__ __forceinline__ float2 ld_pair(const float* p) { return f2(__ldg(p), __ldg(p + 1)); }
 __device__ __forceinline__ float2 round2(float2 v) { return __bfloat1622float2(__float22bfloat162_rn(v)); }
 template <bool kHalf>
 __device__ __forceinline__ void st_out(float* area, int i, int pr, float2 v) {
@@ -909,8 +911,8 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     // (relaxed: the mbarrier-init fence above is what publishes the initialisation)
     if (p.cluster > 1) cluster_arrive_relaxed();
     const int ch0 = strip * kCs + 2 * pr;
-    const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
-    const float2 u2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.u + ch0) : f2(0.f, 0.f);
+    const float2 w2 = (ch0 < p.C) ? ld_pair(p.w + ch0) : f2(0.f, 0.f);
+    const float2 u2 = (ch0 < p.C) ? ld_pair(p.u + ch0) : f2(0.f, 0.f);
     const float2 lam2 = *reinterpret_cast<const float2*>(c.consts + kLam * kCs + 2 * pr);
     const float2 wl2 = *reinterpret_cast<const float2*>(c.consts + kWl2 * kCs + 2 * pr);
     const float2 c2 = *reinterpret_cast<const float2*>(c.consts + kCuw * kCs + 2 * pr);
@@ -1259,8 +1261,8 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                     sm100::tma_load_3d(slot_g + sp * kSpan * kCs, &map_g, full, strip * kCs, tok0 + sp * kSpan, b);
         }
         const int ch0 = strip * kCs + 2 * pr;
-        const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
-        const float2 u2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.u + ch0) : f2(0.f, 0.f);
+        const float2 w2 = (ch0 < p.C) ? ld_pair(p.w + ch0) : f2(0.f, 0.f);
+        const float2 u2 = (ch0 < p.C) ? ld_pair(p.u + ch0) : f2(0.f, 0.f);
         if (!sm100::mbar_wait(full, phase, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
         phase ^= 1u;
         if (kHalf) {
