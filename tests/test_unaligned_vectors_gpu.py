@@ -3,7 +3,7 @@ kernel gives the bits it gives for an aligned copy."""
 import pytest
 import torch
 
-from oracle import biwkv_oracle
+from oracle import biwkv_oracle, wkv6_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -33,3 +33,17 @@ def test_biwkv(cuda_device, B, T, C, dtype, k_scale, by):
     want = results(RUN_CUDA, (w, u, k, v), gy)
     got = results(RUN_CUDA, (shifted(w, by), shifted(u, by), k, v), gy)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("by", [1, 2, 3])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_wkv6(cuda_device, dtype, by):
+    from vision_rwkv_b200.vrwkv6 import RUN_CUDA_RWKV6, inference_rwkv6
+    B, T, H = 2, 70, 3
+    r, k, v, w, u, gy = (x.float().to(cuda_device) for x in wkv6_oracle.make_inputs(B, T, 64 * H, H, seed=1))
+    r, k, v = (x.to(dtype) for x in (r, k, v))
+    run = lambda *xs: RUN_CUDA_RWKV6(B, T, 64 * H, H, *xs)
+    want, got = results(run, (r, k, v, w, u), gy), results(run, (r, k, v, w, shifted(u, by)), gy)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    with torch.no_grad():
+        assert torch.equal(inference_rwkv6(B, T, 64 * H, H, r, k, v, w, shifted(u, by)), inference_rwkv6(B, T, 64 * H, H, r, k, v, w, u))

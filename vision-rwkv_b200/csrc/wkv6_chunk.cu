@@ -1077,9 +1077,19 @@ static int chunks_of(int T) { return (T + kChunk - 1) / kChunk; }
 static size_t state_plane(int B, int T, int H, int parts) {      // uint4 per (pair, direction)
     return static_cast<size_t>(B) * H * chunks_of(T) * parts * (kStateWords / 4);
 }
-size_t forward_workspace(int B, int T, int H, bool exact) { return 256 + 2 * state_plane(B, T, H, exact ? 3 : 1) * sizeof(uint4); }
+// status word, a copy of u, states (and the parts of gu)
+static size_t states_offset(int H) { return 256 + static_cast<size_t>(H) * N * sizeof(float); }
+size_t forward_workspace(int B, int T, int H, bool exact) { return states_offset(H) + 2 * state_plane(B, T, H, exact ? 3 : 1) * sizeof(uint4); }
 size_t backward_workspace(int B, int T, int H, bool exact) {
-    return 256 + 4 * state_plane(B, T, H, exact ? 3 : 2) * sizeof(uint4) + static_cast<size_t>(B) * chunks_of(T) * H * N * sizeof(float);
+    return states_offset(H) + 4 * state_plane(B, T, H, exact ? 3 : 2) * sizeof(uint4) + static_cast<size_t>(B) * chunks_of(T) * H * N * sizeof(float);
+}
+// The kernels read u four floats at a time.  A u that starts elsewhere (a view into a parameter buffer) goes through a copy:
+// scalar loads in the kernels, or a branch, cost every call 0.5 to 1 %.
+static const float* aligned_bonus(const float* u, int H, void* workspace, cudaStream_t stream) {
+    if ((reinterpret_cast<uintptr_t>(u) & 15u) == 0) return u;
+    float* copy = reinterpret_cast<float*>(static_cast<char*>(workspace) + 256);
+    cudaMemcpyAsync(copy, u, static_cast<size_t>(H) * N * sizeof(float), cudaMemcpyDeviceToDevice, stream);
+    return copy;
 }
 
 // dynamic shared memory above 48 KB is a per-device attribute of each kernel: set the first time the kernel meets the device
@@ -1127,7 +1137,7 @@ static bool run_states(int B, int T_, int H, const void* r, const void* k, const
 template <typename T, int kZ, int kX>
 static int run_forward(int B, int T_, int H, const void* r, const void* k, const void* v, const float* w, const float* u, float* y,
                        void* workspace, cudaStream_t stream) {
-    uint4* states = reinterpret_cast<uint4*>(static_cast<char*>(workspace) + 256);
+    uint4* states = reinterpret_cast<uint4*>(static_cast<char*>(workspace) + states_offset(H));
     const size_t plane = state_plane(B, T_, H, kX);
     const int n_chunks = chunks_of(T_);
     int launched = 1;
@@ -1135,7 +1145,7 @@ static int run_forward(int B, int T_, int H, const void* r, const void* k, const
         if (!run_states<T, T, kZ, kX, false>(B, T_, H, nullptr, k, v, w, nullptr, states, plane, workspace, stream)) return -1;
         ++launched;
     }
-    OutArgs o{T_, H, n_chunks, r, k, v, w, u, y, unaligned16({y}), states, plane};
+    OutArgs o{T_, H, n_chunks, r, k, v, w, aligned_bonus(u, H, workspace, stream), y, unaligned16({y}), states, plane};
     const auto kernel = wkv6_forward_kernel<T, kZ, kX>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), forward_smem(kZ, kX))) return -1;
     kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, forward_smem(kZ, kX), stream>>>(o);
@@ -1145,7 +1155,7 @@ static int run_forward(int B, int T_, int H, const void* r, const void* k, const
 template <typename T, typename G, typename O, int kZ, int kX, int kP>
 static int run_backward(int B, int T_, int H, const void* r, const void* k, const void* v, const float* w, const float* u, const void* gy,
                         void* gr, void* gk, void* gv, float* gw, float* gu, void* workspace, cudaStream_t stream) {
-    uint4* states = reinterpret_cast<uint4*>(static_cast<char*>(workspace) + 256);
+    uint4* states = reinterpret_cast<uint4*>(static_cast<char*>(workspace) + states_offset(H));
     const size_t plane = state_plane(B, T_, H, kX);
     const int n_chunks = chunks_of(T_), C = H * N;
     int launched = 2;
@@ -1154,7 +1164,7 @@ static int run_backward(int B, int T_, int H, const void* r, const void* k, cons
         ++launched;
     }
     float* gu_part = reinterpret_cast<float*>(states + 4 * plane);
-    GradArgs o{T_, H, n_chunks, r, k, v, gy, w, u, gr, gk, gv, gw, gu_part, unaligned16({gr, gk, gv, gw}), states, plane};
+    GradArgs o{T_, H, n_chunks, r, k, v, gy, w, aligned_bonus(u, H, workspace, stream), gr, gk, gv, gw, gu_part, unaligned16({gr, gk, gv, gw}), states, plane};
     const auto kernel = wkv6_backward_kernel<T, G, O, kZ, kX, kP>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), backward_smem(kZ, kX, kP))) return -1;
     kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, backward_smem(kZ, kX, kP), stream>>>(o);
