@@ -176,16 +176,16 @@ int vrwkv_biwkv_forward_f32_noalloc(int B, int T, int C, const float* w, const f
  *   cuda_forward(int B,int T,int C,int H,float*r,float*k,float*v,float*w,float*u,float*y)
  *       CLS/cuda_v6/wkv6_op.cpp:4,7-9 (kernel CLS/cuda_v6/wkv6_cuda.cu:6-97,348-353)
  * It takes the raw decay input and forms -exp(w_raw) itself, where the reference's Python
- * wrapper does that in a separate pass (CLS/vrwkv6.py:48).  It needs no scratch memory and walks the
- * sequence token by token; vrwkv_wkv6_forward is several times faster.
+ * wrapper does that in a separate pass (CLS/vrwkv6.py:48).  It needs no scratch memory.
  */
 int vrwkv_wkv6_forward_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
                            const float* w_raw, const float* u, float* y, void* stream);
 
-/* vrwkv_wkv6_forward: the same forward in 64-token chunks on the tensor cores (the states that enter each chunk,
- * then all chunks in parallel).  exact = 1: float32 r, k, v and float32 accuracy.  exact = 0: r, k, v enter the matrix
- * products as bfloat16 (in_bf16 = 1: they are bfloat16 bit patterns and are read as such; 0: float32, rounded on the
- * way in), sums are fp32; results agree with exact = 1 to about 1e-2 of max|y|.  w_raw, u and y are float32.
+/* vrwkv_wkv6_forward.  exact = 1: float32 r, k, v and the kernels of vrwkv_wkv6_forward_f32; the workspace is a status
+ * word.  exact = 0: 64-token chunks on the tensor cores (the states that enter each chunk, then all chunks in parallel):
+ * r, k, v enter the matrix products as bfloat16 (in_bf16 = 1: they are bfloat16 bit patterns and are read as such; 0:
+ * float32, rounded on the way in), sums are fp32; results agree with exact = 1 to about 1e-2 of max|y|.  w_raw, u and y are
+ * float32.
  * Replaces the same reference entry point, and with in_bf16 the `.float()` passes in front of the reference's call
  * (CLS/vrwkv6.py:220 hands whatever dtype the projections produced to a kernel that reads float). */
 size_t vrwkv_wkv6_forward_workspace_bytes(int B, int T, int C, int H, int exact);

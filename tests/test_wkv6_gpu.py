@@ -51,6 +51,39 @@ def test_parity_with_oracle(cuda_device, B, T, H):
     assert all(e <= TOL for e in errs.values()), errs
 
 
+def strong_tokens(B, T, H, seed, levels=(4.0, 8.0, 12.0, 30.0, 100.0), round_to=None):
+    """Mild inputs with single tokens that forget much or everything: in every channel, and in every third channel only."""
+    r, k, v, w, u, gy = O.make_inputs(B, T, 64 * H, H, seed=seed, round_to=round_to)
+    w = w.clone()
+    for i, level in enumerate(levels):
+        w[:, 3 + 11 * i::61] = level
+        w[:, 8 + 11 * i::61, ::3] = level
+    return r, k, v, w, u, gy
+
+
+# a gradient of w_raw is -exp(w_raw) times a difference of sums: what the kernels are measured by is that difference, and it is
+# zero where the decay is (exp(-exp(w_raw)) in float32)
+def check_decay_gradient(gw, ref, w, tol):
+    e = w.float().exp().double()
+    alive = (-w.float().exp()).exp() > 0
+    assert torch.isfinite(gw).all()
+    assert (gw.cpu()[~alive] == 0).all()
+    scale = torch.where(alive, 1 / e, torch.zeros_like(e))
+    clean = torch.where(alive, ref, torch.zeros_like(ref))
+    assert rel_err(gw.double().cpu() * scale, clean * scale) <= tol
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 40, 1), (2, 100, 2), (1, 333, 1)])
+def test_a_token_that_forgets_everything_leaves_the_others_exact(cuda_device, B, T, H):
+    args = strong_tokens(B, T, H, seed=T)
+    got, ref = run_gpu(cuda_device, *args, H), reference(*args, H)
+    for name, g, rf in zip(NAMES, got, ref):
+        if name == "gw":
+            check_decay_gradient(g, rf, args[3], TOL)
+        else:
+            assert rel_err(g.reshape(rf.shape), rf) <= TOL, name
+
+
 @pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(GOLDEN, "wkv6_*.npz"))))
 def test_golden_vectors(cuda_device, path):
     z = np.load(path)

@@ -311,12 +311,12 @@ static inline bool misaligned16(const void* p) { return (reinterpret_cast<uintpt
 
 size_t vrwkv_wkv6_backward_workspace_bytes(int B, int T, int C, int H) {
     if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
-    return wkv6c::backward_workspace(B, T, H, true);
+    return wkv6::backward_workspace(B, T, H);
 }
 
 size_t vrwkv_wkv6_forward_workspace_bytes(int B, int T, int C, int H, int exact) {
     if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
-    return wkv6c::forward_workspace(B, T, H, exact != 0);
+    return exact ? 256 : wkv6c::forward_workspace(B, T, H);      // exact: the status word
 }
 
 int vrwkv_wkv6_forward(int B, int T, int C, int H, const void* r, const void* k, const void* v, int in_bf16, int exact,
@@ -327,10 +327,13 @@ int vrwkv_wkv6_forward(int B, int T, int C, int H, const void* r, const void* k,
     if (misaligned16(r) || misaligned16(k) || misaligned16(v) || misaligned16(w_raw) || misaligned4(u) || misaligned4(y) ||
         (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < wkv6c::forward_workspace(B, T, H, exact != 0)) return VRWKV_ERR_WORKSPACE;
+    if (workspace_bytes < vrwkv_wkv6_forward_workspace_bytes(B, T, C, H, exact)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
-    return finish(wkv6c::forward(B, T, H, r, k, v, w_raw, u, y, in_bf16 != 0, exact != 0, workspace, s));
+    if (exact)
+        return finish(wkv6::forward(B, T, H, static_cast<const float*>(r), static_cast<const float*>(k), static_cast<const float*>(v), w_raw, u,
+                                    y, s));
+    return finish(wkv6c::forward(B, T, H, r, k, v, w_raw, u, y, in_bf16 != 0, workspace, s));
 }
 
 int vrwkv_wkv6_forward_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
@@ -352,7 +355,7 @@ int vrwkv_wkv6_forward_tc_f32(int B, int T, int C, int H, const float* r, const 
         misaligned16(y) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < 256) return VRWKV_ERR_WORKSPACE;
-    if (g_path.load() != 1 && workspace_bytes >= wkv6c::forward_workspace(B, T, H, false))
+    if (g_path.load() != 1 && workspace_bytes >= wkv6c::forward_workspace(B, T, H))
         return vrwkv_wkv6_forward(B, T, C, H, r, k, v, 0, 0, w_raw, u, y, workspace, workspace_bytes, stream);
     return finish(wkv6tc::forward(B, T, H, r, k, v, w_raw, u, y, static_cast<unsigned*>(workspace), static_cast<cudaStream_t>(stream)));
 }
@@ -366,7 +369,7 @@ int vrwkv_wkv6_forward_tc_bf16(int B, int T, int C, int H, const uint16_t* r, co
         misaligned16(y) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < 256) return VRWKV_ERR_WORKSPACE;
-    if (g_path.load() != 1 && workspace_bytes >= wkv6c::forward_workspace(B, T, H, false))
+    if (g_path.load() != 1 && workspace_bytes >= wkv6c::forward_workspace(B, T, H))
         return vrwkv_wkv6_forward(B, T, C, H, r, k, v, 1, 0, w_raw, u, y, workspace, workspace_bytes, stream);
     return finish(wkv6tc::forward_bf16in(B, T, H, r, k, v, w_raw, u, y, static_cast<unsigned*>(workspace),
                                          static_cast<cudaStream_t>(stream)));
@@ -384,15 +387,20 @@ static int wkv6_backward(int B, int T, int C, int H, const void* r, const void* 
         return VRWKV_ERR_ALIGNMENT;
     for (const void* p : {static_cast<const void*>(gr), static_cast<const void*>(gk), static_cast<const void*>(gv)})
         if (reinterpret_cast<uintptr_t>(p) & (out_bf16 ? 1u : 3u)) return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < wkv6c::backward_workspace(B, T, H, exact)) return VRWKV_ERR_WORKSPACE;
+    if (workspace_bytes < (exact ? wkv6::backward_workspace(B, T, H) : wkv6c::backward_workspace(B, T, H))) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
-    return finish(wkv6c::backward(B, T, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, in_bf16, gy_bf16, out_bf16, exact, workspace, s));
+    if (exact) {
+        const auto in = [](const void* p) { return static_cast<const float*>(p); };
+        const auto out = [](void* p) { return static_cast<float*>(p); };
+        return finish(wkv6::backward(B, T, H, in(r), in(k), in(v), w_raw, u, in(gy), out(gr), out(gk), out(gv), gw, gu, workspace, s));
+    }
+    return finish(wkv6c::backward(B, T, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, in_bf16, gy_bf16, out_bf16, workspace, s));
 }
 
 size_t vrwkv_wkv6_backward_bytes(int B, int T, int C, int H, int exact) {
     if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
-    return wkv6c::backward_workspace(B, T, H, exact != 0);
+    return exact ? wkv6::backward_workspace(B, T, H) : wkv6c::backward_workspace(B, T, H);
 }
 
 int vrwkv_wkv6_backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, int in_bf16, int exact,
@@ -412,7 +420,7 @@ int vrwkv_wkv6_backward_f32(int B, int T, int C, int H, const float* r, const fl
 
 size_t vrwkv_wkv6_backward_tc_workspace_bytes(int B, int T, int C, int H) {
     if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
-    return wkv6c::backward_workspace(B, T, H, false);
+    return wkv6c::backward_workspace(B, T, H);
 }
 
 int vrwkv_wkv6_backward_tc_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,

@@ -78,9 +78,13 @@ int backward_bf16(int B, int T, int C, const float* w, const float* u, const voi
 }  // namespace biwkv
 
 namespace wkv6 {
-// float32 forward without scratch memory (wkv6_sweeps.cu)
+// float32 state sweeps (wkv6_sweeps.cu); gv may be null
 int forward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
             const float* u, float* y, cudaStream_t stream);
+size_t backward_workspace(int B, int T, int H);
+int backward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
+             const float* u, const float* gy, float* gr, float* gk, float* gv, float* gw, float* gu,
+             void* workspace, cudaStream_t stream);
 }  // namespace wkv6
 
 namespace wkv6tc {
@@ -93,14 +97,13 @@ int forward_bf16in(int B, int T, int H, const void* r, const void* k, const void
 }  // namespace wkv6tc
 
 namespace wkv6c {
-// Chunked tensor-core kernels (wkv6_chunk.cu).  exact: float32 tensors, float32 accuracy; else bfloat16 operands
-// (r, k, v, gy in bfloat16, or float32 rounded on the way in), scaled operands of gr, gk, gw carried to 16 bits.
-// gv may be null.
-size_t forward_workspace(int B, int T, int H, bool exact);
-size_t backward_workspace(int B, int T, int H, bool exact);
+// Chunked tensor-core kernels (wkv6_chunk.cu): bfloat16 operands (r, k, v, gy in bfloat16, or float32 rounded on the way
+// in), scaled operands of gr, gk, gw carried to 16 bits.  gv may be null.
+size_t forward_workspace(int B, int T, int H);
+size_t backward_workspace(int B, int T, int H);
 int forward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, float* y,
-            bool bf16_in, bool exact, void* workspace, cudaStream_t stream);
+            bool bf16_in, void* workspace, cudaStream_t stream);
 int backward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, const void* gy,
-             void* gr, void* gk, void* gv, float* gw, float* gu, bool bf16_in, bool gy_bf16, bool bf16_out, bool exact,
-             void* workspace, cudaStream_t stream);
+             void* gr, void* gk, void* gv, float* gw, float* gu, bool bf16_in, bool gy_bf16, bool bf16_out, void* workspace,
+             cudaStream_t stream);
 }  // namespace wkv6c

@@ -88,8 +88,8 @@ __device__ __forceinline__ void scale_chunk(const float* wt, const XT* xt, const
     for (int t = 0; t < kBlock; ++t) {
         const float2 w = *reinterpret_cast<const float2*>(wt + (row0 + t) * N + 2 * lane);
         if (row0 + t < valid) {
-            run.x += log2_decay<(kX > 2)>(w.x);
-            run.y += log2_decay<(kX > 2)>(w.y);
+            run.x += log2_decay(w.x);
+            run.y += log2_decay(w.y);
         }
         sum[t] = run;
     }
@@ -108,7 +108,7 @@ __device__ __forceinline__ void scale_chunk(const float* wt, const XT* xt, const
         Pair<ZT> zr;
         xr.lds(xt + (row0 + t) * N + 2 * lane);
         zr.lds(zt + (row0 + t) * N + 2 * lane);
-        const float2 xv = round2<(kX < 3 && sizeof(XT) == 4)>(xr.get()), zv = round2<(kZ < 3 && sizeof(ZT) == 4)>(zr.get());
+        const float2 xv = round2<sizeof(XT) == 4>(xr.get()), zv = round2<sizeof(ZT) == 4>(zr.get());
         const float2 prev = t > 0 ? sum[t > 0 ? t - 1 : 0] : make_float2(0.f, 0.f);
         const float ex = dir == 0 ? edge.x - sum[t].x : edge.x + prev.x, ey = dir == 0 ? edge.y - sum[t].y : edge.y + prev.y;
         col_store<kX>(xs, row0 + t, word, xv.x * ex2(ex), xv.y * ex2(ey));
@@ -449,7 +449,6 @@ __device__ __forceinline__ void bonus_terms(const Block& x, const Block& y, cons
     }
 }
 // sums of l over a block's tokens into the table (a warp per block, lane = two channels)
-template <bool kAccurate>
 __device__ __forceinline__ void scan_block(Table& tab, const float* w, int C, int rows, int blk, int lane) {
     Pair<float> wr[kBlock];
 #pragma unroll
@@ -458,8 +457,8 @@ __device__ __forceinline__ void scan_block(Table& tab, const float* w, int C, in
 #pragma unroll
     for (int t = 0; t < kBlock; ++t) {
         if (t < rows) {
-            run.x += log2_decay<kAccurate>(wr[t].v.x);
-            run.y += log2_decay<kAccurate>(wr[t].v.y);
+            run.x += log2_decay(wr[t].v.x);
+            run.y += log2_decay(wr[t].v.y);
         }
         *reinterpret_cast<float2*>(&tab[blk * kBlock + t][2 * lane]) = run;
     }
@@ -650,7 +649,7 @@ struct OutArgs {
 
 // kX parts of the scaled operands and states, kZ parts of v
 template <typename T, int kZ, int kX>
-__global__ void __launch_bounds__(256, kX == 1 ? 3 : 1) wkv6_forward_kernel(const OutArgs a) {
+__global__ void __launch_bounds__(256, 3) wkv6_forward_kernel(const OutArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __nv_bfloat16* kf = reinterpret_cast<__nv_bfloat16*>(smem);       // k towards the right edge of its block, left edge behind it
     __nv_bfloat16* pairs = kf + 2 * kX * kPlane;
@@ -661,7 +660,7 @@ __global__ void __launch_bounds__(256, kX == 1 ? 3 : 1) wkv6_forward_kernel(cons
     const int n = blockIdx.x % a.n_chunks, bh = blockIdx.x / a.n_chunks;
     const int b = bh / a.H, h = bh - b * a.H, C = a.H * N;
     const size_t base = (static_cast<size_t>(b) * a.T + n * kChunk) * C + static_cast<size_t>(h) * N;
-    constexpr bool kRound = kX < 3 && sizeof(T) == 4;
+    constexpr bool kRound = sizeof(T) == 4;
     {
         const int blk = warp & 3, dir = warp >> 2;
         const int rows = a.T - (n * kChunk + blk * kBlock);
@@ -670,7 +669,7 @@ __global__ void __launch_bounds__(256, kX == 1 ? 3 : 1) wkv6_forward_kernel(cons
         __nv_bfloat16* planes = kf + dir * kX * kPlane;
         Pair<T> kr[kBlock];
         load_rows<T>(kr, k, C, rows, lane);
-        if (dir == 0) scan_block<(kX > 2)>(tab, a.w + at0, C, rows, blk, lane);
+        if (dir == 0) scan_block(tab, a.w + at0, C, rows, blk, lane);
         else stage_rows<T, kZ, kRound>(vs, static_cast<const T*>(a.v) + at0, C, rows, blk, lane);
         __syncthreads();
         stage_scaled<T, kX, kRound>(planes, kr, tab, blk, dir, lane);
@@ -821,7 +820,7 @@ __device__ __forceinline__ void slice_gradient(float (&out)[2][2][2][4], const _
 
 // kZ parts of v, gy; kX parts of scaled operands, token products and states; kP parts where only gv is concerned
 template <typename T, typename G, typename O, int kZ, int kX, int kP>
-__global__ void __launch_bounds__(256, kX < 3 ? 2 : 1) wkv6_backward_kernel(const GradArgs a) {
+__global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __nv_bfloat16* vs = reinterpret_cast<__nv_bfloat16*>(smem);
     __nv_bfloat16* gs = vs + kZ * kPlane;
@@ -840,7 +839,7 @@ __global__ void __launch_bounds__(256, kX < 3 ? 2 : 1) wkv6_backward_kernel(cons
     const int tokens = a.T - n * kChunk, rows = tokens - blk * kBlock;
     const size_t base = (static_cast<size_t>(b) * a.T + n * kChunk) * C + static_cast<size_t>(h) * N;
     const size_t at0 = base + static_cast<size_t>(blk) * kBlock * C;
-    constexpr bool kRound = kX < 3 && sizeof(T) == 4, kRoundG = kX < 3 && sizeof(G) == 4;
+    constexpr bool kRound = sizeof(T) == 4, kRoundG = sizeof(G) == 4;
     constexpr int kState = kX * kStateWords / 4;
     // states entering this chunk, [pair (k v | r gy)][from the left | from the right]
     const uint4* st = a.states + (static_cast<size_t>(bh) * a.n_chunks + n) * kState;
@@ -853,7 +852,7 @@ __global__ void __launch_bounds__(256, kX < 3 ? 2 : 1) wkv6_backward_kernel(cons
     Pair<T> col[kBlock];
     load_rows<T>(col, kp + at0, C, rows, lane);
     if (dir == 0) {
-        scan_block<(kX > 2)>(tab, a.w + at0, C, rows, blk, lane);
+        scan_block(tab, a.w + at0, C, rows, blk, lane);
     } else {
         stage_rows<T, kZ, kRound>(vs, static_cast<const T*>(a.v) + at0, C, rows, blk, lane);
         stage_rows<G, kZ, kRoundG>(gs, static_cast<const G*>(a.gy) + at0, C, rows, blk, lane);
@@ -985,10 +984,11 @@ __global__ void __launch_bounds__(256, kX < 3 ? 2 : 1) wkv6_backward_kernel(cons
     }
     __syncthreads();               // m has been read
     if (a.gv != nullptr) {
-        // gv: rows are k, columns r, values gy: the forward with exchanged roles.  Its edge planes take the room of the
-        // scaled rows' second parts where gv needs only the first, else that of v and one more set of planes.
-        __nv_bfloat16* e0 = kX > kP ? pf + kP * kPlane : vs;
-        __nv_bfloat16* e1 = kX > kP ? pf + (kX + kP) * kPlane : reinterpret_cast<__nv_bfloat16*>(seg + 8 * N);
+        // gv: rows are k, columns r, values gy: the forward with exchanged roles.  It needs only the first part of the scaled
+        // rows; its edge planes take the room of the second.
+        static_assert(kX > kP, "no room for the edge planes");
+        __nv_bfloat16* e0 = pf + kP * kPlane;
+        __nv_bfloat16* e1 = pf + (kX + kP) * kPlane;
         pair_rows<T, kP, kRound>(kp + at0, rp + at0, a.u + h * N, tab, pf + dir * kX * kPlane, ms, dir ? e1 : e0, C, rows, blk, dir, lane);
         __syncthreads();
         float y[2][2][4];
@@ -1041,8 +1041,8 @@ __global__ void __launch_bounds__(256, kX < 3 ? 2 : 1) wkv6_backward_kernel(cons
             if (t0 + t < tokens) {
                 const size_t o = o0 + static_cast<size_t>(t) * C;
                 const float2 w = __ldg(reinterpret_cast<const float2*>(a.w + o));
-                const float gx = (later.x + d[t].x) * (kX > 2 ? -expf(w.x) : -ex2(w.x * kLog2e));
-                const float gz = (later.y + d[t].y) * (kX > 2 ? -expf(w.y) : -ex2(w.y * kLog2e));
+                const float gx = (later.x + d[t].x) * -ex2(w.x * kLog2e);
+                const float gz = (later.y + d[t].y) * -ex2(w.y * kLog2e);
                 if (!a.scalar) *reinterpret_cast<float2*>(a.gw + o) = make_float2(gx, gz);
                 else { a.gw[o] = gx; a.gw[o + 1] = gz; }
             }
@@ -1069,8 +1069,8 @@ __global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, cons
 
 // ---- host side -------------------------------------------------------------------------------------------------
 static size_t forward_smem(int kz, int kx) { return static_cast<size_t>(kz + 5 * kx) * kPlane * 2 + sizeof(Table); }
-static size_t backward_smem(int kz, int kx, int kp) {
-    return static_cast<size_t>(2 * kz + 3 * kx + (kx > kp ? 0 : kp)) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 8) * N * sizeof(float);
+static size_t backward_smem(int kz, int kx) {
+    return static_cast<size_t>(2 * kz + 3 * kx) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 8) * N * sizeof(float);
 }
 
 static int chunks_of(int T) { return (T + kChunk - 1) / kChunk; }
@@ -1079,9 +1079,9 @@ static size_t state_plane(int B, int T, int H, int parts) {      // uint4 per (p
 }
 // status word, a copy of u, states (and the parts of gu)
 static size_t states_offset(int H) { return 256 + static_cast<size_t>(H) * N * sizeof(float); }
-size_t forward_workspace(int B, int T, int H, bool exact) { return states_offset(H) + 2 * state_plane(B, T, H, exact ? 3 : 1) * sizeof(uint4); }
-size_t backward_workspace(int B, int T, int H, bool exact) {
-    return states_offset(H) + 4 * state_plane(B, T, H, exact ? 3 : 2) * sizeof(uint4) + static_cast<size_t>(B) * chunks_of(T) * H * N * sizeof(float);
+size_t forward_workspace(int B, int T, int H) { return states_offset(H) + 2 * state_plane(B, T, H, 1) * sizeof(uint4); }
+size_t backward_workspace(int B, int T, int H) {
+    return states_offset(H) + 4 * state_plane(B, T, H, 2) * sizeof(uint4) + static_cast<size_t>(B) * chunks_of(T) * H * N * sizeof(float);
 }
 // The kernels read u four floats at a time.  A u that starts elsewhere (a view into a parameter buffer) goes through a copy:
 // scalar loads in the kernels, or a branch, cost every call 0.5 to 1 %.
@@ -1166,25 +1166,23 @@ static int run_backward(int B, int T_, int H, const void* r, const void* k, cons
     float* gu_part = reinterpret_cast<float*>(states + 4 * plane);
     GradArgs o{T_, H, n_chunks, r, k, v, gy, w, aligned_bonus(u, H, workspace, stream), gr, gk, gv, gw, gu_part, unaligned16({gr, gk, gv, gw}), states, plane};
     const auto kernel = wkv6_backward_kernel<T, G, O, kZ, kX, kP>;
-    if (!allow_smem(reinterpret_cast<const void*>(kernel), backward_smem(kZ, kX, kP))) return -1;
-    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, backward_smem(kZ, kX, kP), stream>>>(o);
+    if (!allow_smem(reinterpret_cast<const void*>(kernel), backward_smem(kZ, kX))) return -1;
+    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, backward_smem(kZ, kX), stream>>>(o);
     wkv6_bonus_kernel<<<C / 32, dim3(32, 32), 0, stream>>>(B * n_chunks, C, gu_part, gu);
     return launched;
 }
 
 int forward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, float* y, bool bf16_in,
-            bool exact, void* workspace, cudaStream_t stream) {
-    if (exact) return run_forward<float, 3, 3>(B, T, H, r, k, v, w, u, y, workspace, stream);
+            void* workspace, cudaStream_t stream) {
     return bf16_in ? run_forward<__nv_bfloat16, 1, 1>(B, T, H, r, k, v, w, u, y, workspace, stream)
                    : run_forward<float, 1, 1>(B, T, H, r, k, v, w, u, y, workspace, stream);
 }
 
 int backward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, const void* gy, void* gr,
-             void* gk, void* gv, float* gw, float* gu, bool bf16_in, bool gy_bf16, bool bf16_out, bool exact, void* workspace,
+             void* gk, void* gv, float* gw, float* gu, bool bf16_in, bool gy_bf16, bool bf16_out, void* workspace,
              cudaStream_t stream) {
     typedef __nv_bfloat16 H16;
 #define RUN(T_, G_, O_, Z_, X_, P_) run_backward<T_, G_, O_, Z_, X_, P_>(B, T, H, r, k, v, w, u, gy, gr, gk, gv, gw, gu, workspace, stream)
-    if (exact) return RUN(float, float, float, 3, 3, 3);
     if (!bf16_in) return RUN(float, float, float, 1, 2, 1);
     if (gy_bf16) return bf16_out ? RUN(H16, H16, H16, 1, 2, 1) : RUN(H16, H16, float, 1, 2, 1);
     return bf16_out ? RUN(H16, float, H16, 1, 2, 1) : RUN(H16, float, float, 1, 2, 1);

@@ -14,8 +14,8 @@
 // memory as rows of 64 "positions" (position 16 kk + 8 h + 2 q + e holds channel 16 kk + 4 q + 2 h + e) that
 // ldmatrix.trans reads in the right order.
 //
-// Precision.  A value enters a product as a sum of NS bfloat16 numbers (1: rounded; 2: 16 bits; 3: all 24 bits
-// of a float), and the products of parts whose error would be kept are accumulated in float32.
+// Precision.  A value enters a product as a sum of NS bfloat16 numbers (1: rounded; 2: 16 bits), and the products of
+// parts whose error would be kept are accumulated in float32.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -107,20 +107,6 @@ struct AFrag {
     __device__ __forceinline__ void set(const Block& x) {
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) set(kk, x[0][kk], x[1][kk]);
-    }
-};
-// A fragment (one k-step) of a 16 x 16 token-by-token matrix held as two C fragments
-template <int NS>
-struct TFrag {
-    uint32_t w[NS][4];
-    __device__ __forceinline__ void set(const float (&c)[2][4]) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uint32_t t[NS];
-            split<NS>(c[i >> 1][(i & 1) * 2], c[i >> 1][(i & 1) * 2 + 1], t);
-#pragma unroll
-            for (int s = 0; s < NS; ++s) w[s][i] = t[s];
-        }
     }
 };
 
@@ -308,7 +294,6 @@ __device__ __forceinline__ float2 round2(float2 x) {
     return kRound ? make_float2(__bfloat162float(__float2bfloat16(x.x)), __bfloat162float(__float2bfloat16(x.y))) : x;
 }
 // log2 of a token's decay
-template <bool kAccurate>
-__device__ __forceinline__ float log2_decay(float w) { return -kLog2e * (kAccurate ? expf(w) : ex2(w * kLog2e)); }
+__device__ __forceinline__ float log2_decay(float w) { return -kLog2e * ex2(w * kLog2e); }
 
 }  // namespace wkv6c
