@@ -151,6 +151,31 @@ def test_autograd_surface(cuda_device):
         RUN_CUDA_RWKV6(B, T, C, H, xs[0].transpose(0, 1), *xs[1:])
 
 
+@pytest.mark.parametrize("B,T,H", [(1, 40, 1), (2, 100, 2), (1, 333, 1)])
+def test_bf16_inputs_around_a_token_that_forgets_everything(cuda_device, B, T, H):
+    """The decays of the bfloat16 kernels are good to 1e-4 around such tokens: what is left is the operands' rounding."""
+    from vision_rwkv_b200 import ops, vrwkv6
+    args = strong_tokens(B, T, H, seed=T, round_to=torch.bfloat16)
+    ref = reference(*args, H)
+    r, k, v, gy = (args[i].bfloat16().to(cuda_device) for i in (0, 1, 2, 5))
+    w, u = args[3].float().to(cuda_device), args[4].float().to(cuda_device)
+    xs = [x.clone().requires_grad_(True) for x in (r, k, v, w, u)]
+    y = vrwkv6.RUN_CUDA_RWKV6(B, T, 64 * H, H, *xs)
+    grads = torch.autograd.grad(y, xs, gy.float())
+    for name, g, rf in zip(NAMES, (y, *grads), ref):
+        if name == "gw":
+            check_decay_gradient(g, rf, args[3], 1e-2)
+        else:
+            assert rel_err(g.float().reshape(rf.shape), rf) <= 1e-2, name
+    # float32 gradients of the same inputs: the scaled operands are carried to 16 bits
+    fine = ops.wkv6_backward(r, k, v, w, u, gy, H, tensor_cores=True)
+    for name, g, rf, tol in zip(NAMES[1:], fine, ref[1:], (5e-4, 5e-4, 1e-2, None, 5e-4)):
+        if tol is not None:
+            assert rel_err(g.reshape(rf.shape), rf) <= tol, name
+    with torch.no_grad():
+        assert rel_err(vrwkv6.inference_rwkv6(B, T, 64 * H, H, r, k, v, w, u), ref[0]) <= 1e-2
+
+
 def test_bf16_inputs(cuda_device):
     from vision_rwkv_b200.vrwkv6 import RUN_CUDA_RWKV6
     B, T, H = 2, 196, 2

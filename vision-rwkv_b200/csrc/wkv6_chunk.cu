@@ -18,11 +18,12 @@
 // operands, scalings and masks in registers, where tcgen05 would stage each through shared memory and tensor memory for
 // a product that takes 30 cycles.  The chunk length trades state traffic (1 / length) against pairs inside the chunk.
 //
-// Stability.  No exponent is positive except inside 16-token blocks: block b's tokens are scaled towards the block's edges
-// (2^(<= 0)), and a block further away takes the decay across the blocks in between as one more factor <= 1, so nothing
-// overflows however strong the decay is.  Inside a block the pairs are split at its middle token, which needs
-// 2^(8 tokens' decay) on one side; where a channel exceeds 2^kSafe there, the block takes its pairs in four levels of
-// halves (16, 8, 4, 2 tokens), again with factors <= 1 only.
+// Stability.  Exponents are sums of l over stretches of one 16-token block, most of them differences of its running sums; l
+// is bounded below where 2^l is zero anyway (log2_decay), so those differences are good to 1e-4 even next to a token that
+// forgets everything.  Between blocks no exponent is positive: block b's tokens are scaled towards the block's edges
+// (2^(<= 0)), and a block further away takes the decay across the blocks in between as one more factor <= 1.  Inside a block
+// a row is scaled by 2^(-the block's sum) relative to that, up to 2^kSafe; where a channel's sum over the block is below
+// -kSafe, the block takes its pairs in four levels of halves (16, 8, 4, 2 tokens), with factors <= 1 only.
 //
 // Decay gradient.  With R> = r gr>, K> = k gk> (one-sided parts, elementwise) and the mirrored R<, K<, the gradient with
 // respect to l_m counts the pairs that have m strictly between them.  Counted from the chunk's right edge,
@@ -1041,8 +1042,8 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
             if (t0 + t < tokens) {
                 const size_t o = o0 + static_cast<size_t>(t) * C;
                 const float2 w = __ldg(reinterpret_cast<const float2*>(a.w + o));
-                const float gx = (later.x + d[t].x) * -ex2(w.x * kLog2e);
-                const float gz = (later.y + d[t].y) * -ex2(w.y * kLog2e);
+                const float gx = (later.x + d[t].x) * decay_slope(w.x);
+                const float gz = (later.y + d[t].y) * decay_slope(w.y);
                 if (!a.scalar) *reinterpret_cast<float2*>(a.gw + o) = make_float2(gx, gz);
                 else { a.gw[o] = gx; a.gw[o + 1] = gz; }
             }

@@ -293,7 +293,18 @@ template <bool kRound>
 __device__ __forceinline__ float2 round2(float2 x) {
     return kRound ? make_float2(__bfloat162float(__float2bfloat16(x.x)), __bfloat162float(__float2bfloat16(x.y))) : x;
 }
-// log2 of a token's decay
-__device__ __forceinline__ float log2_decay(float w) { return -kLog2e * ex2(w * kLog2e); }
+// log2 of a token's decay, not below -kDead: 2^-kDead is flushed to zero already, and so bounded a sum over a block keeps its
+// smaller terms to 1e-4 (and stays finite) whatever a token's decay is.  NaN stays NaN.
+constexpr float kDead = 128.f;
+__device__ __forceinline__ float log2_decay(float w) {
+    float l;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(l) : "f"(-kLog2e * ex2(w * kLog2e)), "f"(-kDead));
+    return l;
+}
+// d log(decay) / d w_raw; 0 where the decay is (its gradient is, and the sums it multiplies are zero only up to rounding)
+__device__ __forceinline__ float decay_slope(float w) {
+    const float e = ex2(w * kLog2e);
+    return e * kLog2e >= kDead ? 0.f : -e;
+}
 
 }  // namespace wkv6c

@@ -59,6 +59,14 @@ struct Args {
 
 using sm100::smem_u32;
 
+// log of a token's decay, not below -104: e^-104 is zero in float32 already, and so bounded the running sums over a block
+// keep their smaller terms to 1e-4 (and stay finite) whatever a token's decay is.  NaN stays NaN.
+__device__ __forceinline__ float log_decay(float w) {
+    float l;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(l) : "f"(-__expf(w)), "f"(-104.f));
+    return l;
+}
+
 
 // canonical K-major, no swizzle: element (row, k) of a [rows x K] bf16 operand
 __device__ __forceinline__ int op_index(int rows, int row, int k) { return (k >> 3) * (rows * 8) + row * 8 + (k & 7); }
@@ -276,7 +284,7 @@ wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r
                 float pre[8], run = 0.f;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    run += (q * SC + half * 8 + j < T) ? -__expf(wv[j]) : 0.f;
+                    run += (q * SC + half * 8 + j < T) ? log_decay(wv[j]) : 0.f;
                     pre[j] = run;
                 }
                 const float up = __shfl_up_sync(0xffffffffu, run, 16);
