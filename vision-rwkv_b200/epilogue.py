@@ -9,7 +9,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import _lib, normgate, ops
+from . import _lib, normgate, ops, traced
 from .qshift import feeds_autocast_linears
 
 KERNEL_DTYPES = (torch.float32, torch.bfloat16)
@@ -17,7 +17,7 @@ MOST_NORM_CHANNELS = 1024       # a row of norm_residual lives in one warp's reg
 
 
 def _inference(*tensors):
-    return not torch.is_grad_enabled() and all(t.is_cuda and t.dtype in KERNEL_DTYPES for t in tensors)
+    return not torch.is_grad_enabled() and not traced.tracing() and all(t.is_cuda and t.dtype in KERNEL_DTYPES for t in tensors)
 
 
 def relu_square(x):

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import torch
 
+from . import traced
 from .vrwkv import _run, biwkv_backward_as_reference, biwkv_forward_as_reference
 
 
@@ -33,6 +34,8 @@ class WKV(torch.autograd.Function):
 
 def RUN_CUDA(B, T, C, w, u, k, v):
     w, u, k, v = w.cuda(), u.cuda(), k.cuda(), v.cuda()
+    if traced.tracing():
+        return WKV.apply(B, T, C, w, u, k, v)
     if tuple(k.shape) != (B, T, C):
         raise RuntimeError(f"k has shape {tuple(k.shape)}, expected {(B, T, C)}")
     return _run(w, u, k, v)

@@ -14,7 +14,7 @@ above 1024) are refused by the library; `supported(C, group)` tells beforehand.
 """
 from __future__ import annotations
 
-from . import _lib, ops
+from . import _lib, ops, traced
 
 
 def supported(C: int, group: int) -> bool:
@@ -25,4 +25,7 @@ def norm_gate(x, gate, weight, bias, group=None, eps=1e-5, act=None):
     """x, gate: (..., C); weight, bias: (C,); group: channels per normalisation group (default C); act: None when
     `gate` is the gate itself, "sigmoid" / "silu" when it is the projection the gate is that activation of (the
     activation and its derivative then run inside the same pass)."""
-    return _lib.native().norm_gate(x, gate, weight, bias, x.shape[-1] if group is None else group, eps, ops.GATE_ACTIVATIONS[act])
+    group = x.shape[-1] if group is None else group
+    if traced.tracing():
+        return traced.NormGate.apply(x, gate, weight, bias, group, eps, act)
+    return _lib.native().norm_gate(x, gate, weight, bias, group, eps, ops.GATE_ACTIVATIONS[act])

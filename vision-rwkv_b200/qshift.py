@@ -12,20 +12,22 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import _lib, ops
+from . import _lib, ops, traced
 
 
 def feeds_autocast_linears(x, *layers):
     """True when results may leave in bfloat16 because the next step rounds them to it: inference (training keeps the
     float32 graph) under bfloat16 autocast, and every layer that takes them is a stock `nn.Linear` without hooks."""
     return (not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.float32 and torch.is_autocast_enabled("cuda")
-            and torch.get_autocast_dtype("cuda") == torch.bfloat16
+            and torch.get_autocast_dtype("cuda") == torch.bfloat16 and not traced.tracing()
             and all(type(m) is nn.Linear and not m._forward_hooks and not m._forward_pre_hooks for m in layers))
 
 
 def qshift_mix(x, mixes, patch_resolution, shift_pixel=1, channel_gamma=0.25, head_dim=None):
     """head_dim=None: `q_shift` with `channel_gamma` (VRWKV).  head_dim=n: `q_shift_multihead` of VRWKV6
     (classification/mmcls_custom/models/backbones/vrwkv6.py:75-101), the shift its ChannelMix uses."""
+    if traced.tracing():
+        return traced.QShiftMix.apply(x, patch_resolution, shift_pixel, channel_gamma, head_dim, *mixes)
     H, W = patch_resolution
     group = ops.qshift_group(x.shape[-1], channel_gamma, head_dim)
     return tuple(_lib.native().qshift_mix(x, list(mixes), H, W, shift_pixel, group, head_dim is not None))
@@ -46,6 +48,8 @@ def qshift_ddlerp(x, maas, offsets, patch_resolution, shift_pixel=1, head_dim=64
     VRWKV6's spatial mix (classification/mmcls_custom/models/backbones/vrwkv6.py:180-193) in one pass.  `offsets`
     entries may be None (`xxx = x + xx * time_maa_x`).  Results are float32, as the reference's promotion makes them;
     float32 or bfloat16 offsets are read as they are."""
+    if traced.tracing():
+        return traced.QShiftDdlerp.apply(x, patch_resolution, shift_pixel, head_dim, len(maas), *maas, *offsets)
     H, W = patch_resolution
     return tuple(_lib.native().qshift_ddlerp(x, list(maas), list(offsets), H, W, shift_pixel, head_dim))
 

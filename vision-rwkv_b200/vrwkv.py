@@ -29,7 +29,7 @@ import os
 
 import torch
 
-from . import _lib, ops
+from . import _lib, ops, traced
 
 BF16_IO = os.environ.get("VRWKV_BF16_IO", "1") != "0"
 # Off by default: the forward keeps nothing and the backward rebuilds y and Den inside the
@@ -99,9 +99,9 @@ class WKV(torch.autograd.Function):
 
 
 def _run(w, u, k, v):
-    """`WKV.apply` through the C++ autograd node (same rules, about a fifth of the host time); the modes that only the
-    Python node has - kept denominators, synchronous status checks - stay with it."""
-    if SAVE_DENOMINATOR or ops.CHECK_STATUS:
+    """`WKV.apply` through the C++ autograd node (same rules, about a fifth of the host time); what only the
+    Python node has - kept denominators, synchronous status checks, being recorded by torch.jit.trace - stays with it."""
+    if SAVE_DENOMINATOR or ops.CHECK_STATUS or traced.tracing():
         return WKV.apply(w, u, k, v)
     return _lib.native().biwkv(w, u, k, v, BF16_IO)
 
@@ -123,6 +123,6 @@ def inference_biwkv(w, u, k, v):
     """`RUN_CUDA` for a consumer that rounds y to bfloat16 (the gate of a network under autocast): where y would hold bfloat16
     values widened to float32 it stays in bfloat16.  Everything else is `RUN_CUDA`."""
     if (not torch.is_grad_enabled() and k.is_cuda and _bf16_path(k, v) and w.dtype == torch.float32
-            and not (SAVE_DENOMINATOR or ops.CHECK_STATUS)):
+            and not (SAVE_DENOMINATOR or ops.CHECK_STATUS or traced.tracing())):
         return _lib.native().biwkv_half(w, u, k, v)
     return RUN_CUDA(w, u, k, v)

@@ -19,7 +19,7 @@ import os
 
 import torch
 
-from . import _lib, ops
+from . import _lib, ops, traced
 
 HEAD_SIZE = 64
 FORWARD_PATH = os.environ.get("VRWKV6_FORWARD_PATH", "auto")
@@ -82,8 +82,8 @@ class WKV_6(torch.autograd.Function):
 
 
 def RUN_CUDA_RWKV6(B, T, C, H, r, k, v, w, u):
-    """`WKV_6.apply` with the autograd node in C++ (same rules); the modes only the Python node has stay with it."""
-    if ops.CHECK_STATUS or BACKWARD_TC != "full":
+    """`WKV_6.apply` with the autograd node in C++ (same rules); what only the Python node has stays with it."""
+    if ops.CHECK_STATUS or BACKWARD_TC != "full" or traced.tracing():
         return WKV_6.apply(B, T, C, H, r, k, v, w, u)
     assert HEAD_SIZE == C // H
     for x in (r, k, v, w, u):
@@ -103,6 +103,7 @@ def inference_rwkv6(B, T, C, H, r, k, v, w, u):
     kernel that walks 16-token blocks.  In these networks a change of a single rounding anywhere ends up, twelve blocks
     on, as a relative change of about 0.02 to 0.03 of the result (measured with kernels that agree to 1e-6), so a
     network that is only being run keeps the bits it had."""
-    if not torch.is_grad_enabled() and FORWARD_PATH == "auto" and r.dtype == k.dtype == v.dtype == torch.bfloat16 and not ops.CHECK_STATUS:
+    if (not torch.is_grad_enabled() and FORWARD_PATH == "auto" and r.dtype == k.dtype == v.dtype == torch.bfloat16
+            and not (ops.CHECK_STATUS or traced.tracing())):
         return _lib.native().wkv6_walk(r, k, v, w, u)
     return RUN_CUDA_RWKV6(B, T, C, H, r, k, v, w, u)
