@@ -62,3 +62,30 @@ def test_forward_mode_is_refused_and_not_dropped(cuda_device, grad):
         if not grad:
             with pytest.raises(RuntimeError):
                 relu_square(dual)
+
+
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("at", ["x", "vector", "offset", "norm weight", "gate"])
+def test_forward_mode_is_refused_by_the_steps_around_the_operators(cuda_device, grad, at):
+    """... whichever input carries the tangent, and also where the result leaves in bfloat16 without an autograd node."""
+    import torch.autograd.forward_ad as fwAD
+    import torch.nn as nn
+    from vision_rwkv_b200 import epilogue
+    from vision_rwkv_b200.qshift import qshift_ddlerp_to, qshift_mix_to
+    layer = nn.Linear(64, 64).to(cuda_device)
+    x, vector = torch.randn(1, 8, 64, device=cuda_device), torch.rand(64, device=cuda_device)
+    with torch.set_grad_enabled(grad), torch.autocast("cuda", torch.bfloat16), fwAD.dual_level():
+        def mark(name, t):
+            return fwAD.make_dual(t, torch.ones_like(t)) if name == at else t
+        if at in ("x", "vector"):
+            with pytest.raises(RuntimeError):
+                qshift_mix_to((layer,), mark("x", x), (vector, mark("vector", vector)), (2, 4))
+        if at in ("x", "vector", "offset"):
+            with pytest.raises(RuntimeError):
+                qshift_ddlerp_to((layer,), mark("x", x), [vector, mark("vector", vector)], [None, mark("offset", x * 2)], (2, 4))
+        if at != "vector" and at != "offset":
+            norm = nn.GroupNorm(1, 64).to(cuda_device)
+            del norm.weight
+            norm.weight = mark("norm weight", vector)
+            with pytest.raises(RuntimeError):
+                epilogue.head_norm_gate(mark("x", x), mark("gate", x + 1), norm, 64, layer, "silu")

@@ -272,6 +272,7 @@ std::vector<Tensor> qshift_mix_half(const Tensor& x, std::vector<Tensor> mixes, 
     grid_of(x, H, W);
     check_vectors(mixes, x);
     refuse_tangents({&x});
+    refuse_tangents(mixes);
     const c10::cuda::CUDAGuard guard(x.device());
     return qshift_forward(f32(x), flat_f32(mixes), QShiftArgs{H, W, shift, group, per_head}, true);
 }
@@ -285,6 +286,7 @@ std::vector<Tensor> qshift_ddlerp_half(const Tensor& x, std::vector<Tensor> maas
     const Grid g = grid_of(x, H, W);
     check_vectors(maas, x);
     refuse_tangents({&x});
+    refuse_tangents(maas);
     const c10::cuda::CUDAGuard guard(x.device());
     const Tensor xf = f32(x);
     const std::vector<Tensor> flat = flat_f32(maas);
@@ -292,6 +294,7 @@ std::vector<Tensor> qshift_ddlerp_half(const Tensor& x, std::vector<Tensor> maas
     for (const auto& m : offsets)
         if (m.has_value()) {
             TORCH_CHECK(m->sizes() == x.sizes() && m->device() == x.device(), "offsets must have the shape of x and be on its device");
+            refuse_tangents({&*m});
             any = true;
             half = half && is_bf16(*m);
         }

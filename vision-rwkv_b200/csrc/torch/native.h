@@ -33,6 +33,9 @@ inline bool has_tangent(const Tensor& t) { return t._fw_grad(/*level=*/0).define
 inline void refuse_tangents(std::initializer_list<const Tensor*> ts) {
     for (const Tensor* t : ts) TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent(*t), "forward-mode differentiation is not implemented for this operator");
 }
+inline void refuse_tangents(const std::vector<Tensor>& ts) {
+    for (const Tensor& t : ts) refuse_tangents({&t});
+}
 // whether the call needs its autograd node
 inline bool any_requires_grad(std::initializer_list<const Tensor*> ts) {
     for (const Tensor* t : ts)
