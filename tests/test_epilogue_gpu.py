@@ -43,6 +43,38 @@ def test_elementwise_steps(cuda_device, n, r_type, y_type):
         assert a.dtype == r_type and torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(), b.nan_to_num())
 
 
+@pytest.mark.parametrize("n", [1, 7, 2048, 2049])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("autocast", [torch.bfloat16, torch.float16])
+def test_squares_under_autocast_have_the_chains_type(cuda_device, n, dtype, autocast):
+    """torch squares in float32 there; only a linear layer that would round to bfloat16 first may be given bfloat16."""
+    from vision_rwkv_b200 import epilogue
+    x, layer = normal(cuda_device, n, dtype=dtype, seed=n) * 4, nn.Linear(4, 4)
+    with torch.autocast("cuda", autocast):
+        a, b = both(lambda: epilogue.relu_square(x))
+        assert a.dtype == b.dtype == torch.float32 and torch.equal(a, b)
+        a, b = both(lambda: epilogue.relu_square(x, layer))
+        assert torch.equal(a.to(autocast), b.to(autocast))
+        assert a.dtype == (torch.bfloat16 if dtype == autocast == torch.bfloat16 else torch.float32)
+        layer.register_forward_pre_hook(lambda *args: None)
+        assert both(lambda: epilogue.relu_square(x, layer))[0].dtype == torch.float32
+
+
+@pytest.mark.parametrize("version", [4, 6])
+def test_a_norm_behind_the_square_takes_it_in_float32(cuda_device, version):
+    from vision_rwkv_b200 import backbone, backbone6
+    mix = (backbone6.ChannelMixV6 if version == 6 else backbone.ChannelMix)(128, 2, 0, key_norm=True).to(cuda_device)
+    for p in mix.parameters():
+        torch.nn.init.normal_(p, std=0.1)
+    seen, x = [], normal(cuda_device, 2, 16, 128)
+    mix.key_norm.register_forward_pre_hook(lambda m, args: seen.append(args[0]))
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        mix(x, (4, 4))
+    with torch.autocast("cuda", torch.bfloat16):
+        mix(x, (4, 4))
+    assert seen[0].dtype == seen[1].dtype == torch.float32 and torch.equal(seen[0], seen[1])
+
+
 # a row in one lane, a row that fills 128 channels, one vector more, the model widths, the widest
 @pytest.mark.parametrize("rows,C", [(1, 4), (9, 128), (17, 132), (200, 192), (33, 768), (8, 1024)])
 @pytest.mark.parametrize("a_type", [torch.float32, torch.bfloat16])

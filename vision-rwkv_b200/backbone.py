@@ -90,7 +90,7 @@ class ChannelMix(nn.Module):
                                    self.shift_pixel, self.channel_gamma)
         else:
             xk = xr = x
-        k = epilogue.relu_square(self.key(xk))
+        k = epilogue.relu_square(self.key(xk), self.value if self.key_norm is None else None)
         if self.key_norm is not None:
             k = self.key_norm(k)
         return epilogue.sigmoid_gate(self.receptance(xr), self.value(k))

@@ -9,7 +9,8 @@
 //   patch_rows      an image's patches as bfloat16 rows of a matrix         the operand of the patch embedding, vrwkv.py:357
 //
 // All are bound by HBM.  Bytes per element under bfloat16 autocast, the tensor-op chains against these: the gate 4 + 6 + 6
-// (activation, cast of y, product) against 6; relu_square 8 against 4; norm_residual 34 (cast, norm, scale, add) against
+// (activation, cast of y, product) against 6; relu_square 24 (relu, cast, square in float32, the linear layer's cast)
+// against 4, or 6 with the float32 result that a norm behind it takes; norm_residual 34 (cast, norm, scale, add) against
 // 10; head_norm_gate 6 + 4 and the cast of its consumer, 6, against 8.  Every intermediate that a chain holds in bfloat16 is
 // rounded to bfloat16 here too, and products and sums are rounded one by one, so only the order of LayerNorm's sums
 // differs from torch's.
@@ -91,8 +92,8 @@ __global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, con
     }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, const R* __restrict__ x, R* __restrict__ out) {
+template <typename R, typename O>
+__global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, const R* __restrict__ x, O* __restrict__ out) {
     const long long i = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVec;
     if (i + kVec <= n) {
         float a[kVec];
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, cons
         for (int j = 0; j < kVec; ++j) a[j] = relu2(a[j]);
         store(out + i, a);
     } else {
-        for (long long j = i; j < n; ++j) out[j] = static_cast<R>(relu2(static_cast<float>(x[j])));
+        for (long long j = i; j < n; ++j) out[j] = static_cast<O>(relu2(static_cast<float>(x[j])));
     }
 }
 
@@ -302,8 +303,18 @@ extern "C" int vrwkv_relu_square(long long n, const void* x, int is_bf16, void* 
     const unsigned grid = static_cast<unsigned>(blocks_of(n));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     using H = __nv_bfloat16;
-    if (is_bf16) relu_square_kernel<H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(x), static_cast<H*>(out));
-    else relu_square_kernel<float><<<grid, kThreads, 0, s>>>(n, static_cast<const float*>(x), static_cast<float*>(out));
+    if (is_bf16) relu_square_kernel<H, H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(x), static_cast<H*>(out));
+    else relu_square_kernel<float, float><<<grid, kThreads, 0, s>>>(n, static_cast<const float*>(x), static_cast<float*>(out));
+    return record_launches(1);
+}
+
+extern "C" int vrwkv_relu_square_f32out(long long n, const uint16_t* x, float* out, void* stream) {
+    using namespace epilogue;
+    if (n <= 0 || blocks_of(n) > 0x7fffffffLL) return VRWKV_ERR_SHAPE;
+    if (!x || !out) return VRWKV_ERR_NULL;
+    if (misaligned({x, out})) return VRWKV_ERR_ALIGNMENT;
+    relu_square_kernel<__nv_bfloat16, float><<<static_cast<unsigned>(blocks_of(n)), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        n, reinterpret_cast<const __nv_bfloat16*>(x), out);
     return record_launches(1);
 }
 

@@ -27,12 +27,15 @@ Tensor sigmoid_gate(const Tensor& r_, const Tensor& y_) {
     return out;
 }
 
-Tensor relu_square(const Tensor& x_) {
+Tensor relu_square(const Tensor& x_, bool wide) {
     same_place(x_, x_, "x");
     const c10::cuda::CUDAGuard guard(x_.device());
     const Tensor x = flat(x_);
-    Tensor out = at::empty(x.sizes(), x.options());
-    if (x.numel() != 0) check(vrwkv_relu_square(x.numel(), x.data_ptr(), is_bf16(x), out.data_ptr(), stream_of(x)), "vrwkv_relu_square");
+    TORCH_CHECK(!wide || is_bf16(x), "only bfloat16 is widened");
+    Tensor out = at::empty(x.sizes(), wide ? x.options().dtype(at::kFloat) : x.options());
+    if (x.numel() == 0) return out;
+    if (wide) check(vrwkv_relu_square_f32out(x.numel(), static_cast<uint16_t*>(x.data_ptr()), fp(out), stream_of(x)), "vrwkv_relu_square_f32out");
+    else check(vrwkv_relu_square(x.numel(), x.data_ptr(), is_bf16(x), out.data_ptr(), stream_of(x)), "vrwkv_relu_square");
     return out;
 }
 

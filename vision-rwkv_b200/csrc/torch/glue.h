@@ -14,7 +14,7 @@ std::vector<Tensor> qshift_ddlerp_half(const Tensor& x, std::vector<Tensor> maas
 Tensor norm_gate(const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, int64_t group, double eps, int64_t act);
 // epilogue.cpp
 Tensor sigmoid_gate(const Tensor& r, const Tensor& y);
-Tensor relu_square(const Tensor& x);
+Tensor relu_square(const Tensor& x, bool wide);      // wide: bfloat16 x to a float32 result
 Tensor add_rows(const Tensor& table, const Tensor& a);
 Tensor patch_rows(const Tensor& img, int64_t patch);
 Tensor norm_residual(const Tensor& x, const Tensor& a, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,

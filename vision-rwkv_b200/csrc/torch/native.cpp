@@ -319,7 +319,7 @@ PYBIND11_MODULE(_native, m) {
         return vrwkv::guarded([&] { return vrwkv::biwkv_half(w, u, k, v); })();
     });
     m.def("sigmoid_gate", [](const Tensor& r, const Tensor& y) { return vrwkv::guarded([&] { return vrwkv::sigmoid_gate(r, y); })(); });
-    m.def("relu_square", [](const Tensor& x) { return vrwkv::guarded([&] { return vrwkv::relu_square(x); })(); });
+    m.def("relu_square", [](const Tensor& x, bool wide) { return vrwkv::guarded([&] { return vrwkv::relu_square(x, wide); })(); });
     m.def("add_rows", [](const Tensor& table, const Tensor& a) { return vrwkv::guarded([&] { return vrwkv::add_rows(table, a); })(); });
     m.def("patch_rows", [](const Tensor& img, int64_t patch) { return vrwkv::guarded([&] { return vrwkv::patch_rows(img, patch); })(); });
     m.def("norm_residual", [](const Tensor& x, const Tensor& a, std::optional<Tensor> weight, std::optional<Tensor> bias,

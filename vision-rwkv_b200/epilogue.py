@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, normgate, ops, traced
-from .qshift import feeds_autocast_linears
+from .qshift import autocast_linears, feeds_autocast_linears
 
 KERNEL_DTYPES = (torch.float32, torch.bfloat16)
 MOST_NORM_CHANNELS = 1024       # a row of norm_residual lives in one warp's registers
@@ -20,9 +20,13 @@ def _inference(*tensors):
     return not torch.is_grad_enabled() and not traced.tracing() and all(t.is_cuda and t.dtype in KERNEL_DTYPES for t in tensors)
 
 
-def relu_square(x):
-    """relu(x)^2 (classification/mmcls_custom/models/backbones/vrwkv.py:251)."""
-    return _lib.native().relu_square(x) if _inference(x) else torch.square(torch.relu(x))
+def relu_square(x, layer=None):
+    """relu(x)^2 (classification/mmcls_custom/models/backbones/vrwkv.py:251).  Under autocast torch squares bfloat16 x in float32;
+    the result leaves in bfloat16 only for a linear layer `layer` that rounds it to that first anyway."""
+    if not _inference(x):
+        return torch.square(torch.relu(x))
+    wide = x.dtype == torch.bfloat16 and torch.is_autocast_enabled("cuda") and not (layer is not None and autocast_linears(layer))
+    return _lib.native().relu_square(x, wide)
 
 
 def sigmoid_gate(r, y):

@@ -15,12 +15,16 @@ import torch.nn as nn
 from . import _lib, ops, traced
 
 
+def autocast_linears(*layers):
+    """True when `layers` round what they are given to bfloat16 first: inference (training keeps the float32 graph) under
+    bfloat16 autocast, and every layer is a stock `nn.Linear` without hooks."""
+    return (not torch.is_grad_enabled() and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
+            and not traced.tracing() and all(type(m) is nn.Linear and not m._forward_hooks and not m._forward_pre_hooks for m in layers))
+
+
 def feeds_autocast_linears(x, *layers):
-    """True when results may leave in bfloat16 because the next step rounds them to it: inference (training keeps the
-    float32 graph) under bfloat16 autocast, and every layer that takes them is a stock `nn.Linear` without hooks."""
-    return (not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.float32 and torch.is_autocast_enabled("cuda")
-            and torch.get_autocast_dtype("cuda") == torch.bfloat16 and not traced.tracing()
-            and all(type(m) is nn.Linear and not m._forward_hooks and not m._forward_pre_hooks for m in layers))
+    """True when results of float32 x may leave in bfloat16 because the layers that take them round them to it."""
+    return x.is_cuda and x.dtype == torch.float32 and autocast_linears(*layers)
 
 
 def qshift_mix(x, mixes, patch_resolution, shift_pixel=1, channel_gamma=0.25, head_dim=None):
