@@ -109,6 +109,45 @@ def test_layers_that_are_not_stock_keep_their_calls(cuda_device):
     assert seen == [1]
 
 
+def all_modules_hook(fn):
+    return nn.modules.module.register_module_forward_hook(lambda *args: fn())
+
+
+def all_modules_pre_hook(fn):
+    return nn.modules.module.register_module_forward_pre_hook(lambda *args: fn())
+
+
+def own_forward(fn):
+    def watch(module):
+        plain = module.forward
+        module.forward = lambda *args: (fn(), plain(*args))[1]
+    return watch
+
+
+@pytest.mark.parametrize("watch", [all_modules_hook, all_modules_pre_hook, own_forward])
+def test_watched_layers_keep_their_calls(cuda_device, watch):
+    """Hooks for all modules and a replaced forward see the call of every layer whose work a kernel can take over."""
+    from vision_rwkv_b200 import epilogue
+    from vision_rwkv_b200.qshift import feeds_autocast_linears
+    x, a, img = normal(cuda_device, 4, 64), normal(cuda_device, 4, 64, seed=1), normal(cuda_device, 1, 3, 32, 32)
+    norm, conv, layer = nn.LayerNorm(64).to(cuda_device), nn.Conv2d(3, 64, 16, stride=16).to(cuda_device), nn.Linear(64, 64).to(cuda_device)
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        assert epilogue.patch_embedding(img, conv) is not None and feeds_autocast_linears(x, layer)
+        seen, handle = [], None
+        if watch is own_forward:
+            for m in (norm, conv, layer):
+                own_forward(lambda: seen.append(1))(m)
+        else:
+            handle = watch(lambda: seen.append(1))
+        try:
+            epilogue.norm_residual(x, a, norm, None)
+            assert seen == [1]
+            assert epilogue.patch_embedding(img, conv) is None and not feeds_autocast_linears(x, layer)
+        finally:
+            if handle is not None:
+                handle.remove()
+
+
 # a part of one block, exactly one block (64 heads), one head more, odd numbers of heads per row
 @pytest.mark.parametrize("rows,C", [(1, 64), (64, 64), (65, 64), (7, 192), (196, 768)])
 @pytest.mark.parametrize("gate_type", [torch.float32, torch.bfloat16])

@@ -2,7 +2,8 @@
 
 Each function is the reference's expression; when a network is only being run (no gradients wanted) on CUDA tensors in
 float32 or bfloat16 it is one kernel of csrc/mixer_epilogue.cu instead of a chain of tensor operations.  Training keeps the
-tensor operations and their graph.  Layers whose work a kernel takes over must be the stock ones without hooks.
+tensor operations and their graph.  A layer whose work a kernel takes over must be one whose call is torch's own
+(`qshift.stock`).
 """
 from __future__ import annotations
 
@@ -10,7 +11,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, normgate, ops, traced
-from .qshift import autocast_linears, feeds_autocast_linears
+from .qshift import autocast_linears, feeds_autocast_linears, stock
 
 KERNEL_DTYPES = (torch.float32, torch.bfloat16)
 MOST_NORM_CHANNELS = 1024       # a row of norm_residual lives in one warp's registers
@@ -51,9 +52,8 @@ def residual(x, a, gamma):
 def norm_residual(x, a, norm, gamma):
     """x + gamma * norm(a) for a LayerNorm `norm` (post-norm blocks).  Under autocast torch computes that norm in float32."""
     C = x.shape[-1]
-    if (_residual_kernel(x, a, gamma) and type(norm) is nn.LayerNorm and norm.normalized_shape == (C,) and norm.bias is not None
-            and norm.weight.dtype == norm.bias.dtype == torch.float32 and not norm._forward_hooks and not norm._forward_pre_hooks
-            and (a.dtype == torch.float32 or torch.is_autocast_enabled("cuda"))):
+    if (_residual_kernel(x, a, gamma) and stock(norm, nn.LayerNorm) and norm.normalized_shape == (C,) and norm.bias is not None
+            and norm.weight.dtype == norm.bias.dtype == torch.float32 and (a.dtype == torch.float32 or torch.is_autocast_enabled("cuda"))):
         return _lib.native().norm_residual(x, a, norm.weight, norm.bias, gamma, norm.eps)
     return residual(x, norm(a), gamma)
 
@@ -83,9 +83,8 @@ def patch_embedding(img, conv):
     """The tokens (B, h * w, C) of a patch embedding `conv` (kernel = stride; vrwkv.py:357) as one matrix product over the
     patches, or None where the convolution itself has to run (training, other data types, other convolutions)."""
     p = conv.kernel_size[0]
-    if not (feeds_autocast_linears(img) and type(conv) is nn.Conv2d and not conv._forward_hooks and not conv._forward_pre_hooks
-            and conv.kernel_size == conv.stride == (p, p) and conv.padding == (0, 0) and conv.dilation == (1, 1) and conv.groups == 1
-            and img.dim() == 4 and img.shape[1] == conv.in_channels and img.is_contiguous() and p % 8 == 0
+    if not (feeds_autocast_linears(img) and stock(conv, nn.Conv2d) and conv.kernel_size == conv.stride == (p, p)
+            and conv.padding == (0, 0) and conv.dilation == (1, 1) and conv.groups == 1 and img.dim() == 4 and img.shape[1] == conv.in_channels and img.is_contiguous() and p % 8 == 0
             and img.shape[2] >= p and img.shape[3] >= p and img.shape[3] % 4 == 0 and img.numel() < 2 ** 33):
         return None
     tokens = nn.functional.linear(_lib.native().patch_rows(img, p), conv.weight.flatten(1))

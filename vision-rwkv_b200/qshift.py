@@ -15,11 +15,18 @@ import torch.nn as nn
 from . import _lib, ops, traced
 
 
+def stock(module, cls):
+    """Whether calling `module` runs `cls.forward` and nothing else: no subclass, no forward of its own, no hooks (its own or
+    those registered for all modules)."""
+    return (type(module) is cls and "forward" not in module.__dict__ and not module._forward_hooks and not module._forward_pre_hooks
+            and not nn.modules.module._global_forward_hooks and not nn.modules.module._global_forward_pre_hooks)
+
+
 def autocast_linears(*layers):
     """True when `layers` round what they are given to bfloat16 first: inference (training keeps the float32 graph) under
-    bfloat16 autocast, and every layer is a stock `nn.Linear` without hooks."""
+    bfloat16 autocast, and every layer is a stock `nn.Linear`."""
     return (not torch.is_grad_enabled() and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
-            and not traced.tracing() and all(type(m) is nn.Linear and not m._forward_hooks and not m._forward_pre_hooks for m in layers))
+            and not traced.tracing() and all(stock(m, nn.Linear) for m in layers))
 
 
 def feeds_autocast_linears(x, *layers):
