@@ -70,8 +70,9 @@ int vrwkv_set_path(int path);
 int vrwkv_workspace_status(const void* workspace, void* stream, unsigned* status_out);
 
 /* Failure bits (as in vrwkv_workspace_status) that launches on `device` have reported since the last call, and
- * clears them; 0 if none.  Kernels that give up a bounded wait write the word through mapped host memory, so the
- * call is one read of host memory: no synchronisation, no copy.  A launch that is still running reports later:
+ * clears them; 0 if none.  Bits 8 to 11 say whose launches: Bi-WKV forward, Bi-WKV backward, WKV6 forward, WKV6
+ * backward.  Kernels that give up a bounded wait write a word of mapped host memory, so the
+ * call reads host memory: no synchronisation, no copy.  A launch that is still running reports later:
  * synchronise first to see its result.  The first call (per process) sets the word up; launches made before it
  * report through their workspace only. */
 unsigned vrwkv_take_failures(int device);

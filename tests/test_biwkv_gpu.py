@@ -302,8 +302,22 @@ def test_bounded_wait_runs_out_and_reports(cuda_device, kernel_path):
         # into the module or, at the latest, when the caller asks
         ops.CHECK_STATUS = False
         ops.biwkv_forward(w, u, k, v)
-        with pytest.raises(_lib.VrwkvError, match="earlier launch"):
+        with pytest.raises(_lib.VrwkvError, match="earlier launch, Bi-WKV forward:"):
             ops.raise_if_failed()
+        ops.biwkv_backward(w, u, k, v, gy)
+        with pytest.raises(_lib.VrwkvError, match="earlier launch, Bi-WKV backward:"):
+            ops.raise_if_failed()
+        # the report names the launch's operator whatever call sees it, in the extension too, and a checked call that is itself
+        # in order does not swallow it
+        for strict in (False, True):
+            ops.biwkv_backward(w, u, k, v, gy)
+            torch.cuda.synchronize()
+            lib.vrwkv_set_path(0)
+            ops.CHECK_STATUS = strict
+            with pytest.raises(_lib.VrwkvError, match="earlier launch, Bi-WKV backward:"):
+                ops.biwkv_forward(w, u, k, v) if strict else _lib.native().biwkv(w, u, k, v, True)
+            ops.CHECK_STATUS = False
+            lib.vrwkv_set_path(3)
         ops.biwkv_forward(w, u, k, v)
         torch.cuda.synchronize()
         with pytest.raises(_lib.VrwkvError, match="earlier launch"):

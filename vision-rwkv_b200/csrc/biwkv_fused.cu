@@ -1419,7 +1419,7 @@ static int launch(Layout& l, const float* w, const float* u, const E* k, const E
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     p.w = w; p.u = u;
     p.status = reinterpret_cast<unsigned*>(ws + l.off_status);
-    p.mirror = failure_mirror();
+    p.mirror = failure_mirror(kBwd ? Op::biwkv_backward : Op::biwkv_forward);
     p.flags = reinterpret_cast<unsigned*>(ws + l.off_flags);
     p.exch = reinterpret_cast<float*>(ws + l.off_exch);
     p.partial = reinterpret_cast<float*>(ws + l.off_partial);
@@ -1528,7 +1528,7 @@ int backward_saved(int B, int T, int C, const float* w, const float* u, const fl
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     p.w = w; p.u = u;
     p.status = reinterpret_cast<unsigned*>(ws + l.off_status);
-    p.mirror = failure_mirror();
+    p.mirror = failure_mirror(Op::biwkv_backward);
     p.flags = reinterpret_cast<unsigned*>(ws + l.off_flags);
     p.exch = reinterpret_cast<float*>(ws + l.off_exch);
     p.partial = reinterpret_cast<float*>(ws + l.off_partial);

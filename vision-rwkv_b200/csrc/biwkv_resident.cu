@@ -1521,7 +1521,7 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     p.w = w; p.u = u;
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     p.status = reinterpret_cast<unsigned*>(ws);
-    p.mirror = failure_mirror();
+    p.mirror = failure_mirror(kBwd ? Op::biwkv_backward : Op::biwkv_forward);
     const size_t units = static_cast<size_t>(B) * p.n_strips;
     const Carve cv = carve(B, C, pl, kBwd);
     p.redo_count = reinterpret_cast<unsigned*>(ws) + 1;

@@ -42,19 +42,19 @@ void set_error_detail(const char* text) {
 
 int record_launches(int launched) { return finish(launched); }
 
-// One word per device in pinned, mapped host memory: kernels write it only when a bounded wait runs out, the host
+// One word per device and operator in pinned, mapped host memory: kernels write it only when a bounded wait runs out, the host
 // reads it as ordinary memory, so watching for failures costs neither a copy nor an event per launch.
 namespace {
-constexpr int kMirrorDevices = 64;
+constexpr int kMirrorDevices = 64, kMirrorOps = 4;
 std::atomic<unsigned*> g_mirror{nullptr};
 std::mutex g_mirror_mutex;
 }  // namespace
 
-unsigned* failure_mirror() {
+unsigned* failure_mirror(Op op) {
     unsigned* base = g_mirror.load(std::memory_order_acquire);
     int dev = 0;
     if (base == nullptr || cudaGetDevice(&dev) != cudaSuccess || dev >= kMirrorDevices) return nullptr;
-    return base + dev;
+    return base + dev * kMirrorOps + static_cast<int>(op);
 }
 
 extern "C" {
@@ -108,21 +108,26 @@ unsigned vrwkv_take_failures(int device) {
             cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
             cudaThreadExchangeStreamCaptureMode(&mode);
             void* p = nullptr;
-            const cudaError_t err = cudaHostAlloc(&p, kMirrorDevices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+            const cudaError_t err = cudaHostAlloc(&p, kMirrorDevices * kMirrorOps * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
             cudaThreadExchangeStreamCaptureMode(&mode);
             if (err != cudaSuccess) {
                 cudaGetLastError();
                 return 0;
             }
-            std::memset(p, 0, kMirrorDevices * sizeof(unsigned));
+            std::memset(p, 0, kMirrorDevices * kMirrorOps * sizeof(unsigned));
             base = static_cast<unsigned*>(p);
             g_mirror.store(base, std::memory_order_release);
         }
     }
     if (device < 0 || device >= kMirrorDevices) return 0;
-    volatile unsigned* word = base + device;
-    const unsigned bits = *word;
-    if (bits != 0) *word = 0;
+    unsigned bits = 0;
+    for (int op = 0; op < kMirrorOps; ++op) {
+        volatile unsigned* word = base + device * kMirrorOps + op;
+        const unsigned seen = *word;
+        if (seen == 0) continue;
+        *word = 0;
+        bits |= seen | 1u << (8 + op);
+    }
     return bits;
 }
 

@@ -33,10 +33,14 @@ void raise_status(int status, const char* what) {
 void raise_failures(int device, const char* what) {
     const unsigned bits = vrwkv_take_failures(device);
     if (bits == 0) return;
+    static const char* const kNames[] = {"Bi-WKV forward", "Bi-WKV backward", "WKV6 forward", "WKV6 backward"};
+    std::string names;
+    for (int i = 0; i < 4; ++i)
+        if (bits >> (8 + i) & 1u) names += (names.empty() ? "" : ", ") + std::string(kNames[i]);
     char word[16];
-    snprintf(word, sizeof(word), "%#x", bits);
-    raise(std::string("device status word ") + word + ", seen at " + what +
-          " (a bounded device-side wait ran out in an earlier launch: its outputs, and everything computed from them, are invalid)");
+    snprintf(word, sizeof(word), "%#x", bits & 0xffu);
+    raise(std::string("device status word ") + word + ", seen at " + what + " (a bounded device-side wait ran out in an earlier launch, " +
+          names + ": its outputs, and everything computed from them, are invalid)");
 }
 
 namespace {

@@ -8,9 +8,10 @@
 void set_error_detail(const char* text);
 // Add `launched` kernels to the process-wide count and turn the CUDA error state into a status.
 int record_launches(int launched);
-// Host-visible word of the current device that kernels set when a bounded wait runs out (pinned, mapped; null
-// until vrwkv_take_failures() has been called once).  It costs a successful launch nothing.
-unsigned* failure_mirror();
+// Host-visible word of the current device and operator that kernels set when a bounded wait runs out (pinned, mapped;
+// null until vrwkv_take_failures() has been called once).  It costs a successful launch nothing.
+enum class Op { biwkv_forward, biwkv_backward, wkv6_forward, wkv6_backward };
+unsigned* failure_mirror(Op op);
 
 #ifdef __CUDACC__
 // A bounded wait ran out: `status` is the launch's own device word, `mirror` the host-visible one (may be null).

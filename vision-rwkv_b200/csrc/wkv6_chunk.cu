@@ -1128,7 +1128,8 @@ static bool run_states(int B, int T_, int H, const void* r, const void* k, const
         mr = mk;
         mg = mv;
     }
-    const StateArgs a{T_, H, chunks_of(T_), states, plane, static_cast<unsigned*>(workspace), failure_mirror()};
+    const StateArgs a{T_, H, chunks_of(T_), states, plane, static_cast<unsigned*>(workspace),
+                      failure_mirror(kRows ? Op::wkv6_backward : Op::wkv6_forward)};
     const auto kernel = wkv6_state_kernel<T, T, G, kZ, kX, kRows, kPairs>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), S::bytes)) return false;
     kernel<<<dim3(B * H, 2), 128 * kPairs, S::bytes, stream>>>(a, mw, mk, mv, mr, mg);

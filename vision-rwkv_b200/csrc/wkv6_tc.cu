@@ -568,7 +568,7 @@ static int launch(int B, int T, int H, const void* r, const void* k, const void*
         return -1;
     }
     Args a{B, T, H, static_cast<const float*>(r), static_cast<const float*>(k), static_cast<const float*>(v), w_raw, u, y,
-           status, failure_mirror()};
+           status, failure_mirror(Op::wkv6_forward)};
     cudaMemsetAsync(status, 0, sizeof(unsigned), stream);
     // both directions add into y
     cudaMemsetAsync(y, 0, static_cast<size_t>(B) * T * C * sizeof(float), stream);

@@ -84,7 +84,8 @@ def patch_embedding(img, conv):
     patches, or None where the convolution itself has to run (training, other data types, other convolutions)."""
     p = conv.kernel_size[0]
     if not (feeds_autocast_linears(img) and stock(conv, nn.Conv2d) and conv.kernel_size == conv.stride == (p, p)
-            and conv.padding == (0, 0) and conv.dilation == (1, 1) and conv.groups == 1 and img.dim() == 4 and img.shape[1] == conv.in_channels and img.is_contiguous() and p % 8 == 0
+            and conv.padding == (0, 0) and conv.dilation == (1, 1) and conv.groups == 1
+            and img.dim() == 4 and img.shape[1] == conv.in_channels and img.is_contiguous() and p % 8 == 0
             and img.shape[2] >= p and img.shape[3] >= p and img.shape[3] % 4 == 0 and img.numel() < 2 ** 33):
         return None
     tokens = nn.functional.linear(_lib.native().patch_rows(img, p), conv.weight.flatten(1))

@@ -18,15 +18,17 @@ from . import _lib
 # (the kernels then return garbage instead of hanging).  Off by default: it costs a sync.
 CHECK_STATUS = False
 # Without CHECK_STATUS a failed launch is still reported, one or more calls late and with no synchronisation: the
-# kernel that gives up a wait writes a word of mapped host memory (one per device), and the next call into this
-# module (or `raise_if_failed()`) reads it and raises.
+# kernel that gives up a wait writes a word of mapped host memory (one per device and operator), and the next call into
+# this module (or `raise_if_failed()`) reads it and raises.
+OPERATORS = ("Bi-WKV forward", "Bi-WKV backward", "WKV6 forward", "WKV6 backward")     # bits 8.. of vrwkv_take_failures
 
 
 def _raise_failures(lib, index, what):
     bits = lib.vrwkv_take_failures(index)
     if bits:
-        raise _lib.VrwkvError(f"device status word {bits:#x}, seen at {what} (a bounded device-side wait ran out in an earlier "
-                              "launch: its outputs, and everything computed from them, are invalid)")
+        names = ", ".join(name for i, name in enumerate(OPERATORS) if bits >> (8 + i) & 1)
+        raise _lib.VrwkvError(f"device status word {bits & 0xff:#x}, seen at {what} (a bounded device-side wait ran out in an "
+                              f"earlier launch, {names}: its outputs, and everything computed from them, are invalid)")
 
 
 def raise_if_failed(device=None, wait=True):
@@ -49,10 +51,9 @@ def _check_status(lib, ws, what):
         st = lib.vrwkv_workspace_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream,
                                         ctypes.byref(word))
         _lib.check(st, "vrwkv_workspace_status")
-        lib.vrwkv_take_failures(ws.device.index)       # reported here
         if word.value:
+            lib.vrwkv_take_failures(ws.device.index)       # reported here
             raise _lib.VrwkvError(f"{what}: device status word {word.value:#x} (a bounded wait ran out)")
-        return
     _raise_failures(lib, ws.device.index, what)
 
 
