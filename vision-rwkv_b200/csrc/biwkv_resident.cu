@@ -242,8 +242,6 @@ __device__ __forceinline__ float2 ld_in(const float* area, int i, int pr) {
     }
     return *(reinterpret_cast<const float2*>(area + i * kCs) + pr);
 }
-// w and u are vectors that a caller may have cut out of a larger buffer: 4-byte alignment is all they promise
-__device__ __forceinline__ float2 ld_pair(const float* p) { return f2(__ldg(p), __ldg(p + 1)); }
 __device__ __forceinline__ float2 round2(float2 v) { return __bfloat1622float2(__float22bfloat162_rn(v)); }
 template <bool kHalf>
 __device__ __forceinline__ void st_out(float* area, int i, int pr, float2 v) {
@@ -911,8 +909,8 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     // (relaxed: the mbarrier-init fence above is what publishes the initialisation)
     if (p.cluster > 1) cluster_arrive_relaxed();
     const int ch0 = strip * kCs + 2 * pr;
-    const float2 w2 = (ch0 < p.C) ? ld_pair(p.w + ch0) : f2(0.f, 0.f);
-    const float2 u2 = (ch0 < p.C) ? ld_pair(p.u + ch0) : f2(0.f, 0.f);
+    const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
+    const float2 u2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.u + ch0) : f2(0.f, 0.f);
     const float2 lam2 = *reinterpret_cast<const float2*>(c.consts + kLam * kCs + 2 * pr);
     const float2 wl2 = *reinterpret_cast<const float2*>(c.consts + kWl2 * kCs + 2 * pr);
     const float2 c2 = *reinterpret_cast<const float2*>(c.consts + kCuw * kCs + 2 * pr);
@@ -1261,8 +1259,8 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                     sm100::tma_load_3d(slot_g + sp * kSpan * kCs, &map_g, full, strip * kCs, tok0 + sp * kSpan, b);
         }
         const int ch0 = strip * kCs + 2 * pr;
-        const float2 w2 = (ch0 < p.C) ? ld_pair(p.w + ch0) : f2(0.f, 0.f);
-        const float2 u2 = (ch0 < p.C) ? ld_pair(p.u + ch0) : f2(0.f, 0.f);
+        const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
+        const float2 u2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.u + ch0) : f2(0.f, 0.f);
         if (!sm100::mbar_wait(full, phase, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
         phase ^= 1u;
         if (kHalf) {
@@ -1480,9 +1478,9 @@ bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// workspace: status block (256 B) | redo list | backward partials | segment flags | segment records
+// workspace: status block (256 B) | redo list | backward partials | segment flags | segment records | copies of w, u
 struct Carve {
-    size_t off_list, off_partial, off_flags, off_records, total;
+    size_t off_list, off_partial, off_flags, off_records, off_vectors, total;
 };
 static Carve carve(int B, int C, const Plan& pl, bool bwd) {
     const size_t units = static_cast<size_t>(B) * ((C + kCs - 1) / kCs);
@@ -1492,7 +1490,8 @@ static Carve carve(int B, int C, const Plan& pl, bool bwd) {
     cv.off_flags = cv.off_partial + (bwd ? align_up(units * pl.segs * pl.cluster * 2 * kCs * sizeof(float), 256) : 0);
     const size_t recs = pl.segs > 1 ? units * pl.segs * 4 : 0;
     cv.off_records = cv.off_flags + align_up(recs * sizeof(unsigned), 256);
-    cv.total = cv.off_records + align_up(recs * kSegRec * sizeof(float), 256);
+    cv.off_vectors = cv.off_records + align_up(recs * kSegRec * sizeof(float), 256);
+    cv.total = cv.off_vectors + align_up(2 * static_cast<size_t>(C) * sizeof(float), 256);
     return cv;
 }
 
@@ -1507,6 +1506,14 @@ bool multi_segment(int T) {
     return make_plan(T, pl) && pl.segs > 1;
 }
 
+// The kernels read w and u in pairs.  A vector that starts at an odd float (cut out of a parameter buffer) goes through a copy:
+// single loads in the kernels cost every call, up to 7 % where a sequence has several segments (T=16384: 1925 and 2067 us).
+static const float* paired(const float* x, int C, float* copy, cudaStream_t stream) {
+    if ((reinterpret_cast<uintptr_t>(x) & 7u) == 0) return x;
+    cudaMemcpyAsync(copy, x, static_cast<size_t>(C) * sizeof(float), cudaMemcpyDeviceToDevice, stream);
+    return copy;
+}
+
 template <bool kBwd, Types kTypes>
 static int launch(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy,
                   void* o0, void* o1, float* gwgu, void* workspace, cudaStream_t stream) {
@@ -1518,7 +1525,6 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     p.B = B; p.T = T; p.C = C;
     p.n_strips = (C + kCs - 1) / kCs;
     p.cluster = pl.cluster; p.n_warps = pl.n_warps; p.n_tok = pl.n_tok;
-    p.w = w; p.u = u;
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     p.status = reinterpret_cast<unsigned*>(ws);
     p.mirror = failure_mirror(kBwd ? Op::biwkv_backward : Op::biwkv_forward);
@@ -1530,6 +1536,9 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     p.segs = pl.segs;
     p.xflag = reinterpret_cast<unsigned*>(ws + cv.off_flags);
     p.xseg = reinterpret_cast<float*>(ws + cv.off_records);
+    float* const vectors = reinterpret_cast<float*>(ws + cv.off_vectors);
+    p.w = paired(w, C, vectors, stream);
+    p.u = paired(u, C, vectors + C, stream);
     p.spin_limit = g_withhold.load() ? (1u << 10) : kSpinLimit;
     p.withhold_rank = g_withhold.load() ? 1 : -1;
     tensor_map::bind_primary_context();   // the tensor-map encoder is a driver call
