@@ -54,8 +54,8 @@ unsigned long long vrwkv_launch_count(void);
  * cluster-resident single-pass kernels when T <= 32768, C % 4 == 0 (bfloat16: C % 8 == 0) and the
  * tensors are 16-byte aligned - one cluster per sequence strip up to T = 4096, several above -,
  * else the persistent tile kernels, else the generic multi-launch path), 1 = the
- * first-generation kernels (Bi-WKV: the generic multi-launch path; WKV6 tensor-core forward:
- * the serial-phase kernel instead of the warp-specialised one), 2 = Bi-WKV skips the
+ * first-generation kernels (Bi-WKV: the generic multi-launch path; vrwkv_wkv6_forward_tc_*: the walk
+ * that needs no scratch memory, whatever the workspace holds), 2 = Bi-WKV skips the
  * cluster-resident kernels (persistent tile kernels where eligible), 3 = test of the bounded
  * device-side waits: as 0, but one CTA of every cluster withholds what it owes the others and
  * the waits give up after about a thousand polls, so the call returns promptly with bit 0 of the

@@ -191,27 +191,42 @@ def test_bf16_inputs(cuda_device):
         assert rel_err(x.grad.float(), rf) <= 1e-2
 
 
-# ---- tensor-core forward (tcgen05, bf16 operands): tolerance 1e-2 of max|y| -------------------
+# ---- tensor-core forwards (bf16 operands): tolerance 1e-2 of max|y| -------------------
 TC_TOL = 1e-2
 
 
-@pytest.fixture(params=["pipelined", "serial"])
+@pytest.fixture(params=["chunk", "walk", "chunk_bf16", "walk_bf16"])
 def tc_kernel(request):
-    """The tensor-core tests run on both kernels: the warp-specialised one (default) and the
-    first-generation one in which all warps do every phase in turn."""
-    from vision_rwkv_b200 import _lib, ops
-    lib = _lib.load()
+    """The tensor-core tests run on both kernels, the 64-token chunks and the 16-token walk (what a workspace of a status word
+    gets, and network inference), each on float32 tensors and on bfloat16 r, k, v."""
+    from vision_rwkv_b200 import ops
     ops.CHECK_STATUS = True
-    assert lib.vrwkv_set_path(1 if request.param == "serial" else 0) == 0
     yield request.param
-    lib.vrwkv_set_path(0)
     ops.CHECK_STATUS = False
 
 
-def run_tc(dev, r, k, v, w, u, H):
-    from vision_rwkv_b200 import ops
+def run_tc(dev, r, k, v, w, u, H, kernel):
+    from vision_rwkv_b200 import _lib, ops
+    half = kernel.endswith("bf16")
     f = [x.float().contiguous().to(dev) for x in (r, k, v, w, u)]
-    y = ops.wkv6_forward(*f, H, tensor_cores=True)     # raises if the kernel's status word is set
+    if half:
+        f[:3] = [x.bfloat16() for x in f[:3]]
+    if kernel.startswith("chunk"):
+        y = ops.wkv6_forward(*f, H, tensor_cores=True)     # raises if the kernel's status word is set
+    else:
+        lib, y = _lib.load(), torch.empty(f[0].shape, device=dev)
+        ws = torch.empty(256, dtype=torch.uint8, device=dev)
+        entry = lib.vrwkv_wkv6_forward_tc_bf16 if half else lib.vrwkv_wkv6_forward_tc_f32
+        before = lib.vrwkv_launch_count()
+        assert entry(*f[0].shape, H, *[x.data_ptr() for x in f], y.data_ptr(), ws.data_ptr(), 256, torch.cuda.current_stream().cuda_stream) == 0
+        assert lib.vrwkv_launch_count() == before + 1
+        ops._check_status(lib, ws, kernel)
+        if half:       # the same kernel from the torch extension
+            from vision_rwkv_b200.vrwkv6 import inference_rwkv6
+            ops.CHECK_STATUS = False
+            with torch.no_grad():
+                assert torch.equal(y, inference_rwkv6(*f[0].shape, H, *f))
+            ops.CHECK_STATUS = True
     torch.cuda.synchronize()
     return y
 
@@ -220,7 +235,7 @@ def run_tc(dev, r, k, v, w, u, H):
                                    (2, 37, 2), (1, 64, 1), (1, 70, 1), (3, 196, 2), (1, 300, 1), (1, 1024, 1)])
 def test_tensor_core_forward_parity(cuda_device, B, T, H, tc_kernel):
     r, k, v, w, u, _ = O.make_inputs(B, T, 64 * H, H, seed=T, round_to=torch.bfloat16)
-    y = run_tc(cuda_device, r, k, v, w, u, H)
+    y = run_tc(cuda_device, r, k, v, w, u, H, tc_kernel)
     ref = O.wkv6_forward(*[x.float().double() for x in (r, k, v, w, u)], H)
     assert torch.isfinite(y).all()
     assert rel_err(y, ref) <= TC_TOL
@@ -228,13 +243,13 @@ def test_tensor_core_forward_parity(cuda_device, B, T, H, tc_kernel):
 
 @pytest.mark.parametrize("shift", [1.0, 1.7, 2.6, 4.0])
 def test_tensor_core_forward_strong_decay(cuda_device, shift, tc_kernel):
-    """A block whose accumulated log-decay passes 80 in some channel scores pairwise on the CUDA cores; the
-    shifts cover none / some / all blocks taking that path, and one head only."""
+    """A block whose accumulated log-decay is too strong for factors above 1 takes another path (pairs on the CUDA cores in the
+    walk, levels of halves in the chunks); the shifts cover none / some / all blocks taking it, and one head only."""
     B, T, H = 2, 100, 2
     r, k, v, w, u, _ = O.make_inputs(B, T, 64 * H, H, seed=11, round_to=torch.bfloat16)
     w = w.clone()
     w[..., :64] += shift            # head 0 decays fast, head 1 stays mild
-    y = run_tc(cuda_device, r, k, v, w, u, H)
+    y = run_tc(cuda_device, r, k, v, w, u, H, tc_kernel)
     ref = O.wkv6_forward(*[x.float().double() for x in (r, k, v, w, u)], H)
     assert torch.isfinite(y).all()
     assert rel_err(y, ref) <= TC_TOL
@@ -251,17 +266,17 @@ def test_tensor_core_forward_matches_exact_sweeps_at_scale(cuda_device, tc_kerne
     r, k, v = [torch.randn(B, T, C, generator=g).to(cuda_device) for _ in range(3)]
     w = (torch.randn(B, T, C, generator=g) * 0.5 - 0.6).to(cuda_device)
     u = (torch.randn(H, 64, generator=g) * 0.1).to(cuda_device)
-    y_tc = ops.wkv6_forward(r, k, v, w, u, H, tensor_cores=True)
+    y_tc = run_tc(cuda_device, r, k, v, w, u, H, tc_kernel)
     y_ex = ops.wkv6_forward(r, k, v, w, u, H)
     assert rel_err(y_tc, y_ex.double().cpu()) <= TC_TOL
 
 
 def test_tensor_core_forward_reproducible_and_independent(cuda_device, tc_kernel):
     r, k, v, w, u, _ = O.make_inputs(2, 90, 128, 2, seed=5, round_to=torch.bfloat16)
-    a = run_tc(cuda_device, r, k, v, w, u, 2)
-    b = run_tc(cuda_device, r, k, v, w, u, 2)
+    a = run_tc(cuda_device, r, k, v, w, u, 2, tc_kernel)
+    b = run_tc(cuda_device, r, k, v, w, u, 2, tc_kernel)
     assert torch.equal(a, b)
-    one = run_tc(cuda_device, r[1:], k[1:], v[1:], w[1:], u, 2)
+    one = run_tc(cuda_device, r[1:], k[1:], v[1:], w[1:], u, 2, tc_kernel)
     assert torch.equal(one[0], a[1])
 
 
@@ -352,7 +367,7 @@ def run_tc_backward(dev, r, k, v, w, u, gy, H, half=False):
 
 def check_tc_backward(got, ref, tol=TC_TOL, gw_tol=None):
     """gw is a difference of running sums of k*gk and r*gr over the sequence: it is only as good as gr and gk
-    are accurate, which is why the mixing kernel carries its derived operands as hi + lo bfloat16 pairs."""
+    are accurate, which is why the kernels carry their scaled operands as hi + lo bfloat16 pairs."""
     errs = {}
     scale = max(float(rf.abs().max()) for rf in ref)
     for name, g, rf in zip(GRADS, got, ref):
@@ -372,7 +387,7 @@ def gw_bound(T):
 @pytest.mark.parametrize("B,T,H", [(1, 1, 1), (2, 2, 1), (1, 3, 2), (2, 15, 1), (1, 16, 3), (1, 17, 2), (1, 31, 1),
                                    (2, 37, 2), (1, 64, 1), (1, 70, 1), (3, 196, 2), (1, 300, 1), (1, 1024, 1)])
 def test_tensor_core_backward_parity(cuda_device, B, T, H):
-    """gr, gk, gv, gw, gu of the tcgen05 kernels against the float64 oracle on bf16-rounded inputs: 1e-2."""
+    """gr, gk, gv, gw, gu of the chunked kernels against the float64 oracle on bf16-rounded inputs: 1e-2."""
     r, k, v, w, u, gy = O.make_inputs(B, T, 64 * H, H, seed=T, round_to=torch.bfloat16)
     gy = gy.bfloat16().float()
     ref = O.wkv6_backward(*[x.float().double() for x in (r, k, v, w, u, gy)], H)
@@ -382,7 +397,7 @@ def test_tensor_core_backward_parity(cuda_device, B, T, H):
 
 @pytest.mark.parametrize("shift", [1.0, 1.7, 2.6, 4.0])
 def test_tensor_core_backward_strong_decay(cuda_device, shift):
-    """Blocks whose accumulated log-decay passes 80 take their in-block part on the CUDA cores."""
+    """Blocks whose accumulated log-decay is too strong for factors above 1 take their pairs in levels of halves."""
     B, T, H = 2, 100, 2
     r, k, v, w, u, gy = O.make_inputs(B, T, 64 * H, H, seed=11, round_to=torch.bfloat16)
     gy = gy.bfloat16().float()
@@ -390,6 +405,22 @@ def test_tensor_core_backward_strong_decay(cuda_device, shift):
     w[..., :64] += shift
     ref = O.wkv6_backward(*[x.float().double() for x in (r, k, v, w, u, gy)], H)
     check_tc_backward(run_tc_backward(cuda_device, r, k, v, w, u, gy, H), ref, gw_tol=gw_bound(T))
+
+
+# one token fewer and more than a 16-token block, a 64-token chunk, two of them; the third chunk a single token
+@pytest.mark.parametrize("T", [15, 17, 63, 64, 65, 127, 128, 129])
+def test_chunk_edges(cuda_device, T):
+    """Forward and backward of the chunked kernels.  y and gv carry operands rounded to bfloat16 (1e-2); gr, gk and gu operands of
+    16 bits or exact ones (1e-4); gw is a difference of sums of those (1e-3)."""
+    from vision_rwkv_b200 import ops
+    B, H = 2, 3
+    args = O.make_inputs(B, T, 64 * H, H, seed=T, round_to=torch.bfloat16)
+    ref = reference(*args, H)
+    r, k, v, gy = (args[i].bfloat16().to(cuda_device) for i in (0, 1, 2, 5))
+    w, u = args[3].float().to(cuda_device), args[4].float().to(cuda_device)
+    got = (ops.wkv6_forward(r, k, v, w, u, H, tensor_cores=True), *ops.wkv6_backward(r, k, v, w, u, gy, H, tensor_cores=True))
+    for name, g, rf, tol in zip(NAMES, got, ref, (1e-2, 1e-4, 1e-4, 1e-2, 1e-3, 1e-4)):
+        assert rel_err(g.reshape(rf.shape), rf) <= tol, name
 
 
 def test_tensor_core_backward_long_sequence_one_head(cuda_device):
