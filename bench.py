@@ -589,7 +589,7 @@ def sec_vrwkv_b_dense(cx):
 
 def sec_vrwkv6_b_inference(cx):
     """VRWKV6-B (embed 768, 12 heads, 12 blocks) inference, 64 images of 224x224 per GPU: under autocast r, k, v
-    reach the WKV6 operator in bfloat16 and the tcgen05 forward runs."""
+    reach the WKV6 operator in bfloat16 and the tcgen05 walk in 16-token blocks runs."""
     from vision_rwkv_b200.backbone6 import build_v6
     B = 64
     model6 = build_v6("vrwkv6_b").to(cx.dev).eval()
@@ -615,7 +615,7 @@ def _wkv6_inputs(cx, B, T, H, dtype):
 
 def sec_wkv6(cx, total=32, long_only=False):
     """WKV6 as in VRWKV6-B: C=768, 12 heads of 64, 32 sequences split over the ranks, forward + backward.
-    T=196 in fp32 (exact sweeps) and bf16 (tcgen05 kernels); T=4096 in bf16 with its roofline: algorithmic
+    T=196 in fp32 (state sweeps) and bf16 (64-token chunks); T=4096 in bf16 with its roofline: algorithmic
     bytes 28 per element if every tensor moved as bfloat16 (forward reads r, k, v, w and writes y; backward
     reads r, k, v, w, gy and writes gr, gk, gv, gw), 3584 flops per element in the chunked formulation
     (14 head-size products of 2 x 64 flops each: 4 forward, 10 backward)."""
@@ -633,7 +633,7 @@ def sec_wkv6(cx, total=32, long_only=False):
     rh, kh, vh, gh = (x.bfloat16() for x in (r, k, v, gy))
     ms, f, b = _pair_ms(cx, lambda: ops.wkv6_forward(rh, kh, vh, w, u, H, tensor_cores=True),
                         lambda _: ops.wkv6_backward(rh, kh, vh, w, u, gh, H, tensor_cores=True))
-    out["wkv6_fwd_bwd_t196_bf16"] = {"ms": ms, "fwd_ms": f, "bwd_ms": b, "kernels": "tcgen05 forward and backward",
+    out["wkv6_fwd_bwd_t196_bf16"] = {"ms": ms, "fwd_ms": f, "bwd_ms": b, "kernels": "64-token chunks, mma.sync, bf16 operands",
                                      "elements_per_s": total * 196 * C / (ms * 1e-3)}
     del r, k, v, w, gy, rh, kh, vh, gh
     return _wkv6_long(cx, out, total, n, H, exact_too=True)
@@ -651,7 +651,7 @@ def _wkv6_long(cx, out, total, n, H, exact_too):
     tf = 3584 * E / (ms * 1e-3) / 1e12
     moved = 42 * E / (ms * 1e-3) / 1e9
     out["wkv6_fwd_bwd_t4096_bf16"] = {
-        "ms": ms, "fwd_ms": f, "bwd_ms": b, "kernels": "tcgen05 forward and backward", "T": T,
+        "ms": ms, "fwd_ms": f, "bwd_ms": b, "kernels": "64-token chunks, mma.sync, bf16 operands", "T": T,
         "elements_per_s": E / (ms * 1e-3),
         "roofline": {"hbm": {"achieved": gbs, "peak": cx.hbm * cx.world, "unit": "GB/s", "frac": gbs / (cx.hbm * cx.world),
                              "algorithmic_bytes_per_element": 28,

@@ -7,11 +7,9 @@ classification/mmcls_custom/models/backbones/vrwkv6.py:75-477 (`q_shift_multihea
 time_maa_g,time_maa_w1,time_maa_w2,time_decay,time_decay_w1,time_decay_w2,time_faaaa,key,value,
 receptance,gate,output,ln_x}`, `layers.N.ffn.{spatial_mix_k,spatial_mix_r,key,receptance,value}`.
 
-Kernels of this package: the recurrence (`RUN_CUDA_RWKV6`: the tcgen05 forward when r, k, v
-arrive in half / bfloat16, i.e. under autocast; exact fp32 sweeps otherwise and for every
-backward) and the ChannelMix's per-head token shift + two interpolations (`qshift_mix(...,
-head_dim=64)`).  The SpatialMix's shift feeds low-rank data-dependent mixes and stays a torch
-slice copy, like the GroupNorm / gate epilogue.
+Kernels of this package: the recurrence (`inference_rwkv6`; bfloat16 operands on the tensor cores when r, k, v arrive in
+half / bfloat16, i.e. under autocast, float32 state sweeps otherwise), the token shifts with their interpolations
+(`qshift_ddlerp`, `qshift_mix(..., head_dim=64)`), the per-head norm with its gate, and in inference the steps of `epilogue`.
 """
 from __future__ import annotations
 
@@ -153,7 +151,7 @@ class BlockV6(nn.Module):
             x = self.ln0(x)
         g1 = self.gamma1 if self.layer_scale else None
         g2 = self.gamma2 if self.layer_scale else None
-        # torch's own LayerNorm: these networks answer a change of a single rounding with 2 % of their result (see
+        # torch's own LayerNorm: these networks answer a change of a single rounding with 3 % of their result (see
         # vrwkv6.inference_rwkv6), so only steps that keep every bit are taken over
         if self.post_norm:
             x = epilogue.residual(x, self.ln1(self.att(x, resolution)), g1)

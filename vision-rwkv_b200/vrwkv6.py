@@ -100,9 +100,10 @@ def RUN_CUDA_RWKV6(B, T, C, H, r, k, v, w, u):
 
 def inference_rwkv6(B, T, C, H, r, k, v, w, u):
     """The recurrence inside `backbone6` networks: `RUN_CUDA_RWKV6`, except that inference on bfloat16 r, k, v keeps the
-    kernel that walks 16-token blocks.  In these networks a change of a single rounding anywhere ends up, twelve blocks
-    on, as a relative change of about 0.02 to 0.03 of the result (measured with kernels that agree to 1e-6), so a
-    network that is only being run keeps the bits it had."""
+    kernel that walks 16-token blocks.  These networks amplify a change of a single rounding: with the chunked kernels instead
+    of the walk the results differ by 0.031 (small model) and 0.032 (base) in the 2-norm, and neither is the better one,
+    0.0402 and 0.0404, 0.0419 and 0.0416 off a float64 evaluation (2 images of 224 pixels, layer scale 1, bfloat16
+    autocast).  So a network that is only being run keeps the bits it had."""
     if (not torch.is_grad_enabled() and FORWARD_PATH == "auto" and r.dtype == k.dtype == v.dtype == torch.bfloat16
             and not (ops.CHECK_STATUS or traced.tracing())):
         return _lib.native().wkv6_walk(r, k, v, w, u)
