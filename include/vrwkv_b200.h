@@ -182,8 +182,8 @@ int vrwkv_biwkv_forward_f32_noalloc(int B, int T, int C, const float* w, const f
 int vrwkv_wkv6_forward_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,
                            const float* w_raw, const float* u, float* y, void* stream);
 
-/* vrwkv_wkv6_forward.  exact = 1: float32 r, k, v and the kernels of vrwkv_wkv6_forward_f32; the workspace is a status
- * word.  exact = 0: 64-token chunks on the tensor cores (the states that enter each chunk, then all chunks in parallel):
+/* vrwkv_wkv6_forward.  exact = 1: float32 r, k, v and float32 accuracy, as vrwkv_wkv6_forward_f32, but a few sequences
+ * are walked in several segments at a time (at most 19 MB of scratch, none where the sequences fill the device).  exact = 0: 64-token chunks on the tensor cores (the states that enter each chunk, then all chunks in parallel):
  * r, k, v enter the matrix products as bfloat16 (in_bf16 = 1: they are bfloat16 bit patterns and are read as such; 0:
  * float32, rounded on the way in), sums are fp32; results agree with exact = 1 to about 1e-2 of max|y|.  w_raw, u and y are
  * float32.

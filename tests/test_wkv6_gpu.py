@@ -125,6 +125,32 @@ def test_heads_and_batches_are_independent(cuda_device):
         assert torch.equal(f[b:b + 1, :, sl], o), name
 
 
+# few blocks: sequences in segments (forward from T = 48, backward from 96), the last one short, a single token, or full; many: whole
+@pytest.mark.parametrize("B,T,H", [(1, 47, 1), (1, 48, 2), (2, 49, 1), (1, 95, 1), (1, 96, 2), (2, 97, 1), (1, 129, 3), (1, 777, 1),
+                                   (37, 40, 6), (25, 130, 3)])
+def test_segments_against_the_whole_walk(cuda_device, B, T, H):
+    """Forward against the call without scratch memory, which never cuts a sequence: the same products of decays, other places of
+    rounding (1e-6 of the maximum).  Backward against the oracle."""
+    from vision_rwkv_b200 import _lib
+    lib = _lib.load()
+    args = strong_tokens(B, T, H, seed=T + H, levels=(4.0, 30.0))
+    got = run_gpu(cuda_device, *args, H)
+    f = [x.float().contiguous().to(cuda_device) for x in args[:5]]
+    whole = torch.empty(B, T, 64 * H, device=cuda_device)
+    assert lib.vrwkv_wkv6_forward_f32(B, T, 64 * H, H, *[x.data_ptr() for x in f], whole.data_ptr(),
+                                      torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert rel_err(got[0], whole.double().cpu()) <= 1e-6
+    if B * T * H > 3000:      # the oracle keeps every state
+        return
+    ref = reference(*args, H)
+    for name, g, rf in zip(NAMES, got, ref):
+        if name == "gw":
+            check_decay_gradient(g, rf, args[3], TOL)
+        else:
+            assert rel_err(g.reshape(rf.shape), rf) <= TOL, name
+
+
 def test_bitwise_reproducible(cuda_device):
     args = O.make_inputs(2, 90, 128, 2, seed=5)
     a = run_gpu(cuda_device, *args, 2)

@@ -321,7 +321,7 @@ size_t vrwkv_wkv6_backward_workspace_bytes(int B, int T, int C, int H) {
 
 size_t vrwkv_wkv6_forward_workspace_bytes(int B, int T, int C, int H, int exact) {
     if (check_wkv6(B, T, C, H) != VRWKV_OK) return 0;
-    return exact ? 256 : wkv6c::forward_workspace(B, T, H);      // exact: the status word
+    return exact ? wkv6::forward_workspace(B, T, H) : wkv6c::forward_workspace(B, T, H);
 }
 
 int vrwkv_wkv6_forward(int B, int T, int C, int H, const void* r, const void* k, const void* v, int in_bf16, int exact,
@@ -337,7 +337,7 @@ int vrwkv_wkv6_forward(int B, int T, int C, int H, const void* r, const void* k,
     cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
     if (exact)
         return finish(wkv6::forward(B, T, H, static_cast<const float*>(r), static_cast<const float*>(k), static_cast<const float*>(v), w_raw, u,
-                                    y, s));
+                                    y, workspace, s));
     return finish(wkv6c::forward(B, T, H, r, k, v, w_raw, u, y, in_bf16 != 0, workspace, s));
 }
 
@@ -348,7 +348,7 @@ int vrwkv_wkv6_forward_f32(int B, int T, int C, int H, const float* r, const flo
     if (misaligned16(r) || misaligned16(k) || misaligned16(v) || misaligned16(w_raw) || misaligned4(u) ||
         misaligned4(y))
         return VRWKV_ERR_ALIGNMENT;
-    return finish(wkv6::forward(B, T, H, r, k, v, w_raw, u, y, static_cast<cudaStream_t>(stream)));
+    return finish(wkv6::forward(B, T, H, r, k, v, w_raw, u, y, nullptr, static_cast<cudaStream_t>(stream)));
 }
 
 int vrwkv_wkv6_forward_tc_f32(int B, int T, int C, int H, const float* r, const float* k, const float* v,

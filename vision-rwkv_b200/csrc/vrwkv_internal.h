@@ -79,9 +79,10 @@ int backward_bf16(int B, int T, int C, const float* w, const float* u, const voi
 }  // namespace biwkv
 
 namespace wkv6 {
-// float32 state sweeps (wkv6_sweeps.cu); gv may be null
+// float32 state sweeps (wkv6_sweeps.cu); gv may be null, and the forward's workspace
+size_t forward_workspace(int B, int T, int H);
 int forward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
-            const float* u, float* y, cudaStream_t stream);
+            const float* u, float* y, void* workspace, cudaStream_t stream);
 size_t backward_workspace(int B, int T, int H);
 int backward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
              const float* u, const float* gy, float* gr, float* gk, float* gv, float* gw, float* gu,
