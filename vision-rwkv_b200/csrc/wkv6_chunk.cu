@@ -88,10 +88,8 @@ __device__ __forceinline__ void scale_chunk(const float* wt, const XT* xt, const
 #pragma unroll
     for (int t = 0; t < kBlock; ++t) {
         const float2 w = *reinterpret_cast<const float2*>(wt + (row0 + t) * N + 2 * lane);
-        if (row0 + t < valid) {
-            run.x += log2_decay(w.x);
-            run.y += log2_decay(w.y);
-        }
+        run.x += log2_decay(w.x, row0 + t < valid);
+        run.y += log2_decay(w.y, row0 + t < valid);
         sum[t] = run;
     }
     if (writes) *reinterpret_cast<float2*>(&tot[warp][2 * lane]) = run;
@@ -457,10 +455,8 @@ __device__ __forceinline__ void scan_block(Table& tab, const float* w, int C, in
     float2 run = make_float2(0.f, 0.f);
 #pragma unroll
     for (int t = 0; t < kBlock; ++t) {
-        if (t < rows) {
-            run.x += log2_decay(wr[t].v.x);
-            run.y += log2_decay(wr[t].v.y);
-        }
+        run.x += log2_decay(wr[t].v.x, t < rows);
+        run.y += log2_decay(wr[t].v.y, t < rows);
         *reinterpret_cast<float2*>(&tab[blk * kBlock + t][2 * lane]) = run;
     }
 }

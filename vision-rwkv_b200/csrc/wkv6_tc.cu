@@ -59,12 +59,12 @@ struct Args {
 
 using sm100::smem_u32;
 
-// log of a token's decay, not below -104: e^-104 is zero in float32 already, and so bounded the running sums over a block
+// log of a token's decay, bounded at -104: e^-104 is zero in float32 already, and so bounded the running sums over a block
 // keep their smaller terms to 1e-4 (and stay finite) whatever a token's decay is.  NaN stays NaN.
 __device__ __forceinline__ float log_decay(float w) {
-    float l;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(l) : "f"(-__expf(w)), "f"(-104.f));
-    return l;
+    float x;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(x) : "f"(w), "f"(4.6444f));
+    return -__expf(x);
 }
 
 
