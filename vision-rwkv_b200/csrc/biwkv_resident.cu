@@ -784,7 +784,8 @@ __device__ __noinline__ void exact_subchunk(const Ctx& c, int sub, int ch, float
 // kWide (with kHalf): y and gy are float32 tensors, what a model with float32 w, u under autocast has; y still holds
 // bfloat16 values, and gy is rounded to bfloat16 as it is read: the results are those of the bfloat16 kernel.  Without it the caller widens y (6 bytes per element) and narrows gy (6 more) in
 // passes of their own, as many bytes as this kernel's own forward moves.  B=64, T=576, C=1024, forward + backward:
-// 468 us with those passes, 332 us without (forward alone at B=256, T=196, C=384: 103 and 53 us).
+// 468 us with those passes, 332 us without, 327 us now (three CTAs per sequence, and 4 us for gy's rounding); forward alone at B=256,
+// T=196, C=384: 103 and 53 us.
 // kMulti: several clusters per sequence (T above what one cluster holds); compiled apart so that the
 // single-cluster kernels carry none of it.
 template <bool kBwd, int kStash, bool kHalf, bool kWide, bool kMulti>
