@@ -51,8 +51,9 @@ const char* vrwkv_last_error_detail(void);
 unsigned long long vrwkv_launch_count(void);
 
 /* Kernel path selection, for tests and measurements: 0 = automatic (default: Bi-WKV takes the
- * cluster-resident single-pass kernels when T <= 32768, C % 4 == 0 (bfloat16: C % 8 == 0) and the
- * tensors are 16-byte aligned - one cluster per sequence strip up to T = 4096, several above -,
+ * cluster-resident kernels when T <= 32768, C % 4 == 0 (bfloat16: C % 8 == 0) and the
+ * tensors are 16-byte aligned - one cluster per sequence strip up to T = 4096, above it several or, for
+ * many tokens in all, separate launches -,
  * else the persistent tile kernels, else the generic multi-launch path), 1 = the
  * first-generation kernels (Bi-WKV: the generic multi-launch path; vrwkv_wkv6_forward_tc_*: the walk
  * that needs no scratch memory, whatever the workspace holds), 2 = Bi-WKV skips the
@@ -149,6 +150,23 @@ int vrwkv_biwkv_forward_bf16_wide(int B, int T, int C, const float* w, const flo
 int vrwkv_biwkv_backward_bf16_wide(int B, int T, int C, const float* w, const float* u, const uint16_t* k, const uint16_t* v,
                                    const float* gy, float* gwgu, uint16_t* gk, uint16_t* gv, void* workspace, size_t workspace_bytes,
                                    void* stream);
+
+/* The training pair for long sequences: a forward that leaves the states entering every 16 tokens (1.5 bytes per element, in a
+ * caller-owned buffer of vrwkv_biwkv_kept_bytes bytes, 256-byte aligned), and a backward that starts from them instead of
+ * rebuilding them: two passes over the inputs instead of three.  vrwkv_biwkv_kept_bytes is 0 where a backward has no use for
+ * them (T <= 4096, or few tokens in all).
+ * w, u, k, v of the backward must be those of the forward.  `tensors` says what k, v, y, gy, gk, gv hold (enum below, as in the
+ * entry points above); workspaces are those of the other entry points.  VRWKV_ERR_UNSUPPORTED: outside the cluster-resident
+ * kernels (shape, alignment, vrwkv_set_path), nothing ran, use the other entry points; a forward may succeed and the backward
+ * still return it (for an unaligned gy).  Results agree with the pair that keeps nothing to float32 rounding; y is the same bit for bit.
+ * No reference counterpart (its backward rebuilds everything, bi_wkv_kernel.cu:259-302). */
+enum vrwkv_tensors { VRWKV_TENSORS_F32 = 0, VRWKV_TENSORS_BF16 = 1, VRWKV_TENSORS_BF16_WIDE = 2 };
+size_t vrwkv_biwkv_kept_bytes(int B, int T, int C);
+int vrwkv_biwkv_forward_keep(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, int tensors,
+                             void* kept, size_t kept_bytes, void* workspace, size_t workspace_bytes, void* stream);
+int vrwkv_biwkv_backward_kept(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy,
+                              float* gwgu, void* gk, void* gv, int tensors, const void* kept, size_t kept_bytes, void* workspace,
+                              size_t workspace_bytes, void* stream);
 
 /* vrwkv_biwkv_forward_f32_noalloc has no counterpart in the reference.  It is
  * vrwkv_biwkv_forward_f32 for callers that cannot allocate device memory and so have no

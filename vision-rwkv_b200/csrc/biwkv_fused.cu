@@ -1410,6 +1410,7 @@ bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool
 }
 
 size_t workspace_bytes(int B, int T, int C, bool bwd) { return make_layout(B, T, C, bwd).total; }
+size_t cleared_bytes(int B, int T, int C, bool bwd) { return make_layout(B, T, C, bwd).off_exch; }
 
 template <bool kBwd, typename E>
 static int launch(Layout& l, const float* w, const float* u, const E* k, const E* v, const E* gy, E* o0, E* o1,
@@ -1427,14 +1428,16 @@ static int launch(Layout& l, const float* w, const float* u, const E* k, const E
     CUtensorMap mk, mv, mg, m0, m1;
     bool ok = make_map<E>(&mk, k, p.B, p.T, p.C) && make_map<E>(&mv, v, p.B, p.T, p.C) &&
               make_map<E>(&m0, o0, p.B, p.T, p.C);
-    ok = ok && make_map<E>(&mg, kBwd ? gy : k, p.B, p.T, p.C) &&
-         make_map<E>(&m1, (kBwd || o1 != nullptr) ? o1 : o0, p.B, p.T, p.C);
+    if (kBwd) ok = ok && make_map<E>(&mg, gy, p.B, p.T, p.C);
+    else mg = mk;                                            // not used
+    if (kBwd || o1 != nullptr) ok = ok && make_map<E>(&m1, o1, p.B, p.T, p.C);
+    else m1 = m0;                                            // not used
     if (!ok) {
         set_error_detail("cuTensorMapEncodeTiled rejected a (C, T, B) tensor map");
         return -1;
     }
     // status word + flags start at zero
-    cudaMemsetAsync(ws, 0, l.off_exch, stream);
+    if (run_if == nullptr) cudaMemsetAsync(ws, 0, l.off_exch, stream);
     const DeviceInfo& d = device_info();
     const int grid = std::min(p.n_tiles, d.sms * d.resident[std::is_same<E, float>::value ? 0 : 1][kBwd ? 1 : 0]);
     void* args[] = {&mk, &mv, &mg, &m0, &m1, &p};

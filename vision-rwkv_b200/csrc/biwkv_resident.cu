@@ -1,5 +1,5 @@
-// Bi-WKV "resident" path: the whole token range of one (sequence, 32-channel strip) is held in the
-// shared memory of ONE thread-block cluster while it is scanned in both directions, so every
+// Bi-WKV "resident" path (long sequences in number go another way, see biwkv_chain_kernel): the whole token range of one
+// (sequence, 32-channel strip) is held in the shared memory of ONE thread-block cluster while it is scanned in both directions, so every
 // element of k, v (and gy) crosses HBM once in and every output once out, and nothing but the
 // cluster's own CTAs ever has to be waited for.
 //
@@ -73,10 +73,21 @@ enum ConstRow {
     kLam = 0, kWl2, kCuw, kLam16_hi, kLam16_lo, kLam32_hi, kLam32_lo, kLamC_hi, kLamC_lo, kConstRows
 };
 
+// What one launch computes.
+enum class Mode {
+    whole,      // every level: the CTAs of one cluster hold the sequence and exchange their sums
+    linked,     // every level: several clusters hold the sequence, hand-over through global memory
+    sums,       // no clusters: the sums of level 1 (forward) or level 2 (backward, level 1 given) of every sub-chunk and CTA
+    sums_keep,  // forward: as sums, with the first moments that a backward needs
+    spread,     // no clusters: every level given; writes the results
+};
+template <Mode m>
+constexpr bool kUsesCluster = m == Mode::whole || m == Mode::linked;
+
 // rows of kCs floats in the record area behind the data slots
-template <bool kBwd>
-struct Rows {
-    static constexpr int kF = kBwd ? 4 : 2;       // towards later tokens: a, b (, first moments)
+template <bool kMom, bool kBwd>
+struct RowsOf {
+    static constexpr int kF = kMom ? 4 : 2;       // towards later tokens: a, b (, first moments)
     static constexpr int kR = 2;                  // towards earlier tokens: a, b
     static constexpr int kSub = kF + kR;          // per span
     static constexpr int kLevels = kBwd ? 2 : 1;
@@ -85,6 +96,13 @@ struct Rows {
     static constexpr int kBlockR = kCs * kR + 4;   // ... towards earlier tokens
     static constexpr int kPeerFloats = (kMaxCluster - 1) * kBlockF;   // one block slot per other rank (ranks above this CTA's shift down by one)
 };
+template <bool kBwd, Mode kMode = Mode::whole>
+using Rows = RowsOf<kBwd || kMode == Mode::sums_keep, kBwd>;
+constexpr int kStateRows = 6;      // states that enter a sub-chunk: P (n, d), its first moment (n, d), S (n, d)
+constexpr int kPlainRows = 4;      // ... without the moments
+// rows of the state that enters the CTA
+template <bool kBwd, Mode kMode>
+constexpr int kOutsideRows = kUsesCluster<kMode> ? Rows<kBwd, kMode>::kSub : kStateRows;
 
 struct Params {
     int B, T, C;
@@ -101,22 +119,33 @@ struct Params {
     int* redo_list;         // ... and which
     uint32_t spin_limit;  // polls before a wait for the other CTAs gives up
     int withhold_rank;    // test only: this rank of every cluster sends nothing (-1: none)
-    // sequences longer than one cluster holds: `segs` clusters per (sequence, strip), each with
+    int ctas;             // CTAs per (sequence, strip)
+    // sequences longer than one cluster holds, several clusters: `segs` clusters per (sequence, strip), each with
     // cluster * n_tok tokens, which hand their aggregates to one another through global memory
     int segs;
     float* xseg;          // [unit][seg][level][direction][kSegRec]
     unsigned* xflag;      // same index; zero before launch, 1 (| 2: out of range) once the record is there
+    // Without clusters: states that enter sub-chunks, [unit][CTA][sub-chunk][state_rows][kCs], relative to their CTA, and states
+    // that enter CTAs, [unit][CTA][state_rows][kCs], which are the CTAs' own sums until biwkv_chain_kernel has run
+    float* states1;
+    float* ctas1;
+    float* states2;       // level 2 (backward)
+    float* ctas2;
+    int state_rows;       // kStateRows, or kPlainRows where no moments are kept
+    unsigned* out_of_range;   // sequences longer than one cluster holds: inputs outside the plain-float range were seen; else null
+    bool reverse;         // last CTAs first: what the launch before this one read last is still in L2
 };
+
 constexpr int kSegRec = 4 * kCs;      // floats per record (forward: 2 rows used)
 constexpr int kMaxSegs = 8;
 
 // shared memory: data slots | span records | blocks received from the other CTAs | this CTA's two
 // outgoing blocks | state entering this CTA | constants | mbarriers and the flag word
-template <bool kBwd>
+template <bool kBwd, Mode kMode = Mode::whole>
 static inline size_t smem_bytes(int n_warps) {
-    using R = Rows<kBwd>;
+    using R = Rows<kBwd, kMode>;
     const size_t data = static_cast<size_t>(R::kSlots) * n_warps * kSpan * kCs * sizeof(float);
-    const size_t rec = (static_cast<size_t>(n_warps) * R::kSub * kCs + R::kPeerFloats + R::kBlockF + R::kBlockR + R::kSub * kCs + kConstRows * kCs) * sizeof(float);
+    const size_t rec = (static_cast<size_t>(n_warps) * R::kSub * kCs + (kUsesCluster<kMode> ? R::kPeerFloats : 0) + R::kBlockF + R::kBlockR + kOutsideRows<kBwd, kMode> * kCs + kConstRows * kCs) * sizeof(float);
     return data + rec + 192;
 }
 
@@ -212,6 +241,7 @@ struct Ctx {
     int seg, segs, unit;     // this cluster's segment of the sequence
     float* xseg;
     unsigned* xflag;
+    float* cta_sums;         // launches without clusters: where this CTA's sums go, [state_rows][kCs]
 };
 
 // a thread's two channels: numerators (n) and denominators (d) of a state, each packed (ch 2p, ch 2p+1)
@@ -364,9 +394,8 @@ __device__ __noinline__ void seg_exchange_reverse(const Ctx& c, int level, float
     }
 }
 // OR of this CTA's and the other CTAs' out-of-range flags (level 0), from the flag words of the blocks they sent
-template <bool kBwd>
+template <typename RW>
 __device__ __forceinline__ int cluster_flag(const Ctx& c, int any) {
-    using RW = Rows<kBwd>;
     const int lane = c.lane;
     const int other = (lane < c.cluster && lane != c.rank)
                           ? __float_as_int(c.peers[(lane - (lane > c.rank ? 1 : 0)) * RW::kBlockF + kCs * (lane < c.rank ? RW::kF : RW::kR)]) : 0;
@@ -377,10 +406,11 @@ __device__ __forceinline__ int cluster_flag(const Ctx& c, int any) {
 // aggregate relative to the first token after its 16 tokens (and its first moment in distance), R:
 // relative to the last token before them.  Returns with `unsafe` = OR over the cluster of `unsafe`
 // (level 0 only).
-template <bool kBwd, bool kMulti>
+//
+// kLocal: no cluster; the states returned are relative to the CTA, whose own sums go to memory.  kLinked: several clusters.
+template <typename RW, bool kLocal, bool kLinked>
 __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F, Pair2 MF, Pair2 R, bool& unsafe TL_ARGS) {
-    using RW = Rows<kBwd>;
-    constexpr bool kMom = kBwd;
+    constexpr bool kMom = RW::kF == 4;
     const int lane = c.lane, warp = c.warp, nw = c.n_warps;
     const int p = lane & 15;
     const bool upper = lane >= 16;
@@ -444,12 +474,17 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
             }
         }
         if (level == 1) TL_MARK(23);
-        if (kMulti) { ctaP = P; ctaM = M; }
-        // the CTA's aggregate (and its flag) for the higher ranks: into the outgoing block
-        float* st = c.stage;
-        if (kMom) *reinterpret_cast<float4*>(st + lane * 4) = make_float4(P.x, P.y, M.x, M.y);
-        else *reinterpret_cast<float2*>(st + lane * 2) = P;
-        if (lane == 0) st[kCs * RW::kF] = __int_as_float(any);
+        if (kLinked) { ctaP = P; ctaM = M; }
+        if (kLocal) {
+            c.cta_sums[lane] = P.x; c.cta_sums[kCs + lane] = P.y;
+            if (kMom) { c.cta_sums[2 * kCs + lane] = M.x; c.cta_sums[3 * kCs + lane] = M.y; }
+        } else {
+            // the CTA's aggregate (and its flag) for the higher ranks: into the outgoing block
+            float* st = c.stage;
+            if (kMom) *reinterpret_cast<float4*>(st + lane * 4) = make_float4(P.x, P.y, M.x, M.y);
+            else *reinterpret_cast<float2*>(st + lane * 2) = P;
+            if (lane == 0) st[kCs * RW::kF] = __int_as_float(any);
+        }
     }
     if (warp == scanR) {
         const float2 hi2 = dup(c.consts[kLam32_hi * kCs + lane]), lo2 = dup(c.consts[kLam32_lo * kCs + lane]);
@@ -471,19 +506,23 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
                 S = mulc_add(S, hi2, lo2, r[s]);
             }
         }
-        if (kMulti) ctaS = S;
-        float* st = c.stage + RW::kBlockF;
-        *reinterpret_cast<float2*>(st + lane * 2) = S;
-        if (lane == 0) st[kCs * RW::kR] = __int_as_float(any);
+        if (kLinked) ctaS = S;
+        if (kLocal) {
+            c.cta_sums[RW::kF * kCs + lane] = S.x; c.cta_sums[(RW::kF + 1) * kCs + lane] = S.y;
+        } else {
+            float* st = c.stage + RW::kBlockF;
+            *reinterpret_cast<float2*>(st + lane * 2) = S;
+            if (lane == 0) st[kCs * RW::kR] = __int_as_float(any);
+        }
     }
     // every warp sends the blocks to its share of the other CTAs (rank = warp, warp + n_warps, ...):
     // lane = channel, one record per lane, lane 0 also the flag word
     if (level == 1) TL_MARK(24);
-    if (c.cluster > 1) {
+    if (!kLocal && c.cluster > 1) {
         __syncthreads();
     }
     if (level == 1) TL_MARK(25);
-    if (c.cluster > 1 && !c.withhold) {
+    if (!kLocal && c.cluster > 1 && !c.withhold) {
         const uint32_t bar_off = sm100::smem_u32(c.xbar + level) - sm100::smem_u32(c.peers);
         for (int r = warp; r < c.cluster; r += nw) {
             if (r == c.rank) continue;
@@ -501,11 +540,11 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     }
     TL_MARK(13 + level * 5);
     // (3) wait for the other CTAs' bytes, combine them
-    if (c.cluster > 1 && (warp == scanF || warp == scanR)) {
+    if (!kLocal && c.cluster > 1 && (warp == scanF || warp == scanR)) {
         if (!sm100::mbar_wait(c.xbar + level, 0, c.spin_limit) && lane == 0) report_failure(c.status, c.mirror, 1u);
     }
     TL_MARK(14 + level * 5);
-    if (warp == scanF) {
+    if (!kLocal && warp == scanF) {
         float2 X = f2(0.f, 0.f), MX = f2(0.f, 0.f);
         int flag = any;
         if (c.cluster > 1) {
@@ -536,14 +575,14 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
                     }
                 }
             }
-            if (level == 0) flag = cluster_flag<kBwd>(c, any);
+            if (level == 0) flag = cluster_flag<RW>(c, any);
         }
-        if (kMulti) seg_exchange_forward<kMom>(c, level, X, MX, ctaP, ctaM, flag);
+        if (kLinked) seg_exchange_forward<kMom>(c, level, X, MX, ctaP, ctaM, flag);
         c.cta[lane] = X.x; c.cta[kCs + lane] = X.y;
         if (kMom) { c.cta[2 * kCs + lane] = MX.x; c.cta[3 * kCs + lane] = MX.y; }
         if (lane == 0) c.flag[0] = static_cast<unsigned>(flag);
     }
-    if (warp == scanR) {
+    if (!kLocal && warp == scanR) {
         float2 Y = f2(0.f, 0.f);
         if (c.cluster > 1) {
             const float2 hi2 = dup(c.consts[kLamC_hi * kCs + lane]), lo2 = dup(c.consts[kLamC_lo * kCs + lane]);
@@ -559,9 +598,9 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
                     if (r0 - j > c.rank) Y = mulc_add(Y, hi2, lo2, f[j]);
             }
         }
-        if (kMulti) {
+        if (kLinked) {
             int flag = 0;
-            if (level == 0) flag = c.cluster > 1 ? cluster_flag<kBwd>(c, any) : any;
+            if (level == 0) flag = c.cluster > 1 ? cluster_flag<RW>(c, any) : any;
             seg_exchange_reverse(c, level, Y, ctaS, flag);
             if (lane == 0) c.flag[1] = static_cast<unsigned>(flag);
         }
@@ -573,22 +612,23 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     // (4) outside state moved to this span's edges + inside state; then to this half's edges
     Enter e;
     {
-        const float2 wl2 = *reinterpret_cast<const float2*>(c.consts + kWl2 * kCs + 2 * p);
-        const float dP = static_cast<float>(kSpan * warp), dS = static_cast<float>(kSpan * (nw - 1 - warp));
-        const float2 pP = f2(ex2(-wl2.x * dP), ex2(-wl2.y * dP)), pS = f2(ex2(-wl2.x * dS), ex2(-wl2.y * dS));
         const float* s = c.sub + warp * (RW::kSub * kCs) + 2 * p;
-        const float* g = c.cta + 2 * p;
-        const float2 Xn = *reinterpret_cast<const float2*>(g), Xd = *reinterpret_cast<const float2*>(g + kCs);
-        Pair2 Pw{fma2(pP, Xn, *reinterpret_cast<const float2*>(s)), fma2(pP, Xd, *reinterpret_cast<const float2*>(s + kCs))};
-        Pair2 MPw{f2(0.f, 0.f), f2(0.f, 0.f)};
-        if (kMom) {
-            const float2 MXn = *reinterpret_cast<const float2*>(g + 2 * kCs), MXd = *reinterpret_cast<const float2*>(g + 3 * kCs);
-            MPw.n = fma2(pP, fma2(dup(dP), Xn, MXn), *reinterpret_cast<const float2*>(s + 2 * kCs));
-            MPw.d = fma2(pP, fma2(dup(dP), Xd, MXd), *reinterpret_cast<const float2*>(s + 3 * kCs));
+        const auto row = [](const float* x, int r) { return *reinterpret_cast<const float2*>(x + r * kCs); };
+        Pair2 Pw{row(s, 0), row(s, 1)}, MPw{f2(0.f, 0.f), f2(0.f, 0.f)}, Sw{row(s, RW::kF), row(s, RW::kF + 1)};
+        if (kMom) MPw = Pair2{row(s, 2), row(s, 3)};
+        if (!kLocal) {
+            const float2 wl2 = row(c.consts + 2 * p, kWl2);
+            const float dP = static_cast<float>(kSpan * warp), dS = static_cast<float>(kSpan * (nw - 1 - warp));
+            const float2 pP = f2(ex2(-wl2.x * dP), ex2(-wl2.y * dP)), pS = f2(ex2(-wl2.x * dS), ex2(-wl2.y * dS));
+            const float* g = c.cta + 2 * p;
+            const float2 Xn = row(g, 0), Xd = row(g, 1);
+            if (kMom) {
+                MPw.n = fma2(pP, fma2(dup(dP), Xn, row(g, 2)), MPw.n);
+                MPw.d = fma2(pP, fma2(dup(dP), Xd, row(g, 3)), MPw.d);
+            }
+            Pw = Pair2{fma2(pP, Xn, Pw.n), fma2(pP, Xd, Pw.d)};
+            Sw = Pair2{fma2(pS, row(g, RW::kF), Sw.n), fma2(pS, row(g, RW::kF + 1), Sw.d)};
         }
-        const float2 Yn = *reinterpret_cast<const float2*>(g + RW::kF * kCs), Yd = *reinterpret_cast<const float2*>(g + (RW::kF + 1) * kCs);
-        Pair2 Sw{fma2(pS, Yn, *reinterpret_cast<const float2*>(s + RW::kF * kCs)),
-                 fma2(pS, Yd, *reinterpret_cast<const float2*>(s + (RW::kF + 1) * kCs))};
         if (upper) {
             e.P = Pair2{mulc_add(Pw.n, l16h, l16l, keepA.n), mulc_add(Pw.d, l16h, l16l, keepA.d)};
             e.MP = Pair2{mulc_add(fma2(len16, Pw.n, MPw.n), l16h, l16l, keepM.n), mulc_add(fma2(len16, Pw.d, MPw.d), l16h, l16l, keepM.d)};
@@ -598,9 +638,38 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
             e.MP = MPw;
             e.S = Pair2{mulc_add(Sw.n, l16h, l16l, keepA.n), mulc_add(Sw.d, l16h, l16l, keepA.d)};
         }
-        if (level == 0) unsafe = kMulti ? (c.flag[0] | c.flag[1]) != 0u : c.flag[0] != 0u;
+        if (level == 0) unsafe = kLocal ? any != 0 : kLinked ? (c.flag[0] | c.flag[1]) != 0u : c.flag[0] != 0u;
     }
     return e;
+}
+
+// ---- states kept in memory ---------------------------------------------------------------------
+__device__ __forceinline__ void put_state(float* at, int rows, const Enter& e, bool moments) {
+    const auto put = [&](int r, float2 v) { *reinterpret_cast<float2*>(at + r * kCs) = v; };
+    put(0, e.P.n); put(1, e.P.d);
+    if (moments) { put(2, e.MP.n); put(3, e.MP.d); }
+    put(rows - 2, e.S.n); put(rows - 1, e.S.d);
+}
+template <bool kMom>
+__device__ __forceinline__ Enter get_state(const float* at, int rows) {
+    const auto get = [&](int r) { return __ldg(reinterpret_cast<const float2*>(at + r * kCs)); };
+    Enter e;
+    e.P = Pair2{get(0), get(1)};
+    e.MP = Pair2{f2(0.f, 0.f), f2(0.f, 0.f)};
+    if (kMom) e.MP = Pair2{get(2), get(3)};
+    e.S = Pair2{get(rows - 2), get(rows - 1)};
+    return e;
+}
+// e: relative to the CTA; g: what enters the CTA, rows of kCs floats in shared memory; dP, dS: tokens between the CTA's edges
+// and the sub-chunk's
+template <bool kMom>
+__device__ __forceinline__ void add_outside(Enter& e, const float* g, int rows, float2 wl2, float dP, float dS) {
+    const auto row = [&](int r) { return *reinterpret_cast<const float2*>(g + r * kCs); };
+    const float2 pP = f2(ex2(-wl2.x * dP), ex2(-wl2.y * dP)), pS = f2(ex2(-wl2.x * dS), ex2(-wl2.y * dS));
+    const float2 Xn = row(0), Xd = row(1);
+    e.P = Pair2{fma2(pP, Xn, e.P.n), fma2(pP, Xd, e.P.d)};
+    if (kMom) e.MP = Pair2{fma2(pP, fma2(dup(dP), Xn, row(2)), e.MP.n), fma2(pP, fma2(dup(dP), Xd, row(3)), e.MP.d)};
+    e.S = Pair2{fma2(pS, row(rows - 2), e.S.n), fma2(pS, row(rows - 1), e.S.d)};
 }
 
 // ---- exact path: (value, exponent) records, any exponent range -----------------------------------
@@ -786,18 +855,21 @@ __device__ __noinline__ void exact_subchunk(const Ctx& c, int sub, int ch, float
 // passes of their own, as many bytes as this kernel's own forward moves.  B=64, T=576, C=1024, forward + backward:
 // 468 us with those passes, 332 us without, 327 us now (three CTAs per sequence, and 4 us for gy's rounding); forward alone at B=256,
 // T=196, C=384: 103 and 53 us.
-// kMulti: several clusters per sequence (T above what one cluster holds); compiled apart so that the
-// single-cluster kernels carry none of it.
-template <bool kBwd, int kStash, bool kHalf, bool kWide, bool kMulti>
+template <bool kBwd, int kStash, bool kHalf, bool kWide, Mode kMode>
 __global__ void __launch_bounds__(kMaxThreads, kBwd ? 2 : 3)
 biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                       const __grid_constant__ CUtensorMap map_g,     // backward: gy
                       const __grid_constant__ CUtensorMap map_o0,    // forward: y ; backward: gk
                       const __grid_constant__ CUtensorMap map_o1,    // backward: gv
                       const Params p) {
-    using RW = Rows<kBwd>;
+    using RW = Rows<kBwd, kMode>;
     constexpr bool kHalfG = kHalf && !kWide;                    // gy arrives as bfloat16
     constexpr bool kHalfOut = kHalf && (kBwd || !kWide);        // results leave as bfloat16
+    constexpr bool kCluster = kUsesCluster<kMode>, kLinked = kMode == Mode::linked, kSums = kMode == Mode::sums || kMode == Mode::sums_keep;
+    constexpr bool kOwn1 = kCluster || (kSums && !kBwd);        // level 1 is this launch's to sum up; else given
+    constexpr bool kOwn2 = kBwd && kMode != Mode::spread;       // level 2 likewise
+    constexpr bool kMom1 = RW::kF == 4;                         // level 1 carries first moments
+    constexpr bool kResults = !kSums;                           // the launch writes results
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pr = lane & 15, upper = lane >> 4;
@@ -809,9 +881,9 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     Ctx c;
     c.sub = slot_k + RW::kSlots * slot_floats;
     c.peers = c.sub + nw * (RW::kSub * kCs);
-    c.stage = c.peers + RW::kPeerFloats;
+    c.stage = c.peers + (kCluster ? RW::kPeerFloats : 0);
     c.cta = c.stage + RW::kBlockF + RW::kBlockR;
-    c.consts = c.cta + RW::kSub * kCs;
+    c.consts = c.cta + kOutsideRows<kBwd, kMode> * kCs;
     uint64_t* full = reinterpret_cast<uint64_t*>(c.consts + kConstRows * kCs);   // [kMaxWarps]: k, v of one span each
     uint64_t* gfull = full + kMaxWarps;  // [kMaxWarps]: backward, gy of one span each (first needed in pass 2)
     c.xbar = gfull + kMaxWarps;
@@ -819,7 +891,9 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     c.status = p.status;
     c.mirror = p.mirror;
     c.warp = warp; c.lane = lane; c.n_warps = nw; c.n_tok = p.n_tok; c.cluster = p.cluster;
-    c.rank = p.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
+    const int blk_id = kMode == Mode::spread && p.reverse ? static_cast<int>(gridDim.x - 1 - blockIdx.x) : static_cast<int>(blockIdx.x);
+    const int unit = blk_id / p.ctas, cta = blk_id - unit * p.ctas;
+    c.rank = kCluster && p.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
     c.spin_limit = p.spin_limit;
     c.withhold = c.rank == p.withhold_rank;
 
@@ -840,13 +914,16 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     }
 #endif
     TL_MARK(0);
-    const int cl = static_cast<int>(blockIdx.x) / p.cluster;      // segments of a unit are neighbours in launch order
-    const int unit = kMulti ? cl / p.segs : cl, seg = kMulti ? cl - unit * p.segs : 0;
     const int b = unit / p.n_strips, strip = unit - b * p.n_strips;
-    const int tok0 = (seg * p.cluster + c.rank) * p.n_tok;
-    const uint32_t slot_bytes = static_cast<uint32_t>(slot_floats) * 4u;
-    c.seg = seg; c.segs = kMulti ? p.segs : 1; c.unit = unit;
-    c.xseg = p.xseg; c.xflag = p.xflag;
+    const int tok0 = cta * p.n_tok;
+    if (kCluster) {      // the segments of a unit are neighbours in launch order
+        c.seg = kLinked ? cta / p.cluster : 0; c.segs = kLinked ? p.segs : 1; c.unit = unit;
+        c.xseg = p.xseg; c.xflag = p.xflag;
+    }
+    // this thread's sub-chunk among the kept states, and the CTA's place among those of the CTAs
+    const int subs = 2 * nw, sub = 2 * warp + upper;
+    const size_t sub_at = ((static_cast<size_t>(blk_id) * subs + sub) * p.state_rows) * kCs + 2 * pr;
+    c.cta_sums = kSums ? (kBwd ? p.ctas2 : p.ctas1) + static_cast<size_t>(blk_id) * p.state_rows * kCs : nullptr;
 
     if (lane == 0) {
         // every warp fetches its own span: one box per tensor, k and v on one barrier, gy on another;
@@ -879,7 +956,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     if (threadIdx.x == 0) {
         for (int l = 0; l < RW::kLevels; ++l) sm100::mbar_init(c.xbar + l, 1);
         sm100::mbar_init_fence();
-        if (p.cluster > 1) {
+        if (kCluster && p.cluster > 1) {
             // bytes the other CTAs will send per level: a block from every lower rank (towards later
             // tokens) and from every higher rank (towards earlier ones)
             const uint32_t bytes = static_cast<uint32_t>(c.rank) * (kCs * RW::kF + 1) * 4u + static_cast<uint32_t>(p.cluster - 1 - c.rank) * (kCs * RW::kR + 1) * 4u;
@@ -887,6 +964,19 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
             if (kBwd) sm100::mbar_expect_tx(c.xbar + 1, bytes);
         }
     }
+    // given states: fetched while the tiles are on their way.  The rows of the CTA go to c.cta (level 1) and to the unused span
+    // records (level 2).
+    Enter e1, e2;
+    unsigned given_up = 0u;
+    if (!kOwn1) {
+        e1 = get_state<kBwd && !kSums>(p.states1 + sub_at, p.state_rows);
+        given_up = __ldg(p.out_of_range);
+        for (int i = threadIdx.x; i < p.state_rows * kCs; i += blockDim.x) {
+            c.cta[i] = __ldg(p.ctas1 + static_cast<size_t>(blk_id) * p.state_rows * kCs + i);
+            if (kBwd && !kSums) c.sub[i] = __ldg(p.ctas2 + static_cast<size_t>(blk_id) * kStateRows * kCs + i);
+        }
+    }
+    if (kBwd && !kOwn2) e2 = get_state<true>(p.states2 + sub_at, kStateRows);
     {
         // double precision once per channel: a rounded lambda multiplied up over thousands of tokens
         // would drift by distance * 6e-8.  Six exponentials, spread over the warps (lane = channel).
@@ -908,7 +998,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     // every CTA of the cluster has initialised its mbarriers before any other CTA sends to them:
     // arrive here, wait once the tiles have landed (long since complete by then)
     // (relaxed: the mbarrier-init fence above is what publishes the initialisation)
-    if (p.cluster > 1) cluster_arrive_relaxed();
+    if (kCluster && p.cluster > 1) cluster_arrive_relaxed();
     const int ch0 = strip * kCs + 2 * pr;
     const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
     const float2 u2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.u + ch0) : f2(0.f, 0.f);
@@ -918,7 +1008,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 
     TL_MARK(1);
     if (!sm100::mbar_wait(full + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
-    if (p.cluster > 1) cluster_wait();
+    if (kCluster && p.cluster > 1) cluster_wait();
     TL_MARK(2);
 
     const int row0 = warp * kSpan + upper * kL;
@@ -956,30 +1046,45 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
             for (int j = 0; j < kGroup; ++j) {
                 const int i = g + j;
                 const float2 k = kk[j], v = vv[j];
-                if (i < n) kmax = f2(fmaxf(kmax.x, fabsf(k.x)), fmaxf(kmax.y, fabsf(k.y)));
+                if (kOwn1 && i < n) kmax = f2(fmaxf(kmax.x, fabsf(k.x)), fmaxf(kmax.y, fabsf(k.y)));
                 const float2 t = fma2(k, l2e, nwl2);
                 const float2 e = f2(ex2(t.x), ex2(t.y));
                 const float2 zx = mul2(e, v);
-                k2[i * kRow] = zx;
-                v2[i * kRow] = e;
-                F.n = fma2(lam2, F.n, zx);
-                F.d = fma2(lam2, F.d, e);
-                if (kBwd) {
-                    MF.n = fma2(lam2, MF.n, F.n);
-                    MF.d = fma2(lam2, MF.d, F.d);
+                if (kResults || kBwd) {
+                    k2[i * kRow] = zx;
+                    v2[i * kRow] = e;
                 }
-                R.n = fma2(mu, zx, R.n);
-                R.d = fma2(mu, e, R.d);
-                mu = mul2(mu, lam2);
+                if (kOwn1) {
+                    F.n = fma2(lam2, F.n, zx);
+                    F.d = fma2(lam2, F.d, e);
+                    if (kMom1) {
+                        MF.n = fma2(lam2, MF.n, F.n);
+                        MF.d = fma2(lam2, MF.d, F.d);
+                    }
+                    R.n = fma2(mu, zx, R.n);
+                    R.d = fma2(mu, e, R.d);
+                    mu = mul2(mu, lam2);
+                }
             }
         }
     }
-    const float Tf = static_cast<float>(p.T);
-    bool unsafe = (2.f * kmax.x + fabsf(u2.x) + fabsf(w2.x) + fmaxf(-w2.x, 0.f) * Tf > kSafeRange) ||
-                  (2.f * kmax.y + fabsf(u2.y) + fabsf(w2.y) + fmaxf(-w2.y, 0.f) * Tf > kSafeRange);
+    const float dP = static_cast<float>(kL * sub), dS = static_cast<float>(kL * (subs - 1 - sub));    // tokens to the CTA's edges
+    bool unsafe = given_up != 0u;
     TL_MARK(3);
-    const Enter e1 = fast_exchange<kBwd, kMulti>(c, 0, F, MF, R, unsafe TL_PASS);
+    if (kOwn1) {
+        const float Tf = static_cast<float>(p.T);
+        unsafe = (2.f * kmax.x + fabsf(u2.x) + fabsf(w2.x) + fmaxf(-w2.x, 0.f) * Tf > kSafeRange) ||
+                 (2.f * kmax.y + fabsf(u2.y) + fabsf(w2.y) + fmaxf(-w2.y, 0.f) * Tf > kSafeRange);
+        e1 = fast_exchange<RW, kSums, kLinked>(c, 0, F, MF, R, unsafe TL_PASS);
+    } else {
+        add_outside<kBwd && !kSums>(e1, c.cta + 2 * pr, p.state_rows, wl2, dP, dS);
+    }
     TL_MARK(4);
+    if (kSums && !kBwd) {
+        put_state(p.states1 + sub_at, p.state_rows, e1, kMom1);
+        if (unsafe && threadIdx.x == 0) *reinterpret_cast<volatile unsigned*>(p.out_of_range) = 1u;
+        return;
+    }
 
     float2 gw = f2(0.f, 0.f), gu = f2(0.f, 0.f);
     if (kBwd && !sm100::mbar_wait(gfull + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
@@ -987,11 +1092,11 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         // the whole cluster takes this branch together: the unit is left to the exact kernel, which
         // runs right after this one (nothing of this CTA is in flight any more: its tiles have
         // landed and everything the other CTAs sent has been waited for)
-        // (a sequence of several segments is not the exact kernel's to redo: the count alone tells the
-        // launch's last stage to run the chunked kernels over the whole call)
-        if (c.rank == 0 && seg == 0 && threadIdx.x == 0) {
+        // (a sequence of several clusters is not the exact kernel's to redo: the count alone switches on the chunked kernels, which
+        // redo the whole call; without clusters the word that was read does)
+        if (kCluster && cta == 0 && threadIdx.x == 0) {
             const unsigned at = atomicAdd(p.redo_count, 1u);
-            if (!kMulti) p.redo_list[at] = unit;
+            if (!kLinked) p.redo_list[at] = unit;
         }
         return;
     }
@@ -1031,7 +1136,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         // the records the other CTAs sent for level 1 have been consumed: tell them (they wait for
         // this before sending level 2 into the same slots).  The reads are complete: their values
         // went into shared memory before the CTA barrier that precedes this point.
-        if (p.cluster > 1) cluster_arrive_relaxed();
+        if (kCluster && p.cluster > 1) cluster_arrive_relaxed();
         // ---- backward, pass 2: recompute Den, y; G = gy / Den (in place of gy), -H = -G y (registers);
         //      gu; gw from pairs (output later than input); aggregates of [G, -H] ----
         float2 hn[kL];
@@ -1071,16 +1176,19 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                         const float2 ny = f2(nn.x * -inv.x, nn.y * -inv.y);
                         const float2 g_ = mul2(gys[j], inv);
                         const float2 h = mul2(g_, ny);                  // -H
-                        g2[i * kRow] = g_;
-                        hn[i] = h;
-                        gu = fma2(zx, g_, gu);
-                        gu = fma2(zy, h, gu);
-                        gwa = fma2(g_, PM.n, gwa);
-                        gwa = fma2(h, PM.d, gwa);
                         P.n = fma2(lam2, P.n, zx);
                         P.d = fma2(lam2, P.d, zy);
-                        PM.n = fma2(lam2, PM.n, P.n);
-                        PM.d = fma2(lam2, PM.d, P.d);
+                        if (kResults) {
+                            g2[i * kRow] = g_;
+                            hn[i] = h;
+                            gu = fma2(zx, g_, gu);
+                            gu = fma2(zy, h, gu);
+                            gwa = fma2(g_, PM.n, gwa);
+                            gwa = fma2(h, PM.d, gwa);
+                            PM.n = fma2(lam2, PM.n, P.n);
+                            PM.d = fma2(lam2, PM.d, P.d);
+                        }
+                        if (!kOwn2) continue;
                         rr.n = fma2(lam2, rr.n, g_);
                         rr.d = fma2(lam2, rr.d, h);
                         mr.n = fma2(lam2, mr.n, rr.n);
@@ -1097,8 +1205,13 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         }
         bool ignored = false;
         TL_MARK(5);
-        if (p.cluster > 1) cluster_wait();
-        const Enter e2 = fast_exchange<kBwd, kMulti>(c, 1, rr, mr, q, ignored TL_PASS);
+        if (kCluster && p.cluster > 1) cluster_wait();
+        if (kOwn2) e2 = fast_exchange<RW, kSums, kLinked>(c, 1, rr, mr, q, ignored TL_PASS);
+        else add_outside<true>(e2, c.sub + 2 * pr, kStateRows, wl2, dP, dS);
+        if (kSums) {
+            put_state(p.states2 + sub_at, kStateRows, e2, true);
+            return;
+        }
         TL_MARK(6);
         // ---- backward, pass 3: gk, gv in place of the terms; gw from pairs (output earlier than input).
         //      Adjoint states are kept divided by lambda, so that [G, -H] enter without a multiply. ----
@@ -1168,7 +1281,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
             }
             sm100::tma_store_commit();
         }
-    } else if (threadIdx.x == 0 && (!kMulti || tok0 < p.T)) {
+    } else if (threadIdx.x == 0 && (!kLinked || tok0 < p.T)) {
         sm100::tma_store_3d(&map_o0, slot_k, strip * kCs, tok0, b);
         if (kBwd) sm100::tma_store_3d(&map_o1, slot_v, strip * kCs, tok0, b);
         sm100::tma_store_commit();
@@ -1177,7 +1290,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         for (int j = warp; j < 2; j += min(nw, 2)) {
             float acc = 0.f;
             for (int s = 0; s < 2 * nw; ++s) acc += slot_g[(s * kL + j) * kCs + lane];
-            p.partial[(static_cast<size_t>(blockIdx.x) * 2 + j) * kCs + lane] = acc;
+            p.partial[(static_cast<size_t>(blk_id) * 2 + j) * kCs + lane] = acc;
         }
     }
     TL_MARK(8);
@@ -1338,8 +1451,8 @@ reduce_partials(Params p, float* __restrict__ out) {
     __shared__ float red[32][33];
     const int strip = blockIdx.x, j = blockIdx.y, lane = threadIdx.x;
     const int ch = strip * kCs + lane;
-    if (p.segs > 1 && *p.redo_count != 0u) return;       // the chunked kernels redo the whole call and write gw, gu
-    const int per_unit = p.cluster * p.segs;
+    if (p.out_of_range != nullptr && *p.out_of_range != 0u) return;       // the chunked kernels redo the whole call and write gw, gu
+    const int per_unit = p.ctas;
     const int rows = p.B * per_unit;
     float acc = 0.f;
     for (int r = threadIdx.y; r < rows; r += 32) {
@@ -1357,6 +1470,54 @@ reduce_partials(Params p, float* __restrict__ out) {
     }
 }
 
+// Sequences longer than one cluster holds, where there are enough of them.
+//   forward                  k, v -> sums of every 16 tokens and of every CTA (sums); the CTAs' sums chained along the sequence
+//                            (this kernel); k, v and both -> y (spread)
+//   backward                 the first two steps with first moments, unless the forward kept their results; k, v, gy and these
+//                            -> sums of the adjoint pairs (sums); chained; everything -> gk, gv, gw, gu (spread)
+// The launches are plain grids of independent CTAs, so each runs at the rate of HBM (5.9 to 6.4 TB/s; the states of every 16
+// tokens are 1 to 1.5 bytes per element and level).  That is 22 bytes per element forward where k, v, y are 12, and 38 backward
+// where 20 are necessary, but nothing waits for another CTA.  Several clusters per sequence (linked) move the necessary bytes and
+// spend more on the skew between their starts.  B=8, T=16384, C=768 forward + backward: 1926 us linked, 1060 us so; B=16, T=4200
+// 897 and 553 us.  In one launch these steps were slower: with a barrier of all CTAs between them and tiles handed out one by one
+// 1228 us, taken by tickets in the order of the steps 1428 us, and so with neighbouring sequences' steps side by side, so that
+// the second reads come from L2, 1224 us.
+//
+// This kernel: a warp takes one of four parts of a unit - towards later or earlier tokens, numerators or denominators -, lane =
+// channel, T / 256 steps over a few KB.  In double precision: rounded to float at every step, the results were a third further
+// from a float64 evaluation at T=32768.
+// `seen` / `kept_seen`: the word for inputs out of range goes with states that are kept.
+__global__ void __launch_bounds__(128)
+biwkv_chain_kernel(float* __restrict__ sums, const float* __restrict__ w, int n_strips, int n_ctas, int n_tok, int rows, int C,
+                   const unsigned* seen, unsigned* kept_seen) {
+    constexpr int kStep = 16;
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5, unit = blockIdx.x, ch = (unit % n_strips) * kCs + lane;
+    if (kept_seen != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *kept_seen = *seen;
+    const double x = exp(-(ch < C ? static_cast<double>(w[ch]) : 0.0) * n_tok), len = n_tok;
+    const bool back = part >= 2, moments = !back && rows == kStateRows;
+    const int step = (back ? -rows : rows) * kCs;
+    float* at = sums + (static_cast<size_t>(unit) * n_ctas + (back ? n_ctas - 1 : 0)) * rows * kCs + ((part & 1) + (back ? rows - 2 : 0)) * kCs + lane;
+    double P = 0.0, M = 0.0;
+    for (int c0 = 0; c0 < n_ctas; c0 += kStep, at += kStep * step) {
+        float f[kStep], m[kStep];
+#pragma unroll
+        for (int j = 0; j < kStep; ++j) {
+            f[j] = c0 + j < n_ctas ? at[j * step] : 0.f;
+            m[j] = moments && c0 + j < n_ctas ? at[j * step + 2 * kCs] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < kStep; ++j)
+            if (c0 + j < n_ctas) {
+                at[j * step] = static_cast<float>(P);
+                if (moments) {
+                    at[j * step + 2 * kCs] = static_cast<float>(M);
+                    M = fma(fma(len, P, M), x, static_cast<double>(m[j]));
+                }
+                P = fma(P, x, static_cast<double>(f[j]));
+            }
+    }
+}
+
 // ---- host side ------------------------------------------------------------------------------------
 constexpr int kFwdStash = 8;
 constexpr int kBwdStash = 8;
@@ -1367,7 +1528,8 @@ static std::atomic<bool> g_withhold{false};
 void set_withhold_test(bool on) { g_withhold.store(on); }
 
 struct Plan {
-    int cluster = 0, n_warps = 0, n_tok = 0, segs = 1;
+    int cluster = 0, segs = 1, n_warps = 0, n_tok = 0, ctas = 0;
+    bool split = false;      // longer than one cluster holds, in separate launches
 };
 
 // How many CTAs hold a sequence, and in how many clusters.
@@ -1380,44 +1542,70 @@ struct Plan {
 // 3 CTAs of 7 warps share an SM worse than 4 of 5: T=600 244 / 607 against 230 / 565, but T=520 (3 of 6) 257 / 634 against
 // 257 / 652.
 //
-// Several clusters: about 2048 tokens (8 CTAs) each, since clusters of 8 fill more SMs than clusters of 16, up to kMaxSegs of
-// them: T=16384 8 clusters of 8 517 / 1418, 4 of 16 563 / 1618; T=6000 3 of 8 454 / 1177, 2 of 12 464 / 1209; T=4700 2 of 10
-// 449 / 1222, 3 of 7 475 / 1293.  The CTAs of a cluster again follow from the tokens: T=4200 2 of 9 465 / 1217, 2 of 16
-// 626 / 1652.
-static bool make_plan(int T, Plan& pl) {
+// Above, separate launches (see biwkv_chain_kernel) from kSplitCtas CTAs of 256 tokens on.  Below that one launch of linked
+// clusters is as fast or faster, being fewer launches (forward / backward us, float32): B=1, C=192, T=8192 (192 CTAs) linked 25 /
+// 45, separate 27 / 53; T=16384 (384) 29 / 73 and 31 / 72; T=32768 (768) 56 / 178 and 43 / 111; B=2, C=768, T=4200 (816) 49 / 114
+// and 38 / 94.
+// Linked clusters: about 2048 tokens (8 CTAs) each, since clusters of 8 fill more SMs than clusters of 16, up to kMaxSegs of
+// them; the CTAs of a cluster follow from the tokens.
+constexpr long long kSplitCtas = 512;
+static bool make_plan(int B, int T, int C, Plan& pl) {
     constexpr int kCtaMax = kMaxWarps * kSpan;              // tokens one CTA holds
     constexpr int kSegMax = kMaxCluster * kCtaMax;          // tokens one cluster holds
     const auto up = [](int a, int b) { return (a + b - 1) / b; };
     const auto warps = [&](int ctas) { return up(up(T, ctas), kSpan); };
     pl.segs = T <= kSegMax ? 1 : std::max(up(T, kSegMax), std::min(kMaxSegs, (T + 1024) / 2048));
     if (pl.segs > kMaxSegs) return false;
-    pl.cluster = up(up(T, pl.segs), kCtaMax);
-    if (pl.segs == 1 && pl.cluster == 3 && 4 * warps(4) < 3 * warps(3)) pl.cluster = 4;
-    pl.n_warps = warps(pl.segs * pl.cluster);
+    pl.split = pl.segs > 1 && static_cast<long long>(B) * up(C, kCs) * up(T, kCtaMax) >= kSplitCtas;
+    if (pl.split) {
+        pl.segs = pl.cluster = 1;
+        pl.ctas = up(T, kCtaMax);
+    } else {
+        pl.cluster = up(up(T, pl.segs), kCtaMax);
+        if (pl.segs == 1 && pl.cluster == 3 && 4 * warps(4) < 3 * warps(3)) pl.cluster = 4;
+        pl.ctas = pl.segs * pl.cluster;
+    }
+    pl.n_warps = warps(pl.ctas);
     pl.n_tok = pl.n_warps * kSpan;
-    // every CTA of a single cluster owns a token, and so does every segment
-    return static_cast<long long>(pl.segs == 1 ? pl.cluster - 1 : (pl.segs - 1) * pl.cluster) * pl.n_tok < T;
+    // every CTA owns a token, or at least every segment
+    return static_cast<long long>(pl.segs == 1 ? pl.ctas - 1 : (pl.segs - 1) * pl.cluster) * pl.n_tok < T;
 }
 
 struct DeviceState {
     bool probed = false, ok = false;
-    // [segments > 1][tensor types][bwd][cluster][n_warps]: 0 unknown, 1 launchable, -1 not
-    signed char fits[2][3][2][kMaxCluster + 1][kMaxWarps + 1] = {};   // first index: several segments per sequence
+    // [linked][tensor types][bwd][cluster][n_warps]: 0 unknown, 1 launchable, -1 not
+    signed char fits[2][3][2][kMaxCluster + 1][kMaxWarps + 1] = {};
 };
 static std::mutex g_mutex;
 static DeviceState g_dev[64];
 
-// kWide kernels exist for sequences of one segment (the chunked kernels that stand by behind several have no such form)
-template <bool kBwd, Types kTypes, bool kMulti = false>
+// kWide kernels exist for sequences of one cluster (the chunked kernels that stand by behind longer ones have no such form)
+template <bool kBwd, Types kTypes, Mode kMode>
 static auto kernel() {
-    return biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kTypes != Types::f32, kTypes == Types::wide, kMulti && kTypes != Types::wide>;
+    constexpr bool kWide = kTypes == Types::wide && kMode == Mode::whole;
+    return biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kTypes != Types::f32, kWide, kMode>;
 }
 template <bool kBwd, Types kTypes>
 static auto exact_kernel() {
     return biwkv_exact_kernel<kBwd, kTypes != Types::f32, kTypes == Types::wide>;
 }
 template <typename F>
-static const void* ptr(F* f) { return reinterpret_cast<const void*>(f); }
+static bool allow(F* fn, size_t smem, bool cluster) {
+    const void* f = reinterpret_cast<const void*>(fn);
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+           (!cluster || cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess);
+}
+template <bool kBwd, Types kTypes, Mode kMode>
+static bool allow_kernel() { return allow(kernel<kBwd, kTypes, kMode>(), smem_bytes<kBwd, kMode>(kMaxWarps), kUsesCluster<kMode>); }
+template <bool kBwd, Types kTypes>
+static bool allow_types() {
+    bool good = allow_kernel<kBwd, kTypes, Mode::whole>() && allow(exact_kernel<kBwd, kTypes>(), smem_bytes<kBwd>(kMaxWarps), true);
+    if constexpr (kTypes != Types::wide) {
+        good = good && allow_kernel<kBwd, kTypes, Mode::linked>() && allow_kernel<kBwd, kTypes, Mode::sums>() && allow_kernel<kBwd, kTypes, Mode::spread>();
+        good = good && allow_kernel<false, kTypes, Mode::sums_keep>();
+    }
+    return good;
+}
 
 template <bool kBwd, Types kTypes>
 static bool fits(const Plan& pl) {
@@ -1429,23 +1617,12 @@ static bool fits(const Plan& pl) {
         d.probed = true;
         int cl = 0;
         cudaDeviceGetAttribute(&cl, cudaDevAttrClusterLaunch, dev);
-        bool good = cl != 0 && tensor_map::encode_fn() != nullptr;
-        constexpr Types kF = Types::f32, kH = Types::bf16, kW = Types::wide;
-        const void* fn[16] = {ptr(kernel<false, kF>()), ptr(kernel<false, kH>()), ptr(kernel<false, kW>()), ptr(kernel<false, kF, true>()),
-                              ptr(kernel<false, kH, true>()), ptr(exact_kernel<false, kF>()), ptr(exact_kernel<false, kH>()),
-                              ptr(exact_kernel<false, kW>()),
-                              ptr(kernel<true, kF>()), ptr(kernel<true, kH>()), ptr(kernel<true, kW>()), ptr(kernel<true, kF, true>()),
-                              ptr(kernel<true, kH, true>()), ptr(exact_kernel<true, kF>()), ptr(exact_kernel<true, kH>()),
-                              ptr(exact_kernel<true, kW>())};
-        for (int i = 0; i < 16; ++i) {
-            good = good && cudaFuncSetAttribute(fn[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                static_cast<int>(i >= 8 ? smem_bytes<true>(kMaxWarps) : smem_bytes<false>(kMaxWarps))) == cudaSuccess;
-            good = good && cudaFuncSetAttribute(fn[i], cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-        }
-        if (!good) cudaGetLastError();
-        d.ok = good;
+        d.ok = cl != 0 && tensor_map::encode_fn() != nullptr && allow_types<false, Types::f32>() && allow_types<false, Types::bf16>() &&
+               allow_types<false, Types::wide>() && allow_types<true, Types::f32>() && allow_types<true, Types::bf16>() &&
+               allow_types<true, Types::wide>();
+        if (!d.ok) cudaGetLastError();
     }
-    if (!d.ok) return false;
+    if (!d.ok || pl.split) return d.ok;
     signed char& slot = d.fits[pl.segs > 1 ? 1 : 0][static_cast<int>(kTypes)][kBwd ? 1 : 0][pl.cluster][pl.n_warps];
     if (slot == 0) {
         cudaLaunchConfig_t cfg = {};
@@ -1457,7 +1634,8 @@ static bool fits(const Plan& pl) {
         at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
         int n = 0;
-        const cudaError_t err = cudaOccupancyMaxActiveClusters(&n, pl.segs > 1 ? ptr(kernel<kBwd, kTypes, true>()) : ptr(kernel<kBwd, kTypes>()), &cfg);
+        const cudaError_t err = cudaOccupancyMaxActiveClusters(
+            &n, pl.segs > 1 ? reinterpret_cast<const void*>(kernel<kBwd, kTypes, Mode::linked>()) : reinterpret_cast<const void*>(kernel<kBwd, kTypes, Mode::whole>()), &cfg);
         if (err != cudaSuccess) cudaGetLastError();
         slot = (err == cudaSuccess && n > 0) ? 1 : -1;
     }
@@ -1469,114 +1647,198 @@ bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool
     for (const void* q : ptrs)
         if (reinterpret_cast<uintptr_t>(q) & 15u) return false;    // TMA base alignment
     Plan pl;
-    if (!make_plan(T, pl)) return false;
-    const long long ctas = static_cast<long long>(B) * ((C + kCs - 1) / kCs) * pl.cluster * pl.segs;
+    if (!make_plan(B, T, C, pl)) return false;
+    const long long ctas = static_cast<long long>(B) * ((C + kCs - 1) / kCs) * pl.ctas;
     if (ctas > (1LL << 30)) return false;
-    if (types == Types::wide) return pl.segs == 1 && (bwd ? fits<true, Types::wide>(pl) : fits<false, Types::wide>(pl));
+    if (types == Types::wide) return pl.segs == 1 && !pl.split && (bwd ? fits<true, Types::wide>(pl) : fits<false, Types::wide>(pl));
     if (types == Types::bf16) return bwd ? fits<true, Types::bf16>(pl) : fits<false, Types::bf16>(pl);
     return bwd ? fits<true, Types::f32>(pl) : fits<false, Types::f32>(pl);
 }
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// workspace: status block (256 B) | redo list | backward partials | segment flags | segment records | copies of w, u
-struct Carve {
-    size_t off_list, off_partial, off_flags, off_records, off_vectors, total;
+// states of sub-chunks and CTAs: out-of-range word | of the CTAs | of the sub-chunks
+struct StatesCarve {
+    size_t off_ctas, off_subs, total;
 };
-static Carve carve(int B, int C, const Plan& pl, bool bwd) {
-    const size_t units = static_cast<size_t>(B) * ((C + kCs - 1) / kCs);
+static StatesCarve carve_states(size_t units, const Plan& pl, int rows) {
+    StatesCarve cv;
+    cv.off_ctas = 256;
+    cv.off_subs = cv.off_ctas + align_up(units * pl.ctas * rows * kCs * sizeof(float), 256);
+    cv.total = cv.off_subs + align_up(units * pl.ctas * 2 * pl.n_warps * rows * kCs * sizeof(float), 256);
+    return cv;
+}
+static size_t units_of(int B, int C) { return static_cast<size_t>(B) * ((C + kCs - 1) / kCs); }
+
+// workspace: status block (256 B) | longer sequences: segment flags, workspace of the kernels that stand by (all of that but the
+// end of the last to be cleared) | redo list | backward partials | copies of w, u | segment records | states of level 1, of level 2
+constexpr size_t kStatusBytes = 256;
+struct Carve {
+    size_t off_flags, off_stand_by, cleared, off_list, off_partial, off_vectors, off_records, off_states1, off_states2, total;
+};
+static Carve carve(int B, int T, int C, const Plan& pl, bool bwd) {
+    const size_t units = units_of(B, C), recs = pl.segs > 1 ? units * pl.segs * 4 : 0;
+    const bool longer = pl.split || pl.segs > 1;
     Carve cv;
-    cv.off_list = 256;
+    cv.off_flags = kStatusBytes;
+    cv.off_stand_by = cv.off_flags + align_up(recs * sizeof(unsigned), 256);
+    cv.cleared = cv.off_stand_by + (longer ? fused::cleared_bytes(B, T, C, bwd) : 0);
+    cv.off_list = cv.off_stand_by + (longer ? align_up(fused::workspace_bytes(B, T, C, bwd), 256) : 0);
     cv.off_partial = cv.off_list + align_up(units * sizeof(int), 256);
-    cv.off_flags = cv.off_partial + (bwd ? align_up(units * pl.segs * pl.cluster * 2 * kCs * sizeof(float), 256) : 0);
-    const size_t recs = pl.segs > 1 ? units * pl.segs * 4 : 0;
-    cv.off_records = cv.off_flags + align_up(recs * sizeof(unsigned), 256);
-    cv.off_vectors = cv.off_records + align_up(recs * kSegRec * sizeof(float), 256);
-    cv.total = cv.off_vectors + align_up(2 * static_cast<size_t>(C) * sizeof(float), 256);
+    cv.off_vectors = cv.off_partial + (bwd ? align_up(units * pl.ctas * 2 * kCs * sizeof(float), 256) : 0);
+    cv.off_records = cv.off_vectors + align_up(2 * static_cast<size_t>(C) * sizeof(float), 256);
+    cv.off_states1 = cv.off_records + align_up(recs * kSegRec * sizeof(float), 256);
+    cv.off_states2 = cv.off_states1 + (pl.split ? carve_states(units, pl, bwd ? kStateRows : kPlainRows).total : 0);
+    cv.total = cv.off_states2 + (pl.split && bwd ? carve_states(units, pl, kStateRows).total : 0);
     return cv;
 }
 
 size_t workspace_bytes(int B, int T, int C, bool bwd) {
     Plan pl;
-    if (!make_plan(T, pl)) return 256;
-    return carve(B, C, pl, bwd).total;
+    if (!make_plan(B, T, C, pl)) return 256;
+    return carve(B, T, C, pl, bwd).total;
 }
 
-bool multi_segment(int T) {
+size_t kept_bytes(int B, int T, int C) {
     Plan pl;
-    return make_plan(T, pl) && pl.segs > 1;
+    if (!make_plan(B, T, C, pl) || !pl.split) return 0;
+    return carve_states(units_of(B, C), pl, kStateRows).total;
 }
 
+bool stands_by(int B, int T, int C) {
+    Plan pl;
+    return make_plan(B, T, C, pl) && (pl.split || pl.segs > 1);
+}
 // The kernels read w and u in pairs.  A vector that starts at an odd float (cut out of a parameter buffer) goes through a copy:
-// single loads in the kernels cost every call, up to 7 % where a sequence has several segments (T=16384: 1925 and 2067 us).
+// single loads in the kernels cost every call, up to 7 % where a sequence is long.
 static const float* paired(const float* x, int C, float* copy, cudaStream_t stream) {
     if ((reinterpret_cast<uintptr_t>(x) & 7u) == 0) return x;
     cudaMemcpyAsync(copy, x, static_cast<size_t>(C) * sizeof(float), cudaMemcpyDeviceToDevice, stream);
     return copy;
 }
 
+struct Maps {
+    CUtensorMap k, v, g, o0, o1;
+};
+template <bool kBwd, Types kTypes, Mode kMode>
+static bool run(const Params& p, const Maps& m, size_t grid, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(p.n_warps * 32);
+    cfg.dynamicSmemBytes = smem_bytes<kBwd, kMode>(p.n_warps);
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = p.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = kUsesCluster<kMode> ? 1 : 0;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel<kBwd, kTypes, kMode>(), m.k, m.v, m.g, m.o0, m.o1, p);
+    if (err == cudaSuccess) return true;
+    set_error_detail(cudaGetErrorName(err));
+    return false;
+}
+
+// kept: forward: where to leave what a backward needs (may be null); backward: what a forward left (may be null)
 template <bool kBwd, Types kTypes>
 static int launch(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy,
-                  void* o0, void* o1, float* gwgu, void* workspace, cudaStream_t stream) {
+                  void* o0, void* o1, float* gwgu, void* workspace, void* kept, cudaStream_t stream) {
     constexpr bool kHalf = kTypes != Types::f32, kWide = kTypes == Types::wide;
     constexpr bool kHalfOut = kHalf && (kBwd || !kWide), kHalfG = kHalf && !kWide;
     Plan pl;
-    if (!make_plan(T, pl)) return -1;
+    if (!make_plan(B, T, C, pl)) return -1;
     Params p{};
     p.B = B; p.T = T; p.C = C;
     p.n_strips = (C + kCs - 1) / kCs;
-    p.cluster = pl.cluster; p.n_warps = pl.n_warps; p.n_tok = pl.n_tok;
+    p.cluster = pl.cluster; p.n_warps = pl.n_warps; p.n_tok = pl.n_tok; p.ctas = pl.ctas;
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     p.status = reinterpret_cast<unsigned*>(ws);
     p.mirror = failure_mirror(kBwd ? Op::biwkv_backward : Op::biwkv_forward);
-    const size_t units = static_cast<size_t>(B) * p.n_strips;
-    const Carve cv = carve(B, C, pl, kBwd);
+    const size_t units = units_of(B, C), grid = units * pl.ctas;
+    const Carve cv = carve(B, T, C, pl, kBwd);
     p.redo_count = reinterpret_cast<unsigned*>(ws) + 1;
     p.redo_list = reinterpret_cast<int*>(ws + cv.off_list);
-    p.partial = reinterpret_cast<float*>(ws + cv.off_partial);
     p.segs = pl.segs;
     p.xflag = reinterpret_cast<unsigned*>(ws + cv.off_flags);
     p.xseg = reinterpret_cast<float*>(ws + cv.off_records);
+    p.partial = reinterpret_cast<float*>(ws + cv.off_partial);
     float* const vectors = reinterpret_cast<float*>(ws + cv.off_vectors);
     p.w = paired(w, C, vectors, stream);
     p.u = paired(u, C, vectors + C, stream);
     p.spin_limit = g_withhold.load() ? (1u << 10) : kSpinLimit;
     p.withhold_rank = g_withhold.load() ? 1 : -1;
+    p.state_rows = kBwd || kept ? kStateRows : kPlainRows;
+    if (pl.split || pl.segs > 1) p.out_of_range = p.redo_count;
+    if (pl.split) {
+        unsigned char* base = kept ? static_cast<unsigned char*>(kept) : ws + cv.off_states1;
+        StatesCarve sc = carve_states(units, pl, p.state_rows);
+        if (kBwd && kept) p.out_of_range = reinterpret_cast<unsigned*>(base);
+        p.ctas1 = reinterpret_cast<float*>(base + sc.off_ctas);
+        p.states1 = reinterpret_cast<float*>(base + sc.off_subs);
+        if (kBwd) {
+            sc = carve_states(units, pl, kStateRows);
+            p.ctas2 = reinterpret_cast<float*>(ws + cv.off_states2 + sc.off_ctas);
+            p.states2 = reinterpret_cast<float*>(ws + cv.off_states2 + sc.off_subs);
+        }
+    }
     tensor_map::bind_primary_context();   // the tensor-map encoder is a driver call
-    CUtensorMap mk, mv, mg, m0, m1;
+    Maps m;
     // float32: loads one box per 32-token span, stores one box per CTA; bfloat16: one box per 16-token sub-chunk both ways
     const int box_in = kHalf ? kL : kSpan, box_g = kHalfG ? kL : kSpan, box_out = kHalfOut ? kL : pl.n_tok;
-    bool ok = tensor_map::make_btc(&mk, k, B, T, C, kCs, box_in, kHalf) && tensor_map::make_btc(&mv, v, B, T, C, kCs, box_in, kHalf) &&
-              tensor_map::make_btc(&m0, o0, B, T, C, kCs, box_out, kHalfOut);
-    ok = ok && (kBwd ? tensor_map::make_btc(&mg, gy, B, T, C, kCs, box_g, kHalfG) : tensor_map::make_btc(&mg, k, B, T, C, kCs, box_in, kHalf)) &&
-         tensor_map::make_btc(&m1, kBwd ? o1 : o0, B, T, C, kCs, box_out, kHalfOut);
+    bool ok = tensor_map::make_btc(&m.k, k, B, T, C, kCs, box_in, kHalf) && tensor_map::make_btc(&m.v, v, B, T, C, kCs, box_in, kHalf) &&
+              tensor_map::make_btc(&m.o0, o0, B, T, C, kCs, box_out, kHalfOut);
+    if (kBwd) {
+        ok = ok && tensor_map::make_btc(&m.g, gy, B, T, C, kCs, box_g, kHalfG) && tensor_map::make_btc(&m.o1, o1, B, T, C, kCs, box_out, kHalfOut);
+    } else {
+        m.g = m.k;       // not used
+        m.o1 = m.o0;
+    }
     if (!ok) {
         set_error_detail("cuTensorMapEncodeTiled rejected a (C, T, B) tensor map");
         return -1;
     }
-    cudaMemsetAsync(ws, 0, 256, stream);
-    if (pl.segs > 1) cudaMemsetAsync(p.xflag, 0, cv.off_records - cv.off_flags, stream);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(B) * p.n_strips * pl.cluster * pl.segs);
-    cfg.blockDim = dim3(pl.n_warps * 32);
-    cfg.dynamicSmemBytes = smem_bytes<kBwd>(pl.n_warps);
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, pl.segs > 1 ? kernel<kBwd, kTypes, true>() : kernel<kBwd, kTypes>(), mk, mv, mg, m0, m1, p);
-    if (err != cudaSuccess) {
-        set_error_detail(cudaGetErrorName(err));
-        return -1;
+    cudaMemsetAsync(ws, 0, cv.cleared, stream);
+    int launched = 0;
+    bool done = true;
+    if constexpr (kTypes == Types::wide) {
+        if (pl.split || pl.segs > 1) return -1;
+        done = run<kBwd, kTypes, Mode::whole>(p, m, grid, stream);
+    } else if (pl.split) {
+        unsigned* const kept_seen = !kBwd && kept ? static_cast<unsigned*>(kept) : nullptr;
+        const auto chain = [&](float* sums, int rows) {
+            biwkv_chain_kernel<<<static_cast<unsigned>(units), 128, 0, stream>>>(sums, p.w, p.n_strips, pl.ctas, pl.n_tok, rows, C, p.out_of_range, kept_seen);
+        };
+        if (!kBwd || !kept) {
+            done = p.state_rows == kStateRows ? run<false, kTypes, Mode::sums_keep>(p, m, grid, stream) : run<false, kTypes, Mode::sums>(p, m, grid, stream);
+            chain(p.ctas1, p.state_rows);
+            launched += 2;
+        }
+        if (kBwd) {
+            done = done && run<kBwd, kTypes, Mode::sums>(p, m, grid, stream);
+            chain(p.ctas2, kStateRows);
+            launched += 2;
+        }
+        p.reverse = true;
+        done = done && run<kBwd, kTypes, Mode::spread>(p, m, grid, stream);
+    } else if (pl.segs > 1) {
+        done = run<kBwd, kTypes, Mode::linked>(p, m, grid, stream);
+    } else {
+        done = run<kBwd, kTypes, Mode::whole>(p, m, grid, stream);
     }
-    int launched = 1;
-    if (pl.segs == 1) {
+    if (!done) return -1;
+    ++launched;
+    if (!pl.split && pl.segs == 1) {
         // the exact kernel: a few clusters that serve whatever the fast kernel left behind
+        cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(std::min<size_t>(units, 16)) * pl.cluster);
-        const cudaError_t err2 = cudaLaunchKernelEx(&cfg, exact_kernel<kBwd, kTypes>(), mk, mv, mg, m0, m1, p);
-        if (err2 != cudaSuccess) {
-            set_error_detail(cudaGetErrorName(err2));
+        cfg.blockDim = dim3(pl.n_warps * 32);
+        cfg.dynamicSmemBytes = smem_bytes<kBwd>(pl.n_warps);
+        cfg.stream = stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        const cudaError_t err = cudaLaunchKernelEx(&cfg, exact_kernel<kBwd, kTypes>(), m.k, m.v, m.g, m.o0, m.o1, p);
+        if (err != cudaSuccess) {
+            set_error_detail(cudaGetErrorName(err));
             return -1;
         }
         ++launched;
@@ -1585,19 +1847,36 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
         reduce_partials<<<dim3(p.n_strips, 2), dim3(32, 32), 0, stream>>>(p, gwgu);
         ++launched;
     }
+    if constexpr (kTypes != Types::wide) {
+        if (pl.split || pl.segs > 1) {
+            void* const stand_by = ws + cv.off_stand_by;
+            int n;
+            if constexpr (kTypes == Types::bf16) {
+                n = kBwd ? fused::backward_bf16(B, T, C, w, u, k, v, gy, gwgu, o0, o1, stand_by, stream, p.out_of_range)
+                         : fused::forward_bf16(B, T, C, w, u, k, v, o0, stand_by, stream, p.out_of_range);
+            } else {
+                const auto in = [](const void* x) { return static_cast<const float*>(x); };
+                const auto out = [](void* x) { return static_cast<float*>(x); };
+                n = kBwd ? fused::backward(B, T, C, w, u, in(k), in(v), in(gy), gwgu, out(o0), out(o1), stand_by, stream, p.out_of_range)
+                         : fused::forward(B, T, C, w, u, in(k), in(v), out(o0), stand_by, stream, p.out_of_range);
+            }
+            if (n < 0) return n;
+            launched += n;
+        }
+    }
     return launched;
 }
 
 int forward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, Types types,
-            void* workspace, cudaStream_t stream) {
+            void* workspace, cudaStream_t stream, void* keep) {
     const auto fn = types == Types::f32 ? launch<false, Types::f32> : types == Types::bf16 ? launch<false, Types::bf16> : launch<false, Types::wide>;
-    return fn(B, T, C, w, u, k, v, nullptr, y, nullptr, nullptr, workspace, stream);
+    return fn(B, T, C, w, u, k, v, nullptr, y, nullptr, nullptr, workspace, keep, stream);
 }
 
 int backward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, float* gwgu,
-             void* gk, void* gv, Types types, void* workspace, cudaStream_t stream) {
+             void* gk, void* gv, Types types, void* workspace, cudaStream_t stream, const void* kept) {
     const auto fn = types == Types::f32 ? launch<true, Types::f32> : types == Types::bf16 ? launch<true, Types::bf16> : launch<true, Types::wide>;
-    return fn(B, T, C, w, u, k, v, gy, gk, gv, gwgu, workspace, stream);
+    return fn(B, T, C, w, u, k, v, gy, gk, gv, gwgu, workspace, const_cast<void*>(kept), stream);
 }
 
 }  // namespace resident

@@ -131,19 +131,16 @@ unsigned vrwkv_take_failures(int device) {
     return bits;
 }
 
-// The resident kernels' workspace; for sequences of several segments the chunked kernels' workspace follows it
-// (they stand by for inputs outside the plain-float range and run only when the resident launch says so).
-static size_t resident_offset(int B, int T, int C, bool bwd) {
-    return (biwkv::resident::workspace_bytes(B, T, C, bwd) + 255) / 256 * 256;
-}
-static size_t resident_total(int B, int T, int C, bool bwd) {
-    return resident_offset(B, T, C, bwd) + (biwkv::resident::multi_segment(T) ? biwkv::fused::workspace_bytes(B, T, C, bwd) : 0);
+// Whether the resident kernels serve the call, with what stands by behind them.
+static bool resident_serves(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types) {
+    return g_path.load() == 0 && biwkv::resident::eligible(B, T, C, ptrs, bwd, types) &&
+           (!biwkv::resident::stands_by(B, T, C) || biwkv::fused::eligible(B, T, C, ptrs, types == Types::bf16));
 }
 
 size_t vrwkv_biwkv_forward_workspace_bytes(int B, int T, int C) {
     if (check_shape(B, T, C) != VRWKV_OK) return 0;
     return std::max({biwkv::generic_forward_workspace(B, T, C) + 256, biwkv::fused::workspace_bytes(B, T, C, false),
-                     resident_total(B, T, C, false)});
+                     biwkv::resident::workspace_bytes(B, T, C, false)});
 }
 
 int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u, const float* k,
@@ -156,17 +153,8 @@ int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u,
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool multi = biwkv::resident::multi_segment(T);
-    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, y}, false, Types::f32) &&
-        (!multi || biwkv::fused::eligible(B, T, C, {k, v, y}))) {
-        int n = biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::f32, workspace, s);
-        if (n >= 0 && multi) {
-            const int m = biwkv::fused::forward(B, T, C, w, u, k, v, y, static_cast<char*>(workspace) + resident_offset(B, T, C, false), s,
-                                                static_cast<const unsigned*>(workspace) + 1);
-            n = m < 0 ? m : n + m;
-        }
-        return finish(n);
-    }
+    if (resident_serves(B, T, C, {k, v, y}, false, Types::f32))
+        return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::f32, workspace, s));
     if (g_path.load() != 1 && biwkv::fused::eligible(B, T, C, {k, v, y}))
         return finish(biwkv::fused::forward(B, T, C, w, u, k, v, y, workspace, s));
     // generic path: status word (first 256 bytes) is cleared, scratch follows
@@ -177,7 +165,7 @@ int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u,
 size_t vrwkv_biwkv_backward_workspace_bytes(int B, int T, int C) {
     if (check_shape(B, T, C) != VRWKV_OK) return 0;
     return std::max({biwkv::generic_backward_workspace(B, T, C) + 256, biwkv::fused::workspace_bytes(B, T, C, true),
-                     resident_total(B, T, C, true)});
+                     biwkv::resident::workspace_bytes(B, T, C, true)});
 }
 
 int vrwkv_biwkv_backward_f32(int B, int T, int C, const float* w, const float* u, const float* k,
@@ -190,23 +178,54 @@ int vrwkv_biwkv_backward_f32(int B, int T, int C, const float* w, const float* u
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool multi = biwkv::resident::multi_segment(T);
-    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, gy, gk, gv}, true, Types::f32) &&
-        (!multi || biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}))) {
-        int n = biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::f32, workspace, s);
-        if (n >= 0 && multi) {
-            const int m = biwkv::fused::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv,
-                                                 static_cast<char*>(workspace) + resident_offset(B, T, C, true), s,
-                                                 static_cast<const unsigned*>(workspace) + 1);
-            n = m < 0 ? m : n + m;
-        }
-        return finish(n);
-    }
+    if (resident_serves(B, T, C, {k, v, gy, gk, gv}, true, Types::f32))
+        return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::f32, workspace, s));
     if (g_path.load() != 1 && biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}))
         return finish(biwkv::fused::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, workspace, s));
     cudaMemsetAsync(workspace, 0, 256, s);
     return finish(biwkv::generic_backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv,
                                           static_cast<char*>(workspace) + 256, s));
+}
+
+static bool types_of(int types, Types& t) {
+    if (types < VRWKV_TENSORS_F32 || types > VRWKV_TENSORS_BF16_WIDE) return false;
+    t = types == VRWKV_TENSORS_F32 ? Types::f32 : types == VRWKV_TENSORS_BF16 ? Types::bf16 : Types::wide;
+    return true;
+}
+
+size_t vrwkv_biwkv_kept_bytes(int B, int T, int C) {
+    if (check_shape(B, T, C) != VRWKV_OK) return 0;
+    return biwkv::resident::kept_bytes(B, T, C);
+}
+
+int vrwkv_biwkv_forward_keep(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, int tensors,
+                             void* kept, size_t kept_bytes, void* workspace, size_t workspace_bytes, void* stream) {
+    if (int st = check_shape(B, T, C)) return st;
+    Types types;
+    if (!types_of(tensors, types)) return VRWKV_ERR_UNSUPPORTED;
+    if (!w || !u || !k || !v || !y || !kept || !workspace) return VRWKV_ERR_NULL;
+    if (misaligned4(w) || misaligned4(u) || ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(kept)) & 255u)) return VRWKV_ERR_ALIGNMENT;
+    if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    if (!resident_serves(B, T, C, {k, v, y}, false, types)) return VRWKV_ERR_UNSUPPORTED;
+    if (biwkv::resident::kept_bytes(B, T, C) == 0) return VRWKV_ERR_UNSUPPORTED;
+    if (kept_bytes < biwkv::resident::kept_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, types, workspace, static_cast<cudaStream_t>(stream), kept));
+}
+
+int vrwkv_biwkv_backward_kept(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy,
+                              float* gwgu, void* gk, void* gv, int tensors, const void* kept, size_t kept_bytes, void* workspace,
+                              size_t workspace_bytes, void* stream) {
+    if (int st = check_shape(B, T, C)) return st;
+    Types types;
+    if (!types_of(tensors, types)) return VRWKV_ERR_UNSUPPORTED;
+    if (!w || !u || !k || !v || !gy || !gwgu || !gk || !gv || !kept || !workspace) return VRWKV_ERR_NULL;
+    if (misaligned4(w) || misaligned4(u) || misaligned4(gwgu) || ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(kept)) & 255u))
+        return VRWKV_ERR_ALIGNMENT;
+    if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    if (!resident_serves(B, T, C, {k, v, gy, gk, gv}, true, types)) return VRWKV_ERR_UNSUPPORTED;
+    if (biwkv::resident::kept_bytes(B, T, C) == 0) return VRWKV_ERR_UNSUPPORTED;
+    if (kept_bytes < biwkv::resident::kept_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, types, workspace, static_cast<cudaStream_t>(stream), kept));
 }
 
 int vrwkv_biwkv_forward_save_f32(int B, int T, int C, const float* w, const float* u, const float* k,
@@ -241,18 +260,8 @@ int vrwkv_biwkv_forward_bf16(int B, int T, int C, const float* w, const float* u
     if (!w || !u || !k || !v || !y || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
-    const bool multi = biwkv::resident::multi_segment(T);
-    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, y}, false, Types::bf16) &&
-        (!multi || biwkv::fused::eligible(B, T, C, {k, v, y}, true))) {
-        cudaStream_t s = static_cast<cudaStream_t>(stream);
-        int n = biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::bf16, workspace, s);
-        if (n >= 0 && multi) {
-            const int m = biwkv::fused::forward_bf16(B, T, C, w, u, k, v, y, static_cast<char*>(workspace) + resident_offset(B, T, C, false), s,
-                                                     static_cast<const unsigned*>(workspace) + 1);
-            n = m < 0 ? m : n + m;
-        }
-        return finish(n);
-    }
+    if (resident_serves(B, T, C, {k, v, y}, false, Types::bf16))
+        return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
     if (!biwkv::fused::eligible(B, T, C, {k, v, y}, true)) return VRWKV_ERR_UNSUPPORTED;
     return finish(biwkv::fused::forward_bf16(B, T, C, w, u, k, v, y, workspace, static_cast<cudaStream_t>(stream)));
 }
@@ -265,19 +274,8 @@ int vrwkv_biwkv_backward_bf16(int B, int T, int C, const float* w, const float* 
     if (misaligned4(w) || misaligned4(u) || misaligned4(gwgu) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
-    const bool multi = biwkv::resident::multi_segment(T);
-    if (g_path.load() == 0 && biwkv::resident::eligible(B, T, C, {k, v, gy, gk, gv}, true, Types::bf16) &&
-        (!multi || biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}, true))) {
-        cudaStream_t s = static_cast<cudaStream_t>(stream);
-        int n = biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::bf16, workspace, s);
-        if (n >= 0 && multi) {
-            const int m = biwkv::fused::backward_bf16(B, T, C, w, u, k, v, gy, gwgu, gk, gv,
-                                                      static_cast<char*>(workspace) + resident_offset(B, T, C, true), s,
-                                                      static_cast<const unsigned*>(workspace) + 1);
-            n = m < 0 ? m : n + m;
-        }
-        return finish(n);
-    }
+    if (resident_serves(B, T, C, {k, v, gy, gk, gv}, true, Types::bf16))
+        return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
     if (!biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}, true)) return VRWKV_ERR_UNSUPPORTED;
     return finish(biwkv::fused::backward_bf16(B, T, C, w, u, k, v, gy, gwgu, gk, gv, workspace,
                                               static_cast<cudaStream_t>(stream)));

@@ -65,13 +65,31 @@ at::ScalarType result_dtype(const Tensor& w) {
     return w.scalar_type() == at::kHalf || w.scalar_type() == at::kBFloat16 ? w.scalar_type() : at::kFloat;
 }
 
-// k, v float32 or both bfloat16, contiguous; y in their dtype
-Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+// The forward that keeps states for the backward, into `kept`; false (and an undefined `kept`) where it does not serve the call.
+bool biwkv_forward_keep(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& y, int tensors, const Tensor& ws,
+                        Tensor* kept) {
+    const int B = k.size(0), T = k.size(1), C = k.size(2);
+    const size_t bytes = vrwkv_biwkv_kept_bytes(B, T, C);
+    if (bytes == 0) return false;
+    *kept = workspace(bytes, k);
+    const int st = vrwkv_biwkv_forward_keep(B, T, C, fp(w), fp(u), k.data_ptr(), v.data_ptr(), y.data_ptr(), tensors, kept->data_ptr(),
+                                            kept->numel(), ws.data_ptr(), ws.numel(), stream_of(k));
+    if (st != VRWKV_OK) kept->reset();
+    if (st == VRWKV_ERR_UNSUPPORTED) return false;
+    check(st, "vrwkv_biwkv_forward_keep");
+    return true;
+}
+
+// k, v float32 or both bfloat16, contiguous; y in their dtype.  kept: null, or receives the states for a backward (left
+// undefined where none are kept).
+Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, Tensor* kept = nullptr) {
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor y = at::empty_like(k);
     if (k.numel() == 0) return y;
     Tensor ws = workspace(vrwkv_biwkv_forward_workspace_bytes(B, T, C), k);
-    if (is_bf16(k)) {
+    if (kept && biwkv_forward_keep(w, u, k, v, y, is_bf16(k) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_F32, ws, kept)) {
+        // done
+    } else if (is_bf16(k)) {
         const int st = vrwkv_biwkv_forward_bf16(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
                                                 static_cast<uint16_t*>(v.data_ptr()), static_cast<uint16_t*>(y.data_ptr()),
                                                 ws.data_ptr(), ws.numel(), stream_of(k));
@@ -86,34 +104,37 @@ Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, cons
 }
 
 // k, v bfloat16, contiguous; y float32 holding bfloat16 values.  Undefined where the kernel does not cover the call.
-Tensor biwkv_forward_wide(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+Tensor biwkv_forward_wide(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, Tensor* kept) {
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor y = at::empty_like(k, k.options().dtype(at::kFloat));
     if (k.numel() == 0) return y;
     Tensor ws = workspace(vrwkv_biwkv_forward_workspace_bytes(B, T, C), k);
-    const int st = vrwkv_biwkv_forward_bf16_wide(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
-                                                 static_cast<uint16_t*>(v.data_ptr()), fp(y), ws.data_ptr(), ws.numel(), stream_of(k));
-    if (st == VRWKV_ERR_UNSUPPORTED) return Tensor();
-    check(st, "vrwkv_biwkv_forward_bf16_wide");
+    if (!kept || !biwkv_forward_keep(w, u, k, v, y, VRWKV_TENSORS_BF16_WIDE, ws, kept)) {
+        const int st = vrwkv_biwkv_forward_bf16_wide(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
+                                                     static_cast<uint16_t*>(v.data_ptr()), fp(y), ws.data_ptr(), ws.numel(), stream_of(k));
+        if (st == VRWKV_ERR_UNSUPPORTED) return Tensor();
+        check(st, "vrwkv_biwkv_forward_bf16_wide");
+    }
     raise_failures(k.get_device(), "vrwkv_biwkv_forward");
     return y;
 }
 
-Tensor biwkv_forward(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, bool bf16_io) {
+Tensor biwkv_forward(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, bool bf16_io, Tensor* kept = nullptr) {
     const c10::cuda::CUDAGuard guard(k.device());
     const bool half = bf16_io && is_bf16(k) && is_bf16(v);
     if (half && result_dtype(w) == at::kFloat) {
         // float32 w, u under autocast: the kernel writes the widened result itself
-        const Tensor y = biwkv_forward_wide(f32(w), f32(u), k.contiguous(), v.contiguous());
+        const Tensor y = biwkv_forward_wide(f32(w), f32(u), k.contiguous(), v.contiguous(), kept);
         if (y.defined()) return y;
     }
-    const Tensor y = half ? biwkv_forward_raw(f32(w), f32(u), k.contiguous(), v.contiguous())
-                          : biwkv_forward_raw(f32(w), f32(u), f32(k), f32(v));
+    const Tensor y = half ? biwkv_forward_raw(f32(w), f32(u), k.contiguous(), v.contiguous(), kept)
+                          : biwkv_forward_raw(f32(w), f32(u), f32(k), f32(v), kept);
     return y.to(result_dtype(w));
 }
 
-// k, v float32, or bfloat16 (then gy in either type); all contiguous
-std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& gy) {
+// k, v float32, or bfloat16 (then gy in either type); all contiguous.  kept: what the forward left, or undefined.
+std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& gy,
+                                         const Tensor& kept = Tensor()) {
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor gk = at::empty_like(k), gv = at::empty_like(k);
     Tensor gwgu = at::empty({2, C}, k.options().dtype(at::kFloat));
@@ -122,11 +143,20 @@ std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const
         return {gwgu.select(0, 0), gwgu.select(0, 1), gk, gv};
     }
     Tensor ws = workspace(vrwkv_biwkv_backward_workspace_bytes(B, T, C), k);
-    if (is_bf16(k) && !is_bf16(gy)) {
+    int resumed = VRWKV_ERR_UNSUPPORTED;
+    if (kept.defined()) {
+        const int tensors = !is_bf16(k) ? VRWKV_TENSORS_F32 : is_bf16(gy) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_BF16_WIDE;
+        resumed = vrwkv_biwkv_backward_kept(B, T, C, fp(w), fp(u), k.data_ptr(), v.data_ptr(), gy.data_ptr(), fp(gwgu), gk.data_ptr(),
+                                            gv.data_ptr(), tensors, kept.data_ptr(), kept.numel(), ws.data_ptr(), ws.numel(), stream_of(k));
+        if (resumed != VRWKV_ERR_UNSUPPORTED) check(resumed, "vrwkv_biwkv_backward_kept");
+    }
+    if (resumed == VRWKV_OK) {
+        // done
+    } else if (is_bf16(k) && !is_bf16(gy)) {
         const int st = vrwkv_biwkv_backward_bf16_wide(
             B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()), fp(gy), fp(gwgu),
             static_cast<uint16_t*>(gk.data_ptr()), static_cast<uint16_t*>(gv.data_ptr()), ws.data_ptr(), ws.numel(), stream_of(k));
-        if (st == VRWKV_ERR_UNSUPPORTED) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16));
+        if (st == VRWKV_ERR_UNSUPPORTED) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16), kept);
         check(st, "vrwkv_biwkv_backward_bf16_wide");
     } else if (is_bf16(k)) {
         const int st = vrwkv_biwkv_backward_bf16(
@@ -150,20 +180,21 @@ std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const
 struct BiWkv : torch::autograd::Function<BiWkv> {
     static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& w, const Tensor& u, const Tensor& k,
                           const Tensor& v, bool bf16_io) {
-        Tensor y = biwkv_forward(w, u, k, v, bf16_io);
-        ctx->save_for_backward({w, u, k, v});
+        Tensor kept;
+        Tensor y = biwkv_forward(w, u, k, v, bf16_io, &kept);
+        ctx->save_for_backward({w, u, k, v, kept});
         ctx->saved_data["bf16_io"] = bf16_io;
         return y;
     }
     static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grads) {
         const auto saved = ctx->get_saved_variables();
-        const Tensor &w = saved[0], &u = saved[1], &k = saved[2], &v = saved[3], &gy = grads[0];
+        const Tensor &w = saved[0], &u = saved[1], &k = saved[2], &v = saved[3], &kept = saved[4], &gy = grads[0];
         const c10::cuda::CUDAGuard guard(k.device());
         const at::NoGradGuard no_grad;
         const at::ScalarType out = result_dtype(w);
         const bool half = ctx->saved_data["bf16_io"].toBool() && is_bf16(k) && is_bf16(v);
-        auto g = half ? biwkv_backward_raw(f32(w), f32(u), k.contiguous(), v.contiguous(), is_bf16(gy) ? gy.contiguous() : f32(gy))
-                      : biwkv_backward_raw(f32(w), f32(u), f32(k), f32(v), f32(gy));
+        auto g = half ? biwkv_backward_raw(f32(w), f32(u), k.contiguous(), v.contiguous(), is_bf16(gy) ? gy.contiguous() : f32(gy), kept)
+                      : biwkv_backward_raw(f32(w), f32(u), f32(k), f32(v), f32(gy), kept);
         // on the bfloat16 path gk, gv stay bfloat16 (what autograd hands to a bfloat16 k anyway) unless w is half
         if (!half || out == at::kHalf) { g[2] = g[2].to(out); g[3] = g[3].to(out); }
         return {g[0].to(out), g[1].to(out), g[2], g[3], Tensor()};

@@ -42,20 +42,24 @@ enum class Types {
 bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types);
 void set_withhold_test(bool on);   // test only: one rank per cluster sends nothing, waits give up early
 size_t workspace_bytes(int B, int T, int C, bool bwd);
-// Sequences longer than one cluster holds (T > 4096) run as several clusters per sequence.  Inputs outside the
-// plain-float range then leave workspace word 1 non-zero instead of results: the caller follows up with the
-// chunked kernels switched on by that word.
-bool multi_segment(int T);
+// What a forward leaves for the backward: the states entering every 16 tokens, 1.5 bytes per element, and a flag; 0
+// where the backward takes nothing (T <= 4096, or few tokens in all).
+size_t kept_bytes(int B, int T, int C);
+// Behind sequences longer than one cluster holds (T > 4096) the chunked kernels stand by for inputs outside the plain-float
+// range: fused::eligible has to hold too.
+bool stands_by(int B, int T, int C);
 int forward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, Types types,
-            void* workspace, cudaStream_t stream);
+            void* workspace, cudaStream_t stream, void* keep = nullptr);
 int backward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, float* gwgu,
-             void* gk, void* gv, Types types, void* workspace, cudaStream_t stream);
+             void* gk, void* gv, Types types, void* workspace, cudaStream_t stream, const void* kept = nullptr);
 }  // namespace resident
 namespace fused {
 // True when the fused TMA path can serve this call on the current device.
 bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bf16 = false);
 size_t workspace_bytes(int B, int T, int C, bool bwd);
-// run_if: when set, every kernel of the launch returns at once while that device word is zero.
+// run_if: when set, every kernel of the launch returns at once while that device word is zero; the caller then has cleared the
+// first cleared_bytes of the workspace.
+size_t cleared_bytes(int B, int T, int C, bool bwd);
 int forward(int B, int T, int C, const float* w, const float* u, const float* k, const float* v,
             float* y, void* workspace, cudaStream_t stream, const unsigned* run_if = nullptr);
 int backward(int B, int T, int C, const float* w, const float* u, const float* k, const float* v,
