@@ -8,20 +8,21 @@
 // and mirrored for the leftward direction):
 //   gr_t = S_t gy_t (+ bonus)   gk_t = A_{t+1} v_t (+ bonus)   gv_t = A_{t+1}^T k_t (+ bonus)
 // Every one of these is "read out a 64-vector product of the state, then update the state
-// by a decayed rank-1 term", so one sweep engine serves them all.  A block of 64 threads
-// owns either the rows (thread = key channel) or the columns (thread = value channel) of
-// one state, whichever makes the read-out a sum inside the thread, and keeps its 64 state
-// values in registers.  Tokens arrive in shared memory 8 at a time through cp.async,
-// double-buffered.  One block runs the rightward pass and then the leftward one of its
-// kind and adds the second result to the first itself; while twice the blocks still fit the device in one
-// wave, the directions run in two blocks that add into a zeroed output (two addends per element).  Either
-// way results are bit-reproducible.  Where there are too few blocks to fill the device, a sequence is walked in several segments
-// at a time (below).
+// by a decayed rank-1 term", so one sweep engine serves them all: y from a walk of S, gr from a walk
+// of S, gk and gv from one walk of A.  A block of two warps owns one state and keeps it in registers, 8 x 8 values per thread.
+// Tokens arrive in shared memory 8 at a time through cp.async, double-buffered.  The two
+// directions run in two blocks that add into a zeroed output (two addends per element: bit-reproducible).  Where there are too
+// few blocks to fill the device, a sequence is walked in several segments at a time (below).
 //
 // A token's decay enters as the factor d_t alone, never as a difference of summed logarithms, so a token that forgets
-// everything (d_t = 0) leaves the others exact.  What bounds it is the walk's latency (two warps per block, one token
-// after the other).  Three-part bfloat16 products in 64-token chunks took 9.98 ms for forward + backward at B=32, T=4096,
-// H=12 against 12.2 ms here and the same 0.61 ms at T=196, but left five times this error (9e-7 for 1.6e-7 in the 2-norm).
+// everything (d_t = 0) leaves the others exact.
+//
+// What bounds it: the float32 pipe and the dependent steps of a token; 51 % of the pipe, half of the issue slots busy in the
+// forward.  B=32, H=12, forward + backward: T=196 611 us with a row or column of the state per thread, gk and gv in walks of
+// their own and (backward) both directions in one block; 491 with 8 x 8 tiles and gk, gv together; 455 with the directions always
+// in two blocks (shorter pieces of work spread better over the SMs) and the bonus's scalars only where they are used; T=1024
+// 3045 -> 2163.  Sums of eight instead of one chain of 64 also leave half the error (9e-8 for 1.6e-7 in the 2-norm).
+// Three-part bfloat16 products in 64-token chunks left ten times that (9e-7).
 //
 // Decay gradient.  With p_t = r_t * (S_t gy_t) and q_t = k_t * (A_{t+1} v_t) (state parts
 // only, elementwise over key channels),
@@ -30,7 +31,7 @@
 // reader side minus the pairs that do not straddle t).  The sweeps write running sums of
 // p and q (accumulated in double) to scratch; a last elementwise kernel combines them and
 // applies d(d_t)/d(w_raw) = d_t * (-exp(w_raw)), which cancels the division by d_t.  gw is therefore off by the rounding
-// of p and q over the whole sequence (9e-6 in the 2-norm at T=1024; sums kept in double to the end: the same).  Where d_t
+// of p and q over the whole sequence (5e-6 in the 2-norm at T=1024; sums kept in double to the end: the same).  Where d_t
 // is zero in float so is the gradient; the difference is not taken there, since exp(w_raw) would multiply its rounding
 // without bound.
 //
@@ -39,16 +40,16 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
-#include <mutex>
 #include "vrwkv_internal.h"
 
 namespace wkv6 {
 
 constexpr int N = 64;          // head size
-constexpr int kBatch = 8;      // tokens per shared-memory batch (two batches of 10 KB per block: 11 blocks per SM)
+constexpr int kBatch = 8;      // tokens per shared-memory batch (two batches of 10 KB and 6 KB of results per block: 8 blocks per SM)
 constexpr int kParts = N / kBatch;   // threads that share one token's dot products
 constexpr int kVecs = 5;       // r, k, v, gy, decay
-enum Kind { KIND_Y = 0, KIND_GR = 1, KIND_GK = 2, KIND_GV = 3 };
+enum Kind { KIND_Y = 0, KIND_GR = 1, KIND_GK = 2, KIND_GV = 3 };      // results
+enum Walk { WALK_Y, WALK_GR, WALK_GK, WALK_GKV };                    // state S with y or gr read out of it, adjoint A with gk, or gk and gv
 enum Vec { V_R = 0, V_K = 1, V_V = 2, V_G = 3, V_D = 4 };
 
 struct Args {
@@ -79,27 +80,54 @@ struct Batch {
     float vg[kBatch];    // v_t . gy_t
     float ruk[kBatch];   // sum_i r_t[i] u[i] k_t[i]
 };
+struct Shared {
+    Batch buf[2];
+    float out[kBatch][N];         // read-outs of a batch: of the kept dimension,
+    float part[2][kBatch][N];     // and of the other one (gv), each warp's share
+};
+static_assert(sizeof(Shared) <= 48 * 1024, "more shared memory than a kernel has without asking");
 
 __device__ __forceinline__ size_t slot_of(const Args& a, int pair, int dir, int bh, int i) {
     return ((static_cast<size_t>(pair * 2 + dir) * a.B * a.H + bh) * (a.segs - 1) + i) * kSlot;
 }
 
-// One pass of one kind over a segment (with segs = 1, the whole sequence).  kRow: thread owns a row (key channel) of
-// the state, else a column (value channel).  kForward: direction of time.  kOut: how the result
-// meets the other direction's: OUT_WRITE (first pass of a block), OUT_ADD (second pass of the same
-// block), OUT_ATOMIC (the two directions run in two blocks and add into a zeroed output: exactly
-// two addends per element, so the sum does not depend on their order).
-enum OutMode { OUT_WRITE = 0, OUT_ADD = 1, OUT_ATOMIC = 2 };
-template <int kKind, bool kForward, int kOut, bool kSegments>
-__device__ __forceinline__ void sweep(const Args& a, Batch* buf, int b, int h, int seg, float u_self, const float* u_smem,
+__device__ __forceinline__ float2 dup(float x) { return make_float2(x, x); }
+__device__ __forceinline__ void lds8(const float* lo, const float* hi, float2 (&x)[4]) {
+    const float4 a = *reinterpret_cast<const float4*>(lo), b = *reinterpret_cast<const float4*>(hi);
+    x[0] = make_float2(a.x, a.y); x[1] = make_float2(a.z, a.w); x[2] = make_float2(b.x, b.y); x[3] = make_float2(b.z, b.w);
+}
+__device__ __forceinline__ float part_of(const float2 (&x)[4], int i) { return i & 1 ? x[i >> 1].y : x[i >> 1].x; }
+// Sums of v[0 .. 2 kHalf) over the lanes that differ in bit `mask`; a lane keeps the half that its bit names.
+template <int kHalf>
+__device__ __forceinline__ void sum_half(float (&v)[8], bool upper, int mask) {
+#pragma unroll
+    for (int i = 0; i < kHalf; ++i) {
+        const float got = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + kHalf], mask);
+        v[i] = (upper ? v[i + kHalf] : v[i]) + got;
+    }
+}
+
+// One walk over a segment (with segs = 1, the whole sequence).  kForward: direction of time.  The two directions run in two
+// blocks that add into a zeroed output: exactly two addends per element, so the sum does not depend on their order.
+//
+// Tile of a thread.  A read-out keeps one dimension of the state and sums over the other; a warp owns 32 of the kept indices
+// and all 64 of the summed ones, a thread 8 x 8: kept 32 warp + 8 (lane / 8) + e, summed 4 (lane % 8) + f (f < 4) and the same
+// + 32.  So a token costs 8 to 10 16-byte shared loads, none of them in conflict, for 192 to 256 multiply-adds (as pairs, f32x2),
+// where a thread with a whole row or column took 32 to 48 for 192 in one chain of sums; the eight lanes' sums are scattered
+// (7 shuffles) so that lane l ends with kept index 32 warp + l.  gk (kept: rows) and gv (columns) come from one walk of A: gv's
+// sums over a warp's rows meet the other warp's once per batch.
+template <int kWalk, bool kForward, bool kSegments>
+__device__ __forceinline__ void sweep(const Args& a, Shared& sh, int b, int h, int seg, float u_self, const float* u_smem,
                                       float& gu_acc) {
-    constexpr bool kRow = (kKind == KIND_GR || kKind == KIND_GK);
-    constexpr int kA = (kKind == KIND_Y || kKind == KIND_GR) ? V_K : V_R;   // rank-1 update: alpha beta^T
-    constexpr int kB_ = (kKind == KIND_Y || kKind == KIND_GR) ? V_V : V_G;
-    constexpr int kC = kKind == KIND_Y ? V_R : kKind == KIND_GR ? V_G : kKind == KIND_GK ? V_V : V_K;   // read-out
+    constexpr bool kState = kWalk == WALK_Y || kWalk == WALK_GR;               // S, else its adjoint
+    constexpr bool kKeepCols = kWalk == WALK_Y, kBoth = kWalk == WALK_GKV;
+    constexpr int kKind = kWalk == WALK_Y ? KIND_Y : kWalk == WALK_GR ? KIND_GR : KIND_GK;
+    constexpr int kA = kState ? V_K : V_R;                                     // rank-1 update: alpha beta^T
+    constexpr int kB_ = kState ? V_V : V_G;
+    constexpr int kC = kWalk == WALK_Y ? V_R : kWalk == WALK_GR ? V_G : V_V;   // read-out
     // the rightward state S> runs forward in time, its adjoint A> backward; mirrored for "<"
-    constexpr bool kRightward = (kKind == KIND_Y || kKind == KIND_GR) ? kForward : !kForward;
-    const int tid = threadIdx.x;
+    constexpr bool kRightward = kState ? kForward : !kForward;
+    const int tid = threadIdx.x, lane = tid & 31, kept = tid & ~7, summed = 4 * (lane & 7);
     const int first = kSegments ? seg * a.seg_len : 0, T = kSegments ? min(a.seg_len, a.T - first) : a.T, C = a.H * N;
     const size_t base = (static_cast<size_t>(b) * a.T + first) * C + static_cast<size_t>(h) * N;
     const int n_batches = (T + kBatch - 1) / kBatch;
@@ -111,7 +139,7 @@ __device__ __forceinline__ void sweep(const Args& a, Batch* buf, int b, int h, i
             const float* src = a.src[vsel];
             if (src == nullptr) continue;
 #pragma unroll
-            for (int q = 0; q < (kBatch * N / 4) / N; ++q) {          // 256 chunks of 16 B, 64 threads
+            for (int q = 0; q < (kBatch * N / 4) / N; ++q) {          // 128 chunks of 16 B, 64 threads
                 const int chunk = q * N + tid;
                 const int row = chunk >> 4, col4 = (chunk & 15) * 4;      // 16 chunks of 16 bytes per token row
                 const int t = bt0 + row;
@@ -121,31 +149,30 @@ __device__ __forceinline__ void sweep(const Args& a, Batch* buf, int b, int h, i
         cp_async_commit();
     };
 
-    float X[N];
+    float2 X[8][4];       // [kept e][pairs of summed]
 #pragma unroll
-    for (int n = 0; n < N; ++n) X[n] = 0.f;
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) X[e][f] = dup(0.f);
     const int before = !kSegments ? 0 : kForward ? seg : a.segs - 1 - seg;        // segments this direction has walked
     if (kSegments && before > 0) {
-        constexpr int kPair = (kKind == KIND_Y || kKind == KIND_GR) ? 0 : 1;
-        const float* from = a.states + slot_of(a, kPair, kForward ? 0 : 1, b * a.H + h, before - 1);
-        if (kRow) {
+        const float* from = a.states + slot_of(a, kState ? 0 : 1, kForward ? 0 : 1, b * a.H + h, before - 1);
+        const auto at = [&](int e, int f) {
+            const int p = kept + e, q = summed + (f & 3) + 32 * (f >> 2);
+            return kKeepCols ? from[p * N + q] : from[q * N + p];
+        };
 #pragma unroll
-            for (int n = 0; n < N; ++n) X[n] = from[n * N + tid];
-        } else {
+        for (int e = 0; e < 8; ++e)
 #pragma unroll
-            for (int n4 = 0; n4 < N / 4; ++n4) {
-                const float4 x = *reinterpret_cast<const float4*>(from + tid * N + 4 * n4);
-                X[4 * n4] = x.x; X[4 * n4 + 1] = x.y; X[4 * n4 + 2] = x.z; X[4 * n4 + 3] = x.w;
-            }
-        }
+            for (int f = 0; f < 4; ++f) X[e][f] = make_float2(at(e, 2 * f), at(e, 2 * f + 1));
     }
     double run = 0.0;
 
-    issue(0, &buf[0]);
+    issue(0, &sh.buf[0]);
     for (int bi = 0; bi < n_batches; ++bi) {
-        Batch* cur = &buf[bi & 1];
+        Batch* cur = &sh.buf[bi & 1];
         if (bi + 1 < n_batches) {
-            issue(bi + 1, &buf[(bi + 1) & 1]);
+            issue(bi + 1, &sh.buf[(bi + 1) & 1]);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
@@ -153,57 +180,97 @@ __device__ __forceinline__ void sweep(const Args& a, Batch* buf, int b, int h, i
         __syncthreads();
         const int bt0 = (kForward ? bi : n_batches - 1 - bi) * kBatch;
         const int rows = min(kBatch, T - bt0);
-        // decay in place, per-token scalars
+        // decay in place
         for (int row = 0; row < rows; ++row) cur->vec[V_D][row][tid] = expf(-expf(cur->vec[V_D][row][tid]));
-        {
+        if (kRightward) {       // per-token scalars of the bonus
+            constexpr bool kVg = kWalk != WALK_Y, kRuk = kWalk == WALK_Y || kBoth;
             const int row = tid / kParts, part = tid % kParts;
             float s1 = 0.f, s2 = 0.f;
             if (row < rows) {
 #pragma unroll
                 for (int n = part * kBatch; n < part * kBatch + kBatch; ++n) {
-                    if (a.src[V_G] != nullptr) s1 += cur->vec[V_V][row][n] * cur->vec[V_G][row][n];
-                    s2 += cur->vec[V_R][row][n] * u_smem[n] * cur->vec[V_K][row][n];
+                    if (kVg) s1 += cur->vec[V_V][row][n] * cur->vec[V_G][row][n];
+                    if (kRuk) s2 += cur->vec[V_R][row][n] * u_smem[n] * cur->vec[V_K][row][n];
                 }
             }
 #pragma unroll
             for (int m = 1; m < kParts; m <<= 1) {
-                s1 += __shfl_xor_sync(0xffffffffu, s1, m);
-                s2 += __shfl_xor_sync(0xffffffffu, s2, m);
+                if (kVg) s1 += __shfl_xor_sync(0xffffffffu, s1, m);
+                if (kRuk) s2 += __shfl_xor_sync(0xffffffffu, s2, m);
             }
-            if (part == 0 && row < kBatch) { cur->vg[row] = s1; cur->ruk[row] = s2; }
+            if (part == 0) { cur->vg[row] = s1; cur->ruk[row] = s2; }
         }
         __syncthreads();
+        // (two or four tokens at a time were slower: twice the code for the walks that share an SM)
+#pragma unroll 1
         for (int step = 0; step < rows; ++step) {
             const int row = kForward ? step : rows - 1 - step;
-            const int t = bt0 + row;
-            const float4* cv = reinterpret_cast<const float4*>(cur->vec[kC][row]);
-            float out = 0.f;
-            if (kRow) {
-                const float di = cur->vec[V_D][row][tid];
-                const float ai = cur->vec[kA][row][tid];
-                const float4* bv = reinterpret_cast<const float4*>(cur->vec[kB_][row]);
+            const auto by_kept = [&](int v, float2 (&x)[4]) { lds8(&cur->vec[v][row][kept], &cur->vec[v][row][kept + 4], x); };
+            const auto by_summed = [&](int v, float2 (&x)[4]) { lds8(&cur->vec[v][row][summed], &cur->vec[v][row][summed + 32], x); };
+            float out[8];
+            float2 c[4];
+            by_summed(kC, c);
+            if (kKeepCols) {
+                float2 d[4], al[4], be[4];
+                by_summed(V_D, d);
+                by_summed(kA, al);
+                by_kept(kB_, be);
 #pragma unroll
-                for (int n4 = 0; n4 < N / 4; ++n4) {
-                    const float4 c4 = cv[n4], b4 = bv[n4];
-                    out += c4.x * X[4 * n4 + 0]; X[4 * n4 + 0] = fmaf(di, X[4 * n4 + 0], ai * b4.x);
-                    out += c4.y * X[4 * n4 + 1]; X[4 * n4 + 1] = fmaf(di, X[4 * n4 + 1], ai * b4.y);
-                    out += c4.z * X[4 * n4 + 2]; X[4 * n4 + 2] = fmaf(di, X[4 * n4 + 2], ai * b4.z);
-                    out += c4.w * X[4 * n4 + 3]; X[4 * n4 + 3] = fmaf(di, X[4 * n4 + 3], ai * b4.w);
+                for (int e = 0; e < 8; ++e) {
+                    const float2 bj = dup(part_of(be, e));
+                    float2 o = __fmul2_rn(c[0], X[e][0]);
+#pragma unroll
+                    for (int f = 1; f < 4; ++f) o = __ffma2_rn(c[f], X[e][f], o);
+                    out[e] = o.x + o.y;
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) X[e][f] = __ffma2_rn(d[f], X[e][f], __fmul2_rn(al[f], bj));
                 }
             } else {
-                const float bj = cur->vec[kB_][row][tid];
-                const float4* av = reinterpret_cast<const float4*>(cur->vec[kA][row]);
-                const float4* dv = reinterpret_cast<const float4*>(cur->vec[V_D][row]);
+                float2 d[4], al[4], be[4], k4[4], g[4];
+                by_kept(V_D, d);
+                by_kept(kA, al);
+                by_summed(kB_, be);
+                if (kBoth) {
+                    by_kept(V_K, k4);
 #pragma unroll
-                for (int n4 = 0; n4 < N / 4; ++n4) {
-                    const float4 c4 = cv[n4], a4 = av[n4], d4 = dv[n4];
-                    out += c4.x * X[4 * n4 + 0]; X[4 * n4 + 0] = fmaf(d4.x, X[4 * n4 + 0], a4.x * bj);
-                    out += c4.y * X[4 * n4 + 1]; X[4 * n4 + 1] = fmaf(d4.y, X[4 * n4 + 1], a4.y * bj);
-                    out += c4.z * X[4 * n4 + 2]; X[4 * n4 + 2] = fmaf(d4.z, X[4 * n4 + 2], a4.z * bj);
-                    out += c4.w * X[4 * n4 + 3]; X[4 * n4 + 3] = fmaf(d4.w, X[4 * n4 + 3], a4.w * bj);
+                    for (int f = 0; f < 4; ++f) g[f] = dup(0.f);
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float2 di = dup(part_of(d, e)), ai = dup(part_of(al, e));
+                    float2 o = __fmul2_rn(c[0], X[e][0]);
+#pragma unroll
+                    for (int f = 1; f < 4; ++f) o = __ffma2_rn(c[f], X[e][f], o);
+                    out[e] = o.x + o.y;
+                    if (kBoth) {
+                        const float2 ki = dup(part_of(k4, e));
+#pragma unroll
+                        for (int f = 0; f < 4; ++f) g[f] = __ffma2_rn(ki, X[e][f], g[f]);
+                    }
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) X[e][f] = __ffma2_rn(di, X[e][f], __fmul2_rn(ai, be[f]));
+                }
+                if (kBoth) {
+                    float v[8] = {g[0].x, g[0].y, g[1].x, g[1].y, g[2].x, g[2].y, g[3].x, g[3].y};
+                    sum_half<4>(v, (lane & 16) != 0, 16);
+                    sum_half<2>(v, (lane & 8) != 0, 8);
+                    // columns summed + {0, 1} (+ 2: lane bit 3, + 32: lane bit 4)
+                    *reinterpret_cast<float2*>(&sh.part[tid >> 5][row][summed + 2 * ((lane >> 3) & 1) + 32 * (lane >> 4)]) = make_float2(v[0], v[1]);
                 }
             }
-            const size_t idx = base + static_cast<size_t>(t) * C + tid;
+            sum_half<4>(out, (lane & 4) != 0, 4);
+            sum_half<2>(out, (lane & 2) != 0, 2);
+            sum_half<1>(out, (lane & 1) != 0, 1);
+            sh.out[row][tid] = out[0];
+        }
+        if (kBoth) __syncthreads();
+        // results of the batch, thread = channel: running sums, bonus
+#pragma unroll
+        for (int step = 0; step < kBatch; ++step) {
+            const int row = kForward ? step : kBatch - 1 - step;
+            if (row >= rows) continue;
+            const size_t idx = base + static_cast<size_t>(bt0 + row) * C + tid;
+            float out = sh.out[row][tid];
             // running sums for the decay gradient (state part only)
             if (kKind == KIND_GR) {
                 run += static_cast<double>(cur->vec[V_R][row][tid] * out);
@@ -213,10 +280,11 @@ __device__ __forceinline__ void sweep(const Args& a, Batch* buf, int b, int h, i
                 run += static_cast<double>(cur->vec[V_K][row][tid] * out);
                 a.cum[kRightward ? 1 : 3][idx] = static_cast<float>(run);
             }
+            float out_v = kBoth ? sh.part[0][row][tid] + sh.part[1][row][tid] : 0.f;
             // the bonus term lives in the rightward direction only
             if (kRightward) {
                 if (kKind == KIND_Y) out += cur->ruk[row] * cur->vec[V_V][row][tid];
-                if (kKind == KIND_GV) out += cur->ruk[row] * cur->vec[V_G][row][tid];
+                if (kBoth) out_v += cur->ruk[row] * cur->vec[V_G][row][tid];
                 if (kKind == KIND_GR) {
                     const float kvg = cur->vec[V_K][row][tid] * cur->vg[row];
                     out += u_self * kvg;
@@ -224,57 +292,46 @@ __device__ __forceinline__ void sweep(const Args& a, Batch* buf, int b, int h, i
                 }
                 if (kKind == KIND_GK) out += u_self * cur->vec[V_R][row][tid] * cur->vg[row];
             }
-            float* dst = a.out[kKind] + idx;
-            if (kOut == OUT_WRITE) *dst = out;
-            else if (kOut == OUT_ADD) *dst += out;
-            else atomicAdd(dst, out);
+            atomicAdd(a.out[kKind] + idx, out);
+            if (kBoth) atomicAdd(a.out[KIND_GV] + idx, out_v);
         }
         __syncthreads();   // the batch buffer is refilled two iterations later
     }
 }
 
-// How the directions (and segments) of a (batch, head, kind) are spread over blocks.
-enum Mode {
-    WHOLE,         // one block runs both directions in turn
-    SPLIT,         // a block per direction (blockIdx.z); both add into a zeroed output
-    SEGMENTS,      // a block per direction (blockIdx.z & 1) and segment (blockIdx.z >> 1), likewise
-};
-template <bool kBackward, Mode kMode>
-__global__ void __launch_bounds__(N, 9) wkv6_sweep_kernel(const Args a) {
+constexpr int kPerSm = 7;      // blocks, of 128 registers a thread (as fast as 6 of 168, 1 to 4 % faster where there are many)
+// grid (b h, walk, direction + 2 segment)
+template <bool kBackward, bool kSeg>
+__global__ void __launch_bounds__(N, kPerSm) wkv6_sweep_kernel(const Args a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Batch* buf = reinterpret_cast<Batch*>(smem_raw);
+    Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
     __shared__ float u_smem[N];
-    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
-    const int kind = kBackward ? 1 + static_cast<int>(blockIdx.y) : 0;
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, seg = kSeg ? blockIdx.z >> 1 : 0;
+    const bool forward = (blockIdx.z & 1) != 0;      // in time
     const int tid = threadIdx.x;
     u_smem[tid] = a.u[h * N + tid];
     __syncthreads();
     const float u_self = u_smem[tid];
     float gu = 0.f;
-    constexpr bool kSeg = kMode == SEGMENTS;
-    constexpr int kOut1 = kMode == WHOLE ? OUT_WRITE : OUT_ATOMIC, kOut2 = kMode == WHOLE ? OUT_ADD : OUT_ATOMIC;
-    const bool first = kMode == WHOLE || (blockIdx.z & 1) == 0, second = kMode == WHOLE || (blockIdx.z & 1) == 1;
-    const int seg = kSeg ? blockIdx.z >> 1 : 0;
     if (!kBackward) {
-        if (first) sweep<KIND_Y, false, kOut1, kSeg>(a, buf, b, h, seg, u_self, u_smem, gu);   // leftward state first
-        if (second) sweep<KIND_Y, true, kOut2, kSeg>(a, buf, b, h, seg, u_self, u_smem, gu);
-    } else if (kind == KIND_GR) {
-        if (first) {
-            sweep<KIND_GR, true, kOut1, kSeg>(a, buf, b, h, seg, u_self, u_smem, gu);
-            a.gu_part[(static_cast<size_t>(b) * a.segs + seg) * a.H * N + h * N + tid] = gu;            // the bonus lives in this direction
-        }
-        if (second) sweep<KIND_GR, false, kOut2, kSeg>(a, buf, b, h, seg, u_self, u_smem, gu);
-    } else if (kind == KIND_GK) {
-        if (first) sweep<KIND_GK, false, kOut1, kSeg>(a, buf, b, h, seg, u_self, u_smem, gu);  // rightward adjoint: back in time
-        if (second) sweep<KIND_GK, true, kOut2, kSeg>(a, buf, b, h, seg, u_self, u_smem, gu);
+        if (forward) sweep<WALK_Y, true, kSeg>(a, sh, b, h, seg, u_self, u_smem, gu);
+        else sweep<WALK_Y, false, kSeg>(a, sh, b, h, seg, u_self, u_smem, gu);
+    } else if (blockIdx.y == 0 && a.out[KIND_GV] != nullptr) {      // the longest walk first
+        if (forward) sweep<WALK_GKV, true, kSeg>(a, sh, b, h, seg, u_self, u_smem, gu);
+        else sweep<WALK_GKV, false, kSeg>(a, sh, b, h, seg, u_self, u_smem, gu);
+    } else if (blockIdx.y == 0) {
+        if (forward) sweep<WALK_GK, true, kSeg>(a, sh, b, h, seg, u_self, u_smem, gu);
+        else sweep<WALK_GK, false, kSeg>(a, sh, b, h, seg, u_self, u_smem, gu);
+    } else if (forward) {
+        sweep<WALK_GR, true, kSeg>(a, sh, b, h, seg, u_self, u_smem, gu);
+        a.gu_part[(static_cast<size_t>(b) * a.segs + seg) * a.H * N + h * N + tid] = gu;            // the bonus lives in this direction
     } else {
-        if (first) sweep<KIND_GV, false, kOut1, kSeg>(a, buf, b, h, seg, u_self, u_smem, gu);
-        if (second) sweep<KIND_GV, true, kOut2, kSeg>(a, buf, b, h, seg, u_self, u_smem, gu);
+        sweep<WALK_GR, false, kSeg>(a, sh, b, h, seg, u_self, u_smem, gu);
     }
 }
 
 // ---- sequences in segments -------------------------------------------------------------------------------
-// A few sequences leave most of the chip idle, and the walk's latency (0.5 us a token) is all their time.  Such a sequence is
+// A few sequences leave most of the chip idle, and the walk's latency (0.3 us a token) is all their time.  Such a sequence is
 // cut into segments that are walked side by side, still token by token: first the state that each segment would leave
 // from zero, and its decay (wkv6_segment_state_kernel: the update without the read-out, half a token's work), then the states
 // behind every segment, S_j = decay_j S_{j-1} + own_j (wkv6_segment_scan_kernel), then the sweeps, each from the state
@@ -413,46 +470,16 @@ __global__ void wkv6_bonus_grad_kernel(int B, int C, const float* __restrict__ p
     gu[c] = acc;
 }
 
-// Blocks of the sweep kernel that fit the device at once (0 if the kernel cannot be configured).
-static int resident_blocks() {
-    static std::mutex lock;
-    static int cached[64];
-    static bool known[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    dev &= 63;
-    std::lock_guard<std::mutex> guard(lock);
-    if (!known[dev]) {
-        const int smem = static_cast<int>(2 * sizeof(Batch));
-        bool ok = true;
-        for (const auto kernel : {wkv6_sweep_kernel<false, WHOLE>, wkv6_sweep_kernel<false, SPLIT>, wkv6_sweep_kernel<false, SEGMENTS>,
-                                  wkv6_sweep_kernel<true, WHOLE>, wkv6_sweep_kernel<true, SPLIT>, wkv6_sweep_kernel<true, SEGMENTS>})
-            ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
-        int per_sm = 0, sms = 0;
-        ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wkv6_sweep_kernel<true, WHOLE>, N, smem) == cudaSuccess;
-        ok = ok && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
-        if (!ok) cudaGetLastError();
-        cached[dev] = ok ? per_sm * sms : 0;
-        known[dev] = true;
-    }
-    return cached[dev];
-}
-static bool configure() { return resident_blocks() > 0; }
-
-// The two directions of a (batch, head, kind) go to two blocks when that still fits the device in
-// one wave: the walks are latency-bound, so twice the blocks is close to twice the speed then.
-static bool split_directions(int blocks) { return 2 * blocks <= resident_blocks(); }
-
 struct Plan {
     int segs, len;
 };
 // How many segments a sequence is walked in, from the sizes alone (so a sequence's last bits may depend on how many others are in
-// the call).  The device holds nine blocks per SM, but three already hide each other's latency, and the states in front of the
-// segments cost half a walk (a third in the backward, whose three kinds share them).  So: segments until there are `fill`
-// blocks, and the whole walk where fewer than three come out or a segment would be shorter than a few batches.
-// us, whole / segments, forward and forward + backward: H=12 B=1 T=1024 515 / 62, 1053 / 194; T=196 105 / 34, 228 / 116; H=6 B=8
-// T=512 264 / 97, 560 / 319.  Where the line lies: forward, 360 blocks (B H = 180, T=400) 223 / 211, 432 blocks 224 / 235;
-// backward, 444 blocks (B H = 74, T=800) 867 / 644 for the pair, 720 blocks (B H = 120, T=400) 508 / 599.
+// the call).  Three or four blocks per SM already keep it busy, and the states in front of the
+// segments cost half a walk (a third in the backward, whose walks share them).  So: segments until there are `fill`
+// blocks (counted as if gk and gv had walks of their own), and the whole walk where fewer than three come out or a segment would be
+// shorter than a few batches.
+// us, whole / segments: forward + backward H=12 B=3 T=1024 770 / 389, B=4 T=400 325 / 236.  Where the line lies: forward, 312
+// blocks (B H = 156, T=400) 184 / 172, 432 blocks 186 / 202; backward, 74 to 96 sequences x heads (T=400) within 3 % either way.
 static Plan make_plan(int B, int T, int H, int kinds) {
     const long long fill = kinds == 1 ? 1110 : 1332, shortest = kinds == 1 ? 16 : 32, fewest = 3;
     const long long want = std::min(fill / (2LL * B * H * kinds), T / shortest);
@@ -480,7 +507,6 @@ size_t backward_workspace(int B, int T, int H) {
 // workspace: forward_workspace() bytes, or null (a sequence is then walked as a whole)
 int forward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
             const float* u, float* y, void* workspace, cudaStream_t stream) {
-    if (!configure()) return -1;
     const Plan pl = workspace ? make_plan(B, T, H, 1) : Plan{1, T};
     Args a{};
     a.B = B; a.T = T; a.H = H;
@@ -489,18 +515,16 @@ int forward(int B, int T, int H, const float* r, const float* k, const float* v,
     a.out[KIND_Y] = y;
     a.segs = pl.segs; a.seg_len = pl.len;
     a.states = pl.segs > 1 ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kHead) : nullptr;
-    const bool split = pl.segs > 1 || split_directions(B * H);
-    if (split) cudaMemsetAsync(y, 0, static_cast<size_t>(B) * T * H * N * sizeof(float), stream);
+    cudaMemsetAsync(y, 0, static_cast<size_t>(B) * T * H * N * sizeof(float), stream);
     if (pl.segs > 1) run_segment_states(a, 1, stream);
-    const auto kernel = pl.segs > 1 ? wkv6_sweep_kernel<false, SEGMENTS> : split ? wkv6_sweep_kernel<false, SPLIT> : wkv6_sweep_kernel<false, WHOLE>;
-    kernel<<<dim3(B * H, 1, split ? 2 * pl.segs : 1), N, 2 * sizeof(Batch), stream>>>(a);
+    const auto kernel = pl.segs > 1 ? wkv6_sweep_kernel<false, true> : wkv6_sweep_kernel<false, false>;
+    kernel<<<dim3(B * H, 1, 2 * pl.segs), N, sizeof(Shared), stream>>>(a);
     return pl.segs > 1 ? 3 : 1;
 }
 
 int backward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
              const float* u, const float* gy, float* gr, float* gk, float* gv, float* gw, float* gu,
              void* workspace, cudaStream_t stream) {
-    if (!configure()) return -1;
     const Plan pl = make_plan(B, T, H, 3);
     const int C = H * N;
     const size_t E = static_cast<size_t>(B) * T * C;
@@ -515,16 +539,12 @@ int backward(int B, int T, int H, const float* r, const float* k, const float* v
     ws += state_floats(B, H, pl, 2);
     for (int i = 0; i < 4; ++i) a.cum[i] = ws + i * E;
     a.gu_part = ws + 4 * E;
-    const int kinds = gv ? 3 : 2;      // gv == nullptr: the caller gets gv elsewhere (the kinds are gr, gk, gv in this order)
-    const bool split = pl.segs > 1 || split_directions(kinds * B * H);
-    if (split) {
-        cudaMemsetAsync(gr, 0, E * sizeof(float), stream);
-        cudaMemsetAsync(gk, 0, E * sizeof(float), stream);
-        if (gv) cudaMemsetAsync(gv, 0, E * sizeof(float), stream);
-    }
+    cudaMemsetAsync(gr, 0, E * sizeof(float), stream);
+    cudaMemsetAsync(gk, 0, E * sizeof(float), stream);
+    if (gv) cudaMemsetAsync(gv, 0, E * sizeof(float), stream);      // (gv == nullptr: the caller gets gv elsewhere)
     if (pl.segs > 1) run_segment_states(a, 2, stream);
-    const auto kernel = pl.segs > 1 ? wkv6_sweep_kernel<true, SEGMENTS> : split ? wkv6_sweep_kernel<true, SPLIT> : wkv6_sweep_kernel<true, WHOLE>;
-    kernel<<<dim3(B * H, kinds, split ? 2 * pl.segs : 1), N, 2 * sizeof(Batch), stream>>>(a);
+    const auto kernel = pl.segs > 1 ? wkv6_sweep_kernel<true, true> : wkv6_sweep_kernel<true, false>;
+    kernel<<<dim3(B * H, 2, 2 * pl.segs), N, sizeof(Shared), stream>>>(a);
     if (pl.segs > 1) {
         const size_t threads = static_cast<size_t>(B) * pl.segs * ((pl.len + kPiece - 1) / kPiece) * C;
         wkv6_segment_decay_grad_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(a, gw);
