@@ -318,10 +318,12 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
                                      void* workspace, size_t workspace_bytes, void* stream);
 
 /* Inference-only steps between the matrix products of a block.  No reference counterpart as kernels: tensor-op chains there.
- *   vrwkv_sigmoid_gate: out = sigmoid(r) * y, out in the type of r (CLS/vrwkv.py:182-187, 253-257); bfloat16 y needs bfloat16 r
+ *   vrwkv_sigmoid_gate: out = sigmoid(r) * y, out in the type of r (CLS/vrwkv.py:182-187, 253-257); bfloat16 y needs bfloat16 r;
+ *     _f32out: the bfloat16 result widened
  *   vrwkv_relu_square: out = relu(x)^2 in the type of x (CLS/vrwkv.py:251); _f32out: of bfloat16 x in float32 (exact)
  *   vrwkv_norm_residual: out = x + gamma * (normalise(a) * weight + bias) over rows of C <= 1024 channels, C % 4 == 0;
  *     weight and bias NULL: out = x + gamma * a; gamma NULL: 1 (CLS/vrwkv.py:297-318)
+ *   vrwkv_gated_norm_residual: the same with a = sigmoid(r) * y, all bfloat16
  *   vrwkv_head_norm_gate_bf16out: vrwkv_normgate_forward_f32 with group 64, the result rounded to bfloat16
  *   vrwkv_add_rows: out[i] = table[i mod period] + a[i], a bfloat16, float32 result; period a multiple of 8 that divides n
  *     (CLS/vrwkv.py:392, CLS/vrwkv6.py:200)
@@ -329,12 +331,15 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
  *     patch % 8 == 0, W % 4 == 0 (the operand of the patch embedding, CLS/vrwkv.py:357)
  * Sigmoid, its product and y are rounded to bfloat16 where r is.  All tensors 16-byte aligned. */
 int vrwkv_sigmoid_gate(long long n, const void* r, int r_is_bf16, const void* y, int y_is_bf16, void* out, void* stream);
+int vrwkv_sigmoid_gate_f32out(long long n, const uint16_t* r, const uint16_t* y, float* out, void* stream);
 int vrwkv_relu_square(long long n, const void* x, int is_bf16, void* out, void* stream);
 int vrwkv_relu_square_f32out(long long n, const uint16_t* x, float* out, void* stream);
 int vrwkv_add_rows(long long n, long long period, const float* table, const uint16_t* a, float* out, void* stream);
 int vrwkv_patch_rows(int B, int channels, int H, int W, int patch, const float* img, uint16_t* out, void* stream);
 int vrwkv_norm_residual(int rows, int C, float eps, const void* a, int a_is_bf16, const float* weight, const float* bias,
                         const float* gamma, const float* x, float* out, void* stream);
+int vrwkv_gated_norm_residual(int rows, int C, float eps, const uint16_t* r, const uint16_t* y, const float* weight, const float* bias,
+                              const float* gamma, const float* x, float* out, void* stream);
 int vrwkv_head_norm_gate_bf16out(int rows, int C, float eps, const float* x, const void* gate, int gate_is_bf16, int gate_act,
                                  const float* gamma, const float* beta, uint16_t* out, void* stream);
 

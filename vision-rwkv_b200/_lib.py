@@ -33,11 +33,13 @@ SIGNATURES = {
     "vrwkv_biwkv_forward_bf16": (_c_int, [_c_int] * 3 + [_ptr] * 6 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_backward_bf16": (_c_int, [_c_int] * 3 + [_ptr] * 9 + [_c_size_t, _ptr]),
     "vrwkv_sigmoid_gate": (_c_int, [ctypes.c_longlong, _ptr, _c_int, _ptr, _c_int, _ptr, _ptr]),
+    "vrwkv_sigmoid_gate_f32out": (_c_int, [ctypes.c_longlong] + [_ptr] * 4),
     "vrwkv_relu_square": (_c_int, [ctypes.c_longlong, _ptr, _c_int, _ptr, _ptr]),
     "vrwkv_relu_square_f32out": (_c_int, [ctypes.c_longlong] + [_ptr] * 3),
     "vrwkv_add_rows": (_c_int, [ctypes.c_longlong] * 2 + [_ptr] * 4),
     "vrwkv_patch_rows": (_c_int, [_c_int] * 5 + [_ptr] * 3),
     "vrwkv_norm_residual": (_c_int, [_c_int] * 2 + [ctypes.c_float, _ptr, _c_int] + [_ptr] * 6),
+    "vrwkv_gated_norm_residual": (_c_int, [_c_int] * 2 + [ctypes.c_float] + [_ptr] * 7),
     "vrwkv_head_norm_gate_bf16out": (_c_int, [_c_int] * 2 + [ctypes.c_float, _ptr, _ptr, _c_int, _c_int] + [_ptr] * 4),
     "vrwkv_qshift_mix_forward_bf16out": (_c_int, [_c_int] * 8 + [_ptr] * 4),
     "vrwkv_qshift_ddlerp_forward_bf16out": (_c_int, [_c_int] * 7 + [_ptr] * 3 + [_c_int] + [_ptr] * 2),

@@ -21,7 +21,7 @@ import torch.nn.functional as F
 import torch.utils.checkpoint as cp
 
 from . import epilogue, normgate
-from .qshift import qshift_mix_to
+from .qshift import qshift_mix_to, stock
 from .vrwkv import RUN_CUDA, inference_biwkv
 
 
@@ -84,7 +84,8 @@ class ChannelMix(nn.Module):
         self.receptance = nn.Linear(n_embd, n_embd, bias=False)
         self.value = nn.Linear(hidden, n_embd, bias=False)
 
-    def forward(self, x, resolution):
+    def gate_operands(self, x, resolution):
+        """(r, y) of the gate sigmoid(r) * y that ends the mix"""
         if self.shift_pixel > 0:
             xk, xr = qshift_mix_to((self.key, self.receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution,
                                    self.shift_pixel, self.channel_gamma)
@@ -93,7 +94,10 @@ class ChannelMix(nn.Module):
         k = epilogue.relu_square(self.key(xk), self.value if self.key_norm is None else None)
         if self.key_norm is not None:
             k = self.key_norm(k)
-        return epilogue.sigmoid_gate(self.receptance(xr), self.value(k))
+        return self.receptance(xr), self.value(k)
+
+    def forward(self, x, resolution):
+        return epilogue.sigmoid_gate(*self.gate_operands(x, resolution))
 
 
 class Block(nn.Module):
@@ -116,13 +120,17 @@ class Block(nn.Module):
             x = self.ln0(x)
         g1 = self.gamma1 if self.layer_scale else None
         g2 = self.gamma2 if self.layer_scale else None
+        # inference: the gate that ends the channel mix goes with the residual
+        split = not torch.is_grad_enabled() and stock(self.ffn, ChannelMix)
         if self.post_norm:
             x = epilogue.norm_residual(x, self.att(x, resolution), self.ln1, g1)
-            x = epilogue.norm_residual(x, self.ffn(x, resolution), self.ln2, g2)
-        else:
-            x = epilogue.residual(x, self.att(self.ln1(x), resolution), g1)
-            x = epilogue.residual(x, self.ffn(self.ln2(x), resolution), g2)
-        return x
+            if split:
+                return epilogue.gated_residual(x, *self.ffn.gate_operands(x, resolution), self.ln2, g2)
+            return epilogue.norm_residual(x, self.ffn(x, resolution), self.ln2, g2)
+        x = epilogue.residual(x, self.att(self.ln1(x), resolution), g1)
+        if split:
+            return epilogue.gated_residual(x, *self.ffn.gate_operands(self.ln2(x), resolution), None, g2)
+        return epilogue.residual(x, self.ffn(self.ln2(x), resolution), g2)
 
     def forward(self, x, resolution):
         if self.with_cp and x.requires_grad:

@@ -20,7 +20,7 @@ import torch.utils.checkpoint as cp
 
 from .backbone import _PatchEmbed, _ramp
 from . import epilogue, normgate
-from .qshift import qshift_ddlerp_to, qshift_mix_to
+from .qshift import qshift_ddlerp_to, qshift_mix_to, stock
 from .vrwkv6 import HEAD_SIZE, inference_rwkv6
 
 MIX_RANK = 32       # width of the low-rank branch that produces the five mixing offsets
@@ -122,13 +122,17 @@ class ChannelMixV6(nn.Module):
         self.receptance = nn.Linear(n_embd, n_embd, bias=False)
         self.value = nn.Linear(hidden, n_embd, bias=False)
 
-    def forward(self, x, resolution):
+    def gate_operands(self, x, resolution):
+        """(r, y) of the gate sigmoid(r) * y that ends the mix"""
         xk, xr = qshift_mix_to((self.key, self.receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution, self.shift_pixel,
                                head_dim=HEAD_SIZE)       # per-head shift + both interpolations in one pass
         k = epilogue.relu_square(self.key(xk), self.value if self.key_norm is None else None)
         if self.key_norm is not None:
             k = self.key_norm(k)
-        return epilogue.sigmoid_gate(self.receptance(xr), self.value(k))
+        return self.receptance(xr), self.value(k)
+
+    def forward(self, x, resolution):
+        return epilogue.sigmoid_gate(*self.gate_operands(x, resolution))
 
 
 class BlockV6(nn.Module):
@@ -153,13 +157,16 @@ class BlockV6(nn.Module):
         g2 = self.gamma2 if self.layer_scale else None
         # torch's own LayerNorm: these networks answer a change of a single rounding with 3 % of their result (see
         # vrwkv6.inference_rwkv6), so only steps that keep every bit are taken over
+        # inference: the gate that ends the channel mix goes with the residual, or leaves in the norm's type
+        split = not torch.is_grad_enabled() and stock(self.ffn, ChannelMixV6)
         if self.post_norm:
             x = epilogue.residual(x, self.ln1(self.att(x, resolution)), g1)
-            x = epilogue.residual(x, self.ln2(self.ffn(x, resolution)), g2)
-        else:
-            x = epilogue.residual(x, self.att(self.ln1(x), resolution), g1)
-            x = epilogue.residual(x, self.ffn(self.ln2(x), resolution), g2)
-        return x
+            a = epilogue.sigmoid_gate(*self.ffn.gate_operands(x, resolution), norm=self.ln2) if split else self.ffn(x, resolution)
+            return epilogue.residual(x, self.ln2(a), g2)
+        x = epilogue.residual(x, self.att(self.ln1(x), resolution), g1)
+        if split:
+            return epilogue.gated_residual(x, *self.ffn.gate_operands(self.ln2(x), resolution), None, g2)
+        return epilogue.residual(x, self.ffn(self.ln2(x), resolution), g2)
 
     def forward(self, x, resolution):
         if self.with_cp and x.requires_grad:

@@ -2,7 +2,8 @@
 //
 //   sigmoid_gate    sigmoid(r) * y                   classification/mmcls_custom/models/backbones/vrwkv.py:182-187, 253-257
 //   relu_square     relu(x)^2                        vrwkv.py:250-251
-//   norm_residual   x + gamma * LayerNorm(a), or x + gamma * a             vrwkv.py:297-318 (post- and pre-norm blocks)
+//   norm_residual   x + gamma * LayerNorm(a), or x + gamma * a             vrwkv.py:297-318 (post- and pre-norm blocks);
+//                   a may be given as r, y of sigmoid(r) * y, the gate that the channel mix ends with (vrwkv.py:253-257)
 //   head_norm_gate  (GroupNorm per 64-channel head) * activation(gate)     vrwkv6.py:133, 205-212, bfloat16 result
 //
 //   add_rows        rows of a table, repeated, plus bfloat16 a, in float32  vrwkv.py:392 (positions), vrwkv6.py:200 (decay)
@@ -20,6 +21,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include "vrwkv_b200.h"
 #include "vrwkv_internal.h"
 
@@ -76,19 +78,21 @@ __device__ __forceinline__ float relu2(float x) {
 }
 
 // out = sigmoid(r) * y; the last n % kVec elements go to one thread
-template <typename R, typename Y>
-__global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, const R* __restrict__ r, const Y* __restrict__ y, R* __restrict__ out) {
+// O = float with R = bfloat16: the rounded result, widened for a LayerNorm that takes it in float32 (the copy that torch makes of it
+// under autocast is a pass of 6 bytes per element, this one of 2 more: the matrix-state base model on 64 images 10.15 -> 9.90 ms).
+template <typename R, typename Y, typename O>
+__global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, const R* __restrict__ r, const Y* __restrict__ y, O* __restrict__ out) {
     const long long i = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVec;
     if (i + kVec <= n) {
         float a[kVec], b[kVec];
         load(r + i, a);
         load(y + i, b);
 #pragma unroll
-        for (int j = 0; j < kVec; ++j) a[j] = gated<R>(a[j], b[j]);
+        for (int j = 0; j < kVec; ++j) a[j] = rounded<R>(gated<R>(a[j], b[j]));
         store(out + i, a);
     } else {
         for (long long j = i; j < n; ++j)
-            out[j] = static_cast<R>(gated<R>(static_cast<float>(r[j]), static_cast<float>(y[j])));
+            out[j] = static_cast<O>(rounded<R>(gated<R>(static_cast<float>(r[j]), static_cast<float>(y[j]))));
     }
 }
 
@@ -143,16 +147,19 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // One warp per row, lane = 4 channels of each 128; kIters = ceil(C / 128).  Both inputs of a row are requested before the
-// first sum, so 6 C bytes per warp are in flight.
-template <typename A, int kIters>
-__global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C, float eps, const A* __restrict__ a, const float* __restrict__ weight,
+// first sum, so 6 C bytes per warp are in flight.  kGate: a holds y and `gate` r of a gate, whose result is rounded as
+// sigmoid_gate_kernel stores it: 12 bytes per element instead of 6 + 10 and a launch (the small
+// model on 256 images 6.80 -> 6.70 ms).
+template <typename A, int kIters, bool kGate>
+__global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C, float eps, const A* __restrict__ a, const A* __restrict__ gate,
+                                                                 const float* __restrict__ weight,
                                                                  const float* __restrict__ bias, const float* __restrict__ gamma,
                                                                  const float* __restrict__ x, float* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const size_t base = static_cast<size_t>(row) * C + 4 * lane;
-    float v[kIters][4], res[kIters][4];
+    float v[kIters][4], res[kIters][4], r[kGate ? kIters : 1][4];
 #pragma unroll
     for (int i = 0; i < kIters; ++i) {
 #pragma unroll
@@ -160,7 +167,16 @@ __global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C
         if (128 * i + 4 * lane < C) {
             load(a + base + 128 * i, v[i]);
             load(x + base + 128 * i, res[i]);
+            if (kGate) load(gate + base + 128 * i, r[i]);
         }
+    }
+    if (kGate) {
+#pragma unroll
+        for (int i = 0; i < kIters; ++i)
+            if (128 * i + 4 * lane < C) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[i][j] = rounded<A>(gated<A>(r[i][j], v[i][j]));
+            }
     }
     if (weight != nullptr) {
         const float inv = 1.f / static_cast<float>(C);
@@ -269,13 +285,16 @@ static bool misaligned(std::initializer_list<const void*> ps) {
 static long long blocks_of(long long n) { return (n + static_cast<long long>(kThreads) * kVec - 1) / (static_cast<long long>(kThreads) * kVec); }
 
 template <typename A, int kIters = 1>
-static void launch_norm_residual(int rows, int C, float eps, const A* a, const float* weight, const float* bias, const float* gamma, const float* x,
-                                 float* out, cudaStream_t s) {
+static void launch_norm_residual(int rows, int C, float eps, const A* a, const A* gate, const float* weight, const float* bias, const float* gamma,
+                                 const float* x, float* out, cudaStream_t s) {
     if constexpr (kIters < kMaxC / 128) {
-        if (C > 128 * kIters) return launch_norm_residual<A, kIters + 1>(rows, C, eps, a, weight, bias, gamma, x, out, s);
+        if (C > 128 * kIters) return launch_norm_residual<A, kIters + 1>(rows, C, eps, a, gate, weight, bias, gamma, x, out, s);
     }
-    const int per = kThreads / 32;
-    norm_residual_kernel<A, kIters><<<(rows + per - 1) / per, kThreads, 0, s>>>(rows, C, eps, a, weight, bias, gamma, x, out);
+    const int per = kThreads / 32, grid = (rows + per - 1) / per;
+    if constexpr (std::is_same<A, __nv_bfloat16>::value) {
+        if (gate != nullptr) return norm_residual_kernel<A, kIters, true><<<grid, kThreads, 0, s>>>(rows, C, eps, a, gate, weight, bias, gamma, x, out);
+    }
+    norm_residual_kernel<A, kIters, false><<<grid, kThreads, 0, s>>>(rows, C, eps, a, nullptr, weight, bias, gamma, x, out);
 }
 
 }  // namespace epilogue
@@ -289,9 +308,20 @@ extern "C" int vrwkv_sigmoid_gate(long long n, const void* r, int r_is_bf16, con
     const unsigned grid = static_cast<unsigned>(blocks_of(n));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     using H = __nv_bfloat16;
-    if (y_is_bf16) sigmoid_gate_kernel<H, H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(r), static_cast<const H*>(y), static_cast<H*>(out));
-    else if (r_is_bf16) sigmoid_gate_kernel<H, float><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(r), static_cast<const float*>(y), static_cast<H*>(out));
-    else sigmoid_gate_kernel<float, float><<<grid, kThreads, 0, s>>>(n, static_cast<const float*>(r), static_cast<const float*>(y), static_cast<float*>(out));
+    if (y_is_bf16) sigmoid_gate_kernel<H, H, H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(r), static_cast<const H*>(y), static_cast<H*>(out));
+    else if (r_is_bf16) sigmoid_gate_kernel<H, float, H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(r), static_cast<const float*>(y), static_cast<H*>(out));
+    else sigmoid_gate_kernel<float, float, float><<<grid, kThreads, 0, s>>>(n, static_cast<const float*>(r), static_cast<const float*>(y), static_cast<float*>(out));
+    return record_launches(1);
+}
+
+extern "C" int vrwkv_sigmoid_gate_f32out(long long n, const uint16_t* r, const uint16_t* y, float* out, void* stream) {
+    using namespace epilogue;
+    if (n <= 0 || blocks_of(n) > 0x7fffffffLL) return VRWKV_ERR_SHAPE;
+    if (!r || !y || !out) return VRWKV_ERR_NULL;
+    if (misaligned({r, y, out})) return VRWKV_ERR_ALIGNMENT;
+    using H = __nv_bfloat16;
+    sigmoid_gate_kernel<H, H, float><<<static_cast<unsigned>(blocks_of(n)), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        n, reinterpret_cast<const H*>(r), reinterpret_cast<const H*>(y), out);
     return record_launches(1);
 }
 
@@ -352,8 +382,20 @@ extern "C" int vrwkv_norm_residual(int rows, int C, float eps, const void* a, in
     if (C % 4 != 0 || C > kMaxC) return VRWKV_ERR_UNSUPPORTED;
     if (misaligned({a, weight, bias, gamma, x, out})) return VRWKV_ERR_ALIGNMENT;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (a_is_bf16) launch_norm_residual(rows, C, eps, static_cast<const __nv_bfloat16*>(a), weight, bias, gamma, x, out, s);
-    else launch_norm_residual(rows, C, eps, static_cast<const float*>(a), weight, bias, gamma, x, out, s);
+    if (a_is_bf16) launch_norm_residual<__nv_bfloat16>(rows, C, eps, static_cast<const __nv_bfloat16*>(a), nullptr, weight, bias, gamma, x, out, s);
+    else launch_norm_residual<float>(rows, C, eps, static_cast<const float*>(a), nullptr, weight, bias, gamma, x, out, s);
+    return record_launches(1);
+}
+
+extern "C" int vrwkv_gated_norm_residual(int rows, int C, float eps, const uint16_t* r, const uint16_t* y, const float* weight, const float* bias,
+                                         const float* gamma, const float* x, float* out, void* stream) {
+    using namespace epilogue;
+    if (rows <= 0 || C <= 0) return VRWKV_ERR_SHAPE;
+    if (!r || !y || !x || !out || (weight != nullptr) != (bias != nullptr)) return VRWKV_ERR_NULL;
+    if (C % 4 != 0 || C > kMaxC) return VRWKV_ERR_UNSUPPORTED;
+    if (misaligned({r, y, weight, bias, gamma, x, out})) return VRWKV_ERR_ALIGNMENT;
+    launch_norm_residual<__nv_bfloat16>(rows, C, eps, reinterpret_cast<const __nv_bfloat16*>(y), reinterpret_cast<const __nv_bfloat16*>(r), weight, bias,
+                                        gamma, x, out, static_cast<cudaStream_t>(stream));
     return record_launches(1);
 }
 

@@ -16,13 +16,18 @@ void same_place(const Tensor& t, const Tensor& like, const char* name) {
 }
 }  // namespace
 
-Tensor sigmoid_gate(const Tensor& r_, const Tensor& y_) {
+Tensor sigmoid_gate(const Tensor& r_, const Tensor& y_, bool wide) {
     same_place(y_, r_, "y");
     TORCH_CHECK(r_.sizes() == y_.sizes(), "r and y must have the same shape");
     const c10::cuda::CUDAGuard guard(r_.device());
     const Tensor r = flat(r_), y = flat(y_);
-    Tensor out = at::empty(r.sizes(), r.options());
-    if (r.numel() != 0)
+    TORCH_CHECK(!wide || (is_bf16(r) && is_bf16(y)), "only bfloat16 is widened");
+    Tensor out = at::empty(r.sizes(), wide ? r.options().dtype(at::kFloat) : r.options());
+    if (r.numel() == 0) return out;
+    if (wide)
+        check(vrwkv_sigmoid_gate_f32out(r.numel(), static_cast<uint16_t*>(r.data_ptr()), static_cast<uint16_t*>(y.data_ptr()), fp(out), stream_of(r)),
+              "vrwkv_sigmoid_gate_f32out");
+    else
         check(vrwkv_sigmoid_gate(r.numel(), r.data_ptr(), is_bf16(r), y.data_ptr(), is_bf16(y), out.data_ptr(), stream_of(r)), "vrwkv_sigmoid_gate");
     return out;
 }
@@ -63,13 +68,19 @@ Tensor patch_rows(const Tensor& img_, int64_t patch) {
     return out;
 }
 
-Tensor norm_residual(const Tensor& x_, const Tensor& a_, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
-                     const std::optional<Tensor>& gamma, double eps) {
+namespace {
+// r_: null, or a gate's operand (a_ is then what it gates)
+Tensor norm_residual_of(const Tensor& x_, const Tensor& a_, const Tensor* r_, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
+                        const std::optional<Tensor>& gamma, double eps) {
     same_place(a_, x_, "a");
     const int64_t C = x_.size(-1), rows = C ? x_.numel() / C : 0;
     TORCH_CHECK(a_.sizes() == x_.sizes(), "a must have the shape of x");
+    if (r_) {
+        same_place(*r_, x_, "r");
+        TORCH_CHECK(r_->sizes() == x_.sizes() && is_bf16(*r_) && is_bf16(a_), "r and y must be bfloat16 of the shape of x");
+    }
     const c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = flat(x_), a = flat(a_);
+    const Tensor x = flat(x_), a = flat(a_), r = r_ ? flat(*r_) : Tensor();
     Tensor kept[3];
     const std::optional<Tensor>* given[3] = {&weight, &bias, &gamma};
     const float* p[3] = {};
@@ -81,10 +92,25 @@ Tensor norm_residual(const Tensor& x_, const Tensor& a_, const std::optional<Ten
             p[i] = fp(kept[i]);
         }
     Tensor out = at::empty(x.sizes(), x.options());
-    if (x.numel() != 0)
+    if (x.numel() != 0 && r_)
+        check(vrwkv_gated_norm_residual(rows, C, static_cast<float>(eps), static_cast<uint16_t*>(r.data_ptr()), static_cast<uint16_t*>(a.data_ptr()),
+                                        p[0], p[1], p[2], fp(x), fp(out), stream_of(x)),
+              "vrwkv_gated_norm_residual");
+    else if (x.numel() != 0)
         check(vrwkv_norm_residual(rows, C, static_cast<float>(eps), a.data_ptr(), is_bf16(a), p[0], p[1], p[2], fp(x), fp(out), stream_of(x)),
               "vrwkv_norm_residual");
     return out;
+}
+
+}  // namespace
+
+Tensor norm_residual(const Tensor& x, const Tensor& a, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
+                     const std::optional<Tensor>& gamma, double eps) {
+    return norm_residual_of(x, a, nullptr, weight, bias, gamma, eps);
+}
+Tensor gated_norm_residual(const Tensor& x, const Tensor& r, const Tensor& y, const std::optional<Tensor>& weight,
+                           const std::optional<Tensor>& bias, const std::optional<Tensor>& gamma, double eps) {
+    return norm_residual_of(x, y, &r, weight, bias, gamma, eps);
 }
 
 Tensor head_norm_gate_half(const Tensor& x_, const Tensor& gate_, const Tensor& weight_, const Tensor& bias_, double eps, int64_t act) {

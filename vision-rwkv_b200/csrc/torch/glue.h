@@ -13,11 +13,13 @@ std::vector<Tensor> qshift_ddlerp_half(const Tensor& x, std::vector<Tensor> maas
                                        int64_t W, int64_t shift, int64_t head_dim);
 Tensor norm_gate(const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, int64_t group, double eps, int64_t act);
 // epilogue.cpp
-Tensor sigmoid_gate(const Tensor& r, const Tensor& y);
+Tensor sigmoid_gate(const Tensor& r, const Tensor& y, bool wide);      // wide: bfloat16 r, y to a float32 result
 Tensor relu_square(const Tensor& x, bool wide);      // wide: bfloat16 x to a float32 result
 Tensor add_rows(const Tensor& table, const Tensor& a);
 Tensor patch_rows(const Tensor& img, int64_t patch);
 Tensor norm_residual(const Tensor& x, const Tensor& a, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
                      const std::optional<Tensor>& gamma, double eps);
+Tensor gated_norm_residual(const Tensor& x, const Tensor& r, const Tensor& y, const std::optional<Tensor>& weight,
+                           const std::optional<Tensor>& bias, const std::optional<Tensor>& gamma, double eps);
 Tensor head_norm_gate_half(const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, double eps, int64_t act);
 }  // namespace vrwkv

@@ -353,13 +353,17 @@ PYBIND11_MODULE(_native, m) {
     m.def("biwkv_half", [](const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
         return vrwkv::guarded([&] { return vrwkv::biwkv_half(w, u, k, v); })();
     });
-    m.def("sigmoid_gate", [](const Tensor& r, const Tensor& y) { return vrwkv::guarded([&] { return vrwkv::sigmoid_gate(r, y); })(); });
+    m.def("sigmoid_gate", [](const Tensor& r, const Tensor& y, bool wide) { return vrwkv::guarded([&] { return vrwkv::sigmoid_gate(r, y, wide); })(); });
     m.def("relu_square", [](const Tensor& x, bool wide) { return vrwkv::guarded([&] { return vrwkv::relu_square(x, wide); })(); });
     m.def("add_rows", [](const Tensor& table, const Tensor& a) { return vrwkv::guarded([&] { return vrwkv::add_rows(table, a); })(); });
     m.def("patch_rows", [](const Tensor& img, int64_t patch) { return vrwkv::guarded([&] { return vrwkv::patch_rows(img, patch); })(); });
     m.def("norm_residual", [](const Tensor& x, const Tensor& a, std::optional<Tensor> weight, std::optional<Tensor> bias,
                               std::optional<Tensor> gamma, double eps) {
         return vrwkv::guarded([&] { return vrwkv::norm_residual(x, a, weight, bias, gamma, eps); })();
+    });
+    m.def("gated_norm_residual", [](const Tensor& x, const Tensor& r, const Tensor& y, std::optional<Tensor> weight, std::optional<Tensor> bias,
+                                    std::optional<Tensor> gamma, double eps) {
+        return vrwkv::guarded([&] { return vrwkv::gated_norm_residual(x, r, y, weight, bias, gamma, eps); })();
     });
     m.def("head_norm_gate_half", [](const Tensor& x, const Tensor& gate, const Tensor& weight, const Tensor& bias, double eps, int64_t act) {
         return vrwkv::guarded([&] { return vrwkv::head_norm_gate_half(x, gate, weight, bias, eps, act); })();

@@ -30,10 +30,12 @@ def relu_square(x, layer=None):
     return _lib.native().relu_square(x, wide)
 
 
-def sigmoid_gate(r, y):
-    """sigmoid(r) * y in the dtype of r (vrwkv.py:182-187, 253-257)."""
+def sigmoid_gate(r, y, norm=None):
+    """sigmoid(r) * y in the dtype of r (vrwkv.py:182-187, 253-257).  For a LayerNorm `norm` that takes it under autocast, where torch
+    widens a bfloat16 result to float32 first, it leaves widened."""
     if _inference(r, y) and r.shape == y.shape and (y.dtype == torch.float32 or r.dtype == torch.bfloat16):
-        return _lib.native().sigmoid_gate(r, y)
+        wide = norm is not None and r.dtype == y.dtype == torch.bfloat16 and torch.is_autocast_enabled("cuda") and stock(norm, nn.LayerNorm)
+        return _lib.native().sigmoid_gate(r, y, wide)
     return torch.sigmoid(r) * y.to(r.dtype)
 
 
@@ -49,13 +51,28 @@ def residual(x, a, gamma):
     return x + (a if gamma is None else gamma * a)
 
 
+def _norm_kernel(a, norm, C):
+    return (stock(norm, nn.LayerNorm) and norm.normalized_shape == (C,) and norm.bias is not None
+            and norm.weight.dtype == norm.bias.dtype == torch.float32 and (a.dtype == torch.float32 or torch.is_autocast_enabled("cuda")))
+
+
 def norm_residual(x, a, norm, gamma):
     """x + gamma * norm(a) for a LayerNorm `norm` (post-norm blocks).  Under autocast torch computes that norm in float32."""
-    C = x.shape[-1]
-    if (_residual_kernel(x, a, gamma) and stock(norm, nn.LayerNorm) and norm.normalized_shape == (C,) and norm.bias is not None
-            and norm.weight.dtype == norm.bias.dtype == torch.float32 and (a.dtype == torch.float32 or torch.is_autocast_enabled("cuda"))):
+    if _residual_kernel(x, a, gamma) and _norm_kernel(a, norm, x.shape[-1]):
         return _lib.native().norm_residual(x, a, norm.weight, norm.bias, gamma, norm.eps)
     return residual(x, norm(a), gamma)
+
+
+def gated_residual(x, r, y, norm, gamma):
+    """norm_residual(x, sigmoid_gate(r, y), norm, gamma), or residual(x, sigmoid_gate(r, y), gamma) where norm is None: what a block
+    does with its channel mix, in one pass where all of it is kernels."""
+    if (_residual_kernel(x, y, gamma) and _inference(r) and r.dtype == y.dtype == torch.bfloat16 and r.shape == y.shape
+            and (norm is None or _norm_kernel(y, norm, x.shape[-1]))):
+        if norm is None:
+            return _lib.native().gated_norm_residual(x, r, y, None, None, gamma, 0.0)
+        return _lib.native().gated_norm_residual(x, r, y, norm.weight, norm.bias, gamma, norm.eps)
+    a = sigmoid_gate(r, y)
+    return residual(x, a, gamma) if norm is None else norm_residual(x, a, norm, gamma)
 
 
 def head_norm_gate(x, gate, norm, head_size, layer, act):
