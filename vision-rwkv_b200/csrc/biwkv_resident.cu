@@ -75,6 +75,7 @@ enum ConstRow {
 
 // What one launch computes.
 enum class Mode {
+    single,     // every level: one CTA holds the sequence
     whole,      // every level: the CTAs of one cluster hold the sequence and exchange their sums
     linked,     // every level: several clusters hold the sequence, hand-over through global memory
     sums,       // no clusters: the sums of level 1 (forward) or level 2 (backward, level 1 given) of every sub-chunk and CTA
@@ -407,7 +408,8 @@ __device__ __forceinline__ int cluster_flag(const Ctx& c, int any) {
 // relative to the last token before them.  Returns with `unsafe` = OR over the cluster of `unsafe`
 // (level 0 only).
 //
-// kLocal: no cluster; the states returned are relative to the CTA, whose own sums go to memory.  kLinked: several clusters.
+// kLocal: no cluster; the states returned are relative to the CTA, whose own sums go to memory if anyone needs them.  kLinked: several
+// clusters.
 template <typename RW, bool kLocal, bool kLinked>
 __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F, Pair2 MF, Pair2 R, bool& unsafe TL_ARGS) {
     constexpr bool kMom = RW::kF == 4;
@@ -475,7 +477,9 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
         }
         if (level == 1) TL_MARK(23);
         if (kLinked) { ctaP = P; ctaM = M; }
-        if (kLocal) {
+        if (kLocal && c.cta_sums == nullptr) {
+            // one CTA is the whole sequence
+        } else if (kLocal) {
             c.cta_sums[lane] = P.x; c.cta_sums[kCs + lane] = P.y;
             if (kMom) { c.cta_sums[2 * kCs + lane] = M.x; c.cta_sums[3 * kCs + lane] = M.y; }
         } else {
@@ -507,7 +511,8 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
             }
         }
         if (kLinked) ctaS = S;
-        if (kLocal) {
+        if (kLocal && c.cta_sums == nullptr) {
+        } else if (kLocal) {
             c.cta_sums[RW::kF * kCs + lane] = S.x; c.cta_sums[(RW::kF + 1) * kCs + lane] = S.y;
         } else {
             float* st = c.stage + RW::kBlockF;
@@ -866,7 +871,8 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     constexpr bool kHalfG = kHalf && !kWide;                    // gy arrives as bfloat16
     constexpr bool kHalfOut = kHalf && (kBwd || !kWide);        // results leave as bfloat16
     constexpr bool kCluster = kUsesCluster<kMode>, kLinked = kMode == Mode::linked, kSums = kMode == Mode::sums || kMode == Mode::sums_keep;
-    constexpr bool kOwn1 = kCluster || (kSums && !kBwd);        // level 1 is this launch's to sum up; else given
+    constexpr bool kSingle = kMode == Mode::single;
+    constexpr bool kOwn1 = kCluster || kSingle || (kSums && !kBwd);        // level 1 is this launch's to sum up; else given
     constexpr bool kOwn2 = kBwd && kMode != Mode::spread;       // level 2 likewise
     constexpr bool kMom1 = RW::kF == 4;                         // level 1 carries first moments
     constexpr bool kResults = !kSums;                           // the launch writes results
@@ -1075,7 +1081,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         const float Tf = static_cast<float>(p.T);
         unsafe = (2.f * kmax.x + fabsf(u2.x) + fabsf(w2.x) + fmaxf(-w2.x, 0.f) * Tf > kSafeRange) ||
                  (2.f * kmax.y + fabsf(u2.y) + fabsf(w2.y) + fmaxf(-w2.y, 0.f) * Tf > kSafeRange);
-        e1 = fast_exchange<RW, kSums, kLinked>(c, 0, F, MF, R, unsafe TL_PASS);
+        e1 = fast_exchange<RW, kSums || kSingle, kLinked>(c, 0, F, MF, R, unsafe TL_PASS);
     } else {
         add_outside<kBwd && !kSums>(e1, c.cta + 2 * pr, p.state_rows, wl2, dP, dS);
     }
@@ -1094,7 +1100,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         // landed and everything the other CTAs sent has been waited for)
         // (a sequence of several clusters is not the exact kernel's to redo: the count alone switches on the chunked kernels, which
         // redo the whole call; without clusters the word that was read does)
-        if (kCluster && cta == 0 && threadIdx.x == 0) {
+        if ((kCluster || kSingle) && cta == 0 && threadIdx.x == 0) {
             const unsigned at = atomicAdd(p.redo_count, 1u);
             if (!kLinked) p.redo_list[at] = unit;
         }
@@ -1206,7 +1212,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         bool ignored = false;
         TL_MARK(5);
         if (kCluster && p.cluster > 1) cluster_wait();
-        if (kOwn2) e2 = fast_exchange<RW, kSums, kLinked>(c, 1, rr, mr, q, ignored TL_PASS);
+        if (kOwn2) e2 = fast_exchange<RW, kSums || kSingle, kLinked>(c, 1, rr, mr, q, ignored TL_PASS);
         else add_outside<true>(e2, c.sub + 2 * pr, kStateRows, wl2, dP, dS);
         if (kSums) {
             put_state(p.states2 + sub_at, kStateRows, e2, true);
@@ -1534,6 +1540,9 @@ struct Plan {
 
 // How many CTAs hold a sequence, and in how many clusters.
 //
+// One CTA (T <= 256, Mode::single): nothing to hand over or to wait for, and no room for what others send; the kernel without the
+// cluster steps took 51.5 for 53.3 us at B=256, T=196, C=384 (bfloat16, forward).
+//
 // One cluster (T <= 4096): as few CTAs as hold T, 256 tokens each, then only as many warps as the tokens need.  A CTA's life
 // is a chain whose length hardly depends on its tokens, so the fewest CTAs win, whether their number is a power of two or
 // not (forward / backward us at 131072 tokens, C=768): T=1500 6 CTAs 220 / 544, 8 CTAs 266 / 652; T=3000 12 CTAs 249 / 592,
@@ -1582,7 +1591,7 @@ static DeviceState g_dev[64];
 // kWide kernels exist for sequences of one cluster (the chunked kernels that stand by behind longer ones have no such form)
 template <bool kBwd, Types kTypes, Mode kMode>
 static auto kernel() {
-    constexpr bool kWide = kTypes == Types::wide && kMode == Mode::whole;
+    constexpr bool kWide = kTypes == Types::wide && (kMode == Mode::whole || kMode == Mode::single);
     return biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kTypes != Types::f32, kWide, kMode>;
 }
 template <bool kBwd, Types kTypes>
@@ -1599,7 +1608,7 @@ template <bool kBwd, Types kTypes, Mode kMode>
 static bool allow_kernel() { return allow(kernel<kBwd, kTypes, kMode>(), smem_bytes<kBwd, kMode>(kMaxWarps), kUsesCluster<kMode>); }
 template <bool kBwd, Types kTypes>
 static bool allow_types() {
-    bool good = allow_kernel<kBwd, kTypes, Mode::whole>() && allow(exact_kernel<kBwd, kTypes>(), smem_bytes<kBwd>(kMaxWarps), true);
+    bool good = allow_kernel<kBwd, kTypes, Mode::single>() && allow_kernel<kBwd, kTypes, Mode::whole>() && allow(exact_kernel<kBwd, kTypes>(), smem_bytes<kBwd>(kMaxWarps), true);
     if constexpr (kTypes != Types::wide) {
         good = good && allow_kernel<kBwd, kTypes, Mode::linked>() && allow_kernel<kBwd, kTypes, Mode::sums>() && allow_kernel<kBwd, kTypes, Mode::spread>();
         good = good && allow_kernel<false, kTypes, Mode::sums_keep>();
@@ -1800,7 +1809,7 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     bool done = true;
     if constexpr (kTypes == Types::wide) {
         if (pl.split || pl.segs > 1) return -1;
-        done = run<kBwd, kTypes, Mode::whole>(p, m, grid, stream);
+        done = pl.ctas == 1 ? run<kBwd, kTypes, Mode::single>(p, m, grid, stream) : run<kBwd, kTypes, Mode::whole>(p, m, grid, stream);
     } else if (pl.split) {
         unsigned* const kept_seen = !kBwd && kept ? static_cast<unsigned*>(kept) : nullptr;
         const auto chain = [&](float* sums, int rows) {
@@ -1820,6 +1829,8 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
         done = done && run<kBwd, kTypes, Mode::spread>(p, m, grid, stream);
     } else if (pl.segs > 1) {
         done = run<kBwd, kTypes, Mode::linked>(p, m, grid, stream);
+    } else if (pl.ctas == 1) {
+        done = run<kBwd, kTypes, Mode::single>(p, m, grid, stream);
     } else {
         done = run<kBwd, kTypes, Mode::whole>(p, m, grid, stream);
     }
