@@ -617,22 +617,27 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     // (4) outside state moved to this span's edges + inside state; then to this half's edges
     Enter e;
     {
-        const float* s = c.sub + warp * (RW::kSub * kCs) + 2 * p;
         const auto row = [](const float* x, int r) { return *reinterpret_cast<const float2*>(x + r * kCs); };
-        Pair2 Pw{row(s, 0), row(s, 1)}, MPw{f2(0.f, 0.f), f2(0.f, 0.f)}, Sw{row(s, RW::kF), row(s, RW::kF + 1)};
-        if (kMom) MPw = Pair2{row(s, 2), row(s, 3)};
-        if (!kLocal) {
+        const float* s = c.sub + warp * (RW::kSub * kCs) + 2 * p;
+        Pair2 Pw, MPw{f2(0.f, 0.f), f2(0.f, 0.f)}, Sw;
+        if (kLocal) {
+            Pw = Pair2{row(s, 0), row(s, 1)};
+            if (kMom) MPw = Pair2{row(s, 2), row(s, 3)};
+            Sw = Pair2{row(s, RW::kF), row(s, RW::kF + 1)};
+        } else {
             const float2 wl2 = row(c.consts + 2 * p, kWl2);
             const float dP = static_cast<float>(kSpan * warp), dS = static_cast<float>(kSpan * (nw - 1 - warp));
             const float2 pP = f2(ex2(-wl2.x * dP), ex2(-wl2.y * dP)), pS = f2(ex2(-wl2.x * dS), ex2(-wl2.y * dS));
             const float* g = c.cta + 2 * p;
             const float2 Xn = row(g, 0), Xd = row(g, 1);
+            Pw = Pair2{fma2(pP, Xn, row(s, 0)), fma2(pP, Xd, row(s, 1))};
             if (kMom) {
-                MPw.n = fma2(pP, fma2(dup(dP), Xn, row(g, 2)), MPw.n);
-                MPw.d = fma2(pP, fma2(dup(dP), Xd, row(g, 3)), MPw.d);
+                const float2 MXn = row(g, 2), MXd = row(g, 3);
+                MPw.n = fma2(pP, fma2(dup(dP), Xn, MXn), row(s, 2));
+                MPw.d = fma2(pP, fma2(dup(dP), Xd, MXd), row(s, 3));
             }
-            Pw = Pair2{fma2(pP, Xn, Pw.n), fma2(pP, Xd, Pw.d)};
-            Sw = Pair2{fma2(pS, row(g, RW::kF), Sw.n), fma2(pS, row(g, RW::kF + 1), Sw.d)};
+            const float2 Yn = row(g, RW::kF), Yd = row(g, RW::kF + 1);
+            Sw = Pair2{fma2(pS, Yn, row(s, RW::kF)), fma2(pS, Yd, row(s, RW::kF + 1))};
         }
         if (upper) {
             e.P = Pair2{mulc_add(Pw.n, l16h, l16l, keepA.n), mulc_add(Pw.d, l16h, l16l, keepA.d)};
@@ -1182,8 +1187,6 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                         const float2 ny = f2(nn.x * -inv.x, nn.y * -inv.y);
                         const float2 g_ = mul2(gys[j], inv);
                         const float2 h = mul2(g_, ny);                  // -H
-                        P.n = fma2(lam2, P.n, zx);
-                        P.d = fma2(lam2, P.d, zy);
                         if (kResults) {
                             g2[i * kRow] = g_;
                             hn[i] = h;
@@ -1191,6 +1194,10 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                             gu = fma2(zy, h, gu);
                             gwa = fma2(g_, PM.n, gwa);
                             gwa = fma2(h, PM.d, gwa);
+                        }
+                        P.n = fma2(lam2, P.n, zx);
+                        P.d = fma2(lam2, P.d, zy);
+                        if (kResults) {
                             PM.n = fma2(lam2, PM.n, P.n);
                             PM.d = fma2(lam2, PM.d, P.d);
                         }
