@@ -21,7 +21,7 @@ import torch.nn.functional as F
 import torch.utils.checkpoint as cp
 
 from . import epilogue, normgate
-from .qshift import qshift_mix_to, stock
+from .qshift import qshift_mix_to, stock, taken_over
 from .vrwkv import RUN_CUDA, inference_biwkv
 
 
@@ -70,6 +70,7 @@ class SpatialMix(nn.Module):
         return self.output(epilogue.sigmoid_gate(r, y))
 
 
+@taken_over
 class ChannelMix(nn.Module):
     def __init__(self, n_embd, n_layer, layer_id, channel_gamma=0.25, shift_pixel=1, hidden_rate=4,
                  key_norm=False):

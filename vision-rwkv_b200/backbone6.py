@@ -20,7 +20,7 @@ import torch.utils.checkpoint as cp
 
 from .backbone import _PatchEmbed, _ramp
 from . import epilogue, normgate
-from .qshift import qshift_ddlerp_to, qshift_mix_to, stock
+from .qshift import qshift_ddlerp_to, qshift_mix_to, stock, taken_over
 from .vrwkv6 import HEAD_SIZE, inference_rwkv6
 
 MIX_RANK = 32       # width of the low-rank branch that produces the five mixing offsets
@@ -109,6 +109,7 @@ class SpatialMixV6(nn.Module):
         return self.output(y.to(g.dtype) * g)
 
 
+@taken_over
 class ChannelMixV6(nn.Module):
     def __init__(self, n_embd, n_layer, layer_id, shift_pixel=1, hidden_rate=4, key_norm=False):
         super().__init__()

@@ -15,10 +15,26 @@ import torch.nn as nn
 from . import _lib, ops, traced
 
 
+_FORWARDS = {}      # what `forward` of a class was when its work was taken over by kernels
+
+
+def taken_over(cls):
+    """Class decorator: kernels may do the work of `cls.forward` as it stands (torch's own, if it is torch's class)."""
+    f = cls.forward
+    if f.__module__ == cls.__module__ and f.__qualname__ == f"{cls.__qualname__}.forward":
+        _FORWARDS[cls] = f
+    return cls
+
+
+for _cls in (nn.Linear, nn.LayerNorm, nn.Conv2d):
+    taken_over(_cls)
+
+
 def stock(module, cls):
-    """Whether calling `module` runs `cls.forward` and nothing else: no subclass, no forward of its own, no hooks (its own or
-    those registered for all modules)."""
-    return (type(module) is cls and "forward" not in module.__dict__ and not module._forward_hooks and not module._forward_pre_hooks
+    """Whether calling `module` runs the `cls.forward` that was `taken_over` and nothing else: no subclass, no forward put in its
+    place (on the class or the instance), not compiled in place, no hooks (its own or those registered for all modules)."""
+    return (type(module) is cls and _FORWARDS.get(cls) is cls.forward and "forward" not in module.__dict__
+            and module._compiled_call_impl is None and not module._forward_hooks and not module._forward_pre_hooks
             and not nn.modules.module._global_forward_hooks and not nn.modules.module._global_forward_pre_hooks)
 
 
