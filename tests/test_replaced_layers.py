@@ -50,3 +50,22 @@ def test_a_block_calls_a_replaced_channel_mix(monkeypatch, v6, how, post_norm):
         want = x + block.ln1(torch.zeros_like(x)) if post_norm else x
         want = want + block.ln2(want * 2) if post_norm else want + block.ln2(want) * 2
     assert torch.equal(got, want)
+
+
+def test_a_trace_keeps_the_channel_mix_as_a_call():
+    block = backbone.Block(64, 2, 1, shift_pixel=0)
+    block.att = Skip()
+
+    class Net(nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.block = block
+
+        def forward(self, x):
+            return self.block(x, (2, 2))
+
+    x = torch.randn(2, 4, 64)
+    with torch.no_grad():
+        traced = torch.jit.trace(Net(), x)
+        assert "(ffn).forward(" in traced.block.code
+        assert torch.equal(traced(x), block(x, (2, 2)))

@@ -21,7 +21,7 @@ import torch.nn.functional as F
 import torch.utils.checkpoint as cp
 
 from . import epilogue, normgate
-from .qshift import qshift_mix_to, stock, taken_over
+from .qshift import qshift_mix_to, taken_over
 from .vrwkv import RUN_CUDA, inference_biwkv
 
 
@@ -122,7 +122,7 @@ class Block(nn.Module):
         g1 = self.gamma1 if self.layer_scale else None
         g2 = self.gamma2 if self.layer_scale else None
         # inference: the gate that ends the channel mix goes with the residual
-        split = not torch.is_grad_enabled() and stock(self.ffn, ChannelMix)
+        split = epilogue.takes_gate_of(self.ffn, ChannelMix)
         if self.post_norm:
             x = epilogue.norm_residual(x, self.att(x, resolution), self.ln1, g1)
             if split:

@@ -20,7 +20,7 @@ import torch.utils.checkpoint as cp
 
 from .backbone import _PatchEmbed, _ramp
 from . import epilogue, normgate
-from .qshift import qshift_ddlerp_to, qshift_mix_to, stock, taken_over
+from .qshift import qshift_ddlerp_to, qshift_mix_to, taken_over
 from .vrwkv6 import HEAD_SIZE, inference_rwkv6
 
 MIX_RANK = 32       # width of the low-rank branch that produces the five mixing offsets
@@ -159,7 +159,7 @@ class BlockV6(nn.Module):
         # torch's own LayerNorm: these networks answer a change of a single rounding with 3 % of their result (see
         # vrwkv6.inference_rwkv6), so only steps that keep every bit are taken over
         # inference: the gate that ends the channel mix goes with the residual, or leaves in the norm's type
-        split = not torch.is_grad_enabled() and stock(self.ffn, ChannelMixV6)
+        split = epilogue.takes_gate_of(self.ffn, ChannelMixV6)
         if self.post_norm:
             x = epilogue.residual(x, self.ln1(self.att(x, resolution)), g1)
             a = epilogue.sigmoid_gate(*self.ffn.gate_operands(x, resolution), norm=self.ln2) if split else self.ffn(x, resolution)

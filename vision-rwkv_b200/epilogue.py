@@ -63,6 +63,12 @@ def norm_residual(x, a, norm, gamma):
     return residual(x, norm(a), gamma)
 
 
+def takes_gate_of(mix, cls):
+    """Whether a block may take the gate's operands from its channel mix `mix` instead of calling it: when it is only being run, and
+    the call would do nothing else.  (A trace keeps the call, and with it the module in its graph.)"""
+    return not torch.is_grad_enabled() and not traced.tracing() and stock(mix, cls)
+
+
 def gated_residual(x, r, y, norm, gamma):
     """norm_residual(x, sigmoid_gate(r, y), norm, gamma), or residual(x, sigmoid_gate(r, y), gamma) where norm is None: what a block
     does with its channel mix, in one pass where all of it is kernels."""
