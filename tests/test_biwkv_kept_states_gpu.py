@@ -1,0 +1,63 @@
+"""What a forward under autograd keeps for its backward on sequences above 4096 tokens, as autograd's users meet it: saved-tensor
+hooks, a graph used twice, memory.  The bits are those of the pair that keeps nothing (see test_biwkv_split_gpu.py for both against
+the oracle), which takes two launches more."""
+import pytest
+import torch
+
+from oracle import biwkv_oracle as O
+
+pytestmark = pytest.mark.gpu
+SHAPE = (16, 4200, 64)      # 544 CTAs of 256 tokens, the last of a sequence holding 104
+
+
+def leaves(dev, half=False):
+    w, u, k, v, gy = [x.to(dev) for x in O.make_inputs(*SHAPE, dtype=torch.float32, seed=11)]
+    if half:
+        k, v = k.bfloat16(), v.bfloat16()
+    return [x.contiguous().requires_grad_(True) for x in (w, u, k, v)], gy.contiguous()
+
+
+def gradients(dev, pack=lambda t: t, unpack=lambda t: t):
+    """The gradients and the number of launches of the backward."""
+    from vision_rwkv_b200 import launch_count
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    xs, gy = leaves(dev)
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t.dtype), pack(t))[1], unpack):
+        y = RUN_CUDA(*xs)
+    before = launch_count()
+    grads = torch.autograd.grad(y, xs, gy)
+    assert seen.count(torch.uint8) == 1      # the kept states
+    return grads, launch_count() - before
+
+
+def rebuilt(dev):
+    from vision_rwkv_b200 import launch_count, ops
+    xs, gy = leaves(dev)
+    before = launch_count()
+    return ops.biwkv_backward(*[x.detach() for x in xs], gy), launch_count() - before
+
+
+def shifted(t, by):
+    if t.dtype != torch.uint8:
+        return t
+    return torch.empty(t.numel() + by, dtype=torch.uint8, device=t.device)[by:].copy_(t)
+
+
+@pytest.mark.parametrize("hook", ["host memory", "off by 1", "off by 16", "floats", "shorter", "dropped", "folded"])
+def test_saved_tensor_hooks(cuda_device, hook):
+    """Hooks that hand the bytes back, wherever they lie, keep the short backward; after others the states are rebuilt."""
+    pack, unpack, short = {
+        "host memory": (lambda t: t.cpu(), lambda t: t.to(cuda_device), True),
+        "off by 1": (lambda t: shifted(t, 1), lambda t: t, True),
+        "off by 16": (lambda t: shifted(t, 16), lambda t: t, True),
+        "floats": (lambda t: t.float(), lambda t: t, False),
+        "shorter": (lambda t: t[:-1] if t.dtype == torch.uint8 else t, lambda t: t, False),
+        "dropped": (lambda t: t[:0] if t.dtype == torch.uint8 else t, lambda t: t, False),
+        "folded": (lambda t: t.view(2, -1) if t.dtype == torch.uint8 else t, lambda t: t, False),
+    }[hook]
+    want, most = rebuilt(cuda_device)
+    got, launches = gradients(cuda_device, pack, unpack)
+    assert launches == (most - 2 if short else most)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)

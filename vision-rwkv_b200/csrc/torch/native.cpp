@@ -132,6 +132,16 @@ Tensor biwkv_forward(const Tensor& w, const Tensor& u, const Tensor& k, const Te
     return y.to(result_dtype(w));
 }
 
+// What a saved-tensor hook hands back for the kept states need not be what the forward left: the states are taken where it is still
+// a buffer of bytes of that size on this device, copied if it starts off the kernels' boundary, and rebuilt (undefined) otherwise.
+Tensor usable_states(const Tensor& kept, const Tensor& k) {
+    if (!kept.defined() || kept.scalar_type() != at::kByte || kept.device() != k.device() || kept.layout() != at::kStrided || kept.dim() != 1 ||
+        static_cast<size_t>(kept.numel()) != vrwkv_biwkv_kept_bytes(k.size(0), k.size(1), k.size(2)))
+        return Tensor();
+    const bool placed = kept.is_contiguous() && (reinterpret_cast<uintptr_t>(kept.data_ptr()) & 255u) == 0;
+    return placed ? kept : at::empty_like(kept, at::MemoryFormat::Contiguous).copy_(kept);
+}
+
 // k, v float32, or bfloat16 (then gy in either type); all contiguous.  kept: what the forward left, or undefined.
 std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& gy,
                                          const Tensor& kept = Tensor()) {
@@ -188,9 +198,10 @@ struct BiWkv : torch::autograd::Function<BiWkv> {
     }
     static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grads) {
         const auto saved = ctx->get_saved_variables();
-        const Tensor &w = saved[0], &u = saved[1], &k = saved[2], &v = saved[3], &kept = saved[4], &gy = grads[0];
+        const Tensor &w = saved[0], &u = saved[1], &k = saved[2], &v = saved[3], &gy = grads[0];
         const c10::cuda::CUDAGuard guard(k.device());
         const at::NoGradGuard no_grad;
+        const Tensor kept = usable_states(saved[4], k);
         const at::ScalarType out = result_dtype(w);
         const bool half = ctx->saved_data["bf16_io"].toBool() && is_bf16(k) && is_bf16(v);
         auto g = half ? biwkv_backward_raw(f32(w), f32(u), k.contiguous(), v.contiguous(), is_bf16(gy) ? gy.contiguous() : f32(gy), kept)
