@@ -61,3 +61,31 @@ def test_saved_tensor_hooks(cuda_device, hook):
     assert launches == (most - 2 if short else most)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+def allocated(f):
+    """What f() returns, the bytes it allocates in all and the most it holds at once."""
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    total, held = torch.cuda.memory_stats()["allocated_bytes.all.allocated"], torch.cuda.memory_allocated()
+    out = f()
+    return out, torch.cuda.memory_stats()["allocated_bytes.all.allocated"] - total, torch.cuda.max_memory_allocated() - held
+
+
+@pytest.mark.parametrize("half", [False, True])
+def test_nothing_is_allocated_twice(cuda_device, half):
+    """bfloat16 k, v with float32 w, as under autocast, have no kernels for a float32 y or gy above 4096 tokens: y is widened and gy
+    narrowed around the bfloat16 ones, and nothing else is set up first."""
+    from vision_rwkv_b200 import _lib
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    lib = _lib.load()
+    xs, gy = leaves(cuda_device, half)
+    n, size = gy.numel(), 2 if half else 4
+    slack = 5 << 20      # five tensors at most, and the allocator leaves up to 1 MiB of a block in place
+    y, total, _ = allocated(lambda: RUN_CUDA(*xs))
+    states, scratch = lib.vrwkv_biwkv_kept_bytes(*SHAPE), lib.vrwkv_biwkv_forward_workspace_bytes(*SHAPE)
+    assert 0 < states and total <= n * (size + (4 if half else 0)) + states + scratch + slack
+    _, total, most = allocated(lambda: torch.autograd.grad(y, xs, gy, retain_graph=True))
+    scratch = lib.vrwkv_biwkv_backward_workspace_bytes(*SHAPE)
+    assert total <= n * (2 * size + (2 if half else 0)) + scratch + slack
+    assert most <= n * (2 * size + (2 if half else 0)) + scratch + slack

@@ -103,18 +103,19 @@ Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, cons
     return y;
 }
 
+constexpr int64_t kMostWideTokens = 4096;      // of the entry points with float32 y, gy beside bfloat16 k, v
+
 // k, v bfloat16, contiguous; y float32 holding bfloat16 values.  Undefined where the kernel does not cover the call.
-Tensor biwkv_forward_wide(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, Tensor* kept) {
+Tensor biwkv_forward_wide(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+    if (k.size(1) > kMostWideTokens) return Tensor();
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor y = at::empty_like(k, k.options().dtype(at::kFloat));
     if (k.numel() == 0) return y;
     Tensor ws = workspace(vrwkv_biwkv_forward_workspace_bytes(B, T, C), k);
-    if (!kept || !biwkv_forward_keep(w, u, k, v, y, VRWKV_TENSORS_BF16_WIDE, ws, kept)) {
-        const int st = vrwkv_biwkv_forward_bf16_wide(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
-                                                     static_cast<uint16_t*>(v.data_ptr()), fp(y), ws.data_ptr(), ws.numel(), stream_of(k));
-        if (st == VRWKV_ERR_UNSUPPORTED) return Tensor();
-        check(st, "vrwkv_biwkv_forward_bf16_wide");
-    }
+    const int st = vrwkv_biwkv_forward_bf16_wide(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
+                                                 static_cast<uint16_t*>(v.data_ptr()), fp(y), ws.data_ptr(), ws.numel(), stream_of(k));
+    if (st == VRWKV_ERR_UNSUPPORTED) return Tensor();
+    check(st, "vrwkv_biwkv_forward_bf16_wide");
     raise_failures(k.get_device(), "vrwkv_biwkv_forward");
     return y;
 }
@@ -124,7 +125,7 @@ Tensor biwkv_forward(const Tensor& w, const Tensor& u, const Tensor& k, const Te
     const bool half = bf16_io && is_bf16(k) && is_bf16(v);
     if (half && result_dtype(w) == at::kFloat) {
         // float32 w, u under autocast: the kernel writes the widened result itself
-        const Tensor y = biwkv_forward_wide(f32(w), f32(u), k.contiguous(), v.contiguous(), kept);
+        const Tensor y = biwkv_forward_wide(f32(w), f32(u), k.contiguous(), v.contiguous());
         if (y.defined()) return y;
     }
     const Tensor y = half ? biwkv_forward_raw(f32(w), f32(u), k.contiguous(), v.contiguous(), kept)
@@ -145,6 +146,8 @@ Tensor usable_states(const Tensor& kept, const Tensor& k) {
 // k, v float32, or bfloat16 (then gy in either type); all contiguous.  kept: what the forward left, or undefined.
 std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& gy,
                                          const Tensor& kept = Tensor()) {
+    // the kernels for a float32 gy end there: narrowed before anything is allocated
+    if (is_bf16(k) && !is_bf16(gy) && k.size(1) > kMostWideTokens) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16), kept);
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor gk = at::empty_like(k), gv = at::empty_like(k);
     Tensor gwgu = at::empty({2, C}, k.options().dtype(at::kFloat));
@@ -155,9 +158,8 @@ std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const
     Tensor ws = workspace(vrwkv_biwkv_backward_workspace_bytes(B, T, C), k);
     int resumed = VRWKV_ERR_UNSUPPORTED;
     if (kept.defined()) {
-        const int tensors = !is_bf16(k) ? VRWKV_TENSORS_F32 : is_bf16(gy) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_BF16_WIDE;
         resumed = vrwkv_biwkv_backward_kept(B, T, C, fp(w), fp(u), k.data_ptr(), v.data_ptr(), gy.data_ptr(), fp(gwgu), gk.data_ptr(),
-                                            gv.data_ptr(), tensors, kept.data_ptr(), kept.numel(), ws.data_ptr(), ws.numel(), stream_of(k));
+                                            gv.data_ptr(), is_bf16(k) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_F32, kept.data_ptr(), kept.numel(), ws.data_ptr(), ws.numel(), stream_of(k));
         if (resumed != VRWKV_ERR_UNSUPPORTED) check(resumed, "vrwkv_biwkv_backward_kept");
     }
     if (resumed == VRWKV_OK) {
@@ -166,7 +168,7 @@ std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const
         const int st = vrwkv_biwkv_backward_bf16_wide(
             B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()), fp(gy), fp(gwgu),
             static_cast<uint16_t*>(gk.data_ptr()), static_cast<uint16_t*>(gv.data_ptr()), ws.data_ptr(), ws.numel(), stream_of(k));
-        if (st == VRWKV_ERR_UNSUPPORTED) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16), kept);
+        if (st == VRWKV_ERR_UNSUPPORTED) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16));
         check(st, "vrwkv_biwkv_backward_bf16_wide");
     } else if (is_bf16(k)) {
         const int st = vrwkv_biwkv_backward_bf16(
