@@ -89,3 +89,35 @@ def test_nothing_is_allocated_twice(cuda_device, half):
     scratch = lib.vrwkv_biwkv_backward_workspace_bytes(*SHAPE)
     assert total <= n * (2 * size + (2 if half else 0)) + scratch + slack
     assert most <= n * (2 * size + (2 if half else 0)) + scratch + slack
+
+
+def test_kept_states_are_not_in_the_workspace_too(cuda_device):
+    """The workspace of a call with kept states is smaller by them, and enough: memory behind it is not touched."""
+    from vision_rwkv_b200 import _lib, ops
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    lib = _lib.load()
+    B, T, C = SHAPE
+    states = lib.vrwkv_biwkv_kept_bytes(B, T, C)
+    sizes = [lib.vrwkv_biwkv_kept_workspace_bytes(B, T, C, backward) for backward in (0, 1)]
+    assert 0 < sizes[0] <= lib.vrwkv_biwkv_forward_workspace_bytes(B, T, C) - 2 * states // 3      # it would not hold the moments
+    assert 0 < sizes[1] <= lib.vrwkv_biwkv_backward_workspace_bytes(B, T, C) - states
+    assert lib.vrwkv_biwkv_kept_workspace_bytes(B, 4096, C, 0) == 0
+    xs, gy = leaves(cuda_device)
+    w, u, k, v = [x.detach() for x in xs]
+    y, gk, gv = (torch.empty_like(k) for _ in range(3))
+    gwgu, kept = torch.empty(2, C, device=cuda_device), torch.empty(states, dtype=torch.uint8, device=cuda_device)
+    buffers = [torch.full((size + 4096,), 0xA5, dtype=torch.uint8, device=cuda_device) for size in sizes]
+    s = torch.cuda.current_stream().cuda_stream
+    p = lambda t: t.data_ptr()
+    forward = lambda size: lib.vrwkv_biwkv_forward_keep(B, T, C, p(w), p(u), p(k), p(v), p(y), 0, p(kept), states, p(buffers[0]), size, s)
+    backward = lambda size: lib.vrwkv_biwkv_backward_kept(B, T, C, p(w), p(u), p(k), p(v), p(gy), p(gwgu), p(gk), p(gv), 0, p(kept), states,
+                                                          p(buffers[1]), size, s)
+    assert forward(sizes[0] - 1) == 3 and forward(sizes[0]) == 0 and backward(sizes[1] - 1) == 3 and backward(sizes[1]) == 0
+    for buffer, size in zip(buffers, sizes):
+        assert bool((buffer[size:] == 0xA5).all())
+    want = (ops.biwkv_forward(w, u, k, v), *ops.biwkv_backward(w, u, k, v, gy))
+    for got, ref in zip((y, gwgu[0], gwgu[1], gk, gv), want):
+        assert torch.equal(got, ref)
+    # and the autograd node allocates no more than that
+    _, total, _ = allocated(lambda: RUN_CUDA(*xs))
+    assert total <= y.numel() * 4 + states + sizes[0] + (3 << 20)      # three tensors, as above

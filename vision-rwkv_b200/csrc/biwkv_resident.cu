@@ -1687,10 +1687,11 @@ static StatesCarve carve_states(size_t units, const Plan& pl, int rows) {
 static size_t units_of(int B, int C) { return static_cast<size_t>(B) * ((C + kCs - 1) / kCs); }
 
 // workspace: status block (256 B) | longer sequences: segment flags, workspace of the kernels that stand by (all of that but the
-// end of the last to be cleared) | redo list | backward partials | copies of w, u | segment records | states of level 1, of level 2
+// end of the last to be cleared) | redo list | backward partials | copies of w, u | segment records | states of level 2, of level 1 (the
+// last not where they are kept)
 constexpr size_t kStatusBytes = 256;
 struct Carve {
-    size_t off_flags, off_stand_by, cleared, off_list, off_partial, off_vectors, off_records, off_states1, off_states2, total;
+    size_t off_flags, off_stand_by, cleared, off_list, off_partial, off_vectors, off_records, off_states2, off_states1, total;
 };
 static Carve carve(int B, int T, int C, const Plan& pl, bool bwd) {
     const size_t units = units_of(B, C), recs = pl.segs > 1 ? units * pl.segs * 4 : 0;
@@ -1703,16 +1704,17 @@ static Carve carve(int B, int T, int C, const Plan& pl, bool bwd) {
     cv.off_partial = cv.off_list + align_up(units * sizeof(int), 256);
     cv.off_vectors = cv.off_partial + (bwd ? align_up(units * pl.ctas * 2 * kCs * sizeof(float), 256) : 0);
     cv.off_records = cv.off_vectors + align_up(2 * static_cast<size_t>(C) * sizeof(float), 256);
-    cv.off_states1 = cv.off_records + align_up(recs * kSegRec * sizeof(float), 256);
-    cv.off_states2 = cv.off_states1 + (pl.split ? carve_states(units, pl, bwd ? kStateRows : kPlainRows).total : 0);
-    cv.total = cv.off_states2 + (pl.split && bwd ? carve_states(units, pl, kStateRows).total : 0);
+    cv.off_states2 = cv.off_records + align_up(recs * kSegRec * sizeof(float), 256);
+    cv.off_states1 = cv.off_states2 + (pl.split && bwd ? carve_states(units, pl, kStateRows).total : 0);
+    cv.total = cv.off_states1 + (pl.split ? carve_states(units, pl, bwd ? kStateRows : kPlainRows).total : 0);
     return cv;
 }
 
-size_t workspace_bytes(int B, int T, int C, bool bwd) {
+size_t workspace_bytes(int B, int T, int C, bool bwd, bool kept) {
     Plan pl;
     if (!make_plan(B, T, C, pl)) return 256;
-    return carve(B, T, C, pl, bwd).total;
+    const Carve cv = carve(B, T, C, pl, bwd);
+    return kept ? cv.off_states1 : cv.total;
 }
 
 size_t kept_bytes(int B, int T, int C) {

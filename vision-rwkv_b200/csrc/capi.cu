@@ -198,6 +198,10 @@ size_t vrwkv_biwkv_kept_bytes(int B, int T, int C) {
     return biwkv::resident::kept_bytes(B, T, C);
 }
 
+size_t vrwkv_biwkv_kept_workspace_bytes(int B, int T, int C, int backward) {
+    return vrwkv_biwkv_kept_bytes(B, T, C) == 0 ? 0 : biwkv::resident::workspace_bytes(B, T, C, backward != 0, true);
+}
+
 int vrwkv_biwkv_forward_keep(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, int tensors,
                              void* kept, size_t kept_bytes, void* workspace, size_t workspace_bytes, void* stream) {
     if (int st = check_shape(B, T, C)) return st;
@@ -205,7 +209,7 @@ int vrwkv_biwkv_forward_keep(int B, int T, int C, const float* w, const float* u
     if (!types_of(tensors, types)) return VRWKV_ERR_UNSUPPORTED;
     if (!w || !u || !k || !v || !y || !kept || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(kept)) & 255u)) return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    if (workspace_bytes < vrwkv_biwkv_kept_workspace_bytes(B, T, C, 0)) return VRWKV_ERR_WORKSPACE;
     if (!resident_serves(B, T, C, {k, v, y}, false, types)) return VRWKV_ERR_UNSUPPORTED;
     if (biwkv::resident::kept_bytes(B, T, C) == 0) return VRWKV_ERR_UNSUPPORTED;
     if (kept_bytes < biwkv::resident::kept_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
@@ -221,7 +225,7 @@ int vrwkv_biwkv_backward_kept(int B, int T, int C, const float* w, const float* 
     if (!w || !u || !k || !v || !gy || !gwgu || !gk || !gv || !kept || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || misaligned4(gwgu) || ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(kept)) & 255u))
         return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    if (workspace_bytes < vrwkv_biwkv_kept_workspace_bytes(B, T, C, 1)) return VRWKV_ERR_WORKSPACE;
     if (!resident_serves(B, T, C, {k, v, gy, gk, gv}, true, types)) return VRWKV_ERR_UNSUPPORTED;
     if (biwkv::resident::kept_bytes(B, T, C) == 0) return VRWKV_ERR_UNSUPPORTED;
     if (kept_bytes < biwkv::resident::kept_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;

@@ -66,14 +66,15 @@ at::ScalarType result_dtype(const Tensor& w) {
 }
 
 // The forward that keeps states for the backward, into `kept`; false (and an undefined `kept`) where it does not serve the call.
-bool biwkv_forward_keep(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& y, int tensors, const Tensor& ws,
-                        Tensor* kept) {
+bool biwkv_forward_keep(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& y, Tensor* kept) {
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     const size_t bytes = vrwkv_biwkv_kept_bytes(B, T, C);
     if (bytes == 0) return false;
     *kept = workspace(bytes, k);
-    const int st = vrwkv_biwkv_forward_keep(B, T, C, fp(w), fp(u), k.data_ptr(), v.data_ptr(), y.data_ptr(), tensors, kept->data_ptr(),
-                                            kept->numel(), ws.data_ptr(), ws.numel(), stream_of(k));
+    const Tensor ws = workspace(vrwkv_biwkv_kept_workspace_bytes(B, T, C, 0), k);
+    const int st = vrwkv_biwkv_forward_keep(B, T, C, fp(w), fp(u), k.data_ptr(), v.data_ptr(), y.data_ptr(),
+                                            is_bf16(k) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_F32, kept->data_ptr(), kept->numel(), ws.data_ptr(),
+                                            ws.numel(), stream_of(k));
     if (st != VRWKV_OK) kept->reset();
     if (st == VRWKV_ERR_UNSUPPORTED) return false;
     check(st, "vrwkv_biwkv_forward_keep");
@@ -86,10 +87,12 @@ Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, cons
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor y = at::empty_like(k);
     if (k.numel() == 0) return y;
+    if (kept && biwkv_forward_keep(w, u, k, v, y, kept)) {
+        raise_failures(k.get_device(), "vrwkv_biwkv_forward");
+        return y;
+    }
     Tensor ws = workspace(vrwkv_biwkv_forward_workspace_bytes(B, T, C), k);
-    if (kept && biwkv_forward_keep(w, u, k, v, y, is_bf16(k) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_F32, ws, kept)) {
-        // done
-    } else if (is_bf16(k)) {
+    if (is_bf16(k)) {
         const int st = vrwkv_biwkv_forward_bf16(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
                                                 static_cast<uint16_t*>(v.data_ptr()), static_cast<uint16_t*>(y.data_ptr()),
                                                 ws.data_ptr(), ws.numel(), stream_of(k));
@@ -155,13 +158,15 @@ std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const
         gwgu.zero_();
         return {gwgu.select(0, 0), gwgu.select(0, 1), gk, gv};
     }
-    Tensor ws = workspace(vrwkv_biwkv_backward_workspace_bytes(B, T, C), k);
+    Tensor ws;
     int resumed = VRWKV_ERR_UNSUPPORTED;
     if (kept.defined()) {
+        ws = workspace(vrwkv_biwkv_kept_workspace_bytes(B, T, C, 1), k);
         resumed = vrwkv_biwkv_backward_kept(B, T, C, fp(w), fp(u), k.data_ptr(), v.data_ptr(), gy.data_ptr(), fp(gwgu), gk.data_ptr(),
                                             gv.data_ptr(), is_bf16(k) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_F32, kept.data_ptr(), kept.numel(), ws.data_ptr(), ws.numel(), stream_of(k));
         if (resumed != VRWKV_ERR_UNSUPPORTED) check(resumed, "vrwkv_biwkv_backward_kept");
     }
+    if (resumed != VRWKV_OK) ws = workspace(vrwkv_biwkv_backward_workspace_bytes(B, T, C), k);
     if (resumed == VRWKV_OK) {
         // done
     } else if (is_bf16(k) && !is_bf16(gy)) {

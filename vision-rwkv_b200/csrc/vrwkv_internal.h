@@ -41,7 +41,8 @@ enum class Types {
 // True when it can serve this call on the current device.
 bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types);
 void set_withhold_test(bool on);   // test only: one rank per cluster sends nothing, waits give up early
-size_t workspace_bytes(int B, int T, int C, bool bwd);
+// kept: of a call that leaves or starts from kept states
+size_t workspace_bytes(int B, int T, int C, bool bwd, bool kept = false);
 // What a forward leaves for the backward: the states entering every 16 tokens, 1.5 bytes per element, and a flag; 0
 // where the backward takes nothing (T <= 4096, or few tokens in all).
 size_t kept_bytes(int B, int T, int C);
