@@ -208,11 +208,11 @@ __device__ __forceinline__ void st_async1(uint32_t addr, float v, uint32_t bar) 
 }
 
 // Debug timeline: with -DVRWKV_TIMELINE lane 0 of warps 0 and 5 of the first kTlCtas CTAs and of
-// kTlCtas CTAs from the middle of the grid store clock64() at each phase boundary behind the
-// workspace's status block.  Compiled out otherwise.
+// kTlCtas CTAs from the middle of the grid store clock64() at each phase boundary in a buffer of
+// 2 * kTlCtas * 2 * kTlMarks words that g_tl_base points to.  Compiled out otherwise.
 #ifdef VRWKV_TIMELINE
 constexpr int kTlCtas = 64, kTlMarks = 32;
-__device__ long long* g_tl_base = nullptr;      // where the marks go; unset: behind the status block
+__device__ long long* g_tl_base = nullptr;      // unset: no marks
 #define TL_MARK(m)                                                                                         \
     do {                                                                                                   \
         if (tl_slot >= 0 && lane == 0 && (warp == 0 || warp == 5))                                          \
@@ -909,9 +909,9 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     c.withhold = c.rank == p.withhold_rank;
 
 #ifdef VRWKV_TIMELINE
-    long long* tl_base = g_tl_base ? g_tl_base : reinterpret_cast<long long*>(reinterpret_cast<unsigned char*>(p.status) + 256);
+    long long* tl_base = g_tl_base;
     int tl_slot = -1;
-    {
+    if (tl_base != nullptr) {
         const int mid = (static_cast<int>(gridDim.x) / 2 / p.cluster) * p.cluster;
         if (static_cast<int>(blockIdx.x) < kTlCtas) tl_slot = blockIdx.x;
         else if (static_cast<int>(blockIdx.x) >= mid && static_cast<int>(blockIdx.x) < mid + kTlCtas) tl_slot = kTlCtas + blockIdx.x - mid;
