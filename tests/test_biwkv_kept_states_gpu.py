@@ -121,3 +121,55 @@ def test_kept_states_are_not_in_the_workspace_too(cuda_device):
     # and the autograd node allocates no more than that
     _, total, _ = allocated(lambda: RUN_CUDA(*xs))
     assert total <= y.numel() * 4 + states + sizes[0] + (3 << 20)      # three tensors, as above
+
+
+@pytest.mark.parametrize("k_scale", [1.0, 30.0])      # 30: outside the plain-float range, the kept word for that switches the kernels
+def test_a_second_backward_finds_the_states_unchanged(cuda_device, k_scale):
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    xs, gy = leaves(cuda_device)
+    xs[2] = (xs[2].detach() * k_scale).requires_grad_(True)
+    y = RUN_CUDA(*xs)
+    first = torch.autograd.grad(y, xs, gy, retain_graph=True)
+    again = torch.autograd.grad(y, xs, gy)
+    for a, b in zip(first, again):
+        assert torch.equal(a, b) and bool(a.isfinite().all())
+
+
+def test_vectors_that_start_at_an_odd_float(cuda_device):
+    """w and u go through a copy in the workspace, for the chain of the CTAs' sums as for the other launches."""
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    xs, gy = leaves(cuda_device)
+    odd = [torch.empty(x.numel() + 1, device=cuda_device)[1:].copy_(x.detach()).requires_grad_(True) for x in xs[:2]]
+    assert all(x.data_ptr() % 8 == 4 for x in odd)
+    y, y_odd = RUN_CUDA(*xs), RUN_CUDA(*odd, *xs[2:])
+    assert torch.equal(y, y_odd)
+    for a, b in zip(torch.autograd.grad(y, xs, gy), torch.autograd.grad(y_odd, [*odd, *xs[2:]], gy)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("half", [False, True])
+def test_a_captured_step_replays_on_new_inputs(cuda_device, half):
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    xs, gy = leaves(cuda_device, half)
+
+    def step():
+        y = RUN_CUDA(*xs)
+        return (y.detach(), *torch.autograd.grad(y, xs, gy))
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    with torch.no_grad():
+        for k_scale in (0.5, 40.0, 0.025):      # in the plain-float range, outside it, inside again
+            xs[2].mul_(k_scale)
+            graph.replay()
+            torch.cuda.synchronize()
+            with torch.enable_grad():
+                want = step()
+            for a, b in zip(captured, want):
+                assert torch.equal(a, b)

@@ -38,17 +38,26 @@ def test_same_bits_as_gate_then_residual(cuda_device, rows, C, normed, scaled):
 
 @pytest.mark.parametrize("name,overrides", [("vrwkv_t", {}), ("vrwkv_t", dict(post_norm=False)), ("vrwkv6_t", {}),
                                             ("vrwkv6_t", dict(post_norm=True, init_values=1.0))])
-def test_networks_keep_their_bits_and_their_hooks(cuda_device, name, overrides):
-    from vision_rwkv_b200 import backbone, backbone6
+def test_networks_keep_their_bits_and_their_hooks(cuda_device, monkeypatch, name, overrides):
+    from vision_rwkv_b200 import backbone, backbone6, epilogue, launch_count
     torch.manual_seed(3)
     build = backbone6.build_v6 if "6" in name else backbone.build
     model = build(name, img_size=64, depth=2, **overrides).to(cuda_device).eval()
     img = torch.randn(2, 3, 64, 64, device=cuda_device)
     with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        gates, gate = [], epilogue.sigmoid_gate
+        monkeypatch.setattr(epilogue, "sigmoid_gate", lambda r, y, norm=None: (gates.append(norm), gate(r, y, norm))[1])
+        before = launch_count()
         fused = model(img)[0]
-        seen = []
+        launches, widened, seen = launch_count() - before, [g for g in gates if g is not None], []
         handles = [layer.ffn.register_forward_hook(lambda m, i, o: seen.append(o.dtype)) for layer in model.layers]
+        before = launch_count()
         stepwise = model(img)[0]
         assert seen == [torch.bfloat16] * 2 and torch.equal(fused, stepwise)
+        # the fused pass took the gate with the residual, one launch less per layer, or (matrix-state, post-norm) widened it for the norm
+        if "6" in name and overrides.get("post_norm"):
+            assert widened == [layer.ln2 for layer in model.layers] and launch_count() - before == launches
+        else:
+            assert not widened and launch_count() - before == launches + 2
         for h in handles:
             h.remove()
