@@ -24,7 +24,7 @@
 //   3. the same two warps wait (bounded) for the bytes of the other CTAs and combine them;
 //   4. every thread adds the outside state, moved to its own position, to its inside state.
 // Forward: one level (terms e^{k}[v, 1]).  Backward: a second level for the adjoint pairs
-// [gy / Den, gy y / Den]; nothing is kept from the forward, y and Den are recomputed.
+// [gy / Den, gy y / Den]; y and Den are recomputed.  Nothing is kept from the forward, except above 4096 tokens (biwkv_chain_kernel).
 //
 // Arithmetic.  The fast path works on plain floats without any exponent shift: a term is
 // lambda e^{k} [v, 1] with lambda = e^{-w}, recurrences are one packed fused multiply-add per token
@@ -1488,13 +1488,14 @@ reduce_partials(Params p, float* __restrict__ out) {
 //                            (this kernel); k, v and both -> y (spread)
 //   backward                 the first two steps with first moments, unless the forward kept their results; k, v, gy and these
 //                            -> sums of the adjoint pairs (sums); chained; everything -> gk, gv, gw, gu (spread)
-// The launches are plain grids of independent CTAs, so each runs at the rate of HBM (5.9 to 6.4 TB/s; the states of every 16
-// tokens are 1 to 1.5 bytes per element and level).  That is 22 bytes per element forward where k, v, y are 12, and 38 backward
-// where 20 are necessary, but nothing waits for another CTA.  Several clusters per sequence (linked) move the necessary bytes and
-// spend more on the skew between their starts.  B=8, T=16384, C=768 forward + backward: 1926 us linked, 1060 us so; B=16, T=4200
-// 897 and 553 us.  In one launch these steps were slower: with a barrier of all CTAs between them and tiles handed out one by one
-// 1228 us, taken by tickets in the order of the steps 1428 us, and so with neighbouring sequences' steps side by side, so that
-// the second reads come from L2, 1224 us.
+// The launches are plain grids of independent CTAs, so each runs at the rate of HBM (5.9 to 6.9 TB/s for the bytes that it has to
+// move, some of them from L2; the states of every 16 tokens are 1 to 1.5 bytes per element and level).  That is 22 bytes per element
+// forward (23 with states kept) where k, v, y are 12, and 38 backward from kept states (47.5 without) where 20 are necessary, but nothing
+// waits for another CTA.  Several clusters per sequence (linked) move the necessary bytes and spend more on the skew between their
+// starts.  Forward + backward, float32: B=8, T=16384, C=768 1925 us linked, 1115 us so; B=16, T=4200 898 and 588 us.  (Both move by
+// 1 % with where the buffers lie.)  In one launch these steps were slower, beside 1060 us for separate launches of the same build: with a
+// barrier of all CTAs between them and tiles handed out one by one 1228 us, taken by tickets in the order of the steps 1428 us, and so
+// with neighbouring sequences' steps side by side, so that the second reads come from L2, 1224 us.
 //
 // This kernel: a warp takes one of four parts of a unit - towards later or earlier tokens, numerators or denominators -, lane =
 // channel, T / 256 steps over a few KB.  In double precision: rounded to float at every step, the results were a third further
@@ -1561,7 +1562,10 @@ struct Plan {
 // Above, separate launches (see biwkv_chain_kernel) from kSplitCtas CTAs of 256 tokens on.  Below that one launch of linked
 // clusters is as fast or faster, being fewer launches (forward / backward us, float32): B=1, C=192, T=8192 (192 CTAs) linked 25 /
 // 45, separate 27 / 53; T=16384 (384) 29 / 73 and 31 / 72; T=32768 (768) 56 / 178 and 43 / 111; B=2, C=768, T=4200 (816) 49 / 114
-// and 38 / 94.
+// and 38 / 94.  At the line itself, forward + backward, linked / separate, replayed from a graph: B=2, T=8192, C=256 (512) float32 101 /
+// 80, bfloat16 k, v with float32 w 112 / 92, with bfloat16 w 105 / 86; B=6, T=4200, C=192 (612) 116 / 88, 129 / 106, 122 / 96.  Called
+// one by one such steps are host time either way, 112 to 150 us, of which the four more launches take 5 to 10 (B=4, T=4200, C=256, all
+// bfloat16: 143 / 150).
 // Linked clusters: about 2048 tokens (8 CTAs) each, since clusters of 8 fill more SMs than clusters of 16, up to kMaxSegs of
 // them; the CTAs of a cluster follow from the tokens.
 constexpr long long kSplitCtas = 512;

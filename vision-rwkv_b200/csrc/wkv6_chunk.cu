@@ -631,9 +631,11 @@ __device__ __forceinline__ void pair_outputs(float (&y)[2][2][4], const __nv_bfl
 }
 
 // ---- kernel 2 ------------------------------------------------------------------------------------------------
-// A third of its stalls are loads.  Each CTA brings the inputs of the one that starts a little later (half an SM count of CTAs:
-// before that CTA has started, and so shortly that nothing is evicted) into L2.  B=32, H=12, forward / backward us, distance 0, 74,
-// 148, 296, 592: T=4096 1152 / 3311, 1110 / 3247, 1116 / 3297, 1126 / 3435, 1201 / 3461.
+// A third of its stalls are global loads (31 % forward, 30 % backward; shared memory another 13 %).  Each CTA brings the inputs of the
+// one that starts a little later (half an SM count of CTAs: before that CTA has started, and so shortly that nothing is evicted) into
+// L2, which leaves 23 and 27 %.  B=32, H=12, forward / backward us, distance 0, 74, 148, 296, 592: T=4096 1152 / 3311, 1110 / 3247,
+// 1116 / 3297, 1126 / 3435, 1201 / 3461.  The pair, loops of either in turn, each within 0.2 %: 4480 -> 4342; B=16, H=6 1186 -> 1157;
+// B=100, T=196 772 -> 764.
 // The rows of a head's chunk (all 256 threads share the lines):
 template <typename T>
 __device__ __forceinline__ void prefetch_rows(const T* p, int C, int rows) {

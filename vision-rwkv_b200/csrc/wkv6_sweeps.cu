@@ -17,8 +17,8 @@
 // A token's decay enters as the factor d_t alone, never as a difference of summed logarithms, so a token that forgets
 // everything (d_t = 0) leaves the others exact.
 //
-// What bounds it: the float32 pipe and the dependent steps of a token; 51 % of the pipe, half of the issue slots busy in the
-// forward.  B=32, H=12, forward + backward: T=196 611 us with a row or column of the state per thread, gk and gv in walks of
+// What bounds it: the float32 pipe and the dependent steps of a token; 51 % of the pipe and 52 % of the issue slots busy in the
+// forward, 59 % of either in the backward (B=32, T=196, H=12).  B=32, H=12, forward + backward: T=196 611 us with a row or column of the state per thread, gk and gv in walks of
 // their own and (backward) both directions in one block; 491 with 8 x 8 tiles and gk, gv together; 455 with the directions always
 // in two blocks (shorter pieces of work spread better over the SMs) and the bonus's scalars only where they are used; T=1024
 // 3045 -> 2163.  Sums of eight instead of one chain of 64 also leave half the error (9e-8 for 1.6e-7 in the 2-norm).
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(N, kPerSm) wkv6_sweep_kernel(const Args a) {
 // ---- sequences in segments -------------------------------------------------------------------------------
 // A few sequences leave most of the chip idle, and the walk's latency (0.3 us a token) is all their time.  Such a sequence is
 // cut into segments that are walked side by side, still token by token: first the state that each segment would leave
-// from zero, and its decay (wkv6_segment_state_kernel: the update without the read-out, half a token's work), then the states
+// from zero, and its decay (wkv6_segment_state_kernel: the update without the read-out, a row of the state per thread), then the states
 // behind every segment, S_j = decay_j S_{j-1} + own_j (wkv6_segment_scan_kernel), then the sweeps, each from the state
 // in front of its segment.  Decays are products of factors here too, so the accuracy is that of the whole walk.
 __global__ void __launch_bounds__(N, 9) wkv6_segment_state_kernel(const Args a) {
@@ -474,8 +474,8 @@ struct Plan {
     int segs, len;
 };
 // How many segments a sequence is walked in, from the sizes alone (so a sequence's last bits may depend on how many others are in
-// the call).  Three or four blocks per SM already keep it busy, and the states in front of the
-// segments cost half a walk (a third in the backward, whose walks share them).  So: segments until there are `fill`
+// the call).  Three or four blocks per SM already keep it busy, and the states in front of the segments take two thirds of the time
+// of the walks (38 of 60 us at B=3, T=1024, H=12; in the backward, whose walks share them, 69 of 156).  So: segments until there are `fill`
 // blocks (counted as if gk and gv had walks of their own), and the whole walk where fewer than three come out or a segment would be
 // shorter than a few batches.
 // us, whole / segments: forward + backward H=12 B=3 T=1024 770 / 389, B=4 T=400 325 / 236.  Where the line lies: forward, 312
