@@ -61,6 +61,14 @@ def test_argument_validation_without_a_device(lib):
     assert g(2, 4, 4, one, one, one, one, one, one, one, one, one, 8, null) == 3
 
 
+def test_nothing_is_kept_for_kernels_that_cannot_run(lib):
+    """A caller asks for the kept states' size before allocating them: 0 where the rows have no tensor maps."""
+    assert lib.vrwkv_biwkv_kept_bytes(16, 4200, 64) > 0
+    for C in (65, 66, 67):
+        assert lib.vrwkv_biwkv_kept_bytes(16, 4200, C) == 0 and lib.vrwkv_biwkv_kept_workspace_bytes(16, 4200, C, 1) == 0
+        assert lib.vrwkv_biwkv_backward_workspace_bytes(16, 4200, C) > 0
+
+
 def test_python_surface_refuses_cpu_tensors():
     import torch
     from vision_rwkv_b200 import ops

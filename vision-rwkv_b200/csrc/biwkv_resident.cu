@@ -1570,6 +1570,7 @@ struct Plan {
 // them; the CTAs of a cluster follow from the tokens.
 constexpr long long kSplitCtas = 512;
 static bool make_plan(int B, int T, int C, Plan& pl) {
+    if (C % 4 != 0) return false;      // no tensor maps over such rows, in either type
     constexpr int kCtaMax = kMaxWarps * kSpan;              // tokens one CTA holds
     constexpr int kSegMax = kMaxCluster * kCtaMax;          // tokens one cluster holds
     const auto up = [](int a, int b) { return (a + b - 1) / b; };
