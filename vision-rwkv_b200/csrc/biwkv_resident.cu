@@ -1492,8 +1492,8 @@ reduce_partials(Params p, float* __restrict__ out) {
 // move, some of them from L2; the states of every 16 tokens are 1 to 1.5 bytes per element and level).  That is 22 bytes per element
 // forward (23 with states kept) where k, v, y are 12, and 38 backward from kept states (47.5 without) where 20 are necessary, but nothing
 // waits for another CTA.  Several clusters per sequence (linked) move the necessary bytes and spend more on the skew between their
-// starts.  Forward + backward, float32: B=8, T=16384, C=768 1925 us linked, 1115 us so; B=16, T=4200 898 and 588 us.  (Both move by
-// 1 % with where the buffers lie.)  In one launch these steps were slower, beside 1060 us for separate launches of the same build: with a
+// starts.  Forward + backward, float32: B=8, T=16384, C=768 1927 us linked, 1128 us so; B=16, T=4200 899 and 591 us.  (The latter move
+// by 1 to 2 % with the board and with where the buffers lie.)  In one launch these steps were slower, beside 1060 us for separate launches of the same build: with a
 // barrier of all CTAs between them and tiles handed out one by one 1228 us, taken by tickets in the order of the steps 1428 us, and so
 // with neighbouring sequences' steps side by side, so that the second reads come from L2, 1224 us.
 //
