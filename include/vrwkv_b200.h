@@ -156,8 +156,9 @@ int vrwkv_biwkv_backward_bf16_wide(int B, int T, int C, const float* w, const fl
  * rebuilding them: two passes over the inputs instead of three.  vrwkv_biwkv_kept_bytes is 0 where a backward has no use for
  * them (T <= 4096, or few tokens in all).
  * w, u, k, v of the backward must be those of the forward.  `tensors` says what k, v, y, gy, gk, gv hold (enum below, as in the
- * entry points above; VRWKV_TENSORS_BF16_WIDE is refused at present: no kernels for it above 4096 tokens).  The workspaces are smaller than
- * those of the other entry points, by the states: vrwkv_biwkv_kept_workspace_bytes, 0 where nothing is kept.  VRWKV_ERR_UNSUPPORTED: outside the cluster-resident
+ * entry points above; VRWKV_TENSORS_BF16_WIDE is refused at present: no kernels for it above 4096 tokens).  The workspaces hold neither
+ * the states nor room for the other paths: vrwkv_biwkv_kept_workspace_bytes bytes, 0 where nothing is kept (those of the other entry
+ * points are larger and serve too).  VRWKV_ERR_UNSUPPORTED: outside the cluster-resident
  * kernels (shape, alignment, vrwkv_set_path), nothing ran, use the other entry points; a forward may succeed and the backward
  * still return it (for an unaligned gy).  Results agree with the pair that keeps nothing to float32 rounding; y is the same bit for bit.
  * No reference counterpart (its backward rebuilds everything, bi_wkv_kernel.cu:259-302). */
