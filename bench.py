@@ -946,7 +946,7 @@ def main():
     pair = "saved" if args.saved else "recompute"
     roofline = {"bound": "hbm",
                 "kernel": "Bi-WKV backward: " + ("biwkv_backward_saved tile kernel + partial reduction" if args.saved else
-                                                 "biwkv_resident_kernel<backward> (+ idle exact-arithmetic kernel and partial reduction)"),
+                                                 "biwkv_backward_kernel (+ idle exact-arithmetic kernel and partial reduction)"),
                 "achieved": bwd_gbs, "peak": peak, "peak_source": f"{peak_kind} copy bandwidth",
                 "unit": "GB/s", "frac": bwd_gbs / peak,
                 "traffic": NCU_BACKWARD_DRAM_BYTES[pair] * E / NCU_CAPTURE_ELEMENTS,

@@ -1,0 +1,58 @@
+"""Bi-WKV in narrow strips at the edges of its split: a walker's tokens (15 or 17), a warp's span (60, 68, 120, 136), a CTA's (480, 544, 960,
+1088) and those of clusters, one token less or more; strips past the last channel.  Against the float64 oracle with the tolerances
+of test_biwkv_gpu.py (1e-5) and test_biwkv_bf16_gpu.py (1e-2 for bfloat16 results; gw, gu are float32)."""
+import pytest
+import torch
+
+from conftest import rel_err
+from oracle import biwkv_oracle as O
+
+pytestmark = pytest.mark.gpu
+NAMES = ("y", "gw", "gu", "gk", "gv")
+
+
+def errors(dev, B, T, C, types, w_range=None):
+    from vision_rwkv_b200 import ops
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    w, u, k, v, gy = O.make_inputs(B, T, C, dtype=torch.float32, seed=7 * T + C)
+    if w_range is not None:
+        w = torch.linspace(*w_range, C) / T
+    if types != "f32":
+        k, v, gy = k.bfloat16(), v.bfloat16(), gy.bfloat16()
+    if types == "bf16":
+        w, u = w.bfloat16(), u.bfloat16()
+    if types == "wide":
+        gy = gy.float()      # the kernels round it; its rounding is not what is checked here
+    xs = [x.to(dev).contiguous().requires_grad_(True) for x in (w, u, k, v)]
+    y = RUN_CUDA(*xs)
+    got = (y.detach(), *torch.autograd.grad(y, xs, gy.to(dev)))
+    ops.raise_if_failed()
+    f = [x.double() for x in (w, u, k, v, gy)]
+    ref = (O.biwkv_scan_forward(*f[:4]), *O.biwkv_scan_backward(*f))
+    return {n: rel_err(g.float(), r) if r.abs().max() > 0 else g.abs().max().item() for n, g, r in zip(NAMES, got, ref)}
+
+
+def check(errs, types):
+    for name, e in errs.items():
+        assert e <= (1e-5 if types == "f32" or (types == "wide" and name in ("gw", "gu")) else 1e-2), (name, errs)
+
+
+EDGES = [1, 2, 15, 16, 17, 18, 34, 35, 60, 61, 68, 69, 120, 121, 136, 137, 300, 301, 480, 481, 544, 545, 600, 601, 680, 681, 960, 961, 1088, 1089, 1632, 1633,
+         2176, 2177, 3264, 3265, 3808, 3809]
+
+
+@pytest.mark.parametrize("T", EDGES)
+@pytest.mark.parametrize("C,types", [(44, "f32"), (40, "wide"), (24, "bf16")])
+def test_edges(cuda_device, T, C, types):
+    check(errors(cuda_device, 2, T, C, types), types)
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 5, 16, 49, 61, 200])
+@pytest.mark.parametrize("w_range", [(-30.0, -1.0), (1.0, 30.0), (-5.0, 3.0)])
+def test_steep_weights(cuda_device, T, w_range):
+    """Weights that grow or fall by orders of magnitude within the sequence: past its end they would overflow, or leave a denominator of
+    zero, and nothing of that may reach a valid token.  Each is inside the plain-float range for some channels and outside for others.
+    Tolerance: 5e-5, that of test_biwkv_gpu.py for extreme exponents."""
+    for types, tol in (("f32", 5e-5), ("wide", 1e-2)):
+        errs = errors(cuda_device, 3, T, 48, types, w_range)
+        assert all(e <= tol for e in errs.values()), errs

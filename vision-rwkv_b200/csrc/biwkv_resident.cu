@@ -1,10 +1,9 @@
-// Bi-WKV "resident" path (long sequences in number go another way, see biwkv_chain_kernel): the whole token range of one
-// (sequence, 32-channel strip) is held in the shared memory of ONE thread-block cluster while it is scanned in both directions, so every
-// element of k, v (and gy) crosses HBM once in and every output once out, and nothing but the
-// cluster's own CTAs ever has to be waited for.
+// Bi-WKV on sequences of more than 4096 tokens (shorter ones: biwkv_strips.cu).  Many of them: separate launches over independent CTAs,
+// see biwkv_chain_kernel.  Few: the whole token range of one (sequence, 32-channel strip) is held in the shared memory of a few
+// thread-block clusters while it is scanned in both directions (`linked`).
 //
-// Work unit: one (sequence b, strip of kCs = 32 channels).  A cluster of `cluster` CTAs (1 to 16)
-// splits its T tokens into contiguous ranges of n_tok = 32 * n_warps tokens, one per CTA.
+// Work unit: one (sequence b, strip of kCs = 32 channels).  Its T tokens are split into contiguous ranges of n_tok = 32 * n_warps
+// tokens, one per CTA, in clusters of `cluster` CTAs.
 // Inside a CTA warp s owns the span of 32 tokens [32 s, 32 s + 32); its lower half-warp walks the
 // first kL = 16 tokens of the span, its upper half-warp the last 16; lane p of a half-warp owns the
 // channel pair (2p, 2p+1).  A thread walks its 16 tokens sequentially with 64-bit shared accesses
@@ -24,18 +23,14 @@
 //   3. the same two warps wait (bounded) for the bytes of the other CTAs and combine them;
 //   4. every thread adds the outside state, moved to its own position, to its inside state.
 // Forward: one level (terms e^{k}[v, 1]).  Backward: a second level for the adjoint pairs
-// [gy / Den, gy y / Den]; y and Den are recomputed.  Nothing is kept from the forward, except above 4096 tokens (biwkv_chain_kernel).
+// [gy / Den, gy y / Den]; y and Den are recomputed.
 //
-// Arithmetic.  The fast path works on plain floats without any exponent shift: a term is
-// lambda e^{k} [v, 1] with lambda = e^{-w}, recurrences are one packed fused multiply-add per token
-// and direction.  That is exact enough whenever 2 max|k| + |u| + |w| + max(-w, 0) T <= 60 (no
-// overflow, no harmful underflow in float32).  Every thread checks its own tokens, the cluster
-// takes the OR of all checks with the first exchange, and if any thread saw otherwise the whole
-// cluster redoes the unit with the per-token max-shifted (value, exponent) arithmetic of
-// biwkv_math.cuh (k and v are fetched again, since the fast path overwrote them in place).  Decay
-// over long distances never comes from repeated multiplication by a rounded lambda: the
-// per-channel factors for 16, 32 and n_tok tokens are computed once per CTA in double precision
-// and applied as a (high, low) float pair.
+// Arithmetic.  Plain floats without any exponent shift: a term is lambda e^{k} [v, 1] with lambda = e^{-w}, recurrences are one packed
+// fused multiply-add per token and direction.  That is exact enough whenever 2 max|k| + |u| + |w| + max(-w, 0) T <= 60 (no
+// overflow, no harmful underflow in float32).  Every thread checks its own tokens; where one saw otherwise a word in the workspace
+// switches on the chunked kernels (biwkv_fused.cu), which stand by and redo the call.  Decay over long distances never comes from
+// repeated multiplication by a rounded lambda: the per-channel factors for 16, 32 and n_tok tokens are computed once per CTA in
+// double precision and applied as a (high, low) float pair.
 //
 // Recurrence restated: classification/mmcls_custom/models/backbones/cuda_new/
 // bi_wkv_kernel.cu:21-116 (forward), :119-367 (gradients).
@@ -48,12 +43,15 @@
 #include <initializer_list>
 #include <mutex>
 #include "biwkv_math.cuh"
+#include "biwkv_pairs.cuh"
 #include "sm100_async.cuh"
 #include "tensor_map.h"
 #include "vrwkv_internal.h"
 
 namespace biwkv {
 namespace resident {
+
+using namespace pairs;
 
 constexpr int kL = 16;            // tokens per thread
 constexpr int kSpan = 2 * kL;     // tokens per warp
@@ -64,7 +62,6 @@ constexpr int kCs = 32;           // channels per strip
 constexpr int kMaxWarps = 8;      // spans per CTA
 constexpr int kMaxCluster = 16;
 constexpr int kMaxThreads = kMaxWarps * 32;
-constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kSafeRange = 60.f;
 constexpr uint32_t kSpinLimit = 1u << 20;   // ~0.1 s of polling on a barrier
 
@@ -75,15 +72,13 @@ enum ConstRow {
 
 // What one launch computes.
 enum class Mode {
-    single,     // every level: one CTA holds the sequence
-    whole,      // every level: the CTAs of one cluster hold the sequence and exchange their sums
     linked,     // every level: several clusters hold the sequence, hand-over through global memory
     sums,       // no clusters: the sums of level 1 (forward) or level 2 (backward, level 1 given) of every sub-chunk and CTA
     sums_keep,  // forward: as sums, with the first moments that a backward needs
     spread,     // no clusters: every level given; writes the results
 };
 template <Mode m>
-constexpr bool kUsesCluster = m == Mode::whole || m == Mode::linked;
+constexpr bool kUsesCluster = m == Mode::linked;
 
 // rows of kCs floats in the record area behind the data slots
 template <bool kMom, bool kBwd>
@@ -97,7 +92,7 @@ struct RowsOf {
     static constexpr int kBlockR = kCs * kR + 4;   // ... towards earlier tokens
     static constexpr int kPeerFloats = (kMaxCluster - 1) * kBlockF;   // one block slot per other rank (ranks above this CTA's shift down by one)
 };
-template <bool kBwd, Mode kMode = Mode::whole>
+template <bool kBwd, Mode kMode = Mode::linked>
 using Rows = RowsOf<kBwd || kMode == Mode::sums_keep, kBwd>;
 constexpr int kStateRows = 6;      // states that enter a sub-chunk: P (n, d), its first moment (n, d), S (n, d)
 constexpr int kPlainRows = 4;      // ... without the moments
@@ -116,8 +111,7 @@ struct Params {
     unsigned* status;   // device status word
     unsigned* mirror;   // host-visible copy of a failure (may be null)
     float* partial;     // backward: [grid][2][kCs]
-    unsigned* redo_count;   // units the fast kernel left to the exact kernel ...
-    int* redo_list;         // ... and which
+    unsigned* redo_count;   // units that were outside the plain-float range
     uint32_t spin_limit;  // polls before a wait for the other CTAs gives up
     int withhold_rank;    // test only: this rank of every cluster sends nothing (-1: none)
     int ctas;             // CTAs per (sequence, strip)
@@ -142,69 +136,12 @@ constexpr int kMaxSegs = 8;
 
 // shared memory: data slots | span records | blocks received from the other CTAs | this CTA's two
 // outgoing blocks | state entering this CTA | constants | mbarriers and the flag word
-template <bool kBwd, Mode kMode = Mode::whole>
+template <bool kBwd, Mode kMode = Mode::linked>
 static inline size_t smem_bytes(int n_warps) {
     using R = Rows<kBwd, kMode>;
     const size_t data = static_cast<size_t>(R::kSlots) * n_warps * kSpan * kCs * sizeof(float);
     const size_t rec = (static_cast<size_t>(n_warps) * R::kSub * kCs + (kUsesCluster<kMode> ? R::kPeerFloats : 0) + R::kBlockF + R::kBlockR + kOutsideRows<kBwd, kMode> * kCs + kConstRows * kCs) * sizeof(float);
     return data + rec + 192;
-}
-
-// ---- small device helpers -----------------------------------------------------------------------
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float rcp(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 shfl2(float2 a, int mask) {
-    return f2(__shfl_xor_sync(0xffffffffu, a.x, mask), __shfl_xor_sync(0xffffffffu, a.y, mask));
-}
-__device__ __forceinline__ float2 sel2(bool c, float2 a, float2 b) { return c ? a : b; }
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// address of the same shared-memory location in the CTA of rank `rank` of this cluster
-__device__ __forceinline__ uint32_t peer_addr(const void* local, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(sm100::smem_u32(local)), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ float ld_peer(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
-// Asynchronous stores into another CTA's shared memory; the receiving CTA's mbarrier counts the
-// bytes, so data and notification travel together and the sender needs no fence.
-__device__ __forceinline__ void st_async4(uint32_t addr, float4 v, uint32_t bar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
-                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void st_async2(uint32_t addr, float2 v, uint32_t bar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(v.x),
-                 "f"(v.y), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void st_async1(uint32_t addr, float v, uint32_t bar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(v), "r"(bar)
-                 : "memory");
 }
 
 // Debug timeline: with -DVRWKV_TIMELINE lane 0 of warps 0 and 5 of the first kTlCtas CTAs and of
@@ -245,16 +182,9 @@ struct Ctx {
     float* cta_sums;         // launches without clusters: where this CTA's sums go, [state_rows][kCs]
 };
 
-// a thread's two channels: numerators (n) and denominators (d) of a state, each packed (ch 2p, ch 2p+1)
-struct Pair2 {
-    float2 n, d;
-};
 struct Enter {
     Pair2 P, MP, S;   // state (and first moment) entering at the first token; state entering at the last
 };
-
-// x * (hi + lo) + y, both channels
-__device__ __forceinline__ float2 mulc_add(float2 x, float2 hi, float2 lo, float2 y) { return fma2(x, hi, fma2(x, lo, y)); }
 
 // Element access of a thread's sub-chunk in one data slot.  `area` = the sub-chunk's 16 rows of kCs
 // floats (2 KB).  float32 tensors: row i is where it arrived.  bfloat16 tensors: the 16 rows arrive
@@ -273,7 +203,6 @@ __device__ __forceinline__ float2 ld_in(const float* area, int i, int pr) {
     }
     return *(reinterpret_cast<const float2*>(area + i * kCs) + pr);
 }
-__device__ __forceinline__ float2 round2(float2 v) { return __bfloat1622float2(__float22bfloat162_rn(v)); }
 template <bool kHalf>
 __device__ __forceinline__ void st_out(float* area, int i, int pr, float2 v) {
     if (kHalf) {
@@ -477,9 +406,7 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
         }
         if (level == 1) TL_MARK(23);
         if (kLinked) { ctaP = P; ctaM = M; }
-        if (kLocal && c.cta_sums == nullptr) {
-            // one CTA is the whole sequence
-        } else if (kLocal) {
+        if (kLocal) {
             c.cta_sums[lane] = P.x; c.cta_sums[kCs + lane] = P.y;
             if (kMom) { c.cta_sums[2 * kCs + lane] = M.x; c.cta_sums[3 * kCs + lane] = M.y; }
         } else {
@@ -511,8 +438,7 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
             }
         }
         if (kLinked) ctaS = S;
-        if (kLocal && c.cta_sums == nullptr) {
-        } else if (kLocal) {
+        if (kLocal) {
             c.cta_sums[RW::kF * kCs + lane] = S.x; c.cta_sums[(RW::kF + 1) * kCs + lane] = S.y;
         } else {
             float* st = c.stage + RW::kBlockF;
@@ -682,190 +608,11 @@ __device__ __forceinline__ void add_outside(Enter& e, const float* g, int rows, 
     e.S = Pair2{fma2(pS, row(rows - 2), e.S.n), fma2(pS, row(rows - 1), e.S.d)};
 }
 
-// ---- exact path: (value, exponent) records, any exponent range -----------------------------------
-struct Entering {
-    Acc4 left;    // state entering the sub-chunk at its first token (with first moments)
-    Acc2 right;   // state entering it at its last position
-};
-
-__device__ __forceinline__ void cluster_or_cta_sync(const Ctx& c) {
-    __syncwarp();
-    if (c.cluster > 1) {
-        cluster_arrive();
-        cluster_wait();
-    } else {
-        __syncthreads();
-    }
-}
-
-// One channel per thread and call: sub = index of the thread's 16-token sub-chunk in the CTA, ch = its
-// channel within the strip.  Two rounds (one per direction) over the same record area (the span
-// records and the area behind them); every thread walks the records it needs itself and reads the
-// other CTAs' aggregates out of their shared memory.  Slow and simple: this path only runs for
-// inputs outside the fast path's range.
-// kMom = false (forward): the first moments are not carried, a record is 3 rows in both rounds.
-template <bool kMom>
-__device__ __noinline__ Entering exact_exchange(const Ctx& c, int sub, int ch, float w, const Acc4 own_right, const Acc2 own_left) {
-    const int n_sub = 2 * c.n_warps;
-    constexpr int kRec = kMom ? 5 : 3;
-    float* area = c.sub;      // [n_sub][kRec][kCs], then [n_sub][3][kCs]
-    float* agg = c.cta;       // kRec rows
-    Entering out;
-    {
-        float* s = area + sub * kRec * kCs + ch;
-        s[0] = own_right.a; s[kCs] = own_right.b; s[(kRec - 1) * kCs] = own_right.o;
-        if (kMom) { s[2 * kCs] = own_right.ma; s[3 * kCs] = own_right.mb; }
-        __syncwarp();
-        __syncthreads();
-        Acc4 X = acc4_zero();
-        for (int j = 0; j < sub; ++j) {
-            const float* q = area + j * kRec * kCs + ch;
-            acc4_decay(X, w, static_cast<float>(kL));
-            X = acc4_merge(X, Acc4{q[0], q[kCs], kMom ? q[2 * kCs] : 0.f, kMom ? q[3 * kCs] : 0.f, q[(kRec - 1) * kCs]});
-        }
-        if (sub == n_sub - 1) {
-            Acc4 t = X;
-            acc4_decay(t, w, static_cast<float>(kL));
-            t = acc4_merge(t, own_right);
-            agg[ch] = t.a; agg[kCs + ch] = t.b; agg[(kRec - 1) * kCs + ch] = t.o;
-            if (kMom) { agg[2 * kCs + ch] = t.ma; agg[3 * kCs + ch] = t.mb; }
-        }
-        cluster_or_cta_sync(c);
-        Acc4 Y = acc4_zero();
-        for (int r = 0; r < c.rank; ++r) {
-            const uint32_t a = peer_addr(agg + ch, r);
-            acc4_decay(Y, w, static_cast<float>(c.n_tok));
-            Y = acc4_merge(Y, Acc4{ld_peer(a), ld_peer(a + kCs * 4), kMom ? ld_peer(a + 2 * kCs * 4) : 0.f,
-                                   kMom ? ld_peer(a + 3 * kCs * 4) : 0.f, ld_peer(a + (kRec - 1) * kCs * 4)});
-        }
-        acc4_decay(Y, w, static_cast<float>(kL * sub));
-        out.left = acc4_merge(Y, X);
-        cluster_or_cta_sync(c);
-    }
-    {
-        float* s = area + sub * 3 * kCs + ch;
-        s[0] = own_left.a; s[kCs] = own_left.b; s[2 * kCs] = own_left.o;
-        __syncwarp();
-        __syncthreads();
-        Acc2 Z = acc2_zero();
-        for (int j = n_sub - 1; j > sub; --j) {
-            const float* q = area + j * 3 * kCs + ch;
-            acc2_decay(Z, w, static_cast<float>(kL));
-            Z = acc2_merge(Z, Acc2{q[0], q[kCs], q[2 * kCs]});
-        }
-        if (sub == 0) {
-            Acc2 t = Z;
-            acc2_decay(t, w, static_cast<float>(kL));
-            t = acc2_merge(t, own_left);
-            agg[ch] = t.a; agg[kCs + ch] = t.b; agg[2 * kCs + ch] = t.o;
-        }
-        cluster_or_cta_sync(c);
-        Acc2 Y = acc2_zero();
-        for (int r = c.cluster - 1; r > c.rank; --r) {
-            const uint32_t a = peer_addr(agg + ch, r);
-            acc2_decay(Y, w, static_cast<float>(c.n_tok));
-            Y = acc2_merge(Y, Acc2{ld_peer(a), ld_peer(a + kCs * 4), ld_peer(a + 2 * kCs * 4)});
-        }
-        acc2_decay(Y, w, static_cast<float>(kL * (n_sub - 1 - sub)));
-        out.right = acc2_merge(Y, Z);
-        cluster_or_cta_sync(c);
-    }
-    return out;
-}
-
-// One channel of one thread's sub-chunk on the exact path: ks / vs / gs point at its first token
-// (stride kCs), n = valid tokens.  Sweeps are position-anchored (biwkv_math.cuh).  Forward: y into
-// ks.  Backward: gk into ks, gv into vs, the thread's gw / gu shares returned.
-template <bool kBwd>
-__device__ __noinline__ void exact_subchunk(const Ctx& c, int sub, int ch, float* ks, float* vs, float* gs, int n, float w,
-                                            float u, float& gw_out, float& gu_out) {
-    const float last = static_cast<float>(n - 1);
-    Acc4 right = acc4_zero();
-    Acc2 left = acc2_zero();
-    for (int i = 0; i < n; ++i) acc4_absorb(right, ks[i * kCs] + w * static_cast<float>(i), vs[i * kCs], 1.f);
-    for (int i = n - 1; i >= 0; --i) acc2_add(left, ks[i * kCs] - w * static_cast<float>(i), vs[i * kCs], 1.f);
-    // a short sub-chunk still spans kL positions for its right-hand neighbours
-    right.o -= w * static_cast<float>(n);
-    acc4_decay(right, w, static_cast<float>(kL - n));
-    left.o -= w;
-    const Entering e1 = exact_exchange<kBwd>(c, sub, ch, w, right, left);
-    const Acc4 P4 = e1.left;                         // anchored at token 0
-    Acc2 S = e1.right;
-    acc2_decay(S, w, static_cast<float>(kL - n));   // given at position kL-1; anchor it at token n-1
-    Acc2 stash[kL];
-    for (int i = n - 1; i >= 0; --i) {
-        const float d = last - static_cast<float>(i);
-        stash[i] = acc2_at(S, w, d);
-        acc2_add(S, ks[i * kCs] + w * d, vs[i * kCs], 1.f);
-    }
-    if (!kBwd) {
-        Acc2 P{P4.a, P4.b, P4.o};
-        for (int i = 0; i < n; ++i) {
-            const float k = ks[i * kCs], v = vs[i * kCs], d = static_cast<float>(i);
-            const TokenOut o = token_out(acc2_at(P, w, d), stash[i], k, v, u);
-            ks[i * kCs] = o.y;
-            acc2_add(P, k + w * d, v, 1.f);
-        }
-        return;
-    }
-    // backward: G e^{m}, H e^{m}, -m per token; gw from pairs (output later than input)
-    float gg[kL], hh[kL], xo[kL];
-    float gw = 0.f, gu = 0.f;
-    Acc4 PM = P4;   // prefix state with first moments
-    for (int i = 0; i < n; ++i) {
-        const float k = ks[i * kCs], v = vs[i * kCs], d = static_cast<float>(i);
-        const Acc2 Pi{PM.a, PM.b, PM.o - w * d};
-        const TokenOut o = token_out(Pi, stash[i], k, v, u);
-        gg[i] = gs[i * kCs] * o.inv_den;
-        hh[i] = gg[i] * o.y;
-        xo[i] = -o.m;
-        gw -= wkv_exp(Pi.o + xo[i]) * (gg[i] * PM.ma - hh[i] * PM.mb);
-        acc4_absorb(PM, k + w * d, v, 1.f);
-    }
-    Acc4 later = acc4_zero();
-    Acc2 earlier = acc2_zero();
-    for (int i = 0; i < n; ++i) acc4_absorb(later, xo[i] + w * static_cast<float>(i), gg[i], hh[i]);
-    for (int i = n - 1; i >= 0; --i) acc2_add(earlier, xo[i] - w * static_cast<float>(i), gg[i], hh[i]);
-    later.o -= w * static_cast<float>(n);
-    acc4_decay(later, w, static_cast<float>(kL - n));
-    earlier.o -= w;
-    const Entering e2 = exact_exchange<kBwd>(c, sub, ch, w, later, earlier);
-    Acc4 R = e2.left;                                // anchored at token 0
-    Acc2 Q = e2.right;
-    acc2_decay(Q, w, static_cast<float>(kL - n));   // anchored at token n-1
-    float pk[kL], pv[kL];
-    for (int i = n - 1; i >= 0; --i) {
-        const float d = last - static_cast<float>(i);
-        const float e = wkv_exp(ks[i * kCs] + Q.o - w * d);
-        pv[i] = e * Q.a;
-        pk[i] = e * (Q.a * vs[i * kCs] - Q.b);
-        acc2_add(Q, xo[i] + w * d, gg[i], hh[i]);
-    }
-    for (int i = 0; i < n; ++i) {
-        const float k = ks[i * kCs], v = vs[i * kCs], d = static_cast<float>(i);
-        const float e = wkv_exp(k + R.o - w * d);
-        const float es = wkv_exp(u + k + xo[i]);
-        const float self = es * (v * gg[i] - hh[i]);
-        vs[i * kCs] = pv[i] + e * R.a + es * gg[i];
-        ks[i * kCs] = pk[i] + e * (R.a * v - R.b) + self;
-        gu += self;
-        gw -= e * (R.ma * v - R.mb);
-        acc4_absorb(R, xo[i] + w * d, gg[i], hh[i]);
-    }
-    gw_out = gw;
-    gu_out = gu;
-}
-
 // ---- the kernel -----------------------------------------------------------------------------------
 // kStash: tokens whose leftward state a thread keeps in registers at a time (16: one reverse sweep
 // per sub-chunk; 8: the second half is swept twice, for half the registers).
 // kHalf: k, v, gy and the outputs are bfloat16 tensors (float32 arithmetic and shared-memory state all the same).
-// kWide (with kHalf): y and gy are float32 tensors, what a model with float32 w, u under autocast has; y still holds
-// bfloat16 values, and gy is rounded to bfloat16 as it is read: the results are those of the bfloat16 kernel.  Without it the caller widens y (6 bytes per element) and narrows gy (6 more) in
-// passes of their own, as many bytes as this kernel's own forward moves.  B=64, T=576, C=1024, forward + backward:
-// 468 us with those passes, 332 us without, 327 us now (three CTAs per sequence, and 4 us for gy's rounding); forward alone at B=256,
-// T=196, C=384: 103 and 53 us.
-template <bool kBwd, int kStash, bool kHalf, bool kWide, Mode kMode>
+template <bool kBwd, int kStash, bool kHalf, Mode kMode>
 __global__ void __launch_bounds__(kMaxThreads, kBwd ? 2 : 3)
 biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                       const __grid_constant__ CUtensorMap map_g,     // backward: gy
@@ -873,11 +620,8 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                       const __grid_constant__ CUtensorMap map_o1,    // backward: gv
                       const Params p) {
     using RW = Rows<kBwd, kMode>;
-    constexpr bool kHalfG = kHalf && !kWide;                    // gy arrives as bfloat16
-    constexpr bool kHalfOut = kHalf && (kBwd || !kWide);        // results leave as bfloat16
     constexpr bool kCluster = kUsesCluster<kMode>, kLinked = kMode == Mode::linked, kSums = kMode == Mode::sums || kMode == Mode::sums_keep;
-    constexpr bool kSingle = kMode == Mode::single;
-    constexpr bool kOwn1 = kCluster || kSingle || (kSums && !kBwd);        // level 1 is this launch's to sum up; else given
+    constexpr bool kOwn1 = kCluster || (kSums && !kBwd);        // level 1 is this launch's to sum up; else given
     constexpr bool kOwn2 = kBwd && kMode != Mode::spread;       // level 2 likewise
     constexpr bool kMom1 = RW::kF == 4;                         // level 1 carries first moments
     constexpr bool kResults = !kSums;                           // the launch writes results
@@ -946,20 +690,20 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         if (kHalf) {
             // bfloat16: one box per 16-token sub-chunk, into the upper half of the sub-chunk's own area
             sm100::mbar_expect_tx(full + warp, 4 * kHalfAreaBytes);
-            if (kBwd && kHalfG) sm100::mbar_expect_tx(gfull + warp, 2 * kHalfAreaBytes);
+            if (kBwd) sm100::mbar_expect_tx(gfull + warp, 2 * kHalfAreaBytes);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int r = warp * kSpan + h * kL;
                 sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_k + r * kCs) + kHalfAreaBytes, &map_k, full + warp, strip * kCs, tok0 + r, b);
                 sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_v + r * kCs) + kHalfAreaBytes, &map_v, full + warp, strip * kCs, tok0 + r, b);
-                if (kBwd && kHalfG) sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_g + r * kCs) + kHalfAreaBytes, &map_g, gfull + warp, strip * kCs, tok0 + r, b);
+                if (kBwd) sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_g + r * kCs) + kHalfAreaBytes, &map_g, gfull + warp, strip * kCs, tok0 + r, b);
             }
         } else {
             sm100::mbar_expect_tx(full + warp, 2 * kSpanBytes);
             sm100::tma_load_3d(slot_k + warp * kSpan * kCs, &map_k, full + warp, strip * kCs, tok0 + warp * kSpan, b);
             sm100::tma_load_3d(slot_v + warp * kSpan * kCs, &map_v, full + warp, strip * kCs, tok0 + warp * kSpan, b);
         }
-        if (kBwd && !kHalfG) {
+        if (kBwd && !kHalf) {
             sm100::mbar_expect_tx(gfull + warp, kSpanBytes);
             sm100::tma_load_3d(slot_g + warp * kSpan * kCs, &map_g, gfull + warp, strip * kCs, tok0 + warp * kSpan, b);
         }
@@ -1086,7 +830,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         const float Tf = static_cast<float>(p.T);
         unsafe = (2.f * kmax.x + fabsf(u2.x) + fabsf(w2.x) + fmaxf(-w2.x, 0.f) * Tf > kSafeRange) ||
                  (2.f * kmax.y + fabsf(u2.y) + fabsf(w2.y) + fmaxf(-w2.y, 0.f) * Tf > kSafeRange);
-        e1 = fast_exchange<RW, kSums || kSingle, kLinked>(c, 0, F, MF, R, unsafe TL_PASS);
+        e1 = fast_exchange<RW, kSums, kLinked>(c, 0, F, MF, R, unsafe TL_PASS);
     } else {
         add_outside<kBwd && !kSums>(e1, c.cta + 2 * pr, p.state_rows, wl2, dP, dS);
     }
@@ -1100,15 +844,9 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     float2 gw = f2(0.f, 0.f), gu = f2(0.f, 0.f);
     if (kBwd && !sm100::mbar_wait(gfull + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
     if (unsafe) {
-        // the whole cluster takes this branch together: the unit is left to the exact kernel, which
-        // runs right after this one (nothing of this CTA is in flight any more: its tiles have
-        // landed and everything the other CTAs sent has been waited for)
-        // (a sequence of several clusters is not the exact kernel's to redo: the count alone switches on the chunked kernels, which
-        // redo the whole call; without clusters the word that was read does)
-        if ((kCluster || kSingle) && cta == 0 && threadIdx.x == 0) {
-            const unsigned at = atomicAdd(p.redo_count, 1u);
-            if (!kLinked) p.redo_list[at] = unit;
-        }
+        // the whole cluster takes this branch together; the count switches on the chunked kernels that stand by, which redo the whole
+        // call (without clusters the word that was read does)
+        if (kCluster && cta == 0 && threadIdx.x == 0) atomicAdd(p.redo_count, 1u);
         return;
     }
     if (!kBwd) {
@@ -1137,7 +875,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                     const float2 nn = fma2(c2, zx, add2(P.n, sn[g + j]));
                     const float2 dd = fma2(c2, zy, add2(P.d, sd[g + j]));
                     const float2 y = mul2(nn, f2(rcp(dd.x), rcp(dd.y)));
-                    st_out<kHalfOut>(area_k, i, pr, kHalf && kWide ? round2(y) : y);
+                    st_out<kHalf>(area_k, i, pr, y);
                     P.n = fma2(lam2, P.n, zx);
                     P.d = fma2(lam2, P.d, zy);
                 }
@@ -1172,8 +910,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 #pragma unroll
                     for (int j = 0; j < kGroupB; ++j) {
                         const int i = blk * kStash + g + j;
-                        zxs[j] = k2[i * kRow]; zys[j] = v2[i * kRow]; gys[j] = ld_in<kHalfG>(area_g, i, pr);
-                        if (kHalf && kWide) gys[j] = round2(gys[j]);
+                        zxs[j] = k2[i * kRow]; zys[j] = v2[i * kRow]; gys[j] = ld_in<kHalf>(area_g, i, pr);
                     }
                     if (kHalf) __syncwarp();
 #pragma unroll
@@ -1219,7 +956,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         bool ignored = false;
         TL_MARK(5);
         if (kCluster && p.cluster > 1) cluster_wait();
-        if (kOwn2) e2 = fast_exchange<RW, kSums || kSingle, kLinked>(c, 1, rr, mr, q, ignored TL_PASS);
+        if (kOwn2) e2 = fast_exchange<RW, kSums, kLinked>(c, 1, rr, mr, q, ignored TL_PASS);
         else add_outside<true>(e2, c.sub + 2 * pr, kStateRows, wl2, dP, dS);
         if (kSums) {
             put_state(p.states2 + sub_at, kStateRows, e2, true);
@@ -1281,7 +1018,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     }
     sm100::fence_proxy_async_smem();
     __syncthreads();
-    if (kHalfOut) {
+    if (kHalf) {
         // one box per sub-chunk (its 16 dense bfloat16 rows), issued by the warp that wrote them
         if (lane == 0) {
 #pragma unroll
@@ -1307,155 +1044,8 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         }
     }
     TL_MARK(8);
-    if (kHalfOut ? lane == 0 : threadIdx.x == 0) sm100::tma_store_wait_read();   // shared memory may go once the stores have read it
+    if (kHalf ? lane == 0 : threadIdx.x == 0) sm100::tma_store_wait_read();   // shared memory may go once the stores have read it
     TL_MARK(9);
-}
-
-// ---- the exact kernel ----------------------------------------------------------------------------
-// Runs after the fast kernel with a small persistent grid of clusters and serves the units it left
-// behind (normally none: one load and out).  Same shared-memory layout, same tiles, same work split
-// between the CTAs of a cluster, per-token max-shifted arithmetic.
-template <bool kBwd, bool kHalf, bool kWide>
-__global__ void __launch_bounds__(kMaxThreads, 1)
-biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                   const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_o0,
-                   const __grid_constant__ CUtensorMap map_o1, const Params p) {
-    using RW = Rows<kBwd>;
-    constexpr bool kHalfG = kHalf && !kWide;                    // as in biwkv_resident_kernel
-    constexpr bool kHalfOut = kHalf && (kBwd || !kWide);
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pr = lane & 15, upper = lane >> 4;
-    const int nw = p.n_warps;
-    const int slot_floats = p.n_tok * kCs;
-    float* slot_k = reinterpret_cast<float*>(smem_raw);
-    float* slot_v = slot_k + slot_floats;
-    float* slot_g = slot_v + slot_floats;
-    Ctx c;
-    c.sub = slot_k + RW::kSlots * slot_floats;
-    c.peers = c.sub + nw * (RW::kSub * kCs);
-    c.stage = c.peers + RW::kPeerFloats;
-    c.cta = c.stage + RW::kBlockF + RW::kBlockR;
-    c.consts = c.cta + RW::kSub * kCs;
-    uint64_t* full = reinterpret_cast<uint64_t*>(c.consts + kConstRows * kCs);
-    c.xbar = full + 1;
-    c.flag = reinterpret_cast<unsigned*>(full + 4);
-    c.status = p.status;
-    c.mirror = p.mirror;
-    c.spin_limit = kSpinLimit;
-    c.withhold = false;
-    c.seg = 0; c.segs = 1; c.unit = 0; c.xseg = nullptr; c.xflag = nullptr;
-    c.warp = warp; c.lane = lane; c.n_warps = nw; c.n_tok = p.n_tok; c.cluster = p.cluster;
-    c.rank = p.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
-
-    const unsigned n_redo = *reinterpret_cast<volatile unsigned*>(p.redo_count);
-    const int n_clusters = static_cast<int>(gridDim.x) / p.cluster, mine = static_cast<int>(blockIdx.x) / p.cluster;
-    if (static_cast<unsigned>(mine) >= n_redo) return;       // the same for every CTA of a cluster
-    if (threadIdx.x == 0) {
-        sm100::mbar_init(full, 1);
-        sm100::mbar_init_fence();
-    }
-    __syncthreads();
-    const int tok0 = c.rank * p.n_tok;
-    const uint32_t slot_bytes = static_cast<uint32_t>(slot_floats) * 4u;
-    const int row0 = warp * kSpan + upper * kL;
-    const int n = max(0, min(kL, p.T - (tok0 + row0)));
-    float* ks = slot_k + row0 * kCs + 2 * pr;
-    float* vs = slot_v + row0 * kCs + 2 * pr;
-    float* gs = slot_g + row0 * kCs + 2 * pr;
-    uint32_t phase = 0;
-    for (unsigned j = mine; j < n_redo; j += n_clusters) {
-        const int unit = p.redo_list[j];
-        const int b = unit / p.n_strips, strip = unit - b * p.n_strips;
-        if (threadIdx.x == 0) {
-            sm100::mbar_expect_tx(full, 2 * (kHalf ? slot_bytes / 2 : slot_bytes) + (kBwd ? (kHalfG ? slot_bytes / 2 : slot_bytes) : 0));
-            if (kHalf) {
-                for (int r = 0; r < nw * kSpan; r += kL) {   // one box per 16-token sub-chunk, into the upper half of its area
-                    sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_k + r * kCs) + kHalfAreaBytes, &map_k, full, strip * kCs, tok0 + r, b);
-                    sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_v + r * kCs) + kHalfAreaBytes, &map_v, full, strip * kCs, tok0 + r, b);
-                    if (kBwd && kHalfG) sm100::tma_load_3d(reinterpret_cast<unsigned char*>(slot_g + r * kCs) + kHalfAreaBytes, &map_g, full, strip * kCs, tok0 + r, b);
-                }
-            } else {
-                for (int sp = 0; sp < nw; ++sp) {            // the load maps describe one span per box
-                    sm100::tma_load_3d(slot_k + sp * kSpan * kCs, &map_k, full, strip * kCs, tok0 + sp * kSpan, b);
-                    sm100::tma_load_3d(slot_v + sp * kSpan * kCs, &map_v, full, strip * kCs, tok0 + sp * kSpan, b);
-                }
-            }
-            if (kBwd && !kHalfG)
-                for (int sp = 0; sp < nw; ++sp)
-                    sm100::tma_load_3d(slot_g + sp * kSpan * kCs, &map_g, full, strip * kCs, tok0 + sp * kSpan, b);
-        }
-        const int ch0 = strip * kCs + 2 * pr;
-        const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
-        const float2 u2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.u + ch0) : f2(0.f, 0.f);
-        if (!sm100::mbar_wait(full, phase, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
-        phase ^= 1u;
-        if (kHalf) {
-            // widen this thread's 16 rows in place, walking up (see ld_in)
-            for (int i = 0; i < kL; ++i) {
-                const float2 a = ld_in<true>(slot_k + row0 * kCs, i, pr), bb = ld_in<true>(slot_v + row0 * kCs, i, pr);
-                const float2 g_ = kBwd && kHalfG ? ld_in<true>(slot_g + row0 * kCs, i, pr) : f2(0.f, 0.f);
-                __syncwarp();
-                *reinterpret_cast<float2*>(ks + i * kCs) = a;
-                *reinterpret_cast<float2*>(vs + i * kCs) = bb;
-                if (kBwd && kHalfG) *reinterpret_cast<float2*>(gs + i * kCs) = g_;
-                if (kBwd && kWide) *reinterpret_cast<float2*>(gs + i * kCs) = round2(*reinterpret_cast<const float2*>(gs + i * kCs));
-                __syncwarp();
-            }
-        }
-        float2 gw = f2(0.f, 0.f), gu = f2(0.f, 0.f);
-        const int sub = 2 * warp + upper;
-        exact_subchunk<kBwd>(c, sub, 2 * pr, ks, vs, gs, n, w2.x, u2.x, gw.x, gu.x);
-        exact_subchunk<kBwd>(c, sub, 2 * pr + 1, ks + 1, vs + 1, gs + 1, n, w2.y, u2.y, gw.y, gu.y);
-        if (kBwd) {
-            *reinterpret_cast<float2*>(gs) = gw;
-            *reinterpret_cast<float2*>(gs + kCs) = gu;
-        }
-        if (kHalf && kWide && !kBwd)
-            for (int i = 0; i < kL; ++i) {
-                float2* row = reinterpret_cast<float2*>(ks + i * kCs);
-                *row = round2(*row);
-            }
-        if (kHalfOut) {
-            // narrow the results in place, walking up: dense bfloat16 rows at the start of the area
-            __syncwarp();
-            for (int i = 0; i < kL; ++i) {
-                const float2 a = *reinterpret_cast<const float2*>(ks + i * kCs);
-                const float2 bb = kBwd ? *reinterpret_cast<const float2*>(vs + i * kCs) : f2(0.f, 0.f);
-                __syncwarp();
-                st_out<true>(slot_k + row0 * kCs, i, pr, a);
-                if (kBwd) st_out<true>(slot_v + row0 * kCs, i, pr, bb);
-                __syncwarp();
-            }
-        }
-        sm100::fence_proxy_async_smem();
-        __syncthreads();
-        if (kHalfOut) {
-            if (lane == 0) {
-                for (int h = 0; h < 2; ++h) {
-                    const int r = warp * kSpan + h * kL;
-                    if (tok0 + r < p.T) {
-                        sm100::tma_store_3d(&map_o0, slot_k + r * kCs, strip * kCs, tok0 + r, b);
-                        if (kBwd) sm100::tma_store_3d(&map_o1, slot_v + r * kCs, strip * kCs, tok0 + r, b);
-                    }
-                }
-                sm100::tma_store_commit();
-            }
-        } else if (threadIdx.x == 0) {
-            sm100::tma_store_3d(&map_o0, slot_k, strip * kCs, tok0, b);
-            if (kBwd) sm100::tma_store_3d(&map_o1, slot_v, strip * kCs, tok0, b);
-            sm100::tma_store_commit();
-        }
-        if (kBwd && warp < 2) {
-            for (int jj = warp; jj < 2; jj += min(nw, 2)) {
-                float acc = 0.f;
-                for (int s = 0; s < 2 * nw; ++s) acc += slot_g[(s * kL + jj) * kCs + lane];
-                p.partial[((static_cast<size_t>(unit) * p.cluster + c.rank) * 2 + jj) * kCs + lane] = acc;
-            }
-        }
-        if (kHalfOut ? lane == 0 : threadIdx.x == 0) sm100::tma_store_wait_read();
-        __syncthreads();      // the slots are free for the next unit
-    }
 }
 
 // out[j][c] = sum over sequences and cluster ranks of partial[cta][j][c % 32], fixed order
@@ -1543,21 +1133,12 @@ void set_withhold_test(bool on) { g_withhold.store(on); }
 
 struct Plan {
     int cluster = 0, segs = 1, n_warps = 0, n_tok = 0, ctas = 0;
-    bool split = false;      // longer than one cluster holds, in separate launches
+    bool split = false;      // in separate launches
 };
 
 // How many CTAs hold a sequence, and in how many clusters.
 //
-// One CTA (T <= 256, Mode::single): nothing to hand over or to wait for, and no room for what others send; the kernel without the
-// cluster steps took 51.5 for 53.3 us at B=256, T=196, C=384 (bfloat16, forward).
-//
-// One cluster (T <= 4096): as few CTAs as hold T, 256 tokens each, then only as many warps as the tokens need.  A CTA's life
-// is a chain whose length hardly depends on its tokens, so the fewest CTAs win, whether their number is a power of two or
-// not (forward / backward us at 131072 tokens, C=768): T=1500 6 CTAs 220 / 544, 8 CTAs 266 / 652; T=3000 12 CTAs 249 / 592,
-// 16 CTAs 301 / 756.  (Powers of two also left CTAs without tokens at T=2049..2400, 2561..2880 and the like, which the
-// tile kernels then served: T=3136 588 / 1453 against 258 / 689.)  Between 3 and 4 CTAs the smaller padding decides, because
-// 3 CTAs of 7 warps share an SM worse than 4 of 5: T=600 244 / 607 against 230 / 565, but T=520 (3 of 6) 257 / 634 against
-// 257 / 652.
+// Up to 4096 tokens: not here (biwkv_strips.cu).
 //
 // Above, separate launches (see biwkv_chain_kernel) from kSplitCtas CTAs of 256 tokens on.  Below that one launch of linked
 // clusters is as fast or faster, being fewer launches (forward / backward us, float32): B=1, C=192, T=8192 (192 CTAs) linked 25 /
@@ -1574,42 +1155,33 @@ static bool make_plan(int B, int T, int C, Plan& pl) {
     constexpr int kCtaMax = kMaxWarps * kSpan;              // tokens one CTA holds
     constexpr int kSegMax = kMaxCluster * kCtaMax;          // tokens one cluster holds
     const auto up = [](int a, int b) { return (a + b - 1) / b; };
-    const auto warps = [&](int ctas) { return up(up(T, ctas), kSpan); };
-    pl.segs = T <= kSegMax ? 1 : std::max(up(T, kSegMax), std::min(kMaxSegs, (T + 1024) / 2048));
+    if (T <= kSegMax) return false;
+    pl.segs = std::max(up(T, kSegMax), std::min(kMaxSegs, (T + 1024) / 2048));
     if (pl.segs > kMaxSegs) return false;
-    pl.split = pl.segs > 1 && static_cast<long long>(B) * up(C, kCs) * up(T, kCtaMax) >= kSplitCtas;
+    pl.split = static_cast<long long>(B) * up(C, kCs) * up(T, kCtaMax) >= kSplitCtas;
     if (pl.split) {
         pl.segs = pl.cluster = 1;
         pl.ctas = up(T, kCtaMax);
     } else {
         pl.cluster = up(up(T, pl.segs), kCtaMax);
-        if (pl.segs == 1 && pl.cluster == 3 && 4 * warps(4) < 3 * warps(3)) pl.cluster = 4;
         pl.ctas = pl.segs * pl.cluster;
     }
-    pl.n_warps = warps(pl.ctas);
+    pl.n_warps = up(up(T, pl.ctas), kSpan);
     pl.n_tok = pl.n_warps * kSpan;
     // every CTA owns a token, or at least every segment
-    return static_cast<long long>(pl.segs == 1 ? pl.ctas - 1 : (pl.segs - 1) * pl.cluster) * pl.n_tok < T;
+    return static_cast<long long>(pl.split ? pl.ctas - 1 : (pl.segs - 1) * pl.cluster) * pl.n_tok < T;
 }
 
 struct DeviceState {
     bool probed = false, ok = false;
-    // [linked][tensor types][bwd][cluster][n_warps]: 0 unknown, 1 launchable, -1 not
-    signed char fits[2][3][2][kMaxCluster + 1][kMaxWarps + 1] = {};
+    // [tensor types][bwd][cluster][n_warps]: 0 unknown, 1 launchable, -1 not
+    signed char fits[2][2][kMaxCluster + 1][kMaxWarps + 1] = {};
 };
 static std::mutex g_mutex;
 static DeviceState g_dev[64];
 
-// kWide kernels exist for sequences of one cluster (the chunked kernels that stand by behind longer ones have no such form)
 template <bool kBwd, Types kTypes, Mode kMode>
-static auto kernel() {
-    constexpr bool kWide = kTypes == Types::wide && (kMode == Mode::whole || kMode == Mode::single);
-    return biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kTypes != Types::f32, kWide, kMode>;
-}
-template <bool kBwd, Types kTypes>
-static auto exact_kernel() {
-    return biwkv_exact_kernel<kBwd, kTypes != Types::f32, kTypes == Types::wide>;
-}
+static auto kernel() { return biwkv_resident_kernel<kBwd, kBwd ? kBwdStash : kFwdStash, kTypes != Types::f32, kMode>; }
 template <typename F>
 static bool allow(F* fn, size_t smem, bool cluster) {
     const void* f = reinterpret_cast<const void*>(fn);
@@ -1620,12 +1192,8 @@ template <bool kBwd, Types kTypes, Mode kMode>
 static bool allow_kernel() { return allow(kernel<kBwd, kTypes, kMode>(), smem_bytes<kBwd, kMode>(kMaxWarps), kUsesCluster<kMode>); }
 template <bool kBwd, Types kTypes>
 static bool allow_types() {
-    bool good = allow_kernel<kBwd, kTypes, Mode::single>() && allow_kernel<kBwd, kTypes, Mode::whole>() && allow(exact_kernel<kBwd, kTypes>(), smem_bytes<kBwd>(kMaxWarps), true);
-    if constexpr (kTypes != Types::wide) {
-        good = good && allow_kernel<kBwd, kTypes, Mode::linked>() && allow_kernel<kBwd, kTypes, Mode::sums>() && allow_kernel<kBwd, kTypes, Mode::spread>();
-        good = good && allow_kernel<false, kTypes, Mode::sums_keep>();
-    }
-    return good;
+    return allow_kernel<kBwd, kTypes, Mode::linked>() && allow_kernel<kBwd, kTypes, Mode::sums>() && allow_kernel<kBwd, kTypes, Mode::spread>() &&
+           allow_kernel<false, kTypes, Mode::sums_keep>();
 }
 
 template <bool kBwd, Types kTypes>
@@ -1639,12 +1207,11 @@ static bool fits(const Plan& pl) {
         int cl = 0;
         cudaDeviceGetAttribute(&cl, cudaDevAttrClusterLaunch, dev);
         d.ok = cl != 0 && tensor_map::encode_fn() != nullptr && allow_types<false, Types::f32>() && allow_types<false, Types::bf16>() &&
-               allow_types<false, Types::wide>() && allow_types<true, Types::f32>() && allow_types<true, Types::bf16>() &&
-               allow_types<true, Types::wide>();
+               allow_types<true, Types::f32>() && allow_types<true, Types::bf16>();
         if (!d.ok) cudaGetLastError();
     }
     if (!d.ok || pl.split) return d.ok;
-    signed char& slot = d.fits[pl.segs > 1 ? 1 : 0][static_cast<int>(kTypes)][kBwd ? 1 : 0][pl.cluster][pl.n_warps];
+    signed char& slot = d.fits[static_cast<int>(kTypes)][kBwd ? 1 : 0][pl.cluster][pl.n_warps];
     if (slot == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(pl.cluster);
@@ -1655,8 +1222,7 @@ static bool fits(const Plan& pl) {
         at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
         int n = 0;
-        const cudaError_t err = cudaOccupancyMaxActiveClusters(
-            &n, pl.segs > 1 ? reinterpret_cast<const void*>(kernel<kBwd, kTypes, Mode::linked>()) : reinterpret_cast<const void*>(kernel<kBwd, kTypes, Mode::whole>()), &cfg);
+        const cudaError_t err = cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(kernel<kBwd, kTypes, Mode::linked>()), &cfg);
         if (err != cudaSuccess) cudaGetLastError();
         slot = (err == cudaSuccess && n > 0) ? 1 : -1;
     }
@@ -1671,7 +1237,7 @@ bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool
     if (!make_plan(B, T, C, pl)) return false;
     const long long ctas = static_cast<long long>(B) * ((C + kCs - 1) / kCs) * pl.ctas;
     if (ctas > (1LL << 30)) return false;
-    if (types == Types::wide) return pl.segs == 1 && !pl.split && (bwd ? fits<true, Types::wide>(pl) : fits<false, Types::wide>(pl));
+    if (types == Types::wide) return false;      // the kernels that stand by have no such form
     if (types == Types::bf16) return bwd ? fits<true, Types::bf16>(pl) : fits<false, Types::bf16>(pl);
     return bwd ? fits<true, Types::f32>(pl) : fits<false, Types::f32>(pl);
 }
@@ -1696,17 +1262,15 @@ static size_t units_of(int B, int C) { return static_cast<size_t>(B) * ((C + kCs
 // last not where they are kept)
 constexpr size_t kStatusBytes = 256;
 struct Carve {
-    size_t off_flags, off_stand_by, cleared, off_list, off_partial, off_vectors, off_records, off_states2, off_states1, total;
+    size_t off_flags, off_stand_by, cleared, off_partial, off_vectors, off_records, off_states2, off_states1, total;
 };
 static Carve carve(int B, int T, int C, const Plan& pl, bool bwd) {
     const size_t units = units_of(B, C), recs = pl.segs > 1 ? units * pl.segs * 4 : 0;
-    const bool longer = pl.split || pl.segs > 1;
     Carve cv;
     cv.off_flags = kStatusBytes;
     cv.off_stand_by = cv.off_flags + align_up(recs * sizeof(unsigned), 256);
-    cv.cleared = cv.off_stand_by + (longer ? fused::cleared_bytes(B, T, C, bwd) : 0);
-    cv.off_list = cv.off_stand_by + (longer ? align_up(fused::workspace_bytes(B, T, C, bwd), 256) : 0);
-    cv.off_partial = cv.off_list + align_up(units * sizeof(int), 256);
+    cv.cleared = cv.off_stand_by + fused::cleared_bytes(B, T, C, bwd);
+    cv.off_partial = cv.off_stand_by + align_up(fused::workspace_bytes(B, T, C, bwd), 256);
     cv.off_vectors = cv.off_partial + (bwd ? align_up(units * pl.ctas * 2 * kCs * sizeof(float), 256) : 0);
     cv.off_records = cv.off_vectors + align_up(2 * static_cast<size_t>(C) * sizeof(float), 256);
     cv.off_states2 = cv.off_records + align_up(recs * kSegRec * sizeof(float), 256);
@@ -1726,18 +1290,6 @@ size_t kept_bytes(int B, int T, int C) {
     Plan pl;
     if (!make_plan(B, T, C, pl) || !pl.split) return 0;
     return carve_states(units_of(B, C), pl, kStateRows).total;
-}
-
-bool stands_by(int B, int T, int C) {
-    Plan pl;
-    return make_plan(B, T, C, pl) && (pl.split || pl.segs > 1);
-}
-// The kernels read w and u in pairs.  A vector that starts at an odd float (cut out of a parameter buffer) goes through a copy:
-// single loads in the kernels cost every call, up to 7 % where a sequence is long.
-static const float* paired(const float* x, int C, float* copy, cudaStream_t stream) {
-    if ((reinterpret_cast<uintptr_t>(x) & 7u) == 0) return x;
-    cudaMemcpyAsync(copy, x, static_cast<size_t>(C) * sizeof(float), cudaMemcpyDeviceToDevice, stream);
-    return copy;
 }
 
 struct Maps {
@@ -1764,8 +1316,7 @@ static bool run(const Params& p, const Maps& m, size_t grid, cudaStream_t stream
 template <bool kBwd, Types kTypes>
 static int launch(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy,
                   void* o0, void* o1, float* gwgu, void* workspace, void* kept, cudaStream_t stream) {
-    constexpr bool kHalf = kTypes != Types::f32, kWide = kTypes == Types::wide;
-    constexpr bool kHalfOut = kHalf && (kBwd || !kWide), kHalfG = kHalf && !kWide;
+    constexpr bool kHalf = kTypes != Types::f32;
     Plan pl;
     if (!make_plan(B, T, C, pl)) return -1;
     Params p{};
@@ -1778,7 +1329,6 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     const size_t units = units_of(B, C), grid = units * pl.ctas;
     const Carve cv = carve(B, T, C, pl, kBwd);
     p.redo_count = reinterpret_cast<unsigned*>(ws) + 1;
-    p.redo_list = reinterpret_cast<int*>(ws + cv.off_list);
     p.segs = pl.segs;
     p.xflag = reinterpret_cast<unsigned*>(ws + cv.off_flags);
     p.xseg = reinterpret_cast<float*>(ws + cv.off_records);
@@ -1789,7 +1339,7 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     p.spin_limit = g_withhold.load() ? (1u << 10) : kSpinLimit;
     p.withhold_rank = g_withhold.load() ? 1 : -1;
     p.state_rows = kBwd || kept ? kStateRows : kPlainRows;
-    if (pl.split || pl.segs > 1) p.out_of_range = p.redo_count;
+    p.out_of_range = p.redo_count;
     if (pl.split) {
         unsigned char* base = kept ? static_cast<unsigned char*>(kept) : ws + cv.off_states1;
         StatesCarve sc = carve_states(units, pl, p.state_rows);
@@ -1805,11 +1355,11 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     tensor_map::bind_primary_context();   // the tensor-map encoder is a driver call
     Maps m;
     // float32: loads one box per 32-token span, stores one box per CTA; bfloat16: one box per 16-token sub-chunk both ways
-    const int box_in = kHalf ? kL : kSpan, box_g = kHalfG ? kL : kSpan, box_out = kHalfOut ? kL : pl.n_tok;
+    const int box_in = kHalf ? kL : kSpan, box_g = kHalf ? kL : kSpan, box_out = kHalf ? kL : pl.n_tok;
     bool ok = tensor_map::make_btc(&m.k, k, B, T, C, kCs, box_in, kHalf) && tensor_map::make_btc(&m.v, v, B, T, C, kCs, box_in, kHalf) &&
-              tensor_map::make_btc(&m.o0, o0, B, T, C, kCs, box_out, kHalfOut);
+              tensor_map::make_btc(&m.o0, o0, B, T, C, kCs, box_out, kHalf);
     if (kBwd) {
-        ok = ok && tensor_map::make_btc(&m.g, gy, B, T, C, kCs, box_g, kHalfG) && tensor_map::make_btc(&m.o1, o1, B, T, C, kCs, box_out, kHalfOut);
+        ok = ok && tensor_map::make_btc(&m.g, gy, B, T, C, kCs, box_g, kHalf) && tensor_map::make_btc(&m.o1, o1, B, T, C, kCs, box_out, kHalf);
     } else {
         m.g = m.k;       // not used
         m.o1 = m.o0;
@@ -1821,10 +1371,7 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
     cudaMemsetAsync(ws, 0, cv.cleared, stream);
     int launched = 0;
     bool done = true;
-    if constexpr (kTypes == Types::wide) {
-        if (pl.split || pl.segs > 1) return -1;
-        done = pl.ctas == 1 ? run<kBwd, kTypes, Mode::single>(p, m, grid, stream) : run<kBwd, kTypes, Mode::whole>(p, m, grid, stream);
-    } else if (pl.split) {
+    if (pl.split) {
         unsigned* const kept_seen = !kBwd && kept ? static_cast<unsigned*>(kept) : nullptr;
         const auto chain = [&](float* sums, int rows) {
             biwkv_chain_kernel<<<static_cast<unsigned>(units), 128, 0, stream>>>(sums, p.w, p.n_strips, pl.ctas, pl.n_tok, rows, C, p.out_of_range, kept_seen);
@@ -1841,66 +1388,38 @@ static int launch(int B, int T, int C, const float* w, const float* u, const voi
         }
         p.reverse = true;
         done = done && run<kBwd, kTypes, Mode::spread>(p, m, grid, stream);
-    } else if (pl.segs > 1) {
-        done = run<kBwd, kTypes, Mode::linked>(p, m, grid, stream);
-    } else if (pl.ctas == 1) {
-        done = run<kBwd, kTypes, Mode::single>(p, m, grid, stream);
     } else {
-        done = run<kBwd, kTypes, Mode::whole>(p, m, grid, stream);
+        done = run<kBwd, kTypes, Mode::linked>(p, m, grid, stream);
     }
     if (!done) return -1;
     ++launched;
-    if (!pl.split && pl.segs == 1) {
-        // the exact kernel: a few clusters that serve whatever the fast kernel left behind
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(std::min<size_t>(units, 16)) * pl.cluster);
-        cfg.blockDim = dim3(pl.n_warps * 32);
-        cfg.dynamicSmemBytes = smem_bytes<kBwd>(pl.n_warps);
-        cfg.stream = stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-        cfg.attrs = at; cfg.numAttrs = 1;
-        const cudaError_t err = cudaLaunchKernelEx(&cfg, exact_kernel<kBwd, kTypes>(), m.k, m.v, m.g, m.o0, m.o1, p);
-        if (err != cudaSuccess) {
-            set_error_detail(cudaGetErrorName(err));
-            return -1;
-        }
-        ++launched;
-    }
     if (kBwd) {
         reduce_partials<<<dim3(p.n_strips, 2), dim3(32, 32), 0, stream>>>(p, gwgu);
         ++launched;
     }
-    if constexpr (kTypes != Types::wide) {
-        if (pl.split || pl.segs > 1) {
-            void* const stand_by = ws + cv.off_stand_by;
-            int n;
-            if constexpr (kTypes == Types::bf16) {
-                n = kBwd ? fused::backward_bf16(B, T, C, w, u, k, v, gy, gwgu, o0, o1, stand_by, stream, p.out_of_range)
-                         : fused::forward_bf16(B, T, C, w, u, k, v, o0, stand_by, stream, p.out_of_range);
-            } else {
-                const auto in = [](const void* x) { return static_cast<const float*>(x); };
-                const auto out = [](void* x) { return static_cast<float*>(x); };
-                n = kBwd ? fused::backward(B, T, C, w, u, in(k), in(v), in(gy), gwgu, out(o0), out(o1), stand_by, stream, p.out_of_range)
-                         : fused::forward(B, T, C, w, u, in(k), in(v), out(o0), stand_by, stream, p.out_of_range);
-            }
-            if (n < 0) return n;
-            launched += n;
-        }
+    void* const stand_by = ws + cv.off_stand_by;
+    int n;
+    if constexpr (kHalf) {
+        n = kBwd ? fused::backward_bf16(B, T, C, w, u, k, v, gy, gwgu, o0, o1, stand_by, stream, p.out_of_range)
+                 : fused::forward_bf16(B, T, C, w, u, k, v, o0, stand_by, stream, p.out_of_range);
+    } else {
+        const auto in = [](const void* x) { return static_cast<const float*>(x); };
+        const auto out = [](void* x) { return static_cast<float*>(x); };
+        n = kBwd ? fused::backward(B, T, C, w, u, in(k), in(v), in(gy), gwgu, out(o0), out(o1), stand_by, stream, p.out_of_range)
+                 : fused::forward(B, T, C, w, u, in(k), in(v), out(o0), stand_by, stream, p.out_of_range);
     }
-    return launched;
+    return n < 0 ? n : launched + n;
 }
 
 int forward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, Types types,
             void* workspace, cudaStream_t stream, void* keep) {
-    const auto fn = types == Types::f32 ? launch<false, Types::f32> : types == Types::bf16 ? launch<false, Types::bf16> : launch<false, Types::wide>;
+    const auto fn = types == Types::f32 ? launch<false, Types::f32> : launch<false, Types::bf16>;
     return fn(B, T, C, w, u, k, v, nullptr, y, nullptr, nullptr, workspace, keep, stream);
 }
 
 int backward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, float* gwgu,
              void* gk, void* gv, Types types, void* workspace, cudaStream_t stream, const void* kept) {
-    const auto fn = types == Types::f32 ? launch<true, Types::f32> : types == Types::bf16 ? launch<true, Types::bf16> : launch<true, Types::wide>;
+    const auto fn = types == Types::f32 ? launch<true, Types::f32> : launch<true, Types::bf16>;
     return fn(B, T, C, w, u, k, v, gy, gk, gv, gwgu, workspace, const_cast<void*>(kept), stream);
 }
 

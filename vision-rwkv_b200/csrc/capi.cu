@@ -83,6 +83,7 @@ unsigned long long vrwkv_launch_count(void) { return g_launches.load(std::memory
 int vrwkv_set_path(int path) {
     if (path < 0 || path > 3) return VRWKV_ERR_SHAPE;
     biwkv::resident::set_withhold_test(path == 3);
+    biwkv::strips::set_withhold_test(path == 3);
     g_path.store(path == 3 ? 0 : path);
     return VRWKV_OK;
 }
@@ -131,16 +132,19 @@ unsigned vrwkv_take_failures(int device) {
     return bits;
 }
 
-// Whether the resident kernels serve the call, with what stands by behind them.
+// Whether the narrow-strip kernels serve the call.
+static bool strips_serve(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types) {
+    return g_path.load() == 0 && biwkv::strips::eligible(B, T, C, ptrs, bwd, types);
+}
+// Whether the kernels for long sequences serve the call, with what stands by behind them.
 static bool resident_serves(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types) {
-    return g_path.load() == 0 && biwkv::resident::eligible(B, T, C, ptrs, bwd, types) &&
-           (!biwkv::resident::stands_by(B, T, C) || biwkv::fused::eligible(B, T, C, ptrs, types == Types::bf16));
+    return g_path.load() == 0 && biwkv::resident::eligible(B, T, C, ptrs, bwd, types) && biwkv::fused::eligible(B, T, C, ptrs, types == Types::bf16);
 }
 
 size_t vrwkv_biwkv_forward_workspace_bytes(int B, int T, int C) {
     if (check_shape(B, T, C) != VRWKV_OK) return 0;
     return std::max({biwkv::generic_forward_workspace(B, T, C) + 256, biwkv::fused::workspace_bytes(B, T, C, false),
-                     biwkv::resident::workspace_bytes(B, T, C, false)});
+                     biwkv::resident::workspace_bytes(B, T, C, false), biwkv::strips::workspace_bytes(B, T, C, false)});
 }
 
 int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u, const float* k,
@@ -153,6 +157,7 @@ int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u,
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (strips_serve(B, T, C, {k, v, y}, false, Types::f32)) return finish(biwkv::strips::forward(B, T, C, w, u, k, v, y, Types::f32, workspace, s));
     if (resident_serves(B, T, C, {k, v, y}, false, Types::f32))
         return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::f32, workspace, s));
     if (g_path.load() != 1 && biwkv::fused::eligible(B, T, C, {k, v, y}))
@@ -165,7 +170,7 @@ int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u,
 size_t vrwkv_biwkv_backward_workspace_bytes(int B, int T, int C) {
     if (check_shape(B, T, C) != VRWKV_OK) return 0;
     return std::max({biwkv::generic_backward_workspace(B, T, C) + 256, biwkv::fused::workspace_bytes(B, T, C, true),
-                     biwkv::resident::workspace_bytes(B, T, C, true)});
+                     biwkv::resident::workspace_bytes(B, T, C, true), biwkv::strips::workspace_bytes(B, T, C, true)});
 }
 
 int vrwkv_biwkv_backward_f32(int B, int T, int C, const float* w, const float* u, const float* k,
@@ -178,6 +183,8 @@ int vrwkv_biwkv_backward_f32(int B, int T, int C, const float* w, const float* u
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::f32))
+        return finish(biwkv::strips::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::f32, workspace, s));
     if (resident_serves(B, T, C, {k, v, gy, gk, gv}, true, Types::f32))
         return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::f32, workspace, s));
     if (g_path.load() != 1 && biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}))
@@ -264,6 +271,8 @@ int vrwkv_biwkv_forward_bf16(int B, int T, int C, const float* w, const float* u
     if (!w || !u || !k || !v || !y || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    if (strips_serve(B, T, C, {k, v, y}, false, Types::bf16))
+        return finish(biwkv::strips::forward(B, T, C, w, u, k, v, y, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
     if (resident_serves(B, T, C, {k, v, y}, false, Types::bf16))
         return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
     if (!biwkv::fused::eligible(B, T, C, {k, v, y}, true)) return VRWKV_ERR_UNSUPPORTED;
@@ -278,6 +287,8 @@ int vrwkv_biwkv_backward_bf16(int B, int T, int C, const float* w, const float* 
     if (misaligned4(w) || misaligned4(u) || misaligned4(gwgu) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    if (strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::bf16))
+        return finish(biwkv::strips::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
     if (resident_serves(B, T, C, {k, v, gy, gk, gv}, true, Types::bf16))
         return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
     if (!biwkv::fused::eligible(B, T, C, {k, v, gy, gk, gv}, true)) return VRWKV_ERR_UNSUPPORTED;
@@ -291,8 +302,8 @@ int vrwkv_biwkv_forward_bf16_wide(int B, int T, int C, const float* w, const flo
     if (!w || !u || !k || !v || !y || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
-    if (g_path.load() != 0 || !biwkv::resident::eligible(B, T, C, {k, v, y}, false, Types::wide)) return VRWKV_ERR_UNSUPPORTED;
-    return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::wide, workspace, static_cast<cudaStream_t>(stream)));
+    if (!strips_serve(B, T, C, {k, v, y}, false, Types::wide)) return VRWKV_ERR_UNSUPPORTED;
+    return finish(biwkv::strips::forward(B, T, C, w, u, k, v, y, Types::wide, workspace, static_cast<cudaStream_t>(stream)));
 }
 
 int vrwkv_biwkv_backward_bf16_wide(int B, int T, int C, const float* w, const float* u, const uint16_t* k, const uint16_t* v,
@@ -303,8 +314,8 @@ int vrwkv_biwkv_backward_bf16_wide(int B, int T, int C, const float* w, const fl
     if (misaligned4(w) || misaligned4(u) || misaligned4(gwgu) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
-    if (g_path.load() != 0 || !biwkv::resident::eligible(B, T, C, {k, v, gy, gk, gv}, true, Types::wide)) return VRWKV_ERR_UNSUPPORTED;
-    return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::wide, workspace, static_cast<cudaStream_t>(stream)));
+    if (!strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::wide)) return VRWKV_ERR_UNSUPPORTED;
+    return finish(biwkv::strips::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::wide, workspace, static_cast<cudaStream_t>(stream)));
 }
 
 // ---- WKV6 ---------------------------------------------------------------------------------------

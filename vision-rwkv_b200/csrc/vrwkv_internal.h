@@ -31,8 +31,9 @@ int generic_backward(int B, int T, int C, const float* w, const float* u, const 
                      const float* v, const float* gy, float* gwgu, float* gk, float* gv,
                      void* workspace, cudaStream_t stream);
 namespace resident {
-// Cluster-resident single-pass path (biwkv_resident.cu): C % 4 == 0 (f32) or C % 8 == 0 (the others), 16-byte aligned
-// tensors, T <= 32768 (wide: 4096).  w, u, gwgu are float32 always, arithmetic and shared-memory state too.
+// Long sequences (biwkv_resident.cu): 4096 < T <= 32768, C % 4 == 0 (f32) or C % 8 == 0 (bf16; wide: not here), 16-byte aligned
+// tensors.  The chunked kernels stand by for inputs outside the plain-float range: fused::eligible has to hold too.
+// w, u, gwgu are float32 always, arithmetic and shared-memory state too.
 enum class Types {
     f32,      // every tensor float32
     bf16,     // k, v, y, gy, gk, gv bfloat16
@@ -46,14 +47,21 @@ size_t workspace_bytes(int B, int T, int C, bool bwd, bool kept = false);
 // What a forward leaves for the backward: the states entering every 16 tokens, 1.5 bytes per element, and a flag; 0
 // where the backward takes nothing (T <= 4096, or few tokens in all).
 size_t kept_bytes(int B, int T, int C);
-// Behind sequences longer than one cluster holds (T > 4096) the chunked kernels stand by for inputs outside the plain-float
-// range: fused::eligible has to hold too.
-bool stands_by(int B, int T, int C);
 int forward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, Types types,
             void* workspace, cudaStream_t stream, void* keep = nullptr);
 int backward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, float* gwgu,
              void* gk, void* gv, Types types, void* workspace, cudaStream_t stream, const void* kept = nullptr);
 }  // namespace resident
+namespace strips {
+// Narrow strips, whole sequences in one CTA or cluster (biwkv_strips.cu): as resident, T <= 4096, all types.
+bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, resident::Types types);
+void set_withhold_test(bool on);
+size_t workspace_bytes(int B, int T, int C, bool bwd);
+int forward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, resident::Types types,
+            void* workspace, cudaStream_t stream);
+int backward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, float* gwgu,
+             void* gk, void* gv, resident::Types types, void* workspace, cudaStream_t stream);
+}  // namespace strips
 namespace fused {
 // True when the fused TMA path can serve this call on the current device.
 bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bf16 = false);
