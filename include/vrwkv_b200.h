@@ -144,23 +144,30 @@ int vrwkv_biwkv_backward_bf16(int B, int T, int C, const float* w, const float* 
                               uint16_t* gv, void* workspace, size_t workspace_bytes, void* stream);
 /* The same with float32 y and gy, what autograd has when w, u are float32 parameters and k, v come out of autocast
  * (CLS/vrwkv.py:42-44, 56-61 widen y and cast gy there): y holds the bfloat16 result widened, gy is rounded to bfloat16 as it is read.
- * T <= 4096; anything outside the cluster-resident kernels returns VRWKV_ERR_UNSUPPORTED before launching. */
+ * Sizes for which vrwkv_biwkv_one_pass(.., VRWKV_TENSORS_BF16_WIDE) is 1; anything else, and tensors that are not 16-byte aligned,
+ * returns VRWKV_ERR_UNSUPPORTED before launching. */
 int vrwkv_biwkv_forward_bf16_wide(int B, int T, int C, const float* w, const float* u, const uint16_t* k, const uint16_t* v, float* y,
                                   void* workspace, size_t workspace_bytes, void* stream);
 int vrwkv_biwkv_backward_bf16_wide(int B, int T, int C, const float* w, const float* u, const uint16_t* k, const uint16_t* v,
                                    const float* gy, float* gwgu, uint16_t* gk, uint16_t* gv, void* workspace, size_t workspace_bytes,
                                    void* stream);
 
+/* 1 where calls of these sizes (`tensors`: enum below) go through the kernels that read and write every element once, forward and
+ * backward: T <= 4096, and longer sequences up to 17 408 tokens where there are many.  A training pair has nothing to gain there from
+ * kept states (next comment). */
+int vrwkv_biwkv_one_pass(int B, int T, int C, int tensors);
+
 /* The training pair for long sequences: a forward that leaves the states entering every 16 tokens (1.5 bytes per element, in a
  * caller-owned buffer of vrwkv_biwkv_kept_bytes bytes, 256-byte aligned), and a backward that starts from them instead of
  * rebuilding them: two passes over the inputs instead of three.  vrwkv_biwkv_kept_bytes is 0 where a backward has no use for
- * them (T <= 4096, or few tokens in all).
+ * them (T <= 4096, or few tokens in all); where vrwkv_biwkv_one_pass is 1 the entry points above are faster.
  * w, u, k, v of the backward must be those of the forward.  `tensors` says what k, v, y, gy, gk, gv hold (enum below, as in the
  * entry points above; VRWKV_TENSORS_BF16_WIDE is refused at present: no kernels for it above 4096 tokens).  The workspaces hold neither
  * the states nor room for the other paths: vrwkv_biwkv_kept_workspace_bytes bytes, 0 where nothing is kept (those of the other entry
  * points are larger and serve too).  VRWKV_ERR_UNSUPPORTED: outside the cluster-resident
  * kernels (shape, alignment, vrwkv_set_path), nothing ran, use the other entry points; a forward may succeed and the backward
- * still return it (for an unaligned gy).  Results agree with the pair that keeps nothing to float32 rounding; y is the same bit for bit.
+ * still return it (for an unaligned gy).  Results agree with the pair that keeps nothing to float32 rounding (where
+ * vrwkv_biwkv_one_pass is 0, y bit for bit).
  * No reference counterpart (its backward rebuilds everything, bi_wkv_kernel.cu:259-302). */
 enum vrwkv_tensors { VRWKV_TENSORS_F32 = 0, VRWKV_TENSORS_BF16 = 1, VRWKV_TENSORS_BF16_WIDE = 2 };
 size_t vrwkv_biwkv_kept_bytes(int B, int T, int C);

@@ -11,10 +11,11 @@ pytestmark = pytest.mark.gpu
 NAMES = ("y", "gw", "gu", "gk", "gv")
 
 
-def errors(dev, B, T, C, types, w_range=None):
+def errors(dev, B, T, C, types, w_range=None, k_scale=1.0):
     from vision_rwkv_b200 import ops
     from vision_rwkv_b200.vrwkv import RUN_CUDA
     w, u, k, v, gy = O.make_inputs(B, T, C, dtype=torch.float32, seed=7 * T + C)
+    k = k * k_scale
     if w_range is not None:
         w = torch.linspace(*w_range, C) / T
     if types != "f32":
@@ -56,3 +57,33 @@ def test_steep_weights(cuda_device, T, w_range):
     for types, tol in (("f32", 5e-5), ("wide", 1e-2)):
         errs = errors(cuda_device, 3, T, 48, types, w_range)
         assert all(e <= tol for e in errs.values()), errs
+
+
+# enough sequences of more than 4096 tokens: clusters of 4 to 16 CTAs, the longest that a cluster holds; one token more goes back to separate launches
+@pytest.mark.parametrize("B,T", [(23, 4200), (12, 8704), (12, 8705), (6, 17408), (6, 17409)])
+@pytest.mark.parametrize("types", ["f32", "wide", "bf16"])
+def test_long_sequences(cuda_device, B, T, types):
+    from vision_rwkv_b200 import _lib
+    C, lib = 64, _lib.load()
+    before = lib.vrwkv_launch_count()
+    errs = errors(cuda_device, B, T, C, types)
+    one_pass = lib.vrwkv_biwkv_one_pass(B, T, C, ("f32", "bf16", "wide").index(types))
+    assert one_pass == (T <= (8704 if types == "bf16" else 17408))
+    assert (lib.vrwkv_launch_count() - before == 5) == bool(one_pass)
+    for name, e in errs.items():
+        assert e <= (1e-2 if types == "bf16" or (types == "wide" and name not in ("gw", "gu")) else 1e-5 if T <= 8192 else 2e-5), (name, errs)
+
+
+@pytest.mark.parametrize("T", [4200, 9000])
+def test_long_sequences_outside_the_plain_float_range(cuda_device, T):
+    errs = errors(cuda_device, 24, T, 64, "f32", k_scale=30.0)
+    assert all(e <= 5e-5 for e in errs.values()), errs
+
+
+def test_nothing_is_kept_where_one_pass_serves(cuda_device):
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    w, u, k, v, _ = [x.float().to(cuda_device) for x in O.make_inputs(23, 4200, 64, seed=1)]
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t.dtype), t)[1], lambda t: t):
+        RUN_CUDA(w, u, k.requires_grad_(True), v)
+    assert torch.uint8 not in seen

@@ -45,6 +45,7 @@ SIGNATURES = {
     "vrwkv_qshift_ddlerp_forward_bf16out": (_c_int, [_c_int] * 7 + [_ptr] * 3 + [_c_int] + [_ptr] * 2),
     "vrwkv_biwkv_forward_bf16_wide": (_c_int, [_c_int] * 3 + [_ptr] * 6 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_backward_bf16_wide": (_c_int, [_c_int] * 3 + [_ptr] * 9 + [_c_size_t, _ptr]),
+    "vrwkv_biwkv_one_pass": (_c_int, [_c_int] * 4),
     "vrwkv_biwkv_kept_bytes": (_c_size_t, [_c_int] * 3),
     "vrwkv_biwkv_kept_workspace_bytes": (_c_size_t, [_c_int] * 4),
     "vrwkv_biwkv_forward_keep": (_c_int, [_c_int] * 3 + [_ptr] * 5 + [_c_int, _ptr, _c_size_t, _ptr, _c_size_t, _ptr]),

@@ -65,7 +65,6 @@ constexpr int kMaxCluster = 16;
 constexpr int kBatch = 8;                   // other CTAs' blocks read together
 constexpr uint32_t kSpinLimit = 1u << 20;   // ~0.1 s of polling on a barrier
 constexpr float kSafeRange = 60.f;
-constexpr int kMostTokens = 4096;
 
 // P channel pairs, L tokens per walker
 template <int P_, int L_>
@@ -1093,6 +1092,21 @@ static auto with_strip(int strip, F&& f) {
     }
 }
 constexpr int kStrips = 4;
+// The sequences that are served here.  Up to 4096 tokens all.  Above, where there are at least kManyCtas CTAs' worth (of 256 tokens and
+// 32 channels, as biwkv_resident.cu counts them), up to kMostTokens, 16 CTAs of the narrow strips; with every tensor bfloat16 up to
+// kMostHalf, 16 of the others.  Training pairs through autograd, us, separate launches with kept states / here: float32 B=16, T=4200,
+// C=768 546 / 382; 16 x 8192 1022 / 801; 8 x 16384 1053 / 952; bfloat16 k, v beside float32 y, gy 710 / 383, 1286 / 868, 1295 / 1033;
+// all bfloat16 551 / 408, 952 / 915, but 11 x 12000 971 / 1085 (rows of 16 bytes, and two passes over half the bytes are cheap).
+// Below kManyCtas this is faster as well (B=2, T=4200, C=384: forward 31 / 23, backward 65 / 34), but the launches and kept states of
+// the routes there are relied upon by callers that count them.
+constexpr int kAnyTokens = 4096, kMostTokens = kMaxCluster * kMaxWarps * Strip<4, 17>::kSpan, kMostHalf = kMaxCluster * kMaxWarps * Strip<8, 17>::kSpan;
+constexpr long long kManyCtas = 768;
+bool in_range(int B, int T, int C, Types types) {
+    if (C % (types != Types::f32 ? 8 : 4) != 0) return false;      // TMA row pitch must be 16-byte
+    if (T <= kAnyTokens) return true;
+    return T <= (types == Types::bf16 ? kMostHalf : kMostTokens) && static_cast<long long>(B) * ((C + 31) / 32) * ((T + 255) / 256) >= kManyCtas;
+}
+
 // A plan's time for a token, up to a factor: token slots taken, the warps that an SM then has in hand (registers: 16 of the backward,
 // 24 of the forward), the hand-over between a cluster's CTAs, narrow rows.
 static float plan_cost(int T, bool bwd, Types types, const Plan& pl) {
@@ -1102,12 +1116,13 @@ static float plan_cost(int T, bool bwd, Types types, const Plan& pl) {
     const int most = bwd ? 16 : 24, held = most / pl.n_warps * pl.n_warps;
     const float waste = static_cast<float>(pl.cluster * pl.n_tok) / static_cast<float>(T);
     const float idle = 1.f + 0.4f * static_cast<float>(most - held) / static_cast<float>(most);
-    const float hand_over = pl.cluster <= 8 ? (bwd ? kBackward : kForward)[pl.cluster - 1] : 1.1f * (bwd ? kBackward : kForward)[7];
+    // more CTAs: float32 backward of 10, 12, 16 CTAs 544 (5000 tokens), 593, 633; forward 226, 241, 259
+    const float hand_over = (bwd ? kBackward : kForward)[std::min(pl.cluster, 8) - 1] + (bwd ? 0.05f : 0.025f) * static_cast<float>(std::max(pl.cluster - 8, 0));
     const float narrow = pl.cs == 16 ? 1.f : types == Types::f32 ? (bwd ? 1.04f : 1.19f) : (bwd ? 1.14f : 1.09f);
     return waste * idle * hand_over * narrow;
 }
-static bool make_plan(int T, bool bwd, Types types, Plan& best) {
-    if (T > kMostTokens) return false;
+static bool make_plan(int B, int T, int C, bool bwd, Types types, Plan& best) {
+    if (!in_range(B, T, C, types)) return false;
     const auto up = [](int a, int b) { return (a + b - 1) / b; };
     float least = 0.f;
     best.strip = -1;
@@ -1215,11 +1230,10 @@ static bool fits(const Plan& pl, bool bwd, Types types) {
 static size_t strips_of(int C, const Plan& pl) { return (C + pl.cs - 1) / pl.cs; }
 
 bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types) {
-    if (C % (types != Types::f32 ? 8 : 4) != 0) return false;      // TMA row pitch must be 16-byte
     for (const void* q : ptrs)
         if (reinterpret_cast<uintptr_t>(q) & 15u) return false;    // TMA base alignment
     Plan pl;
-    if (!make_plan(T, bwd, types, pl) || B * strips_of(C, pl) * pl.cluster > (1u << 30)) return false;
+    if (!make_plan(B, T, C, bwd, types, pl) || B * strips_of(C, pl) * pl.cluster > (1u << 30)) return false;
     if (static_cast<long long>(T) * C > (1LL << 30)) return false;      // 32-bit offsets within a sequence
     return with_strip(pl.strip, [&](auto st) { return fits<decltype(st)>(pl, bwd, types); });
 }
@@ -1241,7 +1255,7 @@ size_t workspace_bytes(int B, int T, int C, bool bwd) {
     size_t most = 256;
     for (Types types : {Types::f32, Types::bf16, Types::wide}) {
         Plan pl;
-        if (make_plan(T, bwd, types, pl)) most = std::max(most, carve(B, C, pl, bwd).total);
+        if (make_plan(B, T, C, bwd, types, pl)) most = std::max(most, carve(B, C, pl, bwd).total);
     }
     return most;
 }
@@ -1308,7 +1322,7 @@ template <bool kBwd, Types kTypes>
 static int launch(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, void* o0, void* o1,
                   float* gwgu, void* workspace, cudaStream_t stream) {
     Plan pl;
-    if (!make_plan(T, kBwd, kTypes, pl)) return -1;
+    if (!make_plan(B, T, C, kBwd, kTypes, pl)) return -1;
     return with_strip(pl.strip, [&](auto st) { return launch<decltype(st), kBwd, kTypes>(pl, B, T, C, w, u, k, v, gy, o0, o1, gwgu, workspace, stream); });
 }
 

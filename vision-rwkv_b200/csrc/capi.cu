@@ -200,6 +200,11 @@ static bool types_of(int types, Types& t) {
     return true;
 }
 
+int vrwkv_biwkv_one_pass(int B, int T, int C, int tensors) {
+    Types types;
+    return check_shape(B, T, C) == VRWKV_OK && types_of(tensors, types) && biwkv::strips::in_range(B, T, C, types) ? 1 : 0;
+}
+
 size_t vrwkv_biwkv_kept_bytes(int B, int T, int C) {
     if (check_shape(B, T, C) != VRWKV_OK) return 0;
     return biwkv::resident::kept_bytes(B, T, C);

@@ -68,12 +68,13 @@ at::ScalarType result_dtype(const Tensor& w) {
 // The forward that keeps states for the backward, into `kept`; false (and an undefined `kept`) where it does not serve the call.
 bool biwkv_forward_keep(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& y, Tensor* kept) {
     const int B = k.size(0), T = k.size(1), C = k.size(2);
+    const int types = is_bf16(k) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_F32;
     const size_t bytes = vrwkv_biwkv_kept_bytes(B, T, C);
-    if (bytes == 0) return false;
+    if (bytes == 0 || vrwkv_biwkv_one_pass(B, T, C, types)) return false;
     *kept = workspace(bytes, k);
     const Tensor ws = workspace(vrwkv_biwkv_kept_workspace_bytes(B, T, C, 0), k);
     const int st = vrwkv_biwkv_forward_keep(B, T, C, fp(w), fp(u), k.data_ptr(), v.data_ptr(), y.data_ptr(),
-                                            is_bf16(k) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_F32, kept->data_ptr(), kept->numel(), ws.data_ptr(),
+                                            types, kept->data_ptr(), kept->numel(), ws.data_ptr(),
                                             ws.numel(), stream_of(k));
     if (st != VRWKV_OK) kept->reset();
     if (st == VRWKV_ERR_UNSUPPORTED) return false;
@@ -106,11 +107,12 @@ Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, cons
     return y;
 }
 
-constexpr int64_t kMostWideTokens = 4096;      // of the entry points with float32 y, gy beside bfloat16 k, v
+// whether the entry points with float32 y, gy beside bfloat16 k, v are for calls of this size
+bool wide_serves(const Tensor& k) { return vrwkv_biwkv_one_pass(k.size(0), k.size(1), k.size(2), VRWKV_TENSORS_BF16_WIDE) != 0; }
 
 // k, v bfloat16, contiguous; y float32 holding bfloat16 values.  Undefined where the kernel does not cover the call.
 Tensor biwkv_forward_wide(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
-    if (k.size(1) > kMostWideTokens) return Tensor();
+    if (k.numel() != 0 && !wide_serves(k)) return Tensor();
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor y = at::empty_like(k, k.options().dtype(at::kFloat));
     if (k.numel() == 0) return y;
@@ -149,8 +151,8 @@ Tensor usable_states(const Tensor& kept, const Tensor& k) {
 // k, v float32, or bfloat16 (then gy in either type); all contiguous.  kept: what the forward left, or undefined.
 std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, const Tensor& gy,
                                          const Tensor& kept = Tensor()) {
-    // the kernels for a float32 gy end there: narrowed before anything is allocated
-    if (is_bf16(k) && !is_bf16(gy) && k.size(1) > kMostWideTokens) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16), kept);
+    // no kernels for a float32 gy: narrowed before anything is allocated
+    if (k.numel() != 0 && is_bf16(k) && !is_bf16(gy) && !wide_serves(k)) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16), kept);
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor gk = at::empty_like(k), gv = at::empty_like(k);
     Tensor gwgu = at::empty({2, C}, k.options().dtype(at::kFloat));

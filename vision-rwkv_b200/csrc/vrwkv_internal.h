@@ -53,7 +53,9 @@ int backward(int B, int T, int C, const float* w, const float* u, const void* k,
              void* gk, void* gv, Types types, void* workspace, cudaStream_t stream, const void* kept = nullptr);
 }  // namespace resident
 namespace strips {
-// Narrow strips, whole sequences in one CTA or cluster (biwkv_strips.cu): as resident, T <= 4096, all types.
+// Narrow strips, whole sequences in one CTA or cluster (biwkv_strips.cu), all types; 16-byte aligned tensors of these sizes:
+bool in_range(int B, int T, int C, resident::Types types);
+// ... and the current device can launch them
 bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, resident::Types types);
 void set_withhold_test(bool on);
 size_t workspace_bytes(int B, int T, int C, bool bwd);
