@@ -87,3 +87,25 @@ def test_nothing_is_kept_where_one_pass_serves(cuda_device):
     with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t.dtype), t)[1], lambda t: t):
         RUN_CUDA(w, u, k.requires_grad_(True), v)
     assert torch.uint8 not in seen
+
+
+@pytest.mark.parametrize("T,k_scale", [(100, 1.0), (100, 30.0), (1200, 1.0), (1200, 30.0)])      # 30: left to the exact kernel
+@pytest.mark.parametrize("fill", [0x00, 0xFF])
+def test_a_workspace_needs_no_clearing(cuda_device, T, k_scale, fill):
+    from vision_rwkv_b200 import _lib
+    import ctypes
+    B, C, lib = 2, 40, _lib.load()
+    w, u, k, v, gy = [x.float().to(cuda_device).contiguous() for x in O.make_inputs(B, T, C, seed=T)]
+    k = k * k_scale
+    y, gk, gv, gwgu = torch.empty_like(k), torch.empty_like(k), torch.empty_like(k), torch.empty(2, C, device=cuda_device)
+    ws = [torch.full((f(B, T, C),), fill, dtype=torch.uint8, device=cuda_device) for f in (lib.vrwkv_biwkv_forward_workspace_bytes, lib.vrwkv_biwkv_backward_workspace_bytes)]
+    s, p = torch.cuda.current_stream().cuda_stream, lambda t: t.data_ptr()
+    assert lib.vrwkv_biwkv_forward_f32(B, T, C, p(w), p(u), p(k), p(v), p(y), p(ws[0]), ws[0].numel(), s) == 0
+    assert lib.vrwkv_biwkv_backward_f32(B, T, C, p(w), p(u), p(k), p(v), p(gy), p(gwgu), p(gk), p(gv), p(ws[1]), ws[1].numel(), s) == 0
+    for x in ws:
+        status = ctypes.c_uint(9)
+        assert lib.vrwkv_workspace_status(p(x), s, ctypes.byref(status)) == 0 and status.value == 0
+    f = [x.double().cpu() for x in (w, u, k, v, gy)]
+    ref = (O.biwkv_scan_forward(*f[:4]), *O.biwkv_scan_backward(*f))
+    for a, b in zip((y, gwgu[0], gwgu[1], gk, gv), ref):
+        assert rel_err(a, b) <= (1e-5 if k_scale == 1.0 else 5e-5)

@@ -103,11 +103,17 @@ struct Params {
     unsigned* status;
     unsigned* mirror;
     float* partial;         // backward: [b][rank][gw | gu][c_padded]
-    unsigned* redo_count;   // units left to the exact kernel, and which
-    int* redo_list;
+    unsigned* words;        // one per CTA, from the fast kernel to the exact one: kRedo, bits of waits that gave up
     uint32_t spin_limit;
     int withhold_rank;      // test only: this rank of every cluster sends nothing (-1: none)
 };
+
+// What a CTA leaves in its word: its unit is the exact kernel's; status bits of its waits, shifted.  Every CTA writes its own, so nothing
+// has to be cleared before the launch (a memset took 1.5 us of the GPU and as much of the host, in a forward of one image 14).
+constexpr unsigned kRedo = 1u, kFailedShift = 8;
+// what may be launched behind this grid need not wait for its end any longer; what a dependent grid reads of the one before it
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 struct Ctx {
     float* sub;      // [n_warps][kRecRows][kCs]
@@ -116,13 +122,14 @@ struct Ctx {
     float* cta;      // [kRecRows][kCs]: state entering this CTA from the cluster
     float* consts;
     uint64_t* xbar;  // [levels]: bytes the other CTAs send
-    unsigned* flag;
-    unsigned* status;
-    unsigned* mirror;
+    unsigned* flag;  // [0]: the unit's, out of range; [1]: this CTA's waits that gave up
     uint32_t spin_limit;
     bool withhold;
     int warp, lane, n_warps, n_tok, cluster, rank;
 };
+// a wait gave up
+__device__ __forceinline__ void failed(const Ctx& c, unsigned bits) { atomicOr(c.flag + 1, bits); }
+
 struct Enter {
     Pair2 P, S;   // state entering at the first token, at the last
 };
@@ -269,7 +276,7 @@ __device__ __forceinline__ Enter exchange(const Ctx& c, int level, Pair2 F, Pair
         }
         __syncwarp();
         if (warp == 0) {
-            if (!sm100::mbar_wait(c.xbar + level, 0, c.spin_limit) && lane == 0) report_failure(c.status, c.mirror, 1u);
+            if (!sm100::mbar_wait(c.xbar + level, 0, c.spin_limit) && lane == 0) failed(c, 1u);
             if (level == 0) {
                 const int other = (lane < c.cluster && lane != c.rank) ? __float_as_int(peers[(lane - (lane > c.rank ? 1 : 0)) * kB + 2 * kCs]) : 0;
                 const int flag = __any_sync(0xffffffffu, (other | any) != 0) ? 1 : 0;
@@ -362,7 +369,6 @@ static inline size_t smem_bytes(int n_warps, int cluster) {
 // what follows the tiles; returns the mbarriers of the tiles
 template <class St, bool kBwd, bool kSingle>
 __device__ __forceinline__ uint64_t* carve_smem(Ctx& c, float* at, const Params& p) {
-    c.status = p.status; c.mirror = p.mirror;
     c.warp = threadIdx.x >> 5; c.lane = threadIdx.x & 31; c.n_warps = p.n_warps; c.n_tok = p.n_tok;
     c.cluster = kSingle ? 1 : p.cluster;
     c.rank = kSingle ? 0 : static_cast<int>(cluster_rank());
@@ -376,7 +382,18 @@ __device__ __forceinline__ uint64_t* carve_smem(Ctx& c, float* at, const Params&
     uint64_t* const bars = reinterpret_cast<uint64_t*>(c.consts + St::kConstRows * St::kCs);
     c.xbar = bars + 2 * kMaxWarps;
     c.flag = reinterpret_cast<unsigned*>(c.xbar + 2);
+    if (threadIdx.x == 0) c.flag[1] = 0u;      // a CTA barrier follows before anyone waits for anything
     return bars;
+}
+// behind a CTA barrier that follows the last wait
+__device__ __forceinline__ void leave_word(const Ctx& c, const Params& p, unsigned redo) {
+    launch_dependents();
+    if (threadIdx.x == 0) {
+        const unsigned bits = c.flag[1];
+        p.words[blockIdx.x] = redo | bits << kFailedShift;
+        if (bits != 0u && p.mirror != nullptr) *reinterpret_cast<volatile unsigned*>(p.mirror) = bits;
+        if (blockIdx.x == 0) *p.status = 0u;      // the exact kernel collects the bits
+    }
 }
 // the mbarriers of the hand-over between CTAs: a block from every other one, per level
 template <class St, bool kBwd>
@@ -491,7 +508,7 @@ biwkv_forward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     const int ch0 = strip * kCs + 2 * pr;
     const float* const cst = c.consts + 2 * pr;
     const float2 lam2 = at2(cst + kLam * kCs), c2 = at2(cst + kCuw * kCs), lam4 = at2(cst + kLam4 * kCs);
-    if (!sm100::mbar_wait(full + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
+    if (!sm100::mbar_wait(full + warp, 0, kSpinLimit)) failed(c, 2u);
     if (!kSingle) cluster_wait();
 
     const int row0 = wk * L;                                       // of this walker in the warp's areas
@@ -510,9 +527,11 @@ biwkv_forward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     if (unsafe) {
         // the whole cluster takes this branch together: the unit is left to the exact kernel, which runs right behind (nothing of
         // this CTA is in flight any more: its tiles have landed and everything the other CTAs sent has been waited for)
-        if (c.rank == 0 && threadIdx.x == 0) p.redo_list[atomicAdd(p.redo_count, 1u)] = unit;
+        __syncthreads();
+        leave_word(c, p, kRedo);
         return;
     }
+    leave_word(c, p, 0u);      // the last wait of this CTA lies behind its barrier in the exchange
     // ---- pass 2: y = (P + S + e^{u} x) ratio, in place of the numerator term ----
     const int n_out = ch0 < p.C ? n : 0;
     const RowsOut y(p.o0, p, b, tok0 + row0, ch0);
@@ -595,7 +614,7 @@ biwkv_backward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     const int ch0 = strip * kCs + 2 * pr;
     const float* const cst = c.consts + 2 * pr;
     const float2 lam2 = at2(cst + kLam * kCs), lam4 = at2(cst + kLam4 * kCs);
-    if (!sm100::mbar_wait(full + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
+    if (!sm100::mbar_wait(full + warp, 0, kSpinLimit)) failed(c, 2u);
     if (!kSingle) cluster_wait();
 
     const int row0 = wk * L;                                       // of this walker in the warp's areas
@@ -613,9 +632,10 @@ biwkv_backward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     if (n < L) F = zero();
     Enter e1 = exchange<St, kSingle>(c, 0, F, group_sum(r, lam4, cst, kCs), unsafe);
     if (n == 0) e1 = Enter{zero(), zero()};
-    if (!sm100::mbar_wait(gfull + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
+    if (!sm100::mbar_wait(gfull + warp, 0, kSpinLimit)) failed(c, 2u);
     if (unsafe) {      // as in the forward
-        if (c.rank == 0 && threadIdx.x == 0) p.redo_list[atomicAdd(p.redo_count, 1u)] = unit;
+        __syncthreads();
+        leave_word(c, p, kRedo);
         return;
     }
     if (kHalfG) {
@@ -760,6 +780,7 @@ biwkv_backward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         *reinterpret_cast<float2*>(rec + kCs) = gu;
     }
     __syncthreads();
+    leave_word(c, p, 0u);
     if (threadIdx.x < 2 * kCs) {
         const int j = threadIdx.x / kCs, ch = threadIdx.x & (kCs - 1);
         float acc = 0.f;
@@ -961,9 +982,19 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     constexpr bool kHalf = kTypes != Types::f32, kHalfG = kTypes == Types::bf16;
     constexpr bool kHalfOut = kBwd ? kHalf : kTypes == Types::bf16;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    const unsigned n_redo = *reinterpret_cast<volatile unsigned*>(p.redo_count);
     const int n_clusters = static_cast<int>(gridDim.x) / p.cluster, mine = static_cast<int>(blockIdx.x) / p.cluster;
-    if (static_cast<unsigned>(mine) >= n_redo) return;       // the same for every CTA of a cluster
+    const int rank = p.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
+    launch_dependents();
+    wait_for_launch_before();
+    // this cluster's units: mine, mine + n_clusters, ..; all their CTAs wrote the same kRedo
+    bool any = false;
+    unsigned bits = 0u;
+    for (int u = mine + static_cast<int>(threadIdx.x) * n_clusters; u < p.units; u += static_cast<int>(blockDim.x) * n_clusters) {
+        any = any || (__ldcg(p.words + static_cast<size_t>(u) * p.cluster) & kRedo) != 0u;
+        bits |= __ldcg(p.words + static_cast<size_t>(u) * p.cluster + rank) >> kFailedShift;
+    }
+    if (bits != 0u) atomicOr(p.status, bits);
+    if (!__syncthreads_or(any ? 1 : 0)) return;       // the same for every CTA of a cluster
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pr = lane % P, wk = lane / P;
     const int nw = p.n_warps;
@@ -974,7 +1005,7 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     c.n_sub = nw * St::kW; c.n_tok = p.n_tok; c.cluster = p.cluster;
     c.area = reinterpret_cast<float*>(smem_raw) + (kBwd ? 3 : 2) * nw * kArea;
     c.agg = c.area + c.n_sub * 5 * kCs;
-    c.rank = p.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
+    c.rank = rank;
     uint64_t* const full = reinterpret_cast<uint64_t*>(c.agg + 5 * kCs);
     if (threadIdx.x == 0) {
         sm100::mbar_init(full, 1);
@@ -987,8 +1018,8 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     float* const vs = slot_v + row0 * kCs + 2 * pr;
     float* const gs = slot_g + row0 * kCs + 2 * pr;
     uint32_t phase = 0;
-    for (unsigned j = mine; j < n_redo; j += n_clusters) {
-        const int unit = p.redo_list[j];
+    for (int unit = mine; unit < p.units; unit += n_clusters) {
+        if ((__ldcg(p.words + static_cast<size_t>(unit) * p.cluster) & kRedo) == 0u) continue;
         const int b = unit / p.n_strips, strip = unit - b * p.n_strips;
         constexpr int kIn = kHalf ? kArea / 2 : 0, kInG = kHalfG ? kArea / 2 : 0;
         if (threadIdx.x == 0) {
@@ -1057,9 +1088,10 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
 __global__ void __launch_bounds__(1024) reduce_partials(int rows, int c_padded, int C, const float* __restrict__ partial, float* __restrict__ out) {
     __shared__ float red[32][33];
     const int j = blockIdx.y, lane = threadIdx.x, ch = blockIdx.x * 32 + lane;
+    wait_for_launch_before();
     float acc = 0.f;
     if (ch < C)
-        for (int r = threadIdx.y; r < rows; r += 32) acc += partial[(static_cast<size_t>(r) * 2 + j) * c_padded + ch];
+        for (int r = threadIdx.y; r < rows; r += 32) acc += __ldcg(partial + (static_cast<size_t>(r) * 2 + j) * c_padded + ch);
     red[threadIdx.y][lane] = acc;
     __syncthreads();
     if (threadIdx.y == 0 && ch < C) {
@@ -1239,14 +1271,14 @@ bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool
 }
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-// workspace: status block (256 B) | redo list | backward partials | copies of w, u
+// workspace: status block (256 B) | a word per CTA | backward partials | copies of w, u
 struct Carve {
-    size_t off_list, off_partial, off_vectors, total;
+    size_t off_words, off_partial, off_vectors, total;
 };
 static Carve carve(int B, int C, const Plan& pl, bool bwd) {
     Carve cv;
-    cv.off_list = 256;
-    cv.off_partial = cv.off_list + align_up(B * strips_of(C, pl) * sizeof(int), 256);
+    cv.off_words = 256;
+    cv.off_partial = cv.off_words + align_up(B * strips_of(C, pl) * pl.cluster * sizeof(unsigned), 256);
     cv.off_vectors = cv.off_partial + (bwd ? align_up(static_cast<size_t>(B) * pl.cluster * 2 * strips_of(C, pl) * pl.cs * sizeof(float), 256) : 0);
     cv.total = cv.off_vectors + align_up(2 * static_cast<size_t>(C) * sizeof(float), 256);
     return cv;
@@ -1278,8 +1310,7 @@ static int launch(const Plan& pl, int B, int T, int C, const float* w, const flo
     p.status = reinterpret_cast<unsigned*>(ws);
     p.mirror = failure_mirror(kBwd ? Op::biwkv_backward : Op::biwkv_forward);
     p.partial = reinterpret_cast<float*>(ws + cv.off_partial);
-    p.redo_count = p.status + 1;
-    p.redo_list = reinterpret_cast<int*>(ws + cv.off_list);
+    p.words = reinterpret_cast<unsigned*>(ws + cv.off_words);
     p.spin_limit = g_withhold.load() ? (1u << 10) : kSpinLimit;
     p.withhold_rank = g_withhold.load() ? 1 : -1;
     tensor_map::bind_primary_context();   // the tensor-map encoder is a driver call
@@ -1292,17 +1323,24 @@ static int launch(const Plan& pl, int B, int T, int C, const float* w, const flo
         set_error_detail("cuTensorMapEncodeTiled rejected a (C, T, B) tensor map");
         return -1;
     }
-    cudaMemsetAsync(ws, 0, 256, stream);
-    const auto run = [&](auto* fn, size_t clusters, size_t smem, auto... args) {
+    // `behind`: launched behind the kernel before it, which it waits for by itself (wait_for_launch_before)
+    const auto run = [&](auto* fn, bool behind, size_t clusters, size_t smem, auto... args) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(clusters * pl.cluster));
         cfg.blockDim = dim3(pl.n_warps * 32);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-        cfg.attrs = at; cfg.numAttrs = pl.cluster > 1 ? 1 : 0;
+        cudaLaunchAttribute at[2];
+        unsigned n = 0;
+        if (behind) {
+            at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[n++].val.programmaticStreamSerializationAllowed = 1;
+        }
+        if (pl.cluster > 1) {
+            at[n].id = cudaLaunchAttributeClusterDimension;
+            at[n].val.clusterDim.x = pl.cluster; at[n].val.clusterDim.y = 1; at[n++].val.clusterDim.z = 1;
+        }
+        cfg.attrs = at; cfg.numAttrs = n;
         const cudaError_t err = cudaLaunchKernelEx(&cfg, fn, args..., p);
         if (err != cudaSuccess) set_error_detail(cudaGetErrorName(err));
         return err == cudaSuccess;
@@ -1310,12 +1348,22 @@ static int launch(const Plan& pl, int B, int T, int C, const float* w, const flo
     const size_t units = p.units;
     const size_t smem = smem_bytes<St, kBwd>(pl.n_warps, pl.cluster);
     bool done;
-    if constexpr (kBwd) done = run(backward_kernel<St, kTypes>(pl.cluster == 1), units, smem, mk, mv, mg, m0, m1);
-    else done = run(forward_kernel<St, kTypes>(pl.cluster == 1), units, smem, mk, mv, m0);
+    if constexpr (kBwd) done = run(backward_kernel<St, kTypes>(pl.cluster == 1), false, units, smem, mk, mv, mg, m0, m1);
+    else done = run(forward_kernel<St, kTypes>(pl.cluster == 1), false, units, smem, mk, mv, m0);
     if (!done) return -1;
     // the exact kernel: a few clusters that serve whatever the fast kernel left behind
-    if (!run(biwkv_exact_kernel<St, kBwd, kTypes>, std::min<size_t>(units, std::max(16, 128 / pl.cluster)), exact_smem<St, kBwd>(pl.n_warps), mk, mv, mg, m0, m1)) return -1;
-    if (kBwd) reduce_partials<<<dim3((C + 31) / 32, 2), dim3(32, 32), 0, stream>>>(B * pl.cluster, p.c_padded, C, p.partial, gwgu);
+    if (!run(biwkv_exact_kernel<St, kBwd, kTypes>, true, std::min<size_t>(units, std::max(16, 128 / pl.cluster)), exact_smem<St, kBwd>(pl.n_warps), mk, mv, mg, m0, m1)) return -1;
+    if (kBwd) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((C + 31) / 32, 2);
+        cfg.blockDim = dim3(32, 32);
+        cfg.stream = stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, reduce_partials, B * pl.cluster, p.c_padded, C, static_cast<const float*>(p.partial), gwgu);
+    }
     return kBwd ? 3 : 2;
 }
 template <bool kBwd, Types kTypes>
