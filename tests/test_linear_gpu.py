@@ -1,0 +1,48 @@
+"""relu(x W^T)^2 as one matrix product: against the product in float64, rounded where autocast rounds.  A float32 sum p that lies near
+the middle of two bfloat16 numbers may go to the other one, an ulp (2^-7 |p| at most) away, and sums of up to 1024 products of size 1
+are off by 1e-5: the square differs by 2^-6 p^2 + 2e-5 |p| from that, and by its own rounding, 2^-8 p^2.  Few sums do: 1e-2 in the 2-norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# rows around a tile's 128, fewer and more tiles than SMs (several per CTA, both accumulators); K of one slice, of fewer and more than the four stages
+@pytest.mark.parametrize("rows,K,N", [(1, 64, 256), (127, 192, 256), (128, 256, 512), (129, 320, 256), (1000, 384, 1536), (19008, 192, 768),
+                                      (5000, 1024, 4096), (40001, 64, 256)])
+def test_against_float64(cuda_device, rows, K, N):
+    from vision_rwkv_b200 import _lib
+    g = torch.Generator(device=cuda_device).manual_seed(rows + K)
+    x = torch.randn(rows, K, device=cuda_device, generator=g).bfloat16()
+    w = (torch.randn(N, K, device=cuda_device, generator=g) / K ** 0.5).bfloat16()
+    with torch.autocast("cuda", torch.bfloat16):
+        out = _lib.native().linear_relu_square(x, w)
+    ref = (x.double() @ w.double().T).bfloat16().double().relu().square()
+    assert out.shape == (rows, N) and out.dtype == torch.bfloat16
+    assert ((out.double() - ref).norm() / ref.norm()).item() <= 1e-2
+    assert ((out.double() - ref).abs() <= (2.0 ** -6 + 2.0 ** -8) * 1.02 * ref + 2e-5 * ref.sqrt() + 1e-9).all()
+
+
+def test_not_a_number_stays(cuda_device):
+    from vision_rwkv_b200 import _lib
+    x = torch.ones(130, 64, device=cuda_device).bfloat16()
+    x[129, 3] = float("nan")
+    x[5, 1] = float("inf")
+    with torch.autocast("cuda", torch.bfloat16):
+        out = _lib.native().linear_relu_square(x, torch.ones(256, 64, device=cuda_device))
+    assert out[129].isnan().all() and out[5].isinf().all() and (out[6] == 4096).all()
+
+
+def test_layers_that_are_watched_or_replaced_keep_their_call(cuda_device):
+    from vision_rwkv_b200 import epilogue
+    key, value = torch.nn.Linear(192, 768, bias=False, device=cuda_device), torch.nn.Linear(768, 192, bias=False, device=cuda_device)
+    x = torch.randn(20000, 192, device=cuda_device).bfloat16()
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        want = epilogue.relu_square(key(x), value)
+        got = epilogue.linear_relu_square(key, x, value)
+        seen = []
+        hook = key.register_forward_hook(lambda *a: seen.append(1))
+        again = epilogue.linear_relu_square(key, x, value)
+        hook.remove()
+    assert seen == [1] and torch.equal(again, want)
+    assert ((got.float() - want.float()).norm() / want.float().norm()).item() <= 5e-3      # sums in another order: some roundings differ

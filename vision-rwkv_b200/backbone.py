@@ -92,7 +92,7 @@ class ChannelMix(nn.Module):
                                    self.shift_pixel, self.channel_gamma)
         else:
             xk = xr = x
-        k = epilogue.relu_square(self.key(xk), self.value if self.key_norm is None else None)
+        k = epilogue.linear_relu_square(self.key, xk, self.value if self.key_norm is None else None)
         if self.key_norm is not None:
             k = self.key_norm(k)
         return self.receptance(xr), self.value(k)

@@ -127,7 +127,7 @@ class ChannelMixV6(nn.Module):
         """(r, y) of the gate sigmoid(r) * y that ends the mix"""
         xk, xr = qshift_mix_to((self.key, self.receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution, self.shift_pixel,
                                head_dim=HEAD_SIZE)       # per-head shift + both interpolations in one pass
-        k = epilogue.relu_square(self.key(xk), self.value if self.key_norm is None else None)
+        k = epilogue.linear_relu_square(self.key, xk, self.value if self.key_norm is None else None)
         if self.key_norm is not None:
             k = self.key_norm(k)
         return self.receptance(xr), self.value(k)

@@ -45,7 +45,7 @@ int record_launches(int launched) { return finish(launched); }
 // One word per device and operator in pinned, mapped host memory: kernels write it only when a bounded wait runs out, the host
 // reads it as ordinary memory, so watching for failures costs neither a copy nor an event per launch.
 namespace {
-constexpr int kMirrorDevices = 64, kMirrorOps = 4;
+constexpr int kMirrorDevices = 64, kMirrorOps = 5;
 std::atomic<unsigned*> g_mirror{nullptr};
 std::mutex g_mirror_mutex;
 }  // namespace

@@ -1,0 +1,261 @@
+// out = relu(x W^T)^2 in bfloat16 for an inference pass under bfloat16 autocast: the first half of a channel mix
+// (classification/mmcls_custom/models/backbones/vrwkv.py:249-251), as one matrix product on the 5th-generation tensor cores whose
+// epilogue rounds, clips and squares.
+//
+// The product alone is a library's business; what this saves is the pass behind it, which reads and writes the widest activation of
+// the network (2 x 154 MB at 256 images of VRWKV-S, C = 384).
+//
+// A persistent CTA per SM walks 128 x 256 tiles of the result, columns fastest (the rows of x stay in L2).  Warp 0 brings 64-wide slices
+// of x and W by TMA (128-byte swizzle, four stages of 48 KB), warp 1 issues tcgen05.mma into one of two accumulators in tensor memory
+// (2 x 256 columns, all of it), warps 2 to 5 take the other one through registers and shared memory to a TMA store, so the
+// epilogue, about 2 000 cycles, runs under the 3 000 cycles of a tile's products at K = 384.
+//
+// us, library product / and the pass behind it / this: rows 50176 K=192 N=768 24.7 / 51.4 / 30.9, 384 -> 1536 57.5 / 108.8 / 63.5 (HBM's
+// time for x and the result 30, 931 TFLOP/s), 768 -> 3072 180 / 303 / 207, 1024 -> 4096 300 / 469 / 324 (1301 TFLOP/s of a measured 1410);
+// rows 12544 768 -> 3072 47.2 / 74.2 / 52.2; rows 196 (calls one by one, host time in part) 10.5 / 15.1 / 8.3 to 10.9 / 15.6 / 14.5.
+// So it serves every size that its tiles divide.
+//
+// Every wait is bounded; one that gives up sets a flag that ends the other roles, and the host-visible word of failures.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <algorithm>
+#include <mutex>
+#include "../../include/vrwkv_b200.h"
+#include "sm100_async.cuh"
+#include "tensor_map.h"
+#include "vrwkv_internal.h"
+
+namespace lineartc {
+
+constexpr int kM = 128, kN = 256, kK = 64, kStages = 4;
+constexpr uint32_t kABytes = kM * kK * 2, kStageBytes = kABytes + kN * kK * 2, kBoxBytes = kM * 64 * 2;
+constexpr int kThreads = 192;
+constexpr uint32_t kWaitLimit = 1u << 20;
+
+struct Bars {
+    uint64_t full[kStages], empty[kStages], done[2], taken[2], drained;
+    uint32_t tmem;
+    volatile uint32_t dead;
+};
+constexpr size_t kSmem = 1024 + kStages * kStageBytes + 2 * kBoxBytes + sizeof(Bars);
+
+using sm100::smem_u32;
+
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src),
+                 "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
+// K-major operand in 128-byte rows, swizzled; eight rows are 1024 bytes
+__device__ __forceinline__ uint64_t operand(uint32_t addr) {
+    return static_cast<uint64_t>((addr >> 4) & 0x3FFF) | static_cast<uint64_t>(1) << 16 | static_cast<uint64_t>(1024 >> 4) << 32 | static_cast<uint64_t>(1) << 46 |
+           static_cast<uint64_t>(2) << 61;
+}
+constexpr uint32_t kInstr = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kN >> 3) << 17) | (static_cast<uint32_t>(kM >> 4) << 24);
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b),
+                 "r"(kInstr), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void load16(uint32_t at, uint32_t* x) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]), "=r"(x[9]), "=r"(x[10]),
+                   "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
+                 : "r"(at)
+                 : "memory");
+}
+// relu(x)^2 of two sums, rounded to bfloat16 before (what the linear layer returns) and after
+__device__ __forceinline__ uint32_t relu_square2(uint32_t a, uint32_t b) {
+    const float2 x = __bfloat1622float2(__floats2bfloat162_rn(__uint_as_float(a), __uint_as_float(b)));
+    // x < 0 ? 0 : x keeps NaN
+    const float p = x.x < 0.f ? 0.f : x.x, q = x.y < 0.f ? 0.f : x.y;
+    const __nv_bfloat162 r = __floats2bfloat162_rn(p * p, q * q);
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+linear_relu_square_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mo,
+                          int m_tiles, int n_tiles, int k_blocks, unsigned* mirror) {
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t stages = (smem_u32(smem_raw) + 1023u) & ~1023u, out = stages + kStages * kStageBytes;
+    Bars& s = *reinterpret_cast<Bars*>(smem_raw + (out + 2 * kBoxBytes - smem_u32(smem_raw)));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tiles = m_tiles * n_tiles;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStages; ++i) {
+            sm100::mbar_init(s.full + i, 1);
+            sm100::mbar_init(s.empty + i, 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            sm100::mbar_init(s.done + i, 1);
+            sm100::mbar_init(s.taken + i, 4);
+        }
+        sm100::mbar_init(&s.drained, 1);
+        sm100::mbar_init_fence();
+        s.dead = 0u;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s.tmem)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s.tmem;
+    const auto wait = [&](uint64_t* bar, uint32_t parity) {
+        for (uint32_t i = 0; i < kWaitLimit; ++i) {
+            if (sm100::mbar_try_wait(bar, parity)) return true;
+            if (i > 64) {
+                if (s.dead != 0u) return false;
+                __nanosleep(64);
+            }
+        }
+        s.dead = 1u;
+        if (mirror != nullptr) *reinterpret_cast<volatile unsigned*>(mirror) = 1u;
+        return false;
+    };
+    if (warp == 0 && lane == 0) {
+        uint32_t it = 0;
+        bool good = true;
+        for (int tile = blockIdx.x; good && tile < tiles; tile += gridDim.x) {
+            const int m0 = tile / n_tiles * kM, n0 = tile % n_tiles * kN;
+            for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                const uint32_t st = it % kStages;
+                good = wait(s.empty + st, (it / kStages & 1u) ^ 1u);
+                if (!good) break;
+                const uint32_t a = stages + st * kStageBytes;
+                sm100::mbar_expect_tx(s.full + st, kStageBytes);
+                tma_load_2d(a, &mx, s.full + st, kb * kK, m0);
+                tma_load_2d(a + kABytes, &mw, s.full + st, kb * kK, n0);
+            }
+        }
+        // nothing of this CTA is in flight when it goes: its products have read every stage, or at least its copies have landed
+        for (uint32_t j = it > kStages ? it - kStages : 0u; j < it; ++j) {
+            if (good) wait(s.empty + j % kStages, j / kStages & 1u);
+            else sm100::mbar_wait(s.full + j % kStages, j / kStages & 1u, kWaitLimit / 64);
+        }
+    } else if (warp == 1 && lane == 0) {
+        uint32_t it = 0, turn = 0;
+        bool good = true;
+        for (int tile = blockIdx.x; good && tile < tiles; tile += gridDim.x, ++turn) {
+            const uint32_t buf = turn & 1u, d = tmem + buf * kN;
+            good = wait(s.taken + buf, (turn >> 1 & 1u) ^ 1u);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int kb = 0; good && kb < k_blocks; ++kb, ++it) {
+                const uint32_t st = it % kStages;
+                good = wait(s.full + st, it / kStages & 1u);
+                if (!good) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t a = operand(stages + st * kStageBytes), b = operand(stages + st * kStageBytes + kABytes);
+#pragma unroll
+                for (int k = 0; k < kK / 16; ++k) mma(d, a + 2 * k, b + 2 * k, (kb | k) != 0 ? 1u : 0u);      // 16 columns are 32 bytes
+                commit(s.empty + st);
+            }
+            if (good) commit(s.done + buf);
+        }
+        if (!good) {      // products that were issued end before the tensor memory is given back
+            commit(&s.drained);
+            sm100::mbar_wait(&s.drained, 0, kWaitLimit / 64);
+        }
+    } else if (warp >= 2) {
+        const int quadrant = warp & 3, row = quadrant * 32 + lane;      // of the accumulator, as this warp may read it
+        const uint32_t swizzle = row & 7;
+        uint32_t turn = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++turn) {
+            const int m0 = tile / n_tiles * kM, n0 = tile % n_tiles * kN;
+            const uint32_t buf = turn & 1u, d = tmem + (static_cast<uint32_t>(quadrant * 32) << 16) + buf * kN;
+            // all four warps go on or none: they share barriers below
+            bool good = wait(s.done + buf, turn >> 1 & 1u);
+            good = __all_sync(0xffffffffu, good);
+            int all;
+            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}" : "=r"(all) : "r"(good ? 1 : 0) : "memory");
+            if (all == 0) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+            for (int half = 0; half < 2; ++half) {
+                if (threadIdx.x == 64) sm100::tma_store_wait_read();
+                sm100::named_bar_sync(1, 128);      // the boxes are free
+#pragma unroll
+                for (int box = 0; box < 2; ++box) {
+                    uint32_t x[64];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) load16(d + half * 128 + box * 64 + j * 16, x + j * 16);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 64; ++j) asm volatile("" : "+r"(x[j]));
+                    const uint32_t at = out + box * kBoxBytes + row * 128;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t p0 = relu_square2(x[8 * j], x[8 * j + 1]), p1 = relu_square2(x[8 * j + 2], x[8 * j + 3]);
+                        const uint32_t p2 = relu_square2(x[8 * j + 4], x[8 * j + 5]), p3 = relu_square2(x[8 * j + 6], x[8 * j + 7]);
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + ((j ^ swizzle) << 4)), "r"(p0), "r"(p1), "r"(p2), "r"(p3) : "memory");
+                    }
+                }
+                if (half == 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(s.taken + buf);
+                }
+                sm100::fence_proxy_async_smem();
+                sm100::named_bar_sync(1, 128);
+                if (threadIdx.x == 64) {
+                    tma_store_2d(&mo, out, n0 + half * 128, m0);
+                    tma_store_2d(&mo, out + kBoxBytes, n0 + half * 128 + 64, m0);
+                    sm100::tma_store_commit();
+                }
+            }
+        }
+        if (threadIdx.x == 64) sm100::tma_store_wait_all();
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
+static bool allowed(int* sms) {
+    static std::mutex lock;
+    static int state[64] = {};      // 0: not asked, -1: no, else SMs
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
+    std::lock_guard<std::mutex> guard(lock);
+    if (state[dev] == 0) {
+        int n = 0;
+        const bool good = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && tensor_map::encode_fn() != nullptr &&
+                          cudaFuncSetAttribute(reinterpret_cast<const void*>(linear_relu_square_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)) == cudaSuccess;
+        if (!good) cudaGetLastError();
+        state[dev] = good ? n : -1;
+    }
+    *sms = state[dev];
+    return state[dev] > 0;
+}
+
+}  // namespace lineartc
+
+extern "C" int vrwkv_linear_relu_square(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream) {
+    using namespace lineartc;
+    if (rows <= 0 || K <= 0 || N <= 0) return VRWKV_ERR_SHAPE;
+    if (!x || !w || !out) return VRWKV_ERR_NULL;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15u) return VRWKV_ERR_ALIGNMENT;
+    const long long m_tiles = (rows + kM - 1) / kM, tiles = m_tiles * (N / kN);
+    int sms = 0;
+    if (K % kK != 0 || N % kN != 0 || rows > (1LL << 30) || tiles > (1LL << 30) || !allowed(&sms)) return VRWKV_ERR_UNSUPPORTED;
+    tensor_map::bind_primary_context();
+    CUtensorMap mx, mw, mo;
+    if (!tensor_map::make_rows(&mx, x, rows, K, kK, kM) || !tensor_map::make_rows(&mw, w, N, K, kK, kN) || !tensor_map::make_rows(&mo, out, rows, N, 64, kM)) {
+        set_error_detail("cuTensorMapEncodeTiled rejected a matrix");
+        return VRWKV_ERR_DEVICE;
+    }
+    linear_relu_square_kernel<<<static_cast<unsigned>(std::min<long long>(tiles, sms)), kThreads, kSmem, static_cast<cudaStream_t>(stream)>>>(
+        mx, mw, mo, static_cast<int>(m_tiles), N / kN, K / kK, failure_mirror(Op::linear));
+    return record_launches(1);
+}

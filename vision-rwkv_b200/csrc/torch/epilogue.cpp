@@ -1,5 +1,6 @@
 // Host path of the inference-only steps between a block's matrix products (csrc/mixer_epilogue.cu).  The rules that decide
 // whether a call may come here are epilogue.py's.
+#include <ATen/autocast_mode.h>
 #include "glue.h"
 
 namespace vrwkv {
@@ -41,6 +42,20 @@ Tensor relu_square(const Tensor& x_, bool wide) {
     if (x.numel() == 0) return out;
     if (wide) check(vrwkv_relu_square_f32out(x.numel(), static_cast<uint16_t*>(x.data_ptr()), fp(out), stream_of(x)), "vrwkv_relu_square_f32out");
     else check(vrwkv_relu_square(x.numel(), x.data_ptr(), is_bf16(x), out.data_ptr(), stream_of(x)), "vrwkv_relu_square");
+    return out;
+}
+
+Tensor linear_relu_square(const Tensor& x_, const Tensor& weight_) {
+    same_place(x_, weight_, "x");
+    const c10::cuda::CUDAGuard guard(x_.device());
+    TORCH_CHECK(is_bf16(x_) && weight_.dim() == 2 && x_.dim() >= 1 && x_.size(-1) == weight_.size(1), "x must be bfloat16 rows of the weight's width");
+    const Tensor x = flat(x_), weight = flat(at::autocast::cached_cast(at::kBFloat16, weight_, at::kCUDA));      // autocast's own cast, and its cache
+    auto sizes = x.sizes().vec();
+    sizes.back() = weight.size(0);
+    Tensor out = at::empty(sizes, x.options());
+    if (x.numel() == 0) return out;
+    const auto p = [](const Tensor& t) { return static_cast<uint16_t*>(t.data_ptr()); };
+    check(vrwkv_linear_relu_square(x.numel() / x.size(-1), weight.size(1), weight.size(0), p(x), p(weight), p(out), stream_of(x)), "vrwkv_linear_relu_square");
     return out;
 }
 

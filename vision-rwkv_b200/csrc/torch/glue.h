@@ -15,6 +15,8 @@ Tensor norm_gate(const Tensor& x, const Tensor& gate, const Tensor& weight, cons
 // epilogue.cpp
 Tensor sigmoid_gate(const Tensor& r, const Tensor& y, bool wide);      // wide: bfloat16 r, y to a float32 result
 Tensor relu_square(const Tensor& x, bool wide);      // wide: bfloat16 x to a float32 result
+// relu(x weight^T)^2 in bfloat16, as autocast computes it for a linear layer that rounds it
+Tensor linear_relu_square(const Tensor& x, const Tensor& weight);
 Tensor add_rows(const Tensor& table, const Tensor& a);
 Tensor patch_rows(const Tensor& img, int64_t patch);
 Tensor norm_residual(const Tensor& x, const Tensor& a, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,

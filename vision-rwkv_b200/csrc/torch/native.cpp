@@ -33,9 +33,9 @@ void raise_status(int status, const char* what) {
 void raise_failures(int device, const char* what) {
     const unsigned bits = vrwkv_take_failures(device);
     if (bits == 0) return;
-    static const char* const kNames[] = {"Bi-WKV forward", "Bi-WKV backward", "WKV6 forward", "WKV6 backward"};
+    static const char* const kNames[] = {"Bi-WKV forward", "Bi-WKV backward", "WKV6 forward", "WKV6 backward", "linear"};
     std::string names;
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 5; ++i)
         if (bits >> (8 + i) & 1u) names += (names.empty() ? "" : ", ") + std::string(kNames[i]);
     char word[16];
     snprintf(word, sizeof(word), "%#x", bits & 0xffu);
@@ -375,6 +375,7 @@ PYBIND11_MODULE(_native, m) {
     });
     m.def("sigmoid_gate", [](const Tensor& r, const Tensor& y, bool wide) { return vrwkv::guarded([&] { return vrwkv::sigmoid_gate(r, y, wide); })(); });
     m.def("relu_square", [](const Tensor& x, bool wide) { return vrwkv::guarded([&] { return vrwkv::relu_square(x, wide); })(); });
+    m.def("linear_relu_square", [](const Tensor& x, const Tensor& weight) { return vrwkv::guarded([&] { return vrwkv::linear_relu_square(x, weight); })(); });
     m.def("add_rows", [](const Tensor& table, const Tensor& a) { return vrwkv::guarded([&] { return vrwkv::add_rows(table, a); })(); });
     m.def("patch_rows", [](const Tensor& img, int64_t patch) { return vrwkv::guarded([&] { return vrwkv::patch_rows(img, patch); })(); });
     m.def("norm_residual", [](const Tensor& x, const Tensor& a, std::optional<Tensor> weight, std::optional<Tensor> bias,

@@ -10,7 +10,7 @@ void set_error_detail(const char* text);
 int record_launches(int launched);
 // Host-visible word of the current device and operator that kernels set when a bounded wait runs out (pinned, mapped;
 // null until vrwkv_take_failures() has been called once).  It costs a successful launch nothing.
-enum class Op { biwkv_forward, biwkv_backward, wkv6_forward, wkv6_backward };
+enum class Op { biwkv_forward, biwkv_backward, wkv6_forward, wkv6_backward, linear };
 unsigned* failure_mirror(Op op);
 
 #ifdef __CUDACC__

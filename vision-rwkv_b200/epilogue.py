@@ -30,6 +30,16 @@ def relu_square(x, layer=None):
     return _lib.native().relu_square(x, wide)
 
 
+def linear_relu_square(key, x, layer=None):
+    """relu_square(key(x), layer), the linear layer and what follows it in one kernel where `layer` rounds the result to bfloat16 anyway."""
+    if layer is not None and x.dtype == torch.bfloat16 and _inference(x) and autocast_linears(key, layer) and key.bias is None:
+        w = key.weight
+        if (type(w) in (nn.Parameter, torch.Tensor) and w.dtype in KERNEL_DTYPES and w.device == x.device and w.dim() == 2 and w.shape[1] == x.shape[-1]
+                and w.shape[1] % 64 == 0 and w.shape[1] > 0 and w.shape[0] % 256 == 0 and w.shape[0] > 0):
+            return _lib.native().linear_relu_square(x, w)
+    return relu_square(key(x), layer)
+
+
 def sigmoid_gate(r, y, norm=None):
     """sigmoid(r) * y in the dtype of r (vrwkv.py:182-187, 253-257).  For a LayerNorm `norm` that takes it under autocast, where torch
     widens a bfloat16 result to float32 first, it leaves widened."""

@@ -20,7 +20,7 @@ CHECK_STATUS = False
 # Without CHECK_STATUS a failed launch is still reported, one or more calls late and with no synchronisation: the
 # kernel that gives up a wait writes a word of mapped host memory (one per device and operator), and the next call into
 # this module (or `raise_if_failed()`) reads it and raises.
-OPERATORS = ("Bi-WKV forward", "Bi-WKV backward", "WKV6 forward", "WKV6 backward")     # bits 8.. of vrwkv_take_failures
+OPERATORS = ("Bi-WKV forward", "Bi-WKV backward", "WKV6 forward", "WKV6 backward", "linear")     # bits 8.. of vrwkv_take_failures
 
 
 def _raise_failures(lib, index, what):
