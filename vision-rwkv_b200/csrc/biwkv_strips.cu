@@ -1149,7 +1149,9 @@ static float plan_cost(int T, bool bwd, Types types, const Plan& pl) {
     const float waste = static_cast<float>(pl.cluster * pl.n_tok) / static_cast<float>(T);
     const float idle = 1.f + 0.4f * static_cast<float>(most - held) / static_cast<float>(most);
     // more CTAs: float32 backward of 10, 12, 16 CTAs 544 (5000 tokens), 593, 633; forward 226, 241, 259
-    const float hand_over = (bwd ? kBackward : kForward)[std::min(pl.cluster, 8) - 1] + (bwd ? 0.05f : 0.025f) * static_cast<float>(std::max(pl.cluster - 8, 0));
+    const float* const by_cluster = bwd ? kBackward : kForward;
+    const int most_listed = 8, listed = pl.cluster < most_listed ? pl.cluster : most_listed;
+    const float hand_over = by_cluster[listed - 1] + (bwd ? 0.05f : 0.025f) * static_cast<float>(pl.cluster - listed);
     const float narrow = pl.cs == 16 ? 1.f : types == Types::f32 ? (bwd ? 1.04f : 1.19f) : (bwd ? 1.14f : 1.09f);
     return waste * idle * hand_over * narrow;
 }
