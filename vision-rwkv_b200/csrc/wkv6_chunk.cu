@@ -625,9 +625,24 @@ __device__ __forceinline__ void pair_outputs(float (&y)[2][2][4], const __nv_bfl
                 }
     }
 #pragma unroll
-    for (int b = 0; b < kBlocks; ++b)
+    for (int b = 0; b < kBlocks; ++b) {
+        uint32_t r[kZ][4];      // the values of block b, for both tiles
 #pragma unroll
-        for (int m = 0; m < 2; ++m) prod_slice<kX, kZ, false>(y[m], pairs, 2 * th + m, b, values, b, cs, lane);
+        for (int ib = 0; ib < kZ; ++ib) ldsm4t(r[ib], smem_addr(values + ib * kPlane + b * kBlock * kRow + cs * 16 + off_pos(lane)));
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int ia = 0; ia < kX; ++ia) {
+                uint32_t a[4];
+                ldsm4(a, smem_addr(pairs + ia * kPlane + (2 * th + m) * kBlock * kRow + b * kBlock + off_a(lane)));
+#pragma unroll
+                for (int ib = 0; ib < kZ; ++ib)
+                    if (Keep<kX, kZ>::on(ia, ib)) {
+                        mma(y[m][0], a, r[ib][0], r[ib][1]);
+                        mma(y[m][1], a, r[ib][2], r[ib][3]);
+                    }
+            }
+    }
 }
 
 // ---- kernel 2 ------------------------------------------------------------------------------------------------
@@ -781,6 +796,10 @@ __device__ __forceinline__ void slice_gradient(float (&out)[2][2][2][4], const _
             row4(tab[j * kBlock + kBlock - 1], cs, q, d);
 #pragma unroll
             for (int e = 0; e < 4; ++e) d[e] = ex2(d[e]);
+            // the partners' rows of block j, for both tiles of this warp
+            uint32_t r[kX][4];
+#pragma unroll
+            for (int ib = 0; ib < kX; ++ib) ldsm4t(r[ib], smem_addr(pl + ib * kPlane + j * kBlock * kRow + cs * 16 + off_pos(lane)));
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt) {
                 const int blk = 2 * th + mt;
@@ -790,15 +809,13 @@ __device__ __forceinline__ void slice_gradient(float (&out)[2][2][2][4], const _
                 for (int half = 0; half < 2; ++half)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) c[mt][e >> 1][2 * half + (e & 1)] *= d[e];
-                if (j != blk) {
-                    prod_slice<kX, kX, kTransM>(c[mt], m, blk, j, pl, j, cs, lane);
-                } else {
-                    // the block's own tile, masked to this direction
-                    uint32_t a[kX][4];
+                uint32_t a[kX][4];
 #pragma unroll
-                    for (int ia = 0; ia < kX; ++ia) {
-                        if (kTransM) ldsm4t(a[ia], smem_addr(m + ia * kPlane + blk * kBlock * kRow + blk * kBlock + off_tok(lane)));
-                        else ldsm4(a[ia], smem_addr(m + ia * kPlane + blk * kBlock * kRow + blk * kBlock + off_a(lane)));
+                for (int ia = 0; ia < kX; ++ia) {
+                    if (kTransM) ldsm4t(a[ia], smem_addr(m + ia * kPlane + j * kBlock * kRow + blk * kBlock + off_tok(lane)));
+                    else ldsm4(a[ia], smem_addr(m + ia * kPlane + blk * kBlock * kRow + j * kBlock + off_a(lane)));
+                    if (j == blk) {
+                        // the block's own tile, masked to this direction
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const int row = g + 8 * (i & 1), col = 2 * q + 8 * (i >> 1);
@@ -807,18 +824,15 @@ __device__ __forceinline__ void slice_gradient(float (&out)[2][2][2][4], const _
                             a[ia][i] &= keep;
                         }
                     }
-#pragma unroll
-                    for (int ib = 0; ib < kX; ++ib) {
-                        uint32_t r[4];
-                        ldsm4t(r, smem_addr(pl + ib * kPlane + blk * kBlock * kRow + cs * 16 + off_pos(lane)));
-#pragma unroll
-                        for (int ia = 0; ia < kX; ++ia)
-                            if (Keep<kX, kX>::on(ia, ib)) {
-                                mma(c[mt][0], a[ia], r[0], r[1]);
-                                mma(c[mt][1], a[ia], r[2], r[3]);
-                            }
-                    }
                 }
+#pragma unroll
+                for (int ib = 0; ib < kX; ++ib)
+#pragma unroll
+                    for (int ia = 0; ia < kX; ++ia)
+                        if (Keep<kX, kX>::on(ia, ib)) {
+                            mma(c[mt][0], a[ia], r[ib][0], r[ib][1]);
+                            mma(c[mt][1], a[ia], r[ib][2], r[ib][3]);
+                        }
             }
         }
 #pragma unroll

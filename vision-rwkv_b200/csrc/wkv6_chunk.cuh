@@ -136,29 +136,6 @@ __device__ __forceinline__ void prod_tokens(float (&c)[2][4], const AFrag<NA>& a
         }
     }
 }
-// C[16 x 16 positions] += M(16 x 16 tokens) * X(rows of block `b`, positions 16 cs ..): one 16-byte ldmatrix row each
-template <int NM, int NX, bool kTransM>
-__device__ __forceinline__ void prod_slice(float (&c)[2][4], const __nv_bfloat16* m, int mrow, int mcol, const __nv_bfloat16* x, int b, int cs,
-                                           int lane) {
-    uint32_t a[NM][4];
-#pragma unroll
-    for (int ia = 0; ia < NM; ++ia) {
-        // the 16 x 16 tile (mrow, mcol) as an A fragment; kTransM: of the transposed matrix
-        if (kTransM) ldsm4t(a[ia], smem_addr(m + ia * kPlane + mcol * kBlock * kRow + mrow * kBlock + off_tok(lane)));
-        else ldsm4(a[ia], smem_addr(m + ia * kPlane + mrow * kBlock * kRow + mcol * kBlock + off_a(lane)));
-    }
-#pragma unroll
-    for (int ib = 0; ib < NX; ++ib) {
-        uint32_t r[4];
-        ldsm4t(r, smem_addr(x + ib * kPlane + b * kBlock * kRow + cs * 16 + off_pos(lane)));
-#pragma unroll
-        for (int ia = 0; ia < NM; ++ia)
-            if (Keep<NM, NX>::on(ia, ib)) {
-                mma(c[0], a[ia], r[0], r[1]);
-                mma(c[1], a[ia], r[2], r[3]);
-            }
-    }
-}
 // One k-step (positions 16 kk ..) of a slice of a state, from global memory: the B fragments of the two 8-column halves.
 // kTrans: the stored state's rows and columns are exchanged.
 template <int NB, bool kTrans>
