@@ -335,7 +335,8 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
  *     (CLS/vrwkv.py:250-251); K % 64 == 0, N % 256 == 0, else VRWKV_ERR_UNSUPPORTED
  *   vrwkv_norm_residual: out = x + gamma * (normalise(a) * weight + bias) over rows of C <= 1024 channels, C % 4 == 0;
  *     weight and bias NULL: out = x + gamma * a; gamma NULL: 1 (CLS/vrwkv.py:297-318)
- *   vrwkv_gated_norm_residual: the same with a = sigmoid(r) * y, all bfloat16
+ *   vrwkv_layer_norm: out = normalise(x) * weight + bias over such rows
+ *   vrwkv_gated_norm_residual: the same as norm_residual with a = sigmoid(r) * y, all bfloat16
  *   vrwkv_head_norm_gate_bf16out: vrwkv_normgate_forward_f32 with group 64, the result rounded to bfloat16
  *   vrwkv_add_rows: out[i] = table[i mod period] + a[i], a bfloat16, float32 result; period a multiple of 8 that divides n
  *     (CLS/vrwkv.py:392, CLS/vrwkv6.py:200)
@@ -349,6 +350,7 @@ int vrwkv_relu_square_f32out(long long n, const uint16_t* x, float* out, void* s
 int vrwkv_linear_relu_square(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream);
 int vrwkv_add_rows(long long n, long long period, const float* table, const uint16_t* a, float* out, void* stream);
 int vrwkv_patch_rows(int B, int channels, int H, int W, int patch, const float* img, uint16_t* out, void* stream);
+int vrwkv_layer_norm(int rows, int C, float eps, const float* x, const float* weight, const float* bias, float* out, void* stream);
 int vrwkv_norm_residual(int rows, int C, float eps, const void* a, int a_is_bf16, const float* weight, const float* bias,
                         const float* gamma, const float* x, float* out, void* stream);
 int vrwkv_gated_norm_residual(int rows, int C, float eps, const uint16_t* r, const uint16_t* y, const float* weight, const float* bias,

@@ -1,0 +1,27 @@
+"""The plain LayerNorm of the networks in inference, against float64: float32 sums over up to 1024 channels, 1e-6 in the 2-norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,C", [(1, 4), (7, 128), (9, 132), (1000, 384), (33, 1024)])
+def test_against_float64(cuda_device, rows, C):
+    from vision_rwkv_b200 import epilogue, launch_count
+    norm = torch.nn.LayerNorm(C, device=cuda_device)
+    torch.nn.init.normal_(norm.weight)
+    torch.nn.init.normal_(norm.bias)
+    x = torch.randn(rows, C, device=cuda_device) * 3 + 5
+    with torch.no_grad():
+        before = launch_count()
+        got = epilogue.layer_norm(norm, x)
+        assert launch_count() == before + 1
+        ref = torch.nn.functional.layer_norm(x.double(), (C,), norm.weight.double(), norm.bias.double(), norm.eps)
+        assert ((got - ref).norm() / ref.norm()).item() <= 1e-6
+        # a hook, another type and gradients keep the layer's call
+        seen = []
+        hook = norm.register_forward_hook(lambda *a: seen.append(1))
+        epilogue.layer_norm(norm, x)
+        hook.remove()
+        assert seen == [1] and launch_count() == before + 1
+    assert epilogue.layer_norm(norm, x).requires_grad

@@ -118,7 +118,7 @@ class Block(nn.Module):
 
     def _inner(self, x, resolution):
         if self.layer_id == 0:
-            x = self.ln0(x)
+            x = epilogue.layer_norm(self.ln0, x)
         g1 = self.gamma1 if self.layer_scale else None
         g2 = self.gamma2 if self.layer_scale else None
         # inference: the gate that ends the channel mix goes with the residual
@@ -128,10 +128,10 @@ class Block(nn.Module):
             if split:
                 return epilogue.gated_residual(x, *self.ffn.gate_operands(x, resolution), self.ln2, g2)
             return epilogue.norm_residual(x, self.ffn(x, resolution), self.ln2, g2)
-        x = epilogue.residual(x, self.att(self.ln1(x), resolution), g1)
+        x = epilogue.residual(x, self.att(epilogue.layer_norm(self.ln1, x), resolution), g1)
         if split:
-            return epilogue.gated_residual(x, *self.ffn.gate_operands(self.ln2(x), resolution), None, g2)
-        return epilogue.residual(x, self.ffn(self.ln2(x), resolution), g2)
+            return epilogue.gated_residual(x, *self.ffn.gate_operands(epilogue.layer_norm(self.ln2, x), resolution), None, g2)
+        return epilogue.residual(x, self.ffn(epilogue.layer_norm(self.ln2, x), resolution), g2)
 
     def forward(self, x, resolution):
         if self.with_cp and x.requires_grad:
@@ -197,7 +197,7 @@ class VRWKV(nn.Module):
         for i, layer in enumerate(self.layers):
             x = layer(x, resolution)
             if i == len(self.layers) - 1 and self.final_norm:
-                x = self.ln1(x)
+                x = epilogue.layer_norm(self.ln1, x)
             if i in self.out_indices:
                 outs.append(x.reshape(x.shape[0], *resolution, x.shape[2]).permute(0, 3, 1, 2))
         return tuple(outs)

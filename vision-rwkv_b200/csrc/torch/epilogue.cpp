@@ -119,6 +119,18 @@ Tensor norm_residual_of(const Tensor& x_, const Tensor& a_, const Tensor* r_, co
 
 }  // namespace
 
+Tensor layer_norm(const Tensor& x_, const Tensor& weight_, const Tensor& bias_, double eps) {
+    same_place(weight_, x_, "weight");
+    same_place(bias_, x_, "bias");
+    const int64_t C = x_.size(-1), rows = C ? x_.numel() / C : 0;
+    TORCH_CHECK(x_.scalar_type() == at::kFloat && weight_.numel() == C && bias_.numel() == C, "x must be float32; weight and bias must hold C values");
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = flat(x_), weight = flat(f32(weight_)), bias = flat(f32(bias_));
+    Tensor out = at::empty(x.sizes(), x.options());
+    if (x.numel() != 0) check(vrwkv_layer_norm(rows, C, static_cast<float>(eps), fp(x), fp(weight), fp(bias), fp(out), stream_of(x)), "vrwkv_layer_norm");
+    return out;
+}
+
 Tensor norm_residual(const Tensor& x, const Tensor& a, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
                      const std::optional<Tensor>& gamma, double eps) {
     return norm_residual_of(x, a, nullptr, weight, bias, gamma, eps);

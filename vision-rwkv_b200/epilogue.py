@@ -66,6 +66,15 @@ def _norm_kernel(a, norm, C):
             and norm.weight.dtype == norm.bias.dtype == torch.float32 and (a.dtype == torch.float32 or torch.is_autocast_enabled("cuda")))
 
 
+def layer_norm(norm, x):
+    """norm(x) for a LayerNorm `norm` over the channels"""
+    C = x.shape[-1]
+    if (_inference(x) and x.dtype == torch.float32 and C % 4 == 0 and 0 < C <= MOST_NORM_CHANNELS and x.numel() // C < 2 ** 31
+            and _norm_kernel(x, norm, C)):
+        return _lib.native().layer_norm(x, norm.weight, norm.bias, norm.eps)
+    return norm(x)
+
+
 def norm_residual(x, a, norm, gamma):
     """x + gamma * norm(a) for a LayerNorm `norm` (post-norm blocks).  Under autocast torch computes that norm in float32."""
     if _residual_kernel(x, a, gamma) and _norm_kernel(a, norm, x.shape[-1]):
