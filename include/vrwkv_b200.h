@@ -51,9 +51,9 @@ const char* vrwkv_last_error_detail(void);
 unsigned long long vrwkv_launch_count(void);
 
 /* Kernel path selection, for tests and measurements: 0 = automatic (default: Bi-WKV takes the
- * cluster-resident kernels when T <= 32768, C % 4 == 0 (bfloat16: C % 8 == 0) and the
- * tensors are 16-byte aligned - one cluster per sequence strip up to T = 4096, above it several or, for
- * many tokens in all, separate launches -,
+ * kernels that hold sequences in shared memory when T <= 32768, C % 4 == 0 (bfloat16: C % 8 == 0) and the
+ * tensors are 16-byte aligned - one CTA or cluster per sequence strip where vrwkv_biwkv_one_pass is 1, else several
+ * clusters or, for many tokens in all, separate launches -,
  * else the persistent tile kernels, else the generic multi-launch path), 1 = the
  * first-generation kernels (Bi-WKV: the generic multi-launch path; vrwkv_wkv6_forward_tc_*: the walk
  * that needs no scratch memory, whatever the workspace holds), 2 = Bi-WKV skips the
@@ -114,8 +114,8 @@ int vrwkv_biwkv_backward_f32(int B, int T, int C, const float* w, const float* u
  * scratch tensors (bi_wkv_kernel.cu:259-302, 415-417).  Here the forward can write log Den_t next
  * to y (one extra float per element), and vrwkv_biwkv_backward_saved_f32 takes k, v, gy and the
  * saved y, log Den: it needs one cross-tile exchange instead of two, at the price of keeping logden
- * (B*T*C floats) from forward to backward.  The pair runs on the tile kernels; for T <= 4096 the
- * cluster-resident vrwkv_biwkv_forward_f32 + vrwkv_biwkv_backward_f32, which keep nothing, are
+ * (B*T*C floats) from forward to backward.  The pair runs on the tile kernels; where vrwkv_biwkv_one_pass
+ * is 1 vrwkv_biwkv_forward_f32 + vrwkv_biwkv_backward_f32, which keep nothing, are
  * about twice as fast.  Results agree with the recomputing pair to float32 rounding.  Same workspace sizes.  Both are
  * served by the single-pass TMA kernels only (C % 4 == 0, 16-byte aligned tensors, T below about
  * 37 000); otherwise they return VRWKV_ERR_UNSUPPORTED and nothing ran. */
@@ -162,7 +162,7 @@ int vrwkv_biwkv_one_pass(int B, int T, int C, int tensors);
  * rebuilding them: two passes over the inputs instead of three.  vrwkv_biwkv_kept_bytes is 0 where a backward has no use for
  * them (T <= 4096, or few tokens in all); where vrwkv_biwkv_one_pass is 1 the entry points above are faster.
  * w, u, k, v of the backward must be those of the forward.  `tensors` says what k, v, y, gy, gk, gv hold (enum below, as in the
- * entry points above; VRWKV_TENSORS_BF16_WIDE is refused at present: no kernels for it above 4096 tokens).  The workspaces hold neither
+ * entry points above; VRWKV_TENSORS_BF16_WIDE is refused: only the kernels that keep nothing take it).  The workspaces hold neither
  * the states nor room for the other paths: vrwkv_biwkv_kept_workspace_bytes bytes, 0 where nothing is kept (those of the other entry
  * points are larger and serve too).  VRWKV_ERR_UNSUPPORTED: outside the cluster-resident
  * kernels (shape, alignment, vrwkv_set_path), nothing ran, use the other entry points; a forward may succeed and the backward

@@ -38,8 +38,8 @@
 // tiles are waited for but the steps of the arithmetic.
 //
 // Arithmetic, exactness and the exact kernel: plain floats without exponent shift, safe whenever 2 max|k| + |u| + |w| + max(-w, 0) T
-// <= 60 (T in whole walkers); each thread checks its own tokens, the first exchange carries the OR, and units that fail go to
-// biwkv_exact_kernel's list (per-token max-shifted arithmetic, launched behind, returns at once when the list is empty).  Decays over
+// <= 60 (T in whole walkers); each thread checks its own tokens, the first exchange carries the OR, and every CTA leaves a word that
+// says whether its unit is left to biwkv_exact_kernel (per-token max-shifted arithmetic, launched behind).  Decays over
 // half a walker and more come from double precision.
 //
 // Recurrence restated: classification/mmcls_custom/models/backbones/cuda_new/bi_wkv_kernel.cu:21-116 (forward), :119-367

@@ -796,7 +796,8 @@ __device__ __forceinline__ void slice_gradient(float (&out)[2][2][2][4], const _
             row4(tab[j * kBlock + kBlock - 1], cs, q, d);
 #pragma unroll
             for (int e = 0; e < 4; ++e) d[e] = ex2(d[e]);
-            // the partners' rows of block j, for both tiles of this warp
+            // the partners' rows of block j, for both tiles of this warp: read per tile the backward was 157.3 us, now 154.6
+            // (B=32, H=12, T=196; T=4096 2316 and 2304)
             uint32_t r[kX][4];
 #pragma unroll
             for (int ib = 0; ib < kX; ++ib) ldsm4t(r[ib], smem_addr(pl + ib * kPlane + j * kBlock * kRow + cs * 16 + off_pos(lane)));

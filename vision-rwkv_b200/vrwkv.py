@@ -32,9 +32,9 @@ import torch
 from . import _lib, ops, traced
 
 BF16_IO = os.environ.get("VRWKV_BF16_IO", "1") != "0"
-# Off by default: up to 4096 tokens the forward keeps nothing and the backward rebuilds y and Den inside the
-# cluster-resident kernel, which reads k, v, gy once; for many longer sequences the C++ autograd node keeps the states
-# entering every 16 tokens (1.5 bytes per element).  These are the fastest pairs.  When on,
+# Off by default: up to 4096 tokens, and for many longer sequences, the forward keeps nothing and the backward rebuilds
+# y and Den inside its kernel, which reads k, v, gy once; between the two lie calls for which the C++ autograd node keeps
+# the states entering every 16 tokens (1.5 bytes per element).  These are the fastest pairs.  When on,
 # the float32 forward also writes log Den_t (one float per element) and the backward starts from the
 # saved y and log Den: B*T*C floats of extra activation memory per call, served by the older tile
 # kernels; useful only for sequences longer than the resident kernels serve (32768 tokens).
