@@ -340,6 +340,7 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
  *   vrwkv_head_norm_gate_bf16out: vrwkv_normgate_forward_f32 with group 64, the result rounded to bfloat16
  *   vrwkv_add_rows: out[i] = table[i mod period] + a[i], a bfloat16, float32 result; period a multiple of 8 that divides n
  *     (CLS/vrwkv.py:392, CLS/vrwkv6.py:200)
+ *   vrwkv_widen: out = a as float32; n a multiple of 8
  *   vrwkv_patch_rows: img (B, channels, H, W) to (B, H / patch, W / patch, channels, patch, patch) in bfloat16, whole patches only;
  *     patch % 8 == 0, W % 4 == 0 (the operand of the patch embedding, CLS/vrwkv.py:357)
  * Sigmoid, its product and y are rounded to bfloat16 where r is.  All tensors 16-byte aligned. */
@@ -349,6 +350,7 @@ int vrwkv_relu_square(long long n, const void* x, int is_bf16, void* out, void* 
 int vrwkv_relu_square_f32out(long long n, const uint16_t* x, float* out, void* stream);
 int vrwkv_linear_relu_square(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream);
 int vrwkv_add_rows(long long n, long long period, const float* table, const uint16_t* a, float* out, void* stream);
+int vrwkv_widen(long long n, const uint16_t* a, float* out, void* stream);
 int vrwkv_patch_rows(int B, int channels, int H, int W, int patch, const float* img, uint16_t* out, void* stream);
 int vrwkv_layer_norm(int rows, int C, float eps, const float* x, const float* weight, const float* bias, float* out, void* stream);
 int vrwkv_norm_residual(int rows, int C, float eps, const void* a, int a_is_bf16, const float* weight, const float* bias,

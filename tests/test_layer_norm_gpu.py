@@ -25,3 +25,19 @@ def test_against_float64(cuda_device, rows, C):
         hook.remove()
         assert seen == [1] and launch_count() == before + 1
     assert epilogue.layer_norm(norm, x).requires_grad
+
+
+@pytest.mark.parametrize("n", [8, 2048, 2056, 12544 * 768])
+def test_a_widened_input_is_torchs_cast(cuda_device, n):
+    from vision_rwkv_b200 import epilogue, launch_count
+    norm = torch.nn.LayerNorm(8, device=cuda_device)
+    a = torch.randn(n // 8, 8, device=cuda_device).bfloat16()
+    a.view(-1)[:3] = torch.tensor([float("nan"), float("-inf"), -0.0])
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        before = launch_count()
+        got = epilogue.widened(norm, a)
+        assert launch_count() == before + 1 and got.dtype == torch.float32
+        assert torch.equal(got.view(torch.int32), a.float().view(torch.int32))
+        assert epilogue.widened(norm, a[:, :5]).dtype == torch.bfloat16
+        assert epilogue.widened(torch.nn.GroupNorm(8, 8), a) is a
+    assert epilogue.widened(norm, a) is a       # no autocast: the layer refuses or takes it as it is

@@ -161,7 +161,7 @@ class BlockV6(nn.Module):
         # inference: the gate that ends the channel mix goes with the residual, or leaves in the norm's type
         split = epilogue.takes_gate_of(self.ffn, ChannelMixV6)
         if self.post_norm:
-            x = epilogue.residual(x, self.ln1(self.att(x, resolution)), g1)
+            x = epilogue.residual(x, self.ln1(epilogue.widened(self.ln1, self.att(x, resolution))), g1)
             a = epilogue.sigmoid_gate(*self.ffn.gate_operands(x, resolution), norm=self.ln2) if split else self.ffn(x, resolution)
             return epilogue.residual(x, self.ln2(a), g2)
         x = epilogue.residual(x, self.att(self.ln1(x), resolution), g1)

@@ -7,6 +7,7 @@
 //   head_norm_gate  (GroupNorm per 64-channel head) * activation(gate)     vrwkv6.py:133, 205-212, bfloat16 result
 //
 //   add_rows        rows of a table, repeated, plus bfloat16 a, in float32  vrwkv.py:392 (positions), vrwkv6.py:200 (decay)
+//   widen           bfloat16 as float32                                   what autocast puts in front of a LayerNorm
 //   patch_rows      an image's patches as bfloat16 rows of a matrix         the operand of the patch embedding, vrwkv.py:357
 //
 // All are bound by HBM.  Bytes per element under bfloat16 autocast, the tensor-op chains against these: the gate 4 + 6 + 6
@@ -123,6 +124,15 @@ __global__ void __launch_bounds__(kThreads) add_rows_kernel(unsigned vectors, un
     store(out + static_cast<size_t>(i) * kVec, v);
 }
 
+// HBM-bound: 12544 x 768 take 11.4 us (5.1 TB/s), torch's cast 21; the matrix-state base model on 64 images 9.62 -> 9.49 ms.
+__global__ void __launch_bounds__(kThreads) widen_kernel(unsigned vectors, const __nv_bfloat16* __restrict__ a, float* __restrict__ out) {
+    const unsigned i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= vectors) return;
+    float v[kVec];
+    load(a + static_cast<size_t>(i) * kVec, v);
+    store(out + static_cast<size_t>(i) * kVec, v);
+}
+
 // Row (b, h, w) of `out` holds the patch at (h, w) of image b in the order channel, row, column, which is that of a
 // convolution's weights: a patch embedding (kernel = stride) is then one matrix product.  A thread moves 8 pixels of an
 // image row; reads are contiguous over the whole image, writes are whole 32-byte sectors.  With the library's
@@ -148,8 +158,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // One warp per row, lane = 4 channels of each 128; kIters = ceil(C / 128).  Both inputs of a row are requested before the
 // first sum, so 6 C bytes per warp are in flight.  kGate: a holds y and `gate` r of a gate, whose result is rounded as
-// sigmoid_gate_kernel stores it; x null: the norm alone (50176 x 384: 95 us by torch's kernel): 12 bytes per element instead of 6 + 10 and a launch (the small
-// model on 256 images 6.80 -> 6.70 ms).
+// sigmoid_gate_kernel stores it: 12 bytes per element instead of 6 + 10 and a launch (the small model on 256 images 6.80 -> 6.70
+// ms).  x null: the norm alone (50176 x 384: 24 us, torch's kernel 95).
 template <typename A, int kIters, bool kGate>
 __global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C, float eps, const A* __restrict__ a, const A* __restrict__ gate,
                                                                  const float* __restrict__ weight,
@@ -357,6 +367,17 @@ extern "C" int vrwkv_add_rows(long long n, long long period, const float* table,
     const unsigned vectors = static_cast<unsigned>(n / kVec);
     add_rows_kernel<<<(vectors + kThreads - 1) / kThreads, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         vectors, static_cast<unsigned>(period / kVec), table, reinterpret_cast<const __nv_bfloat16*>(a), out);
+    return record_launches(1);
+}
+
+extern "C" int vrwkv_widen(long long n, const uint16_t* a, float* out, void* stream) {
+    using namespace epilogue;
+    if (n <= 0) return VRWKV_ERR_SHAPE;
+    if (!a || !out) return VRWKV_ERR_NULL;
+    if (n % kVec != 0 || n / kVec > 0x7fffffffLL - kThreads) return VRWKV_ERR_UNSUPPORTED;
+    if (misaligned({a, out})) return VRWKV_ERR_ALIGNMENT;
+    const unsigned vectors = static_cast<unsigned>(n / kVec);
+    widen_kernel<<<(vectors + kThreads - 1) / kThreads, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(vectors, reinterpret_cast<const __nv_bfloat16*>(a), out);
     return record_launches(1);
 }
 

@@ -71,6 +71,16 @@ Tensor add_rows(const Tensor& table_, const Tensor& a_) {
     return out;
 }
 
+Tensor widen(const Tensor& a_) {
+    same_place(a_, a_, "a");
+    TORCH_CHECK(is_bf16(a_), "a must be bfloat16");
+    const c10::cuda::CUDAGuard guard(a_.device());
+    const Tensor a = flat(a_);
+    Tensor out = at::empty(a.sizes(), a.options().dtype(at::kFloat));
+    if (a.numel() != 0) check(vrwkv_widen(a.numel(), static_cast<uint16_t*>(a.data_ptr()), fp(out), stream_of(a)), "vrwkv_widen");
+    return out;
+}
+
 Tensor patch_rows(const Tensor& img_, int64_t patch) {
     same_place(img_, img_, "img");
     TORCH_CHECK(img_.dim() == 4 && img_.scalar_type() == at::kFloat && patch > 0, "img must be (B, channels, H, W) in float32");

@@ -19,6 +19,7 @@ Tensor relu_square(const Tensor& x, bool wide);      // wide: bfloat16 x to a fl
 Tensor linear_relu_square(const Tensor& x, const Tensor& weight);
 Tensor add_rows(const Tensor& table, const Tensor& a);
 Tensor patch_rows(const Tensor& img, int64_t patch);
+Tensor widen(const Tensor& a);
 Tensor layer_norm(const Tensor& x, const Tensor& weight, const Tensor& bias, double eps);
 Tensor norm_residual(const Tensor& x, const Tensor& a, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias,
                      const std::optional<Tensor>& gamma, double eps);

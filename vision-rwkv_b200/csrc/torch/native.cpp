@@ -378,6 +378,7 @@ PYBIND11_MODULE(_native, m) {
     m.def("linear_relu_square", [](const Tensor& x, const Tensor& weight) { return vrwkv::guarded([&] { return vrwkv::linear_relu_square(x, weight); })(); });
     m.def("add_rows", [](const Tensor& table, const Tensor& a) { return vrwkv::guarded([&] { return vrwkv::add_rows(table, a); })(); });
     m.def("patch_rows", [](const Tensor& img, int64_t patch) { return vrwkv::guarded([&] { return vrwkv::patch_rows(img, patch); })(); });
+    m.def("widen", [](const Tensor& a) { return vrwkv::guarded([&] { return vrwkv::widen(a); })(); });
     m.def("layer_norm", [](const Tensor& x, const Tensor& weight, const Tensor& bias, double eps) {
         return vrwkv::guarded([&] { return vrwkv::layer_norm(x, weight, bias, eps); })();
     });

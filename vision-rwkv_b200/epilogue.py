@@ -75,6 +75,14 @@ def layer_norm(norm, x):
     return norm(x)
 
 
+def widened(norm, a):
+    """a as a LayerNorm `norm` takes it under autocast: torch widens a bfloat16 input to float32 first."""
+    if (a.dtype == torch.bfloat16 and _inference(a) and a.is_contiguous() and a.numel() % 8 == 0 and a.numel() < 2 ** 33
+            and torch.is_autocast_enabled("cuda") and stock(norm, nn.LayerNorm)):
+        return _lib.native().widen(a)
+    return a
+
+
 def norm_residual(x, a, norm, gamma):
     """x + gamma * norm(a) for a LayerNorm `norm` (post-norm blocks).  Under autocast torch computes that norm in float32."""
     if _residual_kernel(x, a, gamma) and _norm_kernel(a, norm, x.shape[-1]):
