@@ -453,7 +453,7 @@ def sec_sequence_sweep(cx):
         gbs = (BYTES_FWD + BYTES_BWD) * B * T * C / (ms * 1e-3) / 1e9
         rows.append({"T": T, "fwd_ms": f, "bwd_ms": b, "ms": ms, "us_per_token": ms * 1e3 / (B * T),
                      "algorithmic_GBps": gbs, "frac_of_hbm_peak": cx.frac(gbs),
-                     "kernels": "one cluster per sequence strip" if T <= 4096 else "several clusters per sequence strip, aggregates exchanged through global memory"})
+                     "kernels": "one CTA or cluster per sequence strip"})
         del k, v, gy
     return {"B": 8, "C": 768, "dtype": "f32", "per_gpu": True, "rows": rows}
 
