@@ -41,3 +41,16 @@ def test_a_widened_input_is_torchs_cast(cuda_device, n):
         assert epilogue.widened(norm, a[:, :5]).dtype == torch.bfloat16
         assert epilogue.widened(torch.nn.GroupNorm(8, 8), a) is a
     assert epilogue.widened(norm, a) is a       # no autocast: the layer refuses or takes it as it is
+
+
+@pytest.mark.parametrize("C", [192, 384, 768, 1024])
+@pytest.mark.parametrize("mean", [3.0, 100.0])
+def test_rows_with_a_mean_are_no_further_from_float64_than_torchs_layer(cuda_device, C, mean):
+    """4096 rows: the two errors, each an average over millions of roundings, repeat to a few percent; a tenth covers that."""
+    from vision_rwkv_b200 import epilogue
+    norm = torch.nn.LayerNorm(C, device=cuda_device)
+    x = torch.randn(4096, C, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(C)) + mean
+    with torch.no_grad():
+        ref = torch.nn.functional.layer_norm(x.double(), (C,), eps=norm.eps)
+        error = [((y - ref).norm() / ref.norm()).item() for y in (epilogue.layer_norm(norm, x), norm(x))]
+    assert error[0] <= 1.1 * error[1], error

@@ -158,8 +158,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // One warp per row, lane = 4 channels of each 128; kIters = ceil(C / 128).  Both inputs of a row are requested before the
 // first sum, so 6 C bytes per warp are in flight.  kGate: a holds y and `gate` r of a gate, whose result is rounded as
-// sigmoid_gate_kernel stores it: 12 bytes per element instead of 6 + 10 and a launch (the small model on 256 images 6.80 -> 6.70
-// ms).  x null: the norm alone (50176 x 384: 24 us, torch's kernel 95).
+// sigmoid_gate_kernel stores it: 12 bytes per element instead of 6 + 10 and a launch (the small
+// model on 256 images 6.80 -> 6.70 ms).
 template <typename A, int kIters, bool kGate>
 __global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C, float eps, const A* __restrict__ a, const A* __restrict__ gate,
                                                                  const float* __restrict__ weight,
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C
         for (int j = 0; j < 4; ++j) v[i][j] = res[i][j] = 0.f;
         if (128 * i + 4 * lane < C) {
             load(a + base + 128 * i, v[i]);
-            if (x != nullptr) load(x + base + 128 * i, res[i]);
+            load(x + base + 128 * i, res[i]);
             if (kGate) load(gate + base + 128 * i, r[i]);
         }
     }
@@ -222,6 +222,53 @@ __global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C
             float4 o;
             o.x = __fadd_rn(res[i][0], __fmul_rn(g[0], v[i][0])); o.y = __fadd_rn(res[i][1], __fmul_rn(g[1], v[i][1]));
             o.z = __fadd_rn(res[i][2], __fmul_rn(g[2], v[i][2])); o.w = __fadd_rn(res[i][3], __fmul_rn(g[3], v[i][3]));
+            *reinterpret_cast<float4*>(out + base + 128 * i) = o;
+        }
+}
+
+// The norm alone, rows as above.  A mean from one sum is off by its rounding, which on rows whose mean is three times their spread put
+// results 1.35e-7 from float64 (torch's layer 1.07e-7, C = 192 to 768); what rounding left in it is summed up beside the squares and
+// taken off, 5.2e-8 for any mean.  us, torch's layer / the norm as a case of the kernel above / this: 50176 x 384 95 / 25.2 / 24.5,
+// 50176 x 1024 149 / 69.3 / 63.0, 196 x 1024 3.7 / 3.9 / 3.2 (fewer registers and less code).
+template <int kIters>
+__global__ void __launch_bounds__(kThreads) layer_norm_kernel(int rows, int C, float eps, const float* __restrict__ x, const float* __restrict__ weight,
+                                                              const float* __restrict__ bias, float* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const size_t base = static_cast<size_t>(row) * C + 4 * lane;
+    const float inv = 1.f / static_cast<float>(C);
+    float v[kIters][4], s = 0.f, d = 0.f, q = 0.f;
+#pragma unroll
+    for (int i = 0; i < kIters; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[i][j] = 0.f;
+        if (128 * i + 4 * lane < C) load(x + base + 128 * i, v[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kIters; ++i) s += (v[i][0] + v[i][1]) + (v[i][2] + v[i][3]);
+    const float mean = warp_sum(s) * inv;
+#pragma unroll
+    for (int i = 0; i < kIters; ++i)
+        if (128 * i + 4 * lane < C) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[i][j] -= mean;
+                q = fmaf(v[i][j], v[i][j], q);
+            }
+            d += (v[i][0] + v[i][1]) + (v[i][2] + v[i][3]);
+        }
+    const float rest = warp_sum(d) * inv;
+    const float rstd = rsqrtf(fmaxf(fmaf(-rest, rest, warp_sum(q) * inv), 0.f) + eps), shift = -rest * rstd;
+#pragma unroll
+    for (int i = 0; i < kIters; ++i)
+        if (128 * i + 4 * lane < C) {
+            float w[4], b[4];
+            load(weight + 128 * i + 4 * lane, w);
+            load(bias + 128 * i + 4 * lane, b);
+            float4 o;
+            o.x = fmaf(fmaf(v[i][0], rstd, shift), w[0], b[0]); o.y = fmaf(fmaf(v[i][1], rstd, shift), w[1], b[1]);
+            o.z = fmaf(fmaf(v[i][2], rstd, shift), w[2], b[2]); o.w = fmaf(fmaf(v[i][3], rstd, shift), w[3], b[3]);
             *reinterpret_cast<float4*>(out + base + 128 * i) = o;
         }
 }
@@ -305,6 +352,14 @@ static void launch_norm_residual(int rows, int C, float eps, const A* a, const A
         if (gate != nullptr) return norm_residual_kernel<A, kIters, true><<<grid, kThreads, 0, s>>>(rows, C, eps, a, gate, weight, bias, gamma, x, out);
     }
     norm_residual_kernel<A, kIters, false><<<grid, kThreads, 0, s>>>(rows, C, eps, a, nullptr, weight, bias, gamma, x, out);
+}
+template <int kIters = 1>
+static void launch_layer_norm(int rows, int C, float eps, const float* x, const float* weight, const float* bias, float* out, cudaStream_t s) {
+    if constexpr (kIters < kMaxC / 128) {
+        if (C > 128 * kIters) return launch_layer_norm<kIters + 1>(rows, C, eps, x, weight, bias, out, s);
+    }
+    constexpr int kPer = kThreads / 32;
+    layer_norm_kernel<kIters><<<rows / kPer + (rows % kPer != 0 ? 1 : 0), kThreads, 0, s>>>(rows, C, eps, x, weight, bias, out);
 }
 
 }  // namespace epilogue
@@ -414,7 +469,7 @@ extern "C" int vrwkv_layer_norm(int rows, int C, float eps, const float* x, cons
     if (!x || !weight || !bias || !out) return VRWKV_ERR_NULL;
     if (C % 4 != 0 || C > kMaxC) return VRWKV_ERR_UNSUPPORTED;
     if (misaligned({x, weight, bias, out})) return VRWKV_ERR_ALIGNMENT;
-    launch_norm_residual<float>(rows, C, eps, x, nullptr, weight, bias, nullptr, nullptr, out, static_cast<cudaStream_t>(stream));
+    launch_layer_norm(rows, C, eps, x, weight, bias, out, static_cast<cudaStream_t>(stream));
     return record_launches(1);
 }
 
