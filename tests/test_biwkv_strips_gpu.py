@@ -109,3 +109,51 @@ def test_a_workspace_needs_no_clearing(cuda_device, T, k_scale, fill):
     ref = (O.biwkv_scan_forward(*f[:4]), *O.biwkv_scan_backward(*f))
     for a, b in zip((y, gwgu[0], gwgu[1], gk, gv), ref):
         assert rel_err(a, b) <= (1e-5 if k_scale == 1.0 else 5e-5)
+
+
+# Clusters of 2 to 16 CTAs.  `late`: the tokens of the CTA that sends nothing are outside the plain-float range, so that it leaves the unit to the
+# exact kernel while the others do not hear of it.
+@pytest.mark.parametrize("B,T", [(1, 1000), (1, 2000), (3, 4096), (24, 8704)])
+@pytest.mark.parametrize("types", ["f32", "wide", "bf16"])
+@pytest.mark.parametrize("late", [False, True])
+def test_a_call_returns_when_a_cta_sends_nothing(cuda_device, B, T, types, late):
+    from vision_rwkv_b200 import _lib
+    import ctypes
+    C, lib = 64, _lib.load()
+    assert lib.vrwkv_biwkv_one_pass(B, T, C, ("f32", "bf16", "wide").index(types))
+    w, u, k, v, gy = [x.float().to(cuda_device) for x in O.make_inputs(B, T, C, seed=T)]
+    dt = torch.float32 if types == "f32" else torch.bfloat16
+    clean = k.to(dt, copy=True)
+    if late:
+        k[:, 544:560] = 100.0      # of the second CTA, where a CTA holds 544 tokens or fewer
+    k, v, gy = k.to(dt), v.to(dt), gy.to(dt)
+    if types == "wide":
+        gy = gy.float()      # the kernels round it; its rounding is not what is checked here
+    y, gk, gv, gwgu = torch.empty_like(gy), torch.empty_like(k), torch.empty_like(k), torch.empty(2, C, device=cuda_device)
+    name = {"f32": "f32", "bf16": "bf16", "wide": "bf16_wide"}[types]
+    forward, backward = getattr(lib, "vrwkv_biwkv_forward_" + name), getattr(lib, "vrwkv_biwkv_backward_" + name)
+    s, p = torch.cuda.current_stream().cuda_stream, lambda t: t.data_ptr()
+
+    def calls(k):
+        ws = [torch.empty(f(B, T, C), dtype=torch.uint8, device=cuda_device) for f in (lib.vrwkv_biwkv_forward_workspace_bytes, lib.vrwkv_biwkv_backward_workspace_bytes)]
+        assert forward(B, T, C, p(w), p(u), p(k), p(v), p(y), p(ws[0]), ws[0].numel(), s) == 0
+        assert backward(B, T, C, p(w), p(u), p(k), p(v), p(gy), p(gwgu), p(gk), p(gv), p(ws[1]), ws[1].numel(), s) == 0
+        found = []
+        for x in ws:
+            status = ctypes.c_uint(0)
+            assert lib.vrwkv_workspace_status(p(x), s, ctypes.byref(status)) == 0
+            found.append(status.value & 1)
+        return found
+
+    try:
+        assert lib.vrwkv_set_path(3) == 0
+        for _ in range(3):
+            assert calls(k) == [1, 1]
+    finally:
+        lib.vrwkv_set_path(0)
+        lib.vrwkv_take_failures(torch.cuda.current_device())
+    assert calls(clean) == [0, 0]      # the context is intact
+    f = [x.double().cpu() for x in (w, u, clean, v, gy)]
+    ref = (O.biwkv_scan_forward(*f[:4]), *O.biwkv_scan_backward(*f))
+    for a, b, n in zip((y, gwgu[0], gwgu[1], gk, gv), ref, NAMES):
+        assert rel_err(a.float(), b) <= (2e-5 if types == "f32" or n in ("gw", "gu") else 1e-2), n

@@ -276,10 +276,12 @@ __device__ __forceinline__ Enter exchange(const Ctx& c, int level, Pair2 F, Pair
         }
         __syncwarp();
         if (warp == 0) {
-            if (!sm100::mbar_wait(c.xbar + level, 0, c.spin_limit) && lane == 0) failed(c, 1u);
+            const bool heard = sm100::mbar_wait(c.xbar + level, 0, c.spin_limit);
+            if (!heard && lane == 0) failed(c, 1u);
             if (level == 0) {
+                // A CTA that gave up goes no further either: at the next level it would send to CTAs that heard everything and may have left.
                 const int other = (lane < c.cluster && lane != c.rank) ? __float_as_int(peers[(lane - (lane > c.rank ? 1 : 0)) * kB + 2 * kCs]) : 0;
-                const int flag = __any_sync(0xffffffffu, (other | any) != 0) ? 1 : 0;
+                const int flag = __any_sync(0xffffffffu, !heard || (other | any) != 0) ? 1 : 0;
                 if (lane == 0) c.flag[0] = static_cast<unsigned>(flag);
             }
             if (lane < 2 * kCs) {
@@ -394,6 +396,17 @@ __device__ __forceinline__ void leave_word(const Ctx& c, const Params& p, unsign
         if (bits != 0u && p.mirror != nullptr) *reinterpret_cast<volatile unsigned*>(p.mirror) = bits;
         if (blockIdx.x == 0) *p.status = 0u;      // the exact kernel collects the bits
     }
+}
+// Before warp 0 of a CTA goes.  A CTA whose waits for the others all ended has everything that is ever sent to it.  One that gave up
+// stays until every other thread of its cluster has gone or come here, so that all that is sent is on its way (a cluster barrier counts
+// the threads that are left), and then for that to arrive, again with a limit.
+template <bool kBwd>
+__device__ __forceinline__ void stay_for_late_data(const Ctx& c) {
+    if (c.warp != 0 || c.flag[1] == 0u) return;
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    for (int l = 0; l < (kBwd ? 2 : 1); ++l) sm100::mbar_wait(c.xbar + l, 0, c.spin_limit);
 }
 // the mbarriers of the hand-over between CTAs: a block from every other one, per level
 template <class St, bool kBwd>
@@ -525,10 +538,11 @@ biwkv_forward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     Enter e1 = exchange<St, kSingle>(c, 0, F, group_sum(r, lam4, cst, kCs), unsafe);
     if (n == 0) e1 = Enter{zero(), zero()};
     if (unsafe) {
-        // the whole cluster takes this branch together: the unit is left to the exact kernel, which runs right behind (nothing of
-        // this CTA is in flight any more: its tiles have landed and everything the other CTAs sent has been waited for)
+        // The whole cluster takes this branch together, but for the others of a CTA that gave up a wait: the unit is left to the exact
+        // kernel, which runs right behind.
         __syncthreads();
         leave_word(c, p, kRedo);
+        if (!kSingle) stay_for_late_data<false>(c);
         return;
     }
     leave_word(c, p, 0u);      // the last wait of this CTA lies behind its barrier in the exchange
@@ -636,6 +650,7 @@ biwkv_backward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     if (unsafe) {      // as in the forward
         __syncthreads();
         leave_word(c, p, kRedo);
+        if (!kSingle) stay_for_late_data<true>(c);
         return;
     }
     if (kHalfG) {
@@ -788,6 +803,7 @@ biwkv_backward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         p.partial[((static_cast<size_t>(b) * c.cluster + c.rank) * 2 + j) * p.c_padded + strip * kCs + ch] = acc;
     }
     if (!kHalf && lane == 0) sm100::tma_store_wait_read();   // shared memory may go once the stores have read it
+    if (!kSingle) stay_for_late_data<true>(c);
 }
 
 // ---- the exact kernel ----------------------------------------------------------------------------
