@@ -238,6 +238,24 @@ __device__ __forceinline__ HiLo decay_over_blocks(const Ctx& c, int blocks) {
     const float hi = static_cast<float>(x);
     return HiLo{dup(hi), dup(static_cast<float>(x - static_cast<double>(hi)))};
 }
+// A wait for another CTA ran out.  This one goes no further than the first level: at the second it would send to CTAs that heard
+// everything and may have left (out of range).  See stay_for_late_data.
+__device__ __forceinline__ void gave_up(const Ctx& c, unsigned bits) {
+    report_failure(c.status, c.mirror, bits);
+    *reinterpret_cast<volatile unsigned*>(c.flag + 2) = 1u;
+}
+// Before warp 0 of a CTA goes: one that gave up a wait stays until everything that is sent to it is on its way - every other thread of
+// its cluster has gone or come here (a cluster barrier counts the threads that are left) - and then, with a limit, until it is there.
+// `phases`: of the cluster barrier that those that go on still pass.
+__device__ __forceinline__ void stay_for_late_data(const Ctx& c, int phases, int levels) {
+    if (c.warp != 0 || c.flag[2] == 0u) return;
+    __syncwarp();
+    for (int i = 0; i < phases; ++i) {
+        cluster_arrive();
+        cluster_wait();
+    }
+    for (int l = 0; l < levels; ++l) sm100::mbar_wait(c.xbar + l, 0, c.spin_limit);
+}
 // waits for `count` flags starting at segment `first` (lane j takes segment first + j); returns the OR of their values
 __device__ __forceinline__ unsigned seg_wait(const Ctx& c, int first, int count, int level, int dir) {
     unsigned seen = 1u;
@@ -251,8 +269,9 @@ __device__ __forceinline__ unsigned seg_wait(const Ctx& c, int first, int count,
         }
         if (seen) seen = sm100::flag_acquire(f);
     }
-    if (!__all_sync(0xffffffffu, seen != 0u) && c.lane == 0) report_failure(c.status, c.mirror, 4u);
-    unsigned bits = seen;
+    const bool all = __all_sync(0xffffffffu, seen != 0u);
+    if (!all && c.lane == 0) gave_up(c, 4u);
+    unsigned bits = all ? seen : 2u;
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, m);
     return bits;
@@ -471,8 +490,10 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     }
     TL_MARK(13 + level * 5);
     // (3) wait for the other CTAs' bytes, combine them
+    bool heard = true;
     if (!kLocal && c.cluster > 1 && (warp == scanF || warp == scanR)) {
-        if (!sm100::mbar_wait(c.xbar + level, 0, c.spin_limit) && lane == 0) report_failure(c.status, c.mirror, 1u);
+        heard = sm100::mbar_wait(c.xbar + level, 0, c.spin_limit);
+        if (!heard && lane == 0) gave_up(c, 1u);
     }
     TL_MARK(14 + level * 5);
     if (!kLocal && warp == scanF) {
@@ -506,7 +527,7 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
                     }
                 }
             }
-            if (level == 0) flag = cluster_flag<RW>(c, any);
+            if (level == 0) flag = cluster_flag<RW>(c, any || !heard);
         }
         if (kLinked) seg_exchange_forward<kMom>(c, level, X, MX, ctaP, ctaM, flag);
         c.cta[lane] = X.x; c.cta[kCs + lane] = X.y;
@@ -531,7 +552,7 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
         }
         if (kLinked) {
             int flag = 0;
-            if (level == 0) flag = c.cluster > 1 ? cluster_flag<RW>(c, any) : any;
+            if (level == 0) flag = c.cluster > 1 ? cluster_flag<RW>(c, any || !heard) : any;
             seg_exchange_reverse(c, level, Y, ctaS, flag);
             if (lane == 0) c.flag[1] = static_cast<unsigned>(flag);
         }
@@ -709,6 +730,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         }
     }
     if (threadIdx.x == 0) {
+        c.flag[2] = 0u;
         for (int l = 0; l < RW::kLevels; ++l) sm100::mbar_init(c.xbar + l, 1);
         sm100::mbar_init_fence();
         if (kCluster && p.cluster > 1) {
@@ -847,6 +869,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         // the whole cluster takes this branch together; the count switches on the chunked kernels that stand by, which redo the whole
         // call (without clusters the word that was read does)
         if (kCluster && cta == 0 && threadIdx.x == 0) atomicAdd(p.redo_count, 1u);
+        if (kCluster) stay_for_late_data(c, kBwd ? 2 : 1, kBwd ? 2 : 1);
         return;
     }
     if (!kBwd) {
@@ -1046,6 +1069,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     TL_MARK(8);
     if (kHalf ? lane == 0 : threadIdx.x == 0) sm100::tma_store_wait_read();   // shared memory may go once the stores have read it
     TL_MARK(9);
+    if (kCluster) stay_for_late_data(c, 1, kBwd ? 2 : 1);
 }
 
 // out[j][c] = sum over sequences and cluster ranks of partial[cta][j][c % 32], fixed order
