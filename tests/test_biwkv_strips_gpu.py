@@ -161,3 +161,33 @@ def test_a_call_returns_when_a_cta_sends_nothing(cuda_device, B, T, types, late)
     ref = (O.biwkv_scan_forward(*f[:4]), *O.biwkv_scan_backward(*f))
     for a, b, n in zip((y, gwgu[0], gwgu[1], gk, gv), ref, NAMES):
         assert rel_err(a.float(), b) <= (2e-5 if types == "f32" or n in ("gw", "gu") else 1e-2), n
+
+
+# weights that grow by e^5 to e^45 over the sequence, so that 2 max|k| + |u| + |w| + max(-w, 0) T is below 60 by what 14 to 16 rows past T may cost
+@pytest.mark.parametrize("T,growth", [(1, 5.0), (1, 100.0), (2, 7.0), (4, 11.0), (7, 18.0), (12, 30.0), (17, 28.0), (20, 33.0), (31, 34.0), (49, 45.0), (61, 42.0), (200, 45.0)])
+@pytest.mark.parametrize("types", ["f32", "wide"])
+def test_short_sequences_with_steep_weights_need_no_exact_kernel(cuda_device, T, growth, types):
+    """Rows past T fill up a walker's 15 or 17 tokens; the first e^8 that weights grow over them is free, and a single token knows no weights.  The words of the CTAs (256 bytes into a
+    workspace) say whether a unit was left to the exact kernel.  Tolerance: 5e-5, that of test_biwkv_gpu.py for extreme exponents."""
+    from vision_rwkv_b200 import _lib
+    B, C, lib = 3, 48, _lib.load()
+    w, u, k, v, gy = [x.float().to(cuda_device) for x in O.make_inputs(B, T, C, seed=T)]
+    w = torch.linspace(-growth, -growth / 2, C, device=cuda_device) / T
+    k = k.clamp(-1, 1)
+    dt = torch.float32 if types == "f32" else torch.bfloat16
+    k, v, gy = k.to(dt), v.to(dt), gy.to(dt).float()
+    y, gk, gv, gwgu = torch.empty_like(gy), torch.empty_like(k), torch.empty_like(k), torch.empty(2, C, device=cuda_device)
+    name = "f32" if types == "f32" else "bf16_wide"
+    ws = [torch.zeros(f(B, T, C), dtype=torch.uint8, device=cuda_device) for f in (lib.vrwkv_biwkv_forward_workspace_bytes, lib.vrwkv_biwkv_backward_workspace_bytes)]
+    s, p = torch.cuda.current_stream().cuda_stream, lambda t: t.data_ptr()
+    assert getattr(lib, "vrwkv_biwkv_forward_" + name)(B, T, C, p(w), p(u), p(k), p(v), p(y), p(ws[0]), ws[0].numel(), s) == 0
+    assert getattr(lib, "vrwkv_biwkv_backward_" + name)(B, T, C, p(w), p(u), p(k), p(v), p(gy), p(gwgu), p(gk), p(gv), p(ws[1]), ws[1].numel(), s) == 0
+    for x in ws:
+        assert not (x[256:256 + 4 * B * 3].view(torch.int32) & 1).any()
+    f = [x.double().cpu() for x in (w, u, k, v, gy)]
+    ref = (O.biwkv_scan_forward(*f[:4]), *O.biwkv_scan_backward(*f))
+    for a, b, n in zip((y, gwgu[0], gwgu[1], gk, gv), ref, NAMES):
+        if T > 1 or n in ("y", "gv"):      # one token: no gradient but gv = gy
+            assert rel_err(a.float(), b) <= (5e-5 if types == "f32" or n in ("gw", "gu") else 1e-2), n
+        else:
+            assert a.float().abs().max() <= 1e-5 * max(1.0, gy.abs().max().item())

@@ -38,7 +38,7 @@
 // tiles are waited for but the steps of the arithmetic.
 //
 // Arithmetic, exactness and the exact kernel: plain floats without exponent shift, safe whenever 2 max|k| + |u| + |w| + max(-w, 0) T
-// <= 60 (T in whole walkers); each thread checks its own tokens, the first exchange carries the OR, and every CTA leaves a word that
+// <= 60 (and rows past T grow by little, kSafePast); each thread checks its own tokens, the first exchange carries the OR, and every CTA leaves a word that
 // says whether its unit is left to biwkv_exact_kernel (per-token max-shifted arithmetic, launched behind).  Decays over
 // half a walker and more come from double precision.
 //
@@ -89,6 +89,9 @@ enum ConstRow { kLam = 0, kWl2, kCuw, kLam4, kLamFirst, kLamHalf, kFixLo, kFixHi
 // A CTA's sums as sent to another: [channel][a, b] and a flag word
 template <class St>
 constexpr int kBlock = 2 * St::kCs + 4;
+// Rows past T, up to a whole walker, hold zeros, but what the walks carry grows on over them, and must stay finite to vanish against the
+// zeros: e^kSafePast beyond what valid rows may reach is left alone (e^68, and e^20 = 5e8 for T times the inputs' size).
+constexpr float kSafePast = 8.f;
 constexpr int kRecRows = 4;      // of kCs floats, per span: towards later tokens a, b; towards earlier ones a, b
 
 struct Params {
@@ -149,7 +152,8 @@ __device__ __forceinline__ void strip_constants(float* consts, const Params& p, 
     constexpr int kCs = St::kCs;
     if (threadIdx.x >= 2 * kCs) return;
     const int ch = threadIdx.x & (kCs - 1), at = strip * kCs + ch;
-    const float w = at < p.C ? __ldg(p.w + at) : 0.f, u = at < p.C ? __ldg(p.u + at) : 0.f;
+    // a single token is not decayed: whatever w is, the rows that fill up its walker must not grow with it
+    const float w = at < p.C && p.T > 1 ? __ldg(p.w + at) : 0.f, u = at < p.C ? __ldg(p.u + at) : 0.f;
     // no infinity: what lies past the end of a sequence is zero and has to stay so
     const auto put = [&](int row, double x) { consts[row * kCs + ch] = static_cast<float>(x > 1e38 ? 1e38 : x); };
     const double wd = w;
@@ -157,7 +161,8 @@ __device__ __forceinline__ void strip_constants(float* consts, const Params& p, 
     double x = exp(own ? static_cast<double>(u) + wd : -wd);
     if (own) {
         put(kCuw, x);
-        consts[kLimit * kCs + ch] = kSafeRange - (fabsf(u) + fabsf(w) + fmaxf(-w, 0.f) * static_cast<float>((p.T + St::L - 1) / St::L * St::L));
+        const float grows = fmaxf(-w, 0.f), past = grows * static_cast<float>((p.T + St::L - 1) / St::L * St::L - p.T);
+        consts[kLimit * kCs + ch] = kSafeRange - (fabsf(u) + fabsf(w) + grows * static_cast<float>(p.T) + fmaxf(past - kSafePast, 0.f));
         put(kLamL + St::kW + 1, 0.0);
         return;
     }
