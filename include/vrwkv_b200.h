@@ -332,7 +332,8 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
  *     _f32out: the bfloat16 result widened
  *   vrwkv_relu_square: out = relu(x)^2 in the type of x (CLS/vrwkv.py:251); _f32out: of bfloat16 x in float32 (exact)
  *   vrwkv_linear_relu_square: out (rows, N) = relu(x W^T)^2 of x (rows, K) and W (N, K), the product rounded to bfloat16 first
- *     (CLS/vrwkv.py:250-251); K % 64 == 0, N % 256 == 0, else VRWKV_ERR_UNSUPPORTED
+ *     (CLS/vrwkv.py:250-251); K % 64 == 0, N % 256 == 0, else VRWKV_ERR_UNSUPPORTED; _pays: 1 where it takes less of the current
+ *     device's time than a library's product and vrwkv_relu_square
  *   vrwkv_norm_residual: out = x + gamma * (normalise(a) * weight + bias) over rows of C <= 1024 channels, C % 4 == 0;
  *     weight and bias NULL: out = x + gamma * a; gamma NULL: 1 (CLS/vrwkv.py:297-318)
  *   vrwkv_layer_norm: out = normalise(x) * weight + bias over such rows
@@ -348,6 +349,7 @@ int vrwkv_sigmoid_gate(long long n, const void* r, int r_is_bf16, const void* y,
 int vrwkv_sigmoid_gate_f32out(long long n, const uint16_t* r, const uint16_t* y, float* out, void* stream);
 int vrwkv_relu_square(long long n, const void* x, int is_bf16, void* out, void* stream);
 int vrwkv_relu_square_f32out(long long n, const uint16_t* x, float* out, void* stream);
+int vrwkv_linear_relu_square_pays(long long rows, int K, int N);
 int vrwkv_linear_relu_square(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream);
 int vrwkv_add_rows(long long n, long long period, const float* table, const uint16_t* a, float* out, void* stream);
 int vrwkv_widen(long long n, const uint16_t* a, float* out, void* stream);

@@ -46,3 +46,33 @@ def test_layers_that_are_watched_or_replaced_keep_their_call(cuda_device):
         hook.remove()
     assert seen == [1] and torch.equal(again, want)
     assert ((got.float() - want.float()).norm() / want.float().norm()).item() <= 5e-3      # sums in another order: some roundings differ
+
+
+@pytest.mark.parametrize("rows,C", [(1, 192), (196, 384), (196, 1024), (1568, 768), (40, 2048), (25000, 192), (12544, 768)])
+def test_the_key_layer_takes_one_kernel_only_where_it_is_faster(cuda_device, rows, C):
+    """By the measured rule: from four rounds of 128 x 256 tiles over the SMs on, before that where a round's SMs are four fifths busy, up to
+    1024 channels; of calls that are not captured the small ones too.  Elsewhere the product is torch's."""
+    from vision_rwkv_b200 import _lib, epilogue
+    lib = _lib.load()
+    key, value = torch.nn.Linear(C, 4 * C, bias=False, device=cuda_device), torch.nn.Linear(4 * C, C, bias=False, device=cuda_device)
+    x = torch.randn(rows, C, device=cuda_device).bfloat16()
+    sms, tiles = torch.cuda.get_device_properties(cuda_device).multi_processor_count, -(-rows // 128) * 4 * C // 256
+    rounds = -(-tiles // sms)
+    pays = C <= 1024 and (rounds >= 4 or tiles >= 0.8 * rounds * sms)
+    assert bool(lib.vrwkv_linear_relu_square_pays(rows, C, 4 * C)) == pays
+
+    def run():
+        with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+            before = lib.vrwkv_launch_count()
+            out = epilogue.linear_relu_square(key, x, value)
+            assert lib.vrwkv_launch_count() == before + 1
+            return out
+
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        by_torch, by_one = epilogue.relu_square(key(x), value), _lib.native().linear_relu_square(x, key.weight)
+    assert torch.equal(run(), by_one if pays or (C <= 1024 and rows * 4 * C <= 128 * 128 * 256) else by_torch)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = run()
+    graph.replay()
+    assert torch.equal(captured, by_one if pays else by_torch)

@@ -36,6 +36,7 @@ SIGNATURES = {
     "vrwkv_sigmoid_gate_f32out": (_c_int, [ctypes.c_longlong] + [_ptr] * 4),
     "vrwkv_relu_square": (_c_int, [ctypes.c_longlong, _ptr, _c_int, _ptr, _ptr]),
     "vrwkv_layer_norm": (_c_int, [_c_int] * 2 + [ctypes.c_float] + [_ptr] * 5),
+    "vrwkv_linear_relu_square_pays": (_c_int, [ctypes.c_longlong] + [_c_int] * 2),
     "vrwkv_linear_relu_square": (_c_int, [ctypes.c_longlong] + [_c_int] * 2 + [_ptr] * 4),
     "vrwkv_relu_square_f32out": (_c_int, [ctypes.c_longlong] + [_ptr] * 3),
     "vrwkv_widen": (_c_int, [ctypes.c_longlong] + [_ptr] * 3),

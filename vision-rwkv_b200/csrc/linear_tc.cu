@@ -12,8 +12,8 @@
 //
 // us, library product / and the pass behind it / this: rows 50176 K=192 N=768 24.7 / 51.4 / 30.9, 384 -> 1536 57.5 / 108.8 / 63.5 (HBM's
 // time for x and the result 30, 931 TFLOP/s), 768 -> 3072 180 / 303 / 207, 1024 -> 4096 300 / 469 / 324 (1301 TFLOP/s of a measured 1410);
-// rows 12544 768 -> 3072 47.2 / 74.2 / 52.2; rows 196 (calls one by one, host time in part) 10.5 / 15.1 / 8.3 to 10.9 / 15.6 / 14.5.
-// So it serves every size that its tiles divide.
+// rows 12544 768 -> 3072 47.2 / 74.2 / 52.2.  Few tiles, deep products and SMs without a tile in the last round are the library's
+// (vrwkv_linear_relu_square_pays).
 //
 // Every wait is bounded; one that gives up sets a flag that ends the other roles, and the host-visible word of failures.
 #include <cuda_bf16.h>
@@ -240,6 +240,21 @@ static bool allowed(int* sms) {
 }
 
 }  // namespace lineartc
+
+// The GPU's time for a library product and the pass behind it, in a captured loop, over this kernel's, by rounds of tiles: 1.04 and more
+// from four rounds on; before that by how full the rounds are: K = 192 0.94 at half, 1.06 at 0.7, 1.15 at 0.8 (1.2 at one full round);
+// K = 1024 0.86 at 0.6, 0.96 to 1.02 at 0.7, 1.02 to 1.08 at 0.8.  Rows 1 to 196, K = 64 to 1024: 0.54 to 0.8, of 3 to 8 us (a chain of
+// loads; the library splits K).  K = 1536 0.98 to 1.12 at 0.8 and above, K = 4096 0.34 to 0.96 whatever the rows: the library's
+// product is the faster one, and the pass is little beside it.
+extern "C" int vrwkv_linear_relu_square_pays(long long rows, int K, int N) {
+    using namespace lineartc;
+    if (rows <= 0 || K <= 0 || N <= 0 || K % kK != 0 || N % kN != 0 || K > 1024 || rows > (1LL << 30)) return 0;
+    const long long tiles = (rows + kM - 1) / kM * (N / kN);
+    int sms = 0;
+    if (tiles > (1LL << 30) || !allowed(&sms)) return 0;
+    const long long rounds = (tiles + sms - 1) / sms;
+    return rounds >= 4 || 5 * tiles >= 4 * rounds * sms ? 1 : 0;
+}
 
 extern "C" int vrwkv_linear_relu_square(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream) {
     using namespace lineartc;

@@ -1,6 +1,7 @@
 // Host path of the inference-only steps between a block's matrix products (csrc/mixer_epilogue.cu).  The rules that decide
 // whether a call may come here are epilogue.py's.
 #include <ATen/autocast_mode.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include "glue.h"
 
 namespace vrwkv {
@@ -57,6 +58,22 @@ Tensor linear_relu_square(const Tensor& x_, const Tensor& weight_) {
     const auto p = [](const Tensor& t) { return static_cast<uint16_t*>(t.data_ptr()); };
     check(vrwkv_linear_relu_square(x.numel() / x.size(-1), weight.size(1), weight.size(0), p(x), p(weight), p(out), stream_of(x)), "vrwkv_linear_relu_square");
     return out;
+}
+
+constexpr int64_t kOneByOne = 128 * 128 * 256;      // elements of a result: 128 tiles, less than one to an SM
+
+Tensor key_layer(const Tensor& x, const Tensor& weight) {
+    same_place(x, weight, "x");
+    TORCH_CHECK(weight.dim() == 2 && x.dim() >= 1, "x must be rows of the weight's width");
+    const c10::cuda::CUDAGuard guard(x.device());
+    if (x.numel() == 0) return linear_relu_square(x, weight);
+    const int64_t rows = x.numel() / x.size(-1);
+    if (vrwkv_linear_relu_square_pays(rows, weight.size(1), weight.size(0))) return linear_relu_square(x, weight);
+    // Small calls one by one cost the host more than the GPU: 16 us more for torch's product and the pass, where this kernel's GPU time
+    // is 5 to 11 us and theirs 3 to 8 (one image, VRWKV-T to -B: 3.40 ms a forward, else 3.55).  A captured call costs the GPU's time alone.
+    if (weight.size(1) <= 1024 && rows * weight.size(0) <= kOneByOne && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)
+        return linear_relu_square(x, weight);
+    return relu_square(at::linear(x, weight), false);
 }
 
 Tensor add_rows(const Tensor& table_, const Tensor& a_) {

@@ -15,8 +15,10 @@ Tensor norm_gate(const Tensor& x, const Tensor& gate, const Tensor& weight, cons
 // epilogue.cpp
 Tensor sigmoid_gate(const Tensor& r, const Tensor& y, bool wide);      // wide: bfloat16 r, y to a float32 result
 Tensor relu_square(const Tensor& x, bool wide);      // wide: bfloat16 x to a float32 result
-// relu(x weight^T)^2 in bfloat16, as autocast computes it for a linear layer that rounds it
+// relu(x weight^T)^2 in bfloat16, as autocast computes it for a linear layer that rounds it; called under bfloat16 autocast
 Tensor linear_relu_square(const Tensor& x, const Tensor& weight);
+// the same, by one kernel or by torch's product and the pass behind it, whichever takes less time
+Tensor key_layer(const Tensor& x, const Tensor& weight);
 Tensor add_rows(const Tensor& table, const Tensor& a);
 Tensor patch_rows(const Tensor& img, int64_t patch);
 Tensor widen(const Tensor& a);
