@@ -60,7 +60,8 @@ unsigned long long vrwkv_launch_count(void);
  * cluster-resident kernels (persistent tile kernels where eligible), 3 = test of the bounded
  * device-side waits: as 0, but one CTA of every cluster withholds what it owes the others and
  * the waits give up after about a thousand polls, so the call returns promptly with bit 0 of the
- * status word set and meaningless results (nothing hangs, nothing faults).  Process-wide.
+ * status word set and meaningless results (nothing hangs, nothing faults); vrwkv_linear_relu_square likewise, one
+ * role of each CTA.  Process-wide.
  * No reference counterpart. */
 int vrwkv_set_path(int path);
 /* Copies the device status word kept in the first 4 bytes of a workspace to *status_out
@@ -71,11 +72,12 @@ int vrwkv_set_path(int path);
 int vrwkv_workspace_status(const void* workspace, void* stream, unsigned* status_out);
 
 /* Failure bits (as in vrwkv_workspace_status) that launches on `device` have reported since the last call, and
- * clears them; 0 if none.  Bits 8 to 11 say whose launches: Bi-WKV forward, Bi-WKV backward, WKV6 forward, WKV6
- * backward.  Kernels that give up a bounded wait write a word of mapped host memory, so the
+ * clears them; 0 if none.  Bits 8 to 12 say whose launches: Bi-WKV forward, Bi-WKV backward, WKV6 forward, WKV6
+ * backward, vrwkv_linear_relu_square.  Kernels that give up a bounded wait write a word of mapped host memory, so the
  * call reads host memory: no synchronisation, no copy.  A launch that is still running reports later:
  * synchronise first to see its result.  The first call (per process) sets the word up; launches made before it
- * report through their workspace only. */
+ * report through their workspace only (vrwkv_linear_relu_square, which has none, sets the word up by itself: after a
+ * synchronisation this call tells whether its result is whole). */
 unsigned vrwkv_take_failures(int device);
 
 /* ---- Bi-WKV --------------------------------------------------------------------

@@ -76,3 +76,56 @@ def test_the_key_layer_takes_one_kernel_only_where_it_is_faster(cuda_device, row
         captured = run()
     graph.replay()
     assert torch.equal(captured, by_one if pays else by_torch)
+
+
+def withheld_inputs(dev):
+    """Three tiles to a CTA, so that an epilogue's missing arrival is waited for too; K of more slices than stages."""
+    g = torch.Generator(device=dev).manual_seed(1)
+    rows = 128 * torch.cuda.get_device_properties(dev).multi_processor_count
+    return torch.randn(rows, 384, device=dev, generator=g).bfloat16(), torch.randn(768, 384, device=dev, generator=g).bfloat16() / 20
+
+
+def test_bounded_waits_run_out_and_report(cuda_device):
+    """Path 3: in every third CTA the loader, in every third the issuer, in every third the epilogue leaves out what the others wait for."""
+    from vision_rwkv_b200 import _lib, epilogue, ops
+    lib, native = _lib.load(), _lib.native()
+    x, w = withheld_inputs(cuda_device)
+    key, value = torch.nn.Linear(384, 768, bias=False, device=cuda_device), torch.nn.Linear(768, 384, bias=False, device=cuda_device)
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        want = native.linear_relu_square(x, w)
+        try:
+            assert lib.vrwkv_set_path(3) == 0
+            native.linear_relu_square(x, w)
+            with pytest.raises(_lib.VrwkvError, match="earlier launch, linear:"):
+                ops.raise_if_failed()
+            native.linear_relu_square(x, w)
+            torch.cuda.synchronize()
+            with pytest.raises(_lib.VrwkvError, match="earlier launch, linear:"):
+                native.linear_relu_square(x, w)
+            torch.cuda.synchronize()
+            lib.vrwkv_take_failures(torch.cuda.current_device())
+            ops.CHECK_STATUS = True
+            with pytest.raises(_lib.VrwkvError, match="linear:"):
+                epilogue.linear_relu_square(key, x, value)
+        finally:
+            ops.CHECK_STATUS = False
+            lib.vrwkv_set_path(0)
+        ops.raise_if_failed()
+        # the context is intact and the next call is right again
+        assert torch.equal(native.linear_relu_square(x, w), want)
+        ops.raise_if_failed()
+
+
+def test_a_process_that_calls_nothing_else_hears_of_it(cuda_device):
+    import os
+    import subprocess
+    import sys
+    # the library as a C program has it: vrwkv_take_failures (which _lib.load calls) comes after the launch
+    code = ("import ctypes, torch, tests.test_linear_gpu as t\nfrom vision_rwkv_b200 import _lib\nlib = ctypes.CDLL(_lib.LIB_PATH)\n"
+            "for n in ('vrwkv_set_path', 'vrwkv_linear_relu_square', 'vrwkv_take_failures'):\n    getattr(lib, n).restype, getattr(lib, n).argtypes = _lib.SIGNATURES[n]\n"
+            "x, w = t.withheld_inputs(torch.device('cuda'))\nout = torch.empty(x.shape[0], w.shape[0], device='cuda', dtype=torch.bfloat16)\n"
+            "lib.vrwkv_set_path(3)\n"
+            "assert lib.vrwkv_linear_relu_square(x.shape[0], 384, 768, x.data_ptr(), w.data_ptr(), out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0\n"
+            "torch.cuda.synchronize()\nassert lib.vrwkv_take_failures(0) == 1 | 1 << 12\nassert lib.vrwkv_take_failures(0) == 0\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=root, timeout=300)

@@ -50,8 +50,32 @@ std::atomic<unsigned*> g_mirror{nullptr};
 std::mutex g_mirror_mutex;
 }  // namespace
 
-unsigned* failure_mirror(Op op) {
+// the words, set up by the first call; null where that fails
+static unsigned* mirror_base() {
     unsigned* base = g_mirror.load(std::memory_order_acquire);
+    if (base != nullptr) return base;
+    std::lock_guard<std::mutex> lock(g_mirror_mutex);
+    base = g_mirror.load(std::memory_order_acquire);
+    if (base != nullptr) return base;
+    // not an operation a stream capture may contain: leave the thread's capture mode out of it
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    const cudaError_t err = cudaHostAlloc(&p, kMirrorDevices * kMirrorOps * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (err != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::memset(p, 0, kMirrorDevices * kMirrorOps * sizeof(unsigned));
+    base = static_cast<unsigned*>(p);
+    g_mirror.store(base, std::memory_order_release);
+    return base;
+}
+
+unsigned* failure_mirror(Op op) {
+    // a linear layer has no workspace whose status word would tell: its word is there from its first launch on
+    unsigned* base = op == Op::linear ? mirror_base() : g_mirror.load(std::memory_order_acquire);
     int dev = 0;
     if (base == nullptr || cudaGetDevice(&dev) != cudaSuccess || dev >= kMirrorDevices) return nullptr;
     return base + dev * kMirrorOps + static_cast<int>(op);
@@ -84,6 +108,7 @@ int vrwkv_set_path(int path) {
     if (path < 0 || path > 3) return VRWKV_ERR_SHAPE;
     biwkv::resident::set_withhold_test(path == 3);
     biwkv::strips::set_withhold_test(path == 3);
+    lineartc::set_withhold_test(path == 3);
     g_path.store(path == 3 ? 0 : path);
     return VRWKV_OK;
 }
@@ -100,26 +125,8 @@ int vrwkv_workspace_status(const void* workspace, void* stream, unsigned* status
 }
 
 unsigned vrwkv_take_failures(int device) {
-    unsigned* base = g_mirror.load(std::memory_order_acquire);
-    if (base == nullptr) {
-        std::lock_guard<std::mutex> lock(g_mirror_mutex);
-        base = g_mirror.load(std::memory_order_acquire);
-        if (base == nullptr) {
-            // not an operation a stream capture may contain: leave the thread's capture mode out of it
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            void* p = nullptr;
-            const cudaError_t err = cudaHostAlloc(&p, kMirrorDevices * kMirrorOps * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            if (err != cudaSuccess) {
-                cudaGetLastError();
-                return 0;
-            }
-            std::memset(p, 0, kMirrorDevices * kMirrorOps * sizeof(unsigned));
-            base = static_cast<unsigned*>(p);
-            g_mirror.store(base, std::memory_order_release);
-        }
-    }
+    unsigned* const base = mirror_base();
+    if (base == nullptr) return 0;
     if (device < 0 || device >= kMirrorDevices) return 0;
     unsigned bits = 0;
     for (int op = 0; op < kMirrorOps; ++op) {

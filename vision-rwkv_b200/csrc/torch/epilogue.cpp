@@ -57,6 +57,7 @@ Tensor linear_relu_square(const Tensor& x_, const Tensor& weight_) {
     if (x.numel() == 0) return out;
     const auto p = [](const Tensor& t) { return static_cast<uint16_t*>(t.data_ptr()); };
     check(vrwkv_linear_relu_square(x.numel() / x.size(-1), weight.size(1), weight.size(0), p(x), p(weight), p(out), stream_of(x)), "vrwkv_linear_relu_square");
+    raise_failures(x.get_device(), "vrwkv_linear_relu_square");
     return out;
 }
 

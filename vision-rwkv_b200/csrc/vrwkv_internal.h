@@ -9,9 +9,13 @@ void set_error_detail(const char* text);
 // Add `launched` kernels to the process-wide count and turn the CUDA error state into a status.
 int record_launches(int launched);
 // Host-visible word of the current device and operator that kernels set when a bounded wait runs out (pinned, mapped;
-// null until vrwkv_take_failures() has been called once).  It costs a successful launch nothing.
+// null until vrwkv_take_failures() has been called once, but for Op::linear).  It costs a successful launch nothing.
 enum class Op { biwkv_forward, biwkv_backward, wkv6_forward, wkv6_backward, linear };
 unsigned* failure_mirror(Op op);
+
+namespace lineartc {
+void set_withhold_test(bool on);   // test only: one role of every CTA withholds an arrival, waits give up early
+}
 
 #ifdef __CUDACC__
 // A bounded wait ran out: `status` is the launch's own device word, `mirror` the host-visible one (may be null).

@@ -37,7 +37,10 @@ def linear_relu_square(key, x, layer=None):
         w = key.weight
         if (type(w) in (nn.Parameter, torch.Tensor) and w.dtype in KERNEL_DTYPES and w.device == x.device and w.dim() == 2 and w.shape[1] == x.shape[-1]
                 and w.shape[1] % 64 == 0 and w.shape[1] > 0 and w.shape[0] % 256 == 0 and w.shape[0] > 0):
-            return _lib.native().key_layer(x, w)
+            out = _lib.native().key_layer(x, w)
+            if ops.CHECK_STATUS:
+                ops.raise_if_failed(x.device)
+            return out
     return relu_square(key(x), layer)
 
 
