@@ -3,6 +3,7 @@ run under autograd (`torch.enable_grad`) in the same functions."""
 import pytest
 import torch
 import torch.nn as nn
+import torch.utils._python_dispatch
 
 from conftest import rel_err
 
@@ -198,3 +199,57 @@ def test_patch_embedding(cuda_device, B, channels, H, W, patch):
     assert rel_err(tokens.double(), want) < bound and rel_err(by_conv.flatten(2).transpose(1, 2).double(), want) < bound
     with torch.no_grad():
         assert epilogue.patch_embedding(img, conv) is None                       # float32 networks keep the convolution
+
+
+class Seen(torch.overrides.TorchFunctionMode):
+    def __init__(self):
+        self.names = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.names.append(getattr(func, "__name__", ""))
+        return func(*args, **(kwargs or {}))
+
+
+class Dispatched(torch.utils._python_dispatch.TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.products = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        if "mm" in func.__name__:
+            a, b = args[-2:]
+            self.products.append((a.shape[0], a.shape[1], b.shape[1]))
+        return func(*args, **(kwargs or {}))
+
+
+class Wrapped(torch.Tensor):
+    pass
+
+
+def test_layers_are_called_where_a_mode_or_a_tensor_subclass_would_see_it(cuda_device):
+    """What a dispatch mode (a FLOP counter that knows no modules, say), a function mode or a tensor subclass sees are the layers' own
+    operations: key, value and receptance of a channel mix, its norms."""
+    from vision_rwkv_b200 import backbone, epilogue, launch_count
+    C, rows = 192, 20000
+    mix = backbone.ChannelMix(C, 4, 0).to(cuda_device).eval()
+    norm = nn.LayerNorm(C, device=cuda_device)
+    x = torch.randn(1, rows, C, device=cuda_device)
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        with Dispatched() as counter:
+            watched = mix(x, (125, 160))
+        assert sorted(counter.products) == sorted([(rows, C, 4 * C), (rows, 4 * C, C), (rows, C, C)])
+        with Seen() as seen:
+            normed = epilogue.layer_norm(norm, x)
+            widened = epilogue.widened(norm, x.bfloat16())
+            mix(x, (125, 160))
+        assert seen.names.count("linear") == 3 and "layer_norm" in seen.names and widened.dtype == torch.bfloat16
+        assert type(epilogue.layer_norm(norm, x.as_subclass(Wrapped))) is Wrapped
+        norm.weight = nn.Parameter(norm.weight.detach().as_subclass(Wrapped))
+        before = launch_count()
+        epilogue.layer_norm(norm, x)
+        assert launch_count() == before
+        norm.weight = nn.Parameter(torch.ones(C, device=cuda_device))
+        with torch.device(cuda_device):      # a default device is a mode that watches nothing
+            assert torch.equal(epilogue.layer_norm(norm, x), epilogue.layer_norm(norm, x)) and launch_count() == before + 2
+        assert ((epilogue.layer_norm(norm, x) - normed).norm() / normed.norm()).item() <= 1e-6
+        assert ((mix(x, (125, 160)).float() - watched.float()).norm() / watched.float().norm()).item() <= 1e-2

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
+from torch.utils._device import DeviceContext
 
 from . import _lib, normgate, ops, traced
 from .qshift import autocast_linears, feeds_autocast_linears, stock
@@ -19,6 +20,21 @@ MOST_NORM_CHANNELS = 1024       # a row of norm_residual lives in one warp's reg
 
 def _inference(*tensors):
     return not torch.is_grad_enabled() and not traced.tracing() and all(t.is_cuda and t.dtype in KERNEL_DTYPES for t in tensors)
+
+
+_dispatch_modes, _function_modes, _PLAIN = torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack, (nn.Parameter, torch.Tensor)
+
+
+def _unwatched(x, *parameters):
+    """Whether nobody would see a layer's own call on x: it and the parameters are plain tensors, and no mode that watches or replaces
+    tensor operations is active (a default device is not one)."""
+    if type(x) is not torch.Tensor or _dispatch_modes() or (
+            _function_modes() and any(type(m) is not DeviceContext for m in torch.overrides._get_current_function_mode_stack())):
+        return False
+    for p in parameters:
+        if type(p) not in _PLAIN:
+            return False
+    return True
 
 
 def relu_square(x, layer=None):
@@ -35,7 +51,7 @@ def linear_relu_square(key, x, layer=None):
     one kernel where that is faster: vrwkv_linear_relu_square_pays)."""
     if layer is not None and x.dtype == torch.bfloat16 and _inference(x) and autocast_linears(key, layer) and key.bias is None:
         w = key.weight
-        if (type(w) in (nn.Parameter, torch.Tensor) and w.dtype in KERNEL_DTYPES and w.device == x.device and w.dim() == 2 and w.shape[1] == x.shape[-1]
+        if (_unwatched(x, w) and w.dtype in KERNEL_DTYPES and w.device == x.device and w.dim() == 2 and w.shape[1] == x.shape[-1]
                 and w.shape[1] % 64 == 0 and w.shape[1] > 0 and w.shape[0] % 256 == 0 and w.shape[0] > 0):
             out = _lib.native().key_layer(x, w)
             if ops.CHECK_STATUS:
@@ -74,7 +90,7 @@ def layer_norm(norm, x):
     """norm(x) for a LayerNorm `norm` over the channels"""
     C = x.shape[-1]
     if (_inference(x) and x.dtype == torch.float32 and C % 4 == 0 and 0 < C <= MOST_NORM_CHANNELS and x.numel() // C < 2 ** 31
-            and _norm_kernel(x, norm, C)):
+            and _norm_kernel(x, norm, C) and _unwatched(x, norm.weight, norm.bias)):
         return _lib.native().layer_norm(x, norm.weight, norm.bias, norm.eps)
     return norm(x)
 
@@ -82,7 +98,7 @@ def layer_norm(norm, x):
 def widened(norm, a):
     """a as a LayerNorm `norm` takes it under autocast: torch widens a bfloat16 input to float32 first."""
     if (a.dtype == torch.bfloat16 and _inference(a) and a.is_contiguous() and a.numel() % 8 == 0 and a.numel() < 2 ** 33
-            and torch.is_autocast_enabled("cuda") and stock(norm, nn.LayerNorm)):
+            and torch.is_autocast_enabled("cuda") and stock(norm, nn.LayerNorm) and _unwatched(a)):
         return _lib.native().widen(a)
     return a
 
