@@ -158,6 +158,10 @@ int vrwkv_biwkv_backward_bf16_wide(int B, int T, int C, const float* w, const fl
  * backward: T <= 4096, and longer sequences up to 17 408 tokens where there are many.  A training pair has nothing to gain there from
  * kept states (next comment). */
 int vrwkv_biwkv_one_pass(int B, int T, int C, int tensors);
+/* Workspace with which the entry points above serve such calls: at most a few bytes per sequence and channel, where their own queries
+ * have room for every path (up to 8.1 bytes per element).  0 where vrwkv_biwkv_one_pass is 0; too small for calls that go another way
+ * all the same (tensors off a 16-byte boundary, vrwkv_set_path): VRWKV_ERR_WORKSPACE, nothing ran. */
+size_t vrwkv_biwkv_one_pass_workspace_bytes(int B, int T, int C, int tensors, int backward);
 
 /* The training pair for long sequences: a forward that leaves the states entering every 16 tokens (1.5 bytes per element, in a
  * caller-owned buffer of vrwkv_biwkv_kept_bytes bytes, 256-byte aligned), and a backward that starts from them instead of

@@ -191,3 +191,42 @@ def test_short_sequences_with_steep_weights_need_no_exact_kernel(cuda_device, T,
             assert rel_err(a.float(), b) <= (5e-5 if types == "f32" or n in ("gw", "gu") else 1e-2), n
         else:
             assert a.float().abs().max() <= 1e-5 * max(1.0, gy.abs().max().item())
+
+
+@pytest.mark.parametrize("B,T", [(2, 196), (1, 2000), (24, 4200)])
+@pytest.mark.parametrize("types", ["f32", "wide", "bf16"])
+def test_scratch_memory(cuda_device, B, T, types):
+    """Calls that the one-pass kernels serve need a word per CTA and the partial sums of gw and gu, less than a byte per element here, where the
+    entry points' own queries give 1.5 and 8.1; that is what a training step allocates.  Tensors that those kernels cannot take need all of it."""
+    from vision_rwkv_b200 import _lib
+    from vision_rwkv_b200.vrwkv import RUN_CUDA
+    C, lib, n, which = 64, _lib.load(), B * T * 64, ("f32", "bf16", "wide").index(types)
+    small = [lib.vrwkv_biwkv_one_pass_workspace_bytes(B, T, C, which, d) for d in (0, 1)]
+    full = [lib.vrwkv_biwkv_forward_workspace_bytes(B, T, C), lib.vrwkv_biwkv_backward_workspace_bytes(B, T, C)]
+    assert 0 < small[0] <= small[1] <= full[1] and small[0] <= full[0] and small[1] < 0.25 * n + 4096
+    w, u, k, v, gy = [x.float().to(cuda_device) for x in O.make_inputs(B, T, C, seed=T)]
+    dt = torch.float32 if types == "f32" else torch.bfloat16
+    k, v, gy = k.to(dt), v.to(dt), gy.to(dt if types == "bf16" else torch.float32)
+    name = "bf16_wide" if types == "wide" else types
+    forward = getattr(lib, "vrwkv_biwkv_forward_" + name)
+    s, p = torch.cuda.current_stream().cuda_stream, lambda t: t.data_ptr()
+    y, ws = torch.empty_like(gy), torch.empty(full[1], dtype=torch.uint8, device=cuda_device)
+    assert forward(B, T, C, p(w), p(u), p(k), p(v), p(y), p(ws), small[0], s) == 0
+    assert forward(B, T, C, p(w), p(u), p(k), p(v), p(y), p(ws), small[0] - 1, s) == 3
+    odd = torch.empty(n + 8, dtype=dt, device=cuda_device)[2:n + 2].view(B, T, C).copy_(k)      # off a 16-byte boundary
+    assert forward(B, T, C, p(w), p(u), p(odd), p(v), p(y), p(ws), small[0], s) == 3
+    ref = O.biwkv_scan_forward(*[x.double().cpu() for x in (w, u, k, v)])
+    tol = 1e-5 if types == "f32" else 1e-2
+    assert rel_err(y.float(), ref) <= tol
+    assert rel_err(RUN_CUDA(w, u, odd, v).float(), ref) <= tol
+
+    if types == "bf16":
+        w, u = w.bfloat16(), u.bfloat16()
+    xs = [x.requires_grad_(True) for x in (w, u, k, v)]
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    out = RUN_CUDA(*xs)
+    grads = torch.autograd.grad(out, xs, gy.to(out.dtype))
+    kept = out.numel() * out.element_size() + sum(g.numel() * g.element_size() for g in grads)
+    assert torch.cuda.max_memory_allocated() - before - kept < 0.25 * n + (1 << 20)

@@ -50,6 +50,7 @@ SIGNATURES = {
     "vrwkv_biwkv_forward_bf16_wide": (_c_int, [_c_int] * 3 + [_ptr] * 6 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_backward_bf16_wide": (_c_int, [_c_int] * 3 + [_ptr] * 9 + [_c_size_t, _ptr]),
     "vrwkv_biwkv_one_pass": (_c_int, [_c_int] * 4),
+    "vrwkv_biwkv_one_pass_workspace_bytes": (_c_size_t, [_c_int] * 5),
     "vrwkv_biwkv_kept_bytes": (_c_size_t, [_c_int] * 3),
     "vrwkv_biwkv_kept_workspace_bytes": (_c_size_t, [_c_int] * 4),
     "vrwkv_biwkv_forward_keep": (_c_int, [_c_int] * 3 + [_ptr] * 5 + [_c_int, _ptr, _c_size_t, _ptr, _c_size_t, _ptr]),

@@ -1306,13 +1306,9 @@ static Carve carve(int B, int C, const Plan& pl, bool bwd) {
     cv.total = cv.off_vectors + align_up(2 * static_cast<size_t>(C) * sizeof(float), 256);
     return cv;
 }
-size_t workspace_bytes(int B, int T, int C, bool bwd) {
-    size_t most = 256;
-    for (Types types : {Types::f32, Types::bf16, Types::wide}) {
-        Plan pl;
-        if (make_plan(B, T, C, bwd, types, pl)) most = std::max(most, carve(B, C, pl, bwd).total);
-    }
-    return most;
+size_t workspace_bytes(int B, int T, int C, bool bwd, Types types) {
+    Plan pl;
+    return make_plan(B, T, C, bwd, types, pl) ? carve(B, C, pl, bwd).total : 0;
 }
 
 template <class St, bool kBwd, Types kTypes>

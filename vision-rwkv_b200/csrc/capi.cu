@@ -143,15 +143,26 @@ unsigned vrwkv_take_failures(int device) {
 static bool strips_serve(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types) {
     return g_path.load() == 0 && biwkv::strips::eligible(B, T, C, ptrs, bwd, types);
 }
+// The workspace that a call must bring: where those kernels serve it, no room for the others' paths.
+static size_t scratch_bytes(bool one_pass, int B, int T, int C, Types types, bool bwd) {
+    if (one_pass) return biwkv::strips::workspace_bytes(B, T, C, bwd, types);
+    return bwd ? vrwkv_biwkv_backward_workspace_bytes(B, T, C) : vrwkv_biwkv_forward_workspace_bytes(B, T, C);
+}
 // Whether the kernels for long sequences serve the call, with what stands by behind them.
 static bool resident_serves(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, Types types) {
     return g_path.load() == 0 && biwkv::resident::eligible(B, T, C, ptrs, bwd, types) && biwkv::fused::eligible(B, T, C, ptrs, types == Types::bf16);
 }
 
+static size_t one_pass_most(int B, int T, int C, bool bwd) {
+    size_t most = 0;
+    for (Types types : {Types::f32, Types::bf16, Types::wide}) most = std::max(most, biwkv::strips::workspace_bytes(B, T, C, bwd, types));
+    return most;
+}
+
 size_t vrwkv_biwkv_forward_workspace_bytes(int B, int T, int C) {
     if (check_shape(B, T, C) != VRWKV_OK) return 0;
     return std::max({biwkv::generic_forward_workspace(B, T, C) + 256, biwkv::fused::workspace_bytes(B, T, C, false),
-                     biwkv::resident::workspace_bytes(B, T, C, false), biwkv::strips::workspace_bytes(B, T, C, false)});
+                     biwkv::resident::workspace_bytes(B, T, C, false), one_pass_most(B, T, C, false)});
 }
 
 int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u, const float* k,
@@ -162,9 +173,10 @@ int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u,
     if (misaligned4(w) || misaligned4(u) || misaligned4(k) || misaligned4(v) || misaligned4(y) ||
         (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    const bool one_pass = strips_serve(B, T, C, {k, v, y}, false, Types::f32);
+    if (workspace_bytes < scratch_bytes(one_pass, B, T, C, Types::f32, false)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (strips_serve(B, T, C, {k, v, y}, false, Types::f32)) return finish(biwkv::strips::forward(B, T, C, w, u, k, v, y, Types::f32, workspace, s));
+    if (one_pass) return finish(biwkv::strips::forward(B, T, C, w, u, k, v, y, Types::f32, workspace, s));
     if (resident_serves(B, T, C, {k, v, y}, false, Types::f32))
         return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::f32, workspace, s));
     if (g_path.load() != 1 && biwkv::fused::eligible(B, T, C, {k, v, y}))
@@ -177,7 +189,7 @@ int vrwkv_biwkv_forward_f32(int B, int T, int C, const float* w, const float* u,
 size_t vrwkv_biwkv_backward_workspace_bytes(int B, int T, int C) {
     if (check_shape(B, T, C) != VRWKV_OK) return 0;
     return std::max({biwkv::generic_backward_workspace(B, T, C) + 256, biwkv::fused::workspace_bytes(B, T, C, true),
-                     biwkv::resident::workspace_bytes(B, T, C, true), biwkv::strips::workspace_bytes(B, T, C, true)});
+                     biwkv::resident::workspace_bytes(B, T, C, true), one_pass_most(B, T, C, true)});
 }
 
 int vrwkv_biwkv_backward_f32(int B, int T, int C, const float* w, const float* u, const float* k,
@@ -188,9 +200,10 @@ int vrwkv_biwkv_backward_f32(int B, int T, int C, const float* w, const float* u
     if (misaligned4(w) || misaligned4(u) || misaligned4(k) || misaligned4(v) || misaligned4(gy) ||
         misaligned4(gwgu) || misaligned4(gk) || misaligned4(gv) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
+    const bool one_pass = strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::f32);
+    if (workspace_bytes < scratch_bytes(one_pass, B, T, C, Types::f32, true)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::f32))
+    if (one_pass)
         return finish(biwkv::strips::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::f32, workspace, s));
     if (resident_serves(B, T, C, {k, v, gy, gk, gv}, true, Types::f32))
         return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::f32, workspace, s));
@@ -210,6 +223,11 @@ static bool types_of(int types, Types& t) {
 int vrwkv_biwkv_one_pass(int B, int T, int C, int tensors) {
     Types types;
     return check_shape(B, T, C) == VRWKV_OK && types_of(tensors, types) && biwkv::strips::in_range(B, T, C, types) ? 1 : 0;
+}
+
+size_t vrwkv_biwkv_one_pass_workspace_bytes(int B, int T, int C, int tensors, int backward) {
+    Types types;
+    return check_shape(B, T, C) == VRWKV_OK && types_of(tensors, types) ? biwkv::strips::workspace_bytes(B, T, C, backward != 0, types) : 0;
 }
 
 size_t vrwkv_biwkv_kept_bytes(int B, int T, int C) {
@@ -282,8 +300,9 @@ int vrwkv_biwkv_forward_bf16(int B, int T, int C, const float* w, const float* u
     if (int st = check_shape(B, T, C)) return st;
     if (!w || !u || !k || !v || !y || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
-    if (strips_serve(B, T, C, {k, v, y}, false, Types::bf16))
+    const bool one_pass = strips_serve(B, T, C, {k, v, y}, false, Types::bf16);
+    if (workspace_bytes < scratch_bytes(one_pass, B, T, C, Types::bf16, false)) return VRWKV_ERR_WORKSPACE;
+    if (one_pass)
         return finish(biwkv::strips::forward(B, T, C, w, u, k, v, y, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
     if (resident_serves(B, T, C, {k, v, y}, false, Types::bf16))
         return finish(biwkv::resident::forward(B, T, C, w, u, k, v, y, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
@@ -298,8 +317,9 @@ int vrwkv_biwkv_backward_bf16(int B, int T, int C, const float* w, const float* 
     if (!w || !u || !k || !v || !gy || !gwgu || !gk || !gv || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || misaligned4(gwgu) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
-    if (strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::bf16))
+    const bool one_pass = strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::bf16);
+    if (workspace_bytes < scratch_bytes(one_pass, B, T, C, Types::bf16, true)) return VRWKV_ERR_WORKSPACE;
+    if (one_pass)
         return finish(biwkv::strips::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
     if (resident_serves(B, T, C, {k, v, gy, gk, gv}, true, Types::bf16))
         return finish(biwkv::resident::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::bf16, workspace, static_cast<cudaStream_t>(stream)));
@@ -313,8 +333,9 @@ int vrwkv_biwkv_forward_bf16_wide(int B, int T, int C, const float* w, const flo
     if (int st = check_shape(B, T, C)) return st;
     if (!w || !u || !k || !v || !y || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < vrwkv_biwkv_forward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
-    if (!strips_serve(B, T, C, {k, v, y}, false, Types::wide)) return VRWKV_ERR_UNSUPPORTED;
+    const bool one_pass = strips_serve(B, T, C, {k, v, y}, false, Types::wide);
+    if (workspace_bytes < scratch_bytes(one_pass, B, T, C, Types::wide, false)) return VRWKV_ERR_WORKSPACE;
+    if (!one_pass) return VRWKV_ERR_UNSUPPORTED;
     return finish(biwkv::strips::forward(B, T, C, w, u, k, v, y, Types::wide, workspace, static_cast<cudaStream_t>(stream)));
 }
 
@@ -325,8 +346,9 @@ int vrwkv_biwkv_backward_bf16_wide(int B, int T, int C, const float* w, const fl
     if (!w || !u || !k || !v || !gy || !gwgu || !gk || !gv || !workspace) return VRWKV_ERR_NULL;
     if (misaligned4(w) || misaligned4(u) || misaligned4(gwgu) || (reinterpret_cast<uintptr_t>(workspace) & 255u))
         return VRWKV_ERR_ALIGNMENT;
-    if (workspace_bytes < vrwkv_biwkv_backward_workspace_bytes(B, T, C)) return VRWKV_ERR_WORKSPACE;
-    if (!strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::wide)) return VRWKV_ERR_UNSUPPORTED;
+    const bool one_pass = strips_serve(B, T, C, {k, v, gy, gk, gv}, true, Types::wide);
+    if (workspace_bytes < scratch_bytes(one_pass, B, T, C, Types::wide, true)) return VRWKV_ERR_WORKSPACE;
+    if (!one_pass) return VRWKV_ERR_UNSUPPORTED;
     return finish(biwkv::strips::backward(B, T, C, w, u, k, v, gy, gwgu, gk, gv, Types::wide, workspace, static_cast<cudaStream_t>(stream)));
 }
 

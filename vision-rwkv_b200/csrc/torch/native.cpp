@@ -82,6 +82,19 @@ bool biwkv_forward_keep(const Tensor& w, const Tensor& u, const Tensor& k, const
     return true;
 }
 
+// A Bi-WKV entry point with the scratch memory it needs: little where the one-pass kernels serve the sizes, all of it where they cannot
+// be had for these tensors after all.  call(workspace) returns a status; the last one is the result.
+template <typename F>
+int with_scratch(const Tensor& k, int types, bool backward, F&& call) {
+    const int B = k.size(0), T = k.size(1), C = k.size(2);
+    const size_t bytes = vrwkv_biwkv_one_pass_workspace_bytes(B, T, C, types, backward);
+    if (bytes != 0) {
+        const int st = call(workspace(bytes, k));
+        if (st != VRWKV_ERR_WORKSPACE) return st;
+    }
+    return call(workspace(backward ? vrwkv_biwkv_backward_workspace_bytes(B, T, C) : vrwkv_biwkv_forward_workspace_bytes(B, T, C), k));
+}
+
 // k, v float32 or both bfloat16, contiguous; y in their dtype.  kept: null, or receives the states for a backward (left
 // undefined where none are kept).
 Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v, Tensor* kept = nullptr) {
@@ -92,16 +105,17 @@ Tensor biwkv_forward_raw(const Tensor& w, const Tensor& u, const Tensor& k, cons
         raise_failures(k.get_device(), "vrwkv_biwkv_forward");
         return y;
     }
-    Tensor ws = workspace(vrwkv_biwkv_forward_workspace_bytes(B, T, C), k);
     if (is_bf16(k)) {
-        const int st = vrwkv_biwkv_forward_bf16(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
-                                                static_cast<uint16_t*>(v.data_ptr()), static_cast<uint16_t*>(y.data_ptr()),
-                                                ws.data_ptr(), ws.numel(), stream_of(k));
+        const int st = with_scratch(k, VRWKV_TENSORS_BF16, false, [&](const Tensor& ws) {
+            return vrwkv_biwkv_forward_bf16(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()),
+                                            static_cast<uint16_t*>(y.data_ptr()), ws.data_ptr(), ws.numel(), stream_of(k));
+        });
         if (st == VRWKV_ERR_UNSUPPORTED) return biwkv_forward_raw(w, u, f32(k), f32(v)).to(at::kBFloat16);
         check(st, "vrwkv_biwkv_forward_bf16");
     } else {
-        check(vrwkv_biwkv_forward_f32(B, T, C, fp(w), fp(u), fp(k), fp(v), fp(y), ws.data_ptr(), ws.numel(), stream_of(k)),
-              "vrwkv_biwkv_forward_f32");
+        check(with_scratch(k, VRWKV_TENSORS_F32, false, [&](const Tensor& ws) {
+                  return vrwkv_biwkv_forward_f32(B, T, C, fp(w), fp(u), fp(k), fp(v), fp(y), ws.data_ptr(), ws.numel(), stream_of(k));
+              }), "vrwkv_biwkv_forward_f32");
     }
     raise_failures(k.get_device(), "vrwkv_biwkv_forward");
     return y;
@@ -116,9 +130,10 @@ Tensor biwkv_forward_wide(const Tensor& w, const Tensor& u, const Tensor& k, con
     const int B = k.size(0), T = k.size(1), C = k.size(2);
     Tensor y = at::empty_like(k, k.options().dtype(at::kFloat));
     if (k.numel() == 0) return y;
-    Tensor ws = workspace(vrwkv_biwkv_forward_workspace_bytes(B, T, C), k);
-    const int st = vrwkv_biwkv_forward_bf16_wide(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()),
-                                                 static_cast<uint16_t*>(v.data_ptr()), fp(y), ws.data_ptr(), ws.numel(), stream_of(k));
+    const int st = with_scratch(k, VRWKV_TENSORS_BF16_WIDE, false, [&](const Tensor& ws) {
+        return vrwkv_biwkv_forward_bf16_wide(B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()), fp(y),
+                                             ws.data_ptr(), ws.numel(), stream_of(k));
+    });
     if (st == VRWKV_ERR_UNSUPPORTED) return Tensor();
     check(st, "vrwkv_biwkv_forward_bf16_wide");
     raise_failures(k.get_device(), "vrwkv_biwkv_forward");
@@ -160,37 +175,35 @@ std::array<Tensor, 4> biwkv_backward_raw(const Tensor& w, const Tensor& u, const
         gwgu.zero_();
         return {gwgu.select(0, 0), gwgu.select(0, 1), gk, gv};
     }
-    Tensor ws;
     int resumed = VRWKV_ERR_UNSUPPORTED;
     if (kept.defined()) {
-        ws = workspace(vrwkv_biwkv_kept_workspace_bytes(B, T, C, 1), k);
+        const Tensor ws = workspace(vrwkv_biwkv_kept_workspace_bytes(B, T, C, 1), k);
         resumed = vrwkv_biwkv_backward_kept(B, T, C, fp(w), fp(u), k.data_ptr(), v.data_ptr(), gy.data_ptr(), fp(gwgu), gk.data_ptr(),
                                             gv.data_ptr(), is_bf16(k) ? VRWKV_TENSORS_BF16 : VRWKV_TENSORS_F32, kept.data_ptr(), kept.numel(), ws.data_ptr(), ws.numel(), stream_of(k));
         if (resumed != VRWKV_ERR_UNSUPPORTED) check(resumed, "vrwkv_biwkv_backward_kept");
     }
-    if (resumed != VRWKV_OK) ws = workspace(vrwkv_biwkv_backward_workspace_bytes(B, T, C), k);
+    const auto half = [](const Tensor& t) { return static_cast<uint16_t*>(t.data_ptr()); };
     if (resumed == VRWKV_OK) {
         // done
     } else if (is_bf16(k) && !is_bf16(gy)) {
-        const int st = vrwkv_biwkv_backward_bf16_wide(
-            B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()), fp(gy), fp(gwgu),
-            static_cast<uint16_t*>(gk.data_ptr()), static_cast<uint16_t*>(gv.data_ptr()), ws.data_ptr(), ws.numel(), stream_of(k));
+        const int st = with_scratch(k, VRWKV_TENSORS_BF16_WIDE, true, [&](const Tensor& ws) {
+            return vrwkv_biwkv_backward_bf16_wide(B, T, C, fp(w), fp(u), half(k), half(v), fp(gy), fp(gwgu), half(gk), half(gv), ws.data_ptr(), ws.numel(), stream_of(k));
+        });
         if (st == VRWKV_ERR_UNSUPPORTED) return biwkv_backward_raw(w, u, k, v, gy.to(at::kBFloat16));
         check(st, "vrwkv_biwkv_backward_bf16_wide");
     } else if (is_bf16(k)) {
-        const int st = vrwkv_biwkv_backward_bf16(
-            B, T, C, fp(w), fp(u), static_cast<uint16_t*>(k.data_ptr()), static_cast<uint16_t*>(v.data_ptr()),
-            static_cast<uint16_t*>(gy.data_ptr()), fp(gwgu), static_cast<uint16_t*>(gk.data_ptr()),
-            static_cast<uint16_t*>(gv.data_ptr()), ws.data_ptr(), ws.numel(), stream_of(k));
+        const int st = with_scratch(k, VRWKV_TENSORS_BF16, true, [&](const Tensor& ws) {
+            return vrwkv_biwkv_backward_bf16(B, T, C, fp(w), fp(u), half(k), half(v), half(gy), fp(gwgu), half(gk), half(gv), ws.data_ptr(), ws.numel(), stream_of(k));
+        });
         if (st == VRWKV_ERR_UNSUPPORTED) {
             auto g = biwkv_backward_raw(w, u, f32(k), f32(v), f32(gy));
             return {g[0], g[1], g[2].to(at::kBFloat16), g[3].to(at::kBFloat16)};
         }
         check(st, "vrwkv_biwkv_backward_bf16");
     } else {
-        check(vrwkv_biwkv_backward_f32(B, T, C, fp(w), fp(u), fp(k), fp(v), fp(gy), fp(gwgu), fp(gk), fp(gv), ws.data_ptr(),
-                                       ws.numel(), stream_of(k)),
-              "vrwkv_biwkv_backward_f32");
+        check(with_scratch(k, VRWKV_TENSORS_F32, true, [&](const Tensor& ws) {
+                  return vrwkv_biwkv_backward_f32(B, T, C, fp(w), fp(u), fp(k), fp(v), fp(gy), fp(gwgu), fp(gk), fp(gv), ws.data_ptr(), ws.numel(), stream_of(k));
+              }), "vrwkv_biwkv_backward_f32");
     }
     raise_failures(k.get_device(), "vrwkv_biwkv_backward");
     return {gwgu.select(0, 0), gwgu.select(0, 1), gk, gv};

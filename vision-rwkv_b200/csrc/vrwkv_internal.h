@@ -62,7 +62,7 @@ bool in_range(int B, int T, int C, resident::Types types);
 // ... and the current device can launch them
 bool eligible(int B, int T, int C, std::initializer_list<const void*> ptrs, bool bwd, resident::Types types);
 void set_withhold_test(bool on);
-size_t workspace_bytes(int B, int T, int C, bool bwd);
+size_t workspace_bytes(int B, int T, int C, bool bwd, resident::Types types);      // 0 outside in_range
 int forward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, void* y, resident::Types types,
             void* workspace, cudaStream_t stream);
 int backward(int B, int T, int C, const float* w, const float* u, const void* k, const void* v, const void* gy, float* gwgu,
