@@ -52,7 +52,8 @@ def test_edges(cuda_device, T, C, types):
 @pytest.mark.parametrize("w_range", [(-30.0, -1.0), (1.0, 30.0), (-5.0, 3.0)])
 def test_steep_weights(cuda_device, T, w_range):
     """Weights that grow or fall by orders of magnitude within the sequence: past its end they would overflow, or leave a denominator of
-    zero, and nothing of that may reach a valid token.  Each is inside the plain-float range for some channels and outside for others.
+    zero, and nothing of that may reach a valid token.  The shortest sequences are outside the plain-float range where weights grow most, the others
+    inside (both kinds in one call: test_units_inside_and_outside_the_plain_float_range).
     Tolerance: 5e-5, that of test_biwkv_gpu.py for extreme exponents."""
     for types, tol in (("f32", 5e-5), ("wide", 1e-2)):
         errs = errors(cuda_device, 3, T, 48, types, w_range)
@@ -230,3 +231,34 @@ def test_scratch_memory(cuda_device, B, T, types):
     grads = torch.autograd.grad(out, xs, gy.to(out.dtype))
     kept = out.numel() * out.element_size() + sum(g.numel() * g.element_size() for g in grads)
     assert torch.cuda.max_memory_allocated() - before - kept < 0.25 * n + (1 << 20)
+
+
+@pytest.mark.parametrize("T", [50, 200, 1000, 2000, 4096])
+@pytest.mark.parametrize("types", ["f32", "wide"])
+def test_units_inside_and_outside_the_plain_float_range(cuda_device, T, types):
+    """Weights that grow by e^10 to e^100 over the sequence, from channel to channel, and large k in one strip of one sequence: the exact kernel
+    serves some units of a call and skips the others, in single CTAs and in clusters.  Tolerance: 5e-5, that of test_biwkv_gpu.py for extreme exponents."""
+    from vision_rwkv_b200 import _lib
+    B, C, lib = 3, 80, _lib.load()
+    w, u, k, v, gy = [x.float().to(cuda_device) for x in O.make_inputs(B, T, C, seed=T)]
+    w = torch.linspace(-100, -10, C, device=cuda_device) / T
+    k = k.clamp(-1, 1)
+    k[1, ::7, 70] *= 60
+    dt = torch.float32 if types == "f32" else torch.bfloat16
+    k, v, gy = k.to(dt), v.to(dt), gy.to(dt).float()
+    y, gk, gv, gwgu = torch.empty_like(gy), torch.empty_like(k), torch.empty_like(k), torch.empty(2, C, device=cuda_device)
+    name, which = ("f32", 0) if types == "f32" else ("bf16_wide", 2)
+    ws = [torch.full((lib.vrwkv_biwkv_one_pass_workspace_bytes(B, T, C, which, d),), 0xFF, dtype=torch.uint8, device=cuda_device) for d in (0, 1)]
+    s, p = torch.cuda.current_stream().cuda_stream, lambda t: t.data_ptr()
+    assert getattr(lib, "vrwkv_biwkv_forward_" + name)(B, T, C, p(w), p(u), p(k), p(v), p(y), p(ws[0]), ws[0].numel(), s) == 0
+    assert getattr(lib, "vrwkv_biwkv_backward_" + name)(B, T, C, p(w), p(u), p(k), p(v), p(gy), p(gwgu), p(gk), p(gv), p(ws[1]), ws[1].numel(), s) == 0
+    words = ws[0][256:-768].view(torch.int32)      # of the forward's CTAs: 1 for a unit left to the exact kernel, 0 for one that was not
+    words = words[words >= 0]
+    assert set(words.tolist()) == {0, 1}
+    # strips of 8 or 16 channels: the last 32 channels are inside the range, but for one strip of the sequence with large k
+    per_sequence = words.view(B, -1).sum(1)
+    assert per_sequence[0] == per_sequence[2] < per_sequence[1] < words.numel() // B
+    f = [x.double().cpu() for x in (w, u, k, v, gy)]
+    ref = (O.biwkv_scan_forward(*f[:4]), *O.biwkv_scan_backward(*f))
+    for a, b, n in zip((y, gwgu[0], gwgu[1], gk, gv), ref, NAMES):
+        assert rel_err(a.float(), b) <= (5e-5 if types == "f32" or n in ("gw", "gu") else 1e-2), n
