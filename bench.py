@@ -444,7 +444,7 @@ def sec_biwkv_bf16(cx, hl):
 
 def sec_sequence_sweep(cx):
     """Bi-WKV forward+backward against sequence length at B=8, C=768, fp32: cost per token stays flat."""
-    from vision_rwkv_b200 import ops
+    from vision_rwkv_b200 import _lib, ops
     rows = []
     for T in (1024, 4096, 16384):
         B, C = 8, 768
@@ -453,7 +453,8 @@ def sec_sequence_sweep(cx):
         gbs = (BYTES_FWD + BYTES_BWD) * B * T * C / (ms * 1e-3) / 1e9
         rows.append({"T": T, "fwd_ms": f, "bwd_ms": b, "ms": ms, "us_per_token": ms * 1e3 / (B * T),
                      "algorithmic_GBps": gbs, "frac_of_hbm_peak": cx.frac(gbs),
-                     "kernels": "one CTA or cluster per sequence strip"})
+                     "kernels": "one CTA or cluster per sequence strip" if _lib.load().vrwkv_biwkv_one_pass(B, T, C, 0)
+                     else "several clusters per sequence strip, or separate launches"})
         del k, v, gy
     return {"B": 8, "C": 768, "dtype": "f32", "per_gpu": True, "rows": rows}
 

@@ -74,7 +74,7 @@ def allocated(f):
 
 @pytest.mark.parametrize("half", [False, True])
 def test_nothing_is_allocated_twice(cuda_device, half):
-    """bfloat16 k, v with float32 w, as under autocast, have no kernels for a float32 y or gy above 4096 tokens: y is widened and gy
+    """bfloat16 k, v with float32 w, as under autocast, have no kernels for a float32 y or gy at this size (vrwkv_biwkv_one_pass): y is widened and gy
     narrowed around the bfloat16 ones, and nothing else is set up first."""
     from vision_rwkv_b200 import _lib
     from vision_rwkv_b200.vrwkv import RUN_CUDA

@@ -127,7 +127,7 @@ struct Params {
     float* states2;       // level 2 (backward)
     float* ctas2;
     int state_rows;       // kStateRows, or kPlainRows where no moments are kept
-    unsigned* out_of_range;   // sequences longer than one cluster holds: inputs outside the plain-float range were seen; else null
+    unsigned* out_of_range;   // inputs outside the plain-float range were seen
     bool reverse;         // last CTAs first: what the launch before this one read last is still in L2
 };
 
@@ -468,11 +468,11 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     // every warp sends the blocks to its share of the other CTAs (rank = warp, warp + n_warps, ...):
     // lane = channel, one record per lane, lane 0 also the flag word
     if (level == 1) TL_MARK(24);
-    if (!kLocal && c.cluster > 1) {
+    if (!kLocal) {
         __syncthreads();
     }
     if (level == 1) TL_MARK(25);
-    if (!kLocal && c.cluster > 1 && !c.withhold) {
+    if (!kLocal && !c.withhold) {
         const uint32_t bar_off = sm100::smem_u32(c.xbar + level) - sm100::smem_u32(c.peers);
         for (int r = warp; r < c.cluster; r += nw) {
             if (r == c.rank) continue;
@@ -491,7 +491,7 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     TL_MARK(13 + level * 5);
     // (3) wait for the other CTAs' bytes, combine them
     bool heard = true;
-    if (!kLocal && c.cluster > 1 && (warp == scanF || warp == scanR)) {
+    if (!kLocal && (warp == scanF || warp == scanR)) {
         heard = sm100::mbar_wait(c.xbar + level, 0, c.spin_limit);
         if (!heard && lane == 0) gave_up(c, 1u);
     }
@@ -499,36 +499,34 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     if (!kLocal && warp == scanF) {
         float2 X = f2(0.f, 0.f), MX = f2(0.f, 0.f);
         int flag = any;
-        if (c.cluster > 1) {
-            const float2 hi2 = dup(c.consts[kLamC_hi * kCs + lane]), lo2 = dup(c.consts[kLamC_lo * kCs + lane]);
-            const float2 len2 = dup(static_cast<float>(c.n_tok));
-            for (int r0 = 0; r0 < c.rank; r0 += kBatch) {
-                float2 f[kBatch], mf[kBatch];
+        const float2 hi2 = dup(c.consts[kLamC_hi * kCs + lane]), lo2 = dup(c.consts[kLamC_lo * kCs + lane]);
+        const float2 len2 = dup(static_cast<float>(c.n_tok));
+        for (int r0 = 0; r0 < c.rank; r0 += kBatch) {
+            float2 f[kBatch], mf[kBatch];
 #pragma unroll
-                for (int j = 0; j < kBatch; ++j) {
-                    f[j] = f2(0.f, 0.f);
-                    mf[j] = f2(0.f, 0.f);
-                    if (r0 + j < c.rank) {
-                        const float* q = c.peers + (r0 + j) * RW::kBlockF + lane * RW::kF;      // lower ranks: slot = rank
-                        if (kMom) {
-                            const float4 t = *reinterpret_cast<const float4*>(q);
-                            f[j] = f2(t.x, t.y);
-                            mf[j] = f2(t.z, t.w);
-                        } else {
-                            f[j] = *reinterpret_cast<const float2*>(q);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < kBatch; ++j) {
-                    if (r0 + j < c.rank) {
-                        if (kMom) MX = mulc_add(fma2(len2, X, MX), hi2, lo2, mf[j]);
-                        X = mulc_add(X, hi2, lo2, f[j]);
+            for (int j = 0; j < kBatch; ++j) {
+                f[j] = f2(0.f, 0.f);
+                mf[j] = f2(0.f, 0.f);
+                if (r0 + j < c.rank) {
+                    const float* q = c.peers + (r0 + j) * RW::kBlockF + lane * RW::kF;      // lower ranks: slot = rank
+                    if (kMom) {
+                        const float4 t = *reinterpret_cast<const float4*>(q);
+                        f[j] = f2(t.x, t.y);
+                        mf[j] = f2(t.z, t.w);
+                    } else {
+                        f[j] = *reinterpret_cast<const float2*>(q);
                     }
                 }
             }
-            if (level == 0) flag = cluster_flag<RW>(c, any || !heard);
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                if (r0 + j < c.rank) {
+                    if (kMom) MX = mulc_add(fma2(len2, X, MX), hi2, lo2, mf[j]);
+                    X = mulc_add(X, hi2, lo2, f[j]);
+                }
+            }
         }
+        if (level == 0) flag = cluster_flag<RW>(c, any || !heard);
         if (kLinked) seg_exchange_forward<kMom>(c, level, X, MX, ctaP, ctaM, flag);
         c.cta[lane] = X.x; c.cta[kCs + lane] = X.y;
         if (kMom) { c.cta[2 * kCs + lane] = MX.x; c.cta[3 * kCs + lane] = MX.y; }
@@ -536,23 +534,21 @@ __device__ __forceinline__ Enter fast_exchange(const Ctx& c, int level, Pair2 F,
     }
     if (!kLocal && warp == scanR) {
         float2 Y = f2(0.f, 0.f);
-        if (c.cluster > 1) {
-            const float2 hi2 = dup(c.consts[kLamC_hi * kCs + lane]), lo2 = dup(c.consts[kLamC_lo * kCs + lane]);
-            for (int r0 = c.cluster - 1; r0 > c.rank; r0 -= kBatch) {
-                float2 f[kBatch];
+        const float2 hi2 = dup(c.consts[kLamC_hi * kCs + lane]), lo2 = dup(c.consts[kLamC_lo * kCs + lane]);
+        for (int r0 = c.cluster - 1; r0 > c.rank; r0 -= kBatch) {
+            float2 f[kBatch];
 #pragma unroll
-                for (int j = 0; j < kBatch; ++j) {
-                    f[j] = f2(0.f, 0.f);
-                    if (r0 - j > c.rank) f[j] = *reinterpret_cast<const float2*>(c.peers + (r0 - j - 1) * RW::kBlockF + lane * 2);
-                }
-#pragma unroll
-                for (int j = 0; j < kBatch; ++j)
-                    if (r0 - j > c.rank) Y = mulc_add(Y, hi2, lo2, f[j]);
+            for (int j = 0; j < kBatch; ++j) {
+                f[j] = f2(0.f, 0.f);
+                if (r0 - j > c.rank) f[j] = *reinterpret_cast<const float2*>(c.peers + (r0 - j - 1) * RW::kBlockF + lane * 2);
             }
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j)
+                if (r0 - j > c.rank) Y = mulc_add(Y, hi2, lo2, f[j]);
         }
         if (kLinked) {
             int flag = 0;
-            if (level == 0) flag = c.cluster > 1 ? cluster_flag<RW>(c, any || !heard) : any;
+            if (level == 0) flag = cluster_flag<RW>(c, any || !heard);
             seg_exchange_reverse(c, level, Y, ctaS, flag);
             if (lane == 0) c.flag[1] = static_cast<unsigned>(flag);
         }
@@ -669,7 +665,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     c.warp = warp; c.lane = lane; c.n_warps = nw; c.n_tok = p.n_tok; c.cluster = p.cluster;
     const int blk_id = kMode == Mode::spread && p.reverse ? static_cast<int>(gridDim.x - 1 - blockIdx.x) : static_cast<int>(blockIdx.x);
     const int unit = blk_id / p.ctas, cta = blk_id - unit * p.ctas;
-    c.rank = kCluster && p.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
+    c.rank = kCluster ? static_cast<int>(cluster_rank()) : 0;
     c.spin_limit = p.spin_limit;
     c.withhold = c.rank == p.withhold_rank;
 
@@ -733,7 +729,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         c.flag[2] = 0u;
         for (int l = 0; l < RW::kLevels; ++l) sm100::mbar_init(c.xbar + l, 1);
         sm100::mbar_init_fence();
-        if (kCluster && p.cluster > 1) {
+        if (kCluster) {
             // bytes the other CTAs will send per level: a block from every lower rank (towards later
             // tokens) and from every higher rank (towards earlier ones)
             const uint32_t bytes = static_cast<uint32_t>(c.rank) * (kCs * RW::kF + 1) * 4u + static_cast<uint32_t>(p.cluster - 1 - c.rank) * (kCs * RW::kR + 1) * 4u;
@@ -775,7 +771,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     // every CTA of the cluster has initialised its mbarriers before any other CTA sends to them:
     // arrive here, wait once the tiles have landed (long since complete by then)
     // (relaxed: the mbarrier-init fence above is what publishes the initialisation)
-    if (kCluster && p.cluster > 1) cluster_arrive_relaxed();
+    if (kCluster) cluster_arrive_relaxed();
     const int ch0 = strip * kCs + 2 * pr;
     const float2 w2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.w + ch0) : f2(0.f, 0.f);
     const float2 u2 = (ch0 < p.C) ? *reinterpret_cast<const float2*>(p.u + ch0) : f2(0.f, 0.f);
@@ -785,7 +781,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
 
     TL_MARK(1);
     if (!sm100::mbar_wait(full + warp, 0, kSpinLimit)) report_failure(p.status, p.mirror, 2u);
-    if (kCluster && p.cluster > 1) cluster_wait();
+    if (kCluster) cluster_wait();
     TL_MARK(2);
 
     const int row0 = warp * kSpan + upper * kL;
@@ -908,7 +904,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         // the records the other CTAs sent for level 1 have been consumed: tell them (they wait for
         // this before sending level 2 into the same slots).  The reads are complete: their values
         // went into shared memory before the CTA barrier that precedes this point.
-        if (kCluster && p.cluster > 1) cluster_arrive_relaxed();
+        if (kCluster) cluster_arrive_relaxed();
         // ---- backward, pass 2: recompute Den, y; G = gy / Den (in place of gy), -H = -G y (registers);
         //      gu; gw from pairs (output later than input); aggregates of [G, -H] ----
         float2 hn[kL];
@@ -978,7 +974,7 @@ biwkv_resident_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         }
         bool ignored = false;
         TL_MARK(5);
-        if (kCluster && p.cluster > 1) cluster_wait();
+        if (kCluster) cluster_wait();
         if (kOwn2) e2 = fast_exchange<RW, kSums, kLinked>(c, 1, rr, mr, q, ignored TL_PASS);
         else add_outside<true>(e2, c.sub + 2 * pr, kStateRows, wl2, dP, dS);
         if (kSums) {
@@ -1078,7 +1074,7 @@ reduce_partials(Params p, float* __restrict__ out) {
     __shared__ float red[32][33];
     const int strip = blockIdx.x, j = blockIdx.y, lane = threadIdx.x;
     const int ch = strip * kCs + lane;
-    if (p.out_of_range != nullptr && *p.out_of_range != 0u) return;       // the chunked kernels redo the whole call and write gw, gu
+    if (*p.out_of_range != 0u) return;       // the chunked kernels redo the whole call and write gw, gu
     const int per_unit = p.ctas;
     const int rows = p.B * per_unit;
     float acc = 0.f;

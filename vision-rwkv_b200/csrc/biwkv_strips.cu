@@ -1189,7 +1189,7 @@ static bool make_plan(int B, int T, int C, bool bwd, Types types, Plan& best) {
         pl.cluster = up(T, kMaxWarps * span);
         pl.n_warps = up(up(T, pl.cluster), span);
         pl.n_tok = pl.n_warps * span;
-        if (pl.cluster > kMaxCluster || (pl.cluster - 1) * pl.n_tok >= T) continue;      // every CTA owns a token
+        if (pl.cluster > kMaxCluster) continue;      // every CTA owns a token: T > (cluster - 1) kMaxWarps span
         if (g_withhold.load() && pl.cluster == 1 && i != 0) continue;      // the test wants a hand-over where there can be one
         const float cost = plan_cost(T, bwd, types, pl);
         if (best.strip < 0 || cost < least) {
