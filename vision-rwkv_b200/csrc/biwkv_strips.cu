@@ -30,17 +30,23 @@
 // time.  Hence no first moments (biwkv_backward_kernel), one read of the terms, single factors instead of (high, low) pairs within a
 // warp, constants by products.
 //
-// Measured, forward / backward us at 100.7 M elements (C = 768), float32, beside the kernels with strips of 32 channels and 16 tokens per
-// walker that were here: T=64 173 / 349 (173 / 370), 196 174 / 337 (200 / 476), 576 200 / 375 (232 / 567), 1024 190 / 374 (206 / 482),
-// 4096 224 / 486 (257 / 648); bfloat16 k, v beside float32 y, gy: T=196 153 / 356 (214 / 486), 576 174 / 406 (239 / 554), 4096 216 / 506
-// (261 / 629).  HBM at its measured rate: float32 185 / 308, bfloat16 123 / 185.  A persistent kernel that kept the terms in tensor
-// memory, so that tiles of the next unit arrived meanwhile, was slower (T=1024 530 for 431 of the kernel it was made from): not the
-// tiles are waited for but the steps of the arithmetic.
+// Measured, calls in captured loops (all their kernels), forward / backward us at 100.7 M elements (C = 768), float32, beside the kernels
+// with strips of 32 channels and 16 tokens per walker that were here: T=64 190 / 375 (181 / 398), 196 179 / 354 (203 / 488), 576
+// 201 / 388 (233 / 574), 1024 192 / 380 (208 / 490), 4096 219 / 487 (258 / 654), 16384 285 / 658 (358 / 688); bfloat16 k, v beside float32
+// y, gy: T=196 157 / 370 (228 / 488), 576 196 / 400 (242 / 563), 4096 222 / 512 (268 / 641), 16384 281 / 738 (545 / 718).  At the rate of a
+// plain copy float32 would take 185 / 308, bfloat16 123 / 185; a forward, which reads twice what it writes, can be a little faster than
+// that (T=196).  Where a sequence fills less than a warp's span, CTAs of one warp are started and ended faster than they work: 256
+// sequences of 2 to 30 tokens, C = 1024, 27.5 to 29 / 55 to 58 us (24.6 / 47 to 51).
+// A persistent kernel that kept the terms in tensor memory, so that tiles of the next unit arrived meanwhile, was slower (T=1024
+// backward 530 for 431 of the kernel it was made from): not the tiles are waited for but the steps of the arithmetic.
 //
 // Arithmetic, exactness and the exact kernel: plain floats without exponent shift, safe whenever 2 max|k| + |u| + |w| + max(-w, 0) T
-// <= 60 (and rows past T grow by little, kSafePast); each thread checks its own tokens, the first exchange carries the OR, and every CTA leaves a word that
-// says whether its unit is left to biwkv_exact_kernel (per-token max-shifted arithmetic, launched behind).  Decays over
-// half a walker and more come from double precision.
+// <= 60 (and rows past T grow by little, kSafePast); each thread checks its own tokens, the first exchange carries the OR, and every CTA
+// leaves a word that says whether its unit is left to biwkv_exact_kernel (per-token max-shifted arithmetic, launched behind).  Decays over
+// half a walker and more come from double precision, as one float within a warp, as (high, low) pairs between warps and CTAs.  That and
+// the chain of a cluster's CTAs in float32 (it was in double) cost no accuracy: for weights as the models start from, 2-norm errors
+// against float64 at T = 17 .. 17408 are below those of the kernels that were here in every result, at T = 16384 y 2.1e-7 for 2.4e-7, gw
+// 5.7e-7 for 6.3e-7.  (With max(-w, 0) T of 30 to 40 at T = 4096 gk and gv are 3.1e-7 for 2.9e-7, all else below there too.)
 //
 // Recurrence restated: classification/mmcls_custom/models/backbones/cuda_new/bi_wkv_kernel.cu:21-116 (forward), :119-367
 // (gradients).
@@ -152,8 +158,7 @@ __device__ __forceinline__ void strip_constants(float* consts, const Params& p, 
     constexpr int kCs = St::kCs;
     if (threadIdx.x >= 2 * kCs) return;
     const int ch = threadIdx.x & (kCs - 1), at = strip * kCs + ch;
-    // a single token is not decayed: whatever w is, the rows that fill up its walker must not grow with it
-    const float w = at < p.C && p.T > 1 ? __ldg(p.w + at) : 0.f, u = at < p.C ? __ldg(p.u + at) : 0.f;
+    const float w = at < p.C ? __ldg(p.w + at) : 0.f, u = at < p.C ? __ldg(p.u + at) : 0.f;
     // no infinity: what lies past the end of a sequence is zero and has to stay so
     const auto put = [&](int row, double x) { consts[row * kCs + ch] = static_cast<float>(x > 1e38 ? 1e38 : x); };
     const double wd = w;
@@ -161,8 +166,8 @@ __device__ __forceinline__ void strip_constants(float* consts, const Params& p, 
     double x = exp(own ? static_cast<double>(u) + wd : -wd);
     if (own) {
         put(kCuw, x);
-        const float grows = fmaxf(-w, 0.f), past = grows * static_cast<float>((p.T + St::L - 1) / St::L * St::L - p.T);
-        consts[kLimit * kCs + ch] = kSafeRange - (fabsf(u) + fabsf(w) + grows * static_cast<float>(p.T) + fmaxf(past - kSafePast, 0.f));
+        const float grows = fmaxf(-w, 0.f), whole = static_cast<float>((p.T + St::L - 1) / St::L * St::L);
+        consts[kLimit * kCs + ch] = kSafeRange - (fabsf(u) + fabsf(w) + fmaxf(grows * static_cast<float>(p.T), grows * whole - kSafePast));
         put(kLamL + St::kW + 1, 0.0);
         return;
     }
@@ -1150,8 +1155,8 @@ constexpr int kStrips = 4;
 // kMostHalf, 16 of the others.  Training pairs through autograd, us, separate launches with kept states / here: float32 B=16, T=4200,
 // C=768 546 / 382; 16 x 8192 1022 / 801; 8 x 16384 1053 / 952; bfloat16 k, v beside float32 y, gy 710 / 383, 1286 / 868, 1295 / 1033;
 // all bfloat16 551 / 408, 952 / 915, but 11 x 12000 971 / 1085 (rows of 16 bytes, and two passes over half the bytes are cheap).
-// Below kManyCtas this is faster as well (B=2, T=4200, C=384: forward 31 / 23, backward 65 / 34), but the launches and kept states of
-// the routes there are relied upon by callers that count them.
+// Below kManyCtas this is faster as well (B=2, T=4200, C=384: forward 31 / 23, backward 65 / 34): the line is not one of speed.  The routes
+// there keep the shapes at which their tests count launches and kept states.
 constexpr int kAnyTokens = 4096, kMostTokens = kMaxCluster * kMaxWarps * Strip<4, 17>::kSpan, kMostHalf = kMaxCluster * kMaxWarps * Strip<8, 17>::kSpan;
 constexpr long long kManyCtas = 768;
 bool in_range(int B, int T, int C, Types types) {
@@ -1324,6 +1329,10 @@ static int launch(const Plan& pl, int B, int T, int C, const float* w, const flo
     p.n_strips = static_cast<int>(strips_of(C, pl)); p.c_padded = p.n_strips * kCs; p.units = B * p.n_strips;
     p.cluster = pl.cluster; p.n_warps = pl.n_warps; p.n_tok = pl.n_tok;
     p.w = paired(w, C, vectors, stream);
+    if (T == 1) {      // a single token is not decayed: whatever w is, the rows that fill up its walker must not grow with it
+        cudaMemsetAsync(vectors, 0, static_cast<size_t>(C) * sizeof(float), stream);
+        p.w = vectors;
+    }
     p.u = paired(u, C, vectors + C, stream);
     p.o0 = o0; p.o1 = o1;
     p.status = reinterpret_cast<unsigned*>(ws);
