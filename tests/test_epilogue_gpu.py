@@ -253,3 +253,17 @@ def test_layers_are_called_where_a_mode_or_a_tensor_subclass_would_see_it(cuda_d
             assert torch.equal(epilogue.layer_norm(norm, x), epilogue.layer_norm(norm, x)) and launch_count() == before + 2
         assert ((epilogue.layer_norm(norm, x) - normed).norm() / normed.norm()).item() <= 1e-6
         assert ((mix(x, (125, 160)).float() - watched.float()).norm() / watched.float().norm()).item() <= 1e-2
+
+
+def test_the_gate_rounds_every_bfloat16_sigmoid_as_its_float64_value(cuda_device):
+    """All 65536 bfloat16 r: the result is within half a unit of the last place of the float64 sigmoid, but for the approximation's 2^-20
+    (and absolutely below bfloat16's smallest normal number)."""
+    from vision_rwkv_b200 import _lib
+    r = torch.arange(65536, device=cuda_device, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    got = _lib.native().sigmoid_gate(r, torch.ones_like(r), False).double()
+    want = torch.sigmoid(r.double())
+    assert torch.equal(got.isnan(), r.isnan())
+    ok = ~r.isnan()
+    unit = torch.exp2(torch.floor(torch.log2(want[ok].clamp_min(2.0 ** -126))) - 7)
+    # below e^-88.7 the exponential is infinite in float32 and the sigmoid zero
+    assert ((got[ok] - want[ok]).abs() <= 0.5 * unit + 2.0 ** -20 * want[ok] + 2.0 ** -127).all()
