@@ -340,6 +340,9 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
  *   vrwkv_linear_relu_square: out (rows, N) = relu(x W^T)^2 of x (rows, K) and W (N, K), the product rounded to bfloat16 first
  *     (CLS/vrwkv.py:250-251); K % 64 == 0, N % 256 == 0, else VRWKV_ERR_UNSUPPORTED; _pays: 1 where it takes less of the current
  *     device's time than a library's product and vrwkv_relu_square
+ *   vrwkv_linear_batch: out_i (rows, N) = x_i W_i^T rounded to bfloat16, i < count <= 4, in one launch (the layers behind a token shift,
+ *     CLS/vrwkv.py:166-168, vrwkv6.py:194-197); K % 64 == 0, K <= 384, N % 192 == 0, else VRWKV_ERR_UNSUPPORTED; _pays: 1 where it takes
+ *     less of the current device's time than a library's products
  *   vrwkv_norm_residual: out = x + gamma * (normalise(a) * weight + bias) over rows of C <= 1024 channels, C % 4 == 0;
  *     weight and bias NULL: out = x + gamma * a; gamma NULL: 1 (CLS/vrwkv.py:297-318)
  *   vrwkv_layer_norm: out = normalise(x) * weight + bias over such rows
@@ -357,6 +360,8 @@ int vrwkv_relu_square(long long n, const void* x, int is_bf16, void* out, void* 
 int vrwkv_relu_square_f32out(long long n, const uint16_t* x, float* out, void* stream);
 int vrwkv_linear_relu_square_pays(long long rows, int K, int N);
 int vrwkv_linear_relu_square(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream);
+int vrwkv_linear_batch_pays(int count, long long rows, int K, int N);
+int vrwkv_linear_batch(int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream);
 int vrwkv_add_rows(long long n, long long period, const float* table, const uint16_t* a, float* out, void* stream);
 int vrwkv_widen(long long n, const uint16_t* a, float* out, void* stream);
 int vrwkv_patch_rows(int B, int channels, int H, int W, int patch, const float* img, uint16_t* out, void* stream);

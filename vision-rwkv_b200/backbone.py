@@ -56,8 +56,7 @@ class SpatialMix(nn.Module):
                                        resolution, self.shift_pixel, self.channel_gamma)
         else:
             xk = xv = xr = x
-        k, v = self.key(xk), self.value(xv)
-        r = self.receptance(xr)
+        k, v, r = epilogue.linears((self.key, self.value, self.receptance), (xk, xv, xr))
         # the plain gate rounds y to the dtype of r; a norm in between takes it as it is
         run = inference_biwkv if self.key_norm is None and r.dtype == torch.bfloat16 else RUN_CUDA
         y = run(self.spatial_decay / T, self.spatial_first / T, k, v)

@@ -92,10 +92,7 @@ class SpatialMixV6(nn.Module):
         else:
             xw, xk, xv, xr, xg = (x + xx * (maa + m) for maa, m in (
                 (self.time_maa_w, mw), (self.time_maa_k, mk), (self.time_maa_v, mv), (self.time_maa_r, mr), (self.time_maa_g, mg)))
-        r = self.receptance(xr)
-        k = self.key(xk)
-        v = self.value(xv)
-        g_raw = self.gate(xg)
+        r, k, v, g_raw = epilogue.linears((self.receptance, self.key, self.value, self.gate), (xr, xk, xv, xg))
         w = epilogue.add_rows(self.time_decay, torch.tanh(xw @ self.time_decay_w1) @ self.time_decay_w2)
         y = inference_rwkv6(B, T, C, self.n_head, r.contiguous(), k.contiguous(), v.contiguous(),
                             w.float().contiguous(), self.time_faaaa)

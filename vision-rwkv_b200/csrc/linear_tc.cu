@@ -22,16 +22,16 @@
 #include <atomic>
 #include <mutex>
 #include "../../include/vrwkv_b200.h"
+#include "linear_tc.cuh"
 #include "sm100_async.cuh"
 #include "tensor_map.h"
 #include "vrwkv_internal.h"
 
 namespace lineartc {
 
-constexpr int kM = 128, kN = 256, kK = 64, kStages = 4;
+constexpr int kN = 256, kK = 64, kStages = 4;
 constexpr uint32_t kABytes = kM * kK * 2, kStageBytes = kABytes + kN * kK * 2, kBoxBytes = kM * 64 * 2;
 constexpr int kThreads = 192;
-constexpr uint32_t kWaitLimit = 1u << 20;
 
 struct Bars {
     uint64_t full[kStages], empty[kStages], done[2], taken[2], drained;
@@ -39,49 +39,6 @@ struct Bars {
     volatile uint32_t dead;
 };
 constexpr size_t kSmem = 1024 + kStages * kStageBytes + 2 * kBoxBytes + sizeof(Bars);
-
-using sm100::smem_u32;
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src),
-                 "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
-// K-major operand in 128-byte rows, swizzled; eight rows are 1024 bytes
-__device__ __forceinline__ uint64_t operand(uint32_t addr) {
-    return static_cast<uint64_t>((addr >> 4) & 0x3FFF) | static_cast<uint64_t>(1) << 16 | static_cast<uint64_t>(1024 >> 4) << 32 | static_cast<uint64_t>(1) << 46 |
-           static_cast<uint64_t>(2) << 61;
-}
-constexpr uint32_t kInstr = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kN >> 3) << 17) | (static_cast<uint32_t>(kM >> 4) << 24);
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b),
-                 "r"(kInstr), "r"(accumulate)
-                 : "memory");
-}
-__device__ __forceinline__ void commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void load16(uint32_t at, uint32_t* x) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]), "=r"(x[9]), "=r"(x[10]),
-                   "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
-                 : "r"(at)
-                 : "memory");
-}
-// relu(x)^2 of two sums, rounded to bfloat16 before (what the linear layer returns) and after
-__device__ __forceinline__ uint32_t relu_square2(uint32_t a, uint32_t b) {
-    const float2 x = __bfloat1622float2(__floats2bfloat162_rn(__uint_as_float(a), __uint_as_float(b)));
-    // x < 0 ? 0 : x keeps NaN
-    const float p = x.x < 0.f ? 0.f : x.x, q = x.y < 0.f ? 0.f : x.y;
-    const __nv_bfloat162 r = __floats2bfloat162_rn(p * p, q * q);
-    return *reinterpret_cast<const uint32_t*>(&r);
-}
 
 // kTest: one role of a CTA withholds what it owes for the first tile, and waits give up early.  A variant of its own: as arguments the two
 // cost 1.5 to 2.8 %.
@@ -162,7 +119,7 @@ linear_relu_square_kernel(const __grid_constant__ CUtensorMap mx, const __grid_c
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t a = operand(stages + st * kStageBytes), b = operand(stages + st * kStageBytes + kABytes);
 #pragma unroll
-                for (int k = 0; k < kK / 16; ++k) mma(d, a + 2 * k, b + 2 * k, (kb | k) != 0 ? 1u : 0u);      // 16 columns are 32 bytes
+                for (int k = 0; k < kK / 16; ++k) mma<kN>(d, a + 2 * k, b + 2 * k, (kb | k) != 0 ? 1u : 0u);      // 16 columns are 32 bytes
                 commit(s.empty + st);
             }
             if (good && !(kTest && silent == 1 && turn == 0)) commit(s.done + buf);
@@ -230,6 +187,7 @@ linear_relu_square_kernel(const __grid_constant__ CUtensorMap mx, const __grid_c
 
 static std::atomic<bool> g_withhold{false};
 void set_withhold_test(bool on) { g_withhold.store(on); }
+bool withhold_test() { return g_withhold.load(); }
 
 static bool allowed(int* sms) {
     static std::mutex lock;
@@ -276,13 +234,14 @@ extern "C" int vrwkv_linear_relu_square(long long rows, int K, int N, const uint
     const long long m_tiles = (rows + kM - 1) / kM, tiles = m_tiles * (N / kN);
     int sms = 0;
     if (K % kK != 0 || N % kN != 0 || rows > (1LL << 30) || tiles > (1LL << 30) || !allowed(&sms)) return VRWKV_ERR_UNSUPPORTED;
+    if (slab_serves(rows, K, N)) return square_by_slabs(rows, K, N, x, w, out, stream);
     tensor_map::bind_primary_context();
     CUtensorMap mx, mw, mo;
     if (!tensor_map::make_rows(&mx, x, rows, K, kK, kM) || !tensor_map::make_rows(&mw, w, N, K, kK, kN) || !tensor_map::make_rows(&mo, out, rows, N, 64, kM)) {
         set_error_detail("cuTensorMapEncodeTiled rejected a matrix");
         return VRWKV_ERR_DEVICE;
     }
-    const auto kernel = g_withhold.load() ? linear_relu_square_kernel<true> : linear_relu_square_kernel<false>;
+    const auto kernel = withhold_test() ? linear_relu_square_kernel<true> : linear_relu_square_kernel<false>;
     kernel<<<static_cast<unsigned>(std::min<long long>(tiles, sms)), kThreads, kSmem, static_cast<cudaStream_t>(stream)>>>(
         mx, mw, mo, static_cast<int>(m_tiles), N / kN, K / kK, failure_mirror(Op::linear));
     return record_launches(1);

@@ -61,6 +61,35 @@ Tensor linear_relu_square(const Tensor& x_, const Tensor& weight_) {
     return out;
 }
 
+std::vector<Tensor> linear_batch(std::vector<Tensor> xs, std::vector<Tensor> weights) {
+    TORCH_CHECK(!xs.empty() && xs.size() <= 4 && xs.size() == weights.size(), "one to four layers");
+    const c10::cuda::CUDAGuard guard(xs[0].device());
+    const int64_t depth = xs[0].dim() >= 1 ? xs[0].size(-1) : 0, rows = depth ? xs[0].numel() / depth : 0;
+    std::vector<Tensor> outs;
+    if (weights[0].dim() != 2 || !vrwkv_linear_batch_pays(xs.size(), rows, depth, weights[0].size(0))) {
+        for (size_t i = 0; i < xs.size(); ++i) outs.push_back(at::linear(xs[i], weights[i]));
+        return outs;
+    }
+    const uint16_t *x[4], *w[4];
+    uint16_t* out[4];
+    const auto p = [](const Tensor& t) { return static_cast<uint16_t*>(t.data_ptr()); };
+    for (size_t i = 0; i < xs.size(); ++i) {
+        same_place(xs[i], xs[0], "x");
+        same_place(weights[i], xs[0], "weight");
+        TORCH_CHECK(is_bf16(xs[i]) && xs[i].sizes() == xs[0].sizes() && weights[i].sizes() == weights[0].sizes() && weights[0].size(1) == depth,
+                    "the layers must be of one shape, on bfloat16 rows of their weights' width");
+        xs[i] = flat(xs[i]);
+        weights[i] = flat(at::autocast::cached_cast(at::kBFloat16, weights[i], at::kCUDA));      // autocast's own cast, and its cache
+        auto sizes = xs[i].sizes().vec();
+        sizes.back() = weights[i].size(0);
+        outs.push_back(at::empty(sizes, xs[i].options()));
+        x[i] = p(xs[i]); w[i] = p(weights[i]); out[i] = p(outs[i]);
+    }
+    check(vrwkv_linear_batch(xs.size(), rows, depth, weights[0].size(0), x, w, out, stream_of(xs[0])), "vrwkv_linear_batch");
+    raise_failures(xs[0].get_device(), "vrwkv_linear_batch");
+    return outs;
+}
+
 constexpr int64_t kOneByOne = 128 * 128 * 256;      // elements of a result: 128 tiles, less than one to an SM
 
 Tensor key_layer(const Tensor& x, const Tensor& weight) {

@@ -19,6 +19,8 @@ Tensor relu_square(const Tensor& x, bool wide);      // wide: bfloat16 x to a fl
 Tensor linear_relu_square(const Tensor& x, const Tensor& weight);
 // the same, by one kernel or by torch's product and the pass behind it, whichever takes less time
 Tensor key_layer(const Tensor& x, const Tensor& weight);
+// up to four linear layers of one shape without a bias on bfloat16 rows, as autocast computes them, in one launch where that is faster
+std::vector<Tensor> linear_batch(std::vector<Tensor> xs, std::vector<Tensor> weights);
 Tensor add_rows(const Tensor& table, const Tensor& a);
 Tensor patch_rows(const Tensor& img, int64_t patch);
 Tensor widen(const Tensor& a);

@@ -15,6 +15,7 @@ unsigned* failure_mirror(Op op);
 
 namespace lineartc {
 void set_withhold_test(bool on);   // test only: one role of every CTA withholds an arrival, waits give up early
+bool withhold_test();
 }
 
 #ifdef __CUDACC__
