@@ -54,11 +54,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
         "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
-// the same box into L2 only
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int x, int y, int z) {
-    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z)
-                 : "memory");
-}
 // 3-D tiled TMA store from shared memory (rows/columns outside the tensor are clipped).
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* src, int x, int y,
                                              int z) {

@@ -44,7 +44,6 @@ namespace wkv6c {
 
 constexpr float kSafe = 64.f;       // largest |sum of l| over a block for which its own pairs may use factors above 1
 
-typedef float Totals[kBlocks][N];   // sum of l over each block
 typedef float Table[kChunk][kTab];
 
 // ---- kernel 1: states entering every chunk ----------------------------------------------------------------
@@ -57,173 +56,206 @@ struct StateArgs {
 };
 constexpr uint32_t kWaitLimit = 1u << 20;      // polls before a wait for a tile gives up
 
-// Shared memory of a CTA: the raw tiles of one chunk as the copy engine delivers them (w | x, z of every pair), then per
-// pair the operand planes, then twice the totals (the next chunk's are written while this one's are read).  Both pairs
-// read the first one's totals: with a copy each, the backward on bfloat16 tensors and float32 gy was 1 KB above half of an
-// SM's shared memory.  Forward + backward at B=32, H=12
-// with one CTA of it per SM, and with two: T=196 303 and 286 us, T=4096 4.73 and 4.68 ms (280 us and 4.49 ms now, log2_decay).
-template <typename XT, typename ZT0, typename ZT1, int kZ, int kX, int kPairs>
+// Shared memory of a CTA, twice (the next chunk's tiles arrive during the whole of a step): the tiles of one chunk as the copy engine delivers
+// them (w | x, z of every pair).  The operands take their place: a warp reads its tokens' rows and writes the same rows, 16-byte pieces
+// exchanged by the row's number so that ldmatrix meets no bank twice; x's second part lies behind the first in a float row, else in
+// the row of w, which its warp has read by then.
+//
+// What bounds the walk: HBM, since the two directions meet the inputs at different times and each reads them (forward 2 x 8 and backward 2 x 14 bytes an
+// element, states 4 and 16).  B=32, H=12, T=4096, forward / backward us: 308 / 735 (2.0 and 4.4 GB: 6.5 and 6.0 TB/s), T=196 17.3 / 39.3.  Operand planes
+// beside one set of tiles, fetched while the products ran, and each pair's factors computed by its own warps: 450 / 902, 19.6 / 43.2; the
+// present form with one set of tiles, three CTAs instead of two on an SM: 479 / 1000; with sixteen warps of four tokens: 329 / 991 (one CTA on an SM).
+template <typename XT, typename ZT0, typename ZT1, int kX, int kPairs>
 struct StateSmem {
-    static constexpr size_t kTile = kChunk * N;
-    static constexpr size_t w = 0;
-    static constexpr size_t x0 = kTile * 4, z0 = x0 + kTile * sizeof(XT);
-    static constexpr size_t x1 = z0 + kTile * sizeof(ZT0), z1 = x1 + (kPairs > 1 ? kTile * sizeof(XT) : 0);
-    static constexpr size_t planes = z1 + (kPairs > 1 ? kTile * sizeof(ZT1) : 0);
-    static constexpr size_t per_pair = static_cast<size_t>(kZ + kX) * kPlane * 2;
-    static constexpr size_t totals = planes + kPairs * per_pair;
-    static constexpr size_t bar = totals + 2 * sizeof(Totals);
+    static constexpr uint32_t kWPitch = N * 4, kXPitch = N * sizeof(XT), kZ0Pitch = N * sizeof(ZT0), kZ1Pitch = N * sizeof(ZT1);
+    static constexpr uint32_t w = 0, x0 = kChunk * kWPitch, z0 = x0 + kChunk * kXPitch;
+    static constexpr uint32_t x1 = z0 + kChunk * kZ0Pitch, z1 = x1 + (kPairs > 1 ? kChunk * kXPitch : 0);
+    static constexpr uint32_t loaded = z1 + (kPairs > 1 ? kChunk * kZ1Pitch : 0);
+    // sums of l over each warp's tokens, and the state's decay across the chunk: 32 floats to a row.  A float z of the second pair leaves the
+    // second half of its rows free when its warp has read them (1.3 KB too much for two CTAs on an SM otherwise).
+    static constexpr bool kInside = kPairs > 1 && sizeof(ZT1) == 4 && sizeof(XT) == 2;
+    static constexpr uint32_t sums = kInside ? z1 + 128 : 2 * loaded, kSumPitch = kInside ? kZ1Pitch : 128;
+    static constexpr uint32_t bar = 2 * loaded + (kInside ? 0 : (4 * kPairs + 1) * N * 4);
     static constexpr size_t bytes = bar + 16;
-    static constexpr uint32_t loaded = static_cast<uint32_t>(planes);
 };
-
-// The work of one pair's four warps (a block each) on one chunk: lane = two channels, one token after the other, so decays,
-// their running sums and the scaling need no shuffles.  Leaves the scaled operand planes; `tot` gets the blocks' sums
-// (from the pair that `writes`).
-template <typename XT, typename ZT, int kZ, int kX>
-__device__ __forceinline__ void scale_chunk(const float* wt, const XT* xt, const ZT* zt, int valid, int dir, Totals& tot, bool writes,
-                                            __nv_bfloat16* xs, __nv_bfloat16* zs, int warp, int lane) {
-    const int word = col_word(lane), row0 = warp * kBlock;
-    float2 sum[kBlock];
-    float2 run = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int t = 0; t < kBlock; ++t) {
-        const float2 w = *reinterpret_cast<const float2*>(wt + (row0 + t) * N + 2 * lane);
-        run.x += log2_decay(w.x, row0 + t < valid);
-        run.y += log2_decay(w.y, row0 + t < valid);
-        sum[t] = run;
-    }
-    if (writes) *reinterpret_cast<float2*>(&tot[warp][2 * lane]) = run;
-    __syncthreads();       // totals are there; every warp is past the previous chunk's products
-    float2 edge = make_float2(0.f, 0.f);        // decay from the block to the chunk's edge
-    for (int j = dir == 0 ? warp + 1 : 0; j < (dir == 0 ? kBlocks : warp); ++j) {
-        const float2 t = *reinterpret_cast<const float2*>(&tot[j][2 * lane]);
-        edge.x += t.x;
-        edge.y += t.y;
-    }
-    if (dir == 0) { edge.x += run.x; edge.y += run.y; }
-#pragma unroll
-    for (int t = 0; t < kBlock; ++t) {
-        Pair<XT> xr;
-        Pair<ZT> zr;
-        xr.lds(xt + (row0 + t) * N + 2 * lane);
-        zr.lds(zt + (row0 + t) * N + 2 * lane);
-        const float2 xv = round2<sizeof(XT) == 4>(xr.get()), zv = round2<sizeof(ZT) == 4>(zr.get());
-        const float2 prev = t > 0 ? sum[t > 0 ? t - 1 : 0] : make_float2(0.f, 0.f);
-        const float ex = dir == 0 ? edge.x - sum[t].x : edge.x + prev.x, ey = dir == 0 ? edge.y - sum[t].y : edge.y + prev.y;
-        col_store<kX>(xs, row0 + t, word, xv.x * ex2(ex), xv.y * ex2(ey));
-        if (kZ == 1 && sizeof(ZT) == 2) *reinterpret_cast<uint32_t*>(zs + (row0 + t) * kRow + 2 * word) = zr.bits();
-        else col_store<kZ>(zs, row0 + t, word, zv.x, zv.y);
-    }
+struct Rows { uint32_t at, pitch; };      // an operand: 64 rows (tokens) of 128 bytes
+// 32-bit word `word` of a row
+__device__ __forceinline__ uint32_t word_at(Rows p, int row, int word) { return p.at + row * p.pitch + (((word >> 2) ^ (row & 7)) << 4) + ((word & 3) << 2); }
+__device__ __forceinline__ uint32_t chunk_at(Rows p, int row, int chunk) { return p.at + row * p.pitch + ((chunk ^ (row & 7)) << 4); }
+__device__ __forceinline__ void put_word(uint32_t at, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+// a token's channel pair as one bfloat16 pair
+__device__ __forceinline__ uint32_t half_pair(const __nv_bfloat16* row, int lane) { return *reinterpret_cast<const uint32_t*>(row + 2 * lane); }
+__device__ __forceinline__ uint32_t half_pair(const float* row, int lane) {
+    const float2 v = *reinterpret_cast<const float2*>(row + 2 * lane);
+    uint32_t t[1];
+    split<1>(v.x, v.y, t);
+    return t[0];
 }
 
 // grid (b h, direction); direction 0 walks rightward (decay to the chunk's right edge), 1 leftward; four warps per pair of
-// inputs (the backward's two share the decays' tile).  kZ parts of z, kX parts of the scaled x; kRows: the state's rows are
-// the channels of x (else its columns).  A chunk's tiles are fetched while the previous chunk's products run, and the tiles
-// of the two chunks behind it into L2, so a step costs its arithmetic (about 2.4 k cycles) and not a trip to memory.
-template <typename XT, typename ZT0, typename ZT1, int kZ, int kX, bool kRows, int kPairs>
-__global__ void __launch_bounds__(128 * kPairs, kPairs == 1 ? 4 : 2)
+// inputs.  kX parts of the scaled x; kRows: the state's rows are the channels of x (else its columns).  A warp scales kTokens tokens of all
+// pairs, which share the factors: lane = two channels, one token after the other, so decays, their running sums and the scaling need no
+// shuffles.
+template <typename XT, typename ZT0, typename ZT1, int kX, bool kRows, int kPairs>
+__global__ void __launch_bounds__(128 * kPairs, kPairs == 1 ? 3 : 2)
 wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mx0,
                   const __grid_constant__ CUtensorMap mz0, const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mz1) {
-    typedef StateSmem<XT, ZT0, ZT1, kZ, kX, kPairs> S;
+    typedef StateSmem<XT, ZT0, ZT1, kX, kPairs> S;
+    constexpr int kWarps = 4 * kPairs, kTokens = kChunk / kWarps, kZ = 1;
     extern __shared__ __align__(1024) unsigned char smem[];
-    const int bh = blockIdx.x, dir = blockIdx.y, pair = kPairs > 1 ? threadIdx.x >> 7 : 0;
+    const int bh = blockIdx.x, dir = blockIdx.y, w8 = threadIdx.x >> 5, pair = w8 >> 2, warp = w8 & 3;
     const int b = bh / a.H, h = bh - b * a.H;
-    const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int lane = threadIdx.x & 31, g = lane >> 2;
     constexpr int kState = kX * kStateWords / 4;
     uint4* out = a.out + (static_cast<size_t>(pair) * 2 + dir) * a.plane + static_cast<size_t>(bh) * a.n_chunks * kState;
-    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem + S::planes + pair * S::per_pair);
-    __nv_bfloat16* zs = xs + kX * kPlane;
-    Totals* tots = reinterpret_cast<Totals*>(smem + S::totals);
+    // where channel `ch` of warp j's sum is, and (behind another's, or in its writer's third and fourth row) of the state's decay
+    unsigned char* raw = smem;
+    const auto total_at = [&](int j, int ch) {
+        return reinterpret_cast<float*>((S::kInside ? raw : smem) + S::sums + ((S::kInside ? j * kTokens : 2 * j) + (ch >> 5)) * S::kSumPitch + (ch & 31) * 4);
+    };
+    const auto decay_at = [&](int ch) {
+        return reinterpret_cast<float*>((S::kInside ? raw : smem) + S::sums + ((S::kInside ? (dir == 0 ? 2 : kChunk - kTokens + 2) : 2 * kWarps) + (ch >> 5)) * S::kSumPitch + (ch & 31) * 4);
+    };
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::bar);
+    const uint32_t base_at = smem_addr(smem);
+    uint32_t at = base_at;
+    const auto part_of = [&](int p, int part) {      // x's parts
+        const uint32_t x = at + (p == 0 ? S::x0 : S::x1);
+        if (part == 0) return Rows{x, S::kXPitch};
+        return sizeof(XT) == 4 ? Rows{x + 128, S::kXPitch} : Rows{at + S::w + p * 128, S::kWPitch};
+    };
     const auto chunk_of = [&](int step) { return dir == 0 ? step : a.n_chunks - 1 - step; };
     const auto fetch = [&](int step) {
         const int t0 = chunk_of(step) * kChunk;
-        sm100::mbar_expect_tx(bar, S::loaded);
-        sm100::tma_load_3d(smem + S::w, &mw, bar, h * N, t0, b);
-        sm100::tma_load_3d(smem + S::x0, &mx0, bar, h * N, t0, b);
-        sm100::tma_load_3d(smem + S::z0, &mz0, bar, h * N, t0, b);
+        unsigned char* const to = smem + (step & 1) * S::loaded;
+        uint64_t* const full = bar + (step & 1);
+        sm100::mbar_expect_tx(full, S::loaded);
+        sm100::tma_load_3d(to + S::w, &mw, full, h * N, t0, b);
+        sm100::tma_load_3d(to + S::x0, &mx0, full, h * N, t0, b);
+        sm100::tma_load_3d(to + S::z0, &mz0, full, h * N, t0, b);
         if (kPairs > 1) {
-            sm100::tma_load_3d(smem + S::x1, &mx1, bar, h * N, t0, b);
-            sm100::tma_load_3d(smem + S::z1, &mz1, bar, h * N, t0, b);
-        }
-    };
-    const auto fetch_l2 = [&](int step) {
-        const int t0 = chunk_of(step) * kChunk;
-        sm100::tma_prefetch_3d(&mw, h * N, t0, b);
-        sm100::tma_prefetch_3d(&mx0, h * N, t0, b);
-        sm100::tma_prefetch_3d(&mz0, h * N, t0, b);
-        if (kPairs > 1) {
-            sm100::tma_prefetch_3d(&mx1, h * N, t0, b);
-            sm100::tma_prefetch_3d(&mz1, h * N, t0, b);
+            sm100::tma_load_3d(to + S::x1, &mx1, full, h * N, t0, b);
+            sm100::tma_load_3d(to + S::z1, &mz1, full, h * N, t0, b);
         }
     };
     const int last = a.n_chunks - 1;        // steps that update the state
     if (threadIdx.x == 0) {
         sm100::mbar_init(bar, 1);
+        sm100::mbar_init(bar + 1, 1);
         sm100::mbar_init_fence();
         fetch(0);
-        for (int s = 1; s < 3 && s < last; ++s) fetch_l2(s);
+        if (last > 1) fetch(1);
     }
     __syncthreads();
+    const int row0 = w8 * kTokens, word = col_word(lane);
     Acc c;
     zero(c);
     for (int step = 0; step < last; ++step) {
-        const int n = chunk_of(step);
-        const int valid = a.T - n * kChunk;
-        Totals& tot = tots[step & 1];
-        if (!sm100::mbar_wait(bar, step & 1, kWaitLimit)) report_failure(a.status, a.mirror, 2u);
-        const float* wt = reinterpret_cast<const float*>(smem + S::w);
-        if (kPairs == 1 || pair == 0)
-            scale_chunk<XT, ZT0, kZ, kX>(wt, reinterpret_cast<const XT*>(smem + S::x0), reinterpret_cast<const ZT0*>(smem + S::z0), valid, dir, tot,
-                                         true, xs, zs, warp, lane);
-        else
-            scale_chunk<XT, ZT1, kZ, kX>(wt, reinterpret_cast<const XT*>(smem + S::x1), reinterpret_cast<const ZT1*>(smem + S::z1), valid, dir, tot,
-                                         false, xs, zs, warp, lane);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (step + 1 < last) fetch(step + 1);
-            if (step + 3 < last) fetch_l2(step + 3);
+        const int valid = a.T - chunk_of(step) * kChunk;
+        if (!sm100::mbar_wait(bar + (step & 1), step >> 1 & 1, kWaitLimit)) report_failure(a.status, a.mirror, 2u);
+        at = base_at + (step & 1) * S::loaded;
+        raw = smem + (step & 1) * S::loaded;
+        float2 sum[kTokens];
+        float2 run = make_float2(0.f, 0.f);
+        {
+            const float* wt = reinterpret_cast<const float*>(raw + S::w) + row0 * N + 2 * lane;
+#pragma unroll
+            for (int t = 0; t < kTokens; ++t) {
+                const float2 w = *reinterpret_cast<const float2*>(wt + t * N);
+                run.x += log2_decay(w.x, row0 + t < valid);
+                run.y += log2_decay(w.y, row0 + t < valid);
+                sum[t] = run;
+            }
         }
+        uint32_t zi[kTokens];
+        if (S::kInside) {
+#pragma unroll
+            for (int t = 0; t < kTokens; ++t) zi[t] = half_pair(reinterpret_cast<const ZT1*>(raw + S::z1) + (row0 + t) * N, lane);
+            __syncwarp();
+        }
+        *reinterpret_cast<float2*>(total_at(w8, 2 * lane)) = run;
+        __syncthreads();
+        // a token's factor: the decay from it to the chunk's edge.  Small sums first: the way to the end of the warp's tokens, then
+        // the rest of the chunk
+        float2 edge;
+        {
+            float2 t[kWarps];
+#pragma unroll
+            for (int j = 0; j < kWarps; ++j) {
+                t[j] = *reinterpret_cast<const float2*>(total_at(j, 2 * lane));
+                if (dir == 0 ? j <= w8 : j >= w8) t[j] = make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int d = 1; d < kWarps; d *= 2)
+#pragma unroll
+                for (int j = 0; j < kWarps; j += 2 * d) { t[j].x += t[j + d].x; t[j].y += t[j + d].y; }
+            edge = t[0];
+        }
+        if (w8 == (dir == 0 ? 0 : kWarps - 1)) *reinterpret_cast<float2*>(decay_at(2 * lane)) = make_float2(ex2(edge.x + run.x), ex2(edge.y + run.y));
+        if (dir == 0) {
+#pragma unroll
+            for (int t = 0; t < kTokens; ++t) sum[t] = make_float2(ex2(edge.x + (run.x - sum[t].x)), ex2(edge.y + (run.y - sum[t].y)));
+        } else {
+#pragma unroll
+            for (int t = kTokens - 1; t >= 0; --t)
+                sum[t] = t > 0 ? make_float2(ex2(edge.x + sum[t - 1].x), ex2(edge.y + sum[t - 1].y)) : make_float2(ex2(edge.x), ex2(edge.y));
+        }
+#pragma unroll
+        for (int p = 0; p < kPairs; ++p) {
+            const XT* x = reinterpret_cast<const XT*>(raw + (p == 0 ? S::x0 : S::x1)) + row0 * N;
+            float2 xv[kTokens];
+            uint32_t zv[kTokens];
+#pragma unroll
+            for (int t = 0; t < kTokens; ++t) {
+                const uint32_t r = half_pair(x + t * N, lane);      // raw inputs are rounded to bfloat16 where they arrive as float
+                xv[t] = make_float2(lo_f(r) * sum[t].x, hi_f(r) * sum[t].y);
+                zv[t] = p == 0        ? half_pair(reinterpret_cast<const ZT0*>(raw + S::z0) + (row0 + t) * N, lane)
+                        : S::kInside ? zi[t]
+                                     : half_pair(reinterpret_cast<const ZT1*>(raw + S::z1) + (row0 + t) * N, lane);
+            }
+            __syncwarp();      // the rows have been read
+            const Rows z = p == 0 ? Rows{at + S::z0, S::kZ0Pitch} : Rows{at + S::z1, S::kZ1Pitch};
+#pragma unroll
+            for (int t = 0; t < kTokens; ++t) {
+                uint32_t parts[kX];
+                split<kX>(xv[t].x, xv[t].y, parts);
+#pragma unroll
+                for (int i = 0; i < kX; ++i) put_word(word_at(part_of(p, i), row0 + t, word), parts[i]);
+                put_word(word_at(z, row0 + t, word), zv[t]);
+            }
+        }
+        __syncthreads();
         // decay of the state across the chunk
         if (kRows) {
             const int ch = 16 * warp + 4 * (g >> 1) + (g & 1);
-            const float s0 = ex2((tot[0][ch] + tot[1][ch]) + (tot[2][ch] + tot[3][ch]));
-            const float s1 = ex2((tot[0][ch + 2] + tot[1][ch + 2]) + (tot[2][ch + 2] + tot[3][ch + 2]));
+            const float s0 = *decay_at(ch), s1 = *decay_at(ch + 2);
 #pragma unroll
             for (int i = 0; i < 8; ++i) { c[i][0] *= s0; c[i][1] *= s0; c[i][2] *= s1; c[i][3] *= s1; }
         } else {
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
-                float s[4] = {0.f, 0.f, 0.f, 0.f};
+                float s[4];
+                row4(decay_at(16 * kk + 4 * (lane & 3)), 0, 0, s);
 #pragma unroll
-                for (int j = 0; j < kBlocks; ++j) {
-                    float t[4];
-                    row4(tot[j], kk, q, t);
+                for (int half = 0; half < 2; ++half)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) s[e] += t[e];
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float d = ex2(s[e]);
-                    at(c, 0, kk, e) *= d;
-                    at(c, 1, kk, e) *= d;
-                }
+                    for (int e = 0; e < 4; ++e) c[2 * kk + (e >> 1)][half * 2 + (e & 1)] *= s[e];
             }
         }
-        const __nv_bfloat16* pm = kRows ? xs : zs;       // rows of the state
-        const __nv_bfloat16* pn = kRows ? zs : xs;       // columns
+        const Rows z = pair == 0 ? Rows{at + S::z0, S::kZ0Pitch} : Rows{at + S::z1, S::kZ1Pitch};
         constexpr int kM = kRows ? kX : kZ, kN = kRows ? kZ : kX;
 #pragma unroll
         for (int s = 0; s < kBlocks; ++s) {
             uint32_t am[kM][4];
+            const int rm = s * kBlock + ((lane >> 4) << 3) + (lane & 7), rn = s * kBlock + (((lane >> 3) & 1) << 3) + (lane & 7);
 #pragma unroll
-            for (int i = 0; i < kM; ++i) ldsm4t(am[i], smem_addr(pm + i * kPlane + s * kBlock * kRow + 16 * warp + off_tok(lane)));
+            for (int i = 0; i < kM; ++i) ldsm4t(am[i], chunk_at(kRows ? part_of(pair, i) : z, rm, 2 * warp + ((lane >> 3) & 1)));
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
                 for (int ib = 0; ib < kN; ++ib) {
                     uint32_t r[4];
-                    ldsm4t(r, smem_addr(pn + ib * kPlane + s * kBlock * kRow + 16 * kk + off_pos(lane)));
+                    ldsm4t(r, chunk_at(kRows ? z : part_of(pair, ib), rn, 2 * kk + (lane >> 4)));
 #pragma unroll
                     for (int ia = 0; ia < kM; ++ia)
                         if (Keep<kM, kN>::on(ia, ib)) {
@@ -232,6 +264,9 @@ wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, con
                         }
                 }
         }
+        sm100::fence_proxy_async_smem();      // the copy engine writes where the operands were
+        __syncthreads();
+        if (threadIdx.x == 0 && step + 2 < last) fetch(step + 2);
         uint4* o = out + static_cast<size_t>(chunk_of(step + 1)) * kState;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
@@ -1176,7 +1211,8 @@ template <typename T, typename G, int kZ, int kX, bool kRows>
 static bool run_states(int B, int T_, int H, const void* r, const void* k, const void* v, const float* w, const void* gy, uint4* states,
                        size_t plane, void* workspace, cudaStream_t stream) {
     constexpr int kPairs = kRows ? 2 : 1;
-    typedef StateSmem<T, T, G, kZ, kX, kPairs> S;
+    static_assert(kZ == 1, "z enters in one part");
+    typedef StateSmem<T, T, G, kX, kPairs> S;
     tensor_map::bind_primary_context();   // the tensor-map encoder is a driver call
     const int C = H * N;
     const auto map = [&](CUtensorMap* m, const void* p, bool half) { return tensor_map::make_btc(m, p, B, T_, C, N, kChunk, half); };
@@ -1190,7 +1226,7 @@ static bool run_states(int B, int T_, int H, const void* r, const void* k, const
     }
     const StateArgs a{T_, H, chunks_of(T_), states, plane, static_cast<unsigned*>(workspace),
                       failure_mirror(kRows ? Op::wkv6_backward : Op::wkv6_forward)};
-    const auto kernel = wkv6_state_kernel<T, T, G, kZ, kX, kRows, kPairs>;
+    const auto kernel = wkv6_state_kernel<T, T, G, kX, kRows, kPairs>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), S::bytes)) return false;
     kernel<<<dim3(B * H, 2), 128 * kPairs, S::bytes, stream>>>(a, mw, mk, mv, mr, mg);
     return true;

@@ -205,7 +205,12 @@ template <bool kRound>
 __device__ __forceinline__ void round4(float (&x)[4]) {
     if (kRound) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) x[e] = __bfloat162float(__float2bfloat16(x[e]));
+        for (int e = 0; e < 4; e += 2) {      // two at a time: a single conversion goes through the exponential's unit, an eighth of a pair's rate
+            uint32_t t[1];
+            split<1>(x[e], x[e + 1], t);
+            x[e] = lo_f(t[0]);
+            x[e + 1] = hi_f(t[0]);
+        }
     }
 }
 // store 4 contiguous channels (`scalar`: the tensor is not aligned for vector stores)
@@ -268,7 +273,10 @@ struct Pair<__nv_bfloat16> {
 // raw inputs of the half-precision kernels are rounded to bfloat16 where they arrive as float
 template <bool kRound>
 __device__ __forceinline__ float2 round2(float2 x) {
-    return kRound ? make_float2(__bfloat162float(__float2bfloat16(x.x)), __bfloat162float(__float2bfloat16(x.y))) : x;
+    if (!kRound) return x;
+    uint32_t t[1];
+    split<1>(x.x, x.y, t);
+    return make_float2(lo_f(t[0]), hi_f(t[0]));
 }
 // log2 of a token's decay, bounded at -128: 2^-128 is flushed to zero already, and so bounded a sum over a block keeps its
 // smaller terms to 1e-4 (and stays finite) whatever a token's decay is.  The bound is taken on w, which leaves the product and
