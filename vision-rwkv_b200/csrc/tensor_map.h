@@ -37,8 +37,8 @@ inline void bind_primary_context() {
 
 // Box of box_c channels x box_t tokens of one batch entry; out-of-range elements load as zero and
 // are clipped on store.  `base` must be 16-byte aligned and the row pitch C * elem_bytes a multiple
-// of 16 (C % 4 == 0 for float, C % 8 == 0 for bfloat16).
-inline bool make_btc(CUtensorMap* map, const void* base, int B, int T, int C, int box_c, int box_t, bool bf16) {
+// of 16 (C % 4 == 0 for float, C % 8 == 0 for bfloat16).  swizzled: over the 128 bytes of a box's row.
+inline bool make_btc(CUtensorMap* map, const void* base, int B, int T, int C, int box_c, int box_t, bool bf16, bool swizzled = false) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t eb = bf16 ? 2 : 4;
@@ -47,7 +47,7 @@ inline bool make_btc(CUtensorMap* map, const void* base, int B, int T, int C, in
     const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_c), static_cast<cuuint32_t>(box_t), 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base),
-              dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+              dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 // A bfloat16 matrix [rows][cols] in boxes of 64 columns x box_rows, 128-byte swizzle; cols a multiple of 8.

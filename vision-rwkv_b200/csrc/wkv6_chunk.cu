@@ -541,22 +541,87 @@ __device__ __forceinline__ void store_tile(__nv_bfloat16* planes, const float (&
         }
 }
 
+// ---- inputs kept in shared memory: 64 rows of 128 bytes (64 bfloat16), 16-byte pieces exchanged by the row's number as the copy engine's
+// 128-byte swizzle has them.  A row's four channels 4 q .. of 16 kk: rows g of a warp's eight meet each bank twice, the least for 256 bytes.
+__device__ __forceinline__ uint2 raw4(const unsigned char* tile, int row, int kk, int q) {
+    return *reinterpret_cast<const uint2*>(tile + row * 128 + (((2 * kk + (q >> 1)) ^ (row & 7)) << 4) + (q & 1) * 8);
+}
+__device__ __forceinline__ void load4(const unsigned char* tile, int row, int kk, int q, float (&x)[4]) {
+    const uint2 v = raw4(tile, row, kk, q);
+    x[0] = lo_f(v.x); x[1] = hi_f(v.x); x[2] = lo_f(v.y); x[3] = hi_f(v.y);
+}
+__device__ __forceinline__ uint32_t raw_word(int row, int lane) { return row * 128 + (((lane >> 2) ^ (row & 7)) << 4) + ((lane & 3) << 2); }
+__device__ __forceinline__ void load_block(Block& x, const unsigned char* tile, int blk, int g, int q) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) load4(tile, blk * kBlock + g + 8 * half, kk, q, x[half][kk]);
+}
+// a block's rows scaled to its right edge (for partners later than it: dir 0) or left edge (dir 1), into planes
+template <int NS>
+__device__ __forceinline__ void stage_scaled(__nv_bfloat16* planes, const unsigned char* tile, const Table& tab, int blk, int dir, int lane) {
+    const float2 total = *reinterpret_cast<const float2*>(&tab[blk * kBlock + kBlock - 1][2 * lane]);
+    float2 prev = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) {
+        const uint32_t v = *reinterpret_cast<const uint32_t*>(tile + raw_word(blk * kBlock + t, lane));
+        const float2 s = *reinterpret_cast<const float2*>(&tab[blk * kBlock + t][2 * lane]);
+        const float ex = dir == 0 ? total.x - s.x : prev.x, ey = dir == 0 ? total.y - s.y : prev.y;
+        col_store<NS>(planes, blk * kBlock + t, col_word(lane), lo_f(v) * ex2(ex), hi_f(v) * ex2(ey));
+        prev = s;
+    }
+}
+// a block of a tile as the copy engine left it (row after row), into a plane, rounded
+__device__ __forceinline__ void stage_tile(__nv_bfloat16* plane, const __nv_bfloat16* tile, int blk, int lane) {
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t)
+        *reinterpret_cast<uint32_t*>(plane + (blk * kBlock + t) * kRow + 2 * col_word(lane)) = half_pair(tile + (blk * kBlock + t) * N, lane);
+}
+__device__ __forceinline__ void stage_tile(__nv_bfloat16* plane, const float* tile, int blk, int lane) {
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t)
+        *reinterpret_cast<uint32_t*>(plane + (blk * kBlock + t) * kRow + 2 * col_word(lane)) = half_pair(tile + (blk * kBlock + t) * N, lane);
+}
+// a block's rows into such a tile, rounded
+template <typename T>
+__device__ __forceinline__ void keep_rows(unsigned char* tile, const T* p, int C, int rows, int blk, int lane) {
+    Pair<T> x[kBlock];
+    load_rows<T>(x, p, C, rows, lane);
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) {
+        uint32_t w[1];
+        const float2 v = x[t].get();
+        split<1>(v.x, v.y, w);
+        *reinterpret_cast<uint32_t*>(tile + raw_word(blk * kBlock + t, lane)) = w[0];
+    }
+}
+__device__ __forceinline__ void scan_tile(Table& tab, const float* tile, int rows, int blk, int lane) {
+    float2 run = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < kBlock; ++t) {
+        const float2 w = *reinterpret_cast<const float2*>(tile + (blk * kBlock + t) * N + 2 * lane);
+        run.x += log2_decay(w.x, t < rows);
+        run.y += log2_decay(w.y, t < rows);
+        *reinterpret_cast<float2*>(&tab[blk * kBlock + t][2 * lane]) = run;
+    }
+}
+
 // Row-mapped part of y (rows r, columns k) and gv (rows k, columns r): warp (blk, dir) forms its pairs of the token matrix
 // and leaves the rows scaled to the chunk's edge (for the entering state) in the planes `edges`.  The two directions of
 // a diagonal tile are merged by the masks: dir 0 writes below the diagonal and on it, dir 1 above.
-template <typename T, int kX, bool kRound>
-__device__ __forceinline__ void pair_rows(const T* row_in, const T* col_in, const float* u, const Table& tab, const __nv_bfloat16* planes,
-                                          __nv_bfloat16* pairs, __nv_bfloat16* edges, int C, int rows, int blk, int dir, int lane) {
+template <int kX, typename RowsOf, typename ColsOf>
+__device__ __forceinline__ void pair_rows(RowsOf&& rows_of, ColsOf&& cols_of, const float* u, const Table& tab, const __nv_bfloat16* planes,
+                                          __nv_bfloat16* pairs, __nv_bfloat16* edges, int blk, int dir, int lane) {
     const int g = lane >> 2, q = lane & 3;
     const bool safe = block_is_safe(tab, blk, lane);
     Block x;
-    load_block<T, kRound>(x, row_in, C, rows, g, q);
+    rows_of(x);
     AFrag<kX> f;
     {
         float p[2][4] = {}, diag[2] = {0.f, 0.f};
         if (dir == 0 || !safe) {
             Block c;
-            load_block<T, kRound>(c, col_in, C, rows, g, q);
+            cols_of(c);
             if (dir == 0) bonus_terms(x, c, u, q, diag);
             if (!safe) {
                 // copies: what a call takes by reference lives in memory, and x stays in registers
@@ -750,7 +815,8 @@ __global__ void __launch_bounds__(256, 3) wkv6_forward_kernel(const OutArgs a) {
         __syncthreads();
         stage_scaled<T, kX, kRound>(planes, kr, tab, blk, dir, lane);
         __syncthreads();
-        pair_rows<T, kX, kRound>(static_cast<const T*>(a.r) + at0, k, a.u + h * N, tab, planes, pairs, edges + dir * kX * kPlane, C, rows, blk, dir, lane);
+        pair_rows<kX>([&](Block& x) { load_block<T, kRound>(x, static_cast<const T*>(a.r) + at0, C, rows, g, q); },
+                      [&](Block& x) { load_block<T, kRound>(x, k, C, rows, g, q); }, a.u + h * N, tab, planes, pairs, edges + dir * kX * kPlane, blk, dir, lane);
     }
     __syncthreads();
     const int cs = warp & 3, th = warp >> 2;
@@ -786,7 +852,10 @@ struct GradArgs {
     bool scalar;              // an output is not 16-byte aligned: element stores
     const uint4* states;      // [pair][direction][b h][chunk][part][..], rows = channels of r, k
     size_t plane;
+    unsigned* status;         // as in StateArgs
+    unsigned* mirror;
 };
+constexpr uint32_t kRawTile = kChunk * N * 2;
 
 // gr (own = gy, partners k, m = gy v^T) or gk (own = v, partners r, m transposed) for 32 tokens x 16 channels:
 //   early / late[m tile][row half][e] = sum over earlier / later tokens s of (own_t . other_s) D(t, s) (x) partner_s,
@@ -897,9 +966,12 @@ __device__ __forceinline__ void slice_gradient(float (&out)[2][2][2][4], const _
 
 // kZ parts of v, gy; kX parts of scaled operands, token products and states; kP parts where only gv is concerned
 template <typename T, typename G, typename O, int kZ, int kX, int kP>
-__global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a) {
+__global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mr,
+                     const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mg) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __nv_bfloat16* vs = reinterpret_cast<__nv_bfloat16*>(smem);
+    unsigned char* const k_raw = smem;               // k and r stay, as bfloat16
+    unsigned char* const r_raw = smem + kRawTile;
+    __nv_bfloat16* vs = reinterpret_cast<__nv_bfloat16*>(smem + 2 * kRawTile);
     __nv_bfloat16* gs = vs + kZ * kPlane;
     __nv_bfloat16* pf = gs + kZ * kPlane;        // k, then r, towards the right edge of its block, left edge behind it
     __nv_bfloat16* ms = pf + 2 * kX * kPlane;    // gy v^T inside the chunk, later the pairs of gv
@@ -908,6 +980,10 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
     float* edge = dots + N;                                 // [2][N]
     float* gus = edge + 2 * N;                              // [2][N]
     float* seg = gus + 2 * N;                               // [8][N]
+    uint64_t* bar = reinterpret_cast<uint64_t*>(seg + 8 * N);
+    // tiles on their way into planes and table: w where m will be, v and gy where the scaled rows will be
+    unsigned char *const w_raw = reinterpret_cast<unsigned char*>(ms), *const v_raw = reinterpret_cast<unsigned char*>(pf), *const g_raw = v_raw + kRawTile;
+    static_assert(kX == 2, "room for the tiles");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     const int blk = warp & 3, dir = warp >> 2;              // row-mapped phases
     const int cs = warp & 3, th = warp >> 2;                // slice-mapped phases
@@ -926,6 +1002,19 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
     const T* rp = static_cast<const T*>(a.r);
     const T* kp = static_cast<const T*>(a.k);
 
+    if (sizeof(T) == 2) {
+        if (threadIdx.x == 0) {
+            sm100::mbar_init(bar, 1);
+            sm100::mbar_init_fence();
+            sm100::mbar_expect_tx(bar, 3 * kRawTile + kChunk * N * (4 + sizeof(G)));
+            sm100::tma_load_3d(w_raw, &mw, bar, h * N, n * kChunk, b);
+            sm100::tma_load_3d(g_raw, &mg, bar, h * N, n * kChunk, b);
+            sm100::tma_load_3d(v_raw, &mv, bar, h * N, n * kChunk, b);
+            sm100::tma_load_3d(k_raw, &mk, bar, h * N, n * kChunk, b);
+            sm100::tma_load_3d(r_raw, &mr, bar, h * N, n * kChunk, b);
+        }
+        __syncthreads();
+    }
     if (blockIdx.x + a.ahead < gridDim.x) {
         const int id = blockIdx.x + a.ahead, n2 = id % a.n_chunks, bh2 = id / a.n_chunks, b2 = bh2 / a.H, rows2 = a.T - n2 * kChunk;
         const size_t at = (static_cast<size_t>(b2) * a.T + n2 * kChunk) * C + static_cast<size_t>(bh2 - b2 * a.H) * N;
@@ -938,16 +1027,25 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
         for (int i = 0; i < 4; ++i)      // from the left, from the right, of either pair
             if ((i & 1) ? n2 + 1 < a.n_chunks : n2 > 0) prefetch_bytes(st2 + i * a.plane, kState * 16);
     }
-    Pair<T> col[kBlock];
-    load_rows<T>(col, kp + at0, C, rows, lane);
-    if (dir == 0) {
-        scan_block(tab, a.w + at0, C, rows, blk, lane);
+    if (sizeof(T) == 2) {
+        if (!sm100::mbar_wait(bar, 0, kWaitLimit)) report_failure(a.status, a.mirror, 2u);
+        if (dir == 0) {
+            scan_tile(tab, reinterpret_cast<const float*>(w_raw), rows, blk, lane);
+        } else {
+            stage_tile(vs, reinterpret_cast<const __nv_bfloat16*>(v_raw), blk, lane);
+            stage_tile(gs, reinterpret_cast<const G*>(g_raw), blk, lane);
+        }
     } else {
-        stage_rows<T, kZ, kRound>(vs, static_cast<const T*>(a.v) + at0, C, rows, blk, lane);
-        stage_rows<G, kZ, kRoundG>(gs, static_cast<const G*>(a.gy) + at0, C, rows, blk, lane);
+        keep_rows<T>(dir == 0 ? k_raw : r_raw, (dir == 0 ? kp : rp) + at0, C, rows, blk, lane);
+        if (dir == 0) {
+            scan_block(tab, a.w + at0, C, rows, blk, lane);
+        } else {
+            stage_rows<T, kZ, kRound>(vs, static_cast<const T*>(a.v) + at0, C, rows, blk, lane);
+            stage_rows<G, kZ, kRoundG>(gs, static_cast<const G*>(a.gy) + at0, C, rows, blk, lane);
+        }
     }
     __syncthreads();
-    stage_scaled<T, kX, kRound>(pf + dir * kX * kPlane, col, tab, blk, dir, lane);
+    stage_scaled<kX>(pf + dir * kX * kPlane, k_raw, tab, blk, dir, lane);
     // m = gy v^T: two of the sixteen tiles per warp
     {
         AFrag<kZ> own;
@@ -1015,11 +1113,10 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 const int t = 32 * th + 16 * mt + 8 * half + g;
-                float r4[4] = {0.f, 0.f, 0.f, 0.f}, k4[4] = {0.f, 0.f, 0.f, 0.f};
+                float r4[4], k4[4];
                 const size_t at_t = base + static_cast<size_t>(t) * C + 16 * cs + 4 * q;
-                if (t < tokens) { load4(rp + at_t, r4); load4(kp + at_t, k4); }
-                round4<kRound>(r4);
-                round4<kRound>(k4);
+                load4(r_raw, t, cs, q, r4);
+                load4(k_raw, t, cs, q, k4);
                 const float dot = dots[t];
                 float g4[4];
 #pragma unroll
@@ -1039,10 +1136,9 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
             gu[e] += __shfl_xor_sync(0xffffffffu, gu[e], 16);
         }
         if (g == 0) put_row4(gus + th * N, cs, q, gu[0], gu[1], gu[2], gu[3]);
-        load_rows<T>(col, rp + at0, C, rows, lane);
     }
     __syncthreads();               // everyone is done with the planes of k
-    stage_scaled<T, kX, kRound>(pf + dir * kX * kPlane, col, tab, blk, dir, lane);
+    stage_scaled<kX>(pf + dir * kX * kPlane, r_raw, tab, blk, dir, lane);
     __syncthreads();
     {
         float u4[4];
@@ -1054,11 +1150,10 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 const int t = 32 * th + 16 * mt + 8 * half + g;
-                float r4[4] = {0.f, 0.f, 0.f, 0.f}, k4[4] = {0.f, 0.f, 0.f, 0.f};
+                float r4[4], k4[4];
                 const size_t at_t = base + static_cast<size_t>(t) * C + 16 * cs + 4 * q;
-                if (t < tokens) { load4(rp + at_t, r4); load4(kp + at_t, k4); }
-                round4<kRound>(r4);
-                round4<kRound>(k4);
+                load4(r_raw, t, cs, q, r4);
+                load4(k_raw, t, cs, q, k4);
                 const float dot = dots[t];
                 float g4[4];
 #pragma unroll
@@ -1078,7 +1173,8 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
         static_assert(kX > kP, "no room for the edge planes");
         __nv_bfloat16* e0 = pf + kP * kPlane;
         __nv_bfloat16* e1 = pf + (kX + kP) * kPlane;
-        pair_rows<T, kP, kRound>(kp + at0, rp + at0, a.u + h * N, tab, pf + dir * kX * kPlane, ms, dir ? e1 : e0, C, rows, blk, dir, lane);
+        pair_rows<kP>([&](Block& x) { load_block(x, k_raw, blk, g, q); }, [&](Block& x) { load_block(x, r_raw, blk, g, q); }, a.u + h * N, tab,
+                      pf + dir * kX * kPlane, ms, dir ? e1 : e0, blk, dir, lane);
         __syncthreads();
         float y[2][2][4];
         pair_outputs<kZ, kP, true>(y, ms, gs, e0, e1, a_left, a_right, cs, th, lane);
@@ -1095,6 +1191,11 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
     }
     // gw: g_m = edge + sum_{t >= m} diff_t - mine_m
     Table& dt = *reinterpret_cast<Table*>(pf);
+    const int t0 = warp * 8;                       // eight tokens per warp, lane = two channels
+    const size_t o0 = base + static_cast<size_t>(t0) * C + 2 * lane;
+    float2 w_own[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) w_own[t] = t0 + t < tokens ? __ldg(reinterpret_cast<const float2*>(a.w + o0 + static_cast<size_t>(t) * C)) : make_float2(0.f, 0.f);
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
@@ -1105,7 +1206,6 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
         }
     __syncthreads();
     {
-        const int t0 = warp * 8;                       // eight tokens per warp, lane = two channels
         float2 d[8];
         float2 run = make_float2(0.f, 0.f);
 #pragma unroll
@@ -1124,12 +1224,11 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a)
             later.x += s.x;
             later.y += s.y;
         }
-        const size_t o0 = base + static_cast<size_t>(t0) * C + 2 * lane;
 #pragma unroll
         for (int t = 0; t < 8; ++t)
             if (t0 + t < tokens) {
                 const size_t o = o0 + static_cast<size_t>(t) * C;
-                const float2 w = __ldg(reinterpret_cast<const float2*>(a.w + o));
+                const float2 w = w_own[t];
                 const float gx = (later.x + d[t].x) * decay_slope(w.x);
                 const float gz = (later.y + d[t].y) * decay_slope(w.y);
                 if (!a.scalar) *reinterpret_cast<float2*>(a.gw + o) = make_float2(gx, gz);
@@ -1159,7 +1258,7 @@ __global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, cons
 // ---- host side -------------------------------------------------------------------------------------------------
 static size_t forward_smem(int kz, int kx) { return static_cast<size_t>(kz + 5 * kx) * kPlane * 2 + sizeof(Table); }
 static size_t backward_smem(int kz, int kx) {
-    return static_cast<size_t>(2 * kz + 3 * kx) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 8) * N * sizeof(float);
+    return 2 * kRawTile + static_cast<size_t>(2 * kz + 3 * kx) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 8) * N * sizeof(float) + 16;
 }
 
 static int chunks_of(int T) { return (T + kChunk - 1) / kChunk; }
@@ -1262,10 +1361,17 @@ static int run_backward(int B, int T_, int H, const void* r, const void* k, cons
         ++launched;
     }
     float* gu_part = reinterpret_cast<float*>(states + 4 * plane);
-    GradArgs o{T_, H, n_chunks, ahead_of(static_cast<size_t>(B) * H * n_chunks), r, k, v, gy, w, aligned_bonus(u, H, workspace, stream), gr, gk, gv, gw, gu_part, unaligned16({gr, gk, gv, gw}), states, plane};
+    GradArgs o{T_, H, n_chunks, ahead_of(static_cast<size_t>(B) * H * n_chunks), r, k, v, gy, w, aligned_bonus(u, H, workspace, stream), gr, gk, gv, gw, gu_part, unaligned16({gr, gk, gv, gw}), states, plane,
+               static_cast<unsigned*>(workspace), failure_mirror(Op::wkv6_backward)};
+    tensor_map::bind_primary_context();
+    CUtensorMap mw, mk, mr, mv, mg;
+    const auto map = [&](CUtensorMap* m, const void* p, bool half, bool swizzled) { return tensor_map::make_btc(m, p, B, T_, C, N, kChunk, half, swizzled); };
+    if (!(map(&mw, w, false, false) && map(&mk, k, sizeof(T) == 2, sizeof(T) == 2) && map(&mr, r, sizeof(T) == 2, sizeof(T) == 2) &&
+          map(&mv, v, sizeof(T) == 2, false) && map(&mg, gy, sizeof(G) == 2, false)))
+        return -1;
     const auto kernel = wkv6_backward_kernel<T, G, O, kZ, kX, kP>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), backward_smem(kZ, kX))) return -1;
-    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, backward_smem(kZ, kX), stream>>>(o);
+    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, backward_smem(kZ, kX), stream>>>(o, mw, mk, mr, mv, mg);
     wkv6_bonus_kernel<<<C / 32, dim3(32, 32), 0, stream>>>(B * n_chunks, C, gu_part, gu);
     return launched;
 }
