@@ -746,11 +746,12 @@ __device__ __forceinline__ void pair_outputs(float (&y)[2][2][4], const __nv_bfl
 }
 
 // ---- kernel 2 ------------------------------------------------------------------------------------------------
-// A third of its stalls are global loads (31 % forward, 30 % backward; shared memory another 13 %).  Each CTA brings the inputs of the
-// one that starts a little later (half an SM count of CTAs: before that CTA has started, and so shortly that nothing is evicted) into
-// L2, which leaves 23 and 27 %.  B=32, H=12, forward / backward us, distance 0, 74, 148, 296, 592: T=4096 1152 / 3311, 1110 / 3247,
-// 1116 / 3297, 1126 / 3435, 1201 / 3461.  The pair, loops of either in turn, each within 0.2 %: 4480 -> 4342; B=16, H=6 1186 -> 1157;
-// B=100, T=196 772 -> 764.
+// What bounds it: three or two CTAs of eight warps on an SM (shared memory and registers), each waiting for its own results and its own loads.  Inputs
+// come in one set of TMA copies into places that planes take later (B=32, H=12, T=4096, forward / backward us: 661 -> 615 and, where k and r
+// also stay, 2302 -> 2060; T=196 47.0 -> 43.1, 155 -> 145).  Each CTA brings the inputs of the one that starts a little later (half
+// an SM count of CTAs: before that CTA has started, and so shortly that nothing is evicted) into L2: without that 707 / 2143 where 661 / 2055,
+// at a distance of an SM count 667 / 2089.  Tried in the backward: the edge's products while the tiles are under way 2081, states asked for
+// a barrier early 2211 (spills).
 // The rows of a head's chunk (all 256 threads share the lines):
 template <typename T>
 __device__ __forceinline__ void prefetch_rows(const T* p, int C, int rows) {
@@ -761,6 +762,8 @@ __device__ __forceinline__ void prefetch_rows(const T* p, int C, int rows) {
 __device__ __forceinline__ void prefetch_bytes(const void* p, int bytes) {
     for (int i = threadIdx.x * 128; i < bytes; i += 256 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p) + i));
 }
+
+constexpr uint32_t kRawTile = kChunk * N * 2;
 
 // ---- kernel 2, forward ---------------------------------------------------------------------------------------
 struct OutArgs {
@@ -775,22 +778,43 @@ struct OutArgs {
     bool scalar;              // y is not 16-byte aligned: 4-byte stores
     const uint4* states;      // [direction][b h][chunk][part][..], rows = value channels
     size_t plane;
+    unsigned* status;         // as in StateArgs
+    unsigned* mirror;
 };
 
 // kX parts of the scaled operands and states, kZ parts of v
 template <typename T, int kZ, int kX>
-__global__ void __launch_bounds__(256, 3) wkv6_forward_kernel(const OutArgs a) {
+__global__ void __launch_bounds__(256, 3)
+wkv6_forward_kernel(const OutArgs a, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mr,
+                    const __grid_constant__ CUtensorMap mv) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __nv_bfloat16* kf = reinterpret_cast<__nv_bfloat16*>(smem);       // k towards the right edge of its block, left edge behind it
     __nv_bfloat16* pairs = kf + 2 * kX * kPlane;
     __nv_bfloat16* edges = pairs + kX * kPlane;
     __nv_bfloat16* vs = edges + 2 * kX * kPlane;
     Table& tab = *reinterpret_cast<Table*>(vs + kZ * kPlane);
+    // tiles on their way (bfloat16 inputs, by TMA): v and r where k's planes will be, k where the pairs, w where the edges
+    uint64_t* bar = reinterpret_cast<uint64_t*>(&tab + 1);
+    unsigned char *const v_raw = smem, *const r_raw = smem + kRawTile, *const k_raw = reinterpret_cast<unsigned char*>(pairs),
+                  *const w_raw = reinterpret_cast<unsigned char*>(edges);
+    static_assert(2 * kPlane * 2 >= 2 * kRawTile && 2 * kPlane * 2 >= kChunk * N * 4 && 2 * kPlane * 2 % 1024 == 0, "room for the tiles");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     const int n = blockIdx.x % a.n_chunks, bh = blockIdx.x / a.n_chunks;
     const int b = bh / a.H, h = bh - b * a.H, C = a.H * N;
     const size_t base = (static_cast<size_t>(b) * a.T + n * kChunk) * C + static_cast<size_t>(h) * N;
     constexpr bool kRound = sizeof(T) == 4;
+    if (sizeof(T) == 2) {
+        if (threadIdx.x == 0) {
+            sm100::mbar_init(bar, 1);
+            sm100::mbar_init_fence();
+            sm100::mbar_expect_tx(bar, 3 * kRawTile + kChunk * N * 4);
+            sm100::tma_load_3d(w_raw, &mw, bar, h * N, n * kChunk, b);
+            sm100::tma_load_3d(v_raw, &mv, bar, h * N, n * kChunk, b);
+            sm100::tma_load_3d(r_raw, &mr, bar, h * N, n * kChunk, b);
+            sm100::tma_load_3d(k_raw, &mk, bar, h * N, n * kChunk, b);
+        }
+        __syncthreads();
+    }
     if (blockIdx.x + a.ahead < gridDim.x) {
         const int id = blockIdx.x + a.ahead, n2 = id % a.n_chunks, bh2 = id / a.n_chunks, b2 = bh2 / a.H, rows = a.T - n2 * kChunk;
         const size_t at = (static_cast<size_t>(b2) * a.T + n2 * kChunk) * C + static_cast<size_t>(bh2 - b2 * a.H) * N;
@@ -807,16 +831,41 @@ __global__ void __launch_bounds__(256, 3) wkv6_forward_kernel(const OutArgs a) {
         const int rows = a.T - (n * kChunk + blk * kBlock);
         const size_t at0 = base + static_cast<size_t>(blk) * kBlock * C;
         const T* k = static_cast<const T*>(a.k) + at0;
+        const T* r = static_cast<const T*>(a.r) + at0;
         __nv_bfloat16* planes = kf + dir * kX * kPlane;
-        Pair<T> kr[kBlock];
-        load_rows<T>(kr, k, C, rows, lane);
-        if (dir == 0) scan_block(tab, a.w + at0, C, rows, blk, lane);
-        else stage_rows<T, kZ, kRound>(vs, static_cast<const T*>(a.v) + at0, C, rows, blk, lane);
-        __syncthreads();
-        stage_scaled<T, kX, kRound>(planes, kr, tab, blk, dir, lane);
-        __syncthreads();
-        pair_rows<kX>([&](Block& x) { load_block<T, kRound>(x, static_cast<const T*>(a.r) + at0, C, rows, g, q); },
-                      [&](Block& x) { load_block<T, kRound>(x, k, C, rows, g, q); }, a.u + h * N, tab, planes, pairs, edges + dir * kX * kPlane, blk, dir, lane);
+        __nv_bfloat16* mine = edges + dir * kX * kPlane;
+        if constexpr (sizeof(T) == 2) {
+            if (!sm100::mbar_wait(bar, 0, kWaitLimit)) report_failure(a.status, a.mirror, 2u);
+            uint2 rr[2][4], kr[2][4];      // this thread's part of the block, out of the tiles before planes and pairs take their place
+#pragma unroll
+            for (int i = 0; i < 8; ++i) rr[i >> 2][i & 3] = raw4(r_raw, blk * kBlock + g + 8 * (i >> 2), i & 3, q);
+            if (dir == 0) scan_tile(tab, reinterpret_cast<const float*>(w_raw), rows, blk, lane);
+            else stage_tile(vs, reinterpret_cast<const __nv_bfloat16*>(v_raw), blk, lane);
+            __syncthreads();
+            stage_scaled<kX>(planes, k_raw, tab, blk, dir, lane);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) kr[i >> 2][i & 3] = raw4(k_raw, blk * kBlock + g + 8 * (i >> 2), i & 3, q);
+            __syncthreads();
+            const auto widen = [](Block& x, const uint2(&raw)[2][4]) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint2 v = raw[i >> 2][i & 3];
+                    float(&e)[4] = x[i >> 2][i & 3];
+                    e[0] = lo_f(v.x); e[1] = hi_f(v.x); e[2] = lo_f(v.y); e[3] = hi_f(v.y);
+                }
+            };
+            pair_rows<kX>([&](Block& x) { widen(x, rr); }, [&](Block& x) { widen(x, kr); }, a.u + h * N, tab, planes, pairs, mine, blk, dir, lane);
+        } else {
+            Pair<T> kr[kBlock];
+            load_rows<T>(kr, k, C, rows, lane);
+            if (dir == 0) scan_block(tab, a.w + at0, C, rows, blk, lane);
+            else stage_rows<T, kZ, kRound>(vs, static_cast<const T*>(a.v) + at0, C, rows, blk, lane);
+            __syncthreads();
+            stage_scaled<T, kX, kRound>(planes, kr, tab, blk, dir, lane);
+            __syncthreads();
+            pair_rows<kX>([&](Block& x) { load_block<T, kRound>(x, r, C, rows, g, q); }, [&](Block& x) { load_block<T, kRound>(x, k, C, rows, g, q); }, a.u + h * N,
+                          tab, planes, pairs, mine, blk, dir, lane);
+        }
     }
     __syncthreads();
     const int cs = warp & 3, th = warp >> 2;
@@ -855,7 +904,7 @@ struct GradArgs {
     unsigned* status;         // as in StateArgs
     unsigned* mirror;
 };
-constexpr uint32_t kRawTile = kChunk * N * 2;
+
 
 // gr (own = gy, partners k, m = gy v^T) or gk (own = v, partners r, m transposed) for 32 tokens x 16 channels:
 //   early / late[m tile][row half][e] = sum over earlier / later tokens s of (own_t . other_s) D(t, s) (x) partner_s,
@@ -1256,7 +1305,7 @@ __global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, cons
 }
 
 // ---- host side -------------------------------------------------------------------------------------------------
-static size_t forward_smem(int kz, int kx) { return static_cast<size_t>(kz + 5 * kx) * kPlane * 2 + sizeof(Table); }
+static size_t forward_smem(int kz, int kx) { return static_cast<size_t>(kz + 5 * kx) * kPlane * 2 + sizeof(Table) + 16; }
 static size_t backward_smem(int kz, int kx) {
     return 2 * kRawTile + static_cast<size_t>(2 * kz + 3 * kx) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 8) * N * sizeof(float) + 16;
 }
@@ -1342,10 +1391,16 @@ static int run_forward(int B, int T_, int H, const void* r, const void* k, const
         if (!run_states<T, T, kZ, kX, false>(B, T_, H, nullptr, k, v, w, nullptr, states, plane, workspace, stream)) return -1;
         ++launched;
     }
-    OutArgs o{T_, H, n_chunks, ahead_of(static_cast<size_t>(B) * H * n_chunks), r, k, v, w, aligned_bonus(u, H, workspace, stream), y, unaligned16({y}), states, plane};
+    OutArgs o{T_, H, n_chunks, ahead_of(static_cast<size_t>(B) * H * n_chunks), r, k, v, w, aligned_bonus(u, H, workspace, stream), y, unaligned16({y}), states, plane,
+              static_cast<unsigned*>(workspace), failure_mirror(Op::wkv6_forward)};
+    tensor_map::bind_primary_context();
+    CUtensorMap mw, mk, mr, mv;
+    const bool half = sizeof(T) == 2;
+    const auto map = [&](CUtensorMap* m, const void* p, bool narrow, bool swizzled) { return tensor_map::make_btc(m, p, B, T_, H * N, N, kChunk, narrow, swizzled); };
+    if (!(map(&mw, w, false, false) && map(&mk, k, half, half) && map(&mr, r, half, half) && map(&mv, v, half, false))) return -1;
     const auto kernel = wkv6_forward_kernel<T, kZ, kX>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), forward_smem(kZ, kX))) return -1;
-    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, forward_smem(kZ, kX), stream>>>(o);
+    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, forward_smem(kZ, kX), stream>>>(o, mw, mk, mr, mv);
     return launched;
 }
 
