@@ -1293,7 +1293,6 @@ __global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, cons
     __shared__ float red[32][33];
     const int c = blockIdx.x * 32 + threadIdx.x;
     float acc = 0.f;
-#pragma unroll 8
     for (int i = threadIdx.y; i < parts; i += 32) acc += part[static_cast<size_t>(i) * C + c];
     red[threadIdx.y][threadIdx.x] = acc;
     __syncthreads();
