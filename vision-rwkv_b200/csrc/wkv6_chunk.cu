@@ -1028,8 +1028,8 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
     float* dots = reinterpret_cast<float*>(&tab + 1);       // [kChunk]: gy_t . v_t
     float* edge = dots + N;                                 // [2][N]
     float* gus = edge + 2 * N;                              // [2][N]
-    float* seg = gus + 2 * N;                               // [8][N]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(seg + 8 * N);
+    float* seg = gus + 2 * N;                               // [N]: diff over the later half
+    uint64_t* bar = reinterpret_cast<uint64_t*>(seg + N);
     // tiles on their way into planes and table: w where m will be, v and gy where the scaled rows will be
     unsigned char *const w_raw = reinterpret_cast<unsigned char*>(ms), *const v_raw = reinterpret_cast<unsigned char*>(pf), *const g_raw = v_raw + kRawTile;
     static_assert(kX == 2, "room for the tiles");
@@ -1215,7 +1215,53 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
                 if (t < tokens) put4(a.scalar, static_cast<O*>(a.gk) + at_t, g4[0], g4[1], g4[2], g4[3]);
             }
     }
+    // gw: g_m = edge + sum_{t >= m} diff_t - mine_m, from the registers that hold them: a thread has its channels' tokens g of each eight, summed from
+    // the last one on over the lanes of a channel and from the later half of the chunk.  (Through tables in shared memory, behind gv,
+    // the two arrays were kept in local memory meanwhile, which with this much shared memory means L2.)
+    float4 w_own[2][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 32 * th + 8 * i + g;
+        w_own[i >> 1][i & 1] = t < tokens ? __ldg(reinterpret_cast<const float4*>(a.w + base + static_cast<size_t>(t) * C + 16 * cs + 4 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    {
+        float carry[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 3; i >= 0; --i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float& x = diff[i >> 1][i & 1][e];
+#pragma unroll
+                for (int off = 1; off < 8; off *= 2) {
+                    const float later = __shfl_down_sync(0xffffffffu, x, 4 * off);
+                    if (g + off < 8) x += later;
+                }
+                x += carry[e];
+                carry[e] = __shfl_sync(0xffffffffu, x, q);      // of the tokens from here on
+            }
+        if (th == 1 && g == 0) put_row4(seg, cs, q, carry[0], carry[1], carry[2], carry[3]);
+    }
     __syncthreads();               // m has been read
+    {
+        float later[4], e1[4], add[4] = {0.f, 0.f, 0.f, 0.f};
+        row4(edge, cs, q, later);
+        row4(edge + N, cs, q, e1);
+        if (th == 0) row4(seg, cs, q, add);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) later[e] = (later[e] + e1[e]) + add[e];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = 32 * th + 8 * i + g;
+            const float4 w = w_own[i >> 1][i & 1];
+            const float w4[4] = {w.x, w.y, w.z, w.w};
+            float g4[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) g4[e] = (later[e] + (diff[i >> 1][i & 1][e] - mine[i >> 1][i & 1][e])) * decay_slope(w4[e]);
+            if (t < tokens) put4(a.scalar, a.gw + base + static_cast<size_t>(t) * C + 16 * cs + 4 * q, g4[0], g4[1], g4[2], g4[3]);
+        }
+        if (threadIdx.x < N)
+            a.gu_part[(static_cast<size_t>(b) * a.n_chunks + n) * C + h * N + threadIdx.x] = gus[threadIdx.x] + gus[N + threadIdx.x];
+    }
     if (a.gv != nullptr) {
         // gv: rows are k, columns r, values gy: the forward with exchanged roles.  It needs only the first part of the scaled
         // rows; its edge planes take the room of the second.
@@ -1236,55 +1282,6 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
                     put4(a.scalar, static_cast<O*>(a.gv) + base + static_cast<size_t>(t) * C + 16 * cs + 4 * q, y[mt][0][2 * half],
                          y[mt][0][2 * half + 1], y[mt][1][2 * half], y[mt][1][2 * half + 1]);
             }
-        __syncthreads();
-    }
-    // gw: g_m = edge + sum_{t >= m} diff_t - mine_m
-    Table& dt = *reinterpret_cast<Table*>(pf);
-    const int t0 = warp * 8;                       // eight tokens per warp, lane = two channels
-    const size_t o0 = base + static_cast<size_t>(t0) * C + 2 * lane;
-    float2 w_own[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) w_own[t] = t0 + t < tokens ? __ldg(reinterpret_cast<const float2*>(a.w + o0 + static_cast<size_t>(t) * C)) : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int t = 32 * th + 16 * mt + 8 * half + g;
-            put_row4(tab[t], cs, q, mine[mt][half][0], mine[mt][half][1], mine[mt][half][2], mine[mt][half][3]);
-            put_row4(dt[t], cs, q, diff[mt][half][0], diff[mt][half][1], diff[mt][half][2], diff[mt][half][3]);
-        }
-    __syncthreads();
-    {
-        float2 d[8];
-        float2 run = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int t = 7; t >= 0; --t) {
-            const float2 x = *reinterpret_cast<const float2*>(&dt[t0 + t][2 * lane]);
-            const float2 m = *reinterpret_cast<const float2*>(&tab[t0 + t][2 * lane]);
-            run.x += x.x;
-            run.y += x.y;
-            d[t] = make_float2(run.x - m.x, run.y - m.y);
-        }
-        *reinterpret_cast<float2*>(seg + warp * N + 2 * lane) = run;
-        __syncthreads();
-        float2 later = make_float2(edge[2 * lane] + edge[N + 2 * lane], edge[2 * lane + 1] + edge[N + 2 * lane + 1]);
-        for (int j = warp + 1; j < 8; ++j) {
-            const float2 s = *reinterpret_cast<const float2*>(seg + j * N + 2 * lane);
-            later.x += s.x;
-            later.y += s.y;
-        }
-#pragma unroll
-        for (int t = 0; t < 8; ++t)
-            if (t0 + t < tokens) {
-                const size_t o = o0 + static_cast<size_t>(t) * C;
-                const float2 w = w_own[t];
-                const float gx = (later.x + d[t].x) * decay_slope(w.x);
-                const float gz = (later.y + d[t].y) * decay_slope(w.y);
-                if (!a.scalar) *reinterpret_cast<float2*>(a.gw + o) = make_float2(gx, gz);
-                else { a.gw[o] = gx; a.gw[o + 1] = gz; }
-            }
-        if (threadIdx.x < N)
-            a.gu_part[(static_cast<size_t>(b) * a.n_chunks + n) * C + h * N + threadIdx.x] = gus[threadIdx.x] + gus[N + threadIdx.x];
     }
 }
 
@@ -1307,7 +1304,7 @@ __global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, cons
 // ---- host side -------------------------------------------------------------------------------------------------
 static size_t forward_smem(int kz, int kx) { return static_cast<size_t>(kz + 5 * kx) * kPlane * 2 + sizeof(Table) + 16; }
 static size_t backward_smem(int kz, int kx) {
-    return 2 * kRawTile + static_cast<size_t>(2 * kz + 3 * kx) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 8) * N * sizeof(float) + 16;
+    return 2 * kRawTile + static_cast<size_t>(2 * kz + 3 * kx) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 1) * N * sizeof(float) + 16;
 }
 
 static int chunks_of(int T) { return (T + kChunk - 1) / kChunk; }
