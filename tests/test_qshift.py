@@ -201,3 +201,22 @@ def test_data_dependent_walks(cuda_device, B, H, W, C, head_dim, offsets):
     for o, h, r in zip(outs, half, ref):
         assert rel_err(o, r) < 1e-6
         assert torch.equal(h, o.bfloat16())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,W,C,head_dim,shift", [(1, 1, 1, 32, 32, 1), (3, 7, 5, 96, 32, 1), (2, 1, 9, 64, 64, 2), (5, 14, 14, 320, 64, 0), (1, 33, 2, 192, 192, 1)])
+def test_data_dependent_mix_by_tokens_and_along_lines_agree(cuda_device, B, H, W, C, head_dim, shift):
+    """bfloat16 offsets on a 16-byte boundary go by tokens, 8 channels a thread; on an 8-byte one along the lines or token by token.  The
+    same bits, and those of the formula to float32's last ones."""
+    from vision_rwkv_b200 import _lib
+    native = _lib.native()
+    g = torch.Generator(device=cuda_device).manual_seed(H * 100 + W)
+    x = torch.randn(B, H * W, C, device=cuda_device, generator=g)
+    maas = [torch.rand(1, 1, C, device=cuda_device, generator=g) for _ in range(5)]
+    ms = [None if j == 1 else (torch.randn(B, H * W, C, device=cuda_device, generator=g) * 0.3).bfloat16() for j in range(5)]
+    odd = [None if m is None else torch.empty(m.numel() + 4, device=cuda_device, dtype=torch.bfloat16)[4:].view_as(m).copy_(m) for m in ms]
+    ref = O.ddlerp(x.double().cpu(), [a.double().cpu().reshape(-1) for a in maas], [None if m is None else m.double().cpu() for m in ms], (H, W), shift, head_dim)
+    for run in (native.qshift_ddlerp_half, native.qshift_ddlerp):
+        a, b = run(x, maas, ms, H, W, shift, head_dim), run(x, maas, odd, H, W, shift, head_dim)
+        assert all(torch.equal(p, q) for p, q in zip(a, b))
+        assert all(rel_err(p, r) <= (4e-3 if p.dtype == torch.bfloat16 else 1e-6) for p, r in zip(a, ref))

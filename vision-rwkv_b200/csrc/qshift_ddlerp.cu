@@ -189,6 +189,59 @@ __global__ void __launch_bounds__(qlines::kMaxThreads, 2) ddlerp_lines_forward(c
     }
 }
 
+// Where offsets are most of the traffic and groups hold whole 8-channel vectors: a thread per token and vector, every access of 16 bytes, the
+// neighbour's x from L1 or L2.  Bound by HBM: five outputs at 64 x 14 x 14 x 768 in bfloat16, offsets too, 231 MB, 39.6 us (5.8 TB/s) where walks
+// along the lines, 4 channels and 20 requests of 8 bytes a thread, took 67; float32 offsets and bfloat16 results 58 for 93; 256 x 14 x 14 x 384
+// 72 for 116, 2 x 14 x 14 x 768 3.9 for 4.8.  Without offsets the walks are the faster ones (one output 14.2 for 17.0).
+template <bool kHalfM, typename Out>
+__global__ void __launch_bounds__(256, 4) ddlerp_tokens_forward(const Args a, unsigned vectors) {
+    const unsigned v = blockIdx.x * 256u + threadIdx.x;
+    if (v >= vectors) return;
+    const unsigned per_row = static_cast<unsigned>(a.C) / 8, tok = v / per_row, T = static_cast<unsigned>(a.H * a.W);
+    const int c = static_cast<int>(v - tok * per_row) * 8;
+    const unsigned t = tok % T;
+    const int h = static_cast<int>(t) / a.W, w = static_cast<int>(t) - h * a.W;
+    const size_t base = static_cast<size_t>(v) * 8;
+    const int src = source_token(a, h, w, c);
+    float4 x[2], d[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) x[i] = qlines::ld4(a.x + base + 4 * i);
+    const size_t from = static_cast<size_t>(tok - t + static_cast<unsigned>(src >= 0 ? src : 0)) * a.C + c;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) d[i] = src >= 0 ? qlines::ld4(a.x + from + 4 * i) : qlines::zero4();
+    RawM<kHalfM> m[kMaxOut][2];
+    uint4 both[kHalfM ? kMaxOut : 1];
+#pragma unroll
+    for (int j = 0; j < kMaxOut; ++j)
+        if (j < a.n_out && a.m[j] != nullptr) {
+            if (kHalfM) both[kHalfM ? j : 0] = __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.m[j]) + base));
+            else { m[j][0].get(a.m[j], base); m[j][1].get(a.m[j], base + 4); }
+        }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) d[i] = qlines::sub4(d[i], x[i]);
+#pragma unroll
+    for (int j = 0; j < kMaxOut; ++j)
+        if (j < a.n_out) {
+            float4 o[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                float4 offset = qlines::zero4();
+                if (a.m[j] != nullptr) {
+                    if (kHalfM) {
+                        const uint4 t4 = both[kHalfM ? j : 0];
+                        const uint2 half = i == 0 ? make_uint2(t4.x, t4.y) : make_uint2(t4.z, t4.w);
+                        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&half.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&half.y));
+                        offset = make_float4(lo.x, lo.y, hi.x, hi.y);
+                    } else {
+                        offset = m[j][i].f();
+                    }
+                }
+                o[i] = qlines::fma4(d[i], add4(qlines::ld4(a.maa[j] + c + 4 * i), offset), x[i]);
+            }
+            qlines::st8(reinterpret_cast<Out*>(a.out[j]) + base, o[0], o[1]);
+        }
+}
+
 template <bool kHalfM>
 __global__ void __launch_bounds__(kThreads) ddlerp_backward(const Args a) {
     const int cv = (blockIdx.x * kThreads + threadIdx.x) * kVec;
@@ -281,12 +334,21 @@ static bool misaligned(const void* p, uintptr_t a) { return (reinterpret_cast<ui
 }  // namespace ddlerp
 
 namespace ddlerp {
+// offsets of bfloat16 may be 8-byte aligned only
+static bool wide_m(const Args& a, bool half) {
+    for (int j = 0; j < a.n_out; ++j)
+        if (half && misaligned(a.m[j], 16)) return false;
+    return true;
+}
 template <bool kHalfM, typename Out>
 static void launch_forward(const Args& a, cudaStream_t s) {
     bool offsets = false;
     for (int j = 0; j < a.n_out; ++j) offsets = offsets || a.m[j] != nullptr;
     const qlines::Grid g = qlines::make_grid(a.B, a.H, a.W, a.C, a.head_dim / 4, a.head_dim, offsets ? kShort : qlines::kStretch);
-    if (a.shift == 1 && g.lines != 0) {       // any other shift: token by token
+    const long long vectors = static_cast<long long>(a.B) * a.H * a.W * (a.C / 8);
+    if (offsets && a.head_dim % 32 == 0 && wide_m(a, kHalfM) && vectors < (1LL << 31)) {
+        ddlerp_tokens_forward<kHalfM, Out><<<static_cast<unsigned>((vectors + 255) / 256), 256, 0, s>>>(a, static_cast<unsigned>(vectors));
+    } else if (a.shift == 1 && g.lines != 0) {       // any other shift: token by token
         const qlines::Shape shape = qlines::make_shape(g);
         if (offsets) ddlerp_lines_forward<kHalfM, true, Out><<<shape.grid, shape.block, 0, s>>>(a, g);
         else ddlerp_lines_forward<kHalfM, false, Out><<<shape.grid, shape.block, 0, s>>>(a, g);

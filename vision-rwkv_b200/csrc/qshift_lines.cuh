@@ -114,4 +114,14 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = raw;
 }
 
+__device__ __forceinline__ void st8(float* p, float4 a, float4 b) { st4(p, a); st4(p + 4, b); }
+__device__ __forceinline__ void st8(__nv_bfloat16* p, float4 a, float4 b) {
+    uint4 raw;
+    *reinterpret_cast<__nv_bfloat162*>(&raw.x) = __floats2bfloat162_rn(a.x, a.y);
+    *reinterpret_cast<__nv_bfloat162*>(&raw.y) = __floats2bfloat162_rn(a.z, a.w);
+    *reinterpret_cast<__nv_bfloat162*>(&raw.z) = __floats2bfloat162_rn(b.x, b.y);
+    *reinterpret_cast<__nv_bfloat162*>(&raw.w) = __floats2bfloat162_rn(b.z, b.w);
+    *reinterpret_cast<uint4*>(p) = raw;
+}
+
 }  // namespace qlines
