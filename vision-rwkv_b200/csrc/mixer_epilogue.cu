@@ -307,18 +307,20 @@ __global__ void __launch_bounds__(kThreads) layer_norm_kernel(int rows, int C, f
         }
 }
 
-// Per-head norm and gate, a half-warp per 64-channel head: lane q holds channel pairs q and q + 16, which makes the sums'
-// order that of normgate_forward_kernel (a warp per head, one pair per lane; its butterfly adds those two first), and so
-// the bits of the float32 result before it is rounded.  kHeads heads per half-warp are requested together: one 256-byte
-// request per warp in flight left that kernel at about half of the HBM rate.
-constexpr int kHeads = 4;
-__device__ __forceinline__ float half_warp_sum(float v) {
+// Per-head norm and gate, eight lanes per 64-channel head: lane q holds channels 4 q .. 4 q + 3 and 32 behind them, in 16-byte accesses.  The
+// sums go pair by pair in the order of normgate_forward_kernel (a warp per head, one pair per lane), and so give the bits of its float32 result before it
+// is rounded: there lane l, of channels 2 l and 2 l + 1, meets l + 16 first, then 8, 4, 2 and 1 lanes away; here lanes 2 q and 2 q + 1 of that
+// order are one thread's, whose two sums meet last.  12544 x 768 with a bfloat16 gate (77 MB): 19.5 us with a half-warp per head, accesses of 8 and 4
+// bytes and four heads requested together, 14.9 now (two heads together 16.2, four 21.7: fewer threads on an SM); 50176 x 384 42.9 -> 34.3.
+constexpr int kLanes = 8;
+__device__ __forceinline__ float eight_lane_sum(float even, float odd) {
 #pragma unroll
-    for (int m = 8; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-    return v;
+    for (int m = kLanes / 2; m >= 1; m >>= 1) {
+        even += __shfl_xor_sync(0xffffffffu, even, m);
+        odd += __shfl_xor_sync(0xffffffffu, odd, m);
+    }
+    return even + odd;
 }
-__device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
-__device__ __forceinline__ float2 load2(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 __device__ __forceinline__ float activation(float x, int act) {
     if (act == 0) return x;
     const float s = 1.f / (1.f + __expf(-x));
@@ -328,43 +330,39 @@ template <typename G>
 __global__ void __launch_bounds__(kThreads) head_norm_gate_kernel(long long heads, int per_row, float eps, const float* __restrict__ x,
                                                                   const G* __restrict__ gate, int act, const float* __restrict__ gamma,
                                                                   const float* __restrict__ beta, __nv_bfloat16* __restrict__ out) {
-    const int q = threadIdx.x & 15;
-    const long long first = static_cast<long long>(blockIdx.x) * (kThreads / 16 * kHeads) + (threadIdx.x >> 4);
-    float2 v[kHeads][2], g[kHeads][2];
+    const int q = threadIdx.x & (kLanes - 1);
+    const long long mine = static_cast<long long>(blockIdx.x) * (kThreads / kLanes) + threadIdx.x / kLanes;
+    const long long head = min(mine, heads - 1);      // a repeated head is computed and not stored
+    float v[2][4], g[2][4];
 #pragma unroll
-    for (int j = 0; j < kHeads; ++j) {
-        const long long head = min(first + j * (kThreads / 16), heads - 1);      // repeated heads are computed and not stored
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            v[j][i] = load2(x + head * 64 + 2 * q + 32 * i);
-            g[j][i] = load2(gate + head * 64 + 2 * q + 32 * i);
-        }
+    for (int i = 0; i < 2; ++i) {
+        load(x + head * 64 + 4 * q + 32 * i, v[i]);
+        load(gate + head * 64 + 4 * q + 32 * i, g[i]);
     }
     const float inv = 1.f / 64.f;
+    const float mean = eight_lane_sum((v[0][0] + v[0][1]) + (v[1][0] + v[1][1]), (v[0][2] + v[0][3]) + (v[1][2] + v[1][3])) * inv;
+    float part[2][2];
 #pragma unroll
-    for (int j = 0; j < kHeads; ++j) {
-        const long long head = first + j * (kThreads / 16);
-        const float mean = half_warp_sum((v[j][0].x + v[j][0].y) + (v[j][1].x + v[j][1].y)) * inv;
-        float part[2];
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            float s = 0.f;
+            const float dx = v[i][2 * p] - mean, dy = v[i][2 * p + 1] - mean;
+            s += dx * dx + dy * dy;
+            part[p][i] = s;
+        }
+    const float rstd = rsqrtf(eight_lane_sum(part[0][0] + part[0][1], part[1][0] + part[1][1]) * inv + eps);
+    if (mine < heads) {
+        const int c = static_cast<int>(head % per_row) * 64 + 4 * q;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            float s = 0.f;
-            const float dx = v[j][i].x - mean, dy = v[j][i].y - mean;
-            s += dx * dx + dy * dy;
-            part[i] = s;
-        }
-        const float rstd = rsqrtf(half_warp_sum(part[0] + part[1]) * inv + eps);
-        if (head < heads) {
-            const int c = static_cast<int>(head % per_row) * 64 + 2 * q;
+            float ga[4], be[4], o[4];
+            load(gamma + c + 32 * i, ga);
+            load(beta + c + 32 * i, be);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float2 ga = load2(gamma + c + 32 * i), be = load2(beta + c + 32 * i);
-                const float ox = ((v[j][i].x - mean) * rstd * ga.x + be.x) * activation(g[j][i].x, act);
-                const float oy = ((v[j][i].y - mean) * rstd * ga.y + be.y) * activation(g[j][i].y, act);
-                *reinterpret_cast<uint32_t*>(out + head * 64 + 2 * q + 32 * i) = narrow(ox, oy);
-            }
+            for (int e = 0; e < 4; ++e) o[e] = ((v[i][e] - mean) * rstd * ga[e] + be[e]) * activation(g[i][e], act);
+            *reinterpret_cast<uint2*>(out + head * 64 + 4 * q + 32 * i) = make_uint2(narrow(o[0], o[1]), narrow(o[2], o[3]));
         }
-        __syncwarp();
     }
 }
 
@@ -525,7 +523,7 @@ extern "C" int vrwkv_head_norm_gate_bf16out(int rows, int C, float eps, const fl
     if (rows <= 0 || C <= 0 || C % 64 != 0 || gate_act < 0 || gate_act > 2) return VRWKV_ERR_SHAPE;
     if (!x || !gate || !gamma || !beta || !out) return VRWKV_ERR_NULL;
     if (misaligned({x, gate, gamma, beta, out})) return VRWKV_ERR_ALIGNMENT;
-    const long long heads = static_cast<long long>(rows) * (C / 64), per = kThreads / 16 * kHeads, grid = (heads + per - 1) / per;
+    const long long heads = static_cast<long long>(rows) * (C / 64), per = kThreads / kLanes, grid = (heads + per - 1) / per;
     if (grid > 0x7fffffffLL) return VRWKV_ERR_SHAPE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto* const o = reinterpret_cast<__nv_bfloat16*>(out);
