@@ -56,6 +56,7 @@
 #include <mutex>
 #include "biwkv_math.cuh"
 #include "biwkv_pairs.cuh"
+#include "launch.h"
 #include "sm100_async.cuh"
 #include "tensor_map.h"
 #include "vrwkv_internal.h"
@@ -122,7 +123,6 @@ struct Params {
 constexpr unsigned kRedo = 1u, kFailedShift = 8;
 // what may be launched behind this grid need not wait for its end any longer; what a dependent grid reads of the one before it
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 struct Ctx {
     float* sub;      // [n_warps][kRecRows][kCs]
@@ -500,6 +500,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 3)
 biwkv_forward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                      const __grid_constant__ CUtensorMap map_y,     // float32 results
                      const Params p) {
+    wait_for_launch_before();
     constexpr int P = St::P, L = St::L, kCs = St::kCs, kSpan = St::kSpan, kArea = St::kAreaFloats, kG = St::kGroup, kGroups = St::kGroups;
     constexpr bool kHalf = kTypes != Types::f32, kHalfOut = kTypes == Types::bf16;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -605,6 +606,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 2)
 biwkv_backward_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                       const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_gk,     // float32 results
                       const __grid_constant__ CUtensorMap map_gv, const Params p) {
+    wait_for_launch_before();
     constexpr int P = St::P, L = St::L, kCs = St::kCs, kSpan = St::kSpan, kArea = St::kAreaFloats, kG = St::kGroup, kGroups = St::kGroups;
     constexpr bool kHalf = kTypes != Types::f32, kHalfG = kTypes == Types::bf16;            // bfloat16 k, v, gk, gv ; gy
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -1376,8 +1378,8 @@ static int launch(const Plan& pl, int B, int T, int C, const float* w, const flo
     const size_t units = p.units;
     const size_t smem = smem_bytes<St, kBwd>(pl.n_warps, pl.cluster);
     bool done;
-    if constexpr (kBwd) done = run(backward_kernel<St, kTypes>(pl.cluster == 1), false, units, smem, mk, mv, mg, m0, m1);
-    else done = run(forward_kernel<St, kTypes>(pl.cluster == 1), false, units, smem, mk, mv, m0);
+    if constexpr (kBwd) done = run(backward_kernel<St, kTypes>(pl.cluster == 1), true, units, smem, mk, mv, mg, m0, m1);
+    else done = run(forward_kernel<St, kTypes>(pl.cluster == 1), true, units, smem, mk, mv, m0);
     if (!done) return -1;
     // the exact kernel: a few clusters that serve whatever the fast kernel left behind
     if (!run(biwkv_exact_kernel<St, kBwd, kTypes>, true, std::min<size_t>(units, std::max(16, 128 / pl.cluster)), exact_smem<St, kBwd>(pl.n_warps), mk, mv, mg, m0, m1)) return -1;

@@ -23,6 +23,7 @@
 #include <mutex>
 #include <utility>
 #include "../../include/vrwkv_b200.h"
+#include "launch.h"
 #include "linear_tc.cuh"
 #include "sm100_async.cuh"
 #include "tensor_map.h"
@@ -178,6 +179,7 @@ static size_t batch_smem(int K) { return K * kSlab * 2 + kStages * kXBytes + kSl
 template <int kStages, int kSlots, bool kSquare, bool kTest>
 __global__ void __launch_bounds__(kBatchThreads, 1)
 linear_batch_kernel(const __grid_constant__ Products maps, int count, int m_tiles, int n_slabs, int k_blocks, unsigned* mirror) {
+    wait_for_launch_before();
     constexpr int kPerTile = kSlab / 64;
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t slab = smem_u32(smem), stages = slab + k_blocks * kWBytes, outs = stages + kStages * kXBytes;
@@ -270,7 +272,7 @@ static int run_batch(int count, long long rows, int K, int N, const uint16_t* co
                tensor_map::make_rows(maps.out + i, out[i], rows, N, 64, kM);
     if (!made) return refused("cuTensorMapEncodeTiled rejected a matrix");
     const int m_tiles = static_cast<int>((rows + kM - 1) / kM);
-    kernel<<<std::min(m_tiles, sms / slabs) * slabs, kBatchThreads, batch_smem<kStages, kSlots>(K), static_cast<cudaStream_t>(stream)>>>(maps, count, m_tiles, N / kSlab, K / kSlice,
+    launch_behind(kernel, std::min(m_tiles, sms / slabs) * slabs, kBatchThreads, batch_smem<kStages, kSlots>(K), static_cast<cudaStream_t>(stream), maps, count, m_tiles, N / kSlab, K / kSlice,
                                                                                                                 failure_mirror(Op::linear));
     return record_launches(1);
 }

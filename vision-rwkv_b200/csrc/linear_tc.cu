@@ -22,6 +22,7 @@
 #include <atomic>
 #include <mutex>
 #include "../../include/vrwkv_b200.h"
+#include "launch.h"
 #include "linear_tc.cuh"
 #include "sm100_async.cuh"
 #include "tensor_map.h"
@@ -46,6 +47,7 @@ template <bool kTest>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_relu_square_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mo,
                           int m_tiles, int n_tiles, int k_blocks, unsigned* mirror) {
+    wait_for_launch_before();
     extern __shared__ unsigned char smem_raw[];
     const uint32_t stages = (smem_u32(smem_raw) + 1023u) & ~1023u, out = stages + kStages * kStageBytes;
     Bars& s = *reinterpret_cast<Bars*>(smem_raw + (out + 2 * kBoxBytes - smem_u32(smem_raw)));
@@ -242,7 +244,7 @@ extern "C" int vrwkv_linear_relu_square(long long rows, int K, int N, const uint
         return VRWKV_ERR_DEVICE;
     }
     const auto kernel = withhold_test() ? linear_relu_square_kernel<true> : linear_relu_square_kernel<false>;
-    kernel<<<static_cast<unsigned>(std::min<long long>(tiles, sms)), kThreads, kSmem, static_cast<cudaStream_t>(stream)>>>(
-        mx, mw, mo, static_cast<int>(m_tiles), N / kN, K / kK, failure_mirror(Op::linear));
+    launch_behind(kernel, static_cast<unsigned>(std::min<long long>(tiles, sms)), kThreads, kSmem, static_cast<cudaStream_t>(stream),
+                  mx, mw, mo, static_cast<int>(m_tiles), N / kN, K / kK, failure_mirror(Op::linear));
     return record_launches(1);
 }

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <type_traits>
+#include "launch.h"
 #include "vrwkv_b200.h"
 #include "vrwkv_internal.h"
 
@@ -106,6 +107,7 @@ __device__ __forceinline__ float relu2(float x) {
 // under autocast is a pass of 6 bytes per element, this one of 2 more: the matrix-state base model on 64 images 10.15 -> 9.90 ms).
 template <typename R, typename Y, typename O>
 __global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, const R* __restrict__ r, const Y* __restrict__ y, O* __restrict__ out) {
+    wait_for_launch_before();
     const long long i = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVec;
     if (i + kVec <= n) {
         float a[kVec], b[kVec];
@@ -129,6 +131,7 @@ __global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, con
 
 template <typename R, typename O>
 __global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, const R* __restrict__ x, O* __restrict__ out) {
+    wait_for_launch_before();
     const long long i = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVec;
     if (i + kVec <= n) {
         float a[kVec];
@@ -144,6 +147,7 @@ __global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, cons
 // out[i] = table[i mod period] + a[i], eight elements (one 8-element vector of the table) per thread
 __global__ void __launch_bounds__(kThreads) add_rows_kernel(unsigned vectors, unsigned period, const float* __restrict__ table,
                                                             const __nv_bfloat16* __restrict__ a, float* __restrict__ out) {
+    wait_for_launch_before();
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= vectors) return;
     float v[kVec], t[kVec];
@@ -156,6 +160,7 @@ __global__ void __launch_bounds__(kThreads) add_rows_kernel(unsigned vectors, un
 
 // HBM-bound: 12544 x 768 take 11.4 us (5.1 TB/s), torch's cast 21; the matrix-state base model on 64 images 9.62 -> 9.49 ms.
 __global__ void __launch_bounds__(kThreads) widen_kernel(unsigned vectors, const __nv_bfloat16* __restrict__ a, float* __restrict__ out) {
+    wait_for_launch_before();
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= vectors) return;
     float v[kVec];
@@ -169,6 +174,7 @@ __global__ void __launch_bounds__(kThreads) widen_kernel(unsigned vectors, const
 // convolution, 1.14 ms of it, the small model took 8.0 ms for 256 images of 224 pixels, this way 6.7.
 __global__ void __launch_bounds__(kThreads) patch_rows_kernel(unsigned vectors, int channels, int H, int W, int rows, int cols, int patch,
                                                               const float* __restrict__ img, __nv_bfloat16* __restrict__ out) {
+    wait_for_launch_before();
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= vectors) return;
     const unsigned per_row = static_cast<unsigned>(cols * patch) / kVec, lines = static_cast<unsigned>(rows * patch);
@@ -195,6 +201,7 @@ __global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C
                                                                  const float* __restrict__ weight,
                                                                  const float* __restrict__ bias, const float* __restrict__ gamma,
                                                                  const float* __restrict__ x, float* __restrict__ out) {
+    wait_for_launch_before();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -267,6 +274,7 @@ __global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C
 template <int kIters>
 __global__ void __launch_bounds__(kThreads) layer_norm_kernel(int rows, int C, float eps, const float* __restrict__ x, const float* __restrict__ weight,
                                                               const float* __restrict__ bias, float* __restrict__ out) {
+    wait_for_launch_before();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -330,6 +338,7 @@ template <typename G>
 __global__ void __launch_bounds__(kThreads) head_norm_gate_kernel(long long heads, int per_row, float eps, const float* __restrict__ x,
                                                                   const G* __restrict__ gate, int act, const float* __restrict__ gamma,
                                                                   const float* __restrict__ beta, __nv_bfloat16* __restrict__ out) {
+    wait_for_launch_before();
     const int q = threadIdx.x & (kLanes - 1);
     const long long mine = static_cast<long long>(blockIdx.x) * (kThreads / kLanes) + threadIdx.x / kLanes;
     const long long head = min(mine, heads - 1);      // a repeated head is computed and not stored
@@ -381,9 +390,12 @@ static void launch_norm_residual(int rows, int C, float eps, const A* a, const A
     }
     const int per = kThreads / 32, grid = (rows + per - 1) / per;
     if constexpr (std::is_same<A, __nv_bfloat16>::value) {
-        if (gate != nullptr) return norm_residual_kernel<A, kIters, true><<<grid, kThreads, 0, s>>>(rows, C, eps, a, gate, weight, bias, gamma, x, out);
+        if (gate != nullptr) {
+            launch_behind(norm_residual_kernel<A, kIters, true>, grid, kThreads, 0, s, rows, C, eps, a, gate, weight, bias, gamma, x, out);
+            return;
+        }
     }
-    norm_residual_kernel<A, kIters, false><<<grid, kThreads, 0, s>>>(rows, C, eps, a, nullptr, weight, bias, gamma, x, out);
+    launch_behind(norm_residual_kernel<A, kIters, false>, grid, kThreads, 0, s, rows, C, eps, a, nullptr, weight, bias, gamma, x, out);
 }
 template <int kIters = 1>
 static void launch_layer_norm(int rows, int C, float eps, const float* x, const float* weight, const float* bias, float* out, cudaStream_t s) {
@@ -391,7 +403,7 @@ static void launch_layer_norm(int rows, int C, float eps, const float* x, const 
         if (C > 128 * kIters) return launch_layer_norm<kIters + 1>(rows, C, eps, x, weight, bias, out, s);
     }
     constexpr int kPer = kThreads / 32;
-    layer_norm_kernel<kIters><<<rows / kPer + (rows % kPer != 0 ? 1 : 0), kThreads, 0, s>>>(rows, C, eps, x, weight, bias, out);
+    launch_behind(layer_norm_kernel<kIters>, rows / kPer + (rows % kPer != 0 ? 1 : 0), kThreads, 0, s, rows, C, eps, x, weight, bias, out);
 }
 
 }  // namespace epilogue
@@ -405,9 +417,9 @@ extern "C" int vrwkv_sigmoid_gate(long long n, const void* r, int r_is_bf16, con
     const unsigned grid = static_cast<unsigned>(blocks_of(n));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     using H = __nv_bfloat16;
-    if (y_is_bf16) sigmoid_gate_kernel<H, H, H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(r), static_cast<const H*>(y), static_cast<H*>(out));
-    else if (r_is_bf16) sigmoid_gate_kernel<H, float, H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(r), static_cast<const float*>(y), static_cast<H*>(out));
-    else sigmoid_gate_kernel<float, float, float><<<grid, kThreads, 0, s>>>(n, static_cast<const float*>(r), static_cast<const float*>(y), static_cast<float*>(out));
+    if (y_is_bf16) launch_behind(sigmoid_gate_kernel<H, H, H>, grid, kThreads, 0, s, n, static_cast<const H*>(r), static_cast<const H*>(y), static_cast<H*>(out));
+    else if (r_is_bf16) launch_behind(sigmoid_gate_kernel<H, float, H>, grid, kThreads, 0, s, n, static_cast<const H*>(r), static_cast<const float*>(y), static_cast<H*>(out));
+    else launch_behind(sigmoid_gate_kernel<float, float, float>, grid, kThreads, 0, s, n, static_cast<const float*>(r), static_cast<const float*>(y), static_cast<float*>(out));
     return record_launches(1);
 }
 
@@ -417,8 +429,8 @@ extern "C" int vrwkv_sigmoid_gate_f32out(long long n, const uint16_t* r, const u
     if (!r || !y || !out) return VRWKV_ERR_NULL;
     if (misaligned({r, y, out})) return VRWKV_ERR_ALIGNMENT;
     using H = __nv_bfloat16;
-    sigmoid_gate_kernel<H, H, float><<<static_cast<unsigned>(blocks_of(n)), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        n, reinterpret_cast<const H*>(r), reinterpret_cast<const H*>(y), out);
+    launch_behind(sigmoid_gate_kernel<H, H, float>, static_cast<unsigned>(blocks_of(n)), kThreads, 0, static_cast<cudaStream_t>(stream),
+                  n, reinterpret_cast<const H*>(r), reinterpret_cast<const H*>(y), out);
     return record_launches(1);
 }
 
@@ -430,8 +442,8 @@ extern "C" int vrwkv_relu_square(long long n, const void* x, int is_bf16, void* 
     const unsigned grid = static_cast<unsigned>(blocks_of(n));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     using H = __nv_bfloat16;
-    if (is_bf16) relu_square_kernel<H, H><<<grid, kThreads, 0, s>>>(n, static_cast<const H*>(x), static_cast<H*>(out));
-    else relu_square_kernel<float, float><<<grid, kThreads, 0, s>>>(n, static_cast<const float*>(x), static_cast<float*>(out));
+    if (is_bf16) launch_behind(relu_square_kernel<H, H>, grid, kThreads, 0, s, n, static_cast<const H*>(x), static_cast<H*>(out));
+    else launch_behind(relu_square_kernel<float, float>, grid, kThreads, 0, s, n, static_cast<const float*>(x), static_cast<float*>(out));
     return record_launches(1);
 }
 
@@ -440,8 +452,8 @@ extern "C" int vrwkv_relu_square_f32out(long long n, const uint16_t* x, float* o
     if (n <= 0 || blocks_of(n) > 0x7fffffffLL) return VRWKV_ERR_SHAPE;
     if (!x || !out) return VRWKV_ERR_NULL;
     if (misaligned({x, out})) return VRWKV_ERR_ALIGNMENT;
-    relu_square_kernel<__nv_bfloat16, float><<<static_cast<unsigned>(blocks_of(n)), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        n, reinterpret_cast<const __nv_bfloat16*>(x), out);
+    launch_behind(relu_square_kernel<__nv_bfloat16, float>, static_cast<unsigned>(blocks_of(n)), kThreads, 0, static_cast<cudaStream_t>(stream),
+                  n, reinterpret_cast<const __nv_bfloat16*>(x), out);
     return record_launches(1);
 }
 
@@ -452,8 +464,8 @@ extern "C" int vrwkv_add_rows(long long n, long long period, const float* table,
     if (period % kVec != 0 || n / kVec > 0x7fffffffLL - kThreads) return VRWKV_ERR_UNSUPPORTED;
     if (misaligned({table, a, out})) return VRWKV_ERR_ALIGNMENT;
     const unsigned vectors = static_cast<unsigned>(n / kVec);
-    add_rows_kernel<<<(vectors + kThreads - 1) / kThreads, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        vectors, static_cast<unsigned>(period / kVec), table, reinterpret_cast<const __nv_bfloat16*>(a), out);
+    launch_behind(add_rows_kernel, (vectors + kThreads - 1) / kThreads, kThreads, 0, static_cast<cudaStream_t>(stream),
+                  vectors, static_cast<unsigned>(period / kVec), table, reinterpret_cast<const __nv_bfloat16*>(a), out);
     return record_launches(1);
 }
 
@@ -464,7 +476,8 @@ extern "C" int vrwkv_widen(long long n, const uint16_t* a, float* out, void* str
     if (n % kVec != 0 || n / kVec > 0x7fffffffLL - kThreads) return VRWKV_ERR_UNSUPPORTED;
     if (misaligned({a, out})) return VRWKV_ERR_ALIGNMENT;
     const unsigned vectors = static_cast<unsigned>(n / kVec);
-    widen_kernel<<<(vectors + kThreads - 1) / kThreads, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(vectors, reinterpret_cast<const __nv_bfloat16*>(a), out);
+    launch_behind(widen_kernel, (vectors + kThreads - 1) / kThreads, kThreads, 0, static_cast<cudaStream_t>(stream),
+                  vectors, reinterpret_cast<const __nv_bfloat16*>(a), out);
     return record_launches(1);
 }
 
@@ -477,8 +490,8 @@ extern "C" int vrwkv_patch_rows(int B, int channels, int H, int W, int patch, co
     // image rows start on 16-byte boundaries, 8 pixels never span two patches
     if (patch % kVec != 0 || W % 4 != 0 || vectors > 0x7fffffffLL - kThreads) return VRWKV_ERR_UNSUPPORTED;
     if (misaligned({img, out})) return VRWKV_ERR_ALIGNMENT;
-    patch_rows_kernel<<<static_cast<unsigned>((vectors + kThreads - 1) / kThreads), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<unsigned>(vectors), channels, H, W, rows, cols, patch, img, reinterpret_cast<__nv_bfloat16*>(out));
+    launch_behind(patch_rows_kernel, static_cast<unsigned>((vectors + kThreads - 1) / kThreads), kThreads, 0, static_cast<cudaStream_t>(stream),
+                  static_cast<unsigned>(vectors), channels, H, W, rows, cols, patch, img, reinterpret_cast<__nv_bfloat16*>(out));
     return record_launches(1);
 }
 
@@ -528,10 +541,10 @@ extern "C" int vrwkv_head_norm_gate_bf16out(int rows, int C, float eps, const fl
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto* const o = reinterpret_cast<__nv_bfloat16*>(out);
     if (gate_is_bf16)
-        head_norm_gate_kernel<<<static_cast<unsigned>(grid), kThreads, 0, s>>>(heads, C / 64, eps, x, static_cast<const __nv_bfloat16*>(gate), gate_act,
+        launch_behind(head_norm_gate_kernel<__nv_bfloat16>, static_cast<unsigned>(grid), kThreads, 0, s, heads, C / 64, eps, x, static_cast<const __nv_bfloat16*>(gate), gate_act,
                                                                                gamma, beta, o);
     else
-        head_norm_gate_kernel<<<static_cast<unsigned>(grid), kThreads, 0, s>>>(heads, C / 64, eps, x, static_cast<const float*>(gate), gate_act, gamma,
+        launch_behind(head_norm_gate_kernel<float>, static_cast<unsigned>(grid), kThreads, 0, s, heads, C / 64, eps, x, static_cast<const float*>(gate), gate_act, gamma,
                                                                                beta, o);
     return record_launches(1);
 }

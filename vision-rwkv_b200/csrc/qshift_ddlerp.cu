@@ -16,6 +16,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "launch.h"
 #include "qshift_lines.cuh"
 #include "vrwkv_b200.h"
 #include "vrwkv_internal.h"
@@ -149,6 +150,7 @@ struct RawM<false> {
 // kOffsets = false: no output has an offset, nothing but x is read; stretches of qlines::kStretch then.
 template <bool kHalfM, bool kOffsets, typename Out>
 __global__ void __launch_bounds__(qlines::kMaxThreads, 2) ddlerp_lines_forward(const Args a, const qlines::Grid g) {
+    wait_for_launch_before();
     using namespace qlines;
     const int cv = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (cv >= g.C) return;
@@ -195,6 +197,7 @@ __global__ void __launch_bounds__(qlines::kMaxThreads, 2) ddlerp_lines_forward(c
 // 72 for 116, 2 x 14 x 14 x 768 3.9 for 4.8.  Without offsets the walks are the faster ones (one output 14.2 for 17.0).
 template <bool kHalfM, typename Out>
 __global__ void __launch_bounds__(256, 4) ddlerp_tokens_forward(const Args a, unsigned vectors) {
+    wait_for_launch_before();
     const unsigned v = blockIdx.x * 256u + threadIdx.x;
     if (v >= vectors) return;
     const unsigned per_row = static_cast<unsigned>(a.C) / 8, tok = v / per_row, T = static_cast<unsigned>(a.H * a.W);
@@ -304,6 +307,7 @@ struct ReduceArgs {
     float* gmaa[kMaxOut];
 };
 __global__ void __launch_bounds__(1024) ddlerp_reduce(const ReduceArgs r) {
+    wait_for_launch_before();
     __shared__ float red[32][33];
     const int c = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y;
     float acc = 0.f;
@@ -347,11 +351,11 @@ static void launch_forward(const Args& a, cudaStream_t s) {
     const qlines::Grid g = qlines::make_grid(a.B, a.H, a.W, a.C, a.head_dim / 4, a.head_dim, offsets ? kShort : qlines::kStretch);
     const long long vectors = static_cast<long long>(a.B) * a.H * a.W * (a.C / 8);
     if (offsets && a.head_dim % 32 == 0 && wide_m(a, kHalfM) && vectors < (1LL << 31)) {
-        ddlerp_tokens_forward<kHalfM, Out><<<static_cast<unsigned>((vectors + 255) / 256), 256, 0, s>>>(a, static_cast<unsigned>(vectors));
+        launch_behind(ddlerp_tokens_forward<kHalfM, Out>, static_cast<unsigned>((vectors + 255) / 256), 256, 0, s, a, static_cast<unsigned>(vectors));
     } else if (a.shift == 1 && g.lines != 0) {       // any other shift: token by token
         const qlines::Shape shape = qlines::make_shape(g);
-        if (offsets) ddlerp_lines_forward<kHalfM, true, Out><<<shape.grid, shape.block, 0, s>>>(a, g);
-        else ddlerp_lines_forward<kHalfM, false, Out><<<shape.grid, shape.block, 0, s>>>(a, g);
+        if (offsets) launch_behind(ddlerp_lines_forward<kHalfM, true, Out>, shape.grid, shape.block, 0, s, a, g);
+        else launch_behind(ddlerp_lines_forward<kHalfM, false, Out>, shape.grid, shape.block, 0, s, a, g);
     } else {
         ddlerp_forward<kHalfM, Out><<<dim3((a.C / kVec + kThreads - 1) / kThreads, row_blocks(a.B, a.H, a.W)), kThreads, 0, s>>>(a);
     }
@@ -419,6 +423,6 @@ extern "C" int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (m_is_bf16) ddlerp_backward<true><<<grid, kThreads, 0, s>>>(a);
     else ddlerp_backward<false><<<grid, kThreads, 0, s>>>(a);
-    ddlerp_reduce<<<dim3((C + 31) / 32, n_out), dim3(32, 32), 0, s>>>(r);
+    launch_behind(ddlerp_reduce, dim3((C + 31) / 32, n_out), dim3(32, 32), 0, s, r);
     return record_launches(2);
 }

@@ -13,6 +13,7 @@
 // fixed order.  Pure bandwidth work: 4 (1 + n) bytes per element forward, 4 (n + 2) backward.
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "launch.h"
 #include "qshift_lines.cuh"
 #include "vrwkv_internal.h"
 
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(kThreads) qshift_mix_backward(const Args a) {
 // ---- a shift of one pixel: walks along the lines of the grid (qshift_lines.cuh) ----------------------
 template <typename Out>
 __global__ void __launch_bounds__(qlines::kMaxThreads) qshift_lines_forward(const Args a, const qlines::Grid g) {
+    wait_for_launch_before();
     using namespace qlines;
     const int cv = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (cv >= g.C) return;
@@ -194,6 +196,7 @@ __global__ void __launch_bounds__(qlines::kMaxThreads) qshift_lines_forward(cons
 }
 
 __global__ void __launch_bounds__(qlines::kMaxThreads, 2) qshift_lines_backward(const Args a, const qlines::Grid g) {
+    wait_for_launch_before();
     using namespace qlines;
     const int cv = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (cv >= g.C) return;
@@ -250,6 +253,7 @@ __global__ void __launch_bounds__(qlines::kMaxThreads, 2) qshift_lines_backward(
 __global__ void __launch_bounds__(1024) qshift_reduce(const float* __restrict__ partial, int blocks, int n_out, int C,
                                                       float* __restrict__ gmix0, float* __restrict__ gmix1,
                                                       float* __restrict__ gmix2) {
+    wait_for_launch_before();
     __shared__ float red[32][33];
     const int c = blockIdx.x * 32 + threadIdx.x, m = blockIdx.y;
     // kAhead rows asked for together and added up in order (1152 rows of 3 x 1024: 17.7 -> 7.8 us), fewer one by one
@@ -310,7 +314,7 @@ static void forward_as(const Args& a, cudaStream_t stream) {
     const int by = row_blocks(a);
     if (walks(a, g, false)) {
         const qlines::Shape s = qlines::make_shape(g);
-        qshift_lines_forward<Out><<<s.grid, s.block, 0, stream>>>(a, g);
+        launch_behind(qshift_lines_forward<Out>, s.grid, s.block, 0, stream, a, g);
     } else if (vector_ok(a, false)) {
         qshift_mix_forward<4, Out><<<dim3((a.C / 4 + kThreads - 1) / kThreads, by), kThreads, 0, stream>>>(a);
     } else {
@@ -330,14 +334,14 @@ int backward(const Args& a, float* const gmix[kMaxOut], cudaStream_t stream) {
     if (walks(a, g, true)) {
         const qlines::Shape s = qlines::make_shape(g);
         rows = static_cast<int>(s.walkers);
-        qshift_lines_backward<<<s.grid, s.block, 0, stream>>>(a, g);
+        launch_behind(qshift_lines_backward, s.grid, s.block, 0, stream, a, g);
     } else if (a.C % 4 == 0 && a.group % 4 == 0) {
         // the vector form of the general kernel only needs the group boundary rule (scalar loads inside)
         qshift_mix_backward<4><<<dim3((a.C / 4 + kThreads - 1) / kThreads, rows), kThreads, 0, stream>>>(a);
     } else {
         qshift_mix_backward<1><<<dim3((a.C + kThreads - 1) / kThreads, rows), kThreads, 0, stream>>>(a);
     }
-    qshift_reduce<<<dim3((a.C + 31) / 32, a.n_out), dim3(32, 32), 0, stream>>>(a.partial, rows, a.n_out, a.C, gmix[0],
+    launch_behind(qshift_reduce, dim3((a.C + 31) / 32, a.n_out), dim3(32, 32), 0, stream, a.partial, rows, a.n_out, a.C, gmix[0],
                                                                               gmix[1], gmix[2]);
     return 2;
 }

@@ -35,6 +35,7 @@
 #include <mutex>
 #include <set>
 #include <utility>
+#include "launch.h"
 #include "sm100_async.cuh"
 #include "tensor_map.h"
 #include "vrwkv_internal.h"
@@ -100,6 +101,7 @@ template <typename XT, typename ZT0, typename ZT1, int kX, bool kRows, int kPair
 __global__ void __launch_bounds__(128 * kPairs, kPairs == 1 ? 3 : 2)
 wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mx0,
                   const __grid_constant__ CUtensorMap mz0, const __grid_constant__ CUtensorMap mx1, const __grid_constant__ CUtensorMap mz1) {
+    wait_for_launch_before();
     typedef StateSmem<XT, ZT0, ZT1, kX, kPairs> S;
     constexpr int kWarps = 4 * kPairs, kTokens = kChunk / kWarps, kZ = 1;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -787,6 +789,7 @@ template <typename T, int kZ, int kX>
 __global__ void __launch_bounds__(256, 3)
 wkv6_forward_kernel(const OutArgs a, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mr,
                     const __grid_constant__ CUtensorMap mv) {
+    wait_for_launch_before();
     extern __shared__ __align__(1024) unsigned char smem[];
     __nv_bfloat16* kf = reinterpret_cast<__nv_bfloat16*>(smem);       // k towards the right edge of its block, left edge behind it
     __nv_bfloat16* pairs = kf + 2 * kX * kPlane;
@@ -1017,6 +1020,7 @@ __device__ __forceinline__ void slice_gradient(float (&out)[2][2][2][4], const _
 template <typename T, typename G, typename O, int kZ, int kX, int kP>
 __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mr,
                      const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mg) {
+    wait_for_launch_before();
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* const k_raw = smem;               // k and r stay, as bfloat16
     unsigned char* const r_raw = smem + kRawTile;
@@ -1287,6 +1291,7 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
 
 // gu[c] = sum over batch and chunks of the parts, in a fixed order
 __global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, const float* __restrict__ part, float* __restrict__ gu) {
+    wait_for_launch_before();
     __shared__ float red[32][33];
     const int c = blockIdx.x * 32 + threadIdx.x;
     float acc = 0.f;
@@ -1373,7 +1378,7 @@ static bool run_states(int B, int T_, int H, const void* r, const void* k, const
                       failure_mirror(kRows ? Op::wkv6_backward : Op::wkv6_forward)};
     const auto kernel = wkv6_state_kernel<T, T, G, kX, kRows, kPairs>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), S::bytes)) return false;
-    kernel<<<dim3(B * H, 2), 128 * kPairs, S::bytes, stream>>>(a, mw, mk, mv, mr, mg);
+    launch_behind(kernel, dim3(B * H, 2), 128 * kPairs, S::bytes, stream, a, mw, mk, mv, mr, mg);
     return true;
 }
 
@@ -1397,7 +1402,7 @@ static int run_forward(int B, int T_, int H, const void* r, const void* k, const
     if (!(map(&mw, w, false, false) && map(&mk, k, half, half) && map(&mr, r, half, half) && map(&mv, v, half, false))) return -1;
     const auto kernel = wkv6_forward_kernel<T, kZ, kX>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), forward_smem(kZ, kX))) return -1;
-    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, forward_smem(kZ, kX), stream>>>(o, mw, mk, mr, mv);
+    launch_behind(kernel, static_cast<unsigned>(B) * H * n_chunks, 256, forward_smem(kZ, kX), stream, o, mw, mk, mr, mv);
     return launched;
 }
 
@@ -1423,8 +1428,8 @@ static int run_backward(int B, int T_, int H, const void* r, const void* k, cons
         return -1;
     const auto kernel = wkv6_backward_kernel<T, G, O, kZ, kX, kP>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), backward_smem(kZ, kX))) return -1;
-    kernel<<<static_cast<unsigned>(B) * H * n_chunks, 256, backward_smem(kZ, kX), stream>>>(o, mw, mk, mr, mv, mg);
-    wkv6_bonus_kernel<<<C / 32, dim3(32, 32), 0, stream>>>(B * n_chunks, C, gu_part, gu);
+    launch_behind(kernel, static_cast<unsigned>(B) * H * n_chunks, 256, backward_smem(kZ, kX), stream, o, mw, mk, mr, mv, mg);
+    launch_behind(wkv6_bonus_kernel, C / 32, dim3(32, 32), 0, stream, B * n_chunks, C, gu_part, gu);
     return launched;
 }
 
