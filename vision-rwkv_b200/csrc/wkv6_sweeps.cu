@@ -182,17 +182,31 @@ __device__ __forceinline__ void sweep(const Args& a, Shared& sh, int b, int h, i
         __syncthreads();
         const int bt0 = (kForward ? bi : n_batches - 1 - bi) * kBatch;
         const int rows = min(kBatch, T - bt0);
-        // decay in place
-        for (int row = 0; row < rows; ++row) cur->vec[V_D][row][tid] = expf(-expf(cur->vec[V_D][row][tid]));
+        // decay in place (rows behind the last token hold anything and are not used)
+        float d_t[kBatch];
+#pragma unroll
+        for (int row = 0; row < kBatch; ++row) d_t[row] = cur->vec[V_D][row][tid];
+#pragma unroll
+        for (int row = 0; row < kBatch; ++row) cur->vec[V_D][row][tid] = expf(-expf(d_t[row]));
         if (kRightward) {       // per-token scalars of the bonus
             constexpr bool kVg = kWalk != WALK_Y, kRuk = kWalk == WALK_Y || kBoth;
             const int row = tid / kParts, part = tid % kParts;
             float s1 = 0.f, s2 = 0.f;
             if (row < rows) {
+                const auto at = [&](const float* x, float2 (&v)[4]) { lds8(x + 4 * part, x + 4 * part + 32, v); };
+                float2 x[4], z[4], uu[4];
+                if (kVg) {
+                    at(cur->vec[V_V][row], x);
+                    at(cur->vec[V_G][row], z);
 #pragma unroll
-                for (int n = part * kBatch; n < part * kBatch + kBatch; ++n) {
-                    if (kVg) s1 += cur->vec[V_V][row][n] * cur->vec[V_G][row][n];
-                    if (kRuk) s2 += cur->vec[V_R][row][n] * u_smem[n] * cur->vec[V_K][row][n];
+                    for (int n = 0; n < 8; ++n) s1 += part_of(x, n) * part_of(z, n);
+                }
+                if (kRuk) {
+                    at(cur->vec[V_R][row], x);
+                    at(cur->vec[V_K][row], z);
+                    at(u_smem, uu);
+#pragma unroll
+                    for (int n = 0; n < 8; ++n) s2 += part_of(x, n) * part_of(uu, n) * part_of(z, n);
                 }
             }
 #pragma unroll
@@ -307,7 +321,7 @@ template <bool kBackward, bool kSeg>
 __global__ void __launch_bounds__(N, kPerSm) wkv6_sweep_kernel(const Args a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
-    __shared__ float u_smem[N];
+    __shared__ __align__(16) float u_smem[N];
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, seg = kSeg ? blockIdx.z >> 1 : 0;
     const bool forward = (blockIdx.z & 1) != 0;      // in time
     const int tid = threadIdx.x;
