@@ -381,10 +381,10 @@ int vrwkv_wkv6_forward(int B, int T, int C, int H, const void* r, const void* k,
         return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < vrwkv_wkv6_forward_workspace_bytes(B, T, C, H, exact)) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
-    if (exact)
+    if (exact)      // clears the status word itself
         return finish(wkv6::forward(B, T, H, static_cast<const float*>(r), static_cast<const float*>(k), static_cast<const float*>(v), w_raw, u,
                                     y, workspace, s));
+    cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
     return finish(wkv6c::forward(B, T, H, r, k, v, w_raw, u, y, in_bf16 != 0, workspace, s));
 }
 
@@ -441,12 +441,12 @@ static int wkv6_backward(int B, int T, int C, int H, const void* r, const void* 
         if (reinterpret_cast<uintptr_t>(p) & (out_bf16 ? 1u : 3u)) return VRWKV_ERR_ALIGNMENT;
     if (workspace_bytes < (exact ? wkv6::backward_workspace(B, T, H) : wkv6c::backward_workspace(B, T, H))) return VRWKV_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
-    if (exact) {
+    if (exact) {      // clears the status word itself
         const auto in = [](const void* p) { return static_cast<const float*>(p); };
         const auto out = [](void* p) { return static_cast<float*>(p); };
         return finish(wkv6::backward(B, T, H, in(r), in(k), in(v), w_raw, u, in(gy), out(gr), out(gk), out(gv), gw, gu, workspace, s));
     }
+    cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
     return finish(wkv6c::backward(B, T, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, in_bf16, gy_bf16, out_bf16, workspace, s));
 }
 

@@ -40,6 +40,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
+#include "launch.h"
 #include "vrwkv_internal.h"
 
 namespace wkv6 {
@@ -322,6 +323,7 @@ __global__ void __launch_bounds__(N, kPerSm) wkv6_sweep_kernel(const Args a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
     __shared__ __align__(16) float u_smem[N];
+    wait_for_launch_before();
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, seg = kSeg ? blockIdx.z >> 1 : 0;
     const bool forward = (blockIdx.z & 1) != 0;      // in time
     const int tid = threadIdx.x;
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(N, kPerSm) wkv6_sweep_kernel(const Args a) {
 // behind every segment, S_j = decay_j S_{j-1} + own_j (wkv6_segment_scan_kernel), then the sweeps, each from the state
 // in front of its segment.  Decays are products of factors here too, so the accuracy is that of the whole walk.
 __global__ void __launch_bounds__(N, 9) wkv6_segment_state_kernel(const Args a) {
+    wait_for_launch_before();
     __shared__ __align__(16) float buf[2][3][kBatch][N];
     const int tid = threadIdx.x, bh = blockIdx.x, b = bh / a.H, h = bh % a.H;
     const int pair = blockIdx.z >> 1, dir = blockIdx.z & 1, step_i = blockIdx.y;
@@ -410,6 +413,7 @@ __global__ void __launch_bounds__(N, 9) wkv6_segment_state_kernel(const Args a) 
 
 // the slots of a (pair, direction, batch, head) in walking order: own state -> state behind the segment; a thread per element
 __global__ void __launch_bounds__(256) wkv6_segment_scan_kernel(const Args a) {
+    wait_for_launch_before();
     float* const slots = a.states + static_cast<size_t>(blockIdx.x) * (a.segs - 1) * kSlot;
     const int e = blockIdx.y * 256 + threadIdx.x, row = e % N;
     constexpr int kAhead = 4;
@@ -435,6 +439,7 @@ __global__ void __launch_bounds__(256) wkv6_segment_scan_kernel(const Args a) {
 // token (p>, q<) or first one (p<, q>).  A thread per (batch, segment, kPiece tokens, channel).
 constexpr int kPiece = 32;
 __global__ void __launch_bounds__(256) wkv6_segment_decay_grad_kernel(const Args a, float* __restrict__ gw) {
+    wait_for_launch_before();
     const int C = a.H * N, pieces = (a.seg_len + kPiece - 1) / kPiece;
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= static_cast<size_t>(a.B) * a.segs * pieces * C) return;
@@ -465,6 +470,7 @@ __global__ void __launch_bounds__(256) wkv6_segment_decay_grad_kernel(const Args
 __global__ void __launch_bounds__(256) wkv6_decay_grad_kernel(int T, int C, unsigned per_seq, bool scalar, const float* __restrict__ w_raw, const float* __restrict__ cp,
                                                               const float* __restrict__ cq, const float* __restrict__ cp2,
                                                               const float* __restrict__ cq2, float* __restrict__ gw) {
+    wait_for_launch_before();
     const unsigned per_row = static_cast<unsigned>(C) / 4, b = blockIdx.x / per_seq, v = (blockIdx.x - b * per_seq) * 256u + threadIdx.x;
     if (v >= per_row * static_cast<unsigned>(T)) return;
     const size_t seq = static_cast<size_t>(b) * T * C, i = seq + static_cast<size_t>(v) * 4;
@@ -493,12 +499,45 @@ __global__ void __launch_bounds__(256) wkv6_decay_grad_kernel(int T, int C, unsi
 
 // gu[c] = sum over batch (and segments) of gu_part, fixed order
 __global__ void wkv6_bonus_grad_kernel(int B, int C, const float* __restrict__ part, float* __restrict__ gu) {
+    wait_for_launch_before();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     float acc = 0.f;
 #pragma unroll 8
     for (int b = 0; b < B; ++b) acc += part[static_cast<size_t>(b) * C + c];
     gu[c] = acc;
+}
+
+// The status word (which these kernels never set) and the results that two directions add into, in one launch: three results of 19 MB took
+// 15 us as memsets, which the launch behind them also has to wait for in full.
+struct Cleared {
+    float* p[3];           // of n floats each, null: none
+    unsigned* status;      // may be null
+    size_t n;
+};
+constexpr int kClearVecs = 8;      // 16-byte stores of a thread
+__global__ void __launch_bounds__(256) wkv6_clear_kernel(const Cleared z) {
+    wait_for_launch_before();
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && z.status != nullptr) *z.status = 0u;
+    float* const p = z.p[blockIdx.y];
+    if (p == nullptr) return;
+    const bool wide = (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
+    const size_t first = static_cast<size_t>(blockIdx.x) * 256 * kClearVecs + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < kClearVecs; ++i) {
+        const size_t at = (first + static_cast<size_t>(i) * 256) * 4;      // n is a multiple of 64
+        if (at >= z.n) return;
+        if (wide) {
+            *reinterpret_cast<float4*>(p + at) = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) p[at + e] = 0.f;
+        }
+    }
+}
+static void clear(const Cleared& z, cudaStream_t stream) {
+    const size_t per_block = static_cast<size_t>(256) * kClearVecs * 4;
+    launch_behind(wkv6_clear_kernel, dim3(static_cast<unsigned>((z.n + per_block - 1) / per_block), z.p[1] == nullptr ? 1 : 3), 256, 0, stream, z);
 }
 
 struct Plan {
@@ -522,8 +561,8 @@ static size_t state_floats(int B, int H, const Plan& pl, int pairs) {
     return static_cast<size_t>(pairs) * 2 * B * H * (pl.segs - 1) * kSlot;
 }
 static void run_segment_states(const Args& a, int pairs, cudaStream_t stream) {
-    wkv6_segment_state_kernel<<<dim3(a.B * a.H, a.segs - 1, 2 * pairs), N, 0, stream>>>(a);
-    wkv6_segment_scan_kernel<<<dim3(2 * pairs * a.B * a.H, N * N / 256), 256, 0, stream>>>(a);
+    launch_behind(wkv6_segment_state_kernel, dim3(a.B * a.H, a.segs - 1, 2 * pairs), N, 0, stream, a);
+    launch_behind(wkv6_segment_scan_kernel, dim3(2 * pairs * a.B * a.H, N * N / 256), 256, 0, stream, a);
 }
 
 // status word (which this path never sets), states of segments, running sums, parts of gu
@@ -546,11 +585,11 @@ int forward(int B, int T, int H, const float* r, const float* k, const float* v,
     a.out[KIND_Y] = y;
     a.segs = pl.segs; a.seg_len = pl.len;
     a.states = pl.segs > 1 ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kHead) : nullptr;
-    cudaMemsetAsync(y, 0, static_cast<size_t>(B) * T * H * N * sizeof(float), stream);
+    clear(Cleared{{y, nullptr, nullptr}, static_cast<unsigned*>(workspace), static_cast<size_t>(B) * T * H * N}, stream);
     if (pl.segs > 1) run_segment_states(a, 1, stream);
     const auto kernel = pl.segs > 1 ? wkv6_sweep_kernel<false, true> : wkv6_sweep_kernel<false, false>;
-    kernel<<<dim3(B * H, 1, 2 * pl.segs), N, sizeof(Shared), stream>>>(a);
-    return pl.segs > 1 ? 3 : 1;
+    launch_behind(kernel, dim3(B * H, 1, 2 * pl.segs), N, sizeof(Shared), stream, a);
+    return pl.segs > 1 ? 4 : 2;
 }
 
 int backward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
@@ -570,22 +609,20 @@ int backward(int B, int T, int H, const float* r, const float* k, const float* v
     ws += state_floats(B, H, pl, 2);
     for (int i = 0; i < 4; ++i) a.cum[i] = ws + i * E;
     a.gu_part = ws + 4 * E;
-    cudaMemsetAsync(gr, 0, E * sizeof(float), stream);
-    cudaMemsetAsync(gk, 0, E * sizeof(float), stream);
-    if (gv) cudaMemsetAsync(gv, 0, E * sizeof(float), stream);      // (gv == nullptr: the caller gets gv elsewhere)
+    clear(Cleared{{gr, gk, gv}, static_cast<unsigned*>(workspace), E}, stream);      // (gv == nullptr: the caller gets gv elsewhere)
     if (pl.segs > 1) run_segment_states(a, 2, stream);
     const auto kernel = pl.segs > 1 ? wkv6_sweep_kernel<true, true> : wkv6_sweep_kernel<true, false>;
-    kernel<<<dim3(B * H, 2, 2 * pl.segs), N, sizeof(Shared), stream>>>(a);
+    launch_behind(kernel, dim3(B * H, 2, 2 * pl.segs), N, sizeof(Shared), stream, a);
     if (pl.segs > 1) {
         const size_t threads = static_cast<size_t>(B) * pl.segs * ((pl.len + kPiece - 1) / kPiece) * C;
-        wkv6_segment_decay_grad_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(a, gw);
+        launch_behind(wkv6_segment_decay_grad_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, stream, a, gw);
     } else {
         const unsigned per_seq = static_cast<unsigned>((static_cast<size_t>(T) * C / 4 + 255) / 256);
-        wkv6_decay_grad_kernel<<<per_seq * static_cast<unsigned>(B), 256, 0, stream>>>(T, C, per_seq, (reinterpret_cast<uintptr_t>(gw) & 15u) != 0, w_raw, a.cum[0],
-                                                                                     a.cum[1], a.cum[2], a.cum[3], gw);
+        launch_behind(wkv6_decay_grad_kernel, per_seq * static_cast<unsigned>(B), 256, 0, stream, T, C, per_seq, (reinterpret_cast<uintptr_t>(gw) & 15u) != 0, w_raw,
+                      a.cum[0], a.cum[1], a.cum[2], a.cum[3], gw);
     }
-    wkv6_bonus_grad_kernel<<<(C + 127) / 128, 128, 0, stream>>>(B * pl.segs, C, a.gu_part, gu);
-    return pl.segs > 1 ? 5 : 3;
+    launch_behind(wkv6_bonus_grad_kernel, (C + 127) / 128, 128, 0, stream, B * pl.segs, C, a.gu_part, gu);
+    return pl.segs > 1 ? 6 : 4;
 }
 
 }  // namespace wkv6
