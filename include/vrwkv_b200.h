@@ -351,6 +351,7 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
  *   vrwkv_add_rows: out[i] = table[i mod period] + a[i], a bfloat16, float32 result; period a multiple of 8 that divides n
  *     (CLS/vrwkv.py:392, CLS/vrwkv6.py:200)
  *   vrwkv_widen: out = a as float32; n a multiple of 8
+ *   vrwkv_narrow: out_i = src_i rounded to bfloat16, n_i values each, i < count <= 16, in one launch
  *   vrwkv_patch_rows: img (B, channels, H, W) to (B, H / patch, W / patch, channels, patch, patch) in bfloat16, whole patches only;
  *     patch % 8 == 0, W % 4 == 0 (the operand of the patch embedding, CLS/vrwkv.py:357)
  * Sigmoid, its product and y are rounded to bfloat16 where r is.  All tensors 16-byte aligned. */
@@ -363,6 +364,7 @@ int vrwkv_linear_relu_square(long long rows, int K, int N, const uint16_t* x, co
 int vrwkv_linear_batch_pays(int count, long long rows, int K, int N);
 int vrwkv_linear_batch(int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream);
 int vrwkv_add_rows(long long n, long long period, const float* table, const uint16_t* a, float* out, void* stream);
+int vrwkv_narrow(int count, const float* const* src, const long long* n, uint16_t* const* out, void* stream);
 int vrwkv_widen(long long n, const uint16_t* a, float* out, void* stream);
 int vrwkv_patch_rows(int B, int channels, int H, int W, int patch, const float* img, uint16_t* out, void* stream);
 int vrwkv_layer_norm(int rows, int C, float eps, const float* x, const float* weight, const float* bias, float* out, void* stream);

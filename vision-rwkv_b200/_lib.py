@@ -41,6 +41,7 @@ SIGNATURES = {
     "vrwkv_linear_batch_pays": (_c_int, [_c_int, ctypes.c_longlong] + [_c_int] * 2),
     "vrwkv_linear_batch": (_c_int, [_c_int, ctypes.c_longlong] + [_c_int] * 2 + [_ptr] * 4),
     "vrwkv_relu_square_f32out": (_c_int, [ctypes.c_longlong] + [_ptr] * 3),
+    "vrwkv_narrow": (_c_int, [_c_int] + [_ptr] * 4),
     "vrwkv_widen": (_c_int, [ctypes.c_longlong] + [_ptr] * 3),
     "vrwkv_add_rows": (_c_int, [ctypes.c_longlong] * 2 + [_ptr] * 4),
     "vrwkv_patch_rows": (_c_int, [_c_int] * 5 + [_ptr] * 3),

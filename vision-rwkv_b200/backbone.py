@@ -50,23 +50,25 @@ class SpatialMix(nn.Module):
 
     def forward(self, x, resolution):
         T = x.shape[1]
+        key, value, receptance, output = self.key, self.value, self.receptance, self.output
+        weights = epilogue.weights_for(self, x, key, value, receptance, output)
         if self.shift_pixel > 0:
-            xk, xv, xr = qshift_mix_to((self.key, self.value, self.receptance), x,
+            xk, xv, xr = qshift_mix_to((key, value, receptance), x,
                                        (self.spatial_mix_k, self.spatial_mix_v, self.spatial_mix_r),
                                        resolution, self.shift_pixel, self.channel_gamma)
         else:
             xk = xv = xr = x
-        k, v, r = epilogue.linears((self.key, self.value, self.receptance), (xk, xv, xr))
+        k, v, r = epilogue.linears((key, value, receptance), (xk, xv, xr), weights and weights[:3])
         # the plain gate rounds y to the dtype of r; a norm in between takes it as it is
         run = inference_biwkv if self.key_norm is None and r.dtype == torch.bfloat16 else RUN_CUDA
         y = run(self.spatial_decay / T, self.spatial_first / T, k, v)
         if self.key_norm is not None and y.is_cuda and normgate.supported(y.shape[-1], y.shape[-1]):
             # LayerNorm, sigmoid and gate in one pass over y (normgate.py)
-            return self.output(normgate.norm_gate(y, r, self.key_norm.weight, self.key_norm.bias, y.shape[-1],
-                                                  self.key_norm.eps, act="sigmoid"))
+            gated = normgate.norm_gate(y, r, self.key_norm.weight, self.key_norm.bias, y.shape[-1], self.key_norm.eps, act="sigmoid")
+            return epilogue.linear(output, gated, weights and weights[3])
         if self.key_norm is not None:
             y = self.key_norm(y)
-        return self.output(epilogue.sigmoid_gate(r, y))
+        return epilogue.linear(output, epilogue.sigmoid_gate(r, y), weights and weights[3])
 
 
 @taken_over
@@ -86,15 +88,17 @@ class ChannelMix(nn.Module):
 
     def gate_operands(self, x, resolution):
         """(r, y) of the gate sigmoid(r) * y that ends the mix"""
+        key, receptance, value = self.key, self.receptance, self.value
+        wk, wr, wv = epilogue.weights_for(self, x, key, receptance, value) or (None, None, None)
         if self.shift_pixel > 0:
-            xk, xr = qshift_mix_to((self.key, self.receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution,
+            xk, xr = qshift_mix_to((key, receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution,
                                    self.shift_pixel, self.channel_gamma)
         else:
             xk = xr = x
-        k = epilogue.linear_relu_square(self.key, xk, self.value if self.key_norm is None else None)
+        k = epilogue.linear_relu_square(key, xk, value if self.key_norm is None else None, wk)
         if self.key_norm is not None:
             k = self.key_norm(k)
-        return self.receptance(xr), self.value(k)
+        return epilogue.linear(receptance, xr, wr), epilogue.linear(value, k, wv)
 
     def forward(self, x, resolution):
         return epilogue.sigmoid_gate(*self.gate_operands(x, resolution))

@@ -74,17 +74,21 @@ class SpatialMixV6(nn.Module):
 
     def forward(self, x, resolution):
         B, T, C = x.shape
+        receptance, key, value, gate, output = self.receptance, self.key, self.value, self.gate, self.output
+        matrices = (self.time_maa_w1, self.time_maa_w2, self.time_decay_w1, self.time_decay_w2)
+        weights = epilogue.weights_for(self, x, receptance, key, value, gate, output, *matrices)
+        maa_w1, maa_w2, decay_w1, decay_w2 = matrices if weights is None else weights[5:]
         fused = x.is_cuda and C % HEAD_SIZE == 0 and self.shift_pixel > 0
         if fused:
             # the shift and every interpolation in two passes over x (qshift.qshift_ddlerp)
-            layers = (self.key, self.value, self.receptance, self.gate)
+            layers = (key, value, receptance, gate)
             (xxx,) = qshift_ddlerp_to(layers, x, [self.time_maa_x], [None], resolution, self.shift_pixel, HEAD_SIZE)
         else:
             xx = q_shift_multihead(x, self.shift_pixel, resolution) - x
             xxx = x + xx * self.time_maa_x
         # five data-dependent mixing offsets from one low-rank branch
-        low = torch.tanh(xxx @ self.time_maa_w1).view(B * T, 5, MIX_RANK).transpose(0, 1)
-        mw, mk, mv, mr, mg = torch.bmm(low, self.time_maa_w2).view(5, B, T, C).unbind(0)
+        low = torch.tanh(xxx @ maa_w1).view(B * T, 5, MIX_RANK).transpose(0, 1)
+        mw, mk, mv, mr, mg = torch.bmm(low, maa_w2).view(5, B, T, C).unbind(0)
         if fused:
             xw, xk, xv, xr, xg = qshift_ddlerp_to(
                 layers, x, [self.time_maa_w, self.time_maa_k, self.time_maa_v, self.time_maa_r, self.time_maa_g],
@@ -92,18 +96,19 @@ class SpatialMixV6(nn.Module):
         else:
             xw, xk, xv, xr, xg = (x + xx * (maa + m) for maa, m in (
                 (self.time_maa_w, mw), (self.time_maa_k, mk), (self.time_maa_v, mv), (self.time_maa_r, mr), (self.time_maa_g, mg)))
-        r, k, v, g_raw = epilogue.linears((self.receptance, self.key, self.value, self.gate), (xr, xk, xv, xg))
-        w = epilogue.add_rows(self.time_decay, torch.tanh(xw @ self.time_decay_w1) @ self.time_decay_w2)
+        r, k, v, g_raw = epilogue.linears((receptance, key, value, gate), (xr, xk, xv, xg),
+                                         weights and weights[:4])
+        w = epilogue.add_rows(self.time_decay, torch.tanh(xw @ decay_w1) @ decay_w2)
         y = inference_rwkv6(B, T, C, self.n_head, r.contiguous(), k.contiguous(), v.contiguous(),
                             w.float().contiguous(), self.time_faaaa)
         if self.key_norm is not None:
             y = self.key_norm(y)
         if y.is_cuda and normgate.supported(C, HEAD_SIZE):
             # per-head GroupNorm, SiLU and gate in one pass over y (normgate.py)
-            return self.output(epilogue.head_norm_gate(y, g_raw, self.ln_x, HEAD_SIZE, self.output, "silu"))
+            return epilogue.linear(output, epilogue.head_norm_gate(y, g_raw, self.ln_x, HEAD_SIZE, output, "silu"), weights and weights[4])
         g = F.silu(g_raw)
         y = self.ln_x(y.reshape(B * T, C)).view(B, T, C)
-        return self.output(y.to(g.dtype) * g)
+        return epilogue.linear(output, y.to(g.dtype) * g, weights and weights[4])
 
 
 @taken_over
@@ -122,12 +127,14 @@ class ChannelMixV6(nn.Module):
 
     def gate_operands(self, x, resolution):
         """(r, y) of the gate sigmoid(r) * y that ends the mix"""
-        xk, xr = qshift_mix_to((self.key, self.receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution, self.shift_pixel,
+        key, receptance, value = self.key, self.receptance, self.value
+        wk, wr, wv = epilogue.weights_for(self, x, key, receptance, value) or (None, None, None)
+        xk, xr = qshift_mix_to((key, receptance), x, (self.spatial_mix_k, self.spatial_mix_r), resolution, self.shift_pixel,
                                head_dim=HEAD_SIZE)       # per-head shift + both interpolations in one pass
-        k = epilogue.linear_relu_square(self.key, xk, self.value if self.key_norm is None else None)
+        k = epilogue.linear_relu_square(key, xk, value if self.key_norm is None else None, wk)
         if self.key_norm is not None:
             k = self.key_norm(k)
-        return self.receptance(xr), self.value(k)
+        return epilogue.linear(receptance, xr, wr), epilogue.linear(value, k, wv)
 
     def forward(self, x, resolution):
         return epilogue.sigmoid_gate(*self.gate_operands(x, resolution))

@@ -106,6 +106,29 @@ Tensor key_layer(const Tensor& x, const Tensor& weight) {
     return relu_square(at::linear(x, weight), false);
 }
 
+Tensor autocast_copy(const Tensor& t) { return at::autocast::cached_cast(at::kBFloat16, t, at::kCUDA); }
+
+std::vector<Tensor> narrow(std::vector<Tensor> weights) {
+    TORCH_CHECK(!weights.empty() && weights.size() <= 16, "one to sixteen weights");
+    const c10::cuda::CUDAGuard guard(weights[0].device());
+    const float* src[16];
+    uint16_t* out[16];
+    long long n[16];
+    std::vector<Tensor> outs;
+    for (const Tensor& w : weights)
+        if (has_tangent(w)) return {};
+    for (size_t i = 0; i < weights.size(); ++i) {
+        same_place(weights[i], weights[0], "a weight");
+        TORCH_CHECK(weights[i].scalar_type() == at::kFloat && weights[i].is_contiguous() && weights[i].numel() > 0, "weights must be float32 and contiguous");
+        outs.push_back(at::empty(weights[i].sizes(), weights[i].options().dtype(at::kBFloat16)));
+        src[i] = fp(weights[i]);
+        out[i] = static_cast<uint16_t*>(outs[i].data_ptr());
+        n[i] = weights[i].numel();
+    }
+    check(vrwkv_narrow(weights.size(), src, n, out, stream_of(weights[0])), "vrwkv_narrow");
+    return outs;
+}
+
 Tensor add_rows(const Tensor& table_, const Tensor& a_) {
     same_place(table_, a_, "table");
     TORCH_CHECK(is_bf16(a_) && table_.scalar_type() == at::kFloat, "a must be bfloat16 and the table float32");

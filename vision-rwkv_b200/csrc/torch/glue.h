@@ -21,6 +21,10 @@ Tensor linear_relu_square(const Tensor& x, const Tensor& weight);
 Tensor key_layer(const Tensor& x, const Tensor& weight);
 // up to four linear layers of one shape without a bias on bfloat16 rows, as autocast computes them, in one launch where that is faster
 std::vector<Tensor> linear_batch(std::vector<Tensor> xs, std::vector<Tensor> weights);
+// what autocast makes of t for a bfloat16 product, from its cache where it has it
+Tensor autocast_copy(const Tensor& t);
+// bfloat16 copies of float32 weights in one launch; empty where forward-mode differentiation wants the casts themselves
+std::vector<Tensor> narrow(std::vector<Tensor> weights);
 Tensor add_rows(const Tensor& table, const Tensor& a);
 Tensor patch_rows(const Tensor& img, int64_t patch);
 Tensor widen(const Tensor& a);

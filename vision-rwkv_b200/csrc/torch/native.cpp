@@ -390,6 +390,8 @@ PYBIND11_MODULE(_native, m) {
     m.def("relu_square", [](const Tensor& x, bool wide) { return vrwkv::guarded([&] { return vrwkv::relu_square(x, wide); })(); });
     m.def("linear_relu_square", [](const Tensor& x, const Tensor& weight) { return vrwkv::guarded([&] { return vrwkv::linear_relu_square(x, weight); })(); });
     m.def("key_layer", [](const Tensor& x, const Tensor& weight) { return vrwkv::guarded([&] { return vrwkv::key_layer(x, weight); })(); });
+    m.def("autocast_copy", [](const Tensor& t) { return vrwkv::guarded([&] { return vrwkv::autocast_copy(t); })(); });
+    m.def("narrow", [](std::vector<Tensor> weights) { return vrwkv::guarded([&] { return vrwkv::narrow(weights); })(); });
     m.def("linear_batch", [](std::vector<Tensor> xs, std::vector<Tensor> weights) { return vrwkv::guarded([&] { return vrwkv::linear_batch(xs, weights); })(); });
     m.def("add_rows", [](const Tensor& table, const Tensor& a) { return vrwkv::guarded([&] { return vrwkv::add_rows(table, a); })(); });
     m.def("patch_rows", [](const Tensor& img, int64_t patch) { return vrwkv::guarded([&] { return vrwkv::patch_rows(img, patch); })(); });

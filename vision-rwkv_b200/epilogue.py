@@ -15,6 +15,7 @@ from . import _lib, normgate, ops, traced
 from .qshift import autocast_linears, feeds_autocast_linears, stock
 
 KERNEL_DTYPES = (torch.float32, torch.bfloat16)
+DEEPEST_BATCH = 384             # of vrwkv_linear_batch_pays: deeper layers are not worth the questions
 MOST_NORM_CHANNELS = 1024       # a row of norm_residual lives in one warp's registers
 
 
@@ -37,6 +38,52 @@ def _unwatched(x, *parameters):
     return True
 
 
+_NOTHING = {}       # by device: an empty parameter.  Autocast keeps its copy of it, which takes no launch, as long as its copies of others.
+
+
+def _left_to_autocast(owner, device):
+    """Whether `owner` has been called before while autocast keeps what it casts (it forgets that when its outermost context ends, or at once
+    where it is not to keep anything).  The calls are counted on autocast's own copy of an empty parameter, so the count goes where the
+    copies go.  A captured call leaves no copies behind that an eager one could use: it counts for nothing, and takes autocast's only where
+    an earlier call has made them."""
+    nothing = _NOTHING.get(device)
+    if nothing is None:
+        with torch.inference_mode(False):
+            nothing = _NOTHING[device] = nn.Parameter(torch.empty(0, device=device))
+    calls = _lib.native().autocast_copy(nothing).__dict__
+    before = calls.get(key := str(id(owner)), 0)        # (another owner at the same address has its weights cast one by one, no more)
+    if before > 1:
+        return True
+    if torch.cuda.is_current_stream_capturing():
+        return False
+    calls[key] = before + 1
+    return before > 0
+
+
+def weights_for(owner, x, *sources):
+    """The weights of `sources` (linear layers, matrices) as bfloat16 autocast makes them for the products of one call of `owner` on x, cast
+    in one launch instead of one each; None where each is left to its own product.  That is wherever somebody would see the cast or
+    the layer's call, and from the second call of `owner` on in an autocast context that is held: autocast keeps what it casts by itself, and
+    after that second call has no more to cast."""
+    if not x.is_cuda or torch.is_grad_enabled() or not torch.is_autocast_enabled("cuda") or traced.tracing():
+        return None
+    if _left_to_autocast(owner, x.device) and (type(sources[0]) is not nn.Linear or sources[0].weight.requires_grad):
+        return None                                  # (autocast keeps no others)
+    layers = [s for s in sources if isinstance(s, nn.Module)]
+    if x.dtype not in KERNEL_DTYPES or not autocast_linears(*layers) or not _unwatched(x) or any(layer.bias is not None for layer in layers):
+        return None
+    weights = [s.weight if isinstance(s, nn.Module) else s for s in sources]
+    for w in weights:
+        if type(w) is not nn.Parameter or w.dtype != torch.float32 or w.device != x.device or not w.is_contiguous() or w.numel() == 0:
+            return None
+    return _lib.native().narrow(weights) or None
+
+
+def linear(layer, x, weight=None):
+    """layer(x), with the layer's weight as `weights_for` gave it"""
+    return layer(x) if weight is None else nn.functional.linear(x, weight)
+
+
 def relu_square(x, layer=None):
     """relu(x)^2 (classification/mmcls_custom/models/backbones/vrwkv.py:251).  Under autocast torch squares bfloat16 x in float32;
     the result leaves in bfloat16 only for a linear layer `layer` that rounds it to that first anyway."""
@@ -46,34 +93,34 @@ def relu_square(x, layer=None):
     return _lib.native().relu_square(x, wide)
 
 
-def linear_relu_square(key, x, layer=None):
-    """relu_square(key(x), layer), the linear layer and what follows it in one call where `layer` rounds the result to bfloat16 anyway (in
+def linear_relu_square(key, x, layer=None, weight=None):
+    """relu_square(linear(key, x, weight), layer), the linear layer and what follows it in one call where `layer` rounds the result to bfloat16 anyway (in
     one kernel where that is faster: vrwkv_linear_relu_square_pays)."""
     if layer is not None and x.dtype == torch.bfloat16 and _inference(x) and autocast_linears(key, layer) and key.bias is None:
-        w = key.weight
+        w = key.weight if weight is None else weight
         if (_unwatched(x, w) and w.dtype in KERNEL_DTYPES and w.device == x.device and w.dim() == 2 and w.shape[1] == x.shape[-1]
                 and w.shape[1] % 64 == 0 and w.shape[1] > 0 and w.shape[0] % 256 == 0 and w.shape[0] > 0):
             out = _lib.native().key_layer(x, w)
             if ops.CHECK_STATUS:
                 ops.raise_if_failed(x.device)
             return out
-    return relu_square(key(x), layer)
+    return relu_square(linear(key, x, weight), layer)
 
 
-def linears(layers, xs):
-    """[layer(x) for layer, x in zip(layers, xs)] of up to four layers, in one launch where they are of one shape and that is faster
+def linears(layers, xs, weights=None):
+    """[linear(layer, x, weight) for ...] of up to four layers, in one launch where they are of one shape and that is faster
     (vrwkv_linear_batch_pays)."""
     x, w = xs[0], layers[0].weight if type(layers[0]) is nn.Linear else None
-    if (w is not None and len(layers) <= 4 and x.dtype == torch.bfloat16 and _inference(*xs) and autocast_linears(*layers)
+    if (w is not None and len(layers) <= 4 and x.shape[-1] <= DEEPEST_BATCH and x.dtype == torch.bfloat16 and _inference(*xs) and autocast_linears(*layers)
             and all(layer.bias is None and _unwatched(t, layer.weight) and t.dtype == x.dtype and t.shape == x.shape and t.device == x.device
                     and layer.weight.dtype in KERNEL_DTYPES and layer.weight.shape == w.shape and layer.weight.device == x.device
                     for layer, t in zip(layers, xs))
             and w.dim() == 2 and w.shape[1] == x.shape[-1]):
-        outs = _lib.native().linear_batch(list(xs), [layer.weight for layer in layers])
+        outs = _lib.native().linear_batch(list(xs), weights or [layer.weight for layer in layers])
         if ops.CHECK_STATUS:
             ops.raise_if_failed(x.device)
         return outs
-    return [layer(t) for layer, t in zip(layers, xs)]
+    return [linear(layer, t, weight) for layer, t, weight in zip(layers, xs, weights or [None] * len(layers))]
 
 
 def sigmoid_gate(r, y, norm=None):
