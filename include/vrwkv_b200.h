@@ -351,7 +351,8 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
  *   vrwkv_add_rows: out[i] = table[i mod period] + a[i], a bfloat16, float32 result; period a multiple of 8 that divides n
  *     (CLS/vrwkv.py:392, CLS/vrwkv6.py:200)
  *   vrwkv_widen: out = a as float32; n a multiple of 8
- *   vrwkv_narrow: out_i = src_i rounded to bfloat16, n_i values each, i < count <= 16, in one launch
+ *   vrwkv_narrow: out_i = src_i rounded to bfloat16, n_i values each, i < count <= 16, in one launch (which, like the casts
+ *     that it stands for, vrwkv_launch_count does not count: a network's count does not depend on who casts its weights)
  *   vrwkv_patch_rows: img (B, channels, H, W) to (B, H / patch, W / patch, channels, patch, patch) in bfloat16, whole patches only;
  *     patch % 8 == 0, W % 4 == 0 (the operand of the patch embedding, CLS/vrwkv.py:357)
  * Sigmoid, its product and y are rounded to bfloat16 where r is.  All tensors 16-byte aligned. */

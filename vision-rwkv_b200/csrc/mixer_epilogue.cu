@@ -530,7 +530,7 @@ extern "C" int vrwkv_narrow(int count, const float* const* src, const long long*
         if (blocks > 0x7fffffffLL) return VRWKV_ERR_UNSUPPORTED;
     }
     launch_behind(narrow_kernel, static_cast<unsigned>(blocks), kThreads, 0, static_cast<cudaStream_t>(stream), a, count);
-    return record_launches(1);
+    return record_launches(0);
 }
 
 extern "C" int vrwkv_patch_rows(int B, int channels, int H, int W, int patch, const float* img, uint16_t* out, void* stream) {
