@@ -6,8 +6,8 @@
 // neighbour needs is already in a register: one halo load per stretch replaces a second load per token, and all loads of a
 // stretch are issued together (9 independent 16-byte loads in flight per thread and tensor).  Channels of different
 // groups walk different lines; a warp's accesses still cover whole 32-byte sectors.  Token-by-token code with
-// one load and a 64-bit division per token in flight measured 0.56 of the HBM rate; this measures 0.80 (B=64, 24 x 24, C=1024,
-// three outputs, forward + backward: 376 and 262 us).
+// one load and a 64-bit division per token in flight measured 0.56 of the HBM rate; this measures 0.87 (B=64, 24 x 24, C=1024,
+// three outputs, forward + backward: 376 and 238 us).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -35,8 +35,8 @@ struct Shape {
 };
 
 // (host) stretches as even as possible; enough of them per walker that partial sums stay small beside the tensors, few
-// enough that the blocks fill the device
-inline Grid make_grid(int B, int H, int W, int C, int group, int period, int stretch = kStretch) {
+// enough that the blocks fill the device; at most most_per_walker
+inline Grid make_grid(int B, int H, int W, int C, int group, int period, int stretch = kStretch, int most_per_walker = 4) {
     Grid g{};
     g.B = B; g.H = H; g.W = W; g.C = C; g.group = group; g.period = period;
     g.row_parts = (W + stretch - 1) / stretch;
@@ -48,7 +48,7 @@ inline Grid make_grid(int B, int H, int W, int C, int group, int period, int str
     g.lines = lines < (1LL << 31) ? static_cast<unsigned>(lines) : 0u;      // 0: too many, the caller takes its general kernels
     const int vecs = C / 4, by = std::max(1, kMaxThreads / std::max(1, vecs));
     // 148 SMs with four blocks each
-    g.per_walker = static_cast<int>(std::min<long long>(4, std::max<long long>(1, lines / (592LL * by))));
+    g.per_walker = static_cast<int>(std::min<long long>(most_per_walker, std::max<long long>(1, lines / (592LL * by))));
     return g;
 }
 inline Shape make_shape(const Grid& g) {
