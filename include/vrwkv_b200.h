@@ -341,8 +341,8 @@ int vrwkv_qshift_ddlerp_backward_f32(int B, int H, int W, int C, int head_dim, i
  *     (CLS/vrwkv.py:250-251); K % 64 == 0, N % 256 == 0, else VRWKV_ERR_UNSUPPORTED; _pays: 1 where it takes less of the current
  *     device's time than a library's product and vrwkv_relu_square
  *   vrwkv_linear_batch: out_i (rows, N) = x_i W_i^T rounded to bfloat16, i < count <= 4, in one launch (the layers behind a token shift,
- *     CLS/vrwkv.py:166-168, vrwkv6.py:194-197); K % 64 == 0, K <= 384, N % 192 == 0, else VRWKV_ERR_UNSUPPORTED; _pays: 1 where it takes
- *     less of the current device's time than a library's products
+ *     CLS/vrwkv.py:166-168, vrwkv6.py:194-197); K % 64 == 0 and K <= 384, N % 192 == 0, N <= 1536 or K <= 1024, N % 256 == 0, else
+ *     VRWKV_ERR_UNSUPPORTED; _pays: 1 where it takes less of the current device's time than a library's products
  *   vrwkv_norm_residual: out = x + gamma * (normalise(a) * weight + bias) over rows of C <= 1024 channels, C % 4 == 0;
  *     weight and bias NULL: out = x + gamma * a; gamma NULL: 1 (CLS/vrwkv.py:297-318)
  *   vrwkv_layer_norm: out = normalise(x) * weight + bias over such rows

@@ -9,7 +9,9 @@ pytestmark = pytest.mark.gpu
 
 # rows around a tile's 128, fewer and more tiles than CTAs to a slab; depths of one slice, of both kinds of stages, of the most; one to eight slabs
 @pytest.mark.parametrize("count,rows,K,N", [(3, 1, 64, 192), (4, 127, 192, 192), (3, 128, 256, 384), (4, 129, 320, 192), (3, 19008, 384, 384), (4, 6272, 384, 384),
-                                            (3, 40001, 192, 192), (3, 777, 384, 1536), (4, 300, 128, 960)])
+                                            (3, 40001, 192, 192), (3, 777, 384, 1536), (4, 300, 128, 960),
+                                            # by tiles of 128 x 256: deeper, or columns that are no slabs
+                                            (3, 1, 448, 256), (4, 129, 768, 768), (3, 12544, 768, 768), (4, 128, 1024, 512), (3, 300, 64, 256)])
 def test_against_float64(cuda_device, count, rows, K, N):
     from vision_rwkv_b200 import _lib
     lib = _lib.load()
@@ -70,13 +72,14 @@ def test_not_a_number_stays(cuda_device):
             assert out[129].isnan().all() and out[5].isinf().all() and (out[6] == 64).all()
 
 
-def test_bounded_waits_run_out_and_report(cuda_device):
+@pytest.mark.parametrize("K,N", [(384, 192), (512, 256)])
+def test_bounded_waits_run_out_and_report(cuda_device, K, N):
     """Path 3: in every third CTA the loader, in every third the issuer, in every third the epilogue leaves out what the others wait for."""
     from vision_rwkv_b200 import _lib, ops
     lib, native = _lib.load(), _lib.native()
     rows = 128 * torch.cuda.get_device_properties(cuda_device).multi_processor_count      # three tiles to a CTA
-    x = torch.randn(rows, 384, device=cuda_device).bfloat16()
-    w = torch.randn(192, 384, device=cuda_device).bfloat16() / 20
+    x = torch.randn(rows, K, device=cuda_device).bfloat16()
+    w = torch.randn(N, K, device=cuda_device).bfloat16() / 20
     with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
         want = native.linear_batch([x] * 3, [w] * 3)
         try:

@@ -1,6 +1,7 @@
 // Several linear layers of one shape in inference under bfloat16 autocast (the layers behind a token shift:
 // classification/mmcls_custom/models/backbones/vrwkv.py:166-168, vrwkv6.py:194-197) as one matrix product on the 5th-generation tensor
-// cores, results rounded to bfloat16; and the key layer with its squared ReLU (vrwkv.py:249-251) where it is shallow.
+// cores, results rounded to bfloat16; and the key layer with its squared ReLU (vrwkv.py:249-251) where it is shallow.  Deeper layers, and columns
+// that are no whole slabs, go to the tiles of linear_tc.cu.
 //
 // Products up to 384 deep are bound by memory.  With slices of W streamed beside those of x (linear_tc.cu) most of what an SM takes from L2
 // is W: 240 of 290 KB for 128 x 192 results at a depth of 384.  Here W stays: a persistent CTA holds a slab of 192 of its rows in shared memory
@@ -33,7 +34,6 @@ namespace lineartc {
 
 constexpr int kEpilogueWarps = 16, kEpilogueThreads = 32 * kEpilogueWarps, kBatchThreads = 64 + kEpilogueThreads;
 constexpr uint32_t kStrip = kM * 64 * 2;       // bytes of 128 rows x 64 bfloat16
-constexpr int kMostProducts = 4;
 constexpr int kSlab = 192, kSlice = 64;        // columns of a CTA's results; depth of a stage
 constexpr uint32_t kXBytes = kM * kSlice * 2, kWBytes = kSlab * kSlice * 2;
 constexpr int kMostDepth = 384;
@@ -170,9 +170,6 @@ __device__ __forceinline__ void put16(uint32_t at, uint32_t a, uint32_t b, uint3
 }
 
 // ---- products as they are ------------------------------------------------------------------------------------------------------
-struct Products {
-    CUtensorMap x[kMostProducts], w[kMostProducts], out[kMostProducts];
-};
 template <int kStages, int kSlots>
 static size_t batch_smem(int K) { return K * kSlab * 2 + kStages * kXBytes + kSlots * kStrip + sizeof(Control<kStages>); }
 
@@ -272,8 +269,8 @@ static int run_batch(int count, long long rows, int K, int N, const uint16_t* co
                tensor_map::make_rows(maps.out + i, out[i], rows, N, 64, kM);
     if (!made) return refused("cuTensorMapEncodeTiled rejected a matrix");
     const int m_tiles = static_cast<int>((rows + kM - 1) / kM);
-    launch_behind(kernel, std::min(m_tiles, sms / slabs) * slabs, kBatchThreads, batch_smem<kStages, kSlots>(K), static_cast<cudaStream_t>(stream), maps, count, m_tiles, N / kSlab, K / kSlice,
-                                                                                                                failure_mirror(Op::linear));
+    launch_behind(kernel, std::min(m_tiles, sms / slabs) * slabs, kBatchThreads, batch_smem<kStages, kSlots>(K), static_cast<cudaStream_t>(stream), maps,
+                  count, m_tiles, N / kSlab, K / kSlice, failure_mirror(Op::linear));
     return record_launches(1);
 }
 static bool unaligned(std::initializer_list<const void*> ps) {
@@ -309,7 +306,7 @@ extern "C" int vrwkv_linear_batch(int count, long long rows, int K, int N, const
         if (!x[i] || !w[i] || !out[i]) return VRWKV_ERR_NULL;
         if (unaligned({x[i], w[i], out[i]})) return VRWKV_ERR_ALIGNMENT;
     }
-    if (!serves(rows, K, N)) return VRWKV_ERR_UNSUPPORTED;
+    if (!serves(rows, K, N)) return tiles_serve(rows, K, N) ? batch_by_tiles(count, rows, K, N, x, w, out, stream) : VRWKV_ERR_UNSUPPORTED;
     return run<false>(count, rows, K, N, x, w, out, stream);
 }
 
@@ -320,7 +317,13 @@ extern "C" int vrwkv_linear_batch(int count, long long rows, int K, int N, const
 //   three      8.4 / 6.7   10.8 / 8.4   18.3 / 15.8   64.7 / 47.2   116.0 / 87.6   7.6 / 5.5   11.9 / 6.9    31.2 / 20.8   79.8 / 82.7
 //   four       11.1 / 6.7  14.1 / 9.1   26.3 / 19.1   86.1 / 59.6   154.7 / 116.2  9.9 / 5.5   15.9 / 8.1    41.8 / 28.1   106.1 / 108.8
 // A launch saved is worth 2 to 3 us more between other kernels, which covers the last column from three on; single layers and pairs are the
-// library's.
+// library's.  By tiles (linear_tc.cu), three layers:
+//   rows           196          1568         6272         12544        25088         50176         100352
+//   256 -> 256     7.7 / 5.6    9.4 / 5.8    11.2 / 6.4   13.9 / 8.7                 38.5 / 28.0   62.9 / 51.4
+//   512 -> 512     10.0 / 7.3   10.7 / 7.2   16.9 / 10.8  25.9 / 18.1  46.7 / 38.6   79.1 / 75.4
+//   768 -> 768     10.5 / 8.0   13.6 / 8.5   25.2 / 18.8  43.8 / 38.2  76.4 / 76.0   148.0 / 151.1
+//   1024 -> 1024   12.5 / 10.3  16.0 / 16.1  39.9 / 29.7  68.0 / 63.0  126.6 / 125.0 247.0 / 249.2
+// Four layers gain a little more (12544 x 768 58.1 / 50.6); the launches saved cover the last column.  Of the library's bits at every size tried.
 extern "C" int vrwkv_linear_batch_pays(int count, long long rows, int K, int N) {
-    return count >= 3 && count <= lineartc::kMostProducts && rows > 0 && lineartc::serves(rows, K, N) ? 1 : 0;
+    return count >= 3 && count <= lineartc::kMostProducts && rows > 0 && (lineartc::serves(rows, K, N) || lineartc::tiles_serve(rows, K, N)) ? 1 : 0;
 }

@@ -65,7 +65,15 @@ __device__ __forceinline__ uint32_t relu_square2(uint32_t a, uint32_t b) {
     return *reinterpret_cast<const uint32_t*>(&r);
 }
 
-// linear_batch.cu: the same layer where a slab of W fits a CTA's shared memory beside what is on its way
+constexpr int kMostProducts = 4;
+struct Products {
+    CUtensorMap x[kMostProducts], w[kMostProducts], out[kMostProducts];
+};
+
+// linear_tc.cu: several layers of one shape, without the squared ReLU
+bool tiles_serve(long long rows, int K, int N);
+int batch_by_tiles(int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream);
+// linear_batch.cu: the key layer where a slab of W fits a CTA's shared memory beside what is on its way
 bool slab_serves(long long rows, int K, int N);
 int square_by_slabs(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream);
 

@@ -15,7 +15,7 @@ from . import _lib, normgate, ops, traced
 from .qshift import autocast_linears, feeds_autocast_linears, stock
 
 KERNEL_DTYPES = (torch.float32, torch.bfloat16)
-DEEPEST_BATCH = 384             # of vrwkv_linear_batch_pays: deeper layers are not worth the questions
+DEEPEST_BATCH = 1024            # of vrwkv_linear_batch_pays: deeper layers are not worth the questions
 MOST_NORM_CHANNELS = 1024       # a row of norm_residual lives in one warp's registers
 
 
