@@ -384,7 +384,7 @@ int vrwkv_wkv6_forward(int B, int T, int C, int H, const void* r, const void* k,
     if (exact)      // clears the status word itself
         return finish(wkv6::forward(B, T, H, static_cast<const float*>(r), static_cast<const float*>(k), static_cast<const float*>(v), w_raw, u,
                                     y, workspace, s));
-    cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
+    wkv6::clear(wkv6::Cleared{{}, static_cast<unsigned*>(workspace), 0}, s);
     return finish(wkv6c::forward(B, T, H, r, k, v, w_raw, u, y, in_bf16 != 0, workspace, s));
 }
 
@@ -446,7 +446,7 @@ static int wkv6_backward(int B, int T, int C, int H, const void* r, const void* 
         const auto out = [](void* p) { return static_cast<float*>(p); };
         return finish(wkv6::backward(B, T, H, in(r), in(k), in(v), w_raw, u, in(gy), out(gr), out(gk), out(gv), gw, gu, workspace, s));
     }
-    cudaMemsetAsync(workspace, 0, sizeof(unsigned), s);      // status word
+    wkv6::clear(wkv6::Cleared{{}, static_cast<unsigned*>(workspace), 0}, s);
     return finish(wkv6c::backward(B, T, H, r, k, v, w_raw, u, gy, gr, gk, gv, gw, gu, in_bf16, gy_bf16, out_bf16, workspace, s));
 }
 

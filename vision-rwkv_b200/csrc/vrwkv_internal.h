@@ -99,6 +99,14 @@ int backward_bf16(int B, int T, int C, const float* w, const float* u, const voi
 }  // namespace biwkv
 
 namespace wkv6 {
+// What a launch finds at zero: the status word, and results of n floats each that its blocks add into.  In the place of memsets, and like
+// them not among the kernels that a launcher counts.
+struct Cleared {
+    float* p[3];           // null: none
+    unsigned* status;      // may be null
+    size_t n;
+};
+void clear(const Cleared& z, cudaStream_t stream);
 // float32 state sweeps (wkv6_sweeps.cu); gv may be null, and the forward's workspace
 size_t forward_workspace(int B, int T, int H);
 int forward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,

@@ -508,13 +508,8 @@ __global__ void wkv6_bonus_grad_kernel(int B, int C, const float* __restrict__ p
     gu[c] = acc;
 }
 
-// The status word (which these kernels never set) and the results that two directions add into, in one launch: three results of 19 MB took
-// 15 us as memsets, which the launch behind them also has to wait for in full.
-struct Cleared {
-    float* p[3];           // of n floats each, null: none
-    unsigned* status;      // may be null
-    size_t n;
-};
+// The status word and the results that two directions add into, in one launch: three results of 19 MB took 15 us as memsets, which the launch
+// behind them also has to wait for in full.
 constexpr int kClearVecs = 8;      // 16-byte stores of a thread
 __global__ void __launch_bounds__(256) wkv6_clear_kernel(const Cleared z) {
     wait_for_launch_before();
@@ -535,9 +530,9 @@ __global__ void __launch_bounds__(256) wkv6_clear_kernel(const Cleared z) {
         }
     }
 }
-static void clear(const Cleared& z, cudaStream_t stream) {
+void clear(const Cleared& z, cudaStream_t stream) {
     const size_t per_block = static_cast<size_t>(256) * kClearVecs * 4;
-    launch_behind(wkv6_clear_kernel, dim3(static_cast<unsigned>((z.n + per_block - 1) / per_block), z.p[1] == nullptr ? 1 : 3), 256, 0, stream, z);
+    launch_behind(wkv6_clear_kernel, dim3(static_cast<unsigned>(std::max<size_t>(1, (z.n + per_block - 1) / per_block)), z.p[1] == nullptr ? 1 : 3), 256, 0, stream, z);
 }
 
 struct Plan {
@@ -589,7 +584,7 @@ int forward(int B, int T, int H, const float* r, const float* k, const float* v,
     if (pl.segs > 1) run_segment_states(a, 1, stream);
     const auto kernel = pl.segs > 1 ? wkv6_sweep_kernel<false, true> : wkv6_sweep_kernel<false, false>;
     launch_behind(kernel, dim3(B * H, 1, 2 * pl.segs), N, sizeof(Shared), stream, a);
-    return pl.segs > 1 ? 4 : 2;
+    return pl.segs > 1 ? 3 : 1;
 }
 
 int backward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
@@ -622,7 +617,7 @@ int backward(int B, int T, int H, const float* r, const float* k, const float* v
                       a.cum[0], a.cum[1], a.cum[2], a.cum[3], gw);
     }
     launch_behind(wkv6_bonus_grad_kernel, (C + 127) / 128, 128, 0, stream, B * pl.segs, C, a.gu_part, gu);
-    return pl.segs > 1 ? 6 : 4;
+    return pl.segs > 1 ? 5 : 3;
 }
 
 }  // namespace wkv6

@@ -33,6 +33,7 @@
 #include <cuda_runtime.h>
 #include <mutex>
 #include <cstdint>
+#include "launch.h"
 #include "sm100_async.cuh"
 #include "tensor_map.h"
 #include "vrwkv_internal.h"
@@ -215,6 +216,7 @@ __global__ void __launch_bounds__(kPThreads, 2)
 wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_w,
                          const __grid_constant__ CUtensorMap map_y) {
+    wait_for_launch_before();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     SmemP& s = *reinterpret_cast<SmemP*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -569,11 +571,8 @@ static int launch(int B, int T, int H, const void* r, const void* k, const void*
     }
     Args a{B, T, H, static_cast<const float*>(r), static_cast<const float*>(k), static_cast<const float*>(v), w_raw, u, y,
            status, failure_mirror(Op::wkv6_forward)};
-    cudaMemsetAsync(status, 0, sizeof(unsigned), stream);
-    // both directions add into y
-    cudaMemsetAsync(y, 0, static_cast<size_t>(B) * T * C * sizeof(float), stream);
-    if (half_in) wkv6_tc_pipelined_kernel<true><<<2 * B * H, kPThreads, sizeof(SmemP), stream>>>(a, mr, mk, mv, mw, my);
-    else wkv6_tc_pipelined_kernel<false><<<2 * B * H, kPThreads, sizeof(SmemP), stream>>>(a, mr, mk, mv, mw, my);
+    wkv6::clear(wkv6::Cleared{{y}, status, static_cast<size_t>(B) * T * C}, stream);      // both directions add into y
+    launch_behind(half_in ? wkv6_tc_pipelined_kernel<true> : wkv6_tc_pipelined_kernel<false>, 2 * B * H, kPThreads, sizeof(SmemP), stream, a, mr, mk, mv, mw, my);
     return 1;
 }
 
