@@ -10,9 +10,9 @@
 //   2. outputs: one CTA per chunk, all chunks in parallel, both directions at once: read-out of the entering states,
 //      the 64 x 64 pairs inside the chunk, and (backward) the decay gradient.
 //
-// What bounds it: memory.  Per element of a (B, T, C) tensor the bfloat16 forward moves 12 bytes in the first kernel and
-// 18 in the second (the states are 4 of each), the backward 28 and 38; the products are 2.2 and 11 kFLOP, a third of
-// that time.  The walk of the first kernel is serial over T / 64 chunks but holds only the state update; everything else
+// What bounds it: memory in the first kernel, shared-memory accesses in the second (below).  Per element of a (B, T, C) tensor the bfloat16
+// forward moves 20 bytes in the first kernel and 18 in the second (the states are 4 of each), the backward 44 and 40, 2.0 + 1.8 and 4.4 + 4.0 GB
+// at B=32, T=4096, H=12, which take 0.30 + 0.61 and 0.74 + 1.99 ms; the products are 2.2 and 11 kFLOP.  The walk of the first kernel is serial over T / 64 chunks but holds only the state update; everything else
 // is parallel over chunks, which a walk over the whole sequence per CTA (16 tokens at a time with the state in tensor
 // memory: 1.47 + 7.8 ms at B=32, T=4096, H=12) was not.  64-wide heads make 16 x 64 x 64 products: mma.sync keeps their
 // operands, scalings and masks in registers, where tcgen05 would stage each through shared memory and tensor memory for
