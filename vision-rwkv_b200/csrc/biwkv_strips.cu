@@ -158,7 +158,7 @@ __device__ __forceinline__ void strip_constants(float* consts, const Params& p, 
     constexpr int kCs = St::kCs;
     if (threadIdx.x >= 2 * kCs) return;
     const int ch = threadIdx.x & (kCs - 1), at = strip * kCs + ch;
-    const float w = at < p.C ? __ldg(p.w + at) : 0.f, u = at < p.C ? __ldg(p.u + at) : 0.f;
+    const float w = at < p.C ? p.w[at] : 0.f, u = at < p.C ? p.u[at] : 0.f;
     // no infinity: what lies past the end of a sequence is zero and has to stay so
     const auto put = [&](int row, double x) { consts[row * kCs + ch] = static_cast<float>(x > 1e38 ? 1e38 : x); };
     const double wd = w;
@@ -1006,14 +1006,14 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                    const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_o0,
                    const __grid_constant__ CUtensorMap map_o1, const Params p) {
+    launch_dependents();
+    wait_for_launch_before();
     constexpr int P = St::P, L = St::L, kCs = St::kCs, kSpan = St::kSpan, kArea = St::kAreaFloats;
     constexpr bool kHalf = kTypes != Types::f32, kHalfG = kTypes == Types::bf16;
     constexpr bool kHalfOut = kBwd ? kHalf : kTypes == Types::bf16;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int n_clusters = static_cast<int>(gridDim.x) / p.cluster, mine = static_cast<int>(blockIdx.x) / p.cluster;
     const int rank = p.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
-    launch_dependents();
-    wait_for_launch_before();
     // this cluster's units: mine, mine + n_clusters, ..; all their CTAs wrote the same kRedo
     bool any = false;
     unsigned bits = 0u;
@@ -1113,10 +1113,10 @@ biwkv_exact_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
 }
 
 // out[j][c] = sum over sequences and ranks of the partials, fixed order
-__global__ void __launch_bounds__(1024) reduce_partials(int rows, int c_padded, int C, const float* __restrict__ partial, float* __restrict__ out) {
+__global__ void __launch_bounds__(1024) reduce_partials(int rows, int c_padded, int C, const float* partial, float* __restrict__ out) {
+    wait_for_launch_before();
     __shared__ float red[32][33];
     const int j = blockIdx.y, lane = threadIdx.x, ch = blockIdx.x * 32 + lane;
-    wait_for_launch_before();
     float acc = 0.f;
     if (ch < C)
         for (int r = threadIdx.y; r < rows; r += 32) acc += __ldcg(partial + (static_cast<size_t>(r) * 2 + j) * c_padded + ch);

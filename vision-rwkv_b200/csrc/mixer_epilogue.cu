@@ -106,7 +106,7 @@ __device__ __forceinline__ float relu2(float x) {
 // O = float with R = bfloat16: the rounded result, widened for a LayerNorm that takes it in float32 (the copy that torch makes of it
 // under autocast is a pass of 6 bytes per element, this one of 2 more: the matrix-state base model on 64 images 10.15 -> 9.90 ms).
 template <typename R, typename Y, typename O>
-__global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, const R* __restrict__ r, const Y* __restrict__ y, O* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, const R* r, const Y* y, O* __restrict__ out) {
     wait_for_launch_before();
     const long long i = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVec;
     if (i + kVec <= n) {
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kThreads) sigmoid_gate_kernel(long long n, con
 }
 
 template <typename R, typename O>
-__global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, const R* __restrict__ x, O* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, const R* x, O* __restrict__ out) {
     wait_for_launch_before();
     const long long i = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVec;
     if (i + kVec <= n) {
@@ -145,8 +145,8 @@ __global__ void __launch_bounds__(kThreads) relu_square_kernel(long long n, cons
 }
 
 // out[i] = table[i mod period] + a[i], eight elements (one 8-element vector of the table) per thread
-__global__ void __launch_bounds__(kThreads) add_rows_kernel(unsigned vectors, unsigned period, const float* __restrict__ table,
-                                                            const __nv_bfloat16* __restrict__ a, float* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) add_rows_kernel(unsigned vectors, unsigned period, const float* table,
+                                                            const __nv_bfloat16* a, float* __restrict__ out) {
     wait_for_launch_before();
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= vectors) return;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kThreads) add_rows_kernel(unsigned vectors, un
 }
 
 // HBM-bound: 12544 x 768 take 11.4 us (5.1 TB/s), torch's cast 21; the matrix-state base model on 64 images 9.62 -> 9.49 ms.
-__global__ void __launch_bounds__(kThreads) widen_kernel(unsigned vectors, const __nv_bfloat16* __restrict__ a, float* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) widen_kernel(unsigned vectors, const __nv_bfloat16* a, float* __restrict__ out) {
     wait_for_launch_before();
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= vectors) return;
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kThreads) narrow_kernel(const __grid_constant_
 // image row; reads are contiguous over the whole image, writes are whole 32-byte sectors.  With the library's
 // convolution, 1.14 ms of it, the small model took 8.0 ms for 256 images of 224 pixels, this way 6.7.
 __global__ void __launch_bounds__(kThreads) patch_rows_kernel(unsigned vectors, int channels, int H, int W, int rows, int cols, int patch,
-                                                              const float* __restrict__ img, __nv_bfloat16* __restrict__ out) {
+                                                              const float* img, __nv_bfloat16* __restrict__ out) {
     wait_for_launch_before();
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= vectors) return;
@@ -230,10 +230,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 // sigmoid_gate_kernel stores it: 12 bytes per element instead of 6 + 10 and a launch (the small
 // model on 256 images 6.80 -> 6.70 ms).
 template <typename A, int kIters, bool kGate>
-__global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C, float eps, const A* __restrict__ a, const A* __restrict__ gate,
-                                                                 const float* __restrict__ weight,
-                                                                 const float* __restrict__ bias, const float* __restrict__ gamma,
-                                                                 const float* __restrict__ x, float* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C, float eps, const A* a, const A* gate,
+                                                                 const float* weight,
+                                                                 const float* bias, const float* gamma,
+                                                                 const float* x, float* __restrict__ out) {
     wait_for_launch_before();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
@@ -302,11 +302,12 @@ __global__ void __launch_bounds__(kThreads) norm_residual_kernel(int rows, int C
 
 // The norm alone, rows as above.  A mean from one sum is off by its rounding, which on rows whose mean is three times their spread put
 // results 1.35e-7 from float64 (torch's layer 1.07e-7, C = 192 to 768); what rounding left in it is summed up beside the squares and
-// taken off, 5.2e-8 for any mean.  us, torch's layer / the norm as a case of the kernel above / this: 50176 x 384 95 / 25.2 / 24.5,
-// 50176 x 1024 149 / 69.3 / 63.0, 196 x 1024 3.7 / 3.9 / 3.2 (fewer registers and less code).
+// taken off, 5.2e-8 for any mean.  us, torch's layer / the norm as a case of the kernel above / this: 50176 x 384 95 / 25.2 / 24.4,
+// 50176 x 1024 149 / 69.3 / 63.2, 196 x 1024 3.7 / 3.9 / 3.1.  Weight and bias are asked for one piece of the row ahead, two in wide rows, since
+// a load is not moved over a store by itself (1568 x 640 2.9 -> 2.6; everything asked for before the first store 12544 x 1024 19.3 -> 20.3).
 template <int kIters>
-__global__ void __launch_bounds__(kThreads) layer_norm_kernel(int rows, int C, float eps, const float* __restrict__ x, const float* __restrict__ weight,
-                                                              const float* __restrict__ bias, float* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) layer_norm_kernel(int rows, int C, float eps, const float* x, const float* weight,
+                                                              const float* bias, float* __restrict__ out) {
     wait_for_launch_before();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
@@ -335,15 +336,24 @@ __global__ void __launch_bounds__(kThreads) layer_norm_kernel(int rows, int C, f
         }
     const float rest = warp_sum(d) * inv;
     const float rstd = rsqrtf(fmaxf(fmaf(-rest, rest, warp_sum(q) * inv), 0.f) + eps), shift = -rest * rstd;
+    constexpr int kAhead = kIters > 6 ? 2 : 1;
+    float w[kAhead + 1][4], b[kAhead + 1][4];      // asked for before the results in front of them leave
+    const auto scale_at = [&](int i) {
+        if (i < kIters && 128 * i + 4 * lane < C) {
+            load(weight + 128 * i + 4 * lane, w[i % (kAhead + 1)]);
+            load(bias + 128 * i + 4 * lane, b[i % (kAhead + 1)]);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) scale_at(i);
 #pragma unroll
     for (int i = 0; i < kIters; ++i)
         if (128 * i + 4 * lane < C) {
-            float w[4], b[4];
-            load(weight + 128 * i + 4 * lane, w);
-            load(bias + 128 * i + 4 * lane, b);
+            scale_at(i + kAhead);
+            const int at = i % (kAhead + 1);
             float4 o;
-            o.x = fmaf(fmaf(v[i][0], rstd, shift), w[0], b[0]); o.y = fmaf(fmaf(v[i][1], rstd, shift), w[1], b[1]);
-            o.z = fmaf(fmaf(v[i][2], rstd, shift), w[2], b[2]); o.w = fmaf(fmaf(v[i][3], rstd, shift), w[3], b[3]);
+            o.x = fmaf(fmaf(v[i][0], rstd, shift), w[at][0], b[at][0]); o.y = fmaf(fmaf(v[i][1], rstd, shift), w[at][1], b[at][1]);
+            o.z = fmaf(fmaf(v[i][2], rstd, shift), w[at][2], b[at][2]); o.w = fmaf(fmaf(v[i][3], rstd, shift), w[at][3], b[at][3]);
             *reinterpret_cast<float4*>(out + base + 128 * i) = o;
         }
 }
@@ -368,9 +378,9 @@ __device__ __forceinline__ float activation(float x, int act) {
     return act == 1 ? s : x * s;
 }
 template <typename G>
-__global__ void __launch_bounds__(kThreads) head_norm_gate_kernel(long long heads, int per_row, float eps, const float* __restrict__ x,
-                                                                  const G* __restrict__ gate, int act, const float* __restrict__ gamma,
-                                                                  const float* __restrict__ beta, __nv_bfloat16* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) head_norm_gate_kernel(long long heads, int per_row, float eps, const float* x,
+                                                                  const G* gate, int act, const float* gamma,
+                                                                  const float* beta, __nv_bfloat16* __restrict__ out) {
     wait_for_launch_before();
     const int q = threadIdx.x & (kLanes - 1);
     const long long mine = static_cast<long long>(blockIdx.x) * (kThreads / kLanes) + threadIdx.x / kLanes;

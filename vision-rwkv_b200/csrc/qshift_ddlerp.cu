@@ -135,7 +135,7 @@ struct RawM;
 template <>
 struct RawM<true> {
     uint2 v;
-    __device__ __forceinline__ void get(const void* m, size_t at) { v = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(m) + at)); }
+    __device__ __forceinline__ void get(const void* m, size_t at) { v = read_behind(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(m) + at)); }
     __device__ __forceinline__ float4 f() const {
         const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
         return make_float4(lo.x, lo.y, hi.x, hi.y);
@@ -144,7 +144,7 @@ struct RawM<true> {
 template <>
 struct RawM<false> {
     float4 v;
-    __device__ __forceinline__ void get(const void* m, size_t at) { v = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(m) + at)); }
+    __device__ __forceinline__ void get(const void* m, size_t at) { v = read_behind(reinterpret_cast<const float4*>(static_cast<const float*>(m) + at)); }
     __device__ __forceinline__ float4 f() const { return v; }
 };
 // kOffsets = false: no output has an offset, nothing but x is read; stretches of qlines::kStretch then.
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(256, 4) ddlerp_tokens_forward(const Args a, un
 #pragma unroll
     for (int j = 0; j < kMaxOut; ++j)
         if (j < a.n_out && a.m[j] != nullptr) {
-            if (kHalfM) both[kHalfM ? j : 0] = __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.m[j]) + base));
+            if (kHalfM) both[kHalfM ? j : 0] = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.m[j]) + base);
             else { m[j][0].get(a.m[j], base); m[j][1].get(a.m[j], base + 4); }
         }
 #pragma unroll

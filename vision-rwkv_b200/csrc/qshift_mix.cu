@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(qlines::kMaxThreads, 2) qshift_lines_backward(
 }
 
 // gmix[m][c] = sum over row blocks of partial[block][m][c], fixed order
-__global__ void __launch_bounds__(1024) qshift_reduce(const float* __restrict__ partial, int blocks, int n_out, int C,
+__global__ void __launch_bounds__(1024) qshift_reduce(const float* partial, int blocks, int n_out, int C,
                                                       float* __restrict__ gmix0, float* __restrict__ gmix1,
                                                       float* __restrict__ gmix2) {
     wait_for_launch_before();

@@ -1134,7 +1134,7 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
 #pragma unroll
                 for (int i = 0; i < kX; ++i) {
                     const int o = i * (kStateWords / 4) + (blk * 4 + kk) * 32 + lane;
-                    const uint4 fx = __ldg(sx + o), fy = __ldg(sy + o);
+                    const uint4 fx = read_behind(sx + o), fy = read_behind(sy + o);
                     const uint32_t wx[4] = {fx.x, fx.y, fx.z, fx.w}, wy[4] = {fy.x, fy.y, fy.z, fy.w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -1227,7 +1227,7 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int t = 32 * th + 8 * i + g;
-        w_own[i >> 1][i & 1] = t < tokens ? __ldg(reinterpret_cast<const float4*>(a.w + base + static_cast<size_t>(t) * C + 16 * cs + 4 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        w_own[i >> 1][i & 1] = t < tokens ? read_behind(reinterpret_cast<const float4*>(a.w + base + static_cast<size_t>(t) * C + 16 * cs + 4 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     {
         float carry[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1292,7 +1292,7 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
 }
 
 // gu[c] = sum over batch and chunks of the parts, in a fixed order
-__global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, const float* __restrict__ part, float* __restrict__ gu) {
+__global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, const float* part, float* __restrict__ gu) {
     wait_for_launch_before();
     __shared__ float red[32][33];
     const int c = blockIdx.x * 32 + threadIdx.x;

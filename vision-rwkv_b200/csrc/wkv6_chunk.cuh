@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "launch.h"
 
 namespace wkv6c {
 
@@ -142,7 +143,7 @@ template <int NB, bool kTrans>
 __device__ __forceinline__ void state_frag(uint32_t (&f)[NB][4], const uint4* state, int cs, int kk, int lane) {
 #pragma unroll
     for (int ib = 0; ib < NB; ++ib) {
-        const uint4 v = __ldg(state + ib * (kStateWords / 4) + ((kTrans ? kk * 4 + cs : cs * 4 + kk) * 32) + lane);
+        const uint4 v = read_behind(state + ib * (kStateWords / 4) + ((kTrans ? kk * 4 + cs : cs * 4 + kk) * 32) + lane);
         if (kTrans) {
             f[ib][0] = movm_trans(v.x); f[ib][1] = movm_trans(v.z); f[ib][2] = movm_trans(v.y); f[ib][3] = movm_trans(v.w);
         } else {
@@ -170,7 +171,7 @@ struct Raw<float> {
         for (int half = 0; half < 2; ++half)
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                v[half][kk] = g + 8 * half < rows ? __ldg(reinterpret_cast<const float4*>(p + static_cast<size_t>(g + 8 * half) * C + 16 * kk + 4 * q))
+                v[half][kk] = g + 8 * half < rows ? read_behind(reinterpret_cast<const float4*>(p + static_cast<size_t>(g + 8 * half) * C + 16 * kk + 4 * q))
                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __device__ __forceinline__ void get(int half, int kk, float (&x)[4]) const {
@@ -185,7 +186,7 @@ struct Raw<__nv_bfloat16> {
         for (int half = 0; half < 2; ++half)
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                v[half][kk] = g + 8 * half < rows ? __ldg(reinterpret_cast<const uint2*>(p + static_cast<size_t>(g + 8 * half) * C + 16 * kk + 4 * q))
+                v[half][kk] = g + 8 * half < rows ? read_behind(reinterpret_cast<const uint2*>(p + static_cast<size_t>(g + 8 * half) * C + 16 * kk + 4 * q))
                                                   : make_uint2(0u, 0u);
     }
     __device__ __forceinline__ void get(int half, int kk, float (&x)[4]) const {
@@ -193,11 +194,11 @@ struct Raw<__nv_bfloat16> {
     }
 };
 __device__ __forceinline__ void load4(const float* p, float (&x)[4]) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 v = read_behind(reinterpret_cast<const float4*>(p));
     x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
 }
 __device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&x)[4]) {
-    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+    const uint2 v = read_behind(reinterpret_cast<const uint2*>(p));
     x[0] = lo_f(v.x); x[1] = hi_f(v.x); x[2] = lo_f(v.y); x[3] = hi_f(v.y);
 }
 // raw inputs of the half-precision kernels are rounded to bfloat16 where they arrive as float
@@ -257,7 +258,7 @@ struct Pair;        // a lane's two channels of one token, as they lie in memory
 template <>
 struct Pair<float> {
     float2 v;
-    __device__ __forceinline__ void load(const float* p, bool on) { v = on ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(0.f, 0.f); }
+    __device__ __forceinline__ void load(const float* p, bool on) { v = on ? read_behind(reinterpret_cast<const float2*>(p)) : make_float2(0.f, 0.f); }
     __device__ __forceinline__ void lds(const float* p) { v = *reinterpret_cast<const float2*>(p); }
     __device__ __forceinline__ float2 get() const { return v; }
     __device__ __forceinline__ uint32_t bits() const { return 0u; }
@@ -265,7 +266,7 @@ struct Pair<float> {
 template <>
 struct Pair<__nv_bfloat16> {
     uint32_t v;
-    __device__ __forceinline__ void load(const __nv_bfloat16* p, bool on) { v = on ? __ldg(reinterpret_cast<const uint32_t*>(p)) : 0u; }
+    __device__ __forceinline__ void load(const __nv_bfloat16* p, bool on) { v = on ? read_behind(reinterpret_cast<const uint32_t*>(p)) : 0u; }
     __device__ __forceinline__ void lds(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint32_t*>(p); }
     __device__ __forceinline__ float2 get() const { return make_float2(lo_f(v), hi_f(v)); }
     __device__ __forceinline__ uint32_t bits() const { return v; }      // the pair as it is

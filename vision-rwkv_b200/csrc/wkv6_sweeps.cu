@@ -320,10 +320,10 @@ constexpr int kPerSm = 7;      // blocks, of 128 registers a thread (as fast as 
 // grid (b h, walk, direction + 2 segment)
 template <bool kBackward, bool kSeg>
 __global__ void __launch_bounds__(N, kPerSm) wkv6_sweep_kernel(const Args a) {
+    wait_for_launch_before();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
     __shared__ __align__(16) float u_smem[N];
-    wait_for_launch_before();
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H, seg = kSeg ? blockIdx.z >> 1 : 0;
     const bool forward = (blockIdx.z & 1) != 0;      // in time
     const int tid = threadIdx.x;
@@ -467,9 +467,9 @@ __global__ void __launch_bounds__(256) wkv6_segment_decay_grad_kernel(const Args
 // gw_raw = -exp(w_raw) * [ (P>_last - P>_t - Q>_t) + (P<_first - P<_t - Q<_t) ], a thread per 4 channels of a token, per_seq blocks to a
 // sequence.  (A thread per element with 64-bit divisions: 25.8 us at B=32, T=196, H=12, now 19.1.)  `scalar`: gw is not
 // 16-byte aligned.
-__global__ void __launch_bounds__(256) wkv6_decay_grad_kernel(int T, int C, unsigned per_seq, bool scalar, const float* __restrict__ w_raw, const float* __restrict__ cp,
-                                                              const float* __restrict__ cq, const float* __restrict__ cp2,
-                                                              const float* __restrict__ cq2, float* __restrict__ gw) {
+__global__ void __launch_bounds__(256) wkv6_decay_grad_kernel(int T, int C, unsigned per_seq, bool scalar, const float* w_raw, const float* cp,
+                                                              const float* cq, const float* cp2,
+                                                              const float* cq2, float* __restrict__ gw) {
     wait_for_launch_before();
     const unsigned per_row = static_cast<unsigned>(C) / 4, b = blockIdx.x / per_seq, v = (blockIdx.x - b * per_seq) * 256u + threadIdx.x;
     if (v >= per_row * static_cast<unsigned>(T)) return;
@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(256) wkv6_decay_grad_kernel(int T, int C, unsi
 }
 
 // gu[c] = sum over batch (and segments) of gu_part, fixed order
-__global__ void wkv6_bonus_grad_kernel(int B, int C, const float* __restrict__ part, float* __restrict__ gu) {
+__global__ void wkv6_bonus_grad_kernel(int B, int C, const float* part, float* __restrict__ gu) {
     wait_for_launch_before();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
