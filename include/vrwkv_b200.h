@@ -60,8 +60,8 @@ unsigned long long vrwkv_launch_count(void);
  * cluster-resident kernels (persistent tile kernels where eligible), 3 = test of the bounded
  * device-side waits: as 0, but one CTA of every cluster withholds what it owes the others and
  * the waits give up after about a thousand polls, so the call returns promptly with bit 0 of the
- * status word set and meaningless results (nothing hangs, nothing faults); vrwkv_linear_relu_square likewise, one
- * role of each CTA.  Process-wide.
+ * status word set and meaningless results (nothing hangs, nothing faults); the linear layers likewise, one role of each CTA, and
+ * WKV6 on the tensor cores, whose barriers wait for more than is copied (bit 1).  Process-wide.
  * No reference counterpart. */
 int vrwkv_set_path(int path);
 /* Copies the device status word kept in the first 4 bytes of a workspace to *status_out

@@ -129,6 +129,7 @@ int forward_bf16in(int B, int T, int H, const void* r, const void* k, const void
 namespace wkv6c {
 // Chunked tensor-core kernels (wkv6_chunk.cu): bfloat16 operands (r, k, v, gy in bfloat16, or float32 rounded on the way
 // in), scaled operands of gr, gk, gw carried to 16 bits.  gv may be null.
+void set_withhold_test(bool on);   // test only: barriers wait for more than is copied, and give up early
 size_t forward_workspace(int B, int T, int H);
 size_t backward_workspace(int B, int T, int H);
 int forward(int B, int T, int H, const void* r, const void* k, const void* v, const float* w, const float* u, float* y,

@@ -32,6 +32,7 @@
 //
 // Reference being replaced: classification/mmcls_custom/models/backbones/cuda_v6/wkv6_cuda.cu:6-346.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <set>
 #include <utility>
@@ -54,8 +55,12 @@ struct StateArgs {
     size_t plane;            // uint4 per (pair, direction)
     unsigned* status;        // the launch's status word and its host-visible copy
     unsigned* mirror;
+    unsigned limit;          // polls of a wait
+    unsigned extra;          // test only: bytes that a barrier waits for and no copy brings
 };
-constexpr uint32_t kWaitLimit = 1u << 20;      // polls before a wait for a tile gives up
+// Polls before a wait for a tile gives up.  After that nothing is copied to where it would have been, and what is under way is waited for a
+// little longer, so that a CTA leaves no copy behind.
+constexpr uint32_t kWaitLimit = 1u << 20;
 
 // Shared memory of a CTA, twice (the next chunk's tiles arrive during the whole of a step): the tiles of one chunk as the copy engine delivers
 // them (w | x, z of every pair).  The operands take their place: a warp reads its tokens' rows and writes the same rows, 16-byte pieces
@@ -131,7 +136,7 @@ wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, con
         const int t0 = chunk_of(step) * kChunk;
         unsigned char* const to = smem + (step & 1) * S::loaded;
         uint64_t* const full = bar + (step & 1);
-        sm100::mbar_expect_tx(full, S::loaded);
+        sm100::mbar_expect_tx(full, S::loaded + a.extra);
         sm100::tma_load_3d(to + S::w, &mw, full, h * N, t0, b);
         sm100::tma_load_3d(to + S::x0, &mx0, full, h * N, t0, b);
         sm100::tma_load_3d(to + S::z0, &mz0, full, h * N, t0, b);
@@ -152,9 +157,13 @@ wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, con
     const int row0 = w8 * kTokens, word = col_word(lane);
     Acc c;
     zero(c);
+    int gave_up = last;      // the step whose tiles did not come
     for (int step = 0; step < last; ++step) {
         const int valid = a.T - chunk_of(step) * kChunk;
-        if (!sm100::mbar_wait(bar + (step & 1), step >> 1 & 1, kWaitLimit)) report_failure(a.status, a.mirror, 2u);
+        if (step < gave_up && !sm100::mbar_wait(bar + (step & 1), step >> 1 & 1, a.limit)) {
+            gave_up = step;
+            report_failure(a.status, a.mirror, 2u);
+        }
         at = base_at + (step & 1) * S::loaded;
         raw = smem + (step & 1) * S::loaded;
         float2 sum[kTokens];
@@ -268,7 +277,7 @@ wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, con
         }
         sm100::fence_proxy_async_smem();      // the copy engine writes where the operands were
         __syncthreads();
-        if (threadIdx.x == 0 && step + 2 < last) fetch(step + 2);
+        if (threadIdx.x == 0 && step + 2 < last && gave_up == last) fetch(step + 2);
         uint4* o = out + static_cast<size_t>(chunk_of(step + 1)) * kState;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
@@ -282,6 +291,8 @@ wkv6_state_kernel(const StateArgs a, const __grid_constant__ CUtensorMap mw, con
                 o[s * (kStateWords / 4) + (warp * 4 + kk) * 32 + lane] = make_uint4(w0[s], w1[s], w2[s], w3[s]);
         }
     }
+    if (threadIdx.x == 0)
+        for (int s = gave_up; s < last && s < gave_up + 2; ++s) sm100::mbar_wait(bar + (s & 1), s >> 1 & 1, a.limit / 64);
 }
 
 // ---- pieces of kernel 2 ----------------------------------------------------------------------------------------
@@ -767,6 +778,7 @@ __device__ __forceinline__ void prefetch_bytes(const void* p, int bytes) {
 
 constexpr uint32_t kRawTile = kChunk * N * 2;
 
+
 // ---- kernel 2, forward ---------------------------------------------------------------------------------------
 struct OutArgs {
     int T, H, n_chunks;
@@ -782,6 +794,8 @@ struct OutArgs {
     size_t plane;
     unsigned* status;         // as in StateArgs
     unsigned* mirror;
+    unsigned limit;
+    unsigned extra;
 };
 
 // kX parts of the scaled operands and states, kZ parts of v
@@ -810,7 +824,7 @@ wkv6_forward_kernel(const OutArgs a, const __grid_constant__ CUtensorMap mw, con
         if (threadIdx.x == 0) {
             sm100::mbar_init(bar, 1);
             sm100::mbar_init_fence();
-            sm100::mbar_expect_tx(bar, 3 * kRawTile + kChunk * N * 4);
+            sm100::mbar_expect_tx(bar, 3 * kRawTile + kChunk * N * 4 + a.extra);
             sm100::tma_load_3d(w_raw, &mw, bar, h * N, n * kChunk, b);
             sm100::tma_load_3d(v_raw, &mv, bar, h * N, n * kChunk, b);
             sm100::tma_load_3d(r_raw, &mr, bar, h * N, n * kChunk, b);
@@ -838,7 +852,7 @@ wkv6_forward_kernel(const OutArgs a, const __grid_constant__ CUtensorMap mw, con
         __nv_bfloat16* planes = kf + dir * kX * kPlane;
         __nv_bfloat16* mine = edges + dir * kX * kPlane;
         if constexpr (sizeof(T) == 2) {
-            if (!sm100::mbar_wait(bar, 0, kWaitLimit)) report_failure(a.status, a.mirror, 2u);
+            if (!sm100::mbar_wait(bar, 0, a.limit)) report_failure(a.status, a.mirror, 2u);
             uint2 rr[2][4], kr[2][4];      // this thread's part of the block, out of the tiles before planes and pairs take their place
 #pragma unroll
             for (int i = 0; i < 8; ++i) rr[i >> 2][i & 3] = raw4(r_raw, blk * kBlock + g + 8 * (i >> 2), i & 3, q);
@@ -884,6 +898,8 @@ wkv6_forward_kernel(const OutArgs a, const __grid_constant__ CUtensorMap mw, con
                 put4(a.scalar, a.y + base + static_cast<size_t>(t) * C + 16 * cs + 4 * q, y[m][0][2 * half], y[m][0][2 * half + 1],
                      y[m][1][2 * half], y[m][1][2 * half + 1]);
         }
+    // after a wait that gave up (here and not behind it: there the second loop cost 1.5 % of the forward)
+    if (sizeof(T) == 2 && threadIdx.x == 0) sm100::mbar_wait(bar, 0, a.limit / 64);
 }
 
 // ---- kernel 2, backward --------------------------------------------------------------------------------------
@@ -906,6 +922,8 @@ struct GradArgs {
     size_t plane;
     unsigned* status;         // as in StateArgs
     unsigned* mirror;
+    unsigned limit;
+    unsigned extra;
 };
 
 
@@ -1060,7 +1078,7 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
         if (threadIdx.x == 0) {
             sm100::mbar_init(bar, 1);
             sm100::mbar_init_fence();
-            sm100::mbar_expect_tx(bar, 3 * kRawTile + kChunk * N * (4 + sizeof(G)));
+            sm100::mbar_expect_tx(bar, 3 * kRawTile + kChunk * N * (4 + sizeof(G)) + a.extra);
             sm100::tma_load_3d(w_raw, &mw, bar, h * N, n * kChunk, b);
             sm100::tma_load_3d(g_raw, &mg, bar, h * N, n * kChunk, b);
             sm100::tma_load_3d(v_raw, &mv, bar, h * N, n * kChunk, b);
@@ -1082,7 +1100,7 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
             if ((i & 1) ? n2 + 1 < a.n_chunks : n2 > 0) prefetch_bytes(st2 + i * a.plane, kState * 16);
     }
     if (sizeof(T) == 2) {
-        if (!sm100::mbar_wait(bar, 0, kWaitLimit)) report_failure(a.status, a.mirror, 2u);
+        if (!sm100::mbar_wait(bar, 0, a.limit)) report_failure(a.status, a.mirror, 2u);
         if (dir == 0) {
             scan_tile(tab, reinterpret_cast<const float*>(w_raw), rows, blk, lane);
         } else {
@@ -1289,6 +1307,7 @@ __global__ void __launch_bounds__(256, 2) wkv6_backward_kernel(const GradArgs a,
                          y[mt][0][2 * half + 1], y[mt][1][2 * half], y[mt][1][2 * half + 1]);
             }
     }
+    if (sizeof(T) == 2 && threadIdx.x == 0) sm100::mbar_wait(bar, 0, a.limit / 64);
 }
 
 // gu[c] = sum over batch and chunks of the parts, in a fixed order
@@ -1309,6 +1328,12 @@ __global__ void __launch_bounds__(1024) wkv6_bonus_kernel(int parts, int C, cons
 }
 
 // ---- host side -------------------------------------------------------------------------------------------------
+// test mode: barriers wait for 16 bytes that never come, and give up after 2^10 polls
+static std::atomic<bool> g_withhold{false};
+void set_withhold_test(bool on) { g_withhold.store(on); }
+static unsigned wait_limit() { return g_withhold.load() ? 1u << 10 : kWaitLimit; }
+static unsigned extra_bytes() { return g_withhold.load() ? 16u : 0u; }
+
 static size_t forward_smem(int kz, int kx) { return static_cast<size_t>(kz + 5 * kx) * kPlane * 2 + sizeof(Table) + 16; }
 static size_t backward_smem(int kz, int kx) {
     return 2 * kRawTile + static_cast<size_t>(2 * kz + 3 * kx) * kPlane * 2 + sizeof(Table) + (1 + 2 + 2 + 1) * N * sizeof(float) + 16;
@@ -1377,7 +1402,7 @@ static bool run_states(int B, int T_, int H, const void* r, const void* k, const
         mg = mv;
     }
     const StateArgs a{T_, H, chunks_of(T_), states, plane, static_cast<unsigned*>(workspace),
-                      failure_mirror(kRows ? Op::wkv6_backward : Op::wkv6_forward)};
+                      failure_mirror(kRows ? Op::wkv6_backward : Op::wkv6_forward), wait_limit(), extra_bytes()};
     const auto kernel = wkv6_state_kernel<T, T, G, kX, kRows, kPairs>;
     if (!allow_smem(reinterpret_cast<const void*>(kernel), S::bytes)) return false;
     launch_behind(kernel, dim3(B * H, 2), 128 * kPairs, S::bytes, stream, a, mw, mk, mv, mr, mg);
@@ -1396,7 +1421,7 @@ static int run_forward(int B, int T_, int H, const void* r, const void* k, const
         ++launched;
     }
     OutArgs o{T_, H, n_chunks, ahead_of(static_cast<size_t>(B) * H * n_chunks), r, k, v, w, aligned_bonus(u, H, workspace, stream), y, unaligned16({y}), states, plane,
-              static_cast<unsigned*>(workspace), failure_mirror(Op::wkv6_forward)};
+              static_cast<unsigned*>(workspace), failure_mirror(Op::wkv6_forward), wait_limit(), extra_bytes()};
     tensor_map::bind_primary_context();
     CUtensorMap mw, mk, mr, mv;
     const bool half = sizeof(T) == 2;
@@ -1421,7 +1446,7 @@ static int run_backward(int B, int T_, int H, const void* r, const void* k, cons
     }
     float* gu_part = reinterpret_cast<float*>(states + 4 * plane);
     GradArgs o{T_, H, n_chunks, ahead_of(static_cast<size_t>(B) * H * n_chunks), r, k, v, gy, w, aligned_bonus(u, H, workspace, stream), gr, gk, gv, gw, gu_part, unaligned16({gr, gk, gv, gw}), states, plane,
-               static_cast<unsigned*>(workspace), failure_mirror(Op::wkv6_backward)};
+               static_cast<unsigned*>(workspace), failure_mirror(Op::wkv6_backward), wait_limit(), extra_bytes()};
     tensor_map::bind_primary_context();
     CUtensorMap mw, mk, mr, mv, mg;
     const auto map = [&](CUtensorMap* m, const void* p, bool half, bool swizzled) { return tensor_map::make_btc(m, p, B, T_, C, N, kChunk, half, swizzled); };
