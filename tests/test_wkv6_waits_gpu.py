@@ -41,3 +41,10 @@ def test_chunks(cuda_device, T, dtype):
         return      # float32 tensors come by TMA in the walk over chunks only
     check(lambda: [ops.wkv6_forward(r, k, v, w, u, H, tensor_cores=True)], "WKV6 forward")
     check(lambda: ops.wkv6_backward(r, k, v, w, u, gy, H, tensor_cores=True), "WKV6 backward")
+
+
+# one to three steps of 16 tokens (fewer and more than the staging slots), a ragged last one, many
+@pytest.mark.parametrize("T", [1, 16, 17, 33, 48, 200])
+def test_walk(cuda_device, T):
+    r, k, v, w, u, _ = inputs(cuda_device, 3, T, 2, torch.bfloat16)
+    check(lambda: [_lib.native().wkv6_walk(r, k, v, w, u)], "WKV6 forward")

@@ -110,6 +110,7 @@ int vrwkv_set_path(int path) {
     biwkv::strips::set_withhold_test(path == 3);
     lineartc::set_withhold_test(path == 3);
     wkv6c::set_withhold_test(path == 3);
+    wkv6tc::set_withhold_test(path == 3);
     g_path.store(path == 3 ? 0 : path);
     return VRWKV_OK;
 }

@@ -118,6 +118,7 @@ int backward(int B, int T, int H, const float* r, const float* k, const float* v
 }  // namespace wkv6
 
 namespace wkv6tc {
+void set_withhold_test(bool on);   // test only: as in wkv6c
 // Tensor-core forward (bf16 operands, fp32 state) without scratch memory.  `status` points at 4 writable device bytes.
 int forward(int B, int T, int H, const float* r, const float* k, const float* v, const float* w_raw,
             const float* u, float* y, unsigned* status, cudaStream_t stream);

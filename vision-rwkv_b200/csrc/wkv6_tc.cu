@@ -31,6 +31,7 @@
 // Reference being replaced: classification/mmcls_custom/models/backbones/cuda_v6/wkv6_cuda.cu:6-97.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <mutex>
 #include <cstdint>
 #include "launch.h"
@@ -56,6 +57,8 @@ struct Args {
     float* y;
     unsigned* status;    // set to 1 if a bounded wait ran out
     unsigned* mirror;    // host-visible copy (may be null)
+    unsigned limit;      // polls of a wait
+    unsigned extra;      // test only: bytes that the tiles' barriers wait for and no copy brings
 };
 
 using sm100::smem_u32;
@@ -167,7 +170,7 @@ struct __align__(1024) SmemP {
     uint64_t ops_ready[2];
     uint64_t ops_free[2];
     uint64_t bar_main;
-    uint64_t bar_score;
+    uint64_t bar_score, drained;
     uint32_t tmem_base;
 };
 
@@ -245,6 +248,7 @@ wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r
         }
         sm100::mbar_init(&s.bar_main, 1);
         sm100::mbar_init(&s.bar_score, 1);
+        sm100::mbar_init(&s.drained, 1);
         sm100::mbar_init_fence();
     }
     if (warp == 0) {
@@ -261,7 +265,7 @@ wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r
 
     bool failed = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
-        if (!failed && !sm100::mbar_wait(bar, parity, kWaitLimit)) { failed = true; report_failure(a.status, a.mirror, 1u); }
+        if (!failed && !sm100::mbar_wait(bar, parity, a.limit)) { failed = true; report_failure(a.status, a.mirror, 1u); }
     };
 
     if (is_producer) {
@@ -388,15 +392,22 @@ wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r
             sm100::prefetch_tensormap(&map_k);
             sm100::prefetch_tensormap(&map_v);
             sm100::prefetch_tensormap(&map_w);
-            for (int step = 0; step < n_steps; ++step) {
+            int step = 0;
+            for (; step < n_steps; ++step) {
                 const int slot = step & 1, y0 = tile_start(step);
-                if (step >= 2) wait_on(&s.raw_free[slot], ((step >> 1) & 1) ^ 1u);
-                sm100::mbar_expect_tx(&s.raw_full[slot], (kHalfIn ? 3 * 2 + 4 : 4 * 4) * SC * N);
+                if (step >= 2) {
+                    wait_on(&s.raw_free[slot], ((step >> 1) & 1) ^ 1u);
+                    wait_on(&s.raw_full[slot], ((step >> 1) & 1) ^ 1u);      // over, unless the readers gave up waiting for it
+                }
+                if (failed) break;       // nothing is asked for where a copy is missing
+                sm100::mbar_expect_tx(&s.raw_full[slot], (kHalfIn ? 3 * 2 + 4 : 4 * 4) * SC * N + a.extra);
                 sm100::tma_load_3d(&s.raw[slot][0][0][0], &map_r, &s.raw_full[slot], h * N, y0, b);
                 sm100::tma_load_3d(&s.raw[slot][1][0][0], &map_k, &s.raw_full[slot], h * N, y0, b);
                 sm100::tma_load_3d(&s.raw[slot][2][0][0], &map_v, &s.raw_full[slot], h * N, y0, b);
                 sm100::tma_load_3d(&s.raw[slot][3][0][0], &map_w, &s.raw_full[slot], h * N, y0, b);
             }
+            // no copy is left behind
+            for (int last = step < 2 ? 0 : step - 2; last < step; ++last) sm100::mbar_wait(&s.raw_full[last & 1], (last >> 1) & 1, failed ? a.limit / 64 : a.limit);
         }
     } else if (is_control) {
         // =================================== control ===================================
@@ -413,6 +424,7 @@ wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r
             const uint64_t d_p = make_desc(smem_u32(set.opP), 256, 128);
             const uint64_t d_k = make_desc(smem_u32(set.opK), 1024, 128);
             wait_on(&s.ops_ready[slot], (m >> 1) & 1);
+            __syncwarp();      // one answer for all lanes, also where a wait ran out
             const bool pairwise = set.pairwise != 0;
             if (!pairwise) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -456,6 +468,9 @@ wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r
             }
             __syncwarp();
         }
+        if (elect_one()) tc_commit(&s.drained);
+        __syncwarp();
+        sm100::mbar_wait(&s.drained, 0, a.limit);      // the tensor memory is given back behind the last products
     } else {
         // =================================== state ===================================
         const int lg = warp & 1, ch = warp >> 2;               // 32 TMEM lanes x 32 state columns per warp
@@ -537,6 +552,10 @@ wkv6_tc_pipelined_kernel(const Args a, const __grid_constant__ CUtensorMap map_r
 }
 
 
+// test mode: barriers wait for 16 bytes that never come, and give up after 2^10 polls
+static std::atomic<bool> g_withhold{false};
+void set_withhold_test(bool on) { g_withhold.store(on); }
+
 // cudaFuncSetAttribute applies to the current device only: one flag per device, under a lock
 static bool configure_once() {
     static std::mutex lock;
@@ -570,7 +589,7 @@ static int launch(int B, int T, int H, const void* r, const void* k, const void*
         return -1;
     }
     Args a{B, T, H, static_cast<const float*>(r), static_cast<const float*>(k), static_cast<const float*>(v), w_raw, u, y,
-           status, failure_mirror(Op::wkv6_forward)};
+           status, failure_mirror(Op::wkv6_forward), g_withhold.load() ? 1u << 10 : kWaitLimit, g_withhold.load() ? 16u : 0u};
     wkv6::clear(wkv6::Cleared{{y}, status, static_cast<size_t>(B) * T * C}, stream);      // both directions add into y
     launch_behind(half_in ? wkv6_tc_pipelined_kernel<true> : wkv6_tc_pipelined_kernel<false>, 2 * B * H, kPThreads, sizeof(SmemP), stream, a, mr, mk, mv, mw, my);
     return 1;
