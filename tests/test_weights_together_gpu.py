@@ -103,3 +103,22 @@ def test_captured_in_a_held_context(cuda_device, warm):
         assert torch.equal(model(img)[0], want)
         graph.replay()
         assert torch.equal(out, want) and torch.equal(model(img)[0], want)
+
+
+def mixer(device):
+    """four layers and an input for `weights_for`"""
+    return [torch.nn.Linear(64, 64, bias=False, device=device, dtype=torch.float32) for _ in range(4)], torch.randn(2, 8, 64, device=device, dtype=torch.float32)
+
+
+@pytest.mark.parametrize("default", [torch.float64, torch.bfloat16, torch.float16])
+def test_the_count_ends_with_autocasts_copies_whatever_the_default_type_is(cuda_device, monkeypatch, default):
+    layers, x = mixer(cuda_device)
+    monkeypatch.setattr(epilogue, "_NOTHING", {})      # as at a process's first call
+    before = torch.get_default_dtype()
+    try:
+        torch.set_default_dtype(default)
+        for _ in range(4):
+            with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+                assert epilogue.weights_for(layers[0], x, *layers) is not None
+    finally:
+        torch.set_default_dtype(before)

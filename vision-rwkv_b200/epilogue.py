@@ -49,7 +49,7 @@ def _left_to_autocast(owner, device):
     nothing = _NOTHING.get(device)
     if nothing is None:
         with torch.inference_mode(False):
-            nothing = _NOTHING[device] = nn.Parameter(torch.empty(0, device=device))
+            nothing = _NOTHING[device] = nn.Parameter(torch.empty(0, device=device, dtype=torch.float32))      # what autocast copies
     calls = _lib.native().autocast_copy(nothing).__dict__
     before = calls.get(key := str(id(owner)), 0)        # (another owner at the same address has its weights cast one by one, no more)
     if before > 1:
