@@ -122,3 +122,18 @@ def test_the_count_ends_with_autocasts_copies_whatever_the_default_type_is(cuda_
                 assert epilogue.weights_for(layers[0], x, *layers) is not None
     finally:
         torch.set_default_dtype(before)
+
+
+def test_the_count_is_of_the_owner_and_not_of_its_address(cuda_device):
+    class Owner:
+        pass
+    layers, x = mixer(cuda_device)
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        owner = Owner()
+        for cast in (True, False, False):
+            assert (epilogue.weights_for(owner, x, *layers) is not None) == cast
+        address = id(owner)
+        del owner
+        others = [Owner() for _ in range(1000)]
+        again = [o for o in others if id(o) == address]
+        assert again and epilogue.weights_for(again[0], x, *layers) is not None

@@ -7,6 +7,8 @@ tensor operations and their graph.  A layer whose work a kernel takes over must 
 """
 from __future__ import annotations
 
+import weakref
+
 import torch
 import torch.nn as nn
 from torch.utils._device import DeviceContext
@@ -50,8 +52,8 @@ def _left_to_autocast(owner, device):
     if nothing is None:
         with torch.inference_mode(False):
             nothing = _NOTHING[device] = nn.Parameter(torch.empty(0, device=device, dtype=torch.float32))      # what autocast copies
-    calls = _lib.native().autocast_copy(nothing).__dict__
-    before = calls.get(key := str(id(owner)), 0)        # (another owner at the same address has its weights cast one by one, no more)
+    calls = _lib.native().autocast_copy(nothing).__dict__.setdefault("calls", {})
+    before = calls.get(key := weakref.ref(owner), 0)        # equal to another owner's never, also not to that of a gone one at its address
     if before > 1:
         return True
     if torch.cuda.is_current_stream_capturing():
