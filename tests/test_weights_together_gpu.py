@@ -137,3 +137,29 @@ def test_the_count_is_of_the_owner_and_not_of_its_address(cuda_device):
         others = [Owner() for _ in range(1000)]
         again = [o for o in others if id(o) == address]
         assert again and epilogue.weights_for(again[0], x, *layers) is not None
+
+
+def test_a_mode_sees_the_operations_of_layers_only(cuda_device):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.extend(a for a in args if isinstance(a, torch.Tensor) and a.numel() == 0)
+            return func(*args, **(kwargs or {}))
+    layers, x = mixer(cuda_device)
+    seen = []
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16), Watch():
+        assert epilogue.weights_for(layers[0], x, *layers) is None
+        [layer(x) for layer in layers]
+    assert not seen
+    casts = []
+    with pytest.MonkeyPatch.context() as m, torch.no_grad(), torch.autocast("cuda", torch.float16):
+        native = _lib.native()
+
+        class Native:
+            def __getattr__(self, name):
+                casts.append(name)
+                return getattr(native, name)
+        m.setattr(_lib, "native", Native)
+        assert epilogue.weights_for(layers[0], x, *layers) is None
+    assert not casts

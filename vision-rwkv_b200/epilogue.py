@@ -67,12 +67,13 @@ def weights_for(owner, x, *sources):
     in one launch instead of one each; None where each is left to its own product.  That is wherever somebody would see the cast or
     the layer's call, and from the second call of `owner` on in an autocast context that is held: autocast keeps what it casts by itself, and
     after that second call has no more to cast."""
-    if not x.is_cuda or torch.is_grad_enabled() or not torch.is_autocast_enabled("cuda") or traced.tracing():
+    if (not x.is_cuda or torch.is_grad_enabled() or not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") != torch.bfloat16
+            or traced.tracing() or x.dtype not in KERNEL_DTYPES or not _unwatched(x)):
         return None
     if _left_to_autocast(owner, x.device) and (type(sources[0]) is not nn.Linear or sources[0].weight.requires_grad):
         return None                                  # (autocast keeps no others)
     layers = [s for s in sources if isinstance(s, nn.Module)]
-    if x.dtype not in KERNEL_DTYPES or not autocast_linears(*layers) or not _unwatched(x) or any(layer.bias is not None for layer in layers):
+    if not autocast_linears(*layers) or any(layer.bias is not None for layer in layers):
         return None
     weights = [s.weight if isinstance(s, nn.Module) else s for s in sources]
     for w in weights:
