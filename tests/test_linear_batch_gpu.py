@@ -72,7 +72,7 @@ def test_not_a_number_stays(cuda_device):
             assert out[129].isnan().all() and out[5].isinf().all() and (out[6] == 64).all()
 
 
-@pytest.mark.parametrize("K,N", [(384, 192), (512, 256)])
+@pytest.mark.parametrize("K,N", [(384, 192), (512, 256), (192, 192)])
 def test_bounded_waits_run_out_and_report(cuda_device, K, N):
     """Path 3: in every third CTA the loader, in every third the issuer, in every third the epilogue leaves out what the others wait for."""
     from vision_rwkv_b200 import _lib, ops
@@ -91,4 +91,25 @@ def test_bounded_waits_run_out_and_report(cuda_device, K, N):
             lib.vrwkv_set_path(0)
         ops.raise_if_failed()
         assert all(torch.equal(a, b) for a, b in zip(native.linear_batch([x] * 3, [w] * 3), want))
+        ops.raise_if_failed()
+
+
+@pytest.mark.parametrize("K,N", [(64, 768), (192, 768), (256, 768)])
+def test_bounded_waits_of_the_key_layer_by_slabs(cuda_device, K, N):
+    """The same with the squared ReLU, four tiles to a CTA."""
+    from vision_rwkv_b200 import _lib, ops
+    lib, native = _lib.load(), _lib.native()
+    x = torch.randn(128 * torch.cuda.get_device_properties(cuda_device).multi_processor_count, K, device=cuda_device).bfloat16()
+    w = torch.randn(N, K, device=cuda_device).bfloat16() / 20
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        want = native.linear_relu_square(x, w)
+        try:
+            assert lib.vrwkv_set_path(3) == 0
+            native.linear_relu_square(x, w)
+            with pytest.raises(_lib.VrwkvError, match="earlier launch, linear:"):
+                ops.raise_if_failed()
+        finally:
+            lib.vrwkv_set_path(0)
+        ops.raise_if_failed()
+        assert torch.equal(native.linear_relu_square(x, w), want)
         ops.raise_if_failed()

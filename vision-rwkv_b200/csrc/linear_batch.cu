@@ -34,9 +34,7 @@ namespace lineartc {
 
 constexpr int kEpilogueWarps = 16, kEpilogueThreads = 32 * kEpilogueWarps, kBatchThreads = 64 + kEpilogueThreads;
 constexpr uint32_t kStrip = kM * 64 * 2;       // bytes of 128 rows x 64 bfloat16
-constexpr int kSlab = 192, kSlice = 64;        // columns of a CTA's results; depth of a stage
 constexpr uint32_t kXBytes = kM * kSlice * 2, kWBytes = kSlab * kSlice * 2;
-constexpr int kMostDepth = 384;
 
 template <int kStages_>
 struct Control {
@@ -257,9 +255,13 @@ static int refused(const char* why) {
 }
 
 template <int kStages, int kSlots, bool kSquare, bool kTest>
+static int sms_of() {
+    return prepare(reinterpret_cast<const void*>(linear_batch_kernel<kStages, kSlots, kSquare, kTest>), batch_smem<kStages, kSlots>(kStages == 4 ? 256 : kMostSlabDepth));
+}
+template <int kStages, int kSlots, bool kSquare, bool kTest>
 static int run_batch(int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream) {
     const auto kernel = linear_batch_kernel<kStages, kSlots, kSquare, kTest>;
-    const int sms = prepare(reinterpret_cast<const void*>(kernel), batch_smem<kStages, kSlots>(kStages == 4 ? 256 : kMostDepth)), slabs = N / kSlab * count;
+    const int sms = sms_of<kStages, kSlots, kSquare, kTest>(), slabs = N / kSlab * count;
     if (sms < slabs) return VRWKV_ERR_UNSUPPORTED;
     tensor_map::bind_primary_context();
     Products maps;
@@ -278,22 +280,21 @@ static bool unaligned(std::initializer_list<const void*> ps) {
     for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
     return (bits & 15u) != 0;
 }
-template <bool kSquare>
-static int run(int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream) {
-    if (withhold_test()) return run_batch<3, 2, kSquare, true>(count, rows, K, N, x, w, out, stream);
-    // shallow slabs leave room for more slices and strips under way (192 deep, three layers: 22.3 -> 20.8 us at 50176 rows, 85.5 -> 82.7 at 200704)
-    return K <= 256 ? run_batch<4, 4, kSquare, false>(count, rows, K, N, x, w, out, stream) : run_batch<3, 2, kSquare, false>(count, rows, K, N, x, w, out, stream);
+// shallow slabs leave room for more slices and strips under way (192 deep, three layers: 22.3 -> 20.8 us at 50176 rows, 85.5 -> 82.7 at 200704)
+static bool shallow(int K) { return K <= 256; }
+int slab_sms(bool square, int K) {
+    if (withhold_test()) return square ? sms_of<4, 4, true, true>() : shallow(K) ? sms_of<4, 4, false, true>() : sms_of<3, 2, false, true>();
+    return square ? sms_of<4, 4, true, false>() : shallow(K) ? sms_of<4, 4, false, false>() : sms_of<3, 2, false, false>();
 }
-constexpr long long kMostRows = 1LL << 24;      // tiles are counted in 32 bits
-constexpr int kMostColumns = 1536;             // slabs of up to four layers stay fewer than SMs
-
-static bool serves(long long rows, int K, int N) { return K > 0 && K % kSlice == 0 && K <= kMostDepth && N > 0 && N % kSlab == 0 && N <= kMostColumns && rows <= kMostRows; }
-// The key layer by linear_tc.cu's tiles / by slabs, us: 192 deep 12544 rows 9.6 / 9.8, 50176 28.5 / 25.0, 100352 51.9 / 42.2, 200704 99.2 / 78.4;
-// 384 deep 12544 rows 17.8 / 19.6, 50176 60.6 / 60.4, 100352 120.7 / 116.3.
-bool slab_serves(long long rows, int K, int N) { return K <= 256 && serves(rows, K, N); }
-int square_by_slabs(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream) {
-    return run<true>(1, rows, K, N, &x, &w, &out, stream);
+int run_square_by_slabs(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream) {
+    return (withhold_test() ? run_batch<4, 4, true, true> : run_batch<4, 4, true, false>)(1, rows, K, N, &x, &w, &out, stream);
 }
+static int run_by_slabs(int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream) {
+    const auto fn = withhold_test() ? (shallow(K) ? run_batch<4, 4, false, true> : run_batch<3, 2, false, true>)
+                                    : (shallow(K) ? run_batch<4, 4, false, false> : run_batch<3, 2, false, false>);
+    return fn(count, rows, K, N, x, w, out, stream);
+}
+static Route route(int count, long long rows, int K, int N) { return batch_route(count, rows, K, N, K <= kMostSlabDepth ? slab_sms(false, K) : 0, tile_sms()); }
 
 }  // namespace lineartc
 
@@ -306,8 +307,9 @@ extern "C" int vrwkv_linear_batch(int count, long long rows, int K, int N, const
         if (!x[i] || !w[i] || !out[i]) return VRWKV_ERR_NULL;
         if (unaligned({x[i], w[i], out[i]})) return VRWKV_ERR_ALIGNMENT;
     }
-    if (!serves(rows, K, N)) return tiles_serve(rows, K, N) ? batch_by_tiles(count, rows, K, N, x, w, out, stream) : VRWKV_ERR_UNSUPPORTED;
-    return run<false>(count, rows, K, N, x, w, out, stream);
+    const Route by = route(count, rows, K, N);
+    if (by == Route::none) return VRWKV_ERR_UNSUPPORTED;
+    return (by == Route::slabs ? run_by_slabs : batch_by_tiles)(count, rows, K, N, x, w, out, stream);
 }
 
 // Several layers of one shape against as many library products, in a captured loop (us):
@@ -325,5 +327,5 @@ extern "C" int vrwkv_linear_batch(int count, long long rows, int K, int N, const
 //   1024 -> 1024   12.5 / 10.3  16.0 / 16.1  39.9 / 29.7  68.0 / 63.0  126.6 / 125.0 247.0 / 249.2
 // Four layers gain a little more (12544 x 768 58.1 / 50.6); the launches saved cover the last column.  Of the library's bits at every size tried.
 extern "C" int vrwkv_linear_batch_pays(int count, long long rows, int K, int N) {
-    return count >= 3 && count <= lineartc::kMostProducts && rows > 0 && (lineartc::serves(rows, K, N) || lineartc::tiles_serve(rows, K, N)) ? 1 : 0;
+    return count >= 3 && count <= lineartc::kMostProducts && lineartc::route(count, rows, K, N) != lineartc::Route::none ? 1 : 0;
 }

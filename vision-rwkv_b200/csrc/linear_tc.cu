@@ -34,7 +34,7 @@
 
 namespace lineartc {
 
-constexpr int kN = 256, kK = 64, kStages = 4;
+constexpr int kN = kTile, kK = kSlice, kStages = 4;
 constexpr uint32_t kABytes = kM * kK * 2, kStageBytes = kABytes + kN * kK * 2, kBoxBytes = kM * 64 * 2;
 constexpr int kThreads = 192;
 
@@ -224,7 +224,6 @@ static bool allowed(int* sms) {
     return state[dev] > 0;
 }
 
-constexpr int kMostDepth = 1024;
 template <bool kSquare>
 static int run_tiles(int sms, int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream) {
     const long long m_tiles = (rows + kM - 1) / kM, tiles = m_tiles * (N / kN) * count;
@@ -241,10 +240,9 @@ static int run_tiles(int sms, int count, long long rows, int K, int N, const uin
                   static_cast<int>(tiles), static_cast<int>(m_tiles), N / kN, K / kK, failure_mirror(Op::linear));
     return record_launches(1);
 }
-bool tiles_serve(long long rows, int K, int N) {
+int tile_sms() {
     int sms = 0;
-    return rows > 0 && K > 0 && K % kK == 0 && K <= kMostDepth && N > 0 && N % kN == 0 && rows <= (1LL << 24) &&
-           (rows + kM - 1) / kM * (N / kN) <= (1LL << 28) && allowed(&sms);
+    return allowed(&sms) ? sms : 0;
 }
 int batch_by_tiles(int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream) {
     int sms = 0;
@@ -260,7 +258,7 @@ int batch_by_tiles(int count, long long rows, int K, int N, const uint16_t* cons
 // product is the faster one, and the pass is little beside it.
 extern "C" int vrwkv_linear_relu_square_pays(long long rows, int K, int N) {
     using namespace lineartc;
-    if (rows <= 0 || K <= 0 || N <= 0 || K % kK != 0 || N % kN != 0 || K > kMostDepth || rows > (1LL << 30)) return 0;
+    if (rows <= 0 || K <= 0 || N <= 0 || K % kK != 0 || N % kN != 0 || K > kMostTileDepth || rows > (1LL << 30)) return 0;
     const long long tiles = (rows + kM - 1) / kM * (N / kN);
     int sms = 0;
     if (tiles > (1LL << 30) || !allowed(&sms)) return 0;
@@ -276,6 +274,6 @@ extern "C" int vrwkv_linear_relu_square(long long rows, int K, int N, const uint
     const long long m_tiles = (rows + kM - 1) / kM, tiles = m_tiles * (N / kN);
     int sms = 0;
     if (K % kK != 0 || N % kN != 0 || rows > (1LL << 30) || tiles > (1LL << 30) || !allowed(&sms)) return VRWKV_ERR_UNSUPPORTED;
-    if (slab_serves(rows, K, N)) return square_by_slabs(rows, K, N, x, w, out, stream);
+    if (square_by_slabs(rows, K, N, slab_sms(true, K))) return run_square_by_slabs(rows, K, N, x, w, out, stream);
     return run_tiles<true>(sms, 1, rows, K, N, &x, &w, &out, stream);
 }

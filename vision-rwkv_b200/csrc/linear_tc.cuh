@@ -4,13 +4,13 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "linear_routes.h"
 #include "sm100_async.cuh"
 
 namespace lineartc {
 
 using sm100::smem_u32;
 
-constexpr int kM = 128;
 constexpr uint32_t kWaitLimit = 1u << 20;
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
@@ -70,11 +70,12 @@ struct Products {
     CUtensorMap x[kMostProducts], w[kMostProducts], out[kMostProducts];
 };
 
+// SMs of the current device, 0 where the kernels cannot be had: linear_tc.cu's, linear_batch.cu's for layers or the key layer K deep
+int tile_sms();
+int slab_sms(bool square, int K);
 // linear_tc.cu: several layers of one shape, without the squared ReLU
-bool tiles_serve(long long rows, int K, int N);
 int batch_by_tiles(int count, long long rows, int K, int N, const uint16_t* const* x, const uint16_t* const* w, uint16_t* const* out, void* stream);
 // linear_batch.cu: the key layer where a slab of W fits a CTA's shared memory beside what is on its way
-bool slab_serves(long long rows, int K, int N);
-int square_by_slabs(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream);
+int run_square_by_slabs(long long rows, int K, int N, const uint16_t* x, const uint16_t* w, uint16_t* out, void* stream);
 
 }  // namespace lineartc
