@@ -294,7 +294,7 @@ static int run_by_slabs(int count, long long rows, int K, int N, const uint16_t*
                                     : (shallow(K) ? run_batch<4, 4, false, false> : run_batch<3, 2, false, false>);
     return fn(count, rows, K, N, x, w, out, stream);
 }
-static Route route(int count, long long rows, int K, int N) { return batch_route(count, rows, K, N, K <= kMostSlabDepth ? slab_sms(false, K) : 0, tile_sms()); }
+static int batch_sms(int K) { return K <= kMostSlabDepth ? slab_sms(false, K) : 0; }
 
 }  // namespace lineartc
 
@@ -307,7 +307,7 @@ extern "C" int vrwkv_linear_batch(int count, long long rows, int K, int N, const
         if (!x[i] || !w[i] || !out[i]) return VRWKV_ERR_NULL;
         if (unaligned({x[i], w[i], out[i]})) return VRWKV_ERR_ALIGNMENT;
     }
-    const Route by = route(count, rows, K, N);
+    const Route by = batch_route(count, rows, K, N, batch_sms(K), tile_sms());
     if (by == Route::none) return VRWKV_ERR_UNSUPPORTED;
     return (by == Route::slabs ? run_by_slabs : batch_by_tiles)(count, rows, K, N, x, w, out, stream);
 }
@@ -318,14 +318,14 @@ extern "C" int vrwkv_linear_batch(int count, long long rows, int K, int N, const
 //   two        5.6 / 6.7   7.2 / 6.9    12.1 / 11.4   42.5 / 32.9   77.4 / 59.4    5.1 / 5.4   8.1 / 6.9     17.3 / 12.5   53.2 / 55.6
 //   three      8.4 / 6.7   10.8 / 8.4   18.3 / 15.8   64.7 / 47.2   116.0 / 87.6   7.6 / 5.5   11.9 / 6.9    31.2 / 20.8   79.8 / 82.7
 //   four       11.1 / 6.7  14.1 / 9.1   26.3 / 19.1   86.1 / 59.6   154.7 / 116.2  9.9 / 5.5   15.9 / 8.1    41.8 / 28.1   106.1 / 108.8
-// A launch saved is worth 2 to 3 us more between other kernels, which covers the last column from three on; single layers and pairs are the
-// library's.  By tiles (linear_tc.cu), three layers:
+// (a launch saved is worth 2 to 3 us more between other kernels: batch_pays in linear_routes.h); single layers and pairs are the library's.  By tiles (linear_tc.cu), three layers:
 //   rows           196          1568         6272         12544        25088         50176         100352
 //   256 -> 256     7.7 / 5.6    9.4 / 5.8    11.2 / 6.4   13.9 / 8.7                 38.5 / 28.0   62.9 / 51.4
 //   512 -> 512     10.0 / 7.3   10.7 / 7.2   16.9 / 10.8  25.9 / 18.1  46.7 / 38.6   79.1 / 75.4
 //   768 -> 768     10.5 / 8.0   13.6 / 8.5   25.2 / 18.8  43.8 / 38.2  76.4 / 76.0   148.0 / 151.1
 //   1024 -> 1024   12.5 / 10.3  16.0 / 16.1  39.9 / 29.7  68.0 / 63.0  126.6 / 125.0 247.0 / 249.2
-// Four layers gain a little more (12544 x 768 58.1 / 50.6); the launches saved cover the last column.  Of the library's bits at every size tried.
+// Four layers gain a little more (12544 x 768 58.1 / 50.6).
 extern "C" int vrwkv_linear_batch_pays(int count, long long rows, int K, int N) {
-    return count >= 3 && count <= lineartc::kMostProducts && lineartc::route(count, rows, K, N) != lineartc::Route::none ? 1 : 0;
+    using namespace lineartc;
+    return count <= kMostProducts && batch_pays(count, rows, K, N, batch_sms(K), tile_sms()) ? 1 : 0;
 }
