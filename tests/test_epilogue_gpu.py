@@ -267,3 +267,17 @@ def test_the_gate_rounds_every_bfloat16_sigmoid_as_its_float64_value(cuda_device
     unit = torch.exp2(torch.floor(torch.log2(want[ok].clamp_min(2.0 ** -126))) - 7)
     # below e^-88.7 the exponential is infinite in float32 and the sigmoid zero
     assert ((got[ok] - want[ok]).abs() <= 0.5 * unit + 2.0 ** -20 * want[ok] + 2.0 ** -127).all()
+
+
+@pytest.mark.parametrize("wide", [False, True])
+def test_the_gate_has_the_bits_of_the_float32_sigmoid(cuda_device, wide):
+    """All 65536 bfloat16 r: the approximate exponential and reciprocal round to what 1 / (1 + exp(-r)) in float32 rounds to."""
+    from vision_rwkv_b200 import _lib
+    r = torch.arange(65536, device=cuda_device, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    want = (1 / (1 + torch.exp(-r.float()))).bfloat16()
+    got = _lib.native().sigmoid_gate(r, torch.ones_like(r), wide).bfloat16()      # widened bfloat16: exact
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.nan_to_num().view(torch.int16), want.nan_to_num().view(torch.int16))
+    norm_in = torch.zeros(64, 1024, device=cuda_device)
+    gated = _lib.native().gated_norm_residual(norm_in, r.view(64, 1024), torch.ones_like(r).view(64, 1024), None, None, None, 0.0).view(-1)
+    assert torch.equal(gated.nan_to_num(), want.float().nan_to_num())
