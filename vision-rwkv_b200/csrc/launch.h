@@ -44,8 +44,9 @@ __device__ __forceinline__ uint32_t read_behind(const uint32_t* p) {
 // 64 images at 224 pixels 9069 -> 8782 us, a WKV6 layer's training at 196 tokens 259 -> 249.  The blocks start when all those of the kernel before
 // are gone or, behind Bi-WKV's strips (and kernels of libraries), have said that others may start: they are all resident by then and need
 // nothing that the new ones could hold, which do nothing but wait until they are gone.
+// An error of the launch stays until record_launches asks for it (cudaGetLastError), as that of <<<>>> does.
 template <typename... P, typename... A>
-inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+inline void launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -56,5 +57,5 @@ inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, si
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
