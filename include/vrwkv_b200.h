@@ -47,7 +47,8 @@ const char* vrwkv_status_string(int status);
 /* One line about the most recent non-zero status of the calling thread (for instance the name
  * of the CUDA error behind VRWKV_ERR_LAUNCH).  Thread-local storage.  Diagnostic. */
 const char* vrwkv_last_error_detail(void);
-/* Number of kernels this library has launched in the calling process so far. */
+/* Number of kernels this library has launched in the calling process so far, but for two that stand for what others did before and that was
+ * not counted: the clearing of the status word and of results that WKV6's directions add into (memsets), and vrwkv_narrow (casts). */
 unsigned long long vrwkv_launch_count(void);
 
 /* Kernel path selection, for tests and measurements: 0 = automatic (default: Bi-WKV takes the

@@ -12,7 +12,8 @@
 //
 // What bounds it: memory in the first kernel, shared-memory accesses in the second (below).  Per element of a (B, T, C) tensor the bfloat16
 // forward moves 20 bytes in the first kernel and 18 in the second (the states are 4 of each), the backward 44 and 40, 2.0 + 1.8 and 4.4 + 4.0 GB
-// at B=32, T=4096, H=12, which take 0.30 + 0.61 and 0.74 + 1.99 ms; the products are 2.2 and 11 kFLOP.  The walk of the first kernel is serial over T / 64 chunks but holds only the state update; everything else
+// at B=32, T=4096, H=12, which take 0.30 + 0.61 and 0.74 + 1.99 ms; the products are about 0.8 and 3.6 kFLOP
+// (0.26 and 1.0 of them in the first kernel).  The walk of the first kernel is serial over T / 64 chunks but holds only the state update; everything else
 // is parallel over chunks, which a walk over the whole sequence per CTA (16 tokens at a time with the state in tensor
 // memory: 1.47 + 7.8 ms at B=32, T=4096, H=12) was not.  64-wide heads make 16 x 64 x 64 products: mma.sync keeps their
 // operands, scalings and masks in registers, where tcgen05 would stage each through shared memory and tensor memory for
@@ -68,7 +69,7 @@ constexpr uint32_t kWaitLimit = 1u << 20;
 // the row of w, which its warp has read by then.
 //
 // What bounds the walk: HBM, since the two directions meet the inputs at different times and each reads them (forward 2 x 8 and backward 2 x 14 bytes an
-// element, states 4 and 16).  B=32, H=12, T=4096, forward / backward us: 308 / 735 (2.0 and 4.4 GB: 6.5 and 6.0 TB/s), T=196 17.3 / 39.3.  Operand planes
+// element, states 4 and 16).  B=32, H=12, T=4096, forward / backward us: 301 / 745 (2.0 and 4.4 GB: 6.6 and 5.9 TB/s), T=196 17.7 / 40.7.  Operand planes
 // beside one set of tiles, fetched while the products ran, and each pair's factors computed by its own warps: 450 / 902, 19.6 / 43.2; the
 // present form with one set of tiles, three CTAs instead of two on an SM: 479 / 1000; with sixteen warps of four tokens: 329 / 991 (one CTA on an SM).
 template <typename XT, typename ZT0, typename ZT1, int kX, int kPairs>
