@@ -17,7 +17,7 @@
 //
 // The same walk over the tiles of several layers of one shape, without the squared ReLU (batch_by_tiles): the layers behind a token shift where
 // their weights are too deep to stay in shared memory.  One by one, 12544 x 768 x 768 is a single round of the library's tiles, whose start and
-// end nothing covers: four layers 58.1 us, in one launch 50.6; VRWKV6-B on 64 images 8310 -> 8143 us.  Same bits.
+// end nothing covers: four layers 58.1 us, in one launch 50.6; VRWKV6-B on 64 images 8310 -> 8143 us.
 //
 // Every wait is bounded; one that gives up sets a flag that ends the other roles, and the host-visible word of failures.
 #include <cuda_bf16.h>
